@@ -6,6 +6,8 @@ the shared object is missing, importing this module raises.
 import ctypes
 import os
 
+import torch  # noqa: F401  (loads the libraries _host.so links against)
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libftb200.so")
 
@@ -63,6 +65,11 @@ def load():
 
 
 lib = load()
+
+try:
+    from . import _host as host  # native front of the short calls; needs torch and libftb200.so loaded
+except ImportError as e:
+    raise ImportError("_host.so is not built (%s); run `python -m fractaltensor_b200.build`" % e)
 
 
 class FtbError(RuntimeError):

@@ -1,4 +1,5 @@
-"""Builds libftb200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libftb200.so (the C-ABI library) in-tree with nvcc for sm_100a, and _host.so, the
+Python module in front of its short calls, with g++ against the installed torch.
 
 Run as ``python -m fractaltensor_b200.build``.  The library links the CUDA
 runtime statically and looks the driver's tensor-map encoder up at run time, so
@@ -11,6 +12,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libftb200.so")
+HOST_SRC = os.path.join(CSRC, "host_calls.cpp")
+HOST = os.path.join(HERE, "_host.so")
 SOURCES = ["tmap.cu", "pack.cu", "cell_gemm.cu", "cell_simt.cu", "lstm_simt_static.cu", "lstm_static.cu", "lstm_wmajor.cu", "rnn_cluster.cu", "wavefront.cu", "b2b_gemm.cu", "flash_attn.cu",
            "online_softmax.cu", "embedding.cu", "sparse_attn.cu", "rnn_attention.cu"]
 NVCC_FLAGS = [
@@ -24,12 +27,30 @@ def _newer(a, b):
     return (not os.path.exists(b)) or os.path.getmtime(a) > os.path.getmtime(b)
 
 
+def _host_flags():
+    """Compile and link flags of _host.so (a plain CPython module that reads torch tensors)."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [sysconfig.get_paths()["include"], os.path.join(root, "include"),
+           os.path.join(root, "include", "torch", "csrc", "api", "include"), "/usr/local/cuda/include"]
+    cflags = ["-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden",
+              "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + ["-I" + d for d in inc]
+    ldflags = ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+               "-L" + HERE, "-l:libftb200.so", "-Wl,-rpath,$ORIGIN"]
+    return cflags, ldflags
+
+
 def build(verbose=False, force=False):
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
-    headers.append(os.path.join(HERE, "..", "include", "ftb200.h"))
+    api = os.path.join(HERE, "..", "include", "ftb200.h")
+    headers.append(api)
     objs = []
     procs = []
+    start = lambda name, cmd: procs.append(
+        (name, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     for src in SOURCES:
         s = os.path.join(CSRC, src)
         if not os.path.exists(s):
@@ -37,8 +58,13 @@ def build(verbose=False, force=False):
         o = os.path.join(CSRC, src.replace(".cu", ".o"))
         objs.append(o)
         if force or _newer(s, o) or any(_newer(h, o) for h in headers):
-            cmd = [nvcc] + NVCC_FLAGS + ["-c", s, "-o", o]
-            procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+            start(src, [nvcc] + NVCC_FLAGS + ["-c", s, "-o", o])
+    link_lib = bool(procs) or not os.path.exists(LIB)
+    host_obj = HOST_SRC.replace(".cpp", ".o")
+    build_host = force or _newer(HOST_SRC, HOST) or _newer(api, HOST)
+    if build_host:
+        cflags, ldflags = _host_flags()
+        start(os.path.basename(HOST_SRC), ["g++"] + cflags + ["-c", HOST_SRC, "-o", host_obj])
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
@@ -46,10 +72,12 @@ def build(verbose=False, force=False):
             sys.stderr.write("== %s ==\n%s\n" % (src, out))
         failed = failed or p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed")
-    if procs or not os.path.exists(LIB):
+        raise RuntimeError("compilation failed")
+    if link_lib:
         cmd = [nvcc, "-shared", "-Wno-deprecated-gpu-targets", "-o", LIB] + objs + ["-cudart", "static"]
         subprocess.check_call(cmd)
+    if build_host:
+        subprocess.check_call(["g++", "-shared", "-o", HOST, host_obj] + ldflags)
     return LIB
 
 

@@ -1,0 +1,225 @@
+// Native front of the short calls in ops.py.
+//
+// A back-to-back GEMM of 2 MB or one attention head block runs for 5..10 us on the device, while the
+// checks, attribute reads, context managers and ctypes conversions of the Python path cost 17 us of
+// host time per call: such a call was bound by the host, whatever the kernel did.  The functions here
+// take the call's objects as they are, read shapes, types and pointers from the tensors in C++,
+// allocate the result through the same caching allocator and enter the C ABI with the current
+// stream of the inputs' device (4..6 us per call, most of it the allocation and the launch).
+//
+// They are the accepting half only: whatever is not the plain, valid call (a wrong type or shape, a
+// tensor on the CPU, no workspace on that device yet, an error from the library) is answered with
+// None before anything is launched, and ops.py goes through its Python checks, which raise.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/ftb200.h"
+
+namespace {
+
+// A contiguous CUDA tensor, or nullptr.
+const at::Tensor* cuda_tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.is_contiguous() ? &t : nullptr;
+}
+
+int dtype_code(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return FTB_DTYPE_F32;
+    case at::kHalf: return FTB_DTYPE_F16;
+    case at::kBFloat16: return FTB_DTYPE_BF16;
+    default: return -1;
+  }
+}
+
+bool same_kind(const at::Tensor& a, const at::Tensor& b) {
+  return a.scalar_type() == b.scalar_type() && a.device() == b.device();
+}
+
+bool get_int(PyObject* o, int64_t* v) {
+  if (!PyLong_CheckExact(o)) return false;
+  int overflow = 0;
+  *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return overflow == 0 && *v >= -0x7fffffffLL && *v <= 0x7fffffffLL;
+}
+
+bool get_float(PyObject* o, float* v) {
+  if (!PyFloat_CheckExact(o)) return false;
+  *v = static_cast<float>(PyFloat_AS_DOUBLE(o));
+  return true;
+}
+
+// The workspace ops.py keeps for `dev` in its dictionary {device index: uint8 tensor}; nullptr when
+// there is none yet or it is smaller than `bytes`.
+const at::Tensor* workspace_of(PyObject* dict, c10::DeviceIndex dev, size_t bytes) {
+  PyObject* key = PyLong_FromLong(dev);
+  if (key == nullptr) return nullptr;
+  PyObject* t = PyDict_Check(dict) ? PyDict_GetItemWithError(dict, key) : nullptr;
+  Py_DECREF(key);
+  if (t == nullptr) {
+    PyErr_Clear();
+    return nullptr;
+  }
+  const at::Tensor* ws = cuda_tensor(t);
+  return ws != nullptr && static_cast<size_t>(ws->numel()) >= bytes ? ws : nullptr;
+}
+
+void* stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
+
+// `out` if the caller gave one that fits, else a new tensor; false when the given one does not fit.
+bool result(PyObject* out, const at::Tensor& like, at::IntArrayRef shape, at::Tensor* o) {
+  if (out == Py_None) {
+    *o = at::empty(shape, at::TensorOptions().dtype(like.scalar_type()).device(like.device()));
+    return true;
+  }
+  const at::Tensor* t = cuda_tensor(out);
+  if (t == nullptr || !same_kind(*t, like) || t->sizes() != shape) return false;
+  *o = *t;
+  return true;
+}
+
+#define DECLINE_UNLESS(cond) \
+  do {                       \
+    if (!(cond)) Py_RETURN_NONE; \
+  } while (0)
+
+template <typename F>
+PyObject* guarded(F f) {
+  try {
+    return f();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+// (A, B, C, out, workspaces)
+PyObject* b2b_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 5);
+    const at::Tensor *A = cuda_tensor(args[0]), *B = cuda_tensor(args[1]), *C = cuda_tensor(args[2]);
+    DECLINE_UNLESS(A && B && C && same_kind(*A, *B) && same_kind(*A, *C));
+    DECLINE_UNLESS(A->dim() == 3 && B->dim() == 3 && C->dim() == 3);
+    const int64_t batch = A->size(0), M = A->size(1), K = A->size(2), N = B->size(1), P = C->size(1);
+    DECLINE_UNLESS(B->size(0) == batch && B->size(2) == K && C->size(0) == batch && C->size(2) == N);
+    DECLINE_UNLESS(batch <= 0x7fffffff && M <= 0x7fffffff);
+    const int dt = dtype_code(*A);
+    DECLINE_UNLESS(dt >= 0);
+    const c10::DeviceIndex dev = A->device().index();
+    const at::Tensor* ws = workspace_of(args[4], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws);
+    const c10::cuda::CUDAGuard guard(dev);
+    at::Tensor out;
+    DECLINE_UNLESS(result(args[3], *A, {batch, M, P}, &out));
+    const int rc = ftb_b2b_gemm(A->data_ptr(), B->data_ptr(), C->data_ptr(), out.data_ptr(), static_cast<int>(batch),
+                                static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(P), dt,
+                                ws->data_ptr(), ws->numel(), stream_of(dev));
+    DECLINE_UNLESS(rc == 0);
+    return THPVariable_Wrap(out);
+  });
+}
+
+// (q, k, v, out, scale, mode, left, right, workspaces); mode 0 full, 1 causal, 2 window (`left` keys
+// that end at the query), 3 local
+PyObject* flash_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 9);
+    const at::Tensor *q = cuda_tensor(args[0]), *k = cuda_tensor(args[1]), *v = cuda_tensor(args[2]);
+    DECLINE_UNLESS(q && k && v && same_kind(*q, *k) && same_kind(*q, *v) && q->dim() == 4);
+    DECLINE_UNLESS(k->sizes() == q->sizes() && v->sizes() == q->sizes());
+    float scale;
+    int64_t mode, left, right;
+    DECLINE_UNLESS(get_float(args[4], &scale) && get_int(args[5], &mode) && get_int(args[6], &left) &&
+                   get_int(args[7], &right));
+    for (int i = 0; i < 4; ++i) DECLINE_UNLESS(q->size(i) <= 0x7fffffff);
+    const int B = static_cast<int>(q->size(0)), h = static_cast<int>(q->size(1)), S = static_cast<int>(q->size(2)),
+              d = static_cast<int>(q->size(3)), dt = dtype_code(*q);
+    DECLINE_UNLESS(dt >= 0);
+    const c10::DeviceIndex dev = q->device().index();
+    const at::Tensor* ws = workspace_of(args[8], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws);
+    const c10::cuda::CUDAGuard guard(dev);
+    at::Tensor out;
+    DECLINE_UNLESS(result(args[3], *q, q->sizes(), &out));
+    const void *qp = q->data_ptr(), *kp = k->data_ptr(), *vp = v->data_ptr();
+    void *op = out.data_ptr(), *wp = ws->data_ptr(), *st = stream_of(dev);
+    const size_t wb = ws->numel();
+    int rc;
+    switch (mode) {
+      case 0: rc = ftb_flash_attn_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
+      case 1: rc = ftb_flash_attn_causal_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
+      case 2:
+        rc = ftb_flash_attn_window_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), scale, dt, wp, wb, st);
+        break;
+      default:
+        rc = ftb_flash_attn_local_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), static_cast<int>(right),
+                                      scale, dt, wp, wb, st);
+    }
+    DECLINE_UNLESS(rc == 0);
+    return THPVariable_Wrap(out);
+  });
+}
+
+// (q, k, v, rand_pos | None, out, window, dilation, n_global, scale, as_shipped, workspaces)
+PyObject* sparse_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 11);
+    const at::Tensor *q = cuda_tensor(args[0]), *k = cuda_tensor(args[1]), *v = cuda_tensor(args[2]);
+    DECLINE_UNLESS(q && k && v && same_kind(*q, *k) && same_kind(*q, *v) && q->dim() == 4);
+    DECLINE_UNLESS(k->sizes() == q->sizes() && v->sizes() == q->sizes());
+    int64_t window, dilation, ng;
+    float scale;
+    DECLINE_UNLESS(get_int(args[5], &window) && get_int(args[6], &dilation) && get_int(args[7], &ng) &&
+                   get_float(args[8], &scale) && (args[9] == Py_True || args[9] == Py_False));
+    for (int i = 0; i < 4; ++i) DECLINE_UNLESS(q->size(i) <= 0x7fffffff);
+    const int64_t S = q->size(2), inner = S - 2 * ng;
+    DECLINE_UNLESS(ng >= 0 && inner >= 0);
+    int64_t R = 0;
+    const int* pos = nullptr;
+    if (args[3] != Py_None) {
+      const at::Tensor* p = cuda_tensor(args[3]);
+      DECLINE_UNLESS(p && p->scalar_type() == at::kInt && p->device() == q->device() && p->dim() == 4);
+      DECLINE_UNLESS(p->size(0) == q->size(0) && p->size(1) == q->size(1) && p->size(2) == inner);
+      R = p->size(3);
+      DECLINE_UNLESS(R <= 0x7fffffff);
+      if (R > 0) pos = static_cast<const int*>(p->data_ptr());
+    }
+    const int dt = dtype_code(*q);
+    DECLINE_UNLESS(dt >= 0);
+    const c10::DeviceIndex dev = q->device().index();
+    const at::Tensor* ws = workspace_of(args[10], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws);
+    const c10::cuda::CUDAGuard guard(dev);
+    at::Tensor out;
+    DECLINE_UNLESS(result(args[4], *q, q->sizes(), &out));
+    const int rc = ftb_sparse_attn_fwd(q->data_ptr(), k->data_ptr(), v->data_ptr(), pos, out.data_ptr(),
+                                       static_cast<int>(q->size(0)), static_cast<int>(q->size(1)), static_cast<int>(S),
+                                       static_cast<int>(q->size(3)), static_cast<int>(window), static_cast<int>(dilation),
+                                       static_cast<int>(ng), static_cast<int>(R), scale, args[9] == Py_True ? 1 : 0, dt,
+                                       ws->data_ptr(), ws->numel(), stream_of(dev));
+    DECLINE_UNLESS(rc == 0);
+    return THPVariable_Wrap(out);
+  });
+}
+
+template <typename F>
+PyCFunction as_method(F f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)); }
+
+PyMethodDef kMethods[] = {
+    {"b2b_gemm", as_method(b2b_gemm), METH_FASTCALL, nullptr},
+    {"flash_attention", as_method(flash_attention), METH_FASTCALL, nullptr},
+    {"sparse_attention", as_method(sparse_attention), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Native front of the short calls in ops.py.", -1, kMethods,
+                       nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }

@@ -72,12 +72,24 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, u
   return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
 }
 
+namespace {
+// What a device is does not change: its attributes are asked for once (0 = not asked yet).  Devices
+// past the table are asked on every call.
+constexpr int kKnownDevices = 64;
+std::atomic<int> g_major[kKnownDevices], g_sms[kKnownDevices];
+
+int device_attribute(cudaDeviceAttr attr, std::atomic<int>* known) {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+  if (dev < kKnownDevices && (v = known[dev].load(std::memory_order_relaxed)) != 0) return v;
+  if (cudaDeviceGetAttribute(&v, attr, dev) != cudaSuccess) return 0;
+  if (dev < kKnownDevices) known[dev].store(v, std::memory_order_relaxed);
+  return v;
+}
+}  // namespace
+
 int check_device_sm100() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return FTB_ERR_ARCH;
-  int major = 0;
-  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return FTB_ERR_ARCH;
-  return major == 10 ? FTB_OK : FTB_ERR_ARCH;
+  return device_attribute(cudaDevAttrComputeCapabilityMajor, g_major) == 10 ? FTB_OK : FTB_ERR_ARCH;
 }
 
 namespace {
@@ -86,11 +98,6 @@ std::atomic<long long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launches_so_far() { return g_launches.load(std::memory_order_relaxed); }
 
-int current_sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  return n;
-}
+int current_sm_count() { return device_attribute(cudaDevAttrMultiProcessorCount, g_sms); }
 
 }  // namespace ftb

@@ -12,7 +12,7 @@ import ctypes
 import torch
 
 from . import _lib
-from ._lib import check, lib
+from ._lib import check, host, lib
 
 _DT = {torch.float32: _lib.DTYPE_F32, torch.float16: _lib.DTYPE_F16, torch.bfloat16: _lib.DTYPE_BF16}
 
@@ -251,6 +251,9 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
 # ------------------------------------------------------------ B2B GEMM / attention
 def b2b_gemm(A, B, C, out=None):
     """A: [batch,M,K]; B: [batch,N,K]; C: [batch,P,N] -> D [batch,M,P] = (A.B^T).C^T per batch entry."""
+    done = host.b2b_gemm(A, B, C, out, _workspaces)
+    if done is not None:
+        return done
     _req(A, "A")
     _req(B, "B", A.dtype)
     _req(C, "C", A.dtype)
@@ -272,6 +275,18 @@ def b2b_gemm(A, B, C, out=None):
 def flash_attention(q, k, v, scale=None, out=None, causal=False, window=None, local=None):
     """q,k,v: [B,heads,S,d] -> softmax(scale * q k^T) v, same shape; `causal`: keys 0..i for query i;
     `window` (with causal): keys i-window+1..i; `local=(left, right)`: keys i-left..i+right."""
+    # the plain calls, by mask: full, causal, window, local
+    sc = 1.0 if scale is None else scale
+    done = None
+    if local is None and window is None:
+        done = host.flash_attention(q, k, v, out, sc, 1 if causal else 0, 0, 0, _workspaces)
+    elif local is None:
+        if causal:
+            done = host.flash_attention(q, k, v, out, sc, 2, window, 0, _workspaces)
+    elif window is None and not causal:
+        done = host.flash_attention(q, k, v, out, sc, 3, local[0], local[1], _workspaces)
+    if done is not None:
+        return done
     _req(q, "q")
     _req(k, "k", q.dtype)
     _req(v, "v", q.dtype)
@@ -316,6 +331,10 @@ def sparse_attention(q, k, v, rand_pos, window_size=5, dilation=2, n_global=3, s
     `as_shipped=True` reproduces the softmax dimension the example actually runs with (dim 0:
     windowed tokens get the plain sum of their values, the global block is normalised over the
     queries); False normalises over the keys."""
+    done = host.sparse_attention(q, k, v, rand_pos, out, window_size, dilation, n_global, scale, as_shipped,
+                                 _workspaces)
+    if done is not None:
+        return done
     _req(q, "q")
     _req(k, "k", q.dtype)
     _req(v, "v", q.dtype)
