@@ -1,16 +1,22 @@
-// Attention step of the attention RNN (examples/rnn_attention/rnn_attention.py:52-70, attn_func):
+// Attention of the attention RNN (examples/rnn_attention/rnn_attention.py:52-70, attn_func):
 //
 //   scores_j = e_j @ encoder_proj + decoder @ decoder_proj      (one number per encoder position)
 //   weights  = softmax over the encoder positions j
 //   v        = sum_j weights_j * e_j
 //
-// for every sequence of the batch at one decoder step.  The decoder state itself,
+// for every sequence of the batch and every decoder step.  The decoder state itself,
 // tanh(y_t @ W + v_{t-1} @ U + b), is a cell of the wavefront (csrc/cell_gemm.cu / cell_simt.cu);
 // this file holds what surrounds it: the scores e_j @ encoder_proj, which do not depend on the
-// decoder step and are computed once per call, and the softmax-weighted sum of the encoder rows.
+// decoder step and are computed once per call, and the softmax-weighted sums of the encoder rows.
+//
+// The decoder adds the same number to every score of a step, and a softmax does not change when all
+// its scores move by one number: v_t is the softmax-weighted sum over e_j @ encoder_proj alone.  So
+// the recurrent input of every decoder cell is known as soon as the encoder is done, and the
+// decoder, a chain of Lt cells and Lt attention steps as written, runs as one matrix product over all
+// steps followed by one launch of the attention over all steps (ftb_rnn_attention_fwd).
 //
 // Layout: time-major padded batches, row (j, n) of `enc` at (j * N + n) * H.  Sequence n attends to
-// encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  HBM/L2-bound row work: per
+// encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: per
 // decoder step and sequence the kernel reads len * H encoder elements (they stay in L2 across the
 // steps) and writes H.
 #include "../../include/ftb200.h"
@@ -63,19 +69,21 @@ row_dot_kernel(const T* __restrict__ rows, const T* __restrict__ proj, float* __
   }
 }
 
-// One decoder step.  grid = (N, ceil(H / 128)); CTA (n, cb) computes columns cb * 128 .. of v for
-// sequence n.  Every CTA of a sequence recomputes the len weights (a dot product over H and a
+// Attention vectors.  grid = (N, ceil(H / 128), steps); CTA (n, cb, t) computes columns cb * 128 .. of
+// v_t for sequence n from the decoder states dec [Lt, N, H] of its step.  dec == nullptr: the scores
+// of the encoder alone, and the one result goes to the rows of `copies` steps (the recurrent inputs of
+// the decoder cells).  Every CTA of a sequence recomputes the len weights (a dot product over H and a
 // softmax over len numbers: small next to the len x 128 weighted sum).
 template <typename T>
 __global__ void __launch_bounds__(kStepThreads)
-attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores, const T* __restrict__ dec_t,
-                 const T* __restrict__ dec_proj, const int* __restrict__ src_lens, T* __restrict__ out_t, int Ls,
-                 int N, int H) {
+attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores, const T* __restrict__ dec,
+                 const T* __restrict__ dec_proj, const int* __restrict__ src_lens, T* __restrict__ out, int copies,
+                 int Ls, int N, int H) {
   extern __shared__ float s_w[];  // [Ls] scores, then weights
   __shared__ float s_red[kStepThreads / 32];
   const int n = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // Launched behind the decoder cell of this step; the next step's cell may be scheduled now and
-  // waits for this kernel before it reads the attention vectors.
+  const long long step_elems = static_cast<long long>(N) * H;
+  const T* dec_t = dec == nullptr ? nullptr : dec + blockIdx.z * step_elems + static_cast<long long>(n) * H;
   grid_launch_dependents();
   grid_dependency_wait();
   int len = src_lens ? src_lens[n] : Ls;
@@ -83,7 +91,8 @@ attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores
 
   // c = decoder . decoder_proj
   float part = 0.f;
-  for (int h = tid; h < H; h += kStepThreads) part = fmaf(ld_f32<T>(dec_t + static_cast<long long>(n) * H + h), ld_f32<T>(dec_proj + h), part);
+  if (dec_t != nullptr)
+    for (int h = tid; h < H; h += kStepThreads) part = fmaf(ld_f32<T>(dec_t + h), ld_f32<T>(dec_proj + h), part);
   part = warp_sum(part);
   if (lane == 0) s_red[wid] = part;
   __syncthreads();
@@ -124,19 +133,19 @@ attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores
   const int h = blockIdx.y * kStepThreads + tid;
   if (h >= H) return;
   const T* col = enc + static_cast<long long>(n) * H + h;
-  const long long stride = static_cast<long long>(N) * H;
   float acc = 0.f;
   int j = 0;
   for (; j + 4 <= len; j += 4) {
-    const float e0 = ld_f32<T>(col + (j + 0) * stride), e1 = ld_f32<T>(col + (j + 1) * stride);
-    const float e2 = ld_f32<T>(col + (j + 2) * stride), e3 = ld_f32<T>(col + (j + 3) * stride);
+    const float e0 = ld_f32<T>(col + (j + 0) * step_elems), e1 = ld_f32<T>(col + (j + 1) * step_elems);
+    const float e2 = ld_f32<T>(col + (j + 2) * step_elems), e3 = ld_f32<T>(col + (j + 3) * step_elems);
     acc = fmaf(s_w[j], e0, acc);
     acc = fmaf(s_w[j + 1], e1, acc);
     acc = fmaf(s_w[j + 2], e2, acc);
     acc = fmaf(s_w[j + 3], e3, acc);
   }
-  for (; j < len; ++j) acc = fmaf(s_w[j], ld_f32<T>(col + j * stride), acc);
-  st_f32<T>(out_t + static_cast<long long>(n) * H + h, acc * inv);
+  for (; j < len; ++j) acc = fmaf(s_w[j], ld_f32<T>(col + j * step_elems), acc);
+  T* o = out + blockIdx.z * step_elems + static_cast<long long>(n) * H + h;
+  for (int k = 0; k < copies; ++k) st_f32<T>(o + k * step_elems, acc * inv);
 }
 
 template <typename T>
@@ -152,12 +161,13 @@ int enc_scores_t(const void* enc, const void* proj, float* scores, long long n_r
 }
 
 template <typename T>
-int attn_step_t(const void* enc, const float* enc_scores, const void* dec_t, const void* dec_proj, const int* src_lens,
-                void* out_t, int Ls, int N, int H, cudaStream_t stream) {
-  const dim3 grid(N, (H + kStepThreads - 1) / kStepThreads);
+int attn_steps_t(const void* enc, const float* enc_scores, const void* dec, const void* dec_proj, const int* src_lens,
+                 void* out, int steps, int Ls, int N, int H, cudaStream_t stream) {
+  const dim3 grid(N, (H + kStepThreads - 1) / kStepThreads, dec == nullptr ? 1 : steps);
   const cudaError_t err = launch_light(attn_step_kernel<T>, grid, dim3(kStepThreads), static_cast<size_t>(Ls) * sizeof(float),
-                                           stream, static_cast<const T*>(enc), enc_scores, static_cast<const T*>(dec_t),
-                                           static_cast<const T*>(dec_proj), src_lens, static_cast<T*>(out_t), Ls, N, H);
+                                           stream, static_cast<const T*>(enc), enc_scores, static_cast<const T*>(dec),
+                                           static_cast<const T*>(dec_proj), src_lens, static_cast<T*>(out),
+                                           dec == nullptr ? steps : 1, Ls, N, H);
   count_launch();
   if (err != cudaSuccess) cudaGetLastError();
   return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
@@ -177,12 +187,14 @@ int launch_enc_scores(int dtype, const void* enc, const void* proj, float* score
   }
 }
 
-int launch_attn_step(int dtype, const void* enc, const float* enc_scores, const void* dec_t, const void* dec_proj,
-                     const int* src_lens, void* out_t, int Ls, int N, int H, cudaStream_t stream) {
+// The attention vectors of `steps` decoder steps (at most 65535) into out [steps, N, H]; dec == nullptr:
+// without a decoder term, the same vectors in the rows of every step.
+int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
+                      const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream) {
   switch (dtype) {
-    case FTB_F32: return attn_step_t<float>(enc, enc_scores, dec_t, dec_proj, src_lens, out_t, Ls, N, H, stream);
-    case FTB_F16: return attn_step_t<__half>(enc, enc_scores, dec_t, dec_proj, src_lens, out_t, Ls, N, H, stream);
-    default: return attn_step_t<__nv_bfloat16>(enc, enc_scores, dec_t, dec_proj, src_lens, out_t, Ls, N, H, stream);
+    case FTB_F32: return attn_steps_t<float>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
+    case FTB_F16: return attn_steps_t<__half>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
+    default: return attn_steps_t<__nv_bfloat16>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
   }
 }
 

@@ -57,8 +57,8 @@ int pack_rnn(const void* W, const void* U, void* Wp, int I, int H, int dtype, cu
 int rnn_attention_max_src_len();
 int launch_enc_scores(int dtype, const void* enc, const void* proj, float* scores, long long n_rows, int H,
                       cudaStream_t stream);
-int launch_attn_step(int dtype, const void* enc, const float* enc_scores, const void* dec_t, const void* dec_proj,
-                     const int* src_lens, void* out_t, int Ls, int N, int H, cudaStream_t stream);
+int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
+                      const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream);
 int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, cudaStream_t stream);
 
 namespace {
@@ -1180,22 +1180,32 @@ int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, 
   }
   rc = launch_enc_scores(dtype, enc, enc_proj, enc_scores, static_cast<long long>(Ls) * N, H, stream);
   if (rc) return rc;
-  // Decoder: the cell, then the attention over the encoder rows; its result is both the step's
-  // output and the next step's recurrent input.
-  for (int t = 0; t < Lt; ++t) {
+  // Decoder.  The attention vector of a step does not depend on the decoder (its term moves all scores
+  // of a softmax by one number), so the recurrent inputs of steps 1.. are known here: they go to the
+  // rows of `out` they are read from, all decoder cells run as one level, and the attention over all
+  // steps writes the result over them.  (As a chain: two dependent launches per step.)
+  if (Lt > 1) {
+    rc = launch_attn_steps(dtype, enc, enc_scores, nullptr, dec_proj, src_lens, out, Lt - 1, Ls, N, H, stream);
+    if (rc) return rc;
+  }
+  items.clear();
+  for (int t = 0; t < std::min(Lt, 2); ++t) {  // step 0 has no recurrent input; steps 1.. are consecutive rows
     CellItem it = blank_item();
     add_seg(it, 1, static_cast<int64_t>(t) * N, H, 0);
-    if (t > 0) add_seg(it, 3, static_cast<int64_t>(t - 1) * N, H, H);
-    it.rows = N;
+    if (t > 0) add_seg(it, 3, 0, H, H);
+    it.rows = t == 0 ? N : (Lt - 1) * N;
     it.w_map = 1;
     it.bias = bias_trg;
-    char* dec_t = static_cast<char*>(dec) + static_cast<size_t>(t) * N * H * es;
-    it.out = dec_t;
-    items[0] = it;
-    rc = cl.run(items);
-    if (rc) return rc;
-    rc = launch_attn_step(dtype, enc, enc_scores, dec_t, dec_proj, src_lens,
-                          static_cast<char*>(out) + static_cast<size_t>(t) * N * H * es, Ls, N, H, stream);
+    it.out = static_cast<char*>(dec) + static_cast<size_t>(t) * N * H * es;
+    items.push_back(it);
+  }
+  rc = cl.run(items);
+  if (rc) return rc;
+  constexpr int kMostSteps = 65535;  // of one launch
+  for (int t = 0; t < Lt; t += kMostSteps) {
+    const size_t at = static_cast<size_t>(t) * N * H * es;
+    rc = launch_attn_steps(dtype, enc, enc_scores, static_cast<char*>(dec) + at, dec_proj, src_lens,
+                           static_cast<char*>(out) + at, std::min(kMostSteps, Lt - t), Ls, N, H, stream);
     if (rc) return rc;
   }
   return FTB_OK;

@@ -265,7 +265,9 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * Outputs (caller-owned): enc [Ls, N, H] encoder states, enc_scores fp32 [Ls, N] (e_j.enc_proj),
  * dec [Lt, N, H] decoder states, out [Lt, N, H] the attention vectors.  Rows of a sequence past its
  * own source / target length hold values nobody should read.  H % 64 == 0, Ls <= 12288.
- * One launch per source position, one for the scores, two per target position. */
+ * The decoder's term is the same for every score of a step and leaves the softmax as it is, so the
+ * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.
+ * One launch per source position and four for the rest. */
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
