@@ -59,6 +59,9 @@ int launch_enc_scores(int dtype, const void* enc, const void* proj, float* score
                       cudaStream_t stream);
 int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
                       const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream);
+bool rnn_chain_supported(int dtype, int H);
+int launch_rnn_chain(int dtype, const float* pre, const void* Wp, int ldw, int k0, const float* bias,
+                     const void* before, void* out, int steps, int N, int H, int* status, cudaStream_t stream);
 int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, cudaStream_t stream);
 
 namespace {
@@ -1107,6 +1110,16 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
   return pack_rnn(W, U, Wp, I, H, dtype, static_cast<cudaStream_t>(stream));
 }
 
+// Scratch of the encoder's chain kernel: fp32 input halves of as many source steps as this allows (a
+// longer source is scanned in pieces).
+static constexpr size_t kMaxPreBytes = 32u << 20;
+
+size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype) {
+  if (Ls <= 0 || N <= 0 || H <= 0 || !rnn_chain_supported(dtype, H)) return kWorkspaceBytes;
+  const size_t step = static_cast<size_t>(N) * H * sizeof(float);
+  return kWorkspaceBytes + std::min<size_t>(Ls, kMaxPreBytes / step) * step;
+}
+
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
@@ -1165,8 +1178,29 @@ int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, 
   }
 
   std::vector<CellItem> items(1);
-  // Encoder: e_j = tanh(x_j W + e_{j-1} U + b), one level per source position.
-  for (int j = 0; j < Ls; ++j) {
+  // Encoder: e_j = tanh(x_j W + e_{j-1} U + b).  With room for the fp32 input halves x_j W of at least
+  // one step in the workspace: those as one product, then the scan as one launch of the chain kernel
+  // (csrc/rnn_chain.cu), piece by piece; else one level per source position.
+  const size_t pre_step = static_cast<size_t>(N) * H * sizeof(float);
+  const int piece = rnn_chain_supported(dtype, H)
+                        ? static_cast<int>(std::min<size_t>(Ls, (workspace_bytes - kWorkspaceBytes) / pre_step)) : 0;
+  for (int j = 0; j < Ls && piece > 0; j += piece) {
+    const int steps = std::min(piece, Ls - j);
+    float* pre = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceBytes);
+    CellLauncher gemm = cl;
+    gemm.epi = EPI_STORE_F32;
+    items[0] = blank_item();
+    add_seg(items[0], 0, static_cast<int64_t>(j) * N, H, 0);
+    items[0].rows = steps * N;
+    items[0].out = pre;
+    rc = gemm.run(items);
+    if (rc) return rc;
+    char* enc_j = static_cast<char*>(enc) + static_cast<size_t>(j) * N * H * es;
+    rc = launch_rnn_chain(dtype, pre, Wp_src, K, H, bias_src, j > 0 ? enc_j - static_cast<size_t>(N) * H * es : nullptr,
+                          enc_j, steps, N, H, status, stream);
+    if (rc) return rc;
+  }
+  for (int j = 0; j < Ls && piece == 0; ++j) {
     CellItem it = blank_item();
     add_seg(it, 0, static_cast<int64_t>(j) * N, H, 0);
     if (j > 0) add_seg(it, 2, static_cast<int64_t>(j - 1) * N, H, H);

@@ -406,7 +406,7 @@ def rnn_attention(src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc_proj, dec_pr
     dec = torch.empty_like(trg)
     out = torch.empty_like(trg)
     scores = torch.empty(Ls, N, dtype=torch.float32, device=src.device)
-    ws = workspace(src.device)
+    ws = workspace(src.device, lib.ftb_rnn_attention_workspace_bytes(Ls, N, H, _dtype_code(src)))
     opt = lambda t: _ptr(t) if t is not None else None
     with torch.cuda.device(src.device):
         check(lib.ftb_rnn_attention_fwd(_ptr(src), _ptr(trg), _ptr(Wp_src), _ptr(Wp_trg), opt(bias_src), opt(bias_trg),

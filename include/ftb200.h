@@ -267,7 +267,9 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * own source / target length hold values nobody should read.  H % 64 == 0, Ls <= 12288.
  * The decoder's term is the same for every score of a step and leaves the softmax as it is, so the
  * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.
- * One launch per source position and four for the rest. */
+ * With workspace_bytes >= ftb_rnn_attention_workspace_bytes() (16-bit types, H <= 512) the encoder is one
+ * matrix product and one scan kernel; else one launch per source position.  Four launches for the rest. */
+size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype);
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
