@@ -194,7 +194,9 @@ b2b_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    {
+      const bool leader = elect_one();
       constexpr uint32_t idesc1 = make_idesc_f16(128, 128, Fmt<T>::kind, 0, 0);
       constexpr uint32_t idesc2 = make_idesc_f16(128, PP, Fmt<T>::kind, 0, 0);
       const uint32_t aBC = smem_u32(sBC);
@@ -211,30 +213,32 @@ b2b_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         const int b = (first + i) / sh.tiles_per_batch;
         const int n = b - batch0;
         if (b != cur_batch) {
-          if (!mbar_wait(&bc_full[bc_pair(n)], bc_use(n) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
+          if (!mbar_wait_warp(&bc_full[bc_pair(n)], bc_use(n) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
           cur_batch = b;
         }
-        if (c == 0 && !mbar_wait(&a_full[stage], a_phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
+        if (c == 0 && !mbar_wait_warp(&a_full[stage], a_phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
         // (No tcgen05 fence: TMA completes both barriers, and the accumulator's previous contents were
         // consumed by an MMA this thread issued earlier.)
-        if (u == 0) B2B_WALL(1);
+        if (u == 0 && leader) B2B_WALL(1);
         const uint64_t dA = make_sdesc_sw128(smem_u32(sA + stage * sh.a_bytes), 16, 1024);
         const uint64_t dB = make_sdesc_sw128(aBC + bc_pair(n) * bc_pair_bytes + c * (kTile * kSlabBytes), 16, 1024);
         const uint32_t slabB = (sh.N * kSlabBytes) >> 4;
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < KK / 16; ++k) {
-          const uint32_t offA = ((k >> 2) * (kTile * kSlabBytes) + (k & 3) * 32) >> 4;
-          const uint32_t offB = (k >> 2) * slabB + (k & 3) * 2;
-          umma_ss(tmem_base + (u & 1) * 128, dA + offA, dB + offB, idesc1, k != 0 ? 1u : 0u);
+          for (int k = 0; k < KK / 16; ++k) {
+            const uint32_t offA = ((k >> 2) * (kTile * kSlabBytes) + (k & 3) * 32) >> 4;
+            const uint32_t offB = (k >> 2) * slabB + (k & 3) * 2;
+            umma_ss(tmem_base + (u & 1) * 128, dA + offA, dB + offB, idesc1, k != 0 ? 1u : 0u);
+          }
         }
         if (c == nchunks - 1) {
-          umma_commit(&a_empty[stage]);
+          if (leader) umma_commit(&a_empty[stage]);
           if (++stage == kAStages) {
             stage = 0;
             a_phase ^= 1u;
           }
         }
-        umma_commit(&s_full[u & 1]);
+        if (leader) umma_commit(&s_full[u & 1]);
         return true;
       };
       // Second product of unit u: O[i&1] (+)= P_u . C_c^T, P from TMEM (16 of the chunk's 128
@@ -244,19 +248,21 @@ b2b_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         const int ob = i & 1;
         const int n = (first + i) / sh.tiles_per_batch - batch0;
         const uint32_t aC = aBC + bc_pair(n) * bc_pair_bytes + sh.b_bytes;
-        if (c == 0 && !mbar_wait(&o_empty[ob], ((i >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
+        if (c == 0 && !mbar_wait_warp(&o_empty[ob], ((i >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
         // One barrier per S/P buffer: the converting warps can be a whole unit ahead of this wait
         // (S of the next unit is ready early), and a parity wait must not fall two phases behind.
-        if (!mbar_wait(&p_full[u & 1], (u >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
+        if (!mbar_wait_warp(&p_full[u & 1], (u >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
         tc_fence_after();
         const uint64_t dC = make_sdesc_sw128(aC + (2 * c) * (PP * kSlabBytes), 16, 1024);
+        if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t offC = ((kk >> 2) * (PP * kSlabBytes) + (kk & 3) * 32) >> 4;
-          umma_ts(tmem_base + 256 + ob * 128, tmem_base + (u & 1) * 128 + kk * 8, dC + offC, idesc2,
-                  (c | kk) != 0 ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk) {
+            const uint32_t offC = ((kk >> 2) * (PP * kSlabBytes) + (kk & 3) * 32) >> 4;
+            umma_ts(tmem_base + 256 + ob * 128, tmem_base + (u & 1) * 128 + kk * 8, dC + offC, idesc2,
+                    (c | kk) != 0 ? 1u : 0u);
+          }
         }
-        if (c == nchunks - 1) {
+        if (leader && c == nchunks - 1) {
           umma_commit(&o_full[ob]);
           if (last_of_batch) umma_commit(&bc_empty[bc_pair(n)]);
         }

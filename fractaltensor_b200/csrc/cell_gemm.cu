@@ -312,7 +312,9 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && rank == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    if (rank == 0) {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(PAIR ? 2 * BM : BM, BN, Fmt<T>::kind, 0, 0);
       ItemCursor<PERSIST> cur(batch, plan);
       int stage = 0;
@@ -329,28 +331,30 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
         const CellItem* it = cur.seek(tile);
         int nkb = 0;
         for (int s = 0; s < it->nseg; ++s) nkb += it->seg_kb[s];
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) break;
+        if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < nkb; ++kb) {
           // (No tcgen05 fence after a barrier that TMA completes: it would drain the tensor pipe.)
-          if (!mbar_wait(&full_bar[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) {
+          if (!mbar_wait_warp(&full_bar[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) {
             ok = false;
             break;
           }
           const uint64_t ad = a_desc0 + stage_off;
           const uint64_t bd = b_desc0 + stage_off;
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
+            for (int k = 0; k < BK / 16; ++k) {
+              if (PAIR)
+                umma_ss_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+              else
+                umma_ss(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            }
             if (PAIR)
-              umma_ss_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+              umma_commit_pair(&empty_bar[stage]);
             else
-              umma_ss(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+              umma_commit(&empty_bar[stage]);
           }
-          if (PAIR)
-            umma_commit_pair(&empty_bar[stage]);
-          else
-            umma_commit(&empty_bar[stage]);
           stage_off += C::kStageBytes >> 4;
           if (++stage == S) {
             stage = 0;
@@ -359,10 +363,12 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
           }
         }
         if (!ok) break;
-        if (PAIR)
-          umma_commit_pair(&tfull_bar[acc]);
-        else
-          umma_commit(&tfull_bar[acc]);
+        if (leader) {
+          if (PAIR)
+            umma_commit_pair(&tfull_bar[acc]);
+          else
+            umma_commit(&tfull_bar[acc]);
+        }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

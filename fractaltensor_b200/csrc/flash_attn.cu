@@ -214,7 +214,9 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    {
+      const bool leader = elect_one();
       constexpr uint32_t idesc_qk = make_idesc_f16(128, 128, Fmt<T>::kind, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc_f16(128, 128, Fmt<T>::kind, 0, 1);  // V is MN-major
       // This thread's own instructions sit between every softmax hand-off and the MMAs that follow it:
@@ -224,13 +226,13 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       const uint64_t dK = make_sdesc_sw128(smem_u32(sKV), 16, 1024);
       const uint64_t dV = make_sdesc_sw128(smem_u32(sKV), kHalfBytes, 1024);
       uint32_t full_bits = 0;  // bit s: parity of the next fill of slot s
-      bool ok = mbar_wait(&ctl.q_full, 0, s_abort, status, FTB_ERR_TIMEOUT_TMA);
+      bool ok = mbar_wait_warp(&ctl.q_full, 0, s_abort, status, FTB_ERR_TIMEOUT_TMA);
 
       // (No tcgen05 fence after these waits: TMA completes the barriers, and the fence would drain the
       // tensor pipe.)
       auto wait_slot = [&](int n) -> bool {  // n-th tile of the K0, V0, K1, V1, ... stream
         const int slot = n % kKVSlots;
-        if (!mbar_wait(&ctl.kv_full[slot], (full_bits >> slot) & 1u, s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
+        if (!mbar_wait_warp(&ctl.kv_full[slot], (full_bits >> slot) & 1u, s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
         full_bits ^= 1u << slot;
         return true;
       };
@@ -238,30 +240,34 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       auto issue_s = [&](int t, int j) {
         const uint64_t dq = dQ + static_cast<uint64_t>((t * kTileBytes) >> 4);
         const uint64_t dk = dK + static_cast<uint64_t>((((2 * j) % kKVSlots) * kTileBytes) >> 4);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
-          umma_ss(tmem_base + t * 128, dq + off, dk + off, idesc_qk, k != 0 ? 1u : 0u);
+          for (int k = 0; k < 8; ++k) {
+            const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
+            umma_ss(tmem_base + t * 128, dq + off, dk + off, idesc_qk, k != 0 ? 1u : 0u);
+          }
+          umma_commit(&ctl.s_full[t]);
         }
-        umma_commit(&ctl.s_full[t]);
       };
       // O_t += P_t(j) . V_j: A = P_t from TMEM (16 keys = 8 packed columns per step; the two
       // key halves start 64 columns apart); B = V, MN-major: 16 keys = two 8-row groups
       // (1024 B apart), the two 64-column halves of d are 16 KB apart.
       auto issue_pv = [&](int t, int j, bool first) {
         const uint64_t dv = dV + static_cast<uint64_t>((((2 * j + 1) % kKVSlots) * kTileBytes) >> 4);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + (k >> 2) * 64 + (k & 3) * 8, dv + k * (2048 >> 4),
-                  idesc_pv, (!first || k != 0) ? 1u : 0u);
-        umma_commit(&ctl.pv_done[t]);
+          for (int k = 0; k < 8; ++k)
+            umma_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + (k >> 2) * 64 + (k & 3) * 8, dv + k * (2048 >> 4),
+                    idesc_pv, (!first || k != 0) ? 1u : 0u);
+          umma_commit(&ctl.pv_done[t]);
+        }
       };
 
       if (ok) ok = wait_slot(0);
       if (ok) {
         issue_s(0, 0);
         if (first1 == 0) issue_s(1, 0);
-        umma_commit(&ctl.kv_empty[0]);
+        if (leader) umma_commit(&ctl.kv_empty[0]);
       }
       for (int j = 0; j < n_kv && ok; ++j) {
         const bool more = j + 1 < n_kv;
@@ -272,7 +278,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           const int last = t == 0 ? last0 : n_kv - 1;
           if (j >= first && j <= last) {
             // P_t(j) is in TMEM (and the softmax is done with S_t(j)).
-            if (!mbar_wait(&ctl.p_full[t], (j - first) & 1, s_abort, status, FTB_ERR_TIMEOUT_EPI)) {
+            if (!mbar_wait_warp(&ctl.p_full[t], (j - first) & 1, s_abort, status, FTB_ERR_TIMEOUT_EPI)) {
               ok = false;
               break;
             }
@@ -286,8 +292,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           FA_STAMP_MMA(t, j, 6);
         }
         if (!ok) break;
-        umma_commit(&ctl.kv_empty[(2 * j + 1) % kKVSlots]);
-        if (more) umma_commit(&ctl.kv_empty[(2 * j + 2) % kKVSlots]);
+        if (leader) umma_commit(&ctl.kv_empty[(2 * j + 1) % kKVSlots]);
+        if (leader && more) umma_commit(&ctl.kv_empty[(2 * j + 2) % kKVSlots]);
       }
     }
   } else {

@@ -238,7 +238,9 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && rank == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    if (rank == 0) {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(2 * BM, BN, Fmt<T>::kind, 0, 0);
       const uint64_t a_desc0 = make_sdesc_sw128(smem_u32(smem), 16, 1024);
       const uint64_t b_desc0 = make_sdesc_sw128(smem_u32(smem) + kABytes, 16, 1024);
@@ -256,15 +258,15 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
           const int nkb = is_x ? (l == 0 ? kb_x0 : kb_h) : kb_h;
           if (is_x) {
             // First MMA of tile k: its accumulator must have been drained (tile k-2).
-            if (!mbar_wait(&tempty_bar[acc], ((k >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
+            if (!mbar_wait_warp(&tempty_bar[acc], ((k >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI)) return false;
             tc_fence_after();
           }
           const uint32_t d_tmem = tmem_base + acc * BN;
-          uint32_t accumulate = is_x ? 0u : 1u;  // the first MMA of a tile overwrites the accumulator
+          // (the first MMA of a tile overwrites the accumulator)
           for (int kb = 0; kb < nkb; ++kb) {
             // (No tcgen05 fence after a barrier that TMA completes: the fence orders against other threads'
             // tcgen05 operations, which do not touch the stage, and it drains the tensor pipe.)
-            if (!mbar_wait(&full_bar[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
+            if (!mbar_wait_warp(&full_bar[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
 #ifdef FTB_TRACE
             if (a.trace && !is_x && kb == 0) a.trace[(static_cast<size_t>(l * a.L + t) * a.tiles_per_cell + tile) * 4 + 1] = globaltimer_ns();
 #endif
@@ -272,12 +274,12 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
             // stage-0 descriptors plus byte offsets / 16, nothing is rebuilt per MMA.
             const uint64_t ad = a_desc0 + stage_off;
             const uint64_t bd = b_desc0 + stage_off;
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-              umma_ss_pair(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-              accumulate = 1u;
+              for (int kk = 0; kk < BK / 16; ++kk)
+                umma_ss_pair(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, !is_x || kb > 0 || kk > 0);
+              umma_commit_pair(&empty_bar[stage]);
             }
-            umma_commit_pair(&empty_bar[stage]);
             stage_off += kStageBytes >> 4;
             if (++stage == kStages) {
               stage = 0;
@@ -286,7 +288,7 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
             }
           }
           // The tile is complete after its recurrent half (or after the input half at t = 0).
-          if (!is_x || t == 0) umma_commit_pair(&tfull_bar[acc]);
+          if (leader && (!is_x || t == 0)) umma_commit_pair(&tfull_bar[acc]);
           return true;
         });
         k_base += a.L;

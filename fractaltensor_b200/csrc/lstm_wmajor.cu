@@ -310,7 +310,9 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(BMW, NB, Fmt<T>::kind, 0, 0);
       // Operand descriptors of the ring bases; a tile further on is the base plus its byte offset / 16.
       const uint64_t act_desc0 = make_sdesc_sw128(smem_u32(s_act), 16, 1024);
@@ -332,11 +334,11 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
           bool okw = true;
           if (is_x) {
             // First MMA of tile k: its accumulators must have been drained (tile k-2).
-            okw = mbar_wait(&tempty_bar[acc], ((k >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
+            okw = mbar_wait_warp(&tempty_bar[acc], ((k >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
             if (!okw) return false;
             tc_fence_after();
           } else if (!res_ready) {
-            if (!mbar_wait(&res_full, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
+            if (!mbar_wait_warp(&res_full, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
             tc_fence_after();
             res_ready = true;
           }
@@ -346,7 +348,7 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
             if (ab == 0) {
               // (No tcgen05 fence after a barrier that TMA completes: the fence is for data handed over
               // by other threads' tcgen05 operations, and it drains the tensor pipe.)
-              okw = mbar_wait(&act_full[as], aphase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+              okw = mbar_wait_warp(&act_full[as], aphase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
               if (!is_x && kb == 0) { FTB_WM_STAMP(l, t, 2); }
               if (!is_x && kb + C::kActBlocks >= nkb) { FTB_WM_STAMP(l, t, 3); }
               if (!okw) return false;
@@ -354,22 +356,26 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
             const uint64_t bd = act_desc0 + static_cast<uint64_t>((as * kBlockBytes + ab * C::kActBlockBytes) >> 4);
             if (kb < kb_ring) {
               // weights of this K block live in TMEM: 8 columns per 16 of K
+              if (leader) {
 #pragma unroll
-              for (int kk = 0; kk < BK / 16; ++kk)
-                umma_ts(d_tmem, tmem_w + kb * 32 + kk * 8, bd + 2 * kk, idesc, 1u);
+                for (int kk = 0; kk < BK / 16; ++kk)
+                  umma_ts(d_tmem, tmem_w + kb * 32 + kk * 8, bd + 2 * kk, idesc, 1u);
+              }
             } else {
               const int wb = (kb - kb_ring) & 1;  // position inside the weight stage
               if (wb == 0) {
-                okw = mbar_wait(&w_full[ws], wphase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+                okw = mbar_wait_warp(&w_full[ws], wphase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
                 if (!okw) return false;
               }
               const uint64_t ad = w_desc0 + static_cast<uint64_t>(((2 * ws + wb) * kBlockBytes) >> 4);
               // The first MMA of a tile overwrites the accumulator.
+              if (leader) {
 #pragma unroll
-              for (int kk = 0; kk < BK / 16; ++kk)
-                umma_ss(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, (is_x && kb == 0 && kk == 0) ? 0u : 1u);
+                for (int kk = 0; kk < BK / 16; ++kk)
+                  umma_ss(d_tmem, ad + 2 * kk, bd + 2 * kk, idesc, (is_x && kb == 0 && kk == 0) ? 0u : 1u);
+              }
               if (wb == 1 || kb == nkb - 1) {
-                umma_commit(&w_empty[ws]);
+                if (leader) umma_commit(&w_empty[ws]);
                 if (++ws == WS) {
                   ws = 0;
                   wphase ^= 1u;
@@ -377,7 +383,7 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
               }
             }
             if (ab == C::kActBlocks - 1 || kb == nkb - 1) {
-              umma_commit(&act_empty[as]);
+              if (leader) umma_commit(&act_empty[as]);
               if (++as == AS) {
                 as = 0;
                 aphase ^= 1u;
@@ -385,7 +391,7 @@ lstm_wmajor_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
             }
           }
           // The tile is complete after its recurrent half (or after the input half at t = 0).
-          if (!is_x || t == 0) umma_commit(&tfull_bar[acc]);
+          if (leader && (!is_x || t == 0)) umma_commit(&tfull_bar[acc]);
           FTB_WM_STAMP(l, t, is_x ? 5 : 4);
           return true;
         });

@@ -115,6 +115,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same for a warp that waits as one: a result the whole warp shares, so that what follows stays
+// convergent.  The MMA warps loop with all their lanes and issue from one elected lane: an MMA takes its
+// descriptors from uniform registers, and in a loop that a single lane runs every operand is a
+// divergent value that has to be moved there first.  Measured, cycles an MMA of M = 128, A in tensor
+// memory: N 16 / 32 / 64 / 128: 45 / 45 / 45 / 65 from one lane alone, 11 / 17 / 33 / 64 this way
+// (A in shared memory: 40 / 41 / 49 / 64).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* s_abort, int* g_status,
+                                               int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, g_status, code));
+}
+
 // ------------------------------------------------- inter-CTA flags (global memory)
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
     bdesc0 |= static_cast<uint64_t>((smem_u32(slots) & 0x3FFFFu) >> 4);
     bdesc0 |= static_cast<uint64_t>(kCoreK >> 4) << 16;
     bdesc0 |= static_cast<uint64_t>(128u >> 4) << 32;
-    bool ok = mbar_wait(&w_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+    bool ok = mbar_wait_warp(&w_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
     tc_fence_after();
     for (int i = a.before == nullptr ? 1 : 0; i < a.steps; ++i) {
       const int slot = (i + 1) & 1;  // of the step before

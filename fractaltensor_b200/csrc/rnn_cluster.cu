@@ -467,13 +467,15 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // (all lanes walk the loop, one issues: mbar_wait_warp in ptx.cuh says why)
+    {
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(128, NB, Fmt<T>::kind, 0, 0);
       const uint64_t ring_desc0 = make_sdesc_sw128(smem_u32(s_ring), 16, 1024);
       const uint64_t self_desc0 = make_sdesc_plain(smem_u32(s_self), NB * 16, 128);
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = mbar_wait(&res_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+      bool ok = mbar_wait_warp(&res_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
       tc_fence_after();
       ACCT_DECL(6);
 #ifdef FTB_ACCT
@@ -499,18 +501,17 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         }
         const int acc = i & 1;
         ACCT_BEGIN();
-        ok = mbar_wait(&tempty_bar[acc], ((i >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
+        ok = mbar_wait_warp(&tempty_bar[acc], ((i >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
         ACCT_END(0);
         if (!ok) break;
         tc_fence_after();
         FTB_CL_STAMP(i, 0);
         const uint32_t d_tmem = tmem_base + acc * NB;
-        uint32_t accumulate = 0;  // the first MMA of a step overwrites the accumulator
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           if (s >= nseg) break;
           ACCT_BEGIN();
-          ok = mbar_wait(&ring_full[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+          ok = mbar_wait_warp(&ring_full[stage], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
           ACCT_END(1);
           if (!ok) break;
           FTB_CL_STAMP(i, 12 + s);
@@ -518,16 +519,16 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           const uint32_t aw = tmem_w + wkb0[s] * 32;
           ACCT_BEGIN();
           for (int kb = 0; kb < kbh; ++kb) {
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-              umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd0 + static_cast<uint64_t>((kb * kBlockBytes) >> 4) + 2 * kk, idesc,
-                      accumulate);
-              accumulate = 1;
+              for (int kk = 0; kk < BK / 16; ++kk)
+                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd0 + static_cast<uint64_t>((kb * kBlockBytes) >> 4) + 2 * kk, idesc,
+                        s > 0 || kb > 0 || kk > 0);  // the first MMA of a step overwrites the accumulator
             }
           }
           ACCT_END(4);
           ACCT_BEGIN();
-          umma_commit(&ring_empty[stage]);  // the whole segment, on its first stage's barrier
+          if (leader) umma_commit(&ring_empty[stage]);  // the whole segment, on its first stage's barrier
           ACCT_END(5);
           stage += seg_stages;
           if (stage == n_ring) {
@@ -540,27 +541,26 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         if (self) {
           // The cluster's own output of step i-1, copied by its producers into slot (i-1) & 1 of every CTA.
           const int slot = (i - 1) & 1;
-          mbar_arrive_expect_tx(&self_full[slot], self_slot_bytes);
+          if (leader) mbar_arrive_expect_tx(&self_full[slot], self_slot_bytes);
           ACCT_BEGIN();
-          ok = mbar_wait(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+          ok = mbar_wait_warp(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
           ACCT_END(2);
           if (!ok) break;
           FTB_CL_STAMP(i, 2);
           // K = 16 is two 16-byte chunks, NB * 16 bytes apart; 8-row groups are 128 bytes apart; the
           // descriptor of MMA j is the slot's plus j * 2 * NB (bytes / 16): nothing is rebuilt per MMA.
-          uint64_t bd = self_desc0 + static_cast<uint64_t>((slot * self_slot_bytes) >> 4);
-          uint32_t aw = tmem_w + kbh * 32;
-          const int n_self = kbh * (BK / 16);
-#pragma unroll 4
-          for (int j = 0; j < n_self; ++j) {
-            umma_ts(d_tmem, aw, bd, idesc, accumulate);
-            accumulate = 1;
-            aw += 8;
-            bd += 2 * NB;
+          const uint64_t bd = self_desc0 + static_cast<uint64_t>((slot * self_slot_bytes) >> 4);
+          const uint32_t aw = tmem_w + kbh * 32;
+          for (int kb = 0; kb < kbh; ++kb) {
+            if (leader) {
+#pragma unroll
+              for (int kk = 0; kk < BK / 16; ++kk)
+                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd + static_cast<uint64_t>(kb * 4 + kk) * (2 * NB), idesc, 1u);
+            }
           }
-          umma_commit_to(&self_free[slot], producer_mask);
+          if (leader) umma_commit_to(&self_free[slot], producer_mask);
         }
-        umma_commit(&tfull_bar[acc]);
+        if (leader) umma_commit(&tfull_bar[acc]);
         FTB_CL_STAMP(i, 3);
       }
 #ifdef FTB_ACCT
