@@ -38,6 +38,14 @@ bool lstm_wmajor_supported(int dtype, int D, int N, int I, int H, int G, int sm_
 int launch_lstm_wmajor(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, int D, int L,
                        int N, int I, int H, int G, int resident, int* done, int* status, unsigned long long* trace,
                        cudaStream_t stream);
+struct FlowPlan {
+  int nb, S, G;
+  double est_us;
+};
+bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, FlowPlan* plan);
+int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* off,
+                     int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
+                     cudaStream_t stream);
 bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count);
 size_t lstm_dilated_cluster_flag_ints(int D, int L);
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
@@ -438,9 +446,22 @@ int ftb_grid_pack_weights(const void* i2h, const void* h2h, void* Wp, int H, int
 // Upper bound of tiles per cell over the tile shapes the library may pick.
 static int stacked_max_tiles_per_cell(int N, int H) { return 2 * ((N + 255) / 256) * ((4 * H + 127) / 128); }
 
+// Arrival counters of the lstm_flow kernel, one per cell and batch slice (of 16 sequences or more).
+static size_t flow_flag_bytes(int D, int L, int slices) { return sizeof(int) * D * L * static_cast<size_t>(slices); }
+constexpr int kMostFlowSlices = 128;  // of a layer: two CTAs or more each
+
 size_t ftb_lstm_stacked_workspace_bytes(int D, int L, int N, int H) {
   if (D <= 0 || L <= 0 || N <= 0 || H <= 0) return kWorkspaceBytes;
-  return plan_layout(D * L, stacked_max_tiles_per_cell(N, H)).total;
+  return plan_layout(D * L, stacked_max_tiles_per_cell(N, H)).total + flow_flag_bytes(D, L, (N + 15) / 16);
+}
+
+// Layers per group of the static-ownership kernels: at most `G` (what L2 holds) and what fits on the
+// device at `ctas` CTAs a layer, evened out over the groups.
+static int fit_groups(int D, int G, int ctas, int sm_count) {
+  const int most = std::min(std::min(G, D), sm_count / ctas);
+  if (most < 1) return G;
+  const int groups = (D + most - 1) / most;
+  return (D + groups - 1) / groups;
 }
 
 int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, int D, int L,
@@ -530,7 +551,26 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
     // keep their slice of a layer, cell state in registers, for a whole sweep over time.
     // Weights-major static ownership (schedule 4, and the automatic choice for batches of at most
     // 128 sequences): the batch is the N side of the MMA, so a small batch wastes no tensor work.
-    const bool can_wmajor = lstm_wmajor_supported(dtype, D, N, I, H, G, cl.sm_count);
+    const int tiles = 4 * H / 128;
+    const int Gw = layers_per_group > 0 ? G : fit_groups(D, G, tiles, cl.sm_count);
+    const bool can_wmajor = lstm_wmajor_supported(dtype, D, N, I, H, Gw, cl.sm_count);
+    const int Gs = layers_per_group > 0 ? G : fit_groups(D, G, 2 * ((N + 255) / 256) * ((4 * H + 255) / 256), cl.sm_count);
+    // Everything on chip (schedule 5, and the automatic choice where it is expected to be faster than the
+    // kernels that stream weights; their steps as measured: with up to 128 sequences 5.5 us at H 512 and
+    // 9..12 at H 1024, above that 9.5 at H 320 and 14 at H 1024).
+    FlowPlan flow;
+    const bool can_flow = layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, &flow) &&
+                          workspace_bytes >= lay.total + flow_flag_bytes(D, L, flow.S);
+    if (schedule == 5 && !can_flow) return FTB_ERR_ARG;
+    const int Gold = can_wmajor ? Gw : Gs;
+    const double old_step = can_wmajor ? 1.6 + 6.5 * H / 1024 + N * H / 40960.0 : 7.5 + 6.5 * H / 1024;
+    const double old_us = ((D + Gold - 1) / Gold) * (L + Gold - 1) * old_step;
+    if (schedule == 5 || (schedule == 0 && can_flow && flow.est_us < old_us && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
+      rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, nullptr, static_cast<int64_t>(L) * N, D, L, N, I, H, flow,
+                            reinterpret_cast<int*>(ws + lay.total), status, stream);
+      if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
+      goto level_schedule;
+    }
     if (schedule == 4 && !can_wmajor) return FTB_ERR_ARG;
     if (schedule == 4 || (schedule == 0 && can_wmajor && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
       // tuning[6]: 0 = as many recurrent weight blocks on chip as fit, -1 = none, n = n blocks
@@ -540,20 +580,20 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
       trace = reinterpret_cast<unsigned long long*>(ws + lay.trace);
 #endif
       // one flag per (cell, tile), in the per-tile counter area (at least 4H/128 ints per cell)
-      rc = launch_lstm_wmajor(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, G, resident,
+      rc = launch_lstm_wmajor(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, Gw, resident,
                               reinterpret_cast<int*>(ws + lay.tile_done), status, trace, stream);
       if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
       goto level_schedule;
     }
     const bool can_static = tune.pair != 1 && (bn == 0 || bn == 256) && !tune.fine_deps &&
-                            lstm_static_supported(dtype, D, N, I, H, G, cl.sm_count);
+                            lstm_static_supported(dtype, D, N, I, H, Gs, cl.sm_count);
     if (schedule == 3 && !can_static) return FTB_ERR_ARG;
     if ((schedule == 3 || schedule == 0) && can_static) {
       unsigned long long* trace = nullptr;
 #ifdef FTB_TRACE
       trace = reinterpret_cast<unsigned long long*>(ws + lay.trace);
 #endif
-      rc = launch_lstm_static(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, G,
+      rc = launch_lstm_static(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, Gs,
                               reinterpret_cast<int*>(ws + lay.done), status, trace, stream);
       // A cooperative launch can be refused (device shared through MPS, SMs reserved, ...).
       // With an explicit schedule that is the caller's error to see; the automatic choice
@@ -719,6 +759,24 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
 
   const int n_cells = D * L;
   const PlanLayout lay = plan_layout(n_cells, 0);
+  // Everything on chip (csrc/lstm_flow.cu): the first rows of the steps and the arrival counters sit
+  // behind the tables of the generic schedule.
+  FlowPlan flow;
+  const size_t off_bytes = (sizeof(int) * (L + 1) + 255) & ~static_cast<size_t>(255);
+  const bool can_flow = tune.layers_per_group == 0 && tune.pair == 0 && tune.bn == 0 &&
+                        lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, &flow) &&
+                        workspace_bytes >= lay.total + off_bytes + flow_flag_bytes(D, L, flow.S);
+  if (tune.schedule == 5 && !can_flow) return FTB_ERR_ARG;
+  // the generic schedule takes about 14 us a step and group of layers at any size
+  if (tune.schedule == 5 || (tune.schedule == 0 && can_flow && flow.est_us < ((D + G - 1) / G) * (L + G - 1) * 10.0)) {
+    char* ws = static_cast<char*>(workspace);
+    std::vector<int> first(off.begin(), off.end());
+    if (cudaMemcpyAsync(ws + lay.total, first.data(), sizeof(int) * (L + 1), cudaMemcpyHostToDevice, stream) != cudaSuccess)
+      return FTB_ERR_LAUNCH;
+    rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, reinterpret_cast<int*>(ws + lay.total), T, D, L, N, I, H, flow,
+                          reinterpret_cast<int*>(ws + lay.total + off_bytes), status, stream);
+    if (rc != FTB_ERR_LAUNCH || tune.schedule != 0) return rc;
+  }
   bool persistent = dtype != FTB_F32 && tune.schedule != 1 && (tune.schedule >= 2 || workspace_bytes >= lay.total);
   if (persistent) {
     if (workspace_bytes < lay.total) return FTB_ERR_WORKSPACE;
@@ -795,7 +853,8 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
 
 size_t ftb_lstm_stacked_varlen_workspace_bytes(int D, int L) {
   if (D <= 0 || L <= 0) return kWorkspaceBytes;
-  return plan_layout(D * L, 0).total;
+  // tables of the generic schedule; first rows of the steps and arrival counters of the on-chip one
+  return plan_layout(D * L, 0).total + sizeof(int) * (L + 1) + 256 + flow_flag_bytes(D, L, kMostFlowSlices);
 }
 
 int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
@@ -1385,7 +1444,7 @@ int ftb_lstm_stacked_fwd_noalloc(const void* x, const void* Wp, const float* bia
                                  void* stream) {
   if (D <= 0 || L <= 0 || N <= 0 || H <= 0) return FTB_ERR_ARG;
   if (dtype != FTB_F16 && dtype != FTB_BF16) return FTB_ERR_ARG;
-  if (ftb_lstm_stacked_workspace_bytes(D, L, N, H) > FTB_STATIC_SCRATCH_BYTES) return FTB_ERR_SCRATCH_LIMIT;
+  if (plan_layout(D * L, stacked_max_tiles_per_cell(N, H)).total > FTB_STATIC_SCRATCH_BYTES) return FTB_ERR_SCRATCH_LIMIT;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FTB_ERR_ARCH;
   void* scratch = nullptr;

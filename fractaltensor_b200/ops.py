@@ -111,7 +111,8 @@ def lstm_stacked(x, Wp, bias_p=None, hs=None, c=None, layers_per_group=0, bn=0, 
     """x: [L,N,I]; Wp: [D,4H,I+H] -> (hs [D,L,N,H], c fp32 [D,N,H]).
     schedule: 0 auto, 1 one launch per anti-diagonal, 2 one persistent kernel, 3 static tile ownership
     (CTA pairs on 256 batch rows), 4 static tile ownership with the batch on the N side of the MMA
-    (at most 128 sequences; `resident`: recurrent weight blocks kept on chip, 0 auto, -1 none);
+    (at most 128 sequences; `resident`: recurrent weight blocks kept on chip, 0 auto, -1 none), 5 all weights
+    on chip and the states handed on through the output array (layers whose tiles fit on the device);
     pair: 0 auto, 1 single CTAs, 2 CTA pairs."""
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)
@@ -145,7 +146,7 @@ def lstm_stacked_varlen(x, active_rows, Wp, bias_p=None, hs=None, c=None, layers
     active_rows: L non-increasing ints, the sequences still running at each step; x: [T,I] with
     T = sum(active_rows), rows of step t after those of step t-1; Wp: [D,4H,I+H]
     -> (hs [D,T,H] in the same packed order, c fp32 [D,N,H] with N = active_rows[0]).
-    schedule: 0 auto, 1 one launch per anti-diagonal, 2 one persistent kernel."""
+    schedule: 0 auto, 1 one launch per anti-diagonal, 2 one persistent kernel, 5 all weights on chip."""
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)
     active_rows = [int(n) for n in active_rows]

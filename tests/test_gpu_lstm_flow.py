@@ -1,0 +1,82 @@
+"""Stacked LSTM with all weights on chip and states handed on through the output array
+(csrc/lstm_flow.cu): bit for bit the result of one launch per level."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from fractaltensor_b200 import ops as _ops
+    return _ops
+
+
+def _params(ops, D, I, H, dt, g):
+    u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+    return ops.lstm_pack_weights(u(D, 4, I, H), u(D, 4, H, H), u(D, 4, H))
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,L,N,I,H", [
+    (1, 1, 1, 64, 64),       # one step: nothing handed on
+    (3, 7, 16, 128, 128),    # a full slice of 16
+    (2, 6, 17, 256, 256),    # one sequence in the second slice
+    (5, 9, 70, 320, 320),    # odd number of K blocks, slices of 32
+    (8, 5, 64, 512, 512),    # slices of 64, input weights partly in shared memory
+    (12, 6, 30, 640, 640),   # layers in groups: weights replaced between sweeps
+    (2, 5, 8, 768, 768),     # the widest state that fits: two rounds of loads
+    (1, 4, 40, 192, 64),     # input wider than the state
+    (16, 4, 256, 64, 64),    # slices of 32 and more at the narrowest state
+    (4, 5, 256, 256, 256),
+])
+def test_same_bits_as_levels(ops, dt, D, L, N, I, H):
+    g = torch.Generator(device="cuda").manual_seed(D * 100 + N)
+    Wp, b = _params(ops, D, I, H, dt, g)
+    x = torch.randn(L, N, I, device="cuda", generator=g).to(dt)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1, pair=1)
+    for _ in range(3):  # the fill pattern of a call must not survive into the next
+        h, c = ops.lstm_stacked(x, Wp, b, schedule=5)
+        ops.check_status()
+        assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+@pytest.mark.parametrize("D,H,lens", [
+    (3, 128, [9, 9, 7, 3, 1] * 5),                  # ends inside a slice
+    (2, 256, list(range(1, 41))),                   # every length, slices that end early
+    (2, 512, [5] * 16 + [2] * 17),                  # a slice that runs two steps only
+    (10, 640, [6, 6, 4, 1]),                        # groups of layers on a ragged batch
+])
+def test_ragged_same_bits_as_levels(ops, D, H, lens):
+    g = torch.Generator(device="cuda").manual_seed(H + len(lens))
+    dt = torch.bfloat16
+    Wp, b = _params(ops, D, H, H, dt, g)
+    lens = sorted(lens, reverse=True)
+    active = [sum(n > t for n in lens) for t in range(lens[0])]
+    x = torch.randn(sum(lens), H, device="cuda", generator=g).to(dt)
+    ref_h, ref_c = ops.lstm_stacked_varlen(x, active, Wp, b, schedule=1, pair=1)
+    for sched in (5, 0):
+        h, c = ops.lstm_stacked_varlen(x, active, Wp, b, schedule=sched)
+        ops.check_status()
+        assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+def test_nan_states_are_states(ops):
+    """A NaN hidden state is a value like any other (0x7FFF, not the fill pattern): nothing waits for it."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    Wp, b = _params(ops, 2, 128, 128, torch.float16, g)
+    x = torch.randn(6, 5, 128, device="cuda", generator=g).half()
+    x[2, 3] = float("nan")
+    x.view(torch.int16)[2, 4] = -1  # 0xFFFF: a NaN with the fill pattern's bits, as an input
+    h, _ = ops.lstm_stacked(x, Wp, b, schedule=5)
+    ops.check_status()
+    assert not torch.isnan(h[:, :, :3]).any() and torch.isnan(h[:, 2:, 3:]).all() and not torch.isnan(h[:, :2]).any()
+
+
+def test_sizes_that_do_not_fit_are_refused(ops):
+    from fractaltensor_b200._lib import FtbError
+    g = torch.Generator(device="cuda").manual_seed(8)
+    Wp, b = _params(ops, 1, 1024, 1024, torch.float16, g)
+    x = torch.randn(2, 4, 1024, device="cuda", generator=g).half()
+    with pytest.raises(FtbError):
+        ops.lstm_stacked(x, Wp, b, schedule=5)
