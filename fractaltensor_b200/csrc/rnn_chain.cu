@@ -48,41 +48,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "memory");
 }
 
-// 16 bytes into shared memory of a CTA of the cluster, counted on a barrier of that CTA.
-__device__ __forceinline__ void st_async16(uint32_t dst_cluster, uint32_t bar_cluster, const uint32_t (&v)[4]) {
-  asm volatile(
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst_cluster),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar_cluster)
-      : "memory");
-}
-
-// mbar_wait with the ordering of data that another CTA of the cluster has sent.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* s_abort, int* g_status,
-                                                  int code) {
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t it = 1;; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 0x3F) == 0) {
-      if (*s_abort) return false;
-      if (globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS) {
-        *s_abort = 1;
-        atomicCAS(g_status, 0, code);
-        return false;
-      }
-    }
-  }
-}
-
 struct ChainArgs {
   const float* pre;    // [steps, N, H]
   const void* Wp;      // packed rows of ldw elements; the recurrent half starts at element k0

@@ -13,11 +13,14 @@
 //     ("recurrent weights resident on chip");
 //   * the batch is the N side of the MMA (NB = 128 or 64 columns per slice);
 //   * the state a chain hands to its own next step -- h(t) of a layer with dilation 1, h_y of
-//     the grid cell to the left -- never leaves the cluster: each CTA writes its units into a
-//     staging tile and copies it with one bulk shared-memory-to-shared-memory copy per peer into
-//     the next step's B operand in every CTA of the cluster (distributed shared memory),
-//     completion counted on the receiver's mbarrier.  The receiving layout is the un-swizzled
-//     K-major core-matrix layout, in which one CTA's units are one contiguous block;
+//     the grid cell to the left -- never leaves the cluster: it goes into the next step's B operand in
+//     every CTA of the cluster (distributed shared memory), bytes counted on the receiver's mbarrier.
+//     In the grid an epilogue thread packs eight sequences of its unit, one 16-byte row of the
+//     un-swizzled MN-major core-matrix layout, and stores it with st.async straight from its registers: no
+//     staging, no barrier between the warps (32 x 32, H 256, 64 sequences: 280 -> 257 us).  In the
+//     dilated LSTM each CTA writes its units into a staging tile, a contiguous block of the K-major
+//     layout, and copies it with one bulk copy per piece and peer: eight peers' 32 KB a step are bound by
+//     the bytes, and 16 at a time take longer (3.1 us a step instead of 3.0);
 //   * everything that crosses chains (the layer below, the grid row above, a layer's own state
 //     `dilation` >= 2 steps back) goes through global memory with one release flag per
 //     (cell, tile), polled by a whole warp, and TMA loads; those consumers run a few steps behind
@@ -330,8 +333,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   const uint16_t producer_mask = static_cast<uint16_t>(MODE == kDilated ? ((1u << a.CL) - 1u)
                                                                         : (((1u << a.CL) - 1u) & ~((1u << (a.CL / 2)) - 1u)));
   const uint32_t self_slot_bytes = static_cast<uint32_t>(a.H / 8) * NB * 16;  // H units x NB rows, 16-bit
-  const uint32_t stage_tile_bytes = static_cast<uint32_t>(self_units / 8) * NB * 16;
-  // Shared memory: [self slot 0][self slot 1][staging 0][staging 1][output tile 0][output tile 1][ring ...];
+  const uint32_t stage_tile_bytes = MODE == kDilated ? static_cast<uint32_t>(self_units / 8) * NB * 16 : 0u;
+  // Shared memory: [self slot 0][self slot 1][staging 0][staging 1 (dilated)][output tile 0][output tile 1][ring ...];
   // chains without a self operand have the output tiles and a longer ring only.
   uint8_t* s_self = smem;
   uint8_t* s_stg = s_self + (self_chain ? 2 * self_slot_bytes : 0);
@@ -472,7 +475,9 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(128, NB, Fmt<T>::kind, 0, 0);
       const uint64_t ring_desc0 = make_sdesc_sw128(smem_u32(s_ring), 16, 1024);
+      // (K chunks of 16 bytes, or groups of 8 units, NB * 16 bytes apart; groups of 8 sequences 128)
       const uint64_t self_desc0 = make_sdesc_plain(smem_u32(s_self), NB * 16, 128);
+      constexpr uint32_t idesc_self = make_idesc_f16(128, NB, Fmt<T>::kind, 0, MODE == kGrid ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = mbar_wait_warp(&res_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
@@ -543,19 +548,25 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           const int slot = (i - 1) & 1;
           if (leader) mbar_arrive_expect_tx(&self_full[slot], self_slot_bytes);
           ACCT_BEGIN();
-          ok = mbar_wait_warp(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+          if (MODE == kGrid) {
+            ok = __all_sync(0xffffffffu, mbar_wait_cluster(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status,
+                                                           FTB_ERR_TIMEOUT_TMA));
+            fence_proxy_async_smem();  // stored by threads, read by the async proxy
+          } else {
+            ok = mbar_wait_warp(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+          }
           ACCT_END(2);
           if (!ok) break;
           FTB_CL_STAMP(i, 2);
-          // K = 16 is two 16-byte chunks, NB * 16 bytes apart; 8-row groups are 128 bytes apart; the
-          // descriptor of MMA j is the slot's plus j * 2 * NB (bytes / 16): nothing is rebuilt per MMA.
+          // K = 16 is two 16-byte chunks (two groups of 8 units), NB * 16 bytes apart; the descriptor
+          // of MMA j is the slot's plus j * 2 * NB (bytes / 16): nothing is rebuilt per MMA.
           const uint64_t bd = self_desc0 + static_cast<uint64_t>((slot * self_slot_bytes) >> 4);
           const uint32_t aw = tmem_w + kbh * 32;
           for (int kb = 0; kb < kbh; ++kb) {
             if (leader) {
 #pragma unroll
               for (int kk = 0; kk < BK / 16; ++kk)
-                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd + static_cast<uint64_t>(kb * 4 + kk) * (2 * NB), idesc, 1u);
+                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd + static_cast<uint64_t>(kb * 4 + kk) * (2 * NB), idesc_self, 1u);
             }
           }
           if (leader) umma_commit_to(&self_free[slot], producer_mask);
@@ -678,9 +689,11 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) creg[i] = 0.f;
     const int n_valid = min(NB, a.N - slice * NB);  // batch columns of this slice that exist
-    // Where this thread's unit sits (a) in the self operand / its staging tile: 16-byte chunk
-    // (u_local / 8) of NB rows, then row n, then the unit's 2 bytes; (b) in the row-major output tile.
+    // Where this thread's unit sits (a) in the staging tile (dilated): 16-byte chunk (u_local / 8) of NB rows,
+    // then row n, then the unit's 2 bytes; (b) in the self operand (grid): NB * 16 bytes for 8 units, 128 for
+    // 8 sequences of them, 16 for a unit's; (c) in the row-major output tile.
     const uint32_t stg_unit_off = static_cast<uint32_t>(u_local >> 3) * NB * 16 + (u_local & 7) * 2;
+    const uint32_t self_unit_off = smem_u32(s_self) + static_cast<uint32_t>(unit >> 3) * NB * 16 + (unit & 7) * 16;
     const uint32_t out_unit_off = static_cast<uint32_t>(u_local) * 2;
     volatile int* stored = &out_stored;
     ACCT_DECL(2);
@@ -754,12 +767,31 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           if (self_producer) *reinterpret_cast<T*>(stg + n * 16) = h_new;
         }
       } else {
+        const bool send = self_producer && i + 1 < n_steps;
+        if (send && i >= 2)  // the slot's last contents have been multiplied everywhere
+          ok = mbar_wait(&self_free[i & 1], ((i - 2) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
 #pragma unroll
-        for (int k = 0; k < kCols; ++k) {
-          const T h_new = to_elem<T>(tanh_fast(v[k] + bias1));
-          const int n = sub * kCols + k;
-          *reinterpret_cast<T*>(outp + n * (kOutUnits * 2)) = h_new;
-          if (self_producer) *reinterpret_cast<T*>(stg + n * 16) = h_new;
+        for (int g = 0; g < kCols / 8; ++g) {
+          uint32_t row[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            row[k] = Fmt<T>::pack2(tanh_fast(v[8 * g + 2 * k] + bias1), tanh_fast(v[8 * g + 2 * k + 1] + bias1));
+          const int n = sub * kCols + 8 * g;
+          if (send) {
+            const uint32_t dst = self_unit_off + (i & 1) * self_slot_bytes + (n / 8) * 128;
+            const uint32_t bar = smem_u32(&self_full[i & 1]);
+            for (int k = 0; k < a.CL; ++k) {
+              const uint32_t peer = (rank + k) & (a.CL - 1);  // (2 or 4 CTAs)
+              st_async16(map_to_cta(dst, peer), map_to_cta(bar, peer), row);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            *reinterpret_cast<uint16_t*>(outp + (n + k) * (kOutUnits * 2)) = static_cast<uint16_t>(row[k >> 1] >> (16 * (k & 1)));
         }
       }
       if (MODE == kDilated && (dil > 1 || i == n_steps - 1)) {
@@ -774,7 +806,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       fence_proxy_async_smem();  // plain shared-memory stores -> the bulk copies' and the TMA store's reads
       __syncwarp();
       if (warp == kFirstEpiWarp && lane == 0) { FTB_CL_STAMP(i, 14); }
-      if (self_producer && i + 1 < n_steps) {
+      if (MODE == kDilated && self_producer && i + 1 < n_steps) {
         // Hand the step's output to every CTA of the cluster, once all of them have multiplied what the
         // destination slot held before (two steps ago).
         // Once all epilogue warps have staged their parts, the tile goes to every CTA of the cluster by
@@ -782,7 +814,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         // about 64 KB in 1.3-2 us however the tile is cut -- 128 copies of 512 B, 32 of 2 KB or 8 of
         // 8 KB -- so the hand-off is bound by the bytes every CTA must receive, not by the slicing.)
         if (lane == 0) mbar_arrive(&stg_ready);
-        const uint32_t kPiece = MODE == kGrid ? stage_tile_bytes : 2048u;
+        const uint32_t kPiece = 2048u;
         const int n_pieces = static_cast<int>(stage_tile_bytes / kPiece);
         const int n_copies = n_pieces * a.CL;
         const int per_warp = (n_copies + kEpiWarps - 1) / kEpiWarps;
@@ -1086,7 +1118,7 @@ int launch_grid_rnn_cluster(int dtype, const void* X, const void* Y, const void*
   const size_t n_flags = static_cast<size_t>(D) * A * B * a.S * a.CL;
   if (cudaMemsetAsync(flags, 0, sizeof(int) * n_flags, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
   const int grid = D * A * a.S * a.CL;
-  const uint32_t smem = smem_for(true, H, kGridNB, 128, 128, 6);
+  const uint32_t smem = smem_for(true, H, kGridNB, 0, 128, 6);
   if (dtype == FTB_F16) return launch<__half, kGrid, kGridNB>(m, a, grid, smem, stream);
   return launch<__nv_bfloat16, kGrid, kGridNB>(m, a, grid, smem, stream);
 }
