@@ -308,7 +308,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   __shared__ uint64_t self_free[2];   // producers only: every CTA of the cluster has multiplied the slot's contents
   __shared__ uint64_t stg_ready;      // the eight epilogue warps have written the step's staging tile
   __shared__ int seg_seq;             // operand segments issued into the ring so far (two producer warps)
-  __shared__ int out_issued;          // epilogue warps that have staged a step's outputs, summed over steps
+  __shared__ int out_issued[2];       // epilogue warps that have staged an even / odd step's outputs, summed over steps
   __shared__ int out_stored;          // steps whose output staging tile the publisher has finished reading
   __shared__ uint64_t tfull_bar[2], tempty_bar[2];
   __shared__ uint64_t res_full;
@@ -363,7 +363,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     mbar_init(&self_free[1], a.CL);
     mbar_init(&stg_ready, kEpiWarps);
     seg_seq = 0;
-    out_issued = 0;
+    out_issued[0] = out_issued[1] = 0;
     out_stored = 0;
     mbar_init(&tfull_bar[0], 1);
     mbar_init(&tfull_bar[1], 1);
@@ -589,9 +589,10 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     // The epilogue warps count themselves in `out_issued` once their part of a step's output tile is
     // staged in shared memory; this thread writes the tile to global memory with one TMA store, waits
     // for it to complete and releases the step's flag -- all of it off the chain's critical path.
-    // (A running count, not an mbarrier: this thread may fall more than one step behind.)
+    // (A running count, not an mbarrier: this thread may fall more than one step behind.  One for the even
+    // and one for the odd steps: where a step does not need the one before, a warp can stage the next step
+    // while another still works on this one, but not the one after that, which waits for `out_stored`.)
     if (lane == 0) {
-      volatile int* issued = &out_issued;
       volatile int* stored = &out_stored;
       const int n_valid = min(NB, a.N - slice * NB);
       const bool ydir = MODE == kGrid && rank >= a.CL / 2;
@@ -599,7 +600,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       const int unit0 = MODE == kDilated ? rank * 32 : (ydir ? rank - a.CL / 2 : rank) * 128;
       ACCT_DECL(2);
       for (int i = 0; i < n_steps; ++i) {
-        const int want = kEpiWarps * (i + 1);
+        volatile int* issued = &out_issued[i & 1];
+        const int want = kEpiWarps * ((i >> 1) + 1);
         ACCT_BEGIN();
         if (*issued < want) {
           const uint64_t t0 = globaltimer_ns();
@@ -806,7 +808,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       fence_proxy_async_smem();  // plain shared-memory stores -> the bulk copies' and the TMA store's reads
       __syncwarp();
       if (warp == kFirstEpiWarp && lane == 0) { FTB_CL_STAMP(i, 14); }
-      if (MODE == kDilated && self_producer && i + 1 < n_steps) {
+      if constexpr (MODE == kDilated)
+      if (self_producer && i + 1 < n_steps) {
         // Hand the step's output to every CTA of the cluster, once all of them have multiplied what the
         // destination slot held before (two steps ago).
         // Once all epilogue warps have staged their parts, the tile goes to every CTA of the cluster by
@@ -838,7 +841,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       __syncwarp();
       if (lane == 0) {
         __threadfence_block();
-        atomicAdd(&out_issued, 1);
+        atomicAdd(&out_issued[i & 1], 1);
       }
     }
     if (warp == kFirstEpiWarp && lane == 0) { ACCT_WRITE(0, 12); }  // accumulator complete
