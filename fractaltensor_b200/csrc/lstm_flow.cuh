@@ -1,0 +1,519 @@
+// Device side of the stacked LSTM whose hidden states carry their own arrival: csrc/lstm_flow.cu says how it
+// works.  Also a layer of dilation 1 of the dilated LSTM (csrc/rnn_cluster.cu).
+#pragma once
+
+#include "ptx.cuh"
+#include "tmap.h"
+
+namespace ftb {
+
+namespace flow {
+
+constexpr int kGateRows = 128;  // packed gate rows of a CTA
+constexpr int kUnits = kGateRows / 4;
+constexpr int BK = 64;
+constexpr uint32_t kWBlockBytes = kGateRows * BK * 2;
+constexpr int kFirstEpi = 4;
+constexpr int kMaxSlots = 2;     // input tiles [NB x I] in shared memory
+constexpr int kMaxPause = 4000;  // cycles
+constexpr uint32_t kMaxSmem = 226 * 1024;
+
+template <int NB>
+struct FlowCfg {
+  static constexpr int kWarps = NB == 16 ? 4 : (NB == 32 ? 8 : 16);  // epilogue warps
+  static constexpr int kChunks = NB * 4 / kWarps / 16;         // of 16 columns, of a warp
+  static constexpr int kRows = NB / kWarps;                // state rows a warp reads
+  static constexpr int kThreads = 32 * (kFirstEpi + kWarps);
+  static constexpr uint32_t kBlockBytes = NB * BK * 2;     // one K block of a state
+  static constexpr int kCopyKb = 128 / NB;                 // K blocks of one TMA copy (16 KB)
+  static constexpr int kTmemBlocks = (512 - 2 * NB) / 32;  // weight blocks beside the two accumulators
+};
+
+struct FlowArgs {
+  int D, L, N, I, H, G, S;
+  int n_tiles;          // 4H / 128
+  int n_slots;          // input tiles
+  int64_t T;            // rows of a layer's output: off[L], or L * N
+  const int* off;       // [L + 1] first row of every step (ragged batch), or nullptr: t * N
+  const float* bias_p;  // [D, 4H] packed order, or nullptr
+  const void* Wp;       // [D, 4H, I+H]
+  void* hs;             // [D, T, H], all 0xFFFF before the launch
+  float* c_out;         // [D, c_rows, H], the first N of c_rows
+  int c_rows;
+  int* flags;           // [D * L * S] tiles of the slice's cell (l, t) that can be read through TMA
+  int below;            // slices of this layer in one of the layer below (whose flag is that of its first)
+  int* status;
+};
+
+struct Rows {  // rows of a step: the first one and how many sequences still run
+  int64_t first;
+  int active;
+};
+__device__ __forceinline__ Rows rows_of(const FlowArgs& a, int t) {
+  if (a.off == nullptr) return {static_cast<int64_t>(t) * a.N, t < a.L ? a.N : 0};
+  if (t >= a.L) return {0, 0};
+  const int r0 = __ldg(a.off + t);
+  return {r0, __ldg(a.off + t + 1) - r0};
+}
+
+__device__ __forceinline__ void quad_transpose(float& a0, float& a1, float& a2, float& a3, int lane) {
+  const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+  float r;
+  r = __shfl_xor_sync(0xffffffffu, b0 ? a0 : a1, 1);
+  if (b0) a0 = r; else a1 = r;
+  r = __shfl_xor_sync(0xffffffffu, b0 ? a2 : a3, 1);
+  if (b0) a2 = r; else a3 = r;
+  r = __shfl_xor_sync(0xffffffffu, b1 ? a0 : a2, 2);
+  if (b1) a0 = r; else a2 = r;
+  r = __shfl_xor_sync(0xffffffffu, b1 ? a1 : a3, 2);
+  if (b1) a1 = r; else a3 = r;
+}
+
+__device__ __forceinline__ void st_relaxed_gpu64(void* p, uint32_t lo, uint32_t hi) {
+  const uint64_t v = static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32);
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void ld_relaxed_gpu_2x64(const void* p, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+// A word of four hidden states has arrived when its last one is not the fill pattern.
+__device__ __forceinline__ bool arrived(uint64_t w) { return (w >> 48) != 0xFFFFu; }
+
+// One CTA: packed gate rows `tile` of batch slice `slice`, layers j, j + G, ..
+template <typename T, int NB>
+__device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapW,
+                                     const FlowArgs& a, const int tile, const int slice, const int j) {
+  using C = FlowCfg<NB>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t in_full[kMaxSlots], in_empty[kMaxSlots];
+  __shared__ uint64_t st_full;          // the previous step's state is in its operand tile
+  __shared__ uint64_t acc_full[2], acc_empty[2];
+  __shared__ uint64_t w_tmem, w_smem;   // the sweep's weights are in place
+  __shared__ uint64_t swept;            // every MMA of the sweep is done
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int n_stored;              // epilogue warps that have stored a step, summed over steps
+  __shared__ int s_abort;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* status = a.status;
+  const int kb_h = a.H / BK;
+  // Weight blocks in the order tensor memory is filled: recurrent, then input; the rest in shared memory.
+  const int rec_t = min(C::kTmemBlocks, kb_h);
+  // (an input tile is a whole number of copies)
+  const uint32_t slot_bytes = ((max(a.I, a.H) / BK + C::kCopyKb - 1) / C::kCopyKb) * C::kCopyKb * C::kBlockBytes;
+  uint8_t* s_state = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* s_in = s_state + kb_h * C::kBlockBytes;
+  uint8_t* s_w = s_in + a.n_slots * slot_bytes;
+
+  if (threadIdx.x == 0) {
+    prefetch_tmap(&mapX);
+    prefetch_tmap(&mapH);
+    prefetch_tmap(&mapW);
+    for (int i = 0; i < kMaxSlots; ++i) {
+      mbar_init(&in_full[i], 1);
+      mbar_init(&in_empty[i], 1);
+    }
+    mbar_init(&st_full, C::kWarps);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], C::kWarps);
+    }
+    n_stored = 0;
+    mbar_init(&w_tmem, C::kWarps);
+    mbar_init(&w_smem, 1);
+    mbar_init(&swept, 1);
+    s_abort = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(&tmem_base_s, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+  const uint32_t tmem_w = tmem_base + 2 * NB;
+
+  const int n_base = slice * NB;
+  const int n_groups = (a.D + a.G - 1) / a.G;
+  // Steps this slice takes part in (ragged: until its longest sequence, its first one, ends).
+  int steps = a.L;
+  if (a.off != nullptr) {
+    steps = 0;
+    for (int hi = a.L; steps < hi;) {
+      const int mid = (steps + hi) >> 1;
+      if (rows_of(a, mid).active > n_base) steps = mid + 1; else hi = mid;
+    }
+  }
+
+  if (warp == 0) {
+    // -------------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
+    constexpr uint32_t idesc = make_idesc_f16(kGateRows, NB, Fmt<T>::kind, 0, 0);
+    const uint64_t in_desc = make_sdesc_sw128(smem_u32(s_in), 16, 1024);
+    const uint64_t state_desc = make_sdesc_sw128(smem_u32(s_state), 16, 1024);
+    const uint64_t w_desc = make_sdesc_sw128(smem_u32(s_w), 16, 1024);
+    constexpr uint32_t kBlockDesc = C::kBlockBytes >> 4;
+    // K blocks of a half: weights in tensor memory from column `aw` or in shared memory from `ad`, the
+    // other operand from `bd`.  (A wait or a loop turn between K blocks costs more than the four MMAs of
+    // one: 250 cycles a block with a barrier each, 113 as a plain loop, 55 unrolled.)
+    auto blocks_ts = [&](uint32_t d_tmem, uint32_t aw, uint64_t bd, int n, uint32_t accumulate) {
+      for (; n >= 4; n -= 4, aw += 4 * 32, bd += 4 * kBlockDesc, accumulate = 1) {
+        if (leader) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            umma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
+        }
+      }
+      if (n & 2) {
+        if (leader) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            umma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
+        }
+        aw += 2 * 32;
+        bd += 2 * kBlockDesc;
+        accumulate = 1;
+      }
+      if (n & 1) {
+        if (leader) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) umma_ts(d_tmem, aw + 8 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
+        }
+      }
+    };
+    auto blocks_ss = [&](uint32_t d_tmem, uint64_t ad, uint64_t bd, int n, uint32_t accumulate) {
+      for (; n > 0; --n, ad += kWBlockBytes >> 4, bd += kBlockDesc, accumulate = 1) {
+        if (leader) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) umma_ss(d_tmem, ad + 2 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
+        }
+      }
+    };
+    int slot = 0, sweep = 0, k = 0, states = 0;  // k: steps started, states: states received
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int g = 0; g < n_groups && ok; ++g) {
+      const int l = g * a.G + j;
+      if (l >= a.D) continue;
+      const int kb_x = l == 0 ? a.I / BK : kb_h;
+      const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
+      ok = mbar_wait_warp(&w_tmem, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+      if (ok && (in_t < kb_x || rec_t < kb_h))
+        ok = mbar_wait_warp(&w_smem, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+      if (!ok) break;
+      tc_fence_after();
+      for (int t = 0; t < steps; ++t, ++k) {
+        const int acc = k & 1;
+        const uint32_t d_tmem = tmem_base + acc * NB;
+        ok = mbar_wait_warp(&acc_empty[acc], ((k >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI) &&
+             mbar_wait_warp(&in_full[slot], phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t xd = in_desc + static_cast<uint64_t>((slot * slot_bytes) >> 4);
+        blocks_ts(d_tmem, tmem_w + rec_t * 32, xd, in_t, 0u);
+        blocks_ss(d_tmem, w_desc + static_cast<uint64_t>(((kb_h - rec_t) * kWBlockBytes) >> 4), xd + in_t * kBlockDesc,
+                  kb_x - in_t, in_t > 0 ? 1u : 0u);
+        if (leader) umma_commit(&in_empty[slot]);
+        if (++slot == a.n_slots) {
+          slot = 0;
+          phase ^= 1u;
+        }
+        if (t > 0) {
+          ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
+          if (!ok) break;
+          blocks_ts(d_tmem, tmem_w, state_desc, rec_t, 1u);
+          blocks_ss(d_tmem, w_desc, state_desc + rec_t * kBlockDesc, kb_h - rec_t, 1u);
+          ++states;
+        }
+        if (leader) umma_commit(&acc_full[acc]);
+      }
+      if (ok && leader) umma_commit(&swept);
+      ++sweep;
+    }
+  } else if (warp == 1) {
+    // ----------------------------------- TMA: shared-memory weights, input tiles
+    int slot = 0, sweep = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int g = 0; g < n_groups && ok; ++g) {
+      const int l = g * a.G + j;
+      if (l >= a.D) continue;
+      const int kb_x = l == 0 ? a.I / BK : kb_h;
+      const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
+      const int n_rec = kb_h - rec_t, n_in = kb_x - in_t;
+      if (n_rec + n_in > 0) {
+        if (sweep > 0) ok = mbar_wait_warp(&swept, (sweep - 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
+        if (ok && lane == 0) {
+          mbar_arrive_expect_tx(&w_smem, (n_rec + n_in) * kWBlockBytes);
+          for (int b = 0; b < n_rec + n_in; ++b)
+            tma_load_2d(s_w + b * kWBlockBytes, &mapW, &w_smem, b < n_rec ? a.I + (rec_t + b) * BK : (in_t + b - n_rec) * BK,
+                        l * 4 * a.H + tile * kGateRows);
+        }
+      }
+      ++sweep;
+      const int copies = (kb_x + C::kCopyKb - 1) / C::kCopyKb;
+      for (int t = 0; t < steps && ok; ++t) {
+        const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + n_base;
+        if (l > 0) {
+          if (lane == 0)
+            ok = flag_wait_ge(a.flags + (static_cast<int64_t>(l - 1) * a.L + t) * a.S + slice / a.below * a.below, a.n_tiles, &s_abort, status,
+                              FTB_ERR_TIMEOUT_DEP);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          fence_proxy_async_all();  // threads of other CTAs stored what TMA reads
+        }
+        ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
+        if (!ok) break;
+        if (lane == 0) {
+          // (K blocks past the last one arrive as zeros and are not multiplied)
+          mbar_arrive_expect_tx(&in_full[slot], copies * C::kCopyKb * C::kBlockBytes);
+          for (int c = 0; c < copies; ++c)
+            tma_load_3d(s_in + slot * slot_bytes + c * C::kCopyKb * C::kBlockBytes, l == 0 ? &mapX : &mapH,
+                        &in_full[slot], 0, static_cast<int>(row), c * C::kCopyKb);
+        }
+        if (++slot == a.n_slots) {
+          slot = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ----------------------------------- publisher: cell (l, t) can be read through TMA
+    volatile int* abort_flag = &s_abort;
+    volatile int* stored = &n_stored;
+    int want = 0;
+    for (int g = 0; g < n_groups && lane == 0; ++g) {
+      const int l = g * a.G + j;
+      if (l >= a.D) continue;
+      for (int t = 0; t < steps; ++t) {
+        // (A running count, not a barrier: nothing waits for this warp, which may fall several steps
+        // behind, and a parity wait must not.)
+        want += C::kWarps;
+        if (l + 1 == a.D) continue;
+        uint64_t t0 = 0;
+        bool ok = true;
+        for (uint32_t it = 1; *stored < want; ++it) {
+          if ((it & 0x3F) != 0) continue;
+          if (t0 == 0) t0 = globaltimer_ns();
+          if (*abort_flag != 0 || globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS) {
+            ok = false;
+            break;
+          }
+        }
+        if (!ok) {
+          if (*abort_flag == 0) {
+            *abort_flag = 1;
+            atomicCAS(status, 0, FTB_ERR_TIMEOUT_EPI);
+          }
+          g = n_groups;
+          break;
+        }
+        __threadfence_block();
+        fence_proxy_async_all();
+        __threadfence();
+        red_release_gpu_add(a.flags + (static_cast<int64_t>(l) * a.L + t) * a.S + slice, 1);
+      }
+    }
+  } else if (warp >= kFirstEpi && warp < kFirstEpi + C::kWarps) {
+    // ------------------------------------------------------- epilogue and state
+    const int q = warp & 3, w = warp - kFirstEpi, sub = w >> 2;
+    const int r_loc = q * 32 + lane, gate = lane & 3;
+    const int unit = tile * kUnits + (r_loc >> 2);
+    const bool ub0 = (lane & 4) != 0, ub1 = (lane & 8) != 0;
+    // After the exchange below this lane stores four units of sequence n_store of each chunk; it keeps the
+    // cell state of four sequences from n_own on.
+    const int n_own = sub * C::kChunks * 16 + 4 * gate;
+    const int n_store = n_own + (ub0 ? 2 : 0) + (ub1 ? 1 : 0);
+    // What this lane reads of a state: chunk `lane & 7` of every K block of rows n_load, n_load + 4, ..
+    const int n_load = w * C::kRows + (lane >> 3);
+    volatile int* abort_flag = &s_abort;
+    int k = 0, sweep = 0, pause = 300;
+    bool ok = true;
+    for (int g = 0; g < n_groups && ok; ++g) {
+      const int l = g * a.G + j;
+      if (l >= a.D) continue;
+      if (sweep > 0) ok = mbar_wait_warp(&swept, (sweep - 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
+      if (!ok) break;
+      ++sweep;
+      {
+        // Weights -> tensor memory: thread r copies packed row r, two 16-bit values per 32-bit column
+        // (the layout of an A operand there); the warps of a quadrant take K blocks in turn.
+        const int kb_x = l == 0 ? a.I / BK : kb_h;
+        const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
+        const T* wrow = reinterpret_cast<const T*>(a.Wp) +
+                        (static_cast<size_t>(l) * 4 * a.H + tile * kGateRows + r_loc) * (a.I + a.H);
+        for (int b = sub; b < rec_t + in_t; b += C::kWarps / 4) {
+          const uint4* src = reinterpret_cast<const uint4*>(wrow + (b < rec_t ? a.I + b * BK : (b - rec_t) * BK));
+          uint32_t v[32];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 x4 = __ldg(src + i);
+            v[4 * i + 0] = x4.x; v[4 * i + 1] = x4.y; v[4 * i + 2] = x4.z; v[4 * i + 3] = x4.w;
+          }
+          tmem_st32(tmem_w + (static_cast<uint32_t>(q * 32) << 16) + b * 32, v);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&w_tmem);
+      }
+      float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (a.bias_p != nullptr)
+        bias = __ldg(reinterpret_cast<const float4*>(a.bias_p + static_cast<size_t>(l) * 4 * a.H + tile * kGateRows) + (r_loc >> 2));
+      T* hs_l = reinterpret_cast<T*>(a.hs) + static_cast<size_t>(l) * a.T * a.H;
+      float creg[C::kChunks][4];
+#pragma unroll
+      for (int ch = 0; ch < C::kChunks; ++ch)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) creg[ch][i] = 0.f;
+      Rows now = rows_of(a, 0);
+      for (int t = 0; t < steps; ++t, ++k) {
+        const int acc = k & 1;
+        const Rows next = rows_of(a, t + 1);
+        ok = mbar_wait_warp(&acc_full[acc], (k >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t r[C::kChunks][16];
+#pragma unroll
+        for (int ch = 0; ch < C::kChunks; ++ch)
+          tmem_ld16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NB + (sub * C::kChunks + ch) * 16, r[ch]);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+#pragma unroll
+        for (int ch = 0; ch < C::kChunks; ++ch) {
+          float v[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[ch][i]);
+          float h[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            // lane q of a quad: gate q of sequences i, 4 + i, 8 + i, 12 + i -> all gates of sequence 4 q + i
+            quad_transpose(v[i], v[4 + i], v[8 + i], v[12 + i], lane);
+            const float gi = v[i] + bias.x;
+            const float gf = v[4 + i] + bias.y;
+            const float go = v[8 + i] + bias.z;
+            const float gc = v[12 + i] + bias.w;
+            const float c_new = sigmoid_fast(gf) * creg[ch][i] + sigmoid_fast(gi) * tanh_fast(gc);
+            creg[ch][i] = c_new;
+            h[i] = sigmoid_fast(go) * tanh_fast(c_new);
+          }
+          // (unit, 4 sequences) -> (4 units, 1 sequence): trade halves with the units next to this one, twice
+          const uint32_t p01 = Fmt<T>::pack2(h[0], h[1]), p23 = Fmt<T>::pack2(h[2], h[3]);
+          uint32_t other = __shfl_xor_sync(0xffffffffu, ub0 ? p01 : p23, 4);
+          const uint32_t lo = ub0 ? other : p01, hi = ub0 ? p23 : other;  // units u & ~1 and u | 1
+          const uint32_t w0 = __byte_perm(lo, hi, 0x5410), w1 = __byte_perm(lo, hi, 0x7632);
+          other = __shfl_xor_sync(0xffffffffu, ub1 ? w0 : w1, 8);
+          const int n = n_base + n_store + ch * 16;
+          if (n < now.active)
+            st_relaxed_gpu64(hs_l + (now.first + n) * a.H + (unit & ~3), ub1 ? other : w0, ub1 ? w1 : other);
+        }
+        {
+          const long long c0 = clock64();
+          while (clock64() - c0 < pause) {}
+        }
+        int rounds = 0;
+        // The state of this step, for the next: eight K blocks of four rows in flight at a time.
+        const bool more = t + 1 < steps;
+#pragma unroll
+        for (int rh = 0; rh < C::kRows; rh += 4) {
+          const int n = n_load + rh;
+          const bool mine = n_base + n < next.active;
+          const T* src = hs_l + (now.first + n_base + n) * a.H + (lane & 7) * 8;
+          uint8_t* dst = s_state + n * 128 + (((lane & 7) ^ (n & 7)) << 4);
+          for (int kb0 = 0; kb0 < kb_h && more && ok; kb0 += 8) {
+            uint64_t x[8], y[8];
+            uint32_t missing = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              x[i] = y[i] = 0;
+              if (mine && kb0 + i < kb_h) missing |= 1u << i;
+            }
+            uint64_t t0 = 0;
+            for (uint32_t it = 1;; ++it) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (missing & (1u << i)) ld_relaxed_gpu_2x64(src + (kb0 + i) * BK, x[i], y[i]);
+              if (it == 1 && rh == 0 && kb0 == 0) {
+                // this warp's part of the step is on its way: count it in for the publisher
+                __syncwarp();
+                if (lane == 0) {
+                  __threadfence_block();
+                  atomicAdd(&n_stored, 1);
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (arrived(x[i]) && arrived(y[i])) missing &= ~(1u << i);
+              ++rounds;
+              if (__all_sync(0xffffffffu, missing == 0)) break;
+              if ((it & 0x3F) == 0) {
+                if (t0 == 0) t0 = globaltimer_ns();
+                if (__any_sync(0xffffffffu, *abort_flag != 0 || globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS)) {
+                  ok = false;
+                  break;
+                }
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (kb0 + i < kb_h) *reinterpret_cast<ulonglong2*>(dst + (kb0 + i) * C::kBlockBytes) = make_ulonglong2(x[i], y[i]);
+          }
+        }
+        if (more) {
+          // Everything in the first round: try a little earlier next time; else later.
+          const bool early = rounds > (C::kRows / 4) * ((kb_h + 7) / 8);
+          pause = early ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
+          if (!ok) {
+            if (lane == 0 && *abort_flag == 0) {
+              *abort_flag = 1;
+              atomicCAS(status, 0, FTB_ERR_TIMEOUT_DEP);
+            }
+            break;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&st_full);
+        } else {
+          __syncwarp();
+          if (lane == 0) {
+            __threadfence_block();
+            atomicAdd(&n_stored, 1);
+          }
+        }
+        if (next.active < now.active) {
+          // sequences that end here: their final cell state
+#pragma unroll
+          for (int ch = 0; ch < C::kChunks; ++ch)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int n = n_base + n_own + ch * 16 + i;
+              if (n < now.active && n >= next.active)
+                a.c_out[(static_cast<size_t>(l) * a.c_rows + n) * a.H + unit] = creg[ch][i];
+            }
+        }
+        now = next;
+      }
+    }
+  }
+
+  // ------------------------------------------------------------------ teardown
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    if (s_abort) {
+      // Give copies and MMAs still in flight time to land before TMEM and shared memory go back.
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+}  // namespace flow
+
+}  // namespace ftb

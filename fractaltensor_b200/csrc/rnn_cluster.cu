@@ -42,6 +42,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "lstm_flow.cuh"
 #include "ptx.cuh"
 #include "tmap.h"
 
@@ -87,11 +88,13 @@ __device__ unsigned long long* g_cluster_acct = nullptr;
 struct ClusterArgs {
   int D, L, N, H;  // layers, steps of a chain (dilated: time steps; grid: B), batch, hidden size
   int A;           // grid: rows of the grid (chains per layer and slice); dilated: 1
-  int S;           // grid: batch slices of NB columns; dilated: flag slots per cell (slices of 64)
+  int S;           // grid: batch slices of NB columns; dilated: counters per cell, one for `slot` sequences
+  int slot;        // dilated: the narrowest slice of the launch
   int CL;          // CTAs per cluster
   int max_dil;
   int dil[kMaxLayers];
-  int nb[kMaxLayers];              // dilated: batch columns per cluster of the layer (64 or 128)
+  int nb[kMaxLayers];              // dilated: batch columns per chain of the layer
+  bool flow;                       // dilated: layers with dilation 1 run flow::body
   int first_cluster[kMaxLayers + 1];  // dilated: index of the layer's first cluster
   const void* W0;       // dilated: Wp [D,4H,2H]; grid: Wpx [D,H,3H]
   const void* W1;       // grid: Wpy
@@ -100,7 +103,7 @@ struct ClusterArgs {
   void* out0;           // dilated: hs [D,L,N,H]; grid: hx [D,A,B,N,H]
   void* out1;           // grid: hy
   float* c;             // dilated: fp32 [D, max_dil*N, H]
-  int* flags;           // [cells][CL], zero before the launch
+  int* flags;           // grid: [cells][CL] flags; dilated: [cells][S] counters of CTAs; zero before the launch
   int* status;
 };
 
@@ -109,7 +112,7 @@ struct ClusterArgs {
 struct Segment {
   int map, row, nkb, wkb0;
   const int* flags;  // nullptr: an input of the call
-  int nflags;
+  int nflags, target;
 };
 struct StepPlan {
   int nseg;
@@ -122,13 +125,13 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Whole-warp bounded wait until the n flags at `flags` are all non-zero (lane i polls flags i, i+32, ...).
-__device__ __forceinline__ bool warp_wait_flags(const int* flags, int n, int lane, volatile int* s_abort, int* g_status) {
+// Whole-warp bounded wait until the n flags at `flags` have all reached `target` (lane i polls flags i, i+32, ...).
+__device__ __forceinline__ bool warp_wait_flags(const int* flags, int n, int target, int lane, volatile int* s_abort, int* g_status) {
   uint64_t t0 = 0;
   uint32_t it = 0;
   for (;;) {
     bool ready = true;
-    for (int i = lane; i < n; i += 32) ready = ready && (ld_acquire_gpu(flags + i) != 0);
+    for (int i = lane; i < n; i += 32) ready = ready && (ld_acquire_gpu(flags + i) >= target);
     if (__all_sync(0xffffffffu, ready)) return true;
     if (((++it) & 0x3F) == 0) {
       if (t0 == 0) t0 = globaltimer_ns();
@@ -181,18 +184,7 @@ __device__ __forceinline__ void umma_commit_to(uint64_t* bar, uint16_t mask) {
       : "memory");
 }
 
-__device__ __forceinline__ void quad_transpose(float& a0, float& a1, float& a2, float& a3, int lane) {
-  const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
-  float r;
-  r = __shfl_xor_sync(0xffffffffu, b0 ? a0 : a1, 1);
-  if (b0) a0 = r; else a1 = r;
-  r = __shfl_xor_sync(0xffffffffu, b0 ? a2 : a3, 1);
-  if (b0) a2 = r; else a3 = r;
-  r = __shfl_xor_sync(0xffffffffu, b1 ? a0 : a2, 2);
-  if (b1) a0 = r; else a2 = r;
-  r = __shfl_xor_sync(0xffffffffu, b1 ? a1 : a3, 2);
-  if (b1) a1 = r; else a3 = r;
-}
+using flow::quad_transpose;
 
 template <typename T>
 __device__ __forceinline__ T to_elem(float v);
@@ -224,13 +216,14 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
     } else {
       x.map = 1;
       x.row = ((layer - 1) * a.L + i) * a.N + slice * NB;
-      // One flag slot per 64 sequences of a cell; a cluster publishes in the slot of its first 64.  The
-      // layer below may be cut differently: its clusters that hold this slice's rows own consecutive slots.
+      // One counter per `slot` sequences of a cell; a chain's CTAs count in that of its first ones.  The
+      // layer below may be cut differently: its chains that hold this slice's rows own consecutive counters.
       const int nbp = a.nb[layer - 1];
-      const int first = (slice * NB / nbp) * (nbp / 64);
-      x.flags = a.flags + (((layer - 1) * a.L + i) * a.S + first) * a.CL;
-      // (only the clusters that exist: the last slice of the batch may be short)
-      x.nflags = (nbp < NB ? min(NB / nbp, (a.N - slice * NB + nbp - 1) / nbp) : 1) * a.CL;
+      const int first = (slice * NB / nbp) * (nbp / a.slot);
+      x.flags = a.flags + ((layer - 1) * a.L + i) * a.S + first;
+      // (only the chains that exist: the last slice of the batch may be short)
+      x.nflags = nbp < NB ? min(NB / nbp, (a.N - slice * NB + nbp - 1) / nbp) : 1;
+      x.target = a.CL;
     }
     if (i >= d) {
       if (d == 1) {
@@ -243,8 +236,9 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
         h.row = (layer * a.L + i - d) * a.N + slice * NB;
         h.nkb = kbh;
         h.wkb0 = kbh;
-        h.flags = a.flags + ((layer * a.L + i - d) * a.S + slice * (NB / 64)) * a.CL;
-        h.nflags = a.CL;
+        h.flags = a.flags + (layer * a.L + i - d) * a.S + slice * (NB / a.slot);
+        h.nflags = 1;
+        h.target = a.CL;
       }
     }
   } else {
@@ -265,6 +259,7 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
       in.row = below * a.N + slice * NB;
       in.flags = a.flags + (below * a.S + slice) * a.CL + (ydir ? a.CL / 2 : 0);
       in.nflags = a.CL / 2;
+      in.target = 1;
     }
     if (row_a > 0) {
       const int up = (layer * a.A + row_a - 1) * a.L + i;
@@ -275,6 +270,7 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
       sx.wkb0 = 0;
       sx.flags = a.flags + (up * a.S + slice) * a.CL;  // the x-direction tiles come first
       sx.nflags = a.CL / 2;
+      sx.target = 1;
     }
     if (i > 0) {
       p.self = true;
@@ -293,8 +289,8 @@ template <typename T, int MODE, int NB>
 __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUtensorMap& map1, const CUtensorMap& map2,
                                              const CUtensorMap& map3, const CUtensorMap& mapO0,
                                              const CUtensorMap& mapO1, const CUtensorMap& mapT0,
-                                             const CUtensorMap& mapT1, const ClusterArgs& a, const int cid,
-                                             const int layer, const int row_a, const int slice) {
+                                             const CUtensorMap& mapT1, const ClusterArgs& a, const int rank,
+                                             const int cid, const int layer, const int row_a, const int slice) {
   constexpr int kEpiWarps = epi_warps(MODE);
   constexpr int kSub = kEpiWarps / 4;              // epilogue warps per TMEM lane quadrant
   constexpr int kBlocksPerStage = 128 / NB;        // [NB x 64] 16-bit blocks per 16 KB stage
@@ -317,7 +313,6 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int rank = static_cast<int>(cluster_ctarank());
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   int* status = a.status;
 
@@ -414,7 +409,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         const Segment& sg = p.seg[s];
         if ((s & 1) == mine) {
           ACCT_BEGIN();
-          if (sg.flags != nullptr && !warp_wait_flags(sg.flags, sg.nflags, lane, &s_abort, status)) {
+          if (sg.flags != nullptr && !warp_wait_flags(sg.flags, sg.nflags, sg.target, lane, &s_abort, status)) {
             ok = false;
             break;
           }
@@ -422,7 +417,9 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           bool fine = true;
           if (lane == 0) {
             // (Producers write their outputs with TMA stores and consumers read them with TMA loads: both
-            // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.)
+            // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.
+            // Threads store the output of flow::body.)
+            if (MODE == kDilated && a.flow && s == 0 && layer > 0 && a.dil[layer - 1] == 1) fence_proxy_async_all();
             FTB_CL_STAMP(i, 7 + 2 * s);
             ACCT_BEGIN();
             if (*seq != q) {
@@ -626,7 +623,10 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         tma_store_wait_read<0>();
         *stored = i + 1;  // the tile may be overwritten (two steps from now)
         tma_store_wait<0>();
-        st_release_gpu(a.flags + ((my_flag_cell0 + i) * a.S + slice * (MODE == kDilated ? NB / 64 : 1)) * a.CL + rank, 1);
+        if (MODE == kDilated)
+          red_release_gpu_add(a.flags + (my_flag_cell0 + i) * a.S + slice * (NB / a.slot), 1);
+        else
+          st_release_gpu(a.flags + ((my_flag_cell0 + i) * a.S + slice) * a.CL + rank, 1);
         ACCT_END(1);
         FTB_CL_STAMP(i, 11);
       }
@@ -875,7 +875,7 @@ rnn_cluster_kernel(const __grid_constant__ CUtensorMap map0, const __grid_consta
   const int ra = cid / a.S;
   const int layer = ra / a.A;
   const int row_a = ra - layer * a.A;
-  cluster_body<T, MODE, NB>(map0, map1, map2, map3, mapO0, mapO1, mapT0, mapT1, a, cid, layer, row_a, slice);
+  cluster_body<T, MODE, NB>(map0, map1, map2, map3, mapO0, mapO1, mapT0, mapT1, a, cluster_ctarank(), cid, layer, row_a, slice);
 }
 
 // Dilated LSTM: a layer's clusters take 64 or 128 sequences each (a.nb[layer]).  A layer whose step
@@ -896,9 +896,33 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
   while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
   const int slice = cid - a.first_cluster[layer];
   if (a.nb[layer] == 64)
-    cluster_body<T, kDilated, 64>(x64, h64, h64, h64, o64, o64, t64, t64, a, cid, layer, 0, slice);
+    cluster_body<T, kDilated, 64>(x64, h64, h64, h64, o64, o64, t64, t64, a, cluster_ctarank(), cid, layer, 0, slice);
   else
-    cluster_body<T, kDilated, 128>(x128, h128, h128, h128, o128, o128, t128, t128, a, cid, layer, 0, slice);
+    cluster_body<T, kDilated, 128>(x128, h128, h128, h128, o128, o128, t128, t128, a, cluster_ctarank(), cid, layer, 0, slice);
+}
+
+// The same program without clusters, for batches that fit on slices of 64 beside this: what the layers with
+// dilation >= 2 exchange goes through global memory anyway (2.2 us a step on slices of 64, 3.0 on 128: a
+// layer with dilation 2 waits for the trip there and back).  A layer with dilation 1 runs as csrc/lstm_flow.cu
+// does, on slices of kNarrow sequences whose state is its own flag: 1.6 us a step at H 256 where a cluster's
+// hand-off of 64 takes 2.6, and no GPC has to hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).
+template <typename T, int kNarrow>
+__global__ void __launch_bounds__(cta_threads(kDilated), 1)
+rnn_dilated_flow_kernel(const __grid_constant__ CUtensorMap x, const __grid_constant__ CUtensorMap h,
+                        const __grid_constant__ CUtensorMap o, const __grid_constant__ CUtensorMap t,
+                        const __grid_constant__ CUtensorMap nx, const __grid_constant__ CUtensorMap nh,
+                        const __grid_constant__ CUtensorMap nw, const ClusterArgs a, const flow::FlowArgs f) {
+  const int cid = blockIdx.x / a.CL, rank = blockIdx.x - cid * a.CL;
+  int layer = 0;
+  while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
+  const int slice = cid - a.first_cluster[layer];
+  if (a.dil[layer] == 1) {
+    flow::FlowArgs fl = f;
+    fl.below = layer > 0 ? a.nb[layer - 1] / kNarrow : 1;
+    flow::body<T, kNarrow>(nx, nh, nw, fl, rank, slice, layer);
+  } else {
+    cluster_body<T, kDilated, 64>(x, h, h, h, o, o, t, t, a, rank, cid, layer, 0, slice);
+  }
 }
 
 // Tensor map of a row-major [rows, H] activation matrix as the kernel's operand loads see it: three
@@ -909,9 +933,9 @@ int make_operand_map(CUtensorMap* out, const void* base, int dtype, uint64_t row
                       static_cast<uint32_t>(nb), static_cast<uint32_t>(H / 64));
 }
 
-template <typename Kernel>
-int launch_kernel(Kernel kfn, int threads, std::atomic<unsigned long long>& configured, const CUtensorMap* m,
-                  const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
+template <typename Kernel, typename... Args>
+int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned long long>& configured, int grid,
+                  uint32_t smem_bytes, cudaStream_t stream, const Args&... args) {
   // the largest request of this instantiation (static shared memory comes on top of it)
   constexpr int kMaxDynamic = 226 * 1024;
   if (smem_bytes > static_cast<uint32_t>(kMaxDynamic) || !ensure_dynamic_smem(kfn, kMaxDynamic, configured))
@@ -923,11 +947,13 @@ int launch_kernel(Kernel kfn, int threads, std::atomic<unsigned long long>& conf
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   int na = 0;
-  attrs[na].id = cudaLaunchAttributeClusterDimension;
-  attrs[na].val.clusterDim.x = a.CL;
-  attrs[na].val.clusterDim.y = 1;
-  attrs[na].val.clusterDim.z = 1;
-  ++na;
+  if (cluster > 1) {
+    attrs[na].id = cudaLaunchAttributeClusterDimension;
+    attrs[na].val.clusterDim.x = cluster;
+    attrs[na].val.clusterDim.y = 1;
+    attrs[na].val.clusterDim.z = 1;
+    ++na;
+  }
   // FTB_NO_COOPERATIVE=1 drops the cooperative attribute (profilers that cannot replay cooperative
   // launches); residency then rests on the grid fitting an otherwise idle device, and the bounded
   // waits turn a violated assumption into a status code.
@@ -948,7 +974,7 @@ int launch_kernel(Kernel kfn, int threads, std::atomic<unsigned long long>& conf
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  const cudaError_t err = cudaLaunchKernelEx(&cfg, kfn, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kfn, args...);
   if (err != cudaSuccess) {
     if (getenv("FTB_VERBOSE") != nullptr) fprintf(stderr, "rnn_cluster launch: %s\n", cudaGetErrorString(err));
     cudaGetLastError();
@@ -961,12 +987,21 @@ int launch_kernel(Kernel kfn, int threads, std::atomic<unsigned long long>& conf
 template <typename T, int MODE, int NB>
 int launch(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_cluster_kernel<T, MODE, NB>, cta_threads(MODE), configured, m, a, grid, smem_bytes, stream);
+  return launch_kernel(rnn_cluster_kernel<T, MODE, NB>, a.CL, cta_threads(MODE), configured, grid, smem_bytes, stream, m[0],
+                       m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
 }
 template <typename T>
 int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_cluster_dilated_kernel<T>, cta_threads(kDilated), configured, m, a, grid, smem_bytes, stream);
+  return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, cta_threads(kDilated), configured, grid, smem_bytes, stream, m[0],
+                       m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
+}
+template <typename T, int kNarrow>
+int launch_dilated_flow(const CUtensorMap* m, const ClusterArgs& a, const flow::FlowArgs& f, int grid, uint32_t smem_bytes,
+                        cudaStream_t stream) {
+  static std::atomic<unsigned long long> configured{0};
+  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, cta_threads(kDilated), configured, grid, smem_bytes, stream,
+                       m[0], m[1], m[2], m[3], m[4], m[5], m[6], a, f);
 }
 
 uint32_t smem_for(bool any_self, int H, int NB, int self_units, int out_units, int ring_self) {
@@ -996,6 +1031,24 @@ int dilated_slices(const int* dilations, int D, int N, int max_clusters, int* nb
     total += n64 ? s64 : s128;
   }
   return s128 <= 8 && total <= max_clusters ? total : 0;
+}
+
+// Slice width of the layers with dilation 1 when the launch goes without clusters, 0: it does not.  The
+// narrowest that leaves room for the other layers on slices of 64 (with those on slices of 128, dilations 1 to 32
+// at H 256 and 256 sequences took 1654 us, 1610 with clusters).  Clusters of 2 and 4 CTAs hand a state on fast
+// enough for batches of up to 64 (us, 3 layers of 512 steps, with clusters / without: H 64, N 24 895 / 911, N 64
+// 985 / 1105; H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above 64 sequences and at H 256
+// they lose: H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1191).
+constexpr int kFlowWide = 64;
+int dilated_flow_width(const int* dilations, int D, int N, int CL, int sm_count, int* chains) {
+  int ones = 0;
+  for (int l = 0; l < D; ++l) ones += dilations[l] == 1;
+  if (ones == 0 || (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64)) return 0;
+  for (int nb = 16; nb <= 32; nb *= 2) {
+    *chains = ones * ((N + nb - 1) / nb) + (D - ones) * ((N + kFlowWide - 1) / kFlowWide);
+    if (*chains * CL <= sm_count) return nb;
+  }
+  return 0;
 }
 
 // Clusters of `cl` CTAs of the dilated kernel that can be resident at once on the current device (a
@@ -1040,16 +1093,15 @@ bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count
   return dilated_slices(nullptr, D, N, sm_count / (4 * H / 128), nullptr) > 0;
 }
 
-// one flag per (cell, slot of 64 sequences, CTA of the cluster); at most 16 slots (8 slices of 128) x 8 CTAs
-size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 16 * 8; }
+// one counter per (cell, slot of 16 sequences or more); at most 64 slots (8 slices of 128)
+size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 64; }
 
-// x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S*CL ints (zeroed here).
+// x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
-                                const int* dilations, int D, int L, int N, int H, int* flags, int* status,
+                                const int* dilations, int D, int L, int N, int H, int* flags, int* status, int sm_count,
                                 cudaStream_t stream) {
   ClusterArgs a = {};
   a.D = D; a.L = L; a.N = N; a.H = H; a.A = 1;
-  a.S = 2 * ((N + 127) / 128);  // flag slots per cell
   a.CL = 4 * H / 128;
   a.max_dil = 1;
   bool any_self = false;
@@ -1058,15 +1110,55 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     a.max_dil = std::max(a.max_dil, dilations[l]);
     any_self = any_self || dilations[l] == 1;
   }
+  a.W0 = Wp; a.bias0 = bias_p; a.out0 = hs; a.c = c; a.flags = flags; a.status = status;
+  const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
+  CUtensorMap m[8];
+  int rc, chains = 0;
+  const int narrow = dilated_flow_width(dilations, D, N, a.CL, sm_count, &chains);
+  if (narrow > 0) {
+    constexpr int wide = kFlowWide;
+    a.flow = true;
+    a.slot = narrow;
+    a.S = (N + wide - 1) / wide * (wide / narrow);
+    for (int l = 0; l < D; ++l) {
+      a.nb[l] = dilations[l] == 1 ? narrow : wide;
+      a.first_cluster[l + 1] = a.first_cluster[l] + (N + a.nb[l] - 1) / a.nb[l];
+    }
+    const int tail = N - ((N + wide - 1) / wide - 1) * wide;
+    if ((rc = make_operand_map(&m[0], x, dtype, x_rows, H, wide))) return rc;
+    if ((rc = make_operand_map(&m[1], hs, dtype, h_rows, H, wide))) return rc;
+    if ((rc = make_tmap_2d(&m[2], hs, dtype, h_rows, H, H, wide, 32, false))) return rc;
+    if ((rc = make_tmap_2d(&m[3], hs, dtype, h_rows, H, H, tail, 32, false))) return rc;
+    const uint64_t row_bytes = static_cast<uint64_t>(H) * 2;
+    const uint32_t planes = 128 / narrow;  // of a copy of flow::body
+    if ((rc = make_tmap_3d(&m[4], x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
+    if ((rc = make_tmap_3d(&m[5], hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
+    if ((rc = make_tmap_2d(&m[6], Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H, 2 * H, flow::kGateRows, 64))) return rc;
+    flow::FlowArgs f = {};
+    f.D = D; f.L = L; f.N = N; f.I = H; f.H = H; f.G = D; f.S = a.S;
+    f.n_tiles = a.CL;
+    f.n_slots = flow::kMaxSlots;
+    f.T = static_cast<int64_t>(L) * N;
+    f.bias_p = bias_p; f.Wp = Wp; f.hs = hs; f.c_out = c; f.c_rows = a.max_dil * N; f.flags = flags; f.status = status;
+    if (cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(D) * L * a.S, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
+    const size_t layer_bytes = static_cast<size_t>(L) * N * H * 2;
+    for (int l = 0; l < D; ++l)
+      if (dilations[l] == 1 && cudaMemsetAsync(static_cast<char*>(hs) + l * layer_bytes, 0xFF, layer_bytes, stream) != cudaSuccess)
+        return FTB_ERR_LAUNCH;
+    const uint32_t smem = smem_for(false, H, wide, 32, 32, 0);
+    const int grid = chains * a.CL;
+    if (dtype == FTB_F16)
+      return narrow == 16 ? launch_dilated_flow<__half, 16>(m, a, f, grid, smem, stream)
+                          : launch_dilated_flow<__half, 32>(m, a, f, grid, smem, stream);
+    return narrow == 16 ? launch_dilated_flow<__nv_bfloat16, 16>(m, a, f, grid, smem, stream)
+                        : launch_dilated_flow<__nv_bfloat16, 32>(m, a, f, grid, smem, stream);
+  }
   const uint32_t smem = smem_for(any_self, H, 128, 32, 32, 4);
   const int clusters = dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, smem), a.nb);
   if (clusters <= 0) return FTB_ERR_LAUNCH;  // does not fit on this device: the caller's generic wavefront takes it
-  a.first_cluster[0] = 0;
+  a.S = 2 * ((N + 127) / 128);
+  a.slot = 64;
   for (int l = 0; l < D; ++l) a.first_cluster[l + 1] = a.first_cluster[l] + (N + a.nb[l] - 1) / a.nb[l];
-  a.W0 = Wp; a.bias0 = bias_p; a.out0 = hs; a.c = c; a.flags = flags; a.status = status;
-  CUtensorMap m[8];
-  int rc;
-  const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
   if ((rc = make_operand_map(&m[0], x, dtype, x_rows, H, 128))) return rc;
   if ((rc = make_operand_map(&m[1], hs, dtype, h_rows, H, 128))) return rc;
   if ((rc = make_operand_map(&m[2], x, dtype, x_rows, H, 64))) return rc;
@@ -1077,7 +1169,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   if ((rc = make_tmap_2d(&m[5], hs, dtype, h_rows, H, H, 64, 32, false))) return rc;
   if ((rc = make_tmap_2d(&m[6], hs, dtype, h_rows, H, H, tail128, 32, false))) return rc;
   if ((rc = make_tmap_2d(&m[7], hs, dtype, h_rows, H, H, tail64, 32, false))) return rc;
-  const size_t n_flags = static_cast<size_t>(D) * L * a.S * a.CL;
+  const size_t n_flags = static_cast<size_t>(D) * L * a.S;
   if (cudaMemsetAsync(flags, 0, sizeof(int) * n_flags, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
   const int grid = clusters * a.CL;
   if (dtype == FTB_F16) return launch_dilated<__half>(m, a, grid, smem, stream);

@@ -49,7 +49,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
 bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count);
 size_t lstm_dilated_cluster_flag_ints(int D, int L);
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
-                                const int* dilations, int D, int L, int N, int H, int* flags, int* status,
+                                const int* dilations, int D, int L, int N, int H, int* flags, int* status, int sm_count,
                                 cudaStream_t stream);
 bool grid_rnn_cluster_supported(int dtype, int D, int A, int B, int N, int H, int sm_count);
 int launch_grid_rnn_cluster(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy,
@@ -921,7 +921,7 @@ int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, voi
     if ((tune.schedule == 4 || tune.schedule == 0) && can && workspace_bytes >= need) {
       rc = launch_lstm_dilated_cluster(dtype, x, Wp, bias_p, hs, c, dilations, D, L, N, H,
                                        reinterpret_cast<int*>(static_cast<char*>(workspace) + flags_off), status,
-                                       stream);
+                                       cl.sm_count, stream);
       // a refused cooperative cluster launch falls back to the generic wavefront
       if (rc != FTB_ERR_LAUNCH || tune.schedule != 0) return rc;
     }
