@@ -63,7 +63,7 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
   const int tg = threadIdx.x % kGroupThreads;   // thread within the group
   const int tx = tg & 7;   // 4 consecutive columns: one LSTM unit
   const int ty = tg >> 3;  // 2 consecutive rows
-  float acc[2][4] = {};
+  float acc[2][4] = {};  // sums of the chunks so far
 
   // K is walked in chunks of TK over the cell's segments; this group takes chunks [c_begin, c_end) of
   // the walk.  The next chunk's global loads are issued into registers before the current chunk is
@@ -110,6 +110,7 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
       nk0 = 0;
     }
     if (c + 1 < c_end) fetch(ns, nk0);
+    float part[2][4] = {};  // this chunk's
 #pragma unroll
     for (int k4 = 0; k4 < TK; k4 += 4) {
       const float4 r0 = *reinterpret_cast<const float4*>(&sA[grp][2 * ty][k4]);
@@ -118,12 +119,16 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float4 w = *reinterpret_cast<const float4*>(&sW[grp][k4 + j][4 * tx]);
-        acc[0][0] = fmaf(a0[j], w.x, acc[0][0]); acc[0][1] = fmaf(a0[j], w.y, acc[0][1]);
-        acc[0][2] = fmaf(a0[j], w.z, acc[0][2]); acc[0][3] = fmaf(a0[j], w.w, acc[0][3]);
-        acc[1][0] = fmaf(a1[j], w.x, acc[1][0]); acc[1][1] = fmaf(a1[j], w.y, acc[1][1]);
-        acc[1][2] = fmaf(a1[j], w.z, acc[1][2]); acc[1][3] = fmaf(a1[j], w.w, acc[1][3]);
+        part[0][0] = fmaf(a0[j], w.x, part[0][0]); part[0][1] = fmaf(a0[j], w.y, part[0][1]);
+        part[0][2] = fmaf(a0[j], w.z, part[0][2]); part[0][3] = fmaf(a0[j], w.w, part[0][3]);
+        part[1][0] = fmaf(a1[j], w.x, part[1][0]); part[1][1] = fmaf(a1[j], w.y, part[1][1]);
+        part[1][2] = fmaf(a1[j], w.z, part[1][2]); part[1][3] = fmaf(a1[j], w.w, part[1][3]);
       }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
     group_barrier(grp);
     s = ns;
     k0 = nk0;

@@ -170,7 +170,7 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
       // ---- this group's chunks of K, in the level kernel's order.  One warp per group multiplies:
       // a lane holds 4 rows x 8 columns of the tile, so 12 shared-memory loads feed 128 FMAs (the
       // level kernel's 2 x 4 per thread needs 6 per 32 and is bound by shared-memory bandwidth).
-      // Every partial sum is still one chain over the group's K range in ascending order.
+      // Every chunk's sum is one chain in ascending order of K, as there.
       if ((tid >> 5) == grp * 5) {  // warps 0, 5, 10, 15: one per scheduler
         const int lane = tid & 31;
         const int cx = lane & 3;   // columns 8 cx .. 8 cx + 7
@@ -180,23 +180,31 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
         float acc[4][8] = {};
         const float* Ar = sA + (4 * ry) * lda;
         const float* Wc = sW + 8 * cx;
-        for (int k0 = c_begin * TK; k0 < c_end * TK; k0 += 4) {
-          float av[4][4];
+        for (int c = c_begin; c < c_end; ++c) {
+          float part[4][8] = {};
+#pragma unroll 1
+          for (int k0 = c * TK; k0 < (c + 1) * TK; k0 += 4) {
+            float av[4][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 r = *reinterpret_cast<const float4*>(Ar + i * lda + k0);
-            av[i][0] = r.x; av[i][1] = r.y; av[i][2] = r.z; av[i][3] = r.w;
+            for (int i = 0; i < 4; ++i) {
+              const float4 r = *reinterpret_cast<const float4*>(Ar + i * lda + k0);
+              av[i][0] = r.x; av[i][1] = r.y; av[i][2] = r.z; av[i][3] = r.w;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 w0 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw);
+              const float4 w1 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw + 4);
+              const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int n = 0; n < 8; ++n) part[i][n] = fmaf(av[i][q], wv[n], part[i][n]);
+            }
           }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 w0 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw);
-            const float4 w1 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw + 4);
-            const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-              for (int c = 0; c < 8; ++c) acc[i][c] = fmaf(av[i][q], wv[c], acc[i][c]);
-          }
+            for (int n = 0; n < 8; ++n) acc[i][n] += part[i][n];
         }
         float* p = sP + static_cast<size_t>(grp) * TM * TN + (4 * ry) * TN + 8 * cx;
 #pragma unroll

@@ -1,0 +1,50 @@
+"""fp32 stacked LSTM whose states carry their own arrival (csrc/lstm_simt_flow.cu): bit for bit the result
+of one launch per level."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from fractaltensor_b200 import ops as _ops
+    return _ops
+
+
+def _params(ops, D, H, g):
+    u = lambda *s: (torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5
+    return ops.lstm_pack_weights(u(D, 4, H, H), u(D, 4, H, H), u(D, 4, H))
+
+
+@pytest.mark.parametrize("D,L,N,H", [
+    (1, 1, 1, 64),      # one step: nothing handed on
+    (3, 6, 8, 64),      # a full tile of 8 rows
+    (2, 5, 9, 192),     # one sequence in the second tile; a row is not a whole number of warp loads
+    (1, 7, 33, 256),    # one layer: narrow tiles spread over the device
+    (4, 64, 32, 256),   # tiles of 32, a CTA per tile and layer
+    (4, 9, 64, 256),    # layers in groups: weights replaced between sweeps
+    (3, 2, 31, 320),    # the widest state: one input tile beside the weights
+    (16, 3, 5, 128),
+])
+def test_same_bits_as_levels(ops, D, L, N, H):
+    g = torch.Generator(device="cuda").manual_seed(D * 100 + N)
+    Wp, b = _params(ops, D, H, g)
+    x = torch.randn(L, N, H, device="cuda", generator=g)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1)
+    for _ in range(3):  # the fill pattern of a call must not survive into the next
+        h, c = ops.lstm_stacked(x, Wp, b, schedule=2)
+        ops.check_status()
+        assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+def test_nan_states_are_states(ops):
+    """A NaN hidden state is a value like any other (0x7FFFFFFF, not the fill pattern): nothing waits for it."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    Wp, b = _params(ops, 2, 128, g)
+    x = torch.randn(6, 5, 128, device="cuda", generator=g)
+    x[2, 3] = float("nan")
+    x.view(torch.int32)[2, 4] = -1  # 0xFFFFFFFF: a NaN with the fill pattern's bits, as an input
+    h, _ = ops.lstm_stacked(x, Wp, b, schedule=2)
+    ops.check_status()
+    assert not torch.isnan(h[:, :, :3]).any() and torch.isnan(h[:, 2:, 3:]).all() and not torch.isnan(h[:, :2]).any()
