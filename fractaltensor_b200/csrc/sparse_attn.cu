@@ -299,8 +299,8 @@ __device__ __forceinline__ void attend_token(const SparseArgs& a, const Rows<T>&
   store_row_global<T, LPT>(out_row, gl, acc);
 }
 
-// One token of an interior tile with the numbers of window and random keys known at compile time
-// (the example's 5 and 3): no per-key bookkeeping, one softmax over the KW + KR scores.  Window rows
+// One token of an interior tile with the number of random keys known at compile time, and that of window keys
+// (KW > 0) or a bound on it (KW < 0: up to -KW): no per-key bookkeeping, one softmax over the scores.  Window rows
 // come from the stage, random rows from global memory; the random rows of K and V are requested
 // first, so that they arrive while the window part is computed out of shared memory.
 template <typename T, int LPT, int KW, int KR>
@@ -308,7 +308,9 @@ __device__ __forceinline__ void attend_fast(const SparseArgs& a, const T* sk, co
                                             const T* vh, int i, int gl, unsigned gmask, const float (&qv)[kEPL],
                                             const int* sp, T* __restrict__ out_row, int* __restrict__ status) {
   constexpr int d = kEPL * LPT;
-  const int half = (KW - 1) * a.dilation / 2;
+  constexpr int NW = KW > 0 ? KW : -KW;
+  const int n_window = KW > 0 ? KW : a.window;
+  const int half = (n_window - 1) * a.dilation / 2;
   const float scale2 = a.scale * 1.4426950408889634f;
   float kr[KR][kEPL], vr[KR][kEPL];
 #pragma unroll
@@ -321,22 +323,26 @@ __device__ __forceinline__ void attend_fast(const SparseArgs& a, const T* sk, co
     load_row_global<T, LPT>(kh + static_cast<long long>(x) * d, gl, kr[r]);
     load_row_global<T, LPT>(vh + static_cast<long long>(x) * d, gl, vr[r]);
   }
-  float sc[KW + KR];
+  float sc[NW + KR];
   const int row0 = i - half - lo;  // the first window row inside the stage
 #pragma unroll
-  for (int j = 0; j < KW; ++j) {
+  for (int j = 0; j < NW; ++j) {
+    if (KW < 0 && j >= n_window) {
+      sc[j] = -INFINITY;
+      continue;
+    }
     float kw[kEPL];
     load_row_shared<T, LPT>(sk + (row0 + j * a.dilation) * d, gl, kw);
     sc[j] = group_dot<LPT>(qv, kw, gmask) * scale2;
   }
 #pragma unroll
-  for (int r = 0; r < KR; ++r) sc[KW + r] = group_dot<LPT>(qv, kr[r], gmask) * scale2;
+  for (int r = 0; r < KR; ++r) sc[NW + r] = group_dot<LPT>(qv, kr[r], gmask) * scale2;
   float m = sc[0];
 #pragma unroll
-  for (int j = 1; j < KW + KR; ++j) m = fmaxf(m, sc[j]);
+  for (int j = 1; j < NW + KR; ++j) m = fmaxf(m, sc[j]);
   float z = 0.f;
 #pragma unroll
-  for (int j = 0; j < KW + KR; ++j) {
+  for (int j = 0; j < NW + KR; ++j) {
     sc[j] = exp2_fast(sc[j] - m);
     z += sc[j];
   }
@@ -344,7 +350,8 @@ __device__ __forceinline__ void attend_fast(const SparseArgs& a, const T* sk, co
 #pragma unroll
   for (int e = 0; e < kEPL; ++e) acc[e] = 0.f;
 #pragma unroll
-  for (int j = 0; j < KW; ++j) {
+  for (int j = 0; j < NW; ++j) {
+    if (KW < 0 && j >= n_window) continue;
     float vw[kEPL];
     load_row_shared<T, LPT>(sv + (row0 + j * a.dilation) * d, gl, vw);
 #pragma unroll
@@ -353,7 +360,7 @@ __device__ __forceinline__ void attend_fast(const SparseArgs& a, const T* sk, co
 #pragma unroll
   for (int r = 0; r < KR; ++r) {
 #pragma unroll
-    for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[KW + r], vr[r][e], acc[e]);
+    for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[NW + r], vr[r][e], acc[e]);
   }
   const float inv = 1.f / z;
 #pragma unroll
@@ -407,8 +414,9 @@ sparse_attn_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
 // ------------------------------------------------------------------ tiled kernel
 // The walk of one CTA over its work items: item number first, first + step, ... of the enumeration
 // (per_head, lead, skip).  it_base = tiles the CTA has walked before (the stages and barrier phases
-// carry on from there); returns that count plus the tiles of this walk, or -1 after a wait ran out.  KW > 0: the items are interior tiles and a token has KW window and KR
-// random keys (attend_fast); KW = 0: any tile, any key counts (attend_token).
+// carry on from there); returns that count plus the tiles of this walk, or -1 after a wait ran out.  KW != 0: the
+// items are interior tiles and a token has KW (up to -KW) window and KR random keys (attend_fast); KW = 0: any
+// tile, any key counts (attend_token).
 template <typename T, int LPT, int KW, int KR>
 __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                           const int* __restrict__ rand_pos, T* __restrict__ o, const SparseArgs& a,
@@ -516,7 +524,7 @@ __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __re
       const int i = x.t0 + tok;
       float qv[kEPL];
       load_row_shared<T, LPT>(stage_q(s) + tok * d, gl, qv);
-      if constexpr (KW > 0) {
+      if constexpr (KW != 0) {
         attend_fast<T, LPT, KW, KR>(a, rw.sk, rw.sv, x.lo, rw.kh, rw.vh, i, gl, gmask, qv, sp + tok * KR,
                                     o + (x.head * S + i) * d, status);
       } else {
@@ -531,9 +539,9 @@ __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __re
 }
 
 // ------------------------------------------------------------------ tiled kernel
-// KW = 0: every CTA walks the enumeration (per_head, lead, skip) with the general routine.  KW > 0:
+// KW = 0: every CTA walks the enumeration (per_head, lead, skip) with the general routine.  KW != 0:
 // every CTA first walks its share of the edge tiles with the general routine, then its share of the
-// interior tiles with the routine built for KW window and KR random keys; the two walks are separate
+// interior tiles with the routine built for its key counts; the two walks are separate
 // pieces of code, so the register count is the larger of the two, not their sum.
 template <typename T, int LPT, int KW, int KR>
 __global__ void __launch_bounds__(kSparseThreads)
@@ -551,7 +559,7 @@ sparse_attn_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   grid_launch_dependents();
   __syncthreads();
   grid_dependency_wait();  // set-up done; the first copy of the walk reads global memory
-  if constexpr (KW > 0) {
+  if constexpr (KW != 0) {
     // Edge tiles are handed out from the last CTA down, interior tiles from the first up: when the
     // edge tiles are fewer than the CTAs, the CTAs with one interior tile more do not get them.
     const int done = walk_tiles<T, LPT, 0, 0>(q, k, v, rand_pos, o, a, a.edge_per_head, a.edge_lead, a.edge_skip,
@@ -585,10 +593,18 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
     }
   }
   if (TT > 0) {
-    static std::atomic<unsigned long long> configured{0}, configured_fast{0};
-    auto kfn = sparse_attn_tile_kernel<T, LPT, 0, 0>;
-    auto kfast = sparse_attn_tile_kernel<T, LPT, 5, 3>;
-    if (ensure_dynamic_smem(kfn, kMaxTileSmem, configured) && ensure_dynamic_smem(kfast, kMaxTileSmem, configured_fast)) {
+    static std::atomic<unsigned long long> configured[6];
+    using Kernel = decltype(&sparse_attn_tile_kernel<T, LPT, 0, 0>);
+    // The example's key counts have a routine of their own, 1 to 4 random keys beside a window of up to 7 one
+    // that is told the window's; the rest take the general one, which is issue-bound on its bookkeeping (us, B 2, 16 heads, S 4096, d 64, general /
+    // told the window: window 7 and 4 random keys fp32 67.0 / 53.0, fp16 78.9 / 51.5; 5 and 2 48.4 / 44.4, 54.8 / 39.4;
+    // 3 and 1 34.9 / 30.9, 35.4 / 31.8; the example's 5 and 3 52.8 / 44.3 with its own).
+    const Kernel kernels[6] = {sparse_attn_tile_kernel<T, LPT, 0, 0>, sparse_attn_tile_kernel<T, LPT, -7, 1>,
+                               sparse_attn_tile_kernel<T, LPT, -7, 2>, sparse_attn_tile_kernel<T, LPT, -7, 3>,
+                               sparse_attn_tile_kernel<T, LPT, -7, 4>, sparse_attn_tile_kernel<T, LPT, 5, 3>};
+    const int fast = a.as_shipped || a.window > 7 || a.R < 1 || a.R > 4 ? 0 : (a.window == 5 && a.R == 3 ? 5 : a.R);
+    if (ensure_dynamic_smem(kernels[0], kMaxTileSmem, configured[0]) &&
+        ensure_dynamic_smem(kernels[fast], kMaxTileSmem, configured[fast])) {
       a.TT = TT;
       a.tiles_per_head = (a.S + TT - 1) / TT;
       a.stage_bytes = stage;
@@ -608,9 +624,8 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
         return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
       };
       a.edge_per_head = a.edge_lead = a.edge_skip = 0;
-      if (a.window == 5 && a.R == 3 && !a.as_shipped && interior > 0) {
-        // The example's key counts: interior tiles by the routine built for them, the edge tiles of
-        // every head by the general one on a share of the CTAs in proportion to their number.
+      if (fast != 0 && interior > 0) {
+        // Interior tiles by the routine built for their key counts, the edge tiles of every head by the general one on a share of the CTAs in proportion to their number.
         a.per_head = interior;
         a.lead = 0;
         a.skip = lead;
@@ -618,11 +633,11 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
         a.edge_lead = lead;
         a.edge_skip = interior;
         const long long ctas = a.heads_total * a.tiles_per_head;
-        return run(kfast, a, ctas);
+        return run(kernels[fast], a, ctas);
       }
       a.per_head = a.tiles_per_head;
       a.lead = a.skip = 0;
-      return run(kfn, a, a.heads_total * a.tiles_per_head);
+      return run(kernels[0], a, a.heads_total * a.tiles_per_head);
     }
   }
   a.TT = a.tiles_per_head = a.stage_bytes = a.per_head = a.lead = a.skip = 0;

@@ -157,3 +157,17 @@ def test_sparse_attention_empty_batch_and_single_tile_edges(ops):
     ops.check_status()
     ref = dense.sparse_attention_dense(q.double(), k.double(), v.double(), pos)
     assert (out.cpu().double() - ref).abs().max().item() <= 2e-6 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("case", [
+    # interior tiles by the routine that is told the window: 1 to 4 random keys, windows 1 to 7
+    (1, 2, 300, 64, 1, 1, 0, 1),
+    (2, 1, 257, 128, 3, 3, 2, 2),
+    (1, 2, 300, 32, 7, 2, 4, 3),
+    (1, 1, 333, 256, 5, 1, 1, 4),
+    (1, 2, 300, 64, 7, 3, 3, 5),     # one random key more: the general routine
+    (1, 1, 300, 64, 9, 1, 3, 4),     # a wider window: the general routine
+])
+def test_sparse_attention_key_counts(ops, dt, case):
+    test_sparse_attention_matches_oracle(ops, dt, False, case)
