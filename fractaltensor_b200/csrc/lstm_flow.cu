@@ -157,7 +157,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   a.hs = hs;
   a.c_out = c;
   a.c_rows = N;
-  a.below = 1;
+  a.nb_below = plan.nb;
   a.flags = flags;
   a.status = status;
   const uint32_t nb = plan.nb, planes = 128 / plan.nb;

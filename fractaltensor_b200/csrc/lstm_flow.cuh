@@ -20,7 +20,7 @@ constexpr uint32_t kMaxSmem = 226 * 1024;
 
 template <int NB>
 struct FlowCfg {
-  static constexpr int kWarps = NB == 16 ? 4 : (NB == 32 ? 8 : 16);  // epilogue warps
+  static constexpr int kWarps = NB == 16 ? 4 : (NB == 32 ? 8 : (NB == 48 ? 12 : 16));  // epilogue warps
   static constexpr int kChunks = NB * 4 / kWarps / 16;         // of 16 columns, of a warp
   static constexpr int kRows = NB / kWarps;                // state rows a warp reads
   static constexpr int kThreads = 32 * (kFirstEpi + kWarps);
@@ -41,7 +41,7 @@ struct FlowArgs {
   float* c_out;         // [D, c_rows, H], the first N of c_rows
   int c_rows;
   int* flags;           // [D * L * S] tiles of the slice's cell (l, t) that can be read through TMA
-  int below;            // slices of this layer in one of the layer below (whose flag is that of its first)
+  int nb_below;         // sequences of a slice of the layer below
   int* status;
 };
 
@@ -257,9 +257,13 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       for (int t = 0; t < steps && ok; ++t) {
         const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + n_base;
         if (l > 0) {
-          if (lane == 0)
-            ok = flag_wait_ge(a.flags + (static_cast<int64_t>(l - 1) * a.L + t) * a.S + slice / a.below * a.below, a.n_tiles, &s_abort, status,
-                              FTB_ERR_TIMEOUT_DEP);
+          if (lane == 0) {
+            // the layer below may be cut differently: its slices that hold this one's rows
+            const int* flags = a.flags + (static_cast<int64_t>(l - 1) * a.L + t) * a.S;
+            const int last = (min(n_base + NB, a.N) - 1) / a.nb_below;
+            for (int i = n_base / a.nb_below; i <= last && ok; ++i)
+              ok = flag_wait_ge(flags + i, a.n_tiles, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
+          }
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           fence_proxy_async_all();  // threads of other CTAs stored what TMA reads

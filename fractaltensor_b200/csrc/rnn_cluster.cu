@@ -88,8 +88,7 @@ __device__ unsigned long long* g_cluster_acct = nullptr;
 struct ClusterArgs {
   int D, L, N, H;  // layers, steps of a chain (dilated: time steps; grid: B), batch, hidden size
   int A;           // grid: rows of the grid (chains per layer and slice); dilated: 1
-  int S;           // grid: batch slices of NB columns; dilated: counters per cell, one for `slot` sequences
-  int slot;        // dilated: the narrowest slice of the launch
+  int S;           // grid: batch slices of NB columns; dilated: counters per cell (the most slices of a layer)
   int CL;          // CTAs per cluster
   int max_dil;
   int dil[kMaxLayers];
@@ -216,13 +215,12 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
     } else {
       x.map = 1;
       x.row = ((layer - 1) * a.L + i) * a.N + slice * NB;
-      // One counter per `slot` sequences of a cell; a chain's CTAs count in that of its first ones.  The
-      // layer below may be cut differently: its chains that hold this slice's rows own consecutive counters.
+      // One counter per slice of a cell.  The layer below may be cut differently: its slices that hold this
+      // one's rows own consecutive counters.
       const int nbp = a.nb[layer - 1];
-      const int first = (slice * NB / nbp) * (nbp / a.slot);
+      const int first = slice * NB / nbp;
       x.flags = a.flags + ((layer - 1) * a.L + i) * a.S + first;
-      // (only the chains that exist: the last slice of the batch may be short)
-      x.nflags = nbp < NB ? min(NB / nbp, (a.N - slice * NB + nbp - 1) / nbp) : 1;
+      x.nflags = (min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
       x.target = a.CL;
     }
     if (i >= d) {
@@ -236,7 +234,7 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
         h.row = (layer * a.L + i - d) * a.N + slice * NB;
         h.nkb = kbh;
         h.wkb0 = kbh;
-        h.flags = a.flags + (layer * a.L + i - d) * a.S + slice * (NB / a.slot);
+        h.flags = a.flags + (layer * a.L + i - d) * a.S + slice;
         h.nflags = 1;
         h.target = a.CL;
       }
@@ -624,7 +622,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         *stored = i + 1;  // the tile may be overwritten (two steps from now)
         tma_store_wait<0>();
         if (MODE == kDilated)
-          red_release_gpu_add(a.flags + (my_flag_cell0 + i) * a.S + slice * (NB / a.slot), 1);
+          red_release_gpu_add(a.flags + (my_flag_cell0 + i) * a.S + slice, 1);
         else
           st_release_gpu(a.flags + ((my_flag_cell0 + i) * a.S + slice) * a.CL + rank, 1);
         ACCT_END(1);
@@ -901,27 +899,32 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
     cluster_body<T, kDilated, 128>(x128, h128, h128, h128, o128, o128, t128, t128, a, cluster_ctarank(), cid, layer, 0, slice);
 }
 
-// The same program without clusters, for batches that fit on slices of 64 beside this: what the layers with
-// dilation >= 2 exchange goes through global memory anyway (2.2 us a step on slices of 64, 3.0 on 128: a
-// layer with dilation 2 waits for the trip there and back).  A layer with dilation 1 runs as csrc/lstm_flow.cu
-// does, on slices of kNarrow sequences whose state is its own flag: 1.6 us a step at H 256 where a cluster's
-// hand-off of 64 takes 2.6, and no GPC has to hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).
+// The same program without clusters, where it fits: what the layers with dilation >= 2 exchange goes through
+// global memory anyway (2.2 us a step on slices of 64; on 128 a layer with dilation 2, which waits for the trip
+// there and back, takes 3.0).  A layer with dilation 1 runs as csrc/lstm_flow.cu does, on slices of kNarrow
+// sequences whose state is its own flag: 1.6 us a step at H 256 and 32 sequences where a cluster's hand-off of
+// 64 takes 2.6, and no GPC has to hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).
+struct DilatedMaps {
+  CUtensorMap x64, h64, o64, t64, x128, h128, o128, t128;  // as above
+  CUtensorMap nx, nh, nw;                                   // of flow::body
+};
 template <typename T, int kNarrow>
 __global__ void __launch_bounds__(cta_threads(kDilated), 1)
-rnn_dilated_flow_kernel(const __grid_constant__ CUtensorMap x, const __grid_constant__ CUtensorMap h,
-                        const __grid_constant__ CUtensorMap o, const __grid_constant__ CUtensorMap t,
-                        const __grid_constant__ CUtensorMap nx, const __grid_constant__ CUtensorMap nh,
-                        const __grid_constant__ CUtensorMap nw, const ClusterArgs a, const flow::FlowArgs f) {
+rnn_dilated_flow_kernel(const __grid_constant__ DilatedMaps m, const __grid_constant__ ClusterArgs a,
+                        const __grid_constant__ flow::FlowArgs f) {
   const int cid = blockIdx.x / a.CL, rank = blockIdx.x - cid * a.CL;
   int layer = 0;
   while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
   const int slice = cid - a.first_cluster[layer];
   if (a.dil[layer] == 1) {
     flow::FlowArgs fl = f;
-    fl.below = layer > 0 ? a.nb[layer - 1] / kNarrow : 1;
-    flow::body<T, kNarrow>(nx, nh, nw, fl, rank, slice, layer);
+    fl.nb_below = layer > 0 ? a.nb[layer - 1] : kNarrow;
+    flow::body<T, kNarrow>(m.nx, m.nh, m.nw, fl, rank, slice, layer);
+  } else if (a.nb[layer] == 64) {
+    cluster_body<T, kDilated, 64>(m.x64, m.h64, m.h64, m.h64, m.o64, m.o64, m.t64, m.t64, a, rank, cid, layer, 0, slice);
   } else {
-    cluster_body<T, kDilated, 64>(x, h, h, h, o, o, t, t, a, rank, cid, layer, 0, slice);
+    cluster_body<T, kDilated, 128>(m.x128, m.h128, m.h128, m.h128, m.o128, m.o128, m.t128, m.t128, a, rank, cid, layer, 0,
+                                   slice);
   }
 }
 
@@ -997,11 +1000,18 @@ int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_
                        m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
 }
 template <typename T, int kNarrow>
-int launch_dilated_flow(const CUtensorMap* m, const ClusterArgs& a, const flow::FlowArgs& f, int grid, uint32_t smem_bytes,
+int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs& f, int grid, uint32_t smem_bytes,
                         cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, cta_threads(kDilated), configured, grid, smem_bytes, stream,
-                       m[0], m[1], m[2], m[3], m[4], m[5], m[6], a, f);
+  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, cta_threads(kDilated), configured, grid, smem_bytes, stream, m,
+                       a, f);
+}
+template <typename T>
+int launch_dilated_flow(int narrow, const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs& f, int grid,
+                        uint32_t smem_bytes, cudaStream_t stream) {
+  if (narrow == 16) return launch_dilated_flow<T, 16>(m, a, f, grid, smem_bytes, stream);
+  if (narrow == 32) return launch_dilated_flow<T, 32>(m, a, f, grid, smem_bytes, stream);
+  return launch_dilated_flow<T, 48>(m, a, f, grid, smem_bytes, stream);
 }
 
 uint32_t smem_for(bool any_self, int H, int NB, int self_units, int out_units, int ring_self) {
@@ -1033,22 +1043,27 @@ int dilated_slices(const int* dilations, int D, int N, int max_clusters, int* nb
   return s128 <= 8 && total <= max_clusters ? total : 0;
 }
 
-// Slice width of the layers with dilation 1 when the launch goes without clusters, 0: it does not.  The
-// narrowest that leaves room for the other layers on slices of 64 (with those on slices of 128, dilations 1 to 32
-// at H 256 and 256 sequences took 1654 us, 1610 with clusters).  Clusters of 2 and 4 CTAs hand a state on fast
-// enough for batches of up to 64 (us, 3 layers of 512 steps, with clusters / without: H 64, N 24 895 / 911, N 64
-// 985 / 1105; H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above 64 sequences and at H 256
-// they lose: H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1191).
-constexpr int kFlowWide = 64;
-int dilated_flow_width(const int* dilations, int D, int N, int CL, int sm_count, int* chains) {
+// Slice widths of the layers when the launch goes without clusters, false: it does not.  Dilation 1: 16, 32 or 48;
+// the others 64, or 128 from dilation 3 on (a step's trip through global memory is hidden behind the steps
+// between); the narrowest that fit beside each other.  Clusters of 2 and 4 CTAs hand a state on fast enough for
+// batches of up to 64 (us, 3 layers of 512 steps, with clusters / without: H 64, N 24 895 / 911, N 64 985 / 1105;
+// H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above 64 sequences and at H 256 they lose:
+// H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1164, N 256 and six layers 1613 / 1330, 1654 with every layer
+// but the first on slices of 128).
+bool dilated_flow_widths(const int* dilations, int D, int N, int CL, int sm_count, int* nb) {
   int ones = 0;
   for (int l = 0; l < D; ++l) ones += dilations[l] == 1;
-  if (ones == 0 || (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64)) return 0;
-  for (int nb = 16; nb <= 32; nb *= 2) {
-    *chains = ones * ((N + nb - 1) / nb) + (D - ones) * ((N + kFlowWide - 1) / kFlowWide);
-    if (*chains * CL <= sm_count) return nb;
-  }
-  return 0;
+  if (ones == 0 || (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64)) return false;
+  for (int wide = 64; wide <= 128; wide *= 2)
+    for (int narrow = 16; narrow <= 48; narrow += 16) {
+      int ctas = 0;
+      for (int l = 0; l < D; ++l) {
+        nb[l] = dilations[l] == 1 ? narrow : (dilations[l] == 2 ? 64 : wide);
+        ctas += CL * ((N + nb[l] - 1) / nb[l]);
+      }
+      if (ctas <= sm_count) return true;
+    }
+  return false;
 }
 
 // Clusters of `cl` CTAs of the dilated kernel that can be resident at once on the current device (a
@@ -1093,7 +1108,7 @@ bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count
   return dilated_slices(nullptr, D, N, sm_count / (4 * H / 128), nullptr) > 0;
 }
 
-// one counter per (cell, slot of 16 sequences or more); at most 64 slots (8 slices of 128)
+// one counter per (cell, slice of 16 sequences or more); at most 64 (1024 sequences)
 size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 64; }
 
 // x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).
@@ -1113,27 +1128,29 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   a.W0 = Wp; a.bias0 = bias_p; a.out0 = hs; a.c = c; a.flags = flags; a.status = status;
   const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
   CUtensorMap m[8];
-  int rc, chains = 0;
-  const int narrow = dilated_flow_width(dilations, D, N, a.CL, sm_count, &chains);
-  if (narrow > 0) {
-    constexpr int wide = kFlowWide;
+  int rc;
+  if (dilated_flow_widths(dilations, D, N, a.CL, sm_count, a.nb)) {
     a.flow = true;
-    a.slot = narrow;
-    a.S = (N + wide - 1) / wide * (wide / narrow);
+    int narrow = 0;
     for (int l = 0; l < D; ++l) {
-      a.nb[l] = dilations[l] == 1 ? narrow : wide;
-      a.first_cluster[l + 1] = a.first_cluster[l] + (N + a.nb[l] - 1) / a.nb[l];
+      const int slices = (N + a.nb[l] - 1) / a.nb[l];
+      a.S = std::max(a.S, slices);
+      a.first_cluster[l + 1] = a.first_cluster[l] + slices;
+      if (dilations[l] == 1) narrow = a.nb[l];
     }
-    const int tail = N - ((N + wide - 1) / wide - 1) * wide;
-    if ((rc = make_operand_map(&m[0], x, dtype, x_rows, H, wide))) return rc;
-    if ((rc = make_operand_map(&m[1], hs, dtype, h_rows, H, wide))) return rc;
-    if ((rc = make_tmap_2d(&m[2], hs, dtype, h_rows, H, H, wide, 32, false))) return rc;
-    if ((rc = make_tmap_2d(&m[3], hs, dtype, h_rows, H, H, tail, 32, false))) return rc;
+    DilatedMaps dm;
+    for (int wide = 64; wide <= 128; wide *= 2) {
+      const int tail = N - ((N + wide - 1) / wide - 1) * wide;
+      if ((rc = make_operand_map(wide == 64 ? &dm.x64 : &dm.x128, x, dtype, x_rows, H, wide))) return rc;
+      if ((rc = make_operand_map(wide == 64 ? &dm.h64 : &dm.h128, hs, dtype, h_rows, H, wide))) return rc;
+      if ((rc = make_tmap_2d(wide == 64 ? &dm.o64 : &dm.o128, hs, dtype, h_rows, H, H, wide, 32, false))) return rc;
+      if ((rc = make_tmap_2d(wide == 64 ? &dm.t64 : &dm.t128, hs, dtype, h_rows, H, H, tail, 32, false))) return rc;
+    }
     const uint64_t row_bytes = static_cast<uint64_t>(H) * 2;
     const uint32_t planes = 128 / narrow;  // of a copy of flow::body
-    if ((rc = make_tmap_3d(&m[4], x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
-    if ((rc = make_tmap_3d(&m[5], hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
-    if ((rc = make_tmap_2d(&m[6], Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H, 2 * H, flow::kGateRows, 64))) return rc;
+    if ((rc = make_tmap_3d(&dm.nx, x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
+    if ((rc = make_tmap_3d(&dm.nh, hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
+    if ((rc = make_tmap_2d(&dm.nw, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H, 2 * H, flow::kGateRows, 64))) return rc;
     flow::FlowArgs f = {};
     f.D = D; f.L = L; f.N = N; f.I = H; f.H = H; f.G = D; f.S = a.S;
     f.n_tiles = a.CL;
@@ -1145,19 +1162,15 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     for (int l = 0; l < D; ++l)
       if (dilations[l] == 1 && cudaMemsetAsync(static_cast<char*>(hs) + l * layer_bytes, 0xFF, layer_bytes, stream) != cudaSuccess)
         return FTB_ERR_LAUNCH;
-    const uint32_t smem = smem_for(false, H, wide, 32, 32, 0);
-    const int grid = chains * a.CL;
-    if (dtype == FTB_F16)
-      return narrow == 16 ? launch_dilated_flow<__half, 16>(m, a, f, grid, smem, stream)
-                          : launch_dilated_flow<__half, 32>(m, a, f, grid, smem, stream);
-    return narrow == 16 ? launch_dilated_flow<__nv_bfloat16, 16>(m, a, f, grid, smem, stream)
-                        : launch_dilated_flow<__nv_bfloat16, 32>(m, a, f, grid, smem, stream);
+    const uint32_t smem = smem_for(false, H, 128, 32, 32, 0);
+    const int grid = a.first_cluster[D] * a.CL;
+    if (dtype == FTB_F16) return launch_dilated_flow<__half>(narrow, dm, a, f, grid, smem, stream);
+    return launch_dilated_flow<__nv_bfloat16>(narrow, dm, a, f, grid, smem, stream);
   }
   const uint32_t smem = smem_for(any_self, H, 128, 32, 32, 4);
   const int clusters = dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, smem), a.nb);
   if (clusters <= 0) return FTB_ERR_LAUNCH;  // does not fit on this device: the caller's generic wavefront takes it
-  a.S = 2 * ((N + 127) / 128);
-  a.slot = 64;
+  a.S = (N + 63) / 64;
   for (int l = 0; l < D; ++l) a.first_cluster[l + 1] = a.first_cluster[l] + (N + a.nb[l] - 1) / a.nb[l];
   if ((rc = make_operand_map(&m[0], x, dtype, x_rows, H, 128))) return rc;
   if ((rc = make_operand_map(&m[1], hs, dtype, h_rows, H, 128))) return rc;

@@ -1,0 +1,40 @@
+"""Dilated LSTM without clusters (csrc/rnn_cluster.cu): layers of dilation 1 on slices of 16, 32 or 48 sequences
+that hand their state on through the output array, the others on slices of 64 or 128; bit for bit the
+result of one launch per level."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from fractaltensor_b200 import ops as _ops
+    return _ops
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("L,N,H,dils", [
+    (9, 17, 256, [1]),                       # 16 wide, one sequence in the second slice
+    (12, 128, 256, [1, 2, 4]),               # 16 beside 64
+    (13, 256, 256, [1, 2, 4]),               # 32 beside 64
+    (40, 256, 256, [1, 2, 4, 8, 16, 32]),    # 48 beside 64 and 128: slices that straddle those below
+    (11, 200, 256, [4, 1, 2, 8, 3, 5]),      # the same with the narrow layer on top of a wide one
+    (10, 300, 128, [2, 1, 1, 4]),            # two narrow layers
+    (7, 90, 64, [1, 2]),
+])
+def test_same_bits_as_levels(ops, dt, L, N, H, dils):
+    D = len(dils)
+    g = torch.Generator(device="cuda").manual_seed(N + L)
+    u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+    Wp, b = ops.lstm_pack_weights(u(D, 4, H, H), u(D, 4, H, H), u(D, 4, H))
+    x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
+    ref, ref_c = ops.lstm_dilated(x, Wp, dils, b, schedule=1)
+    for _ in range(3):
+        h, c = ops.lstm_dilated(x, Wp, dils, b)
+        ops.check_status()
+        assert torch.equal(h, ref)
+        for l, d in enumerate(dils):
+            rows = min(d, L) * N
+            cl, rl = c.view(D, -1, H)[l], ref_c.view(D, -1, H)[l]
+            assert torch.equal(cl[:rows], rl[:rows])
