@@ -41,7 +41,9 @@ SIGNATURES = {
     "ftb_flash_attn_local_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_rnn_pack_weights": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "ftb_rnn_attention_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "ftb_rnn_attention_scratch_bytes": (_sz, [_i, _i, _i, _i]),
     "ftb_rnn_attention_fwd": (_i, [_vp] * 13 + [_i, _i, _i, _i, _i, _vp, _sz, _vp]),
+    "ftb_rnn_attention_fwd_scratch": (_i, [_vp] * 13 + [_i, _i, _i, _i, _i, _vp, _sz, _vp, _sz, _vp]),
     "ftb_sparse_attn_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp]),
     "ftb_embedding_gather": (_i, [_vp, _vp, _vp, ctypes.c_longlong, ctypes.c_longlong, _i, _i, _vp, _sz, _vp]),
     "ftb_online_softmax": (_i, [_vp, _vp, _i, _i, _vp]),

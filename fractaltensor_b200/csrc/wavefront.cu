@@ -1183,23 +1183,39 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
 // longer source is scanned in pieces).
 static constexpr size_t kMaxPreBytes = 32u << 20;
 
-size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype) {
-  if (Ls <= 0 || N <= 0 || H <= 0 || !rnn_chain_supported(dtype, H)) return kWorkspaceBytes;
+size_t ftb_rnn_attention_scratch_bytes(int Ls, int N, int H, int dtype) {
+  if (Ls <= 0 || N <= 0 || H <= 0 || !rnn_chain_supported(dtype, H)) return 0;
   const size_t step = static_cast<size_t>(N) * H * sizeof(float);
-  return kWorkspaceBytes + std::min<size_t>(Ls, kMaxPreBytes / step) * step;
+  return std::min<size_t>(Ls, kMaxPreBytes / step) * step;
+}
+
+size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype) {
+  return kWorkspaceBytes + ftb_rnn_attention_scratch_bytes(Ls, N, H, dtype);
 }
 
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
-                          int N, int H, int dtype, void* workspace, size_t workspace_bytes, void* stream_) {
+                          int N, int H, int dtype, void* workspace, size_t workspace_bytes, void* stream) {
+  const bool room = workspace != nullptr && workspace_bytes > kWorkspaceBytes;
+  return ftb_rnn_attention_fwd_scratch(src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc_proj, dec_proj, src_lens, enc,
+                                       enc_scores, dec, out, Ls, Lt, N, H, dtype,
+                                       room ? static_cast<char*>(workspace) + kWorkspaceBytes : nullptr,
+                                       room ? workspace_bytes - kWorkspaceBytes : 0, workspace, workspace_bytes, stream);
+}
+
+int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
+                                  const float* bias_src, const float* bias_trg, const void* enc_proj,
+                                  const void* dec_proj, const int* src_lens, void* enc, float* enc_scores, void* dec,
+                                  void* out, int Ls, int Lt, int N, int H, int dtype, void* scratch,
+                                  size_t scratch_bytes, void* workspace, size_t workspace_bytes, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!src || !trg || !Wp_src || !Wp_trg || !enc_proj || !dec_proj || !enc || !enc_scores || !dec || !out)
     return FTB_ERR_ARG;
   if (Ls <= 0 || Lt <= 0 || N <= 0 || H <= 0 || H % 64 != 0 || !valid_dtype(dtype)) return FTB_ERR_ARG;
   if (Ls > rnn_attention_max_src_len()) return FTB_ERR_ARG;
   if (static_cast<int64_t>(std::max(Ls, Lt)) * N > 0x7fffffffLL) return FTB_ERR_ARG;
-  if (!aligned16({src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc, dec, out})) return FTB_ERR_ALIGN;
+  if (!aligned16({src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc, dec, out, scratch})) return FTB_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(enc_scores) & 3) != 0 || (reinterpret_cast<uintptr_t>(src_lens) & 3) != 0)
     return FTB_ERR_ALIGN;
   int* status = nullptr;
@@ -1248,14 +1264,14 @@ int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, 
 
   std::vector<CellItem> items(1);
   // Encoder: e_j = tanh(x_j W + e_{j-1} U + b).  With room for the fp32 input halves x_j W of at least
-  // one step in the workspace: those as one product, then the scan as one launch of the chain kernel
+  // one step in the scratch: those as one product, then the scan as one launch of the chain kernel
   // (csrc/rnn_chain.cu), piece by piece; else one level per source position.
   const size_t pre_step = static_cast<size_t>(N) * H * sizeof(float);
-  const int piece = rnn_chain_supported(dtype, H)
-                        ? static_cast<int>(std::min<size_t>(Ls, (workspace_bytes - kWorkspaceBytes) / pre_step)) : 0;
+  const int piece = rnn_chain_supported(dtype, H) && scratch != nullptr
+                        ? static_cast<int>(std::min<size_t>(Ls, scratch_bytes / pre_step)) : 0;
   for (int j = 0; j < Ls && piece > 0; j += piece) {
     const int steps = std::min(piece, Ls - j);
-    float* pre = reinterpret_cast<float*>(static_cast<char*>(workspace) + kWorkspaceBytes);
+    float* pre = static_cast<float*>(scratch);
     CellLauncher gemm = cl;
     gemm.epi = EPI_STORE_F32;
     items[0] = blank_item();

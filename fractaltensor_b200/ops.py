@@ -407,13 +407,17 @@ def rnn_attention(src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc_proj, dec_pr
     dec = torch.empty_like(trg)
     out = torch.empty_like(trg)
     scores = torch.empty(Ls, N, dtype=torch.float32, device=src.device)
-    ws = workspace(src.device, lib.ftb_rnn_attention_workspace_bytes(Ls, N, H, _dtype_code(src)))
+    # operands of the call's own, not of the workspace, which calls on other streams use at the same time
+    scratch = torch.empty(lib.ftb_rnn_attention_scratch_bytes(Ls, N, H, _dtype_code(src)), dtype=torch.uint8,
+                          device=src.device)
+    ws = workspace(src.device)
     opt = lambda t: _ptr(t) if t is not None else None
     with torch.cuda.device(src.device):
-        check(lib.ftb_rnn_attention_fwd(_ptr(src), _ptr(trg), _ptr(Wp_src), _ptr(Wp_trg), opt(bias_src), opt(bias_trg),
-                                        _ptr(enc_proj), _ptr(dec_proj), opt(src_lens), _ptr(enc), _ptr(scores),
-                                        _ptr(dec), _ptr(out), Ls, Lt, N, H, _dtype_code(src), _ptr(ws), ws.numel(),
-                                        _stream()), "ftb_rnn_attention_fwd")
+        check(lib.ftb_rnn_attention_fwd_scratch(_ptr(src), _ptr(trg), _ptr(Wp_src), _ptr(Wp_trg), opt(bias_src),
+                                                opt(bias_trg), _ptr(enc_proj), _ptr(dec_proj), opt(src_lens), _ptr(enc),
+                                                _ptr(scores), _ptr(dec), _ptr(out), Ls, Lt, N, H, _dtype_code(src),
+                                                _ptr(scratch), scratch.numel(), _ptr(ws), ws.numel(), _stream()),
+              "ftb_rnn_attention_fwd_scratch")
     return enc, out
 
 

@@ -268,12 +268,22 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * The decoder's term is the same for every score of a step and leaves the softmax as it is, so the
  * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.
  * With workspace_bytes >= ftb_rnn_attention_workspace_bytes() (16-bit types, H <= 512) the encoder is one
- * matrix product and one scan kernel; else one launch per source position.  Four launches for the rest. */
+ * matrix product and one scan kernel; else one launch per source position.  Four launches for the rest.
+ * The product's result lies in the workspace behind the status word while the call runs.
+ * ftb_rnn_attention_fwd_scratch takes it in a buffer of its own instead (ftb_rnn_attention_scratch_bytes, 0:
+ * none needed; scratch may be NULL), so that a workspace shared by calls on several streams holds the
+ * status word only. */
 size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype);
+size_t ftb_rnn_attention_scratch_bytes(int Ls, int N, int H, int dtype);
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
                           int N, int H, int dtype, void* workspace, size_t workspace_bytes, void* stream);
+int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
+                                  const float* bias_src, const float* bias_trg, const void* enc_proj,
+                                  const void* dec_proj, const int* src_lens, void* enc, float* enc_scores, void* dec,
+                                  void* out, int Ls, int Lt, int N, int H, int dtype, void* scratch,
+                                  size_t scratch_bytes, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Embedding lookup out[t, :] = table[ids[t], :] for t < T.  Stands in for the lookup in front of
  * the reference's RNN examples, ops.index(ops.slices(embedding, dim=0), word) mapped over a batch
