@@ -196,7 +196,11 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
         p[n] = has_unit && n < n_mine ? __ldg(pre + i * step_elems + static_cast<size_t>(n) * a.H) : 0.f;
     };
     load_pre(0);
-    for (int i = 0; i < a.steps; ++i) {
+    // Warps without units (the upper half of the last CTA when H is an odd multiple of 64) are done: nobody waits
+    // for anything of theirs, so that nothing would keep acc_full, which is followed by parity, from running two
+    // phases ahead of them.  A warp with units is at most one behind: the next MMAs need what it sends.
+    const int steps = has_unit ? a.steps : 0;
+    for (int i = 0; i < steps; ++i) {
       float v[8];
       if (i > 0 || a.before != nullptr) {
         // accumulator i & 1 completes once every two steps; the first of a scan from zeros has none
@@ -218,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
 #pragma unroll
       for (int n = 0; n < 4; ++n)
         h[n] = Fmt<T>::pack2(tanh_fast(p[2 * n] + v[2 * n] + bias), tanh_fast(p[2 * n + 1] + v[2 * n + 1] + bias));
-      if (has_unit && i + 1 < a.steps) {
+      if (i + 1 < steps) {
         const uint32_t dst = my_chunk + (i & 1) * slot_bytes, bar = smem_u32(&full[i & 1][rank]);
         for (int k = 0; k < a.CL; ++k) {
           int r = rank + k;
@@ -226,13 +230,11 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
           st_async16(map_to_cta(dst, r), map_to_cta(bar, r), h);
         }
       }
-      if (i + 1 < a.steps) load_pre(i + 1);
-      if (has_unit) {
+      if (i + 1 < steps) load_pre(i + 1);
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
-          const uint16_t bits = static_cast<uint16_t>(h[n >> 1] >> (16 * (n & 1)));
-          if (n < n_mine) *reinterpret_cast<uint16_t*>(out + i * step_elems + static_cast<size_t>(n) * a.H) = bits;
-        }
+      for (int n = 0; n < 8; ++n) {
+        const uint16_t bits = static_cast<uint16_t>(h[n >> 1] >> (16 * (n & 1)));
+        if (n < n_mine) *reinterpret_cast<uint16_t*>(out + i * step_elems + static_cast<size_t>(n) * a.H) = bits;
       }
     }
   }

@@ -53,3 +53,24 @@ def test_chain_matches_levels_and_fp64(dt, H, N, Ls):
         h = torch.tanh(x[t].double() @ W.double() + h @ U.double() + bias.double())
         assert (whole[t].double() - h).abs().max().item() <= tol
         assert (levels[t].double() - h).abs().max().item() <= tol
+
+
+@pytest.mark.parametrize("H", [64, 192, 320, 448])  # odd multiples of 64: half of the last CTA's warps have no units
+def test_long_scans_with_warps_without_units(H):
+    """Those warps take no part in the steps: a scan of many steps ends with status 0 and the states of the
+    level launches' arithmetic."""
+    from fractaltensor_b200 import ops
+    from fractaltensor_b200._lib import lib
+    N, Ls, dt = 40, 400, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(H)
+    u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+    W, U, bias, proj = u(H, H), u(H, H), u(H).float(), u(H)
+    x, y = (torch.randn(n, N, H, device="cuda", generator=g).to(dt) for n in (Ls, 2))
+    Wp = ops.rnn_pack_weights(W, U)
+    tol = 4 * (2.0 ** -11 + 2.0 ** -12)  # as above
+    for _ in range(5):
+        enc, _out = _run(ops, lib, x, y, Wp, bias, proj, Ls)
+    h = torch.zeros(N, H, dtype=torch.float64, device="cuda")
+    for t in range(Ls):
+        h = torch.tanh(x[t].double() @ W.double() + h @ U.double() + bias.double())
+        assert (enc[t].double() - h).abs().max().item() <= tol
