@@ -41,6 +41,13 @@ constexpr uint32_t kCoreK = 128 * (kNB / 8);  // bytes of 8 units x 16 sequences
 // tensor memory, and two clusters holding one SM each of a pair would wait for each other.
 constexpr uint32_t kSmemBytes = 120 * 1024;
 
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -65,6 +72,7 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
   __shared__ uint64_t first_full;         // the state before the first step is in slot 1
   __shared__ uint64_t w_full;             // U is in tensor memory
   __shared__ uint64_t acc_full[2];
+  __shared__ uint64_t acc_ready[2];       // the step's input half is in the accumulator
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort;
 
@@ -74,11 +82,17 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
   uint8_t* slots = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   const uint32_t slot_bytes = static_cast<uint32_t>(a.H / 8) * kCoreK;
   int* status = a.status;
+  // Without a state before the first step that step multiplies nothing; accumulators 1 and 0 then begin with
+  // steps 1 and 2.  Which use of its accumulator a step is (parity waits):
+  const bool from_zero = a.before == nullptr;
+  auto use_of = [&](int i) { return from_zero ? ((i - 1 - ((i + 1) & 1)) >> 1) : (i >> 1); };
 
   if (threadIdx.x == 0) {
+    const int unit_warps = min(128, a.H - 128 * rank) / 32 * (kNB / 8);
     for (int s = 0; s < 2; ++s) {
       for (int r = 0; r < kMaxCtas; ++r) mbar_init(&full[s][r], 1);
       mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_ready[s], unit_warps);
     }
     mbar_init(&first_full, kEpiWarps);
     mbar_init(&w_full, kEpiWarps);
@@ -111,35 +125,34 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
     bdesc0 |= static_cast<uint64_t>(128u >> 4) << 32;
     bool ok = mbar_wait_warp(&w_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
     tc_fence_after();
-    for (int i = a.before == nullptr ? 1 : 0; i < a.steps; ++i) {
+    for (int i = from_zero ? 1 : 0; i < a.steps; ++i) {
       const int slot = (i + 1) & 1;  // of the step before
       const uint32_t d_tmem = tmem_base + (i & 1) * kAccCols;
+      ok = ok && mbar_wait(&acc_ready[i & 1], use_of(i) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
       if (i == 0) {
         ok = ok && mbar_wait(&first_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
       } else if (lane < a.CL) {
         mbar_arrive_expect_tx(&full[slot][lane], static_cast<uint32_t>(min(128, a.H - 128 * lane)) * kNB * 2);
       }
-      for (int k = 0; k < a.CL; ++k) {
-        int r = rank + k;
-        if (r >= a.CL) r -= a.CL;
+      for (int r = 0; r < a.CL; ++r) {
         if (i > 0) {
           ok = ok && mbar_wait_cluster(&full[slot][r], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
           fence_proxy_async_smem();  // the state was stored by threads, the MMA reads it by the async proxy
         }
         if (!__all_sync(0xffffffffu, ok)) break;
-        if (k == 0) tc_fence_after();
+        if (r == 0) tc_fence_after();
         const uint64_t bd = bdesc0 + static_cast<uint64_t>((slot * slot_bytes + r * 16 * kCoreK) >> 4);
         const uint32_t aw = tmem_w + r * 64;
         if (128 * r + 128 <= a.H) {
           if (leader) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              umma_ts(d_tmem, aw + 8 * j, bd + j * ((2 * kCoreK) >> 4), idesc, k > 0 || j > 0);
+              umma_ts(d_tmem, aw + 8 * j, bd + j * ((2 * kCoreK) >> 4), idesc, 1u);
           }
         } else if (leader) {  // the last CTA of an H that is not a multiple of 128 has 64 units
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_ts(d_tmem, aw + 8 * j, bd + j * ((2 * kCoreK) >> 4), idesc, k > 0 || j > 0);
+            umma_ts(d_tmem, aw + 8 * j, bd + j * ((2 * kCoreK) >> 4), idesc, 1u);
         }
       }
       if (!__all_sync(0xffffffffu, ok)) break;
@@ -195,33 +208,50 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
       for (int n = 0; n < 8; ++n)
         p[n] = has_unit && n < n_mine ? __ldg(pre + i * step_elems + static_cast<size_t>(n) * a.H) : 0.f;
     };
-    load_pre(0);
     // Warps without units (the upper half of the last CTA when H is an odd multiple of 64) are done: nobody waits
     // for anything of theirs, so that nothing would keep acc_full, which is followed by parity, from running two
     // phases ahead of them.  A warp with units is at most one behind: the next MMAs need what it sends.
     const int steps = has_unit ? a.steps : 0;
+    const uint32_t my_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 8;
+    // The input half of step i, which p holds, into the accumulator that the step's MMAs add to.
+    auto begin_acc = [&](int i) {
+      tmem_st8(my_acc + (i & 1) * kAccCols, p);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_ready[i & 1]);
+    };
+    float v[8];
+    if (steps > 0) {
+      load_pre(0);
+      if (from_zero) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) v[n] = p[n];
+      } else {
+        begin_acc(0);
+      }
+      if (steps > 1) {
+        load_pre(1);
+        begin_acc(1);
+      }
+      if (steps > 2) load_pre(2);
+    }
     for (int i = 0; i < steps; ++i) {
-      float v[8];
-      if (i > 0 || a.before != nullptr) {
-        // accumulator i & 1 completes once every two steps; the first of a scan from zeros has none
-        const int use = a.before != nullptr ? (i >> 1) : ((i - 1 - ((i + 1) & 1)) >> 1);
-        const bool ok = mbar_wait(&acc_full[i & 1], use & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
+      if (i > 0 || !from_zero) {
+        const bool ok = mbar_wait(&acc_full[i & 1], use_of(i) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
         uint32_t r[8];
-        tmem_ld8(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (i & 1) * kAccCols + half * 8, r);
+        tmem_ld8(my_acc + (i & 1) * kAccCols, r);
         tmem_ld_wait();
         tc_fence_before();
 #pragma unroll
         for (int n = 0; n < 8; ++n) v[n] = __uint_as_float(r[n]);
-      } else {
-#pragma unroll
-        for (int n = 0; n < 8; ++n) v[n] = 0.f;
       }
       uint32_t h[4];
 #pragma unroll
       for (int n = 0; n < 4; ++n)
-        h[n] = Fmt<T>::pack2(tanh_fast(p[2 * n] + v[2 * n] + bias), tanh_fast(p[2 * n + 1] + v[2 * n + 1] + bias));
+        h[n] = Fmt<T>::pack2(tanh_fast(v[2 * n] + bias), tanh_fast(v[2 * n + 1] + bias));
       if (i + 1 < steps) {
         const uint32_t dst = my_chunk + (i & 1) * slot_bytes, bar = smem_u32(&full[i & 1][rank]);
         for (int k = 0; k < a.CL; ++k) {
@@ -230,7 +260,10 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
           st_async16(map_to_cta(dst, r), map_to_cta(bar, r), h);
         }
       }
-      if (i + 1 < steps) load_pre(i + 1);
+      if (i + 2 < steps) {
+        begin_acc(i + 2);  // (the accumulator just read)
+        if (i + 3 < steps) load_pre(i + 3);
+      }
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
         const uint16_t bits = static_cast<uint16_t>(h[n >> 1] >> (16 * (n & 1)));

@@ -74,3 +74,20 @@ def test_long_scans_with_warps_without_units(H):
     for t in range(Ls):
         h = torch.tanh(x[t].double() @ W.double() + h @ U.double() + bias.double())
         assert (enc[t].double() - h).abs().max().item() <= tol
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H,N,Ls", [(64, 16, 6), (192, 17, 9), (320, 5, 3), (512, 33, 40), (256, 3, 1), (384, 50, 2)])
+def test_chain_has_the_bits_of_the_level_launches(dt, H, N, Ls):
+    """The scan adds the state's products to the input half in the order of the cell kernel, so that a call's
+    result does not depend on how much scratch it had, whole or in pieces of any length."""
+    from fractaltensor_b200 import ops
+    from fractaltensor_b200._lib import lib
+    g = torch.Generator(device="cuda").manual_seed(H + Ls)
+    u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+    x, y = (torch.randn(n, N, H, device="cuda", generator=g).to(dt) for n in (Ls, 3))
+    Wp, bias, proj = ops.rnn_pack_weights(u(H, H), u(H, H)), u(H).float(), u(H)
+    levels, out = _run(ops, lib, x, y, Wp, bias, proj, 0)
+    for pieces in sorted({1, 2, 3, Ls}):
+        enc, o = _run(ops, lib, x, y, Wp, bias, proj, min(pieces, Ls))
+        assert torch.equal(enc, levels) and torch.equal(o, out)
