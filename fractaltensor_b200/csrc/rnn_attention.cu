@@ -13,7 +13,9 @@
 // its scores move by one number: v_t is the softmax-weighted sum over e_j @ encoder_proj alone.  So
 // the recurrent input of every decoder cell is known as soon as the encoder is done, and the
 // decoder, a chain of Lt cells and Lt attention steps as written, runs as one matrix product over all
-// steps followed by one launch of the attention over all steps (ftb_rnn_attention_fwd).
+// steps followed by one launch of the attention over all steps (ftb_rnn_attention_fwd).  Only a number that
+// is not finite does not cancel: it makes every weight of its step NaN, and in the chain every later step
+// of the sequence.  carry_nan_kernel, one warp a sequence behind the attention, does that (2 us of the call).
 //
 // Layout: time-major padded batches, row (j, n) of `enc` at (j * N + n) * H.  Sequence n attends to
 // encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: per
@@ -30,6 +32,7 @@ namespace ftb {
 namespace {
 
 constexpr int kStepThreads = 128;  // one output column per thread
+constexpr int kCarryThreads = 128;
 
 template <typename T> __device__ __forceinline__ float ld_f32(const T* p);
 template <> __device__ __forceinline__ float ld_f32<float>(const float* p) { return __ldg(p); }
@@ -148,6 +151,42 @@ attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores
   for (int k = 0; k < copies; ++k) st_f32<T>(o + k * step_elems, acc * inv);
 }
 
+// Where step t of a sequence has NaN for its vector, so have the steps behind it and their decoder states.
+// (Encoder states are at most 1 and weights too: a vector is finite or NaN, and NaN weights make all of its
+// columns NaN.  A NaN encoder state alone is in every step's vector already.)
+template <typename T>
+__global__ void __launch_bounds__(kCarryThreads)
+carry_nan_kernel(T* __restrict__ dec, T* __restrict__ out, int Lt, int N, int H) {
+  const int n = blockIdx.x * (kCarryThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (n >= N) return;
+  const long long step_elems = static_cast<long long>(N) * H, row = static_cast<long long>(n) * H;
+  int first = Lt;
+  for (int t0 = 0; t0 < Lt && first == Lt; t0 += 32) {
+    const int t = t0 + lane;
+    const bool bad = t < Lt && isnan(ld_f32<T>(out + t * step_elems + row));
+    const unsigned who = __ballot_sync(0xffffffffu, bad);
+    if (who != 0) first = t0 + __ffs(who) - 1;
+  }
+  const float nan = __int_as_float(0x7FFFFFFF);
+  for (int t = first + 1; t < Lt; ++t)
+    for (int h = lane; h < H; h += 32) {
+      st_f32<T>(dec + t * step_elems + row + h, nan);
+      st_f32<T>(out + t * step_elems + row + h, nan);
+    }
+}
+
+template <typename T>
+int carry_nan_t(void* dec, void* out, int Lt, int N, int H, cudaStream_t stream) {
+  constexpr int kRows = kCarryThreads / 32;
+  const cudaError_t err = launch_light(carry_nan_kernel<T>, dim3((N + kRows - 1) / kRows), dim3(kCarryThreads), 0, stream,
+                                       static_cast<T*>(dec), static_cast<T*>(out), Lt, N, H);
+  count_launch();
+  if (err != cudaSuccess) cudaGetLastError();
+  return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+}
+
 template <typename T>
 int enc_scores_t(const void* enc, const void* proj, float* scores, long long n_rows, int H, cudaStream_t stream) {
   const long long ctas = (n_rows + 7) / 8;
@@ -184,6 +223,14 @@ int launch_enc_scores(int dtype, const void* enc, const void* proj, float* score
     case FTB_F32: return enc_scores_t<float>(enc, proj, scores, n_rows, H, stream);
     case FTB_F16: return enc_scores_t<__half>(enc, proj, scores, n_rows, H, stream);
     default: return enc_scores_t<__nv_bfloat16>(enc, proj, scores, n_rows, H, stream);
+  }
+}
+
+int launch_carry_nan(int dtype, void* dec, void* out, int Lt, int N, int H, cudaStream_t stream) {
+  switch (dtype) {
+    case FTB_F32: return carry_nan_t<float>(dec, out, Lt, N, H, stream);
+    case FTB_F16: return carry_nan_t<__half>(dec, out, Lt, N, H, stream);
+    default: return carry_nan_t<__nv_bfloat16>(dec, out, Lt, N, H, stream);
   }
 }
 

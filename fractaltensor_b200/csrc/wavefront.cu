@@ -70,6 +70,7 @@ int launch_enc_scores(int dtype, const void* enc, const void* proj, float* score
                       cudaStream_t stream);
 int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
                       const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream);
+int launch_carry_nan(int dtype, void* dec, void* out, int Lt, int N, int H, cudaStream_t stream);
 bool rnn_chain_supported(int dtype, int H);
 int launch_rnn_chain(int dtype, const float* pre, const void* Wp, int ldw, int k0, const float* bias,
                      const void* before, void* out, int steps, int N, int H, int* status, cudaStream_t stream);
@@ -1302,7 +1303,8 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
   // Decoder.  The attention vector of a step does not depend on the decoder (its term moves all scores
   // of a softmax by one number), so the recurrent inputs of steps 1.. are known here: they go to the
   // rows of `out` they are read from, all decoder cells run as one level, and the attention over all
-  // steps writes the result over them.  (As a chain: two dependent launches per step.)
+  // steps writes the result over them.  (As a chain: two dependent launches per step.)  A term that is
+  // not finite is carried to the steps behind it at the end.
   if (Lt > 1) {
     rc = launch_attn_steps(dtype, enc, enc_scores, nullptr, dec_proj, src_lens, out, Lt - 1, Ls, N, H, stream);
     if (rc) return rc;
@@ -1327,7 +1329,7 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
                            static_cast<char*>(out) + at, std::min(kMostSteps, Lt - t), Ls, N, H, stream);
     if (rc) return rc;
   }
-  return FTB_OK;
+  return Lt > 1 ? launch_carry_nan(dtype, dec, out, Lt, N, H, stream) : FTB_OK;
 }
 
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {

@@ -266,9 +266,10 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * dec [Lt, N, H] decoder states, out [Lt, N, H] the attention vectors.  Rows of a sequence past its
  * own source / target length hold values nobody should read.  H % 64 == 0, Ls <= 12288.
  * The decoder's term is the same for every score of a step and leaves the softmax as it is, so the
- * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.
+ * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.  A decoder
+ * term that is not finite makes the vectors of its step and of all later steps of that sequence NaN.
  * With workspace_bytes >= ftb_rnn_attention_workspace_bytes() (16-bit types, H <= 512) the encoder is one
- * matrix product and one scan kernel; else one launch per source position.  Four launches for the rest.
+ * matrix product and one scan kernel; else one launch per source position.  Five launches for the rest.
  * The product's result lies in the workspace behind the status word while the call runs.
  * ftb_rnn_attention_fwd_scratch takes it in a buffer of its own instead (ftb_rnn_attention_scratch_bytes, 0:
  * none needed; scratch may be NULL), so that a workspace shared by calls on several streams holds the

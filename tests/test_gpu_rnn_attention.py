@@ -131,3 +131,45 @@ def test_rnn_attention_smallest_shapes(ops, dt):
         if src_lens == [1]:
             enc1 = torch.tanh(src.double() @ d64["Ws"] + d64["bs"])
             assert (out.data.reshape(-1, H).cpu().double() - enc1).abs().max().item() <= (1e-5 if dt == torch.float32 else 2e-2)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Lt", [2, 40])
+def test_what_is_not_finite_reaches_the_later_steps(ops, dt, Lt):
+    """A decoder state that is not finite makes its step's weights NaN, and by the recurrent input every later
+    step of that sequence; the others and the steps before keep their values."""
+    Ls, N, H = 7, 9, 64
+    p, g = _params(H, 5, 1.0 / 8)
+    q = {k: v.to(dt).cuda() for k, v in p.items()}
+    src, trg = (torch.randn(n, N, H, generator=g).to(dt).cuda() for n in (Ls, Lt))
+    lens = torch.tensor([7, 3, 5, 7, 1, 2, 6, 0, 4], dtype=torch.int32, device="cuda")
+    clean = trg.clone()
+    trg[0, 1, 3] = float("nan")            # from the first step on
+    trg[Lt - 1, 2, 0] = float("nan")       # the last step alone
+    trg[Lt // 2, 4, :2] = float("inf")     # inf - inf in some units, where their weights differ in sign
+    trg[Lt // 2, 7, 5] = float("nan")      # a sequence that attends to nothing
+    src[2, 5, 0] = float("nan")            # past that sequence's length
+    call = lambda t: ops.rnn_attention(src, t, ops.rnn_pack_weights(q["Ws"], q["Us"]),
+                                       ops.rnn_pack_weights(q["Wt"], q["Ut"]), q["bs"].float().reshape(-1),
+                                       q["bt"].float().reshape(-1), q["enc_proj"].reshape(-1), q["dec_proj"].reshape(-1),
+                                       lens)[1]
+    out, finite = call(trg), call(clean)
+    ops.check_status()
+    d = {k: v.double() for k, v in q.items()}
+    h, enc = torch.zeros(N, H, dtype=torch.float64, device="cuda"), []
+    for t in range(Ls):
+        h = torch.tanh(src[t].double() @ d["Ws"] + h @ d["Us"] + d["bs"])
+        enc.append(h)
+    enc = torch.stack(enc)
+    keys = (torch.arange(Ls, device="cuda")[:, None] < lens[None]).unsqueeze(-1)
+    enc = torch.where(keys, enc, torch.zeros_like(enc))
+    s0 = torch.where(keys[..., 0], (enc @ d["enc_proj"])[..., 0], torch.full((Ls, N), -np.inf, device="cuda").double())
+    v, bad = torch.zeros(N, H, dtype=torch.float64, device="cuda"), []
+    for t in range(Lt):
+        dec = torch.tanh(trg[t].double() @ d["Wt"] + v @ d["Ut"] + d["bt"])
+        w = torch.softmax(s0 + (dec @ d["dec_proj"])[:, 0], 0)
+        v = (torch.where(keys, w.unsqueeze(-1) * enc, torch.zeros_like(enc))).sum(0)
+        bad.append(torch.isnan(v))
+    bad = torch.stack(bad)
+    assert torch.equal(torch.isnan(out), bad) and bad.any() and not bad.all()
+    assert torch.equal(out[~bad], finite[~bad])
