@@ -54,33 +54,46 @@ bool get_float(PyObject* o, float* v) {
   return true;
 }
 
-// The workspace ops.py keeps for `dev` in its dictionary {device index: uint8 tensor}; nullptr when
-// there is none yet or it is smaller than `bytes`.
-const at::Tensor* workspace_of(PyObject* dict, c10::DeviceIndex dev, size_t bytes) {
+// The workspace ops.py keeps for `dev` in its dictionary {device index: uint8 tensor}; undefined when
+// there is none yet or it is smaller than `bytes`.  (Held by value: another thread may put a larger one
+// in its place while this call runs.)
+at::Tensor workspace_of(PyObject* dict, c10::DeviceIndex dev, size_t bytes) {
   PyObject* key = PyLong_FromLong(dev);
-  if (key == nullptr) return nullptr;
-  PyObject* t = PyDict_Check(dict) ? PyDict_GetItemWithError(dict, key) : nullptr;
-  Py_DECREF(key);
+  PyObject* t = key != nullptr && PyDict_Check(dict) ? PyDict_GetItemWithError(dict, key) : nullptr;
+  Py_XDECREF(key);
   if (t == nullptr) {
     PyErr_Clear();
-    return nullptr;
+    return at::Tensor();
   }
   const at::Tensor* ws = cuda_tensor(t);
-  return ws != nullptr && static_cast<size_t>(ws->numel()) >= bytes ? ws : nullptr;
+  return ws != nullptr && static_cast<size_t>(ws->numel()) >= bytes ? *ws : at::Tensor();
 }
+
+// What follows runs without the GIL: allocating may free memory and wait, and a launch waits while the
+// stream's queue is full.  Other Python threads go on meanwhile, as they do around a ctypes call.
+class WithoutGil {
+ public:
+  WithoutGil() : state_(PyEval_SaveThread()) {}
+  ~WithoutGil() { PyEval_RestoreThread(state_); }
+  WithoutGil(const WithoutGil&) = delete;
+  WithoutGil& operator=(const WithoutGil&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
 
 void* stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
 
-// `out` if the caller gave one that fits, else a new tensor; false when the given one does not fit.
-bool result(PyObject* out, const at::Tensor& like, at::IntArrayRef shape, at::Tensor* o) {
-  if (out == Py_None) {
-    *o = at::empty(shape, at::TensorOptions().dtype(like.scalar_type()).device(like.device()));
-    return true;
-  }
+// *o: `out` if the caller gave one, undefined for None; false when the given one does not fit.
+bool given_result(PyObject* out, const at::Tensor& like, at::IntArrayRef shape, at::Tensor* o) {
+  if (out == Py_None) return true;
   const at::Tensor* t = cuda_tensor(out);
   if (t == nullptr || !same_kind(*t, like) || t->sizes() != shape) return false;
   *o = *t;
   return true;
+}
+at::Tensor new_result(const at::Tensor& like, at::IntArrayRef shape) {
+  return at::empty(shape, at::TensorOptions().dtype(like.scalar_type()).device(like.device()));
 }
 
 #define DECLINE_UNLESS(cond) \
@@ -112,14 +125,19 @@ PyObject* b2b_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int dt = dtype_code(*A);
     DECLINE_UNLESS(dt >= 0);
     const c10::DeviceIndex dev = A->device().index();
-    const at::Tensor* ws = workspace_of(args[4], dev, ftb_workspace_bytes());
-    DECLINE_UNLESS(ws);
-    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor ws = workspace_of(args[4], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws.defined());
     at::Tensor out;
-    DECLINE_UNLESS(result(args[3], *A, {batch, M, P}, &out));
-    const int rc = ftb_b2b_gemm(A->data_ptr(), B->data_ptr(), C->data_ptr(), out.data_ptr(), static_cast<int>(batch),
-                                static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(P), dt,
-                                ws->data_ptr(), ws->numel(), stream_of(dev));
+    DECLINE_UNLESS(given_result(args[3], *A, {batch, M, P}, &out));
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::cuda::CUDAGuard guard(dev);
+      if (!out.defined()) out = new_result(*A, {batch, M, P});
+      rc = ftb_b2b_gemm(A->data_ptr(), B->data_ptr(), C->data_ptr(), out.data_ptr(), static_cast<int>(batch),
+                        static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(P), dt,
+                        ws.data_ptr(), ws.numel(), stream_of(dev));
+    }
     DECLINE_UNLESS(rc == 0);
     return THPVariable_Wrap(out);
   });
@@ -142,24 +160,28 @@ PyObject* flash_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
               d = static_cast<int>(q->size(3)), dt = dtype_code(*q);
     DECLINE_UNLESS(dt >= 0);
     const c10::DeviceIndex dev = q->device().index();
-    const at::Tensor* ws = workspace_of(args[8], dev, ftb_workspace_bytes());
-    DECLINE_UNLESS(ws);
-    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor ws = workspace_of(args[8], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws.defined());
     at::Tensor out;
-    DECLINE_UNLESS(result(args[3], *q, q->sizes(), &out));
-    const void *qp = q->data_ptr(), *kp = k->data_ptr(), *vp = v->data_ptr();
-    void *op = out.data_ptr(), *wp = ws->data_ptr(), *st = stream_of(dev);
-    const size_t wb = ws->numel();
+    DECLINE_UNLESS(given_result(args[3], *q, q->sizes(), &out));
     int rc;
-    switch (mode) {
-      case 0: rc = ftb_flash_attn_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
-      case 1: rc = ftb_flash_attn_causal_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
-      case 2:
-        rc = ftb_flash_attn_window_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), scale, dt, wp, wb, st);
-        break;
-      default:
-        rc = ftb_flash_attn_local_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), static_cast<int>(right),
-                                      scale, dt, wp, wb, st);
+    {
+      const WithoutGil released;
+      const c10::cuda::CUDAGuard guard(dev);
+      if (!out.defined()) out = new_result(*q, q->sizes());
+      const void *qp = q->data_ptr(), *kp = k->data_ptr(), *vp = v->data_ptr();
+      void *op = out.data_ptr(), *wp = ws.data_ptr(), *st = stream_of(dev);
+      const size_t wb = ws.numel();
+      switch (mode) {
+        case 0: rc = ftb_flash_attn_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
+        case 1: rc = ftb_flash_attn_causal_fwd(qp, kp, vp, op, B, h, S, d, scale, dt, wp, wb, st); break;
+        case 2:
+          rc = ftb_flash_attn_window_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), scale, dt, wp, wb, st);
+          break;
+        default:
+          rc = ftb_flash_attn_local_fwd(qp, kp, vp, op, B, h, S, d, static_cast<int>(left), static_cast<int>(right),
+                                        scale, dt, wp, wb, st);
+      }
     }
     DECLINE_UNLESS(rc == 0);
     return THPVariable_Wrap(out);
@@ -193,16 +215,22 @@ PyObject* sparse_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int dt = dtype_code(*q);
     DECLINE_UNLESS(dt >= 0);
     const c10::DeviceIndex dev = q->device().index();
-    const at::Tensor* ws = workspace_of(args[10], dev, ftb_workspace_bytes());
-    DECLINE_UNLESS(ws);
-    const c10::cuda::CUDAGuard guard(dev);
+    const int as_shipped = args[9] == Py_True ? 1 : 0;
+    const at::Tensor ws = workspace_of(args[10], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws.defined());
     at::Tensor out;
-    DECLINE_UNLESS(result(args[4], *q, q->sizes(), &out));
-    const int rc = ftb_sparse_attn_fwd(q->data_ptr(), k->data_ptr(), v->data_ptr(), pos, out.data_ptr(),
-                                       static_cast<int>(q->size(0)), static_cast<int>(q->size(1)), static_cast<int>(S),
-                                       static_cast<int>(q->size(3)), static_cast<int>(window), static_cast<int>(dilation),
-                                       static_cast<int>(ng), static_cast<int>(R), scale, args[9] == Py_True ? 1 : 0, dt,
-                                       ws->data_ptr(), ws->numel(), stream_of(dev));
+    DECLINE_UNLESS(given_result(args[4], *q, q->sizes(), &out));
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::cuda::CUDAGuard guard(dev);
+      if (!out.defined()) out = new_result(*q, q->sizes());
+      rc = ftb_sparse_attn_fwd(q->data_ptr(), k->data_ptr(), v->data_ptr(), pos, out.data_ptr(),
+                               static_cast<int>(q->size(0)), static_cast<int>(q->size(1)), static_cast<int>(S),
+                               static_cast<int>(q->size(3)), static_cast<int>(window), static_cast<int>(dilation),
+                               static_cast<int>(ng), static_cast<int>(R), scale, as_shipped, dt, ws.data_ptr(),
+                               ws.numel(), stream_of(dev));
+    }
     DECLINE_UNLESS(rc == 0);
     return THPVariable_Wrap(out);
   });

@@ -28,3 +28,33 @@ def test_no_room_for_the_result_is_torch_s_own_error():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert ops.b2b_gemm(A, B, C).shape == (4, 1 << 17, 64)
+
+
+def test_a_full_launch_queue_does_not_stop_other_threads():
+    """More calls than a stream's queue holds, behind 0.6 s of waiting: the thread that makes them stands still
+    until the queue moves, the other threads of the program do not."""
+    import threading
+    import time
+    from fractaltensor_b200 import ops
+    A, B, C = _b2b()
+    out = ops.b2b_gemm(A, B, C)
+    torch.cuda.synchronize()
+    took = []
+
+    def many_calls():
+        torch.cuda._sleep(int(0.6 * 1.9e9))
+        t0 = time.perf_counter()
+        for _ in range(4000):
+            ops.b2b_gemm(A, B, C, out)
+        took.append(time.perf_counter() - t0)
+
+    caller = threading.Thread(target=many_calls)
+    gap, last = 0.0, time.perf_counter()
+    caller.start()
+    while caller.is_alive():
+        time.sleep(0.002)
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+    torch.cuda.synchronize()
+    assert took[0] > 0.4  # the queue was full
+    assert gap < 0.25
