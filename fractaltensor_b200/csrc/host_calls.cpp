@@ -8,8 +8,9 @@
 // stream of the inputs' device (4..6 us per call, most of it the allocation and the launch).
 //
 // They are the accepting half only: whatever is not the plain, valid call (a wrong type or shape, a
-// tensor on the CPU, no workspace on that device yet, an error from the library) is answered with
-// None before anything is launched, and ops.py goes through its Python checks, which raise.
+// tensor on the CPU, no workspace on that device yet, no memory for the result) is answered with
+// None before the library is entered, and ops.py goes through its Python checks, which raise.  An error of
+// the library is answered with its status number: it may come after a launch, and the call is not made again.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -138,8 +139,7 @@ PyObject* b2b_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
                         static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(P), dt,
                         ws.data_ptr(), ws.numel(), stream_of(dev));
     }
-    DECLINE_UNLESS(rc == 0);
-    return THPVariable_Wrap(out);
+    return rc == 0 ? THPVariable_Wrap(out) : PyLong_FromLong(rc);
   });
 }
 
@@ -183,8 +183,7 @@ PyObject* flash_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                         scale, dt, wp, wb, st);
       }
     }
-    DECLINE_UNLESS(rc == 0);
-    return THPVariable_Wrap(out);
+    return rc == 0 ? THPVariable_Wrap(out) : PyLong_FromLong(rc);
   });
 }
 
@@ -231,8 +230,7 @@ PyObject* sparse_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                static_cast<int>(ng), static_cast<int>(R), scale, as_shipped, dt, ws.data_ptr(),
                                ws.numel(), stream_of(dev));
     }
-    DECLINE_UNLESS(rc == 0);
-    return THPVariable_Wrap(out);
+    return rc == 0 ? THPVariable_Wrap(out) : PyLong_FromLong(rc);
   });
 }
 

@@ -250,11 +250,18 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
 
 
 # ------------------------------------------------------------ B2B GEMM / attention
+def _done(result, where):
+    """The answer of the native front: the result, or the library's status number, which raises."""
+    if type(result) is int:
+        check(result, where)
+    return result
+
+
 def b2b_gemm(A, B, C, out=None):
     """A: [batch,M,K]; B: [batch,N,K]; C: [batch,P,N] -> D [batch,M,P] = (A.B^T).C^T per batch entry."""
     done = host.b2b_gemm(A, B, C, out, _workspaces)
     if done is not None:
-        return done
+        return _done(done, "ftb_b2b_gemm")
     _req(A, "A")
     _req(B, "B", A.dtype)
     _req(C, "C", A.dtype)
@@ -278,16 +285,18 @@ def flash_attention(q, k, v, scale=None, out=None, causal=False, window=None, lo
     `window` (with causal): keys i-window+1..i; `local=(left, right)`: keys i-left..i+right."""
     # the plain calls, by mask: full, causal, window, local
     sc = 1.0 if scale is None else scale
-    done = None
+    done, where = None, "ftb_flash_attn_causal_fwd" if causal else "ftb_flash_attn_fwd"
     if local is None and window is None:
         done = host.flash_attention(q, k, v, out, sc, 1 if causal else 0, 0, 0, _workspaces)
     elif local is None:
         if causal:
+            where = "ftb_flash_attn_window_fwd"
             done = host.flash_attention(q, k, v, out, sc, 2, window, 0, _workspaces)
     elif window is None and not causal:
+        where = "ftb_flash_attn_local_fwd"
         done = host.flash_attention(q, k, v, out, sc, 3, local[0], local[1], _workspaces)
     if done is not None:
-        return done
+        return _done(done, where)
     _req(q, "q")
     _req(k, "k", q.dtype)
     _req(v, "v", q.dtype)
@@ -335,7 +344,7 @@ def sparse_attention(q, k, v, rand_pos, window_size=5, dilation=2, n_global=3, s
     done = host.sparse_attention(q, k, v, rand_pos, out, window_size, dilation, n_global, scale, as_shipped,
                                  _workspaces)
     if done is not None:
-        return done
+        return _done(done, "ftb_sparse_attn_fwd")
     _req(q, "q")
     _req(k, "k", q.dtype)
     _req(v, "v", q.dtype)

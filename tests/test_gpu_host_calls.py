@@ -58,3 +58,21 @@ def test_a_full_launch_queue_does_not_stop_other_threads():
     torch.cuda.synchronize()
     assert took[0] > 0.4  # the queue was full
     assert gap < 0.25
+
+
+def test_an_error_of_the_library_is_raised_without_a_second_call(monkeypatch):
+    from fractaltensor_b200 import ops
+    from fractaltensor_b200._lib import FtbError
+    ops.b2b_gemm(*_b2b())
+    again = []
+    for name in ("ftb_b2b_gemm", "ftb_flash_attn_fwd", "ftb_flash_attn_window_fwd", "ftb_sparse_attn_fwd"):
+        monkeypatch.setattr(ops.lib, name, lambda *a, name=name: again.append(name) or 0)
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.half)
+    for where, call in (("ftb_b2b_gemm", lambda: ops.b2b_gemm(z(1, 100, 64), z(1, 128, 64), z(1, 64, 128))),
+                        ("ftb_flash_attn_fwd", lambda: ops.flash_attention(z(1, 1, 100, 128), *[z(1, 1, 100, 128)] * 2)),
+                        ("ftb_flash_attn_window_fwd", lambda: ops.flash_attention(*[z(1, 1, 256, 128)] * 3, causal=True, window=0)),
+                        ("ftb_sparse_attn_fwd", lambda: ops.sparse_attention(*[z(1, 1, 64, 48)] * 3, None))):
+        with pytest.raises(FtbError, match=where) as e:
+            call()
+        assert e.value.code == 1
+    assert again == []
