@@ -5,6 +5,7 @@ the shared object is missing, importing this module raises.
 """
 import ctypes
 import os
+import warnings
 
 import torch  # noqa: F401  (loads the libraries _host.so links against)
 
@@ -69,10 +70,35 @@ def load():
 
 lib = load()
 
-try:
-    from . import _host as host  # native front of the short calls; needs torch and libftb200.so loaded
-except ImportError as e:
-    raise ImportError("_host.so is not built (%s); run `python -m fractaltensor_b200.build`" % e)
+
+class _NoHost:
+    """Declines every short call, as the native front does with what it does not take: ops.py goes on with its
+    own checks and ctypes, to the same kernels."""
+
+    @staticmethod
+    def _decline(*args):
+        return None
+
+    b2b_gemm = flash_attention = sparse_attention = _decline
+
+
+def _load_host():
+    """The native front of the short calls.  It is built against one torch, and with another it must not be
+    used; the package works without it, at 17 us of host time a short call instead of 5."""
+    try:
+        from . import _host  # needs torch and libftb200.so loaded
+        built_for = _host.torch_version
+        if built_for == torch.__version__.split("+")[0]:
+            return _host
+        why = "built against torch %s, this is %s" % (built_for, torch.__version__)
+    except (ImportError, AttributeError) as e:
+        why = str(e)
+    warnings.warn("_host.so is not usable (%s): short calls take longer; run `python -m fractaltensor_b200.build`" % why,
+                  RuntimeWarning, stacklevel=2)
+    return _NoHost
+
+
+host = _load_host()
 
 
 class FtbError(RuntimeError):

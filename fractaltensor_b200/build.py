@@ -42,6 +42,18 @@ def _host_flags():
     return cflags, ldflags
 
 
+def _host_object():
+    """The object file of _host.so: named by the torch and the Python it is built against, so that with
+    another of either there is none yet."""
+    import torch
+    return HOST_SRC.replace(".cpp", ".%s.%s.o" % (torch.__version__, sys.implementation.cache_tag))
+
+
+def _host_is_stale(api):
+    obj = _host_object()
+    return _newer(HOST_SRC, obj) or _newer(api, obj) or _newer(obj, HOST)
+
+
 def build(verbose=False, force=False):
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
@@ -60,8 +72,8 @@ def build(verbose=False, force=False):
         if force or _newer(s, o) or any(_newer(h, o) for h in headers):
             start(src, [nvcc] + NVCC_FLAGS + ["-c", s, "-o", o])
     link_lib = bool(procs) or not os.path.exists(LIB)
-    host_obj = HOST_SRC.replace(".cpp", ".o")
-    build_host = force or _newer(HOST_SRC, HOST) or _newer(api, HOST)
+    host_obj = _host_object()
+    build_host = force or _host_is_stale(api)
     if build_host:
         cflags, ldflags = _host_flags()
         start(os.path.basename(HOST_SRC), ["g++"] + cflags + ["-c", HOST_SRC, "-o", host_obj])

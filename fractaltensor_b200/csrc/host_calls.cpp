@@ -17,6 +17,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include "../../include/ftb200.h"
 
@@ -249,4 +250,9 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Native front of the shor
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&kModule);
+  // the torch whose headers this was built against: _lib.py uses the module with that one only
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) Py_CLEAR(m);
+  return m;
+}

@@ -14,6 +14,49 @@ def test_declines_what_is_not_a_cuda_tensor():
     assert host.sparse_attention(q, q, q, None, None, 5, 2, 3, 1.0, False, {}) is None
 
 
+def _import_with(prelude):
+    """Runs `prelude` and imports the package in a process of its own -> what it printed."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = prelude + """
+import warnings
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    from fractaltensor_b200 import ops
+mine = [str(w.message) for w in seen if "_host.so" in str(w.message)]
+q = torch.zeros(1, 1, 256, 128, dtype=torch.float16)
+for call in (lambda: ops.b2b_gemm(q[0], q[0], q[0]), lambda: ops.flash_attention(q, q, q),
+             lambda: ops.sparse_attention(q, q, q, None)):
+    try:
+        call()
+        print("no error")
+    except RuntimeError as e:
+        assert "CUDA device" in str(e)
+print(len(mine), ops.host.__name__)
+"""
+    return subprocess.run([sys.executable, "-c", code], cwd=root, check=True, capture_output=True, text=True).stdout.split()
+
+
+def test_the_package_works_without_the_native_front():
+    assert _import_with("import torch, sys\nsys.modules['fractaltensor_b200._host'] = None") == ["1", "_NoHost"]
+
+
+def test_the_native_front_is_not_used_with_another_torch():
+    assert _import_with("import torch\ntorch.__version__ = '1.0.0+cpu'") == ["1", "_NoHost"]
+    assert _import_with("import torch") == ["0", "fractaltensor_b200._host"]
+
+
+def test_the_native_front_is_built_again_for_another_torch(monkeypatch):
+    import os
+    import fractaltensor_b200.build as b
+    api = os.path.join(b.HERE, "..", "include", "ftb200.h")
+    assert not b._host_is_stale(api)
+    monkeypatch.setattr(torch, "__version__", "1.0.0+cpu")
+    assert b._host_is_stale(api)
+
+
 @pytest.mark.gpu
 def test_same_errors_and_results_as_the_checked_path():
     from fractaltensor_b200 import ops
