@@ -39,12 +39,14 @@ __device__ __forceinline__ void group_barrier(int group) {
 // four groups of 128 threads (each with its own shared-memory buffers and its own named barrier),
 // every group accumulates its quarter of K in the same 32 x 32 layout, and group 0 adds the four
 // partial sums in a fixed order and runs the epilogue.
+constexpr int kSmemBytes = kSplitK * (2 * TM * (TK + 4) + TK * (TN + 4)) * sizeof(float);
+
 template <int EPI>
 __global__ void __launch_bounds__(kSimtThreads)
 cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ CellBatch batch) {
-  __shared__ __align__(16) float sA[kSplitK][TM][TK + 4];  // [group][row][k]: a thread reads four k of a row at once
-  __shared__ __align__(16) float sW[kSplitK][TK][TN + 4];  // [group][k][column]
-  __shared__ __align__(16) float sP[kSplitK - 1][kGroupThreads][8];  // partial sums of groups 1..3
+  extern __shared__ __align__(16) float smem[];
+  auto& sA = *reinterpret_cast<float(*)[kSplitK][2][TM][TK + 4]>(smem);  // [group][buffer][row][k]
+  auto& sW = *reinterpret_cast<float(*)[kSplitK][TK][TN + 4]>(smem + sizeof(sA) / sizeof(float));  // [group][k][column]
 
   // A kernel launched behind this one as a dependent (the attention step of the attention RNN) may
   // be scheduled while this one drains; this kernel itself waits for the one before it.
@@ -63,7 +65,7 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
   const int tg = threadIdx.x % kGroupThreads;   // thread within the group
   const int tx = tg & 7;   // 4 consecutive columns: one LSTM unit
   const int ty = tg >> 3;  // 2 consecutive rows
-  float acc[2][4] = {};  // sums of the chunks so far
+  uint64_t acc[2][2] = {};  // sums of the chunks so far, two columns each
 
   // K is walked in chunks of TK over the cell's segments; this group takes chunks [c_begin, c_end) of
   // the walk.  The next chunk's global loads are issued into registers before the current chunk is
@@ -74,15 +76,16 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
   const int ld_r = tg >> 3;        // first row (A) / column (W) this thread loads; second is +16
   const int ld_kq = (tg & 7) * 4;  // its four consecutive k
   const bool a_ok0 = m_tile * TM + ld_r < it.rows, a_ok1 = m_tile * TM + ld_r + 16 < it.rows;
-  float4 va0 = make_float4(0.f, 0.f, 0.f, 0.f), va1 = va0, vw0 = va0, vw1 = va0;
-  auto fetch = [&](int s, int k0) {
+  float4 vw0 = make_float4(0.f, 0.f, 0.f, 0.f), vw1 = vw0;
+  auto fetch = [&](int s, int k0, int buf) {
     const float* A = args.act[it.seg_map[s]];
     const int lda = args.ld_act[it.seg_map[s]];
     const int row0 = it.seg_row[s] + m_tile * TM;
     const float* W = args.w[it.w_map] + static_cast<size_t>(it.w_row0 + n_tile * TN) * args.ldw + it.seg_wk[s];
-    va0 = va1 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a_ok0) va0 = *reinterpret_cast<const float4*>(A + static_cast<size_t>(row0 + ld_r) * lda + k0 + ld_kq);
-    if (a_ok1) va1 = *reinterpret_cast<const float4*>(A + static_cast<size_t>(row0 + ld_r + 16) * lda + k0 + ld_kq);
+    copy16_async(&sA[grp][buf][ld_r][ld_kq], A + static_cast<size_t>(a_ok0 ? row0 + ld_r : row0) * lda + k0 + ld_kq, a_ok0);
+    copy16_async(&sA[grp][buf][ld_r + 16][ld_kq], A + static_cast<size_t>(a_ok1 ? row0 + ld_r + 16 : row0) * lda + k0 + ld_kq,
+                 a_ok1);
+    copies_commit();
     vw0 = *reinterpret_cast<const float4*>(W + static_cast<size_t>(ld_r) * args.ldw + k0 + ld_kq);
     vw1 = *reinterpret_cast<const float4*>(W + static_cast<size_t>(ld_r + 16) * args.ldw + k0 + ld_kq);
   };
@@ -96,25 +99,25 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
     }
     k0 = skip * TK;
   }
-  if (c_begin < c_end) fetch(s, k0);
+  int buf = 0;
+  if (c_begin < c_end) fetch(s, k0, 0);
   for (int c = c_begin; c < c_end; ++c) {
-    *reinterpret_cast<float4*>(&sA[grp][ld_r][ld_kq]) = va0;
-    *reinterpret_cast<float4*>(&sA[grp][ld_r + 16][ld_kq]) = va1;
     sW[grp][ld_kq + 0][ld_r] = vw0.x; sW[grp][ld_kq + 1][ld_r] = vw0.y; sW[grp][ld_kq + 2][ld_r] = vw0.z; sW[grp][ld_kq + 3][ld_r] = vw0.w;
     sW[grp][ld_kq + 0][ld_r + 16] = vw1.x; sW[grp][ld_kq + 1][ld_r + 16] = vw1.y;
     sW[grp][ld_kq + 2][ld_r + 16] = vw1.z; sW[grp][ld_kq + 3][ld_r + 16] = vw1.w;
+    copies_wait();
     group_barrier(grp);
     int ns = s, nk0 = k0 + TK;
     if (nk0 >= it.seg_kb[s] * 64) {
       ++ns;
       nk0 = 0;
     }
-    if (c + 1 < c_end) fetch(ns, nk0);
+    if (c + 1 < c_end) fetch(ns, nk0, buf ^ 1);
     float part[2][4] = {};  // this chunk's
 #pragma unroll
     for (int k4 = 0; k4 < TK; k4 += 4) {
-      const float4 r0 = *reinterpret_cast<const float4*>(&sA[grp][2 * ty][k4]);
-      const float4 r1 = *reinterpret_cast<const float4*>(&sA[grp][2 * ty + 1][k4]);
+      const float4 r0 = *reinterpret_cast<const float4*>(&sA[grp][buf][2 * ty][k4]);
+      const float4 r1 = *reinterpret_cast<const float4*>(&sA[grp][buf][2 * ty + 1][k4]);
       const float a0[4] = {r0.x, r0.y, r0.z, r0.w}, a1[4] = {r1.x, r1.y, r1.z, r1.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -128,52 +131,51 @@ cell_simt_kernel(const __grid_constant__ SimtArgs args, const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+      for (int j = 0; j < 2; ++j) add_f32x2(acc[i][j], pair_f32x2(part[i][2 * j], part[i][2 * j + 1]));
     group_barrier(grp);
     s = ns;
     k0 = nk0;
+    buf ^= 1;
   }
 
-  // Partial sums of groups 1..3 to group 0, added in group order.
-  if (grp > 0) {
-    *reinterpret_cast<float4*>(&sP[grp - 1][tg][0]) = make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
-    *reinterpret_cast<float4*>(&sP[grp - 1][tg][4]) = make_float4(acc[1][0], acc[1][1], acc[1][2], acc[1][3]);
+  // Every group's partial sums, over its rows of A, which all of its threads have read.
+  {
+    float* p = &sA[grp][0][0][0] + 2 * ty * TN + 4 * tx;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      *reinterpret_cast<ulonglong2*>(p + i * TN) = make_ulonglong2(acc[i][0], acc[i][1]);
   }
   __syncthreads();
-  if (grp > 0) return;
+  if (threadIdx.x >= TM * TN / 4) return;
+  const int r = threadIdx.x >> 3, row = m_tile * TM + r;
+  if (row >= it.rows) return;
+  const int col = 4 * (threadIdx.x & 7), col0 = n_tile * TN + col;  // 4 consecutive columns: one LSTM unit
+  float4 v = *reinterpret_cast<const float4*>(&sA[0][0][0][0] + r * TN + col);
 #pragma unroll
-  for (int g = 0; g < kSplitK - 1; ++g) {
-    const float4 p0 = *reinterpret_cast<const float4*>(&sP[g][tg][0]);
-    const float4 p1 = *reinterpret_cast<const float4*>(&sP[g][tg][4]);
-    acc[0][0] += p0.x; acc[0][1] += p0.y; acc[0][2] += p0.z; acc[0][3] += p0.w;
-    acc[1][0] += p1.x; acc[1][1] += p1.y; acc[1][2] += p1.z; acc[1][3] += p1.w;
+  for (int g = 1; g < kSplitK; ++g) {
+    const float4 p = *reinterpret_cast<const float4*>(&sA[g][0][0][0] + r * TN + col);
+    v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
   }
-
-  const int col0 = n_tile * TN + 4 * tx;
-  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (it.bias != nullptr) b = *reinterpret_cast<const float4*>(it.bias + col0);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int row = m_tile * TM + 2 * ty + i;
-    if (row >= it.rows) continue;
-    if (EPI == EPI_LSTM) {
-      const int unit = col0 >> 2;
-      float* cp = it.c + static_cast<size_t>(row) * batch.ld_c + unit;
-      const float cprev = it.c_zero ? 0.f : *cp;
-      const float gi = sigmoid_acc(acc[i][0] + b.x);
-      const float gf = sigmoid_acc(acc[i][1] + b.y);
-      const float go = sigmoid_acc(acc[i][2] + b.z);
-      const float gc = tanhf(acc[i][3] + b.w);
-      const float cn = gf * cprev + gi * gc;
-      *cp = cn;
-      reinterpret_cast<float*>(it.out)[static_cast<size_t>(row) * batch.ld_out + unit] = go * tanhf(cn);
-    } else {
-      float4 v = make_float4(acc[i][0] + b.x, acc[i][1] + b.y, acc[i][2] + b.z, acc[i][3] + b.w);
-      if (EPI == EPI_TANH) {
-        v.x = tanhf(v.x); v.y = tanhf(v.y); v.z = tanhf(v.z); v.w = tanhf(v.w);
-      }
-      *reinterpret_cast<float4*>(reinterpret_cast<float*>(it.out) + static_cast<size_t>(row) * batch.ld_out + col0) = v;
+  if (it.bias != nullptr) {
+    const float4 b = *reinterpret_cast<const float4*>(it.bias + col0);
+    v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+  }
+  if (EPI == EPI_LSTM) {
+    const int unit = col0 >> 2;
+    float* cp = it.c + static_cast<size_t>(row) * batch.ld_c + unit;
+    const float cprev = it.c_zero ? 0.f : *cp;
+    const float gi = sigmoid_acc(v.x);
+    const float gf = sigmoid_acc(v.y);
+    const float go = sigmoid_acc(v.z);
+    const float gc = tanhf(v.w);
+    const float cn = gf * cprev + gi * gc;
+    *cp = cn;
+    reinterpret_cast<float*>(it.out)[static_cast<size_t>(row) * batch.ld_out + unit] = go * tanhf(cn);
+  } else {
+    if (EPI == EPI_TANH) {
+      v.x = tanhf(v.x); v.y = tanhf(v.y); v.z = tanhf(v.z); v.w = tanhf(v.w);
     }
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(it.out) + static_cast<size_t>(row) * batch.ld_out + col0) = v;
   }
 }
 
@@ -194,12 +196,20 @@ int launch_cell_simt(int epi, const float* const* act, const int* ld_act, const 
   // Plain launches: as a dependent launch this kernel was measured 45 % slower on the 67 levels of a
   // depth-4 stack (it has no set-up to run early, and the wait for the level before it costs more
   // than an ordinary launch behind it).
+  static std::atomic<unsigned long long> configured[3];
+  auto run = [&](auto kfn, int which) -> bool {
+    if (!ensure_dynamic_smem(kfn, kSmemBytes, configured[which])) return false;
+    kfn<<<batch.total_tiles, kSimtThreads, kSmemBytes, stream>>>(a, batch);
+    return true;
+  };
+  bool ok = false;
   switch (epi) {
-    case EPI_STORE: cell_simt_kernel<EPI_STORE><<<batch.total_tiles, kSimtThreads, 0, stream>>>(a, batch); break;
-    case EPI_LSTM: cell_simt_kernel<EPI_LSTM><<<batch.total_tiles, kSimtThreads, 0, stream>>>(a, batch); break;
-    case EPI_TANH: cell_simt_kernel<EPI_TANH><<<batch.total_tiles, kSimtThreads, 0, stream>>>(a, batch); break;
+    case EPI_STORE: ok = run(cell_simt_kernel<EPI_STORE>, 0); break;
+    case EPI_LSTM: ok = run(cell_simt_kernel<EPI_LSTM>, 1); break;
+    case EPI_TANH: ok = run(cell_simt_kernel<EPI_TANH>, 2); break;
     default: return FTB_ERR_ARG;
   }
+  if (!ok) return FTB_ERR_LAUNCH;
   count_launch();
   return cudaGetLastError() == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
 }

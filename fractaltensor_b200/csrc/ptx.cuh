@@ -126,6 +126,33 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, g_status, code));
 }
 
+// ------------------------------------------------- two fp32 numbers to an instruction
+// (each half rounds as the scalar instruction does)
+__device__ __forceinline__ uint64_t dup_f32x2(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void add_f32x2(uint64_t& acc, uint64_t a) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a));
+}
+
+// ------------------------------------------------- global -> shared without a register on the way
+// 16 bytes through L2; zeros when !valid (src is not read then, but has to be an address of the array).
+__device__ __forceinline__ void copy16_async(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 // ------------------------------------------------- inter-CTA flags (global memory)
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
