@@ -54,12 +54,6 @@ __device__ __forceinline__ void group_barrier(int group) {
   asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kGroupThreads) : "memory");
 }
 
-__device__ __forceinline__ float4 ld_cg4(const float* p) {
-  float4 v;
-  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
-  return v;
-}
-
 // Thread 0 of the CTA: wait until `*counter >= target`.  False on time-out or when another CTA has
 // already reported an error (its dependants would only time out one after another).
 __device__ __forceinline__ bool wait_cell(const int* counter, int target, int* status) {
@@ -94,7 +88,7 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
   const int tile = blockIdx.x - j * tiles;
   const int n_tile = tile / a.m_tiles;
   const int m_tile = tile - n_tile * a.m_tiles;
-  const int row0 = m_tile * TM;
+  const int row0 = m_tile * TM, rows = min(TM, a.N - row0);
 
   const int tid = threadIdx.x;
   const int grp = tid / kGroupThreads;
@@ -120,6 +114,8 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
         sW[(k + 3) * ldw + col] = v.w;
       }
     }
+    // (rows past the batch are multiplied as zeros)
+    for (int e = tid; e < (TM - rows) * lda; e += kThreads) sA[rows * lda + e] = 0.f;
     const int col0 = n_tile * TN + 4 * tx;
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.bias != nullptr) b = *reinterpret_cast<const float4*>(a.bias + static_cast<size_t>(l) * 4 * a.H + col0);
@@ -142,48 +138,44 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
         const float* in = l == 0 ? a.x + static_cast<size_t>(t) * a.N * a.I
                                  : a.hs + (static_cast<size_t>(l - 1) * a.L + t) * a.N * a.H;
         const float* rec = t > 0 ? a.hs + (static_cast<size_t>(l) * a.L + t - 1) * a.N * a.H : nullptr;
-        const int k4s = Kt / 4, n4 = TM * k4s;
-        // eight loads in flight per thread before the first store (one round trip to L2 for K = 512)
-        constexpr int kBatch = 8;
-        for (int e0 = tid; e0 < n4; e0 += kBatch * kThreads) {
-          float4 v[kBatch];
-#pragma unroll
-          for (int u = 0; u < kBatch; ++u) {
-            const int e = e0 + u * kThreads;
-            const int r = e / k4s, k = (e - r * k4s) * 4;
-            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (e < n4 && row0 + r < a.N) {
-              v[u] = k < Il ? ld_cg4(in + static_cast<size_t>(row0 + r) * Il + k)
-                            : ld_cg4(rec + static_cast<size_t>(row0 + r) * a.H + (k - Il));
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < kBatch; ++u) {
-            const int e = e0 + u * kThreads;
-            const int r = e / k4s, k = (e - r * k4s) * 4;
-            if (e < n4) *reinterpret_cast<float4*>(sA + r * lda + k) = v[u];
-          }
+        // A warp to a row: 16-byte copies that bypass L1 and the registers, all in flight at once.
+        for (int r = tid >> 5; r < rows; r += kThreads / 32) {
+          const float* in_r = in + static_cast<size_t>(row0 + r) * Il;
+          const float* rec_r = t > 0 ? rec + static_cast<size_t>(row0 + r) * a.H : nullptr;
+          for (int k = 4 * (tid & 31); k < Kt; k += 128)
+            copy16_async(sA + r * lda + k, k < Il ? in_r + k : rec_r + (k - Il), true);
         }
+        copies_commit();
+        copies_wait();
       }
       __syncthreads();
 
       // ---- this group's chunks of K, in the level kernel's order.  One warp per group multiplies:
-      // a lane holds 4 rows x 8 columns of the tile, so 12 shared-memory loads feed 128 FMAs (the
-      // level kernel's 2 x 4 per thread needs 6 per 32 and is bound by shared-memory bandwidth).
-      // Every chunk's sum is one chain in ascending order of K, as there.
+      // a lane holds 4 rows x 8 columns of the tile, so 12 shared-memory loads feed 128 products, two to an
+      // FMA (the level kernel's 2 x 4 per thread needs 6 per 32 and is bound by shared-memory bandwidth).
+      // Every chunk's sum is one chain in ascending order of K, as there.  The group's sum waits in shared memory:
+      // beside a chunk's sums its 32 registers leave no room to load ahead (D 1, L 64, N 32, I 512, H 256: 848 us
+      // with both in registers, 651 this way).
       if ((tid >> 5) == grp * 5) {  // warps 0, 5, 10, 15: one per scheduler
         const int lane = tid & 31;
         const int cx = lane & 3;   // columns 8 cx .. 8 cx + 7
         const int ry = lane >> 2;  // rows 4 ry .. 4 ry + 3
         const int total_chunks = Kt / TK;
         const int c_begin = total_chunks * grp / kSplitK, c_end = total_chunks * (grp + 1) / kSplitK;
-        float acc[4][8] = {};
+        float* p = sP + static_cast<size_t>(grp) * TM * TN + (4 * ry) * TN + 8 * cx;
+        if (c_begin == c_end)  // fewer chunks than groups
+          for (int i = 0; i < 4; ++i) {
+            *reinterpret_cast<float4*>(p + i * TN) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(p + i * TN + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         const float* Ar = sA + (4 * ry) * lda;
         const float* Wc = sW + 8 * cx;
-        for (int c = c_begin; c < c_end; ++c) {
-          float part[4][8] = {};
 #pragma unroll 1
-          for (int k0 = c * TK; k0 < (c + 1) * TK; k0 += 4) {
+        for (int c = c_begin; c < c_end; ++c) {
+          uint64_t part[4][4] = {};
+#pragma unroll
+          for (int kk = 0; kk < TK; kk += 4) {
+            const int k0 = c * TK + kk;
             float av[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -192,25 +184,30 @@ lstm_simt_static_kernel(const __grid_constant__ SimtStaticArgs a) {
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const float4 w0 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw);
-              const float4 w1 = *reinterpret_cast<const float4*>(Wc + (k0 + q) * ldw + 4);
-              const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+              const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(Wc + (k0 + q) * ldw);
+              const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(Wc + (k0 + q) * ldw + 4);
+              const uint64_t wv[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
+              for (int i = 0; i < 4; ++i) {
+                const uint64_t xx = dup_f32x2(av[i][q]);
 #pragma unroll
-                for (int n = 0; n < 8; ++n) part[i][n] = fmaf(av[i][q], wv[n], part[i][n]);
+                for (int n = 0; n < 4; ++n) fma_f32x2(part[i][n], xx, wv[n]);
+              }
             }
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < 4; ++i) {
+            ulonglong2 s0 = make_ulonglong2(0, 0), s1 = s0;
+            if (c > c_begin) {
+              s0 = *reinterpret_cast<const ulonglong2*>(p + i * TN);
+              s1 = *reinterpret_cast<const ulonglong2*>(p + i * TN + 4);
+            }
+            uint64_t sum[4] = {s0.x, s0.y, s1.x, s1.y};
 #pragma unroll
-            for (int n = 0; n < 8; ++n) acc[i][n] += part[i][n];
-        }
-        float* p = sP + static_cast<size_t>(grp) * TM * TN + (4 * ry) * TN + 8 * cx;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          *reinterpret_cast<float4*>(p + i * TN) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-          *reinterpret_cast<float4*>(p + i * TN + 4) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+            for (int n = 0; n < 4; ++n) add_f32x2(sum[n], part[i][n]);
+            *reinterpret_cast<ulonglong2*>(p + i * TN) = make_ulonglong2(sum[0], sum[1]);
+            *reinterpret_cast<ulonglong2*>(p + i * TN + 4) = make_ulonglong2(sum[2], sum[3]);
+          }
         }
       }
       __syncthreads();

@@ -48,3 +48,22 @@ def test_nan_states_are_states(ops):
     h, _ = ops.lstm_stacked(x, Wp, b, schedule=2)
     ops.check_status()
     assert not torch.isnan(h[:, :, :3]).any() and torch.isnan(h[:, 2:, 3:]).all() and not torch.isnan(h[:, :2]).any()
+
+
+@pytest.mark.parametrize("L,N,I,H", [
+    (5, 1, 64, 64),      # two chunks of K in the first step: groups without one
+    (4, 32, 64, 128),    # a whole tile
+    (6, 33, 320, 192),   # one sequence in the second tile
+    (3, 7, 192, 320),
+    (4, 40, 512, 256),   # the widest K
+])
+def test_an_input_of_another_width(ops, L, N, I, H):
+    """csrc/lstm_simt_static.cu, the fp32 kernel of models whose input is wider or narrower than the state."""
+    g = torch.Generator(device="cuda").manual_seed(I + H)
+    u = lambda *s: (torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5
+    Wp, b = ops.lstm_pack_weights(u(1, 4, I, H), u(1, 4, H, H), u(1, 4, H))
+    x = torch.randn(L, N, I, device="cuda", generator=g)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1)
+    h, c = ops.lstm_stacked(x, Wp, b, schedule=2)
+    ops.check_status()
+    assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
