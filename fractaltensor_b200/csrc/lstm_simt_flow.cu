@@ -372,30 +372,37 @@ int launch(const SimtFlowArgs& a, size_t smem, cudaStream_t stream) {
 
 }  // namespace
 
-// Rows of a CTA's tile (8, 16 or 32) for a problem, 0: not for this kernel.  Layers that do not fit on the device
-// beside each other cost a sweep each.  Measured steps, us: 8 rows 2.5 / 2.8 / 3.1 at H 64 / 128 / 256, 16 rows
-// 3.8 / 3.9 at H 192 / 256, 32 rows 5.4 / 7.2 at H 128 / 256.
-int lstm_simt_flow_rows(int D, int L, int N, int I, int H, int sm_count) {
-  if (I != H || H % 64 != 0) return 0;
-  int best = 0;
-  double best_us = 0;
+// How the kernel would run a problem: rows of a CTA's tile (8, 16 or 32); est_us: about what that takes.
+struct SimtFlowPlan {
+  int rows;
+  double est_us;
+};
+
+// False: not for this kernel.  Layers that do not fit on the device beside each other cost a sweep each.  Measured
+// steps, us, at H 64 / 128 / 192 / 256 / 320 / 384: 8 rows 2.7 / 2.9 / 3.1 / 3.2 / 4.3 / 4.5, 16 rows 3.4 / 3.4 / 3.7 /
+// 3.8 / 5.6 / 5.7, 32 rows 5.3 / 5.4 / 5.8 / 7.0.  A row of more than 256 is read in two rounds; 32 rows at H 256 leave
+// room for one input tile only.
+bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFlowPlan* plan) {
+  if (I != H || H % 64 != 0) return false;
+  bool found = false;
   for (int tm = 8; tm <= 32; tm *= 2) {
     if (smem_bytes(tm, H, 1) > static_cast<size_t>(kMaxSmem)) continue;
     const long long tiles = static_cast<long long>((N + tm - 1) / tm) * (4 * H / TN);
     if (tiles > sm_count) continue;
     const int per_sweep = std::min<int>(D, static_cast<int>(sm_count / tiles));
     const int sweeps = (D + per_sweep - 1) / per_sweep;
-    const double step = tm == 8 ? 2.4 + 0.7 * H / 256 : (tm == 16 ? 2.9 + 1.0 * H / 256 : 3.6 + 3.6 * H / 256);
+    const double h = H / 256.0;
+    const double step = tm == 8    ? 2.6 + 0.55 * h + (H > 256 ? 1.0 : 0.0)
+                        : tm == 16 ? 3.2 + 0.6 * h + (H > 256 ? 1.65 : 0.0)
+                                   : 5.0 + 0.8 * h + (H >= 256 ? 1.2 : 0.0);
     const double us = static_cast<double>(sweeps) * (L + per_sweep - 1) * step;
-    if (best == 0 || us < best_us) {
-      best = tm;
-      best_us = us;
-    }
+    if (!found || us < plan->est_us) *plan = {tm, us};
+    found = true;
   }
-  return best;
+  return found;
 }
 
-// x: [L,N,H]; Wp: [D,4H,2H] fp32 packed; hs: [D,L,N,H]; c: [D,N,H]; tm: lstm_simt_flow_rows.
+// x: [L,N,H]; Wp: [D,4H,2H] fp32 packed; hs: [D,L,N,H]; c: [D,N,H]; tm: SimtFlowPlan::rows.
 int launch_lstm_simt_flow(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L, int N,
                           int H, int tm, int* status, int sm_count, cudaStream_t stream) {
   SimtFlowArgs a;

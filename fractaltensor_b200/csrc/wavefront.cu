@@ -27,10 +27,15 @@ int launch_cell_gemm(int dtype, int epi, int bn, int pair, const CUtensorMap* ma
 int launch_cell_gemm_persistent(int dtype, int epi, int bn, int pair, const CUtensorMap* maps,
                                 const CUtensorMap& mapW, const CUtensorMap& mapC, const CellBatch& header,
                                 const PlanView& plan, int* status, int sm_count, cudaStream_t stream);
-int lstm_simt_flow_rows(int D, int L, int N, int I, int H, int sm_count);
+struct SimtFlowPlan {
+  int rows;
+  double est_us;
+};
+bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFlowPlan* plan);
 int launch_lstm_simt_flow(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L, int N,
                           int H, int tm, int* status, int sm_count, cudaStream_t stream);
 bool lstm_simt_static_supported(int D, int N, int I, int H, int sm_count);
+double lstm_simt_static_us(int D, int L, int N, int I, int H, int sm_count);
 int launch_lstm_simt_static(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L,
                             int N, int I, int H, int* done, int* status, int sm_count, cudaStream_t stream);
 bool lstm_static_supported(int dtype, int D, int N, int I, int H, int G, int sm_count);
@@ -536,20 +541,24 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
     // fp32: one persistent launch, a CTA per accumulator tile with its weights in shared memory
     // (csrc/lstm_simt_static.cu), when a layer's tiles fit on the device.
     if (workspace_bytes < lay.total) return FTB_ERR_WORKSPACE;
-    // With I == H the one whose states carry their own arrival (csrc/lstm_simt_flow.cu: 8.2 -> 7.2 us a step at
-    // H 256 and 32 sequences, 7.6 -> 3.1 at 8).
     const bool can = lstm_simt_static_supported(D, N, I, H, cl.sm_count);
-    const int flow_rows = can ? lstm_simt_flow_rows(D, L, N, I, H, cl.sm_count) : 0;
     if (schedule >= 2 && !can) return FTB_ERR_ARG;
     if (can) {
-      if (flow_rows > 0)
+      // With I == H there is also the kernel whose states carry their own arrival (csrc/lstm_simt_flow.cu; schedule
+      // 5 names it, 2 to 4 the other one).  A step of its is shorter, but its tiles need more CTAs where 32 rows do
+      // not fit beside the weights (H of 320 and more) or the batch is large, and layers that do not fit beside each
+      // other cost a sweep each: the automatic choice takes the one with the smaller estimate (us, this one / the other,
+      // L 64: D 3, N 32 at H 256 478 / 518, at H 320 1069 / 594; D 3, N 16, H 320 382 / 581; D 3, N 200, H 64 650 / 512).
+      SimtFlowPlan flow;
+      const bool can_flow = lstm_simt_flow_plan(D, L, N, I, H, cl.sm_count, &flow);
+      if (can_flow && (schedule == 5 || (schedule == 0 && flow.est_us < lstm_simt_static_us(D, L, N, I, H, cl.sm_count))))
         rc = launch_lstm_simt_flow(static_cast<const float*>(x), static_cast<const float*>(Wp), bias_p,
-                                   static_cast<float*>(hs), c, D, L, N, H, flow_rows, status, cl.sm_count, stream);
+                                   static_cast<float*>(hs), c, D, L, N, H, flow.rows, status, cl.sm_count, stream);
       else
         rc = launch_lstm_simt_static(static_cast<const float*>(x), static_cast<const float*>(Wp), bias_p,
-                                   static_cast<float*>(hs), c, D, L, N, I, H,
-                                   reinterpret_cast<int*>(static_cast<char*>(workspace) + lay.done), status,
-                                   cl.sm_count, stream);
+                                     static_cast<float*>(hs), c, D, L, N, I, H,
+                                     reinterpret_cast<int*>(static_cast<char*>(workspace) + lay.done), status,
+                                     cl.sm_count, stream);
       // A refused cooperative launch falls back to one launch per level under the automatic choice.
       if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
     }

@@ -113,6 +113,7 @@ def lstm_stacked(x, Wp, bias_p=None, hs=None, c=None, layers_per_group=0, bn=0, 
     (CTA pairs on 256 batch rows), 4 static tile ownership with the batch on the N side of the MMA
     (at most 128 sequences; `resident`: recurrent weight blocks kept on chip, 0 auto, -1 none), 5 all weights
     on chip and the states handed on through the output array (layers whose tiles fit on the device);
+    fp32: 2 to 4 one persistent kernel with a counter per cell, 5 as above (I == H);
     pair: 0 auto, 1 single CTAs, 2 CTA pairs."""
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)

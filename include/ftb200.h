@@ -62,21 +62,25 @@ int ftb_lstm_pack_weights(const void* W, const void* U, const void* bias, void* 
  *  [1] bn                accumulator tile width, 128 or 256
  *  [2] schedule          1 = one kernel launch per wavefront level; 2 = one persistent
  *                        cooperative kernel, cells chained through completion counters
- *                        in the workspace (16-bit dtypes; for the fp32 stacked LSTM 2 and 3 both
- *                        name its one persistent kernel: a CTA keeps a 32 x 32 tile of one layer
- *                        with its weights in shared memory and its cell state in registers over
- *                        the whole sweep, the automatic choice when [I + H] x 32 weights and 32
- *                        rows of operands fit in shared memory and a layer's tiles fit on the
- *                        device); 3 = persistent with static
+ *                        in the workspace (16-bit dtypes); 3 = persistent with static
  *                        tile ownership (stacked LSTM: every CTA pair keeps its slice of a
  *                        layer, cell state in registers, over a whole sweep; needs a layer
- *                        group's tiles to fit on the device; the automatic choice when so and
- *                        the batch exceeds 128 sequences); 4 = static tile ownership with the
+ *                        group's tiles to fit on the device); 4 = static tile ownership with the
  *                        weights as the M side of the MMA and the batch (at most 128 sequences)
  *                        as its N side, cell state in registers, recurrent weights resident in
- *                        tensor memory (stacked LSTM; the automatic choice for such batches: it
- *                        is the kernel a batch of 256 sharded over 2, 4 or 8 GPUs runs); every
- *                        schedule gives the same bits
+ *                        tensor memory (stacked LSTM); 5 = all weights on chip for a whole sweep
+ *                        over time, hidden states handed on through the output array, which is
+ *                        filled with a pattern beforehand (stacked LSTM, rectangular and ragged,
+ *                        where a layer's tiles fit on the device).  The automatic choice of the
+ *                        16-bit stacked LSTM is 5 where it is expected to be faster, else 4 for
+ *                        at most 128 sequences, else 3 where it fits, else 2.
+ *                        fp32 stacked LSTM: 2, 3 and 4 name one persistent kernel (a CTA keeps a
+ *                        32 x 32 tile of one layer with its weights in shared memory and its
+ *                        cell state in registers, a counter per cell; needs [I + H] x 32 weights
+ *                        and 32 rows of operands to fit in shared memory and a layer's tiles on
+ *                        the device); 5 the one that hands states on through the output array
+ *                        (I == H; else as 2); automatic: the one expected to be faster.
+ *                        Every schedule gives the same bits
  *  [3] skew              persistent schedule: layer j of a group runs `skew` levels
  *                        behind layer j-1
  *  [4] pair              1 = single CTAs, 2 = CTA pairs (tcgen05 cta_group::2) on
@@ -109,8 +113,9 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
  * fully committed memory pool).  Same arguments and results as ftb_lstm_stacked_fwd with the
  * persistent schedule, but the schedule tables, completion counters and status word live in
  * a 4 MiB array inside the library image (held on every GPU that loads the library).
- * Returns FTB_ERR_SCRATCH_LIMIT (7) when ftb_lstm_stacked_workspace_bytes(D, L, N, H) exceeds
- * 4 MiB; fp16/bf16 only.  The array is shared by all calls on a device: calls that can
+ * Returns FTB_ERR_SCRATCH_LIMIT (7) when the tables and counters of schedule 2 exceed 4 MiB
+ * (ftb_lstm_stacked_workspace_bytes(D, L, N, H) less the counters of schedule 5, which is taken where
+ * they fit too); fp16/bf16 only.  The array is shared by all calls on a device: calls that can
  * overlap on the GPU race and must be serialised by the caller; consecutive calls on one
  * stream are safe.  The first call on a device looks the array's address up and should be
  * made outside stream capture.  `scratch_out` (may be NULL) receives the array's device
@@ -132,7 +137,8 @@ int ftb_lstm_stacked_fwd_noalloc(const void* x, const void* Wp, const float* bia
  * packed order; c (out): fp32 [D,N,H], the cell state of each sequence after its own last step.
  * Only tiles that hold active rows are computed.  With ftb_lstm_stacked_varlen_workspace_bytes(D, L)
  * bytes of workspace (16-bit dtypes) the wavefront runs as one persistent launch whose schedule
- * tables are copied from host memory on `stream`; with less it runs one launch per level. */
+ * tables (schedule 5: the first rows of the steps) are copied from host memory on `stream`, so that
+ * form is not for stream capture; with less it runs one launch per level. */
 size_t ftb_lstm_stacked_varlen_workspace_bytes(int D, int L);
 int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
                                 const int* active_rows, int D, int L, int I, int H, int dtype, const int* tuning,
