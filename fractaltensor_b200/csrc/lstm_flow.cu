@@ -129,9 +129,10 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, 
     int G = std::min(D, sm_count / (S * tiles));
     const int sweeps = (D + G - 1) / G;
     G = (D + sweeps - 1) / sweeps;
-    // Measured steps: 1.7 / 1.9 us at 16 columns and H 256 / 512, 2.1 / 2.7 at 32, 3.0 / 4.2 at 64; a state of
-    // more than eight K blocks is read in two rounds.
-    const double step = 1.4 + nb / 80.0 + nb * H / 16384.0 + (H > 512 ? 0.5 : 0.0);
+    // Measured steps: 1.8 / 2.0 us at 16 columns and H 256 / 512, 2.2 / 2.6 at 32, 3.0 / 4.3 at 64, more with more CTAs
+    // at work; a state of more than eight K blocks is read in two rounds.
+    const double busy = static_cast<double>(S * tiles * G) / sm_count;
+    const double step = 1.2 + nb / 64.0 + nb * H / 16800.0 + (H > 512 ? 0.5 : 0.0) + 0.3 * busy * nb / 64.0;
     const double us = sweeps * ((L + G - 1) * step + 10.0);
     if (!found || us < plan->est_us) *plan = {nb, S, G, us};
     found = true;

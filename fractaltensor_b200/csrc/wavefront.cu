@@ -473,6 +473,31 @@ static int fit_groups(int D, int G, int ctas, int sm_count) {
   return (D + groups - 1) / groups;
 }
 
+// About what the 16-bit kernels that stream weights take (us), by groups of G layers: sweeps * (L + G - 1) steps of
+// a length fitted to 504 problems (H 128..1024, D 1..16, N 16..256, L 64; within 20 %, 6 % in the root mean
+// square).  Measured, us (generic / static / weights on the M side / everything on chip; * taken): D 8, N 200, H 640 1013*
+// / 1436 / - / 1747; D 12, N 200, H 512 1092* / 1369 / - / 1792; D 16, N 256, H 512 1423 / 1118* / - / 2507; D 4, N 256, H 512
+// 716 / 550* / - / 596; D 12, N 160, H 320 974 / 781 / - / 678*; D 12, N 128, H 512 983 / 1073 / 819* / 943; D 12, N 128, H 128
+// 541 / 506 / 291 / 236*.
+struct StackedEstimate {
+  int D, L, N, sm_count, m, n_tiles;
+  double h;
+  StackedEstimate(int D, int L, int N, int H, int sm_count)
+      : D(D), L(L), N(N), sm_count(sm_count), m((N + 255) / 256), n_tiles((4 * H + 255) / 256), h(H / 1024.0) {}
+  double steps(int G) const { return static_cast<double>((D + G - 1) / G) * (L + G - 1); }
+  // one CTA per 128 gate rows; the batch is the N side of the MMA, 16 to 128 wide
+  double wmajor(int G) const {
+    const double n = (N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128) / 128.0;
+    return steps(G) * (1.77 + 5.65 * h + 1.1 * n + 1.15 * n * h + 0.45 * (32 * h * G / sm_count));
+  }
+  // a CTA pair per 256 sequences x 256 gate columns; without full tiles of 128 sequences it stores row by row
+  double static_pairs(int G) const {
+    const double busy = static_cast<double>(2 * m * n_tiles * G) / sm_count;
+    return steps(G) * (N % 128 == 0 ? 6.4 - 0.9 * h + 6.0 * h * h + 3.2 * h * busy : 8.3 + 5.0 * h * h * h + 2.2 * busy);
+  }
+  double generic(int G) const { return steps(G) * (11.9 + 1.2 * h + 0.23 * m * G); }
+};
+
 int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, int D, int L,
                          int N, int I, int H, int dtype, const int* tuning, void* workspace, size_t workspace_bytes,
                          void* stream_) {
@@ -575,16 +600,20 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
     const int Gw = layers_per_group > 0 ? G : fit_groups(D, G, tiles, cl.sm_count);
     const bool can_wmajor = lstm_wmajor_supported(dtype, D, N, I, H, Gw, cl.sm_count);
     const int Gs = layers_per_group > 0 ? G : fit_groups(D, G, 2 * ((N + 255) / 256) * ((4 * H + 255) / 256), cl.sm_count);
-    // Everything on chip (schedule 5, and the automatic choice where it is expected to be faster than the
-    // kernels that stream weights; their steps as measured: with up to 128 sequences 5.5 us at H 512 and
-    // 9..12 at H 1024, above that 9.5 at H 320 and 14 at H 1024).
+    const bool can_static = tune.pair != 1 && (bn == 0 || bn == 256) && !tune.fine_deps &&
+                            lstm_static_supported(dtype, D, N, I, H, Gs, cl.sm_count);
+    // Everything on chip: schedule 5, and the automatic choice where that is expected to be faster.
     FlowPlan flow;
     const bool can_flow = layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, &flow) &&
                           workspace_bytes >= lay.total + flow_flag_bytes(D, L, flow.S);
     if (schedule == 5 && !can_flow) return FTB_ERR_ARG;
-    const int Gold = can_wmajor ? Gw : Gs;
-    const double old_step = can_wmajor ? 1.6 + 6.5 * H / 1024 + N * H / 40960.0 : 7.5 + 6.5 * H / 1024;
-    const double old_us = ((D + Gold - 1) / Gold) * (L + Gold - 1) * old_step;
+    const StackedEstimate est(D, L, N, H, cl.sm_count);
+    const double wmajor_us = est.wmajor(Gw), static_us = est.static_pairs(Gs), generic_us = est.generic(G);
+    // Groups that had to be cut to what fits on the device, for static ownership, are more sweeps than those of the
+    // generic kernel, which takes groups of any size.
+    const bool cut = 2 * ((N + 255) / 256) * ((4 * H + 255) / 256) * G > cl.sm_count;
+    const bool take_static = can_static && (!cut || static_us < 1.03 * generic_us);
+    const double old_us = can_wmajor ? wmajor_us : (take_static ? static_us : generic_us);
     if (schedule == 5 || (schedule == 0 && can_flow && flow.est_us < old_us && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
       rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, nullptr, static_cast<int64_t>(L) * N, D, L, N, I, H, flow,
                             reinterpret_cast<int*>(ws + lay.total), status, stream);
@@ -605,10 +634,8 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
       if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
       goto level_schedule;
     }
-    const bool can_static = tune.pair != 1 && (bn == 0 || bn == 256) && !tune.fine_deps &&
-                            lstm_static_supported(dtype, D, N, I, H, Gs, cl.sm_count);
     if (schedule == 3 && !can_static) return FTB_ERR_ARG;
-    if ((schedule == 3 || schedule == 0) && can_static) {
+    if (schedule == 3 || (schedule == 0 && take_static)) {
       unsigned long long* trace = nullptr;
 #ifdef FTB_TRACE
       trace = reinterpret_cast<unsigned long long*>(ws + lay.trace);
