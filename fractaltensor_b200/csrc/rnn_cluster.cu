@@ -1043,17 +1043,13 @@ int dilated_slices(const int* dilations, int D, int N, int max_clusters, int* nb
   return s128 <= 8 && total <= max_clusters ? total : 0;
 }
 
-// Slice widths of the layers when the launch goes without clusters, false: it does not.  Dilation 1: 16, 32 or 48;
-// the others 64, or 128 from dilation 3 on (a step's trip through global memory is hidden behind the steps
-// between); the narrowest that fit beside each other.  Clusters of 2 and 4 CTAs hand a state on fast enough for
-// batches of up to 64 (us, 3 layers of 512 steps, with clusters / without: H 64, N 24 895 / 911, N 64 985 / 1105;
-// H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above 64 sequences and at H 256 they lose:
-// H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1164, N 256 and six layers 1613 / 1330, 1654 with every layer
-// but the first on slices of 128).
+// Slice widths of the layers for a launch without clusters, false: it does not fit or no layer has dilation 1.
+// Dilation 1: 16, 32 or 48; the others 64, or 128 from dilation 3 on (a step's trip through global memory is hidden
+// behind the steps between); the narrowest that fit beside each other.
 bool dilated_flow_widths(const int* dilations, int D, int N, int CL, int sm_count, int* nb) {
   int ones = 0;
   for (int l = 0; l < D; ++l) ones += dilations[l] == 1;
-  if (ones == 0 || (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64)) return false;
+  if (ones == 0) return false;
   for (int wide = 64; wide <= 128; wide *= 2)
     for (int narrow = 16; narrow <= 48; narrow += 16) {
       int ctas = 0;
@@ -1065,6 +1061,11 @@ bool dilated_flow_widths(const int* dilations, int D, int N, int CL, int sm_coun
     }
   return false;
 }
+// Clusters of 2 and 4 CTAs hand a state on fast enough for batches of up to 64 (us, 3 layers of 512 steps, with
+// clusters / without: H 64, N 24 895 / 911, N 64 985 / 1105; H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above
+// 64 sequences and at H 256 they lose: H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1164, N 256 and six layers 1613 / 1330,
+// 1654 with every layer but the first on slices of 128).
+bool dilated_prefers_clusters(int N, int CL) { return (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64); }
 
 // Clusters of `cl` CTAs of the dilated kernel that can be resident at once on the current device (a
 // cluster needs its CTAs' SMs inside one GPC, so this is less than SMs / cl: 15 clusters of 8 on a
@@ -1111,10 +1112,12 @@ bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count
 // one counter per (cell, slice of 16 sequences or more); at most 64 (1024 sequences)
 size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 64; }
 
-// x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).
+// x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).  schedule 4: with
+// clusters where they fit, 5: without (FTB_ERR_ARG where that does not
+// fit), 0: the faster of the two.
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
-                                const int* dilations, int D, int L, int N, int H, int* flags, int* status, int sm_count,
-                                cudaStream_t stream) {
+                                const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
+                                int sm_count, cudaStream_t stream) {
   ClusterArgs a = {};
   a.D = D; a.L = L; a.N = N; a.H = H; a.A = 1;
   a.CL = 4 * H / 128;
@@ -1129,7 +1132,10 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
   CUtensorMap m[8];
   int rc;
-  if (dilated_flow_widths(dilations, D, N, a.CL, sm_count, a.nb)) {
+  const uint32_t cluster_smem = smem_for(any_self, H, 128, 32, 32, 4);
+  auto cut_for_clusters = [&] { return dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, cluster_smem), a.nb); };
+  int clusters = schedule == 4 || (schedule == 0 && dilated_prefers_clusters(N, a.CL)) ? cut_for_clusters() : 0;
+  if (clusters <= 0 && dilated_flow_widths(dilations, D, N, a.CL, sm_count, a.nb)) {
     a.flow = true;
     int narrow = 0;
     for (int l = 0; l < D; ++l) {
@@ -1167,8 +1173,8 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     if (dtype == FTB_F16) return launch_dilated_flow<__half>(narrow, dm, a, f, grid, smem, stream);
     return launch_dilated_flow<__nv_bfloat16>(narrow, dm, a, f, grid, smem, stream);
   }
-  const uint32_t smem = smem_for(any_self, H, 128, 32, 32, 4);
-  const int clusters = dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, smem), a.nb);
+  if (schedule == 5) return FTB_ERR_ARG;
+  if (clusters <= 0) clusters = cut_for_clusters();
   if (clusters <= 0) return FTB_ERR_LAUNCH;  // does not fit on this device: the caller's generic wavefront takes it
   a.S = (N + 63) / 64;
   for (int l = 0; l < D; ++l) a.first_cluster[l + 1] = a.first_cluster[l] + (N + a.nb[l] - 1) / a.nb[l];
@@ -1185,8 +1191,8 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   const size_t n_flags = static_cast<size_t>(D) * L * a.S;
   if (cudaMemsetAsync(flags, 0, sizeof(int) * n_flags, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
   const int grid = clusters * a.CL;
-  if (dtype == FTB_F16) return launch_dilated<__half>(m, a, grid, smem, stream);
-  return launch_dilated<__nv_bfloat16>(m, a, grid, smem, stream);
+  if (dtype == FTB_F16) return launch_dilated<__half>(m, a, grid, cluster_smem, stream);
+  return launch_dilated<__nv_bfloat16>(m, a, grid, cluster_smem, stream);
 }
 
 // --------------------------------------------------------------------- grid RNN

@@ -57,8 +57,8 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
 bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count);
 size_t lstm_dilated_cluster_flag_ints(int D, int L);
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
-                                const int* dilations, int D, int L, int N, int H, int* flags, int* status, int sm_count,
-                                cudaStream_t stream);
+                                const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
+                                int sm_count, cudaStream_t stream);
 bool grid_rnn_cluster_supported(int dtype, int D, int A, int B, int N, int H, int sm_count);
 int launch_grid_rnn_cluster(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy,
                             const float* bias_x, const float* bias_y, void* hx, void* hy, int D, int A, int B, int N,
@@ -956,21 +956,22 @@ int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, voi
     if (rc) return rc;
   }
 
-  // Cluster schedule (schedule 4, and the automatic choice when it applies): one thread-block
-  // cluster per (layer, batch slice), weights resident in tensor memory, the state of a layer with
-  // dilation 1 handed on through the cluster's shared memory.  Its flags sit behind the tables of
-  // the generic persistent schedule in the workspace.
+  // Schedules 4 and 5, and the automatic choice when one applies: a chain of CTAs per (layer, batch slice), weights
+  // resident in tensor memory, the state of a layer with dilation 1 handed on through the shared memory of a
+  // thread-block cluster (4) or, without clusters, through the output array (5).  Their counters sit behind the
+  // tables of the generic persistent schedule in the workspace.
   {
     const size_t flags_off = plan_layout(D * L, 0).total;
     const size_t need = flags_off + sizeof(int) * lstm_dilated_cluster_flag_ints(D, L);
     const bool can = lstm_dilated_cluster_supported(dtype, D, N, H, cl.sm_count) && tune.pair == 0 && bn == 0;
     if (tune.schedule == 4 && (!can || workspace_bytes < need)) return can ? FTB_ERR_WORKSPACE : FTB_ERR_ARG;
-    if ((tune.schedule == 4 || tune.schedule == 0) && can && workspace_bytes >= need) {
-      rc = launch_lstm_dilated_cluster(dtype, x, Wp, bias_p, hs, c, dilations, D, L, N, H,
+    if ((tune.schedule == 4 || tune.schedule == 5 || tune.schedule == 0) && can && workspace_bytes >= need) {
+      rc = launch_lstm_dilated_cluster(dtype, x, Wp, bias_p, hs, c, dilations, D, L, N, H, tune.schedule,
                                        reinterpret_cast<int*>(static_cast<char*>(workspace) + flags_off), status,
                                        cl.sm_count, stream);
-      // a refused cooperative cluster launch falls back to the generic wavefront
-      if (rc != FTB_ERR_LAUNCH || tune.schedule != 0) return rc;
+      // A refused cooperative launch falls back to the generic wavefront under the automatic choice, as does schedule 5
+      // where it does not apply.
+      if (rc != (tune.schedule == 5 ? FTB_ERR_ARG : FTB_ERR_LAUNCH) || tune.schedule == 4) return rc;
     }
   }
 

@@ -180,8 +180,9 @@ def lstm_stacked_varlen(x, active_rows, Wp, bias_p=None, hs=None, c=None, layers
 
 def lstm_dilated(x, Wp, dilations, bias_p=None, hs=None, c=None, bn=0, pair=0, schedule=0):
     """x: [L,N,H]; Wp: [D,4H,2H]; dilations: D ints -> (hs [D,L,N,H], c fp32 [D,max_dil*N,H]).
-    schedule: 0 auto, 1 one launch per level, 2 generic persistent kernel, 4 cluster kernel (H of 64, 128
-    or 256: weights resident in tensor memory, one thread-block cluster per layer and batch slice)."""
+    schedule: 0 auto, 1 one launch per level, 2 generic persistent kernel; H of 64, 128 or 256, weights resident in
+    tensor memory: 4 one thread-block cluster per layer and batch slice, 5 no clusters, states of layers with
+    dilation 1 through the output array."""
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)
     L, N, H = x.shape

@@ -149,12 +149,15 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
  * and DilatedLstmRegion1/2 (kaleido/core/device/kernels/lstm/dilated_lstm/region{1,2}.h).
  * x: [L,N,H]; hs (out): [D,L,N,H]; c (scratch/out): fp32 [D, max_dilation*N, H].
  * `dilations` is a HOST array of D ints.  With ftb_lstm_dilated_workspace_bytes(D, L) bytes of
- * workspace (16-bit dtypes) the whole forward pass is one launch.  For H of 64, 128 or 256 that is the
- * cluster schedule (tuning[2] = 4, and the automatic choice): one thread-block cluster per layer and
- * slice of 128 sequences, each CTA's slice of the weights resident in tensor memory for the whole
- * launch, the state of a layer with dilation 1 handed to its next step through the cluster's
- * shared memory.  Otherwise (or with tuning[2] = 2) it is the generic persistent wavefront, whose
- * schedule tables are copied from host memory on `stream`, so that form is not for stream capture.
+ * workspace (16-bit dtypes) the whole forward pass is one launch.  For H of 64, 128 or 256 that is one of
+ * two kernels that keep each CTA's slice of the weights in tensor memory for the whole launch, whichever
+ * is expected to be faster: tuning[2] = 4, one thread-block cluster per layer and slice of 64 or 128
+ * sequences, the state of a layer with dilation 1 handed to its next step through the cluster's shared
+ * memory (where the clusters do not fit on the device: 5); tuning[2] = 5, no clusters, the state of a
+ * layer with dilation 1 handed on through the output array in slices of 16, 32 or 48 sequences (needs
+ * such a layer and a CTA per SM for all slices; else as 2).  Otherwise (or with tuning[2] = 2) it is the
+ * generic persistent wavefront, whose schedule tables are copied from host memory on `stream`, so that
+ * form is not for stream capture.
  * All schedules give the same bits. */
 size_t ftb_lstm_dilated_workspace_bytes(int D, int L);
 int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,

@@ -24,6 +24,32 @@ def ops():
     (7, 90, 64, [1, 2]),
 ])
 def test_same_bits_as_levels(ops, dt, L, N, H, dils):
+    _against_levels(ops, dt, L, N, H, dils, 5)
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("L,N,H,dils", [
+    (9, 33, 128, [1]),              # the automatic choice at 2 and 4 CTAs and up to 64 sequences
+    (20, 64, 128, [1, 2, 4]),
+    (20, 64, 64, [1, 1, 2]),
+    (7, 5, 64, [1, 3]),
+    (12, 128, 256, [1, 2, 4]),      # 8 CTAs: state pieces for eight peers
+    (11, 256, 256, [1, 2, 4, 8]),   # slices of 64 below slices of 128
+    (9, 256, 256, [4, 1, 2]),       # slices of 128 below slices of 64
+    (6, 300, 128, [4, 1, 2]),       # partly filled slices
+])
+@pytest.mark.parametrize("schedule", [4, 0])
+def test_clusters_same_bits_as_levels(ops, dt, L, N, H, dils, schedule):
+    """One thread-block cluster per layer and slice (schedule 4), which the automatic choice takes for some of these."""
+    _against_levels(ops, dt, L, N, H, dils, schedule)
+
+
+def test_schedule_5_where_it_does_not_apply(ops):
+    """No layer of dilation 1: the generic persistent kernel, as for schedule 2."""
+    _against_levels(ops, torch.float16, 9, 40, 128, [2, 3], 5)
+
+
+def _against_levels(ops, dt, L, N, H, dils, schedule):
     D = len(dils)
     g = torch.Generator(device="cuda").manual_seed(N + L)
     u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
@@ -31,7 +57,7 @@ def test_same_bits_as_levels(ops, dt, L, N, H, dils):
     x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
     ref, ref_c = ops.lstm_dilated(x, Wp, dils, b, schedule=1)
     for _ in range(3):
-        h, c = ops.lstm_dilated(x, Wp, dils, b)
+        h, c = ops.lstm_dilated(x, Wp, dils, b, schedule=schedule)
         ops.check_status()
         assert torch.equal(h, ref)
         for l, d in enumerate(dils):
