@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "flow_plan.h"
 #include "lstm_flow.cuh"
 
 namespace ftb {
@@ -111,11 +112,6 @@ int input_slots(int nb, int I, int H, uint32_t* smem) {
 }  // namespace
 
 // How the kernel would run a problem; est_us: about what that takes.
-struct FlowPlan {
-  int nb, S, G;
-  double est_us;
-};
-
 bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, FlowPlan* plan) {
   if (dtype != FTB_F16 && dtype != FTB_BF16) return false;
   if (N < 1 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return false;

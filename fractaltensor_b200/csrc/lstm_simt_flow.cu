@@ -27,6 +27,7 @@
 // Cooperative launch: CTAs wait for each other's states.  That wait is bounded; when it runs out, or another
 // CTA has reported an error, the CTA goes through the rest of its steps without waiting for data.
 #include "../../include/ftb200.h"
+#include "flow_plan.h"
 #include "ptx.cuh"
 #include "tmap.h"
 
@@ -372,13 +373,7 @@ int launch(const SimtFlowArgs& a, size_t smem, cudaStream_t stream) {
 
 }  // namespace
 
-// How the kernel would run a problem: rows of a CTA's tile (8, 16 or 32); est_us: about what that takes.
-struct SimtFlowPlan {
-  int rows;
-  double est_us;
-};
-
-// False: not for this kernel.  Layers that do not fit on the device beside each other cost a sweep each.  Measured
+// How the kernel would run a problem; est_us: about what that takes.  False: not for this kernel.  Layers that do not fit on the device beside each other cost a sweep each.  Measured
 // steps, us, at H 64 / 128 / 192 / 256 / 320 / 384: 8 rows 2.7 / 2.9 / 3.1 / 3.2 / 4.3 / 4.5, 16 rows 3.4 / 3.4 / 3.7 /
 // 3.8 / 5.6 / 5.7, 32 rows 5.3 / 5.4 / 5.8 / 7.0.  A row of more than 256 is read in two rounds; 32 rows at H 256 leave
 // room for one input tile only.
@@ -402,9 +397,10 @@ bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFl
   return found;
 }
 
-// x: [L,N,H]; Wp: [D,4H,2H] fp32 packed; hs: [D,L,N,H]; c: [D,N,H]; tm: SimtFlowPlan::rows.
+// x: [L,N,H]; Wp: [D,4H,2H] fp32 packed; hs: [D,L,N,H]; c: [D,N,H]; plan: lstm_simt_flow_plan.
 int launch_lstm_simt_flow(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L, int N,
-                          int H, int tm, int* status, int sm_count, cudaStream_t stream) {
+                          int H, const SimtFlowPlan& plan, int* status, int sm_count, cudaStream_t stream) {
+  const int tm = plan.rows;
   SimtFlowArgs a;
   a.x = x;
   a.w = Wp;

@@ -598,7 +598,8 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
     // The example's key counts have a routine of their own, 1 to 4 random keys beside a window of up to 7 one
     // that is told the window's; the rest take the general one, which is issue-bound on its bookkeeping (us, B 2, 16 heads, S 4096, d 64, general /
     // told the window: window 7 and 4 random keys fp32 67.0 / 53.0, fp16 78.9 / 51.5; 5 and 2 48.4 / 44.4, 54.8 / 39.4;
-    // 3 and 1 34.9 / 30.9, 35.4 / 31.8; the example's 5 and 3 52.8 / 44.3 with its own).
+    // 3 and 1 34.9 / 30.9, 35.4 / 31.8; the example's 5 and 3, told the window / with its own: fp32 50.7 / 42.9, fp16 39.0 /
+    // 31.6, bf16 36.2 / 30.0).
     const Kernel kernels[6] = {sparse_attn_tile_kernel<T, LPT, 0, 0>, sparse_attn_tile_kernel<T, LPT, -7, 1>,
                                sparse_attn_tile_kernel<T, LPT, -7, 2>, sparse_attn_tile_kernel<T, LPT, -7, 3>,
                                sparse_attn_tile_kernel<T, LPT, -7, 4>, sparse_attn_tile_kernel<T, LPT, 5, 3>};

@@ -16,6 +16,7 @@
 
 #include "../../include/ftb200.h"
 #include "cell.h"
+#include "flow_plan.h"
 #include "ptx.cuh"
 #include "tmap.h"
 
@@ -27,13 +28,6 @@ int launch_cell_gemm(int dtype, int epi, int bn, int pair, const CUtensorMap* ma
 int launch_cell_gemm_persistent(int dtype, int epi, int bn, int pair, const CUtensorMap* maps,
                                 const CUtensorMap& mapW, const CUtensorMap& mapC, const CellBatch& header,
                                 const PlanView& plan, int* status, int sm_count, cudaStream_t stream);
-struct SimtFlowPlan {
-  int rows;
-  double est_us;
-};
-bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFlowPlan* plan);
-int launch_lstm_simt_flow(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L, int N,
-                          int H, int tm, int* status, int sm_count, cudaStream_t stream);
 bool lstm_simt_static_supported(int D, int N, int I, int H, int sm_count);
 double lstm_simt_static_us(int D, int L, int N, int I, int H, int sm_count);
 int launch_lstm_simt_static(const float* x, const float* Wp, const float* bias_p, float* hs, float* c, int D, int L,
@@ -46,14 +40,6 @@ bool lstm_wmajor_supported(int dtype, int D, int N, int I, int H, int G, int sm_
 int launch_lstm_wmajor(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, int D, int L,
                        int N, int I, int H, int G, int resident, int* done, int* status, unsigned long long* trace,
                        cudaStream_t stream);
-struct FlowPlan {
-  int nb, S, G;
-  double est_us;
-};
-bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, FlowPlan* plan);
-int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* off,
-                     int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
-                     cudaStream_t stream);
 bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count);
 size_t lstm_dilated_cluster_flag_ints(int D, int L);
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
@@ -578,7 +564,7 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
       const bool can_flow = lstm_simt_flow_plan(D, L, N, I, H, cl.sm_count, &flow);
       if (can_flow && (schedule == 5 || (schedule == 0 && flow.est_us < lstm_simt_static_us(D, L, N, I, H, cl.sm_count))))
         rc = launch_lstm_simt_flow(static_cast<const float*>(x), static_cast<const float*>(Wp), bias_p,
-                                   static_cast<float*>(hs), c, D, L, N, H, flow.rows, status, cl.sm_count, stream);
+                                   static_cast<float*>(hs), c, D, L, N, H, flow, status, cl.sm_count, stream);
       else
         rc = launch_lstm_simt_static(static_cast<const float*>(x), static_cast<const float*>(Wp), bias_p,
                                      static_cast<float*>(hs), c, D, L, N, I, H,
