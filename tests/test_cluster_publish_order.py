@@ -1,5 +1,8 @@
 """The count by which the cluster kernels' publisher knows that a step's output tile is whole
-(csrc/rnn_cluster.cu): on a model of it, with a warp held up as long as the kernel's waits allow."""
+(csrc/rnn_cluster.cu), on a model of that count alone, with a warp held up as long as the kernel's waits
+allow: why one count for all steps is not enough and one for each parity is.  The kernel itself is
+compared bit for bit with the level launches on a device (test_gpu_dilated_flow.py, clusters; the grid's
+in test_gpu_parity.py); an order of its warps that fails only rarely cannot be forced there."""
 import random
 
 import pytest
@@ -40,6 +43,7 @@ def test_one_count_is_not():
 
 
 def test_kernel_counts_by_parity():
+    """That the source keeps the count the model is of (nothing more)."""
     import os
     import fractaltensor_b200.build as b
     src = open(os.path.join(b.CSRC, "rnn_cluster.cu")).read()

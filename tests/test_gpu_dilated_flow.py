@@ -44,6 +44,23 @@ def test_clusters_same_bits_as_levels(ops, dt, L, N, H, dils, schedule):
     _against_levels(ops, dt, L, N, H, dils, schedule)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_nan_states_are_states(ops, dt):
+    """A NaN hidden state of a layer with dilation 1 is not the fill pattern: nothing waits for it."""
+    N, H, dils = 20, 64, [1, 2, 1]
+    g = torch.Generator(device="cuda").manual_seed(7)
+    u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+    Wp, b = ops.lstm_pack_weights(u(3, 4, H, H), u(3, 4, H, H), u(3, 4, H))
+    x = torch.randn(6, N, H, device="cuda", generator=g).to(dt)
+    x[2, 3] = float("nan")
+    x.view(torch.int16)[2, 4] = -1  # 0xFFFF: a NaN with the fill pattern's bits, as an input
+    ref, _ = ops.lstm_dilated(x, Wp, dils, b, schedule=1)
+    h, _ = ops.lstm_dilated(x, Wp, dils, b, schedule=5)
+    ops.check_status()
+    assert torch.isnan(h[:, 2:, 3:5]).any() and torch.equal(torch.isnan(h), torch.isnan(ref))
+    assert torch.equal(torch.nan_to_num(h), torch.nan_to_num(ref))
+
+
 def test_schedule_5_where_it_does_not_apply(ops):
     """No layer of dilation 1: the generic persistent kernel, as for schedule 2."""
     _against_levels(ops, torch.float16, 9, 40, 128, [2, 3], 5)

@@ -61,11 +61,12 @@ def test_ragged_same_bits_as_levels(ops, D, H, lens):
         assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
 
 
-def test_nan_states_are_states(ops):
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_nan_states_are_states(ops, dt):
     """A NaN hidden state is a value like any other (0x7FFF, not the fill pattern): nothing waits for it."""
     g = torch.Generator(device="cuda").manual_seed(7)
-    Wp, b = _params(ops, 2, 128, 128, torch.float16, g)
-    x = torch.randn(6, 5, 128, device="cuda", generator=g).half()
+    Wp, b = _params(ops, 2, 128, 128, dt, g)
+    x = torch.randn(6, 5, 128, device="cuda", generator=g).to(dt)
     x[2, 3] = float("nan")
     x.view(torch.int16)[2, 4] = -1  # 0xFFFF: a NaN with the fill pattern's bits, as an input
     h, _ = ops.lstm_stacked(x, Wp, b, schedule=5)
