@@ -81,6 +81,10 @@ class _NoHost:
 
     b2b_gemm = flash_attention = sparse_attention = _decline
 
+    @staticmethod
+    def current_stream(dev):
+        return torch.cuda.current_stream(dev if dev >= 0 else None).cuda_stream
+
 
 def _load_host():
     """The native front of the short calls.  It is built against one torch, and with another it must not be

@@ -56,11 +56,13 @@ bool get_float(PyObject* o, float* v) {
   return true;
 }
 
-// The workspace ops.py keeps for `dev` in its dictionary {device index: uint8 tensor}; undefined when
-// there is none yet or it is smaller than `bytes`.  (Held by value: another thread may put a larger one
-// in its place while this call runs.)
+void* stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
+
+// The workspace ops.py keeps for the current stream of `dev` in its dictionary {(device index, stream
+// handle): uint8 tensor}; undefined when there is none yet or it is smaller than `bytes`.  (Held by value:
+// another thread may put a larger one in its place while this call runs.)
 at::Tensor workspace_of(PyObject* dict, c10::DeviceIndex dev, size_t bytes) {
-  PyObject* key = PyLong_FromLong(dev);
+  PyObject* key = Py_BuildValue("(iK)", static_cast<int>(dev), reinterpret_cast<unsigned long long>(stream_of(dev)));
   PyObject* t = key != nullptr && PyDict_Check(dict) ? PyDict_GetItemWithError(dict, key) : nullptr;
   Py_XDECREF(key);
   if (t == nullptr) {
@@ -83,8 +85,6 @@ class WithoutGil {
  private:
   PyThreadState* state_;
 };
-
-void* stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
 
 // *o: `out` if the caller gave one, undefined for None; false when the given one does not fit.
 bool given_result(PyObject* out, const at::Tensor& like, at::IntArrayRef shape, at::Tensor* o) {
@@ -235,6 +235,22 @@ PyObject* sparse_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
+// (device index, -1: the current one) -> handle of its current stream.  (torch.cuda.current_stream makes a
+// stream object for it: 2 us, three times in a call of the word program.)
+PyObject* current_stream(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  int64_t dev;
+  if (n != 1 || !get_int(args[0], &dev) || dev < -1 || dev > 127) {
+    PyErr_SetString(PyExc_TypeError, "current_stream: expected a device index");
+    return nullptr;
+  }
+  try {
+    return PyLong_FromVoidPtr(stream_of(static_cast<c10::DeviceIndex>(dev)));
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
 template <typename F>
 PyCFunction as_method(F f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)); }
 
@@ -242,6 +258,7 @@ PyMethodDef kMethods[] = {
     {"b2b_gemm", as_method(b2b_gemm), METH_FASTCALL, nullptr},
     {"flash_attention", as_method(flash_attention), METH_FASTCALL, nullptr},
     {"sparse_attention", as_method(sparse_attention), METH_FASTCALL, nullptr},
+    {"current_stream", as_method(current_stream), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 

@@ -16,7 +16,9 @@ from ._lib import check, host, lib
 
 _DT = {torch.float32: _lib.DTYPE_F32, torch.float16: _lib.DTYPE_F16, torch.bfloat16: _lib.DTYPE_BF16}
 
-_workspaces = {}
+_workspaces = {}  # (device index, stream handle): uint8 tensor
+_MAX_WORKSPACES = 64
+_STATUS_BYTES = lib.ftb_workspace_bytes()
 
 
 def _dtype_code(t):
@@ -54,19 +56,32 @@ def _ptr(t):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(host.current_stream(-1))
 
 
 def workspace(device, nbytes=0):
-    """The per-device workspace handed to every call: the status word, plus the
-    schedule tables and completion counters of a persistent wavefront.  Grown on demand."""
-    key = torch.device(device).index
-    if key is None:
-        key = torch.cuda.current_device()
-    need = max(int(nbytes), lib.ftb_workspace_bytes())
+    """The workspace handed to every call: the status word, plus the schedule tables and completion
+    counters of a persistent wavefront.  One for each stream of a device, so that calls on several
+    streams do not meet; grown on demand.  A capture takes the largest one that the device has (a
+    tensor made while capturing would hold nothing before the graph's first replay), so that graphs
+    of stacked, dilated and grid calls must not be replayed at the same time."""
+    dev = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if dev is None:
+        dev = torch.cuda.current_device()
+    need = max(nbytes, _STATUS_BYTES)
+    key = (dev, host.current_stream(dev))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
-        ws = torch.zeros(need, dtype=torch.uint8, device=torch.device("cuda", key))
+        with torch.cuda.device(dev):
+            if torch.cuda.is_current_stream_capturing():
+                ws = max((w for k, w in list(_workspaces.items()) if k[0] == dev), key=torch.Tensor.numel, default=None)
+                if ws is not None and ws.numel() >= need:
+                    return ws
+            # (on the stream that uses it: what it replaces goes back to the allocator in that stream's order)
+            ws = torch.zeros(need, dtype=torch.uint8, device=torch.device("cuda", dev))
+        _workspaces.pop(key, None)
+        while len(_workspaces) >= _MAX_WORKSPACES:
+            _workspaces.pop(next(iter(list(_workspaces))), None)
         _workspaces[key] = ws
     return ws
 
@@ -78,13 +93,16 @@ def _tuning(layers_per_group=0, bn=0, schedule=0, skew=0, pair=0, fine_deps=0, r
 
 def check_status(device=None):
     """Synchronises the current stream and raises if a device wait ran out in
-    the last call on `device`."""
-    ws = workspace(device if device is not None else torch.cuda.current_device())
-    out = ctypes.c_int(0)
-    check(lib.ftb_read_status(_ptr(ws), ctypes.byref(out), _stream()), "ftb_read_status")
-    if out.value != 0:
-        ws[:8].zero_()  # the status word is sticky for some entry points: clear it for the next call
-    check(out.value, "device kernel")
+    the last call on `device`, on this stream or another."""
+    own = workspace(device if device is not None else torch.cuda.current_device())
+    failed = 0
+    for ws in [own] + [w for w in list(_workspaces.values()) if w.device == own.device and w is not own]:
+        out = ctypes.c_int(0)
+        check(lib.ftb_read_status(_ptr(ws), ctypes.byref(out), _stream()), "ftb_read_status")
+        if out.value != 0:
+            ws[:8].zero_()  # the status word is sticky for some entry points: clear it for the next call
+            failed = failed or out.value
+    check(failed, "device kernel")
 
 
 # ----------------------------------------------------------------------- LSTM

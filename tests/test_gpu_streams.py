@@ -53,3 +53,80 @@ def test_rnn_attention_on_two_streams():
     for one, other in zip(alone, both):
         assert all(torch.equal(a, b) for a, b in zip(one, other))
     ops.check_status()
+
+
+@pytest.mark.parametrize("program", ["stacked", "fp32", "ragged", "dilated", "grid"])
+def test_recurrent_programs_on_two_streams(program):
+    """Tables and counters of a call are in the workspace of its stream."""
+    from fractaltensor_b200 import ops
+
+    def call(seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        dt = torch.float32 if program == "fp32" else torch.float16
+        H, D, L, N = 128, 2, 24, 20
+        u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).to(dt)
+        r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dt)
+        if program == "grid":
+            X, Y = r(5, 6, N, H), r(5, 6, N, H)
+            Wx, Wy = (ops.grid_pack_weights(u(1, 2 * H, H), u(1, H, H)) for _ in range(2))
+            return lambda: ops.grid_rnn(X, Y, Wx, Wy)
+        Wp, b = ops.lstm_pack_weights(u(D, 4, H, H), u(D, 4, H, H), u(D, 4, H))
+        if program == "ragged":
+            active = [N] * 5 + [9] * 6 + [2] * 3
+            x = r(sum(active), H)
+            return lambda: ops.lstm_stacked_varlen(x, active, Wp, b)
+        x = r(L, N, H)
+        if program == "dilated":
+            return lambda: ops.lstm_dilated(x, Wp, [1, 2], b)[:1]
+        return lambda: ops.lstm_stacked(x, Wp, b)
+
+    calls = [call(s) for s in (1, 2)]
+    alone = [c() for c in calls]
+    both = _together(calls)
+    ops.check_status()
+    for one, other in zip(alone, both):
+        assert all(torch.equal(a, b) for a, b in zip(one, other))
+
+
+def test_workspaces_are_bounded_and_their_status_is_found(monkeypatch):
+    from fractaltensor_b200 import ops
+    from fractaltensor_b200._lib import FtbError
+    monkeypatch.setattr(ops, "_workspaces", {})
+    monkeypatch.setattr(ops, "_MAX_WORKSPACES", 3)
+    seen = []
+    for _ in range(5):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            seen.append(ops.workspace("cuda"))
+            assert ops.workspace("cuda") is seen[-1] and len(ops._workspaces) <= 3
+    assert len({w.data_ptr() for w in seen[-3:]}) == 3
+    torch.cuda.synchronize()
+    seen[-1][:4].view(torch.int32).fill_(22)  # as a call on that stream would leave it
+    torch.cuda.synchronize()
+    with pytest.raises(FtbError):
+        ops.check_status()
+    ops.check_status()  # cleared
+
+
+def test_the_handle_of_the_current_stream():
+    from fractaltensor_b200._lib import _NoHost, host
+    side = torch.cuda.Stream()
+    for stream in (torch.cuda.current_stream(), side):
+        with torch.cuda.stream(stream):
+            for h in (host, _NoHost):
+                assert h.current_stream(-1) == h.current_stream(0) == stream.cuda_stream
+
+
+def test_a_capture_takes_a_workspace_that_is_there():
+    from fractaltensor_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A, B, C = (torch.randn(s, device="cuda", generator=g).half() * 0.1 for s in ((1, 128, 64), (1, 128, 64), (1, 64, 128)))
+    ref = ops.b2b_gemm(A, B, C)
+    before = dict(ops._workspaces)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = ops.b2b_gemm(A, B, C)
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref) and ops._workspaces == before
