@@ -215,11 +215,6 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         blocks_ts(d_tmem, tmem_w + rec_t * 32, xd, in_t, 0u);
         blocks_ss(d_tmem, w_desc + static_cast<uint64_t>(((kb_h - rec_t) * kWBlockBytes) >> 4), xd + in_t * kBlockDesc,
                   kb_x - in_t, in_t > 0 ? 1u : 0u);
-        if (leader) umma_commit(&in_empty[slot]);
-        if (++slot == a.n_slots) {
-          slot = 0;
-          phase ^= 1u;
-        }
         if (t > 0) {
           ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           if (!ok) break;
@@ -228,6 +223,14 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           ++states;
         }
         if (leader) umma_commit(&acc_full[acc]);
+        // The input tile goes back behind the recurrent half, not before it: its next copy would otherwise be under way
+        // while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64 sequences:
+        // D8 L100 505 us, behind it 476).
+        if (leader) umma_commit(&in_empty[slot]);
+        if (++slot == a.n_slots) {
+          slot = 0;
+          phase ^= 1u;
+        }
       }
       if (ok && leader) umma_commit(&swept);
       ++sweep;
