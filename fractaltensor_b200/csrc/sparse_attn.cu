@@ -117,6 +117,17 @@ __device__ __forceinline__ void load_row_global(const T* __restrict__ row, int g
     unpack16(w, out + c * (kEPL / Pieces<T>::n), T());
   }
 }
+// The same in two steps, so that a row under way takes no more registers than its bytes.
+template <typename T, int LPT>
+__device__ __forceinline__ void request_row(const T* __restrict__ row, int gl, uint4 (&raw)[Pieces<T>::n]) {
+#pragma unroll
+  for (int c = 0; c < Pieces<T>::n; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(row) + c * LPT + gl);
+}
+template <typename T>
+__device__ __forceinline__ void unpack_row(const uint4 (&raw)[Pieces<T>::n], float (&out)[kEPL]) {
+#pragma unroll
+  for (int c = 0; c < Pieces<T>::n; ++c) unpack16(raw[c], out + c * (kEPL / Pieces<T>::n), T());
+}
 template <typename T, int LPT>
 __device__ __forceinline__ void load_row_shared(const T* row, int gl, float (&out)[kEPL]) {
 #pragma unroll
@@ -299,75 +310,6 @@ __device__ __forceinline__ void attend_token(const SparseArgs& a, const Rows<T>&
   store_row_global<T, LPT>(out_row, gl, acc);
 }
 
-// One token of an interior tile with the number of random keys known at compile time, and that of window keys
-// (KW > 0) or a bound on it (KW < 0: up to -KW): no per-key bookkeeping, one softmax over the scores.  Window rows
-// come from the stage, random rows from global memory; the random rows of K and V are requested
-// first, so that they arrive while the window part is computed out of shared memory.
-template <typename T, int LPT, int KW, int KR>
-__device__ __forceinline__ void attend_fast(const SparseArgs& a, const T* sk, const T* sv, int lo, const T* kh,
-                                            const T* vh, int i, int gl, unsigned gmask, const float (&qv)[kEPL],
-                                            const int* sp, T* __restrict__ out_row, int* __restrict__ status) {
-  constexpr int d = kEPL * LPT;
-  constexpr int NW = KW > 0 ? KW : -KW;
-  const int n_window = KW > 0 ? KW : a.window;
-  const int half = (n_window - 1) * a.dilation / 2;
-  const float scale2 = a.scale * 1.4426950408889634f;
-  float kr[KR][kEPL], vr[KR][kEPL];
-#pragma unroll
-  for (int r = 0; r < KR; ++r) {
-    int x = sp[r];
-    if (x < 0 || x >= a.S) {
-      if (gl == 0) atomicCAS(status, 0, FTB_ERR_INDEX);
-      x = 0;
-    }
-    load_row_global<T, LPT>(kh + static_cast<long long>(x) * d, gl, kr[r]);
-    load_row_global<T, LPT>(vh + static_cast<long long>(x) * d, gl, vr[r]);
-  }
-  float sc[NW + KR];
-  const int row0 = i - half - lo;  // the first window row inside the stage
-#pragma unroll
-  for (int j = 0; j < NW; ++j) {
-    if (KW < 0 && j >= n_window) {
-      sc[j] = -INFINITY;
-      continue;
-    }
-    float kw[kEPL];
-    load_row_shared<T, LPT>(sk + (row0 + j * a.dilation) * d, gl, kw);
-    sc[j] = group_dot<LPT>(qv, kw, gmask) * scale2;
-  }
-#pragma unroll
-  for (int r = 0; r < KR; ++r) sc[NW + r] = group_dot<LPT>(qv, kr[r], gmask) * scale2;
-  float m = sc[0];
-#pragma unroll
-  for (int j = 1; j < NW + KR; ++j) m = fmaxf(m, sc[j]);
-  float z = 0.f;
-#pragma unroll
-  for (int j = 0; j < NW + KR; ++j) {
-    sc[j] = exp2_fast(sc[j] - m);
-    z += sc[j];
-  }
-  float acc[kEPL];
-#pragma unroll
-  for (int e = 0; e < kEPL; ++e) acc[e] = 0.f;
-#pragma unroll
-  for (int j = 0; j < NW; ++j) {
-    if (KW < 0 && j >= n_window) continue;
-    float vw[kEPL];
-    load_row_shared<T, LPT>(sv + (row0 + j * a.dilation) * d, gl, vw);
-#pragma unroll
-    for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[j], vw[e], acc[e]);
-  }
-#pragma unroll
-  for (int r = 0; r < KR; ++r) {
-#pragma unroll
-    for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[NW + r], vr[r][e], acc[e]);
-  }
-  const float inv = 1.f / z;
-#pragma unroll
-  for (int e = 0; e < kEPL; ++e) acc[e] *= inv;
-  store_row_global<T, LPT>(out_row, gl, acc);
-}
-
 template <int LPT>
 __device__ __forceinline__ unsigned group_mask(int lane) {
   return LPT == 32 ? 0xffffffffu : (((1u << (LPT & 31)) - 1u) << (lane - lane % LPT));
@@ -412,16 +354,54 @@ sparse_attn_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
 }
 
 // ------------------------------------------------------------------ tiled kernel
-// The walk of one CTA over its work items: item number first, first + step, ... of the enumeration
-// (per_head, lead, skip).  it_base = tiles the CTA has walked before (the stages and barrier phases
-// carry on from there); returns that count plus the tiles of this walk, or -1 after a wait ran out.  KW != 0: the
-// items are interior tiles and a token has KW (up to -KW) window and KR random keys (attend_fast); KW = 0: any
-// tile, any key counts (attend_token).
-template <typename T, int LPT, int KW, int KR>
-__device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+// A tile: tokens t0 .. t0 + nt - 1 of a head and the key / value rows [lo, hi) that their windows touch.
+struct Tile {
+  long long head;
+  int t0, nt, lo, hi;
+};
+__device__ __forceinline__ Tile tile_of(const SparseArgs& a, int per_head, int lead, int skip, long long t) {
+  const int half = (a.window - 1) * a.dilation / 2;
+  Tile x;
+  x.head = t / per_head;
+  const int idx = static_cast<int>(t - x.head * per_head);
+  x.t0 = (idx < lead ? idx : idx + skip) * a.TT;
+  x.nt = min(a.TT, a.S - x.t0);
+  x.lo = max(0, x.t0 - half);
+  x.hi = min(a.S, x.t0 + x.nt + half);
+  return x;
+}
+// Stage s: K rows, V rows, queries, positions.
+template <typename T>
+struct Stage {
+  T *k, *v, *q;
+  int* pos;
+  __device__ __forceinline__ Stage(unsigned char* smem, const SparseArgs& a, int d, int s) {
+    const int rows_max = a.TT + (a.window - 1) * a.dilation / 2 * 2;
+    k = reinterpret_cast<T*>(smem + static_cast<size_t>(s) * a.stage_bytes);
+    v = k + static_cast<size_t>(rows_max) * d;
+    q = v + static_cast<size_t>(rows_max) * d;
+    pos = reinterpret_cast<int*>(q + static_cast<size_t>(a.TT) * d);
+  }
+};
+// One thread: the three bulk copies of a tile into a stage.
+template <typename T>
+__device__ __forceinline__ void copy_tile(const T* q, const T* k, const T* v, const SparseArgs& a, int d, const Tile& x,
+                                          const Stage<T>& st, uint64_t* full) {
+  const uint32_t kv_bytes = static_cast<uint32_t>(x.hi - x.lo) * d * sizeof(T);
+  const uint32_t q_bytes = static_cast<uint32_t>(x.nt) * d * sizeof(T);
+  mbar_arrive_expect_tx(full, 2 * kv_bytes + q_bytes);
+  bulk_load_1d(st.k, k + (x.head * a.S + x.lo) * d, kv_bytes, full);
+  bulk_load_1d(st.v, v + (x.head * a.S + x.lo) * d, kv_bytes, full);
+  bulk_load_1d(st.q, q + (x.head * a.S + x.t0) * d, q_bytes, full);
+}
+
+// The walk of one CTA over its work items with the general routine: item number first, first + step, ... of the
+// enumeration (per_head, lead, skip); any tile, any key counts.
+template <typename T, int LPT>
+__device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                           const int* __restrict__ rand_pos, T* __restrict__ o, const SparseArgs& a,
                                           int per_head, int lead, int skip, long long first, long long step,
-                                          int it_base, unsigned char* smem, uint64_t* full, int* s_abort_p,
+                                          unsigned char* smem, uint64_t* full, int* s_abort_p,
                                           int* __restrict__ status) {
   constexpr int d = kEPL * LPT;
   constexpr int TPW = 32 / LPT;
@@ -431,37 +411,7 @@ __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __re
   const unsigned gmask = group_mask<LPT>(lane);
   const int S = a.S, ng = a.n_global, G = 2 * a.n_global, TT = a.TT;
   const int half = (a.window - 1) * a.dilation / 2;
-  const int rows_max = TT + 2 * half;
   const long long n_tiles = a.heads_total * per_head;  // work items of this enumeration
-
-  auto stage_k = [&](int s) { return reinterpret_cast<T*>(smem + static_cast<size_t>(s) * a.stage_bytes); };
-  auto stage_v = [&](int s) { return stage_k(s) + static_cast<size_t>(rows_max) * d; };
-  auto stage_q = [&](int s) { return stage_v(s) + static_cast<size_t>(rows_max) * d; };
-  auto stage_pos = [&](int s) { return reinterpret_cast<int*>(stage_q(s) + static_cast<size_t>(TT) * d); };
-
-  struct Tile {
-    long long head;
-    int t0, nt, lo, hi;
-  };
-  auto tile_of = [&](long long t) {
-    Tile x;
-    x.head = t / per_head;
-    const int idx = static_cast<int>(t - x.head * per_head);
-    x.t0 = (idx < lead ? idx : idx + skip) * TT;
-    x.nt = min(TT, S - x.t0);
-    x.lo = max(0, x.t0 - half);
-    x.hi = min(S, x.t0 + x.nt + half);
-    return x;
-  };
-  // Thread 0: the three bulk copies of a tile into stage s.
-  auto issue = [&](const Tile& x, int s) {
-    const uint32_t kv_bytes = static_cast<uint32_t>(x.hi - x.lo) * d * sizeof(T);
-    const uint32_t q_bytes = static_cast<uint32_t>(x.nt) * d * sizeof(T);
-    mbar_arrive_expect_tx(&full[s], 2 * kv_bytes + q_bytes);
-    bulk_load_1d(stage_k(s), k + (x.head * S + x.lo) * d, kv_bytes, &full[s]);
-    bulk_load_1d(stage_v(s), v + (x.head * S + x.lo) * d, kv_bytes, &full[s]);
-    bulk_load_1d(stage_q(s), q + (x.head * S + x.t0) * d, q_bytes, &full[s]);
-  };
   // Every thread: its share of the tile's random positions (entry e = token * R + r of the tile).
   auto fetch_pos = [&](const Tile& x, int (&pre)[kPosRegs]) {
 #pragma unroll
@@ -476,66 +426,220 @@ __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __re
     }
   };
   auto park_pos = [&](int s, const int (&pre)[kPosRegs]) {
+    const Stage<T> st(smem, a, d, s);
 #pragma unroll
     for (int u = 0; u < kPosRegs; ++u) {
       const int e = tid + u * kSparseThreads;
-      if (e < TT * a.R) stage_pos(s)[e] = pre[u];
+      if (e < TT * a.R) st.pos[e] = pre[u];
     }
   };
 
   long long tile = first;
-  if (tile >= n_tiles) return it_base;
+  if (tile >= n_tiles) return;
   {
-    const Tile x = tile_of(tile);
-    if (tid == 0) issue(x, it_base & 1);
+    const Tile x = tile_of(a, per_head, lead, skip, tile);
+    if (tid == 0) copy_tile(q, k, v, a, d, x, Stage<T>(smem, a, d, 0), &full[0]);
     int pre[kPosRegs];
     fetch_pos(x, pre);
-    park_pos(it_base & 1, pre);
+    park_pos(0, pre);
   }
   __syncthreads();
 
-  int it = it_base;
-  for (; tile < n_tiles; tile += step, ++it) {
+  for (int it = 0; tile < n_tiles; tile += step, ++it) {
     const int s = it & 1;
-    const Tile x = tile_of(tile);
+    const Tile x = tile_of(a, per_head, lead, skip, tile);
+    const Stage<T> st(smem, a, d, s);
     const long long next = tile + step;
     int pre[kPosRegs];
     if (next < n_tiles) {
       // stage s ^ 1 was last read in the previous round; the barrier that closed it orders those
       // reads before these writes
-      const Tile y = tile_of(next);
-      if (tid == 0) issue(y, s ^ 1);
+      const Tile y = tile_of(a, per_head, lead, skip, next);
+      if (tid == 0) copy_tile(q, k, v, a, d, y, Stage<T>(smem, a, d, s ^ 1), &full[s ^ 1]);
       fetch_pos(y, pre);
     }
-    if (!mbar_wait(&full[s], (it >> 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_TMA)) return -1;
+    const bool ok = mbar_wait(&full[s], (it >> 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_TMA);
 
     Rows<T> rw;
     rw.kh = k + x.head * S * d;
     rw.vh = v + x.head * S * d;
     rw.qh = q + x.head * S * d;
-    rw.sk = stage_k(s);
-    rw.sv = stage_v(s);
+    rw.sk = st.k;
+    rw.sv = st.v;
     rw.lo = x.lo;
     rw.hi = x.hi;
-    const int* sp = stage_pos(s);
     // no global token in the tile and no window position that wraps
     const bool interior = x.t0 >= ng && x.t0 + x.nt <= S - ng && x.t0 - half >= 0 && x.t0 + x.nt - 1 + half < S;
-    for (int tok = (tid >> 5) * TPW + lane / LPT; tok < x.nt; tok += (kSparseThreads / 32) * TPW) {
+    for (int tok = (tid >> 5) * TPW + lane / LPT; tok < x.nt && ok; tok += (kSparseThreads / 32) * TPW) {
       const int i = x.t0 + tok;
       float qv[kEPL];
-      load_row_shared<T, LPT>(stage_q(s) + tok * d, gl, qv);
-      if constexpr (KW != 0) {
-        attend_fast<T, LPT, KW, KR>(a, rw.sk, rw.sv, x.lo, rw.kh, rw.vh, i, gl, gmask, qv, sp + tok * KR,
-                                    o + (x.head * S + i) * d, status);
-      } else {
-        attend_token<T, LPT>(a, rw, i, gl, gmask, interior, qv, [&](int r) { return sp[tok * a.R + r]; },
-                             o + (x.head * S + i) * d, status);
-      }
+      load_row_shared<T, LPT>(st.q + tok * d, gl, qv);
+      attend_token<T, LPT>(a, rw, i, gl, gmask, interior, qv, [&](int r) { return st.pos[tok * a.R + r]; },
+                           o + (x.head * S + i) * d, status);
     }
     if (next < n_tiles) park_pos(s ^ 1, pre);
     __syncthreads();
+    if (*s_abort != 0) return;  // (set before the barrier: every thread leaves here)
   }
-  return it;
+}
+
+// The walk of one warp over interior tiles (no global token, no wrapped window position), with the number of random
+// keys known at compile time, and that of window keys (KW > 0) or a bound on it (KW < 0: up to -KW): no per-key
+// bookkeeping, one softmax over the scores.  Window rows and queries come from the stage, random rows from global
+// memory.
+//   What bounds it is the latency of the random rows: 6 rows of 256 bytes a token at the example's counts, with 16
+// warps an SM.  So a warp works one pass (32 / LPT tokens) ahead of itself: the random keys of its next pass are
+// requested into the registers that the scores of this one have just freed, the random values behind the
+// weighted sum, and the positions of the pass after that behind them.  And warps do not wait for one another:
+// the last warp that has read a stage fills it with the tile after the next.  (B 2, 16 heads, S 4096, d 64, the example's
+// counts, fp32: 44.8 us with a pass's rows requested at its beginning and a barrier of the CTA a tile, 41.8 so.)
+template <typename T, int LPT, int KW, int KR>
+__device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                                              const int* __restrict__ rand_pos, T* __restrict__ o, const SparseArgs& a,
+                                              unsigned char* smem, uint64_t* full, int* n_read, int* s_abort_p,
+                                              int* __restrict__ status) {
+  constexpr int d = kEPL * LPT, TPW = 32 / LPT, NW = KW > 0 ? KW : -KW;
+  constexpr int kTokens = kSparseThreads / 32 * TPW;  // of a pass of the CTA
+  volatile int* s_abort = s_abort_p;
+  const int lane = threadIdx.x & 31, gl = lane % LPT, mine = (threadIdx.x >> 5) * TPW + lane / LPT;
+  const unsigned gmask = group_mask<LPT>(lane);
+  const int n_window = KW > 0 ? KW : a.window;
+  const int half = (n_window - 1) * a.dilation / 2;
+  const float scale2 = a.scale * 1.4426950408889634f;
+  const long long n_tiles = a.heads_total * a.per_head;
+
+  // A pass: its tile and this lane's token in it.  Lanes behind the tile's last token repeat that one and store nothing.
+  struct Pass {
+    long long tile;
+    Tile x;
+    int tok;
+  };
+  auto next_pass = [&](Pass& p) {
+    p.tok += kTokens;
+    if (p.tok - mine < p.x.nt) return;
+    p.tok = mine;
+    p.tile += gridDim.x;
+    if (p.tile < n_tiles) p.x = tile_of(a, a.per_head, a.lead, a.skip, p.tile);
+  };
+  auto request_positions = [&](const Pass& p, int (&x)[KR]) {
+    if (p.tile >= n_tiles) return;
+    const int i = p.x.t0 + min(p.tok, p.x.nt - 1);
+    const int* at = rand_pos + (p.x.head * (a.S - 2 * a.n_global) + (i - a.n_global)) * KR;
+#pragma unroll
+    for (int r = 0; r < KR; ++r) x[r] = __ldg(at + r);
+  };
+  auto check_positions = [&](int (&x)[KR]) {
+#pragma unroll
+    for (int r = 0; r < KR; ++r)
+      if (x[r] < 0 || x[r] >= a.S) {
+        if (gl == 0) atomicCAS(status, 0, FTB_ERR_INDEX);
+        x[r] = 0;
+      }
+  };
+  auto request = [&](const Pass& p, const T* rows, const int (&x)[KR], uint4 (&raw)[KR][Pieces<T>::n]) {
+    if (p.tile >= n_tiles) return;
+    const T* head = rows + p.x.head * a.S * d;
+#pragma unroll
+    for (int r = 0; r < KR; ++r) request_row<T, LPT>(head + static_cast<long long>(x[r]) * d, gl, raw[r]);
+  };
+
+  Pass now;
+  now.tile = blockIdx.x;
+  if (now.tile >= n_tiles) return;
+  now.x = tile_of(a, a.per_head, a.lead, a.skip, now.tile);
+  now.tok = mine;
+  if (threadIdx.x == 0) {
+    copy_tile(q, k, v, a, d, now.x, Stage<T>(smem, a, d, 0), &full[0]);
+    if (now.tile + gridDim.x < n_tiles)
+      copy_tile(q, k, v, a, d, tile_of(a, a.per_head, a.lead, a.skip, now.tile + gridDim.x), Stage<T>(smem, a, d, 1), &full[1]);
+  }
+  Pass next = now;
+  int pos[KR];  // of the pass `next`
+  uint4 kr[KR][Pieces<T>::n], vr[KR][Pieces<T>::n];
+  request_positions(next, pos);
+  check_positions(pos);
+  request(next, k, pos, kr);
+  request(next, v, pos, vr);
+  next_pass(next);
+  request_positions(next, pos);
+
+  for (int it = 0; now.tile < n_tiles; ++it) {
+    const int s = it & 1;
+    const Stage<T> st(smem, a, d, s);
+    const Tile x = now.x;
+    const bool ok = mbar_wait(&full[s], (it >> 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_TMA);
+    if (!__all_sync(0xffffffffu, ok)) return;
+    for (int t0 = 0; t0 < x.nt; t0 += kTokens) {
+      const int tok = min(t0 + mine, x.nt - 1);
+      const int row0 = x.t0 + tok - half - x.lo;  // the first window row inside the stage
+      float qv[kEPL];
+      load_row_shared<T, LPT>(st.q + tok * d, gl, qv);
+      float sc[NW + KR];
+#pragma unroll
+      for (int j = 0; j < NW; ++j) {
+        if (KW < 0 && j >= n_window) {
+          sc[j] = -INFINITY;
+          continue;
+        }
+        float kw[kEPL];
+        load_row_shared<T, LPT>(st.k + (row0 + j * a.dilation) * d, gl, kw);
+        sc[j] = group_dot<LPT>(qv, kw, gmask) * scale2;
+      }
+#pragma unroll
+      for (int r = 0; r < KR; ++r) {
+        float kx[kEPL];
+        unpack_row<T>(kr[r], kx);
+        sc[NW + r] = group_dot<LPT>(qv, kx, gmask) * scale2;
+      }
+      if (next.tile < n_tiles) check_positions(pos);
+      request(next, k, pos, kr);
+      float m = sc[0];
+#pragma unroll
+      for (int j = 1; j < NW + KR; ++j) m = fmaxf(m, sc[j]);
+      float z = 0.f;
+#pragma unroll
+      for (int j = 0; j < NW + KR; ++j) {
+        sc[j] = exp2_fast(sc[j] - m);
+        z += sc[j];
+      }
+      float acc[kEPL];
+#pragma unroll
+      for (int e = 0; e < kEPL; ++e) acc[e] = 0.f;
+#pragma unroll
+      for (int j = 0; j < NW; ++j) {
+        if (KW < 0 && j >= n_window) continue;
+        float vw[kEPL];
+        load_row_shared<T, LPT>(st.v + (row0 + j * a.dilation) * d, gl, vw);
+#pragma unroll
+        for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[j], vw[e], acc[e]);
+      }
+#pragma unroll
+      for (int r = 0; r < KR; ++r) {
+        float vx[kEPL];
+        unpack_row<T>(vr[r], vx);
+#pragma unroll
+        for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[NW + r], vx[e], acc[e]);
+      }
+      request(next, v, pos, vr);
+      next_pass(next);
+      request_positions(next, pos);
+      const float inv = 1.f / z;
+#pragma unroll
+      for (int e = 0; e < kEPL; ++e) acc[e] *= inv;
+      if (t0 + mine < x.nt) store_row_global<T, LPT>(o + (x.head * a.S + x.t0 + tok) * d, gl, acc);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence_block();
+      const bool last = atomicAdd(&n_read[s], 1) % (kSparseThreads / 32) == kSparseThreads / 32 - 1;
+      __threadfence_block();
+      const long long after = now.tile + 2 * static_cast<long long>(gridDim.x);
+      if (last && after < n_tiles) copy_tile(q, k, v, a, d, tile_of(a, a.per_head, a.lead, a.skip, after), st, &full[s]);
+    }
+    __syncwarp();
+    now.tile += gridDim.x;
+    if (now.tile < n_tiles) now.x = tile_of(a, a.per_head, a.lead, a.skip, now.tile);
+  }
 }
 
 // ------------------------------------------------------------------ tiled kernel
@@ -544,15 +648,19 @@ __device__ __forceinline__ int walk_tiles(const T* __restrict__ q, const T* __re
 // interior tiles with the routine built for its key counts; the two walks are separate
 // pieces of code, so the register count is the larger of the two, not their sum.
 template <typename T, int LPT, int KW, int KR>
-__global__ void __launch_bounds__(kSparseThreads)
+__global__ void __launch_bounds__(kSparseThreads, 2)
 sparse_attn_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                         const int* __restrict__ rand_pos, T* __restrict__ o, SparseArgs a, int* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[2];
+  __shared__ __align__(8) uint64_t full[2], interior_full[2];
+  __shared__ int n_read[2];
   __shared__ int s_abort;
   if (threadIdx.x == 0) {
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&interior_full[s], 1);
+      n_read[s] = 0;
+    }
     s_abort = 0;
     fence_barrier_init();
   }
@@ -562,14 +670,14 @@ sparse_attn_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   if constexpr (KW != 0) {
     // Edge tiles are handed out from the last CTA down, interior tiles from the first up: when the
     // edge tiles are fewer than the CTAs, the CTAs with one interior tile more do not get them.
-    const int done = walk_tiles<T, LPT, 0, 0>(q, k, v, rand_pos, o, a, a.edge_per_head, a.edge_lead, a.edge_skip,
-                                              gridDim.x - 1 - blockIdx.x, gridDim.x, 0, smem, full, &s_abort, status);
-    if (done >= 0)
-      walk_tiles<T, LPT, KW, KR>(q, k, v, rand_pos, o, a, a.per_head, a.lead, a.skip, blockIdx.x, gridDim.x, done,
-                                 smem, full, &s_abort, status);
+    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.edge_per_head, a.edge_lead, a.edge_skip, gridDim.x - 1 - blockIdx.x,
+                       gridDim.x, smem, full, &s_abort, status);
+    // (behind its last barrier: every warp has left the stages, and sees s_abort alike)
+    if (s_abort == 0)
+      walk_interior<T, LPT, KW, KR>(q, k, v, rand_pos, o, a, smem, interior_full, n_read, &s_abort, status);
   } else {
-    walk_tiles<T, LPT, 0, 0>(q, k, v, rand_pos, o, a, a.per_head, a.lead, a.skip, blockIdx.x, gridDim.x, 0, smem, full,
-                             &s_abort, status);
+    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.per_head, a.lead, a.skip, blockIdx.x, gridDim.x, smem, full, &s_abort,
+                       status);
   }
 }
 

@@ -171,3 +171,45 @@ def test_sparse_attention_empty_batch_and_single_tile_edges(ops):
 ])
 def test_sparse_attention_key_counts(ops, dt, case):
     test_sparse_attention_matches_oracle(ops, dt, False, case)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,heads,S,d,window,dilation,ng,R", [
+    (1, 1, 200, 32, 5, 2, 3, 3),       # one interior tile and a last one that is not full
+    (2, 5, 333, 64, 7, 3, 1, 4),       # the most keys of the routine
+    (1, 3, 1000, 128, 3, 1, 4, 1),
+    (1, 40, 1500, 64, 5, 2, 3, 3),     # more tiles than CTAs: stages filled behind the last warp that has read them
+    (1, 70, 700, 128, 5, 1, 2, 2),
+    (1, 2, 130, 256, 1, 1, 0, 2),      # no global token, no window beyond the token itself
+])
+def test_interior_walk_matches_oracle(ops, dt, B, heads, S, d, window, dilation, ng, R):
+    """Tiles of 1 to 4 random keys and windows up to 7 (positions and random rows requested a pass ahead) against the
+    oracle, random positions at both ends of the sequence among them."""
+    q, k, v, pos = _inputs(B, heads, S, d, ng, R, S + d, dt)
+    pos[..., 0].view(-1)[::7] = 0
+    pos[..., -1].view(-1)[::5] = S - 1
+    sc = 1.0 / d ** 0.5
+    out = ops.sparse_attention(q.cuda(), k.cuda(), v.cuda(), pos.cuda(), window, dilation, ng, sc)
+    ops.check_status()
+    for b, h in {(0, 0), (B - 1, heads - 1)}:
+        ref = dense.sparse_attention_dense(q[b, h].double() * sc, k[b, h].double(), v[b, h].double(), pos[b, h], window, dilation, ng)
+        assert (out[b, h].cpu().double() - ref).abs().max().item() <= (1e-5 if dt == torch.float32 else 1e-2)
+    # every head is the program of that head alone
+    one = ops.sparse_attention(q[-1:, -1:].cuda(), k[-1:, -1:].cuda(), v[-1:, -1:].cuda(), pos[-1:, -1:].cuda(), window,
+                               dilation, ng, sc)
+    assert torch.equal(one[0, 0], out[-1, -1])
+
+
+def test_interior_walk_reports_positions_outside(ops):
+    from fractaltensor_b200._lib import FtbError
+    q, k, v, pos = _inputs(1, 2, 512, 64, 3, 3, 4, torch.float32)
+    good = ops.sparse_attention(q.cuda(), k.cuda(), v.cuda(), pos.cuda(), 5, 2, 3, 1.0)
+    ops.check_status()
+    bad = pos.clone()
+    bad[0, 1, 250, 1] = 512
+    out = ops.sparse_attention(q.cuda(), k.cuda(), v.cuda(), bad.cuda(), 5, 2, 3, 1.0)
+    with pytest.raises(FtbError):
+        ops.check_status()
+    same = torch.ones(512, dtype=torch.bool)
+    same[253] = False
+    assert torch.equal(out[0, 0], good[0, 0]) and torch.equal(out[0, 1][same.cuda()], good[0, 1][same.cuda()])
