@@ -10,17 +10,19 @@
 // decoder step and are computed once per call, and the softmax-weighted sums of the encoder rows.
 //
 // The decoder adds the same number to every score of a step, and a softmax does not change when all
-// its scores move by one number: v_t is the softmax-weighted sum over e_j @ encoder_proj alone.  So
-// the recurrent input of every decoder cell is known as soon as the encoder is done, and the
-// decoder, a chain of Lt cells and Lt attention steps as written, runs as one matrix product over all
-// steps followed by one launch of the attention over all steps (ftb_rnn_attention_fwd).  Only a number that
-// is not finite does not cancel: it makes every weight of its step NaN, and in the chain every later step
-// of the sequence.  carry_nan_kernel, one warp a sequence behind the attention, does that (2 us of the call).
+// its scores move by one number: v_t is the softmax-weighted sum over e_j @ encoder_proj alone, one
+// vector a sequence.  So the recurrent input of every decoder cell is known as soon as the encoder is
+// done, and the decoder, a chain of Lt cells and Lt attention steps as written, is one launch that puts
+// the vector of every sequence into the rows of its steps (attn_vector_kernel), one matrix product over
+// all steps, and one launch that looks at the decoder's terms (attn_finish_kernel).  Only a term that is
+// not finite does not cancel: it makes every weight of its step NaN, and in the chain every later step
+// of the sequence.
 //
 // Layout: time-major padded batches, row (j, n) of `enc` at (j * N + n) * H.  Sequence n attends to
-// encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: per
-// decoder step and sequence the kernel reads len * H encoder elements (they stay in L2 across the
-// steps) and writes H.
+// encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: len * H encoder
+// elements a sequence in (twice: for the scores and for the sum), Lt * H out; then Lt * H decoder elements in.
+// With the scores in a launch of their own and the weights and sums anew for every step, the whole program (H 512, 64
+// sequences, 50 + 50 positions, bf16) took 155.8 us; as here 114.9.
 #include "../../include/ftb200.h"
 #include "ptx.cuh"
 #include "tmap.h"
@@ -31,8 +33,8 @@
 namespace ftb {
 namespace {
 
-constexpr int kStepThreads = 128;  // one output column per thread
-constexpr int kCarryThreads = 128;
+constexpr int kAttnThreads = 256;
+constexpr int kAttnCols = 128;  // output columns of a CTA
 
 template <typename T> __device__ __forceinline__ float ld_f32(const T* p);
 template <> __device__ __forceinline__ float ld_f32<float>(const float* p) { return __ldg(p); }
@@ -54,72 +56,96 @@ __device__ __forceinline__ float warp_max(float x) {
   return x;
 }
 
-// scores[r] = rows[r, :] . proj for r < n_rows: one warp per row.
+// 16 bytes of a row as fp32 numbers.
 template <typename T>
-__global__ void __launch_bounds__(256)
-row_dot_kernel(const T* __restrict__ rows, const T* __restrict__ proj, float* __restrict__ scores, long long n_rows,
-               int H) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long n_warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  grid_launch_dependents();
-  grid_dependency_wait();  // the encoder's last level wrote the rows
-  for (long long r = warp; r < n_rows; r += n_warps) {
-    float s = 0.f;
-    for (int h = lane; h < H; h += 32) s = fmaf(ld_f32<T>(rows + r * H + h), ld_f32<T>(proj + h), s);
-    s = warp_sum(s);
-    if (lane == 0) scores[r] = s;
-  }
+struct Piece {
+  static constexpr int n = 16 / sizeof(T);
+};
+__device__ __forceinline__ void ld_piece(const float* p, float (&v)[4]) {
+  const float4 x = *reinterpret_cast<const float4*>(p);
+  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+template <typename T>
+__device__ __forceinline__ void ld_piece(const T* p, float (&v)[8]) {
+  const uint4 x = *reinterpret_cast<const uint4*>(p);
+  const T* e = reinterpret_cast<const T*>(&x);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = ld_f32<T>(e + i);
 }
 
-// Attention vectors.  grid = (N, ceil(H / 128), steps); CTA (n, cb, t) computes columns cb * 128 .. of
-// v_t for sequence n from the decoder states dec [Lt, N, H] of its step.  dec == nullptr: the scores
-// of the encoder alone, and the one result goes to the rows of `copies` steps (the recurrent inputs of
-// the decoder cells).  Every CTA of a sequence recomputes the len weights (a dot product over H and a
-// softmax over len numbers: small next to the len x 128 weighted sum).
+// The dot products of up to kDots rows, `stride` elements apart, with proj (of any alignment): a warp's work; every
+// lane gets them.
+constexpr int kDots = 4;
 template <typename T>
-__global__ void __launch_bounds__(kStepThreads)
-attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores, const T* __restrict__ dec,
-                 const T* __restrict__ dec_proj, const int* __restrict__ src_lens, T* __restrict__ out, int copies,
-                 int Ls, int N, int H) {
+__device__ __forceinline__ void row_dots(const T* rows, long long stride, int count, const T* proj, int H, int lane,
+                                         float (&s)[kDots]) {
+  constexpr int n = Piece<T>::n;
+#pragma unroll
+  for (int r = 0; r < kDots; ++r) s[r] = 0.f;
+  for (int h = lane * n; h < H; h += 32 * n) {
+    float p[n];
+#pragma unroll
+    for (int i = 0; i < n; ++i) p[i] = ld_f32<T>(proj + h + i);
+#pragma unroll
+    for (int r = 0; r < kDots; ++r) {
+      if (r >= count) continue;
+      float x[n];
+      ld_piece(rows + r * stride + h, x);
+#pragma unroll
+      for (int i = 0; i < n; ++i) s[r] = fmaf(x[i], p[i], s[r]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kDots; ++r) s[r] = warp_sum(s[r]);
+}
+
+__device__ __forceinline__ int source_len(const int* src_lens, int n, int Ls) {
+  const int len = src_lens ? src_lens[n] : Ls;
+  return len < 0 ? 0 : (len > Ls ? Ls : len);
+}
+
+// The attention vector of sequence blockIdx.x, columns 128 * blockIdx.y .., into the rows of all Lt steps; the scores
+// into `scores` [Ls, N].  The CTAs of a sequence compute its len scores each for itself.  Latency: a chain of reads
+// of the encoder's rows for the scores, two reductions over the CTA, and reads of the rows again (from L2) for the sum.
+template <typename T>
+__global__ void __launch_bounds__(kAttnThreads)
+attn_vector_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, const int* __restrict__ src_lens,
+                   float* __restrict__ scores, T* __restrict__ out, int Lt, int Ls, int N, int H) {
+  constexpr int kN = Piece<T>::n, kColGroups = kAttnCols / kN, kRowGroups = kAttnThreads / kColGroups;
+  constexpr int kWarps = kAttnThreads / 32;
   extern __shared__ float s_w[];  // [Ls] scores, then weights
-  __shared__ float s_red[kStepThreads / 32];
+  __shared__ float s_red[kWarps];
+  __shared__ float s_part[kRowGroups][kAttnCols];
+  __shared__ __align__(16) T s_out[kAttnCols];
   const int n = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const long long step_elems = static_cast<long long>(N) * H;
-  const T* dec_t = dec == nullptr ? nullptr : dec + blockIdx.z * step_elems + static_cast<long long>(n) * H;
+  const T* mine = enc + static_cast<long long>(n) * H;
   grid_launch_dependents();
   grid_dependency_wait();
-  int len = src_lens ? src_lens[n] : Ls;
-  len = len < 0 ? 0 : (len > Ls ? Ls : len);
+  const int len = source_len(src_lens, n, Ls);
 
-  // c = decoder . decoder_proj
-  float part = 0.f;
-  if (dec_t != nullptr)
-    for (int h = tid; h < H; h += kStepThreads) part = fmaf(ld_f32<T>(dec_t + h), ld_f32<T>(dec_proj + h), part);
-  part = warp_sum(part);
-  if (lane == 0) s_red[wid] = part;
-  __syncthreads();
-  float c = 0.f;
-#pragma unroll
-  for (int w = 0; w < kStepThreads / 32; ++w) c += s_red[w];
-  __syncthreads();
-
-  // scores and their maximum
   float mx = -INFINITY;
-  for (int j = tid; j < len; j += kStepThreads) {
-    const float s = enc_scores[static_cast<long long>(j) * N + n] + c;
-    s_w[j] = s;
-    mx = fmaxf(mx, s);
+  for (int j0 = wid * kDots; j0 < len; j0 += kWarps * kDots) {
+    float s[kDots];
+    row_dots(mine + j0 * step_elems, step_elems, len - j0, enc_proj, H, lane, s);
+#pragma unroll
+    for (int r = 0; r < kDots; ++r) {
+      if (j0 + r >= len) continue;
+      mx = fmaxf(mx, s[r]);
+      if (lane == r) {
+        s_w[j0 + r] = s[r];
+        if (blockIdx.y == 0) scores[static_cast<long long>(j0 + r) * N + n] = s[r];
+      }
+    }
   }
-  mx = warp_max(mx);
   if (lane == 0) s_red[wid] = mx;
   __syncthreads();
   mx = s_red[0];
 #pragma unroll
-  for (int w = 1; w < kStepThreads / 32; ++w) mx = fmaxf(mx, s_red[w]);
+  for (int w = 1; w < kWarps; ++w) mx = fmaxf(mx, s_red[w]);
   __syncthreads();
   float sum = 0.f;
-  for (int j = tid; j < len; j += kStepThreads) {
+  for (int j = tid; j < len; j += kAttnThreads) {
     const float e = expf(s_w[j] - mx);
     s_w[j] = e;
     sum += e;
@@ -129,84 +155,95 @@ attn_step_kernel(const T* __restrict__ enc, const float* __restrict__ enc_scores
   __syncthreads();
   sum = 0.f;
 #pragma unroll
-  for (int w = 0; w < kStepThreads / 32; ++w) sum += s_red[w];
+  for (int w = 0; w < kWarps; ++w) sum += s_red[w];
   const float inv = len > 0 ? 1.f / sum : 0.f;
 
-  // weighted sum of the encoder rows, one column per thread, four rows in flight
-  const int h = blockIdx.y * kStepThreads + tid;
-  if (h >= H) return;
-  const T* col = enc + static_cast<long long>(n) * H + h;
-  float acc = 0.f;
-  int j = 0;
-  for (; j + 4 <= len; j += 4) {
-    const float e0 = ld_f32<T>(col + (j + 0) * step_elems), e1 = ld_f32<T>(col + (j + 1) * step_elems);
-    const float e2 = ld_f32<T>(col + (j + 2) * step_elems), e3 = ld_f32<T>(col + (j + 3) * step_elems);
-    acc = fmaf(s_w[j], e0, acc);
-    acc = fmaf(s_w[j + 1], e1, acc);
-    acc = fmaf(s_w[j + 2], e2, acc);
-    acc = fmaf(s_w[j + 3], e3, acc);
+  // weighted sum: a thread takes 16 bytes of every kRowGroups-th row
+  const int cg = tid % kColGroups, rg = tid / kColGroups, h = blockIdx.y * kAttnCols + cg * kN;
+  float acc[kN];
+#pragma unroll
+  for (int i = 0; i < kN; ++i) acc[i] = 0.f;
+  if (h < H) {
+#pragma unroll 4
+    for (int j = rg; j < len; j += kRowGroups) {
+      float x[kN];
+      ld_piece(mine + j * step_elems + h, x);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) acc[i] = fmaf(s_w[j], x[i], acc[i]);
+    }
   }
-  for (; j < len; ++j) acc = fmaf(s_w[j], ld_f32<T>(col + j * step_elems), acc);
-  T* o = out + blockIdx.z * step_elems + static_cast<long long>(n) * H + h;
-  for (int k = 0; k < copies; ++k) st_f32<T>(o + k * step_elems, acc * inv);
+#pragma unroll
+  for (int i = 0; i < kN; ++i) s_part[rg][cg * kN + i] = acc[i];
+  __syncthreads();
+  if (tid < kAttnCols) {
+    float v = 0.f;
+#pragma unroll
+    for (int r = 0; r < kRowGroups; ++r) v += s_part[r][tid];
+    st_f32<T>(s_out + tid, v * inv);
+  }
+  __syncthreads();
+  if (h < H) {
+    const uint4 v = *reinterpret_cast<const uint4*>(s_out + cg * kN);
+    T* o = out + static_cast<long long>(n) * H + h;
+    for (int t = rg; t < Lt; t += kRowGroups) *reinterpret_cast<uint4*>(o + t * step_elems) = v;
+  }
 }
 
-// Where step t of a sequence has NaN for its vector, so have the steps behind it and their decoder states.
-// (Encoder states are at most 1 and weights too: a vector is finite or NaN, and NaN weights make all of its
-// columns NaN.  A NaN encoder state alone is in every step's vector already.)
+// The decoder's terms dec_t . dec_proj of sequence blockIdx.x.  The largest score of a step is the largest of the
+// encoder's scores plus the term; if that is not finite the step's vector is NaN, and so are the decoder states and
+// vectors of the steps behind it.  (Encoder scores that are not finite are in every step's vector already.)
 template <typename T>
-__global__ void __launch_bounds__(kCarryThreads)
-carry_nan_kernel(T* __restrict__ dec, T* __restrict__ out, int Lt, int N, int H) {
-  const int n = blockIdx.x * (kCarryThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(kAttnThreads)
+attn_finish_kernel(T* __restrict__ dec, const T* __restrict__ dec_proj, const float* __restrict__ scores,
+                   const int* __restrict__ src_lens, T* __restrict__ out, int Lt, int Ls, int N, int H) {
+  constexpr int kWarps = kAttnThreads / 32;
+  __shared__ int s_first;
+  const int n = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const long long step_elems = static_cast<long long>(N) * H, row = static_cast<long long>(n) * H;
+  if (tid == 0) s_first = Lt;
   grid_launch_dependents();
   grid_dependency_wait();
-  if (n >= N) return;
-  const long long step_elems = static_cast<long long>(N) * H, row = static_cast<long long>(n) * H;
-  int first = Lt;
-  for (int t0 = 0; t0 < Lt && first == Lt; t0 += 32) {
-    const int t = t0 + lane;
-    const bool bad = t < Lt && isnan(ld_f32<T>(out + t * step_elems + row));
-    const unsigned who = __ballot_sync(0xffffffffu, bad);
-    if (who != 0) first = t0 + __ffs(who) - 1;
+  __syncthreads();
+  const int len = source_len(src_lens, n, Ls);
+  if (len == 0) return;  // nothing to attend to: zeros
+  float mx = -INFINITY;
+  for (int j = lane; j < len; j += 32) mx = fmaxf(mx, scores[static_cast<long long>(j) * N + n]);
+  mx = warp_max(mx);
+  for (int t0 = wid * kDots; t0 < Lt; t0 += kWarps * kDots) {
+    float c[kDots];
+    row_dots(dec + t0 * step_elems + row, step_elems, Lt - t0, dec_proj, H, lane, c);
+#pragma unroll
+    for (int r = 0; r < kDots; ++r)
+      if (lane == r && t0 + r < Lt && !isfinite(mx + c[r])) atomicMin(&s_first, t0 + r);
   }
+  __syncthreads();
   const float nan = __int_as_float(0x7FFFFFFF);
-  for (int t = first + 1; t < Lt; ++t)
+  for (int t = s_first + wid; t < Lt; t += kWarps)
     for (int h = lane; h < H; h += 32) {
-      st_f32<T>(dec + t * step_elems + row + h, nan);
+      if (t > s_first) st_f32<T>(dec + t * step_elems + row + h, nan);
       st_f32<T>(out + t * step_elems + row + h, nan);
     }
 }
 
 template <typename T>
-int carry_nan_t(void* dec, void* out, int Lt, int N, int H, cudaStream_t stream) {
-  constexpr int kRows = kCarryThreads / 32;
-  const cudaError_t err = launch_light(carry_nan_kernel<T>, dim3((N + kRows - 1) / kRows), dim3(kCarryThreads), 0, stream,
-                                       static_cast<T*>(dec), static_cast<T*>(out), Lt, N, H);
+int attn_vectors_t(const void* enc, const void* enc_proj, const int* src_lens, float* scores, void* out, int Lt, int Ls,
+                   int N, int H, cudaStream_t stream) {
+  static std::atomic<unsigned long long> configured{0};
+  if (!ensure_dynamic_smem(attn_vector_kernel<T>, 48 * 1024, configured)) return FTB_ERR_LAUNCH;
+  const cudaError_t err =
+      launch_light(attn_vector_kernel<T>, dim3(N, (H + kAttnCols - 1) / kAttnCols), dim3(kAttnThreads),
+                   static_cast<size_t>(Ls) * sizeof(float), stream, static_cast<const T*>(enc),
+                   static_cast<const T*>(enc_proj), src_lens, scores, static_cast<T*>(out), Lt, Ls, N, H);
   count_launch();
   if (err != cudaSuccess) cudaGetLastError();
   return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
 }
 
 template <typename T>
-int enc_scores_t(const void* enc, const void* proj, float* scores, long long n_rows, int H, cudaStream_t stream) {
-  const long long ctas = (n_rows + 7) / 8;
-  const long long full = static_cast<long long>(current_sm_count()) * 8;
-  const int grid = static_cast<int>(ctas < full ? ctas : full);
-  const cudaError_t err = launch_light(row_dot_kernel<T>, dim3(grid), dim3(256), 0, stream, static_cast<const T*>(enc),
-                                           static_cast<const T*>(proj), scores, n_rows, H);
-  count_launch();
-  if (err != cudaSuccess) cudaGetLastError();
-  return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
-}
-
-template <typename T>
-int attn_steps_t(const void* enc, const float* enc_scores, const void* dec, const void* dec_proj, const int* src_lens,
-                 void* out, int steps, int Ls, int N, int H, cudaStream_t stream) {
-  const dim3 grid(N, (H + kStepThreads - 1) / kStepThreads, dec == nullptr ? 1 : steps);
-  const cudaError_t err = launch_light(attn_step_kernel<T>, grid, dim3(kStepThreads), static_cast<size_t>(Ls) * sizeof(float),
-                                           stream, static_cast<const T*>(enc), enc_scores, static_cast<const T*>(dec),
-                                           static_cast<const T*>(dec_proj), src_lens, static_cast<T*>(out),
-                                           dec == nullptr ? steps : 1, Ls, N, H);
+int attn_finish_t(void* dec, const void* dec_proj, const float* scores, const int* src_lens, void* out, int Lt, int Ls,
+                  int N, int H, cudaStream_t stream) {
+  const cudaError_t err = launch_light(attn_finish_kernel<T>, dim3(N), dim3(kAttnThreads), 0, stream, static_cast<T*>(dec),
+                                       static_cast<const T*>(dec_proj), scores, src_lens, static_cast<T*>(out), Lt, Ls, N, H);
   count_launch();
   if (err != cudaSuccess) cudaGetLastError();
   return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
@@ -214,34 +251,26 @@ int attn_steps_t(const void* enc, const float* enc_scores, const void* dec, cons
 
 }  // namespace
 
-// Longest source sequence the step kernel takes: its scores sit in 48 KB of shared memory.
+// Longest source sequence the attention takes: its scores sit in 48 KB of shared memory.
 int rnn_attention_max_src_len() { return 48 * 1024 / static_cast<int>(sizeof(float)); }
 
-int launch_enc_scores(int dtype, const void* enc, const void* proj, float* scores, long long n_rows, int H,
-                      cudaStream_t stream) {
+// The attention vector of every sequence into its rows of out [Lt, N, H]; the encoder's scores into scores [Ls, N].
+int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, void* out,
+                        int Lt, int Ls, int N, int H, cudaStream_t stream) {
   switch (dtype) {
-    case FTB_F32: return enc_scores_t<float>(enc, proj, scores, n_rows, H, stream);
-    case FTB_F16: return enc_scores_t<__half>(enc, proj, scores, n_rows, H, stream);
-    default: return enc_scores_t<__nv_bfloat16>(enc, proj, scores, n_rows, H, stream);
+    case FTB_F32: return attn_vectors_t<float>(enc, enc_proj, src_lens, scores, out, Lt, Ls, N, H, stream);
+    case FTB_F16: return attn_vectors_t<__half>(enc, enc_proj, src_lens, scores, out, Lt, Ls, N, H, stream);
+    default: return attn_vectors_t<__nv_bfloat16>(enc, enc_proj, src_lens, scores, out, Lt, Ls, N, H, stream);
   }
 }
 
-int launch_carry_nan(int dtype, void* dec, void* out, int Lt, int N, int H, cudaStream_t stream) {
+// What decoder terms that are not finite make of the vectors in `out` and the states in `dec`.
+int launch_attn_finish(int dtype, void* dec, const void* dec_proj, const float* scores, const int* src_lens, void* out,
+                       int Lt, int Ls, int N, int H, cudaStream_t stream) {
   switch (dtype) {
-    case FTB_F32: return carry_nan_t<float>(dec, out, Lt, N, H, stream);
-    case FTB_F16: return carry_nan_t<__half>(dec, out, Lt, N, H, stream);
-    default: return carry_nan_t<__nv_bfloat16>(dec, out, Lt, N, H, stream);
-  }
-}
-
-// The attention vectors of `steps` decoder steps (at most 65535) into out [steps, N, H]; dec == nullptr:
-// without a decoder term, the same vectors in the rows of every step.
-int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
-                      const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream) {
-  switch (dtype) {
-    case FTB_F32: return attn_steps_t<float>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
-    case FTB_F16: return attn_steps_t<__half>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
-    default: return attn_steps_t<__nv_bfloat16>(enc, enc_scores, dec, dec_proj, src_lens, out, steps, Ls, N, H, stream);
+    case FTB_F32: return attn_finish_t<float>(dec, dec_proj, scores, src_lens, out, Lt, Ls, N, H, stream);
+    case FTB_F16: return attn_finish_t<__half>(dec, dec_proj, scores, src_lens, out, Lt, Ls, N, H, stream);
+    default: return attn_finish_t<__nv_bfloat16>(dec, dec_proj, scores, src_lens, out, Lt, Ls, N, H, stream);
   }
 }
 

@@ -57,11 +57,10 @@ int pack_grid(const void* i2h, const void* h2h, void* Wp, int H, int dtype, cuda
 int pack_projection(const void* P, void* Pt, int H, int V, int Vp, int dtype, cudaStream_t s);
 int pack_rnn(const void* W, const void* U, void* Wp, int I, int H, int dtype, cudaStream_t s);
 int rnn_attention_max_src_len();
-int launch_enc_scores(int dtype, const void* enc, const void* proj, float* scores, long long n_rows, int H,
-                      cudaStream_t stream);
-int launch_attn_steps(int dtype, const void* enc, const float* enc_scores, const void* dec, const void* dec_proj,
-                      const int* src_lens, void* out, int steps, int Ls, int N, int H, cudaStream_t stream);
-int launch_carry_nan(int dtype, void* dec, void* out, int Lt, int N, int H, cudaStream_t stream);
+int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, void* out,
+                        int Lt, int Ls, int N, int H, cudaStream_t stream);
+int launch_attn_finish(int dtype, void* dec, const void* dec_proj, const float* scores, const int* src_lens, void* out,
+                       int Lt, int Ls, int N, int H, cudaStream_t stream);
 bool rnn_chain_supported(int dtype, int H);
 int launch_rnn_chain(int dtype, const float* pre, const void* Wp, int ldw, int k0, const float* bias,
                      const void* before, void* out, int steps, int N, int H, int* status, cudaStream_t stream);
@@ -1321,17 +1320,12 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
     rc = cl.run(items);
     if (rc) return rc;
   }
-  rc = launch_enc_scores(dtype, enc, enc_proj, enc_scores, static_cast<long long>(Ls) * N, H, stream);
-  if (rc) return rc;
   // Decoder.  The attention vector of a step does not depend on the decoder (its term moves all scores
-  // of a softmax by one number), so the recurrent inputs of steps 1.. are known here: they go to the
-  // rows of `out` they are read from, all decoder cells run as one level, and the attention over all
-  // steps writes the result over them.  (As a chain: two dependent launches per step.)  A term that is
-  // not finite is carried to the steps behind it at the end.
-  if (Lt > 1) {
-    rc = launch_attn_steps(dtype, enc, enc_scores, nullptr, dec_proj, src_lens, out, Lt - 1, Ls, N, H, stream);
-    if (rc) return rc;
-  }
+  // of a softmax by one number), so the vectors of all steps are known here: they go to their rows of
+  // `out`, where the decoder cells read them as recurrent inputs, all cells run as one level, and a
+  // term that is not finite is carried to the steps behind it at the end.
+  rc = launch_attn_vectors(dtype, enc, enc_proj, src_lens, enc_scores, out, Lt, Ls, N, H, stream);
+  if (rc) return rc;
   items.clear();
   for (int t = 0; t < std::min(Lt, 2); ++t) {  // step 0 has no recurrent input; steps 1.. are consecutive rows
     CellItem it = blank_item();
@@ -1345,14 +1339,7 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
   }
   rc = cl.run(items);
   if (rc) return rc;
-  constexpr int kMostSteps = 65535;  // of one launch
-  for (int t = 0; t < Lt; t += kMostSteps) {
-    const size_t at = static_cast<size_t>(t) * N * H * es;
-    rc = launch_attn_steps(dtype, enc, enc_scores, static_cast<char*>(dec) + at, dec_proj, src_lens,
-                           static_cast<char*>(out) + at, std::min(kMostSteps, Lt - t), Ls, N, H, stream);
-    if (rc) return rc;
-  }
-  return Lt > 1 ? launch_carry_nan(dtype, dec, out, Lt, N, H, stream) : FTB_OK;
+  return launch_attn_finish(dtype, dec, dec_proj, enc_scores, src_lens, out, Lt, Ls, N, H, stream);
 }
 
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {

@@ -278,7 +278,7 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * decoder's recurrent inputs follow from the encoder alone and all its steps run side by side.  A decoder
  * term that is not finite makes the vectors of its step and of all later steps of that sequence NaN.
  * With workspace_bytes >= ftb_rnn_attention_workspace_bytes() (16-bit types, H <= 512) the encoder is one
- * matrix product and one scan kernel; else one launch per source position.  Five launches for the rest.
+ * matrix product and one scan kernel; else one launch per source position.  Three launches for the rest.
  * The product's result lies in the workspace behind the status word while the call runs.
  * ftb_rnn_attention_fwd_scratch takes it in a buffer of its own instead (ftb_rnn_attention_scratch_bytes, 0:
  * none needed; scratch may be NULL), so that a workspace shared by calls on several streams holds the

@@ -173,3 +173,33 @@ def test_what_is_not_finite_reaches_the_later_steps(ops, dt, Lt):
     bad = torch.stack(bad)
     assert torch.equal(torch.isnan(out), bad) and bad.any() and not bad.all()
     assert torch.equal(out[~bad], finite[~bad])
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H,Ls,Lt,lens", [
+    (64, 300, 3, [300, 1, 77, 0]),       # more source positions than threads; nothing to attend to
+    (192, 5, 70, [5, 3, 4]),             # more target steps than row groups; columns that end inside a CTA's 128
+    (640, 9, 2, [9, 8, 2, 1, 5]),        # wider than the scan kernel takes
+])
+def test_vectors_of_all_steps(ops, dt, H, Ls, Lt, lens):
+    """One attention vector a sequence in the rows of all its steps, scores and sums in one launch."""
+    N = len(lens)
+    p, g = _params(H, H + Ls, 1.0 / (H ** 0.5))
+    src, trg = torch.randn(Ls, N, H, generator=g).to(dt), torch.randn(Lt, N, H, generator=g).to(dt)
+    pq = {k: v.to(dt) for k, v in p.items()}
+    enc, out = ops.rnn_attention(src.cuda(), trg.cuda(), ops.rnn_pack_weights(pq["Ws"].cuda(), pq["Us"].cuda()),
+                                 ops.rnn_pack_weights(pq["Wt"].cuda(), pq["Ut"].cuda()),
+                                 pq["bs"].reshape(H).float().cuda(), pq["bt"].reshape(H).float().cuda(),
+                                 pq["enc_proj"].reshape(H).cuda(), pq["dec_proj"].reshape(H).cuda(),
+                                 torch.tensor(lens, dtype=torch.int32).cuda())
+    ops.check_status()
+    for n, m in enumerate(lens):
+        if m == 0:
+            assert out[:, n].eq(0).all()
+            continue
+        e = enc[:m, n].double().cpu()
+        w = torch.softmax(e @ pq["enc_proj"].double().reshape(H), 0)
+        ref = (w @ e).expand(Lt, H)  # the decoder's term moves all scores alike
+        # fp32 scores of H products (relative 2^-24 * sqrt(H)) in the exponent, then the rounding of the result
+        tol = {torch.float32: 1e-5, torch.float16: 1e-3, torch.bfloat16: 8e-3}[dt]
+        assert (out[:, n].double().cpu() - ref).abs().max().item() <= tol
