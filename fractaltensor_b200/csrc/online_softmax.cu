@@ -52,7 +52,7 @@ __device__ __forceinline__ void push(MD& s, float v) {
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int width, int ld,
+online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int width, int ld, int ld_out,
                       int cache_floats) {
   extern __shared__ float4 row_cache4[];
   float* row_cache = reinterpret_cast<float*>(row_cache4);
@@ -62,16 +62,18 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
   const int cached_floats = width < cache_floats ? width : cache_floats;  // prefix of the row kept on chip
   grid_launch_dependents();
   grid_dependency_wait();  // the kernel before this one (the projection GEMM, say) wrote x
-  // 16-byte accesses need rows that start on a 16-byte boundary.
-  const bool vec = ((width | ld) & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  // 16-byte accesses need rows that start on a 16-byte boundary; what is left behind the last whole one goes singly.
+  const bool vec_in = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool vec = vec_in && (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  const int tail = width & ~3;
 
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const float* xr = x + static_cast<size_t>(r) * ld;
-    float* yr = y + static_cast<size_t>(r) * ld;
+    float* yr = y + static_cast<size_t>(r) * ld_out;
     MD s;
     s.m = -FLT_MAX;
     s.d = 0.f;
-    if (vec) {
+    if (vec_in) {
       const float4* x4 = reinterpret_cast<const float4*>(xr);
 #pragma unroll 4
       for (int i = tid; i < width / 4; i += THREADS) {
@@ -84,12 +86,11 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
         push(s, v.z);
         push(s, v.w);
       }
-    } else {
-      for (int i = tid; i < width; i += THREADS) {
-        const float v = xr[i];
-        if (i < cached_floats) row_cache[i] = v;
-        push(s, v);
-      }
+    }
+    for (int i = (vec_in ? tail : 0) + tid; i < width; i += THREADS) {
+      const float v = xr[i];
+      if (i < cached_floats) row_cache[i] = v;
+      push(s, v);
     }
     // Threads that saw no element hold (-FLT_MAX, 0): neutral in a merge.
 #pragma unroll
@@ -135,11 +136,10 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
         v.w = exp_fast(fmaxf(v.w - m, kClamp)) * inv_d;
         __stcs(y4 + i, v);
       }
-    } else {
-      for (int i = tid; i < width; i += THREADS) {
-        const float v = i < cached_floats ? row_cache[i] : xr[i];
-        yr[i] = exp_fast(fmaxf(v - m, kClamp)) * inv_d;
-      }
+    }
+    for (int i = (vec ? tail : 0) + tid; i < width; i += THREADS) {
+      const float v = i < cached_floats ? row_cache[i] : xr[i];
+      __stcs(yr + i, exp_fast(fmaxf(v - m, kClamp)) * inv_d);
     }
     __syncthreads();  // the cache and the reduction slots are reused by the next row
   }
@@ -148,7 +148,7 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
 // Short rows (width % 4 == 0, up to 32 * 4 * kMaxV floats): one warp per row, the row in registers.
 constexpr int kMaxV = 16;
 __global__ void __launch_bounds__(kSoftmaxThreads)
-online_softmax_warp_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int width, int ld) {
+online_softmax_warp_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int width, int ld, int ld_out) {
   const int lane = threadIdx.x & 31;
   const int warps_per_cta = kSoftmaxThreads / 32;
   const int n4 = width / 4;
@@ -156,7 +156,7 @@ online_softmax_warp_kernel(const float* __restrict__ x, float* __restrict__ y, i
   grid_dependency_wait();
   for (int r = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); r < rows; r += gridDim.x * warps_per_cta) {
     const float4* x4 = reinterpret_cast<const float4*>(x + static_cast<size_t>(r) * ld);
-    float4* y4 = reinterpret_cast<float4*>(y + static_cast<size_t>(r) * ld);
+    float4* y4 = reinterpret_cast<float4*>(y + static_cast<size_t>(r) * ld_out);
     float4 v[kMaxV];
 #pragma unroll
     for (int j = 0; j < kMaxV; ++j)
@@ -199,19 +199,19 @@ online_softmax_warp_kernel(const float* __restrict__ x, float* __restrict__ y, i
 using namespace ftb;
 
 namespace ftb {
-// Softmax over the first `width` floats of each row of x (rows `ld` floats apart), written to the
-// same positions of y; x == y is allowed when a row fits the on-chip cache (width <= 48 K floats).
-int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, cudaStream_t stream) {
-  if (!x || !y || rows <= 0 || width <= 0 || ld < width) return FTB_ERR_ARG;
+// Softmax over the first `width` floats of each row of x (rows `ld` floats apart) into rows of y (`ld_out` apart);
+// x == y (with ld_out == ld) is allowed when a row fits the on-chip cache (width <= 48 K floats).
+int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, int ld_out, cudaStream_t stream) {
+  if (!x || !y || rows <= 0 || width <= 0 || ld < width || ld_out < width) return FTB_ERR_ARG;
   if (static_cast<int64_t>(rows) * ld > 0x7fffffffffLL) return FTB_ERR_ARG;
   int rc = check_device_sm100();
   if (rc) return rc;
   const bool aligned16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  if (aligned16 && ((width | ld) & 3) == 0 && width <= 32 * 4 * kMaxV && rows >= 8) {
+  if (aligned16 && ((width | ld | ld_out) & 3) == 0 && width <= 32 * 4 * kMaxV && rows >= 8) {
     const int64_t ctas = (static_cast<int64_t>(rows) + kSoftmaxThreads / 32 - 1) / (kSoftmaxThreads / 32);
     const int64_t full = static_cast<int64_t>(current_sm_count()) * 4;
     const cudaError_t err = launch_light(online_softmax_warp_kernel, dim3(static_cast<int>(ctas < full ? ctas : full)),
-                                             dim3(kSoftmaxThreads), 0, stream, x, y, rows, width, ld);
+                                             dim3(kSoftmaxThreads), 0, stream, x, y, rows, width, ld, ld_out);
     count_launch();
     if (err != cudaSuccess) cudaGetLastError();
     return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
@@ -236,10 +236,10 @@ int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, c
   cudaError_t err;
   if (per_sm <= 2)
     err = launch_light(online_softmax_kernel<1024>, dim3(grid), dim3(1024), smem, stream, x, y, rows, width, ld,
-                           cache_floats);
+                       ld_out, cache_floats);
   else
-    err = launch_light(online_softmax_kernel<kSoftmaxThreads>, dim3(grid), dim3(kSoftmaxThreads), smem, stream, x, y,
-                           rows, width, ld, cache_floats);
+    err = launch_light(online_softmax_kernel<kSoftmaxThreads>, dim3(grid), dim3(kSoftmaxThreads), smem, stream, x, y, rows,
+                       width, ld, ld_out, cache_floats);
   count_launch();
   if (err != cudaSuccess) cudaGetLastError();
   return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
@@ -247,5 +247,5 @@ int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, c
 }  // namespace ftb
 
 extern "C" int ftb_online_softmax(const float* x, float* y, int rows, int width, void* stream_) {
-  return ftb::online_softmax_rows(x, y, rows, width, width, static_cast<cudaStream_t>(stream_));
+  return ftb::online_softmax_rows(x, y, rows, width, width, width, static_cast<cudaStream_t>(stream_));
 }

@@ -64,7 +64,7 @@ int launch_attn_finish(int dtype, void* dec, const void* dec_proj, const float* 
 bool rnn_chain_supported(int dtype, int H);
 int launch_rnn_chain(int dtype, const float* pre, const void* Wp, int ldw, int k0, const float* bias,
                      const void* before, void* out, int steps, int N, int H, int* status, cudaStream_t stream);
-int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, cudaStream_t stream);
+int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, int ld_out, cudaStream_t stream);
 
 namespace {
 
@@ -1405,19 +1405,20 @@ int ftb_projection_pack(const void* P, void* Pt, int H, int V, int dtype, void* 
   return pack_projection(P, Pt, H, V, ftb_projection_padded_cols(V), dtype, static_cast<cudaStream_t>(stream));
 }
 
-int ftb_lstm_project_softmax(const void* h, const void* Pt, float* probs, long long T, int V, int H, int dtype,
-                             void* workspace, size_t workspace_bytes, void* stream_) {
+// logits: [T, Vp]; probs: [T, V] without gaps, or the same buffer as logits, with its rows Vp apart.
+static int project_softmax(const void* h, const void* Pt, float* logits, float* probs, long long T, int V, int H, int dtype,
+                           void* workspace, size_t workspace_bytes, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (!h || !Pt || !probs || T <= 0 || T > 0x7fffffffLL || V <= 0 || H <= 0 || H % 64 != 0) return FTB_ERR_ARG;
+  if (!h || !Pt || !logits || !probs || T <= 0 || T > 0x7fffffffLL || V <= 0 || H <= 0 || H % 64 != 0) return FTB_ERR_ARG;
   if (dtype != FTB_F16 && dtype != FTB_BF16) return FTB_ERR_ARG;
   if (V > 48 * 1024) return FTB_ERR_ARG;  // the softmax runs in place on rows that fit its on-chip row cache
-  if (!aligned16({h, Pt, probs})) return FTB_ERR_ALIGN;
+  if (!aligned16({h, Pt, logits, probs})) return FTB_ERR_ALIGN;
   const int Vp = ftb_projection_padded_cols(V);
   if (static_cast<int64_t>(T) * Vp > 0x7fffffffffLL) return FTB_ERR_ARG;
   int* status = nullptr;
   int rc = begin_call(workspace, workspace_bytes, stream, &status);
   if (rc) return rc;
-  // 1. logits = h . Pt^T, fp32, written straight into `probs` (row stride Vp)
+  // 1. logits = h . Pt^T, fp32
   CellLauncher cl;
   cl.dtype = dtype;
   cl.epi = EPI_STORE_F32;
@@ -1437,11 +1438,22 @@ int ftb_lstm_project_softmax(const void* h, const void* Pt, float* probs, long l
   std::vector<CellItem> items(1, blank_item());
   add_seg(items[0], 0, 0, H, 0);
   items[0].rows = static_cast<int32_t>(T);
-  items[0].out = probs;
+  items[0].out = logits;
   rc = cl.run(items);
   if (rc) return rc;
-  // 2. softmax over the first V logits of every row, in place, one read and one write per logit
-  return online_softmax_rows(probs, probs, static_cast<int>(T), V, Vp, stream);
+  // 2. softmax over the first V logits of every row, one read and one write per logit
+  return online_softmax_rows(logits, probs, static_cast<int>(T), V, Vp, probs == logits ? Vp : V, stream);
+}
+
+int ftb_lstm_project_softmax(const void* h, const void* Pt, float* probs, long long T, int V, int H, int dtype,
+                             void* workspace, size_t workspace_bytes, void* stream) {
+  return project_softmax(h, Pt, probs, probs, T, V, H, dtype, workspace, workspace_bytes, stream);
+}
+
+int ftb_lstm_project_softmax_rows(const void* h, const void* Pt, float* logits, float* probs, long long T, int V, int H,
+                                  int dtype, void* workspace, size_t workspace_bytes, void* stream) {
+  if (probs == logits) return FTB_ERR_ARG;
+  return project_softmax(h, Pt, logits, probs, T, V, H, dtype, workspace, workspace_bytes, stream);
 }
 
 // ------------------------------------------------------------------------------

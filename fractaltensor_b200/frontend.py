@@ -134,10 +134,11 @@ def project_softmax(hs, prev_softmax_proj):
     h = _cuda(hs.data if not isinstance(hs, torch.Tensor) else hs)
     H = P.shape[0]
     P = _cuda(P, h.dtype).reshape(H, -1).contiguous()
-    probs = ops.lstm_project_softmax(h.reshape(-1, H).contiguous(), ops.projection_pack(P), P.shape[1])
+    h = h.reshape(-1, H).contiguous()
     if isinstance(hs, torch.Tensor):
-        return probs
-    return FractalTensor(probs.contiguous(), hs.indices, (1, P.shape[1]))
+        return ops.lstm_project_softmax(h, ops.projection_pack(P), P.shape[1])
+    probs = ops.lstm_project_softmax_rows(h, ops.projection_pack(P), P.shape[1])
+    return FractalTensor(probs, hs.indices, (1, P.shape[1]))
 
 
 def _is_ragged(x):

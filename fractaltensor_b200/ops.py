@@ -514,6 +514,27 @@ def lstm_project_softmax(h, Pt, V, out=None):
     return out[:, :V]
 
 
+def lstm_project_softmax_rows(h, Pt, V):
+    """lstm_project_softmax into a contiguous fp32 [T,V] (the logits take a buffer of their own)."""
+    V = int(V)
+    Vp = lib.ftb_projection_padded_cols(V)
+    if Vp == V:
+        return lstm_project_softmax(h, Pt, V)
+    _req(h, "h")
+    _req(Pt, "Pt", h.dtype)
+    H = h.shape[-1]
+    T = h.numel() // H
+    if tuple(Pt.shape) != (Vp, H) or Pt.device != h.device:
+        raise ValueError("lstm_project_softmax: Pt %s does not match h %s and V=%d" % (tuple(Pt.shape), tuple(h.shape), V))
+    logits = torch.empty(T, Vp, dtype=torch.float32, device=h.device)
+    probs = torch.empty(T, V, dtype=torch.float32, device=h.device)
+    ws = workspace(h.device)
+    with torch.cuda.device(h.device):
+        check(lib.ftb_lstm_project_softmax_rows(_ptr(h), _ptr(Pt), _ptr(logits), _ptr(probs), T, V, H, _dtype_code(h),
+                                                _ptr(ws), ws.numel(), _stream()), "ftb_lstm_project_softmax_rows")
+    return probs
+
+
 def embedding_gather(table, ids, out=None):
     """table: [V,H]; ids: int64 [T] (any nesting flattened) -> out [T,H] = table[ids]."""
     _req(table, "table")

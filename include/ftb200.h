@@ -328,6 +328,10 @@ int ftb_projection_padded_cols(int V);
 int ftb_projection_pack(const void* P, void* Pt, int H, int V, int dtype, void* stream);
 int ftb_lstm_project_softmax(const void* h, const void* Pt, float* probs, long long T, int V, int H, int dtype,
                              void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the logits in a scratch buffer of their own, fp32 [T,Vp], and rows of V numbers without gaps in
+ * probs, fp32 [T,V]. */
+int ftb_lstm_project_softmax_rows(const void* h, const void* Pt, float* logits, float* probs, long long T, int V, int H,
+                                  int dtype, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Plain GEMM out[M,N] = A[M,K] . Bt[N,K]^T through the cell kernel's main loop
  * (support op; the reference's KeCuteGemm, kaleido/core/device/kernels/cutlass_wmma.h:115-181).
