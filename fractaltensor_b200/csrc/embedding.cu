@@ -48,7 +48,40 @@ embedding_gather_kernel(const unsigned char* __restrict__ table, const long long
   }
 }
 
+// Rows of a ragged batch from the order of its sequences (row t of a sequence at start + t) to the packed time-major
+// order (step t of the length-sorted sequence r at off[t] + r), or back.  One warp a row, 16 bytes a lane; the
+// place of a row follows from two small tables, so that no index of every row has to be made or read.
+constexpr int kPermuteWarps = kGatherThreads / 32;
+__global__ void __launch_bounds__(kGatherThreads)
+ragged_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const int* __restrict__ start,
+                   const int* __restrict__ off, int groups, int row16, bool to_time_major) {
+  const int t = blockIdx.x / groups, r = (blockIdx.x - t * groups) * kPermuteWarps + (threadIdx.x >> 5);
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int first = off[t];
+  if (r >= off[t + 1] - first) return;
+  const size_t mine = (static_cast<size_t>(start[r]) + t) * row16, packed = (static_cast<size_t>(first) + r) * row16;
+  src += to_time_major ? mine : packed;
+  dst += to_time_major ? packed : mine;
+  for (int i = threadIdx.x & 31; i < row16; i += 32) dst[i] = src[i];
+}
+
 }  // namespace
+
+// start: [N] first row of the length-sorted sequences; off: [L + 1] first row of the steps; rows of `row_bytes`, a
+// multiple of 16.
+int launch_ragged_rows(const void* src, void* dst, const int* start, const int* off, int N, int L, long long row_bytes,
+                       bool to_time_major, cudaStream_t stream) {
+  const int groups = (N + kPermuteWarps - 1) / kPermuteWarps;
+  const long long grid = static_cast<long long>(L) * groups;
+  if (grid > 0x7fffffffLL || row_bytes % 16 != 0) return FTB_ERR_ARG;
+  const cudaError_t err = launch_light(ragged_rows_kernel, dim3(static_cast<unsigned>(grid)), dim3(kGatherThreads), 0, stream,
+                                       static_cast<const uint4*>(src), static_cast<uint4*>(dst), start, off, groups,
+                                       static_cast<int>(row_bytes / 16), to_time_major);
+  count_launch();
+  if (err != cudaSuccess) cudaGetLastError();
+  return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+}
 }  // namespace ftb
 
 using namespace ftb;

@@ -61,6 +61,8 @@ int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const 
                         int Lt, int Ls, int N, int H, cudaStream_t stream);
 int launch_attn_finish(int dtype, void* dec, const void* dec_proj, const float* scores, const int* src_lens, void* out,
                        int Lt, int Ls, int N, int H, cudaStream_t stream);
+int launch_ragged_rows(const void* src, void* dst, const int* start, const int* off, int N, int L, long long row_bytes,
+                       bool to_time_major, cudaStream_t stream);
 bool rnn_chain_supported(int dtype, int H);
 int launch_rnn_chain(int dtype, const float* pre, const void* Wp, int ldw, int k0, const float* bias,
                      const void* before, void* out, int steps, int N, int H, int* status, cudaStream_t stream);
@@ -881,6 +883,64 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
     }
   }
   return FTB_OK;
+}
+
+// Tables of a ragged batch behind the workspace of the packed entry point.
+static size_t ragged_table_bytes(int L, int N) { return sizeof(int) * (static_cast<size_t>(L) + 1 + N) + 16; }
+
+size_t ftb_lstm_stacked_ragged_workspace_bytes(int D, int L, int N) {
+  if (D <= 0 || L <= 0 || N <= 0) return kWorkspaceBytes;
+  return ftb_lstm_stacked_varlen_workspace_bytes(D, L) + ragged_table_bytes(L, N);
+}
+
+int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt, void* hs,
+                                float* c, void* out, int D, int N, int I, int H, int dtype, void* workspace,
+                                size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!x || !Wp || !lens || !xt || !hs || !c || !out || D <= 0 || N <= 0 || !valid_dtype(dtype)) return FTB_ERR_ARG;
+  if (H <= 0 || I <= 0 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return FTB_ERR_ARG;
+  int L = 0;
+  int64_t T = 0;
+  for (int n = 0; n < N; ++n) {
+    if (lens[n] <= 0) return FTB_ERR_ARG;
+    L = std::max(L, lens[n]);
+    T += lens[n];
+  }
+  if (static_cast<int64_t>(D) * T > 0x7fffffffLL) return FTB_ERR_ARG;
+  if (!aligned16({x, Wp, bias_p, xt, hs, c, out})) return FTB_ERR_ALIGN;
+  if (workspace == nullptr || workspace_bytes < ftb_lstm_stacked_ragged_workspace_bytes(D, L, N)) return FTB_ERR_WORKSPACE;
+  int rc = check_device_sm100();
+  if (rc) return rc;
+  // Sequences by decreasing length (equal ones in their order): active[t] of them are longer than t, and those of
+  // length n go to the places from active[n] on.
+  std::vector<int> active(static_cast<size_t>(L) + 1, 0), table(static_cast<size_t>(L) + 1 + N);
+  for (int n = 0; n < N; ++n) ++active[lens[n] - 1];
+  for (int t = L - 1; t > 0; --t) active[t - 1] += active[t];
+  int* off = table.data();
+  int* start = off + L + 1;
+  off[0] = 0;
+  for (int t = 0; t < L; ++t) off[t + 1] = off[t] + active[t];
+  {
+    std::vector<int> place(active.begin() + 1, active.end());  // [n - 1]: of the next sequence of length n
+    int row = 0;
+    for (int n = 0; n < N; ++n) {
+      start[place[lens[n] - 1]++] = row;
+      row += lens[n];
+    }
+  }
+  const size_t packed_bytes = ftb_lstm_stacked_varlen_workspace_bytes(D, L);
+  int* d_off = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + packed_bytes + 15) & ~static_cast<uintptr_t>(15));
+  const int* d_start = d_off + L + 1;
+  if (cudaMemcpyAsync(d_off, table.data(), sizeof(int) * table.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess)
+    return FTB_ERR_LAUNCH;
+  const long long es = static_cast<long long>(dtype_size(dtype));
+  rc = launch_ragged_rows(x, xt, d_start, d_off, N, L, I * es, true, stream);
+  if (rc) return rc;
+  rc = ftb_lstm_stacked_varlen_fwd(xt, Wp, bias_p, hs, c, active.data(), D, L, I, H, dtype, nullptr, workspace, packed_bytes,
+                                   stream_);
+  if (rc) return rc;
+  return launch_ragged_rows(static_cast<const char*>(hs) + static_cast<size_t>(D - 1) * T * H * es, out, d_start, d_off, N, L,
+                            H * es, false, stream);
 }
 
 size_t ftb_lstm_stacked_varlen_workspace_bytes(int D, int L) {

@@ -178,27 +178,18 @@ def stacked_lstm_time_major(embs, Wss, Uss, bss, dtype=None):
 
 
 def _stacked_lstm_ragged(embs, Wss, Uss, bss, dtype):
-    """Batch-major ragged batch [N][L_n]: sort by decreasing length, transpose into the
-    time-major packed layout on the device, run, and put the rows back where they were."""
+    """Batch-major ragged batch [N][L_n]: sorted by decreasing length, put into the time-major packed layout, run,
+    and the rows put back where they were, in one call of the library."""
     lens = [len(seq) for seq in embs.indices]
     if min(lens) <= 0:
         raise ValueError("empty sequence in the batch")
-    flat = _cuda(embs.data.reshape(sum(lens), -1), dtype)
-    dev = flat.device
-    order = sorted(range(len(lens)), key=lambda n: -lens[n])
-    start = [0]
-    for n in lens:
-        start.append(start[-1] + n)
-    L = lens[order[0]]
-    active = [sum(1 for n in lens if n > t) for t in range(L)]
-    # src[k] = position in the batch-major buffer of the k-th row of the time-major one
-    src = torch.tensor([start[order[r]] + t for t in range(L) for r in range(active[t])], dtype=torch.long,
-                       device=dev)
+    flat = _cuda(embs.data.reshape(sum(lens), -1), dtype).contiguous()
+    if flat.data_ptr() % 16 != 0:  # a slice of a larger buffer
+        flat = flat.clone()
     Wp, bias_p, D, H = _packed_weights(Wss, Uss, bss, flat.dtype)
-    hs, _ = ops.lstm_stacked_varlen(flat.index_select(0, src).contiguous(), active, Wp, bias_p)
-    out = torch.empty(sum(lens), H, dtype=hs.dtype, device=dev)
-    out.index_copy_(0, src, hs[D - 1])
-    return FractalTensor(out, [list(range(n)) for n in lens], (1, H))
+    out = ops.lstm_stacked_ragged(flat, lens, Wp, bias_p)
+    steps = list(range(max(lens)))
+    return FractalTensor(out, [steps[:n] for n in lens], (1, H))
 
 
 def stacked_lstm(embs, Wss, Uss, bss, dtype=None):

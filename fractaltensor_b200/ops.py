@@ -196,6 +196,33 @@ def lstm_stacked_varlen(x, active_rows, Wp, bias_p=None, hs=None, c=None, layers
     return hs, c
 
 
+def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
+    """Stacked LSTM over a batch of sequences of different lengths, one behind the other and in any order.
+
+    x: [T,I] with T = sum(lens), lens: N positive ints; Wp: [D,4H,I+H] -> the top layer's states [T,H] in x's order."""
+    _req(x, "x")
+    _req(Wp, "Wp", x.dtype)
+    N, L, T = len(lens), max(lens), sum(lens)
+    D, H4, K = Wp.shape
+    H, I = H4 // 4, x.shape[1]
+    if min(lens) <= 0:
+        raise ValueError("empty sequence in the batch")
+    if x.shape[0] != T or K != I + H or H4 != 4 * H or Wp.device != x.device:
+        raise ValueError("Wp %s / lens (sum %d) do not match x %s" % (tuple(Wp.shape), T, tuple(x.shape)))
+    if bias_p is not None:
+        _req_like(bias_p, "bias_p", torch.float32, (D, 4 * H), x)
+    xt = torch.empty_like(x)
+    hs = torch.empty(D, T, H, dtype=x.dtype, device=x.device)
+    c = torch.empty(D, N, H, dtype=torch.float32, device=x.device)
+    out = torch.empty(T, H, dtype=x.dtype, device=x.device)
+    ws = workspace(x.device, lib.ftb_lstm_stacked_ragged_workspace_bytes(D, L, N))
+    with torch.cuda.device(x.device):
+        check(lib.ftb_lstm_stacked_ragged_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N)(*lens), _ptr(xt), _ptr(hs),
+                                              _ptr(c), _ptr(out), D, N, I, H, _dtype_code(x), _ptr(ws), ws.numel(),
+                                              _stream()), "ftb_lstm_stacked_ragged_fwd")
+    return out
+
+
 def lstm_dilated(x, Wp, dilations, bias_p=None, hs=None, c=None, bn=0, pair=0, schedule=0):
     """x: [L,N,H]; Wp: [D,4H,2H]; dilations: D ints -> (hs [D,L,N,H], c fp32 [D,max_dil*N,H]).
     schedule: 0 auto, 1 one launch per level, 2 generic persistent kernel; H of 64, 128 or 256, weights resident in

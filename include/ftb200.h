@@ -144,6 +144,17 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
                                 const int* active_rows, int D, int L, int I, int H, int dtype, const int* tuning,
                                 void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same for a batch-major ragged batch in any order, FractalTensor [N][lens[n]] of the batch-major program
+ * (examples/stacked_rnn/stacked_lstm1.py:66-76): sorted, put into the packed time-major layout, run, and the top
+ * layer's states put back, all on `stream`.  `lens` is a HOST array of N ints >= 1.  With T = sum(lens) and
+ * L = max(lens): x: [T,I], the sequences one behind the other; out: [T,H] in the same order, the top layer's hidden
+ * states; xt [T,I], hs [D,T,H] and c fp32 [D,N,H] (caller-owned) receive the packed input and the packed results of
+ * ftb_lstm_stacked_varlen_fwd.  Not for stream capture. */
+size_t ftb_lstm_stacked_ragged_workspace_bytes(int D, int L, int N);
+int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt, void* hs,
+                                float* c, void* out, int D, int N, int I, int H, int dtype, void* workspace,
+                                size_t workspace_bytes, void* stream);
+
 /* Dilated stacked LSTM forward: layer l reads its own state dilations[l] steps
  * back.  Stands in for dilated_layer()/model() (examples/dilated_rnn/dilated_rnn.py:16-41)
  * and DilatedLstmRegion1/2 (kaleido/core/device/kernels/lstm/dilated_lstm/region{1,2}.h).
