@@ -10,115 +10,131 @@ namespace ftb {
 
 namespace {
 
-// out[(u * gates + g) * ldo + k_off + k] = in[g][k][u], in: [gates, K, H].
+// A stack of transposes in one launch: blockIdx.z is (layer, matrix, gate), matrix 0 or 1 (W, U).
+//   out[layer][(u * gates + g) * ldo + off + k] = in[layer][g][k][u],  k < K, u < U;  0 for U <= u < u_end
+struct TransposeArgs {
+  const void* in[2];
+  int K[2];    // rows of a matrix
+  int off[2];  // where they go in a packed row
+  int matrices, gates, U, u_end, ldo;
+  void* out;
+  size_t out_layer;  // elements
+};
+
+// Bound by memory: 64 x 64 tiles through shared memory, 16 bytes a thread on both sides (reads go singly where rows do
+// not begin on 16 bytes).  With 32 x 32 tiles moved element by element, a launch for each matrix of each layer, the
+// word program's parameters (3 layers of 512, 10000 words, 22.6 MB) took 42 us a pass; so 15.
+constexpr int kTile = 64, kPackThreads = 256;
 template <typename E>
-__global__ void pack_transpose_kernel(const E* __restrict__ in, E* __restrict__ out, int gates, int K, int H,
-                                      int ldo, int k_off) {
-  __shared__ E tile[32][33];
-  const int g = blockIdx.z;
-  const int k0 = blockIdx.y * 32, u0 = blockIdx.x * 32;
-  const E* src = in + static_cast<size_t>(g) * K * H;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int k = k0 + i, u = u0 + threadIdx.x;
-    if (k < K && u < H) tile[i][threadIdx.x] = src[static_cast<size_t>(k) * H + u];
+__global__ void __launch_bounds__(kPackThreads) pack_transpose_kernel(const TransposeArgs a) {
+  constexpr int kN = 16 / sizeof(E), kVecs = kTile / kN;
+  __shared__ E tile[kTile][kTile + 4 / sizeof(E)];
+  const int g = blockIdx.z % a.gates, m = blockIdx.z / a.gates % a.matrices, layer = blockIdx.z / (a.gates * a.matrices);
+  const int K = m == 0 ? a.K[0] : a.K[1], k0 = blockIdx.y * kTile, u0 = blockIdx.x * kTile;
+  if (k0 >= K) return;
+  const E* src = static_cast<const E*>(m == 0 ? a.in[0] : a.in[1]) + (static_cast<size_t>(layer) * a.gates + g) * K * a.U;
+  const bool vec_in = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && a.U % kN == 0;
+  if (vec_in) {
+    for (int e = threadIdx.x; e < kTile * kVecs; e += kPackThreads) {
+      const int k = e / kVecs, u = e % kVecs * kN;
+      if (k0 + k >= K) continue;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (u0 + u < a.U) v = __ldcs(reinterpret_cast<const uint4*>(src + static_cast<size_t>(k0 + k) * a.U + u0 + u));
+      const E* x = reinterpret_cast<const E*>(&v);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) tile[k][u + i] = x[i];
+    }
+  } else {
+    for (int e = threadIdx.x; e < kTile * kTile; e += kPackThreads) {
+      const int k = e / kTile, u = e % kTile;
+      if (k0 + k < K) tile[k][u] = u0 + u < a.U ? src[static_cast<size_t>(k0 + k) * a.U + u0 + u] : E(0);
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int u = u0 + i, k = k0 + threadIdx.x;
-    if (k < K && u < H) out[(static_cast<size_t>(u) * gates + g) * ldo + k_off + k] = tile[threadIdx.x][i];
+  E* dst = static_cast<E*>(a.out) + layer * a.out_layer + (m == 0 ? a.off[0] : a.off[1]);
+  const bool vec_out = ((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>(a.ldo) * sizeof(E)) & 15) == 0 && K % kN == 0;
+  for (int e = threadIdx.x; e < kTile * kVecs; e += kPackThreads) {
+    const int u = e / kVecs, k = e % kVecs * kN;
+    if (u0 + u >= a.u_end || k0 + k >= K) continue;
+    E* row = dst + (static_cast<size_t>(u0 + u) * a.gates + g) * a.ldo + k0 + k;
+    uint4 v;
+    E* x = reinterpret_cast<E*>(&v);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) x[i] = tile[k + i][u];
+    if (vec_out) {
+      *reinterpret_cast<uint4*>(row) = v;
+    } else {
+      for (int i = 0; i < kN && k0 + k + i < K; ++i) row[i] = x[i];
+    }
   }
 }
 
 template <typename E>
-__global__ void pack_bias_kernel(const E* __restrict__ bias, float* __restrict__ out, int gates, int H) {
+__global__ void pack_bias_kernel(const E* __restrict__ bias, float* __restrict__ out, int gates, int H, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gates * H) return;
-  const int g = i / H, u = i - g * H;
-  out[u * gates + g] = static_cast<float>(bias[i]);
+  if (i >= n) return;
+  const int layer = i / (gates * H), r = i - layer * gates * H, g = r / H, u = r - g * H;
+  out[static_cast<size_t>(layer) * gates * H + u * gates + g] = static_cast<float>(bias[i]);
 }
 
-template <typename E>
-int pack_matrix(const E* in, E* out, int gates, int K, int H, int ldo, int k_off, cudaStream_t s) {
-  dim3 grid((H + 31) / 32, (K + 31) / 32, gates), block(32, 8);
-  pack_transpose_kernel<E><<<grid, block, 0, s>>>(in, out, gates, K, H, ldo, k_off);
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+int pack_stack(const TransposeArgs& a, int layers, int dtype, cudaStream_t s) {
+  const int K = a.matrices > 1 && a.K[1] > a.K[0] ? a.K[1] : a.K[0], per_layer = a.gates * a.matrices;
+  // (gridDim.z is 65535 at most)
+  for (int l0 = 0, step = 65535 / per_layer; l0 < layers; l0 += step) {
+    TransposeArgs b = a;
+    const int n = layers - l0 < step ? layers - l0 : step;
+    for (int m = 0; m < a.matrices; ++m)
+      b.in[m] = static_cast<const char*>(a.in[m]) + static_cast<size_t>(l0) * a.gates * a.K[m] * a.U * dtype_size(dtype);
+    b.out = static_cast<char*>(a.out) + l0 * a.out_layer * dtype_size(dtype);
+    const dim3 grid((a.u_end + kTile - 1) / kTile, (K + kTile - 1) / kTile, n * per_layer);
+    if (dtype_size(dtype) == 4)
+      pack_transpose_kernel<uint32_t><<<grid, kPackThreads, 0, s>>>(b);
+    else
+      pack_transpose_kernel<uint16_t><<<grid, kPackThreads, 0, s>>>(b);
+    count_launch();
+    if (cudaGetLastError() != cudaSuccess) return FTB_ERR_LAUNCH;
+  }
+  return FTB_OK;
 }
 
 }  // namespace
 
 int pack_lstm(const void* W, const void* U, const void* bias, void* Wp, float* bias_p, int D, int I, int H, int dtype,
               cudaStream_t s) {
-  const size_t es = dtype_size(dtype);
   const int K = I + H;
-  for (int d = 0; d < D; ++d) {
-    const char* w = static_cast<const char*>(W) + static_cast<size_t>(d) * 4 * I * H * es;
-    const char* u = static_cast<const char*>(U) + static_cast<size_t>(d) * 4 * H * H * es;
-    char* o = static_cast<char*>(Wp) + static_cast<size_t>(d) * 4 * H * K * es;
-    int rc;
-    if (es == 4) {
-      rc = pack_matrix<float>(reinterpret_cast<const float*>(w), reinterpret_cast<float*>(o), 4, I, H, K, 0, s);
-      if (rc) return rc;
-      rc = pack_matrix<float>(reinterpret_cast<const float*>(u), reinterpret_cast<float*>(o), 4, H, H, K, I, s);
-    } else {
-      rc = pack_matrix<uint16_t>(reinterpret_cast<const uint16_t*>(w), reinterpret_cast<uint16_t*>(o), 4, I, H, K, 0, s);
-      if (rc) return rc;
-      rc = pack_matrix<uint16_t>(reinterpret_cast<const uint16_t*>(u), reinterpret_cast<uint16_t*>(o), 4, H, H, K, I, s);
-    }
-    if (rc) return rc;
-    if (bias != nullptr && bias_p != nullptr) {
-      const char* b = static_cast<const char*>(bias) + static_cast<size_t>(d) * 4 * H * es;
-      float* bo = bias_p + static_cast<size_t>(d) * 4 * H;
-      const int n = 4 * H, thr = 256;
-      if (dtype == FTB_F32)
-        pack_bias_kernel<float><<<(n + thr - 1) / thr, thr, 0, s>>>(reinterpret_cast<const float*>(b), bo, 4, H);
-      else if (dtype == FTB_F16)
-        pack_bias_kernel<__half><<<(n + thr - 1) / thr, thr, 0, s>>>(reinterpret_cast<const __half*>(b), bo, 4, H);
-      else
-        pack_bias_kernel<__nv_bfloat16><<<(n + thr - 1) / thr, thr, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(b), bo, 4, H);
-      if (cudaGetLastError() != cudaSuccess) return FTB_ERR_LAUNCH;
-      count_launch();
-    }
+  const TransposeArgs a = {{W, U}, {I, H}, {0, I}, 2, 4, H, H, K, Wp, static_cast<size_t>(4) * H * K};
+  const int rc = pack_stack(a, D, dtype, s);
+  if (rc) return rc;
+  if (bias != nullptr && bias_p != nullptr) {
+    const int n = D * 4 * H, thr = 256, grid = (n + thr - 1) / thr;
+    if (dtype == FTB_F32)
+      pack_bias_kernel<float><<<grid, thr, 0, s>>>(static_cast<const float*>(bias), bias_p, 4, H, n);
+    else if (dtype == FTB_F16)
+      pack_bias_kernel<__half><<<grid, thr, 0, s>>>(static_cast<const __half*>(bias), bias_p, 4, H, n);
+    else
+      pack_bias_kernel<__nv_bfloat16><<<grid, thr, 0, s>>>(static_cast<const __nv_bfloat16*>(bias), bias_p, 4, H, n);
+    if (cudaGetLastError() != cudaSuccess) return FTB_ERR_LAUNCH;
+    count_launch();
   }
   return FTB_OK;
 }
 
 // P: [H, V] (x @ P orientation) -> Pt: [Vp, H] K-major, row v = column v of P, rows V..Vp-1 zero.
 int pack_projection(const void* P, void* Pt, int H, int V, int Vp, int dtype, cudaStream_t s) {
-  const size_t es = dtype_size(dtype);
-  if (cudaMemsetAsync(Pt, 0, static_cast<size_t>(Vp) * H * es, s) != cudaSuccess) return FTB_ERR_LAUNCH;
-  // pack_matrix with one "gate": out[u * ldo + k] = in[k][u] for k < K = H, u < V
-  if (es == 4) return pack_matrix<float>(static_cast<const float*>(P), static_cast<float*>(Pt), 1, H, V, H, 0, s);
-  return pack_matrix<uint16_t>(static_cast<const uint16_t*>(P), static_cast<uint16_t*>(Pt), 1, H, V, H, 0, s);
+  const TransposeArgs a = {{P, nullptr}, {H, 0}, {0, 0}, 1, 1, V, Vp, H, Pt, 0};
+  return pack_stack(a, 1, dtype, s);
 }
 
+// Grid cell: Wp[u, k] = i2h[k, u] for the 2H states, then h2h for the H inputs.
 int pack_grid(const void* i2h, const void* h2h, void* Wp, int H, int dtype, cudaStream_t s) {
-  int rc;
-  if (dtype_size(dtype) == 4) {
-    rc = pack_matrix<float>(static_cast<const float*>(i2h), static_cast<float*>(Wp), 1, 2 * H, H, 3 * H, 0, s);
-    if (rc) return rc;
-    rc = pack_matrix<float>(static_cast<const float*>(h2h), static_cast<float*>(Wp), 1, H, H, 3 * H, 2 * H, s);
-  } else {
-    rc = pack_matrix<uint16_t>(static_cast<const uint16_t*>(i2h), static_cast<uint16_t*>(Wp), 1, 2 * H, H, 3 * H, 0, s);
-    if (rc) return rc;
-    rc = pack_matrix<uint16_t>(static_cast<const uint16_t*>(h2h), static_cast<uint16_t*>(Wp), 1, H, H, 3 * H, 2 * H, s);
-  }
-  return rc;
+  const TransposeArgs a = {{i2h, h2h}, {2 * H, H}, {0, 2 * H}, 2, 1, H, H, 3 * H, Wp, 0};
+  return pack_stack(a, 1, dtype, s);
 }
 
 // Tanh RNN cell: Wp[u, k] = W[k, u] for k < I, U[k - I, u] for the H recurrent inputs behind them.
 int pack_rnn(const void* W, const void* U, void* Wp, int I, int H, int dtype, cudaStream_t s) {
-  int rc;
-  if (dtype_size(dtype) == 4) {
-    rc = pack_matrix<float>(static_cast<const float*>(W), static_cast<float*>(Wp), 1, I, H, I + H, 0, s);
-    if (rc) return rc;
-    rc = pack_matrix<float>(static_cast<const float*>(U), static_cast<float*>(Wp), 1, H, H, I + H, I, s);
-  } else {
-    rc = pack_matrix<uint16_t>(static_cast<const uint16_t*>(W), static_cast<uint16_t*>(Wp), 1, I, H, I + H, 0, s);
-    if (rc) return rc;
-    rc = pack_matrix<uint16_t>(static_cast<const uint16_t*>(U), static_cast<uint16_t*>(Wp), 1, H, H, I + H, I, s);
-  }
-  return rc;
+  const TransposeArgs a = {{W, U}, {I, H}, {0, I}, 2, 1, H, H, I + H, Wp, 0};
+  return pack_stack(a, 1, dtype, s);
 }
 
 }  // namespace ftb
