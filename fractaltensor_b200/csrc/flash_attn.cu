@@ -14,7 +14,8 @@
 // the reference's online softmax (kaleido/core/device/kernels/online_softmax.h:15-112).
 //
 // One CTA handles 256 query rows of one (batch, head): two 128-row query tiles
-// that ping-pong through the tensor pipe.
+// that ping-pong through the tensor pipe (or, where those CTAs would be too few, 128 rows whose keys
+// its two slots share: kHalves below).
 //   warp 0        TMA producer: Q tiles, ring of K and V tiles
 //   warp 1        MMA issuer: S_t = Q_t K^T and O_t += P_t V, accumulators in TMEM
 //   warps 2..9    softmax of query tile 0: two threads per query row, one per half
@@ -31,6 +32,9 @@
 // row-major tile.  Per query tile the tensor pipe sees S(j), [softmax], PV(j),
 // S(j+1), ...; the two query tiles are offset so that one is in its softmax while
 // the other one's MMAs run.
+#include <algorithm>
+#include <cmath>
+
 #include "../../include/ftb200.h"
 #include "ptx.cuh"
 #include "tmap.h"
@@ -40,7 +44,7 @@ namespace {
 
 constexpr int kHalfBytes = 128 * 128;  // 128 rows x 64 16-bit columns
 constexpr int kTileBytes = 2 * kHalfBytes;
-constexpr int kKVSlots = 5;
+constexpr int kKVSlots = 5, kMostSlots = 6;
 constexpr int kThreads = 64 + 512;
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kCausalGroup = 16;   // (batch, head) entries whose CTAs are ordered longest first together
@@ -50,13 +54,14 @@ constexpr int kCausalGroup = 16;   // (batch, head) entries whose CTAs are order
 struct Control {
   float xchg[2][2][128];  // [query tile][key half][row]: partial row maximum / row sum
   uint64_t q_full;
-  uint64_t kv_full[kKVSlots], kv_empty[kKVSlots];
+  uint64_t kv_full[kMostSlots], kv_empty[kMostSlots];
   uint64_t s_full[2], p_full[2], pv_done[2], o_staged[2];
   uint64_t pair_bar[2][4];  // [query tile][TMEM lane quadrant]: the two warps that share 32 rows
   uint32_t tmem_base;
-  int abort;
+  int abort, dead;
 };
 constexpr uint32_t kTilesBytes = (2 + kKVSlots) * kTileBytes;  // Q0, Q1 (reused as output staging), KV ring
+static_assert(2 + kKVSlots == 1 + kMostSlots, "one query tile leaves room for one K/V tile more");
 constexpr uint32_t kSmemBytes = 232448;                        // everything an SM offers one CTA
 static_assert(kTilesBytes + sizeof(Control) + 512 <= kSmemBytes, "shared memory budget");
 
@@ -88,30 +93,50 @@ __device__ unsigned long long g_fa_trace[2][32][8];
 #define FA_STAMP_MMA(tt, jj, k)
 #endif
 
-template <typename T, bool kMasked>
+// kHalves: both query slots of a CTA hold the same 128 rows, slot 0 walks the first half of their key/value blocks and
+// slot 1 the second, and the two results are put together in shared memory at the end.  A CTA's time is set by its
+// slots' chains, not by the tensor pipe, so that half the blocks are half the time; the price is that a K/V tile
+// serves one slot and not two.  For calls whose query tiles leave SMs idle (halved_walks below).
+// The K/V stream of a walk of n0 and n1 blocks (n1 = n0 or n0 - 1): K(0,0), K(1,0), then for j = 0, 1, ..: V(0,j),
+// K(0,j+1), V(1,j), K(1,j+1), without the tiles that do not exist.
+struct StreamTile {
+  int t, j;
+  bool is_v;
+};
+__device__ __forceinline__ StreamTile stream_tile(int n, int n0, int n1) {
+  if (n == 0) return {0, 0, false};
+  if (n == 1) return n1 > 0 ? StreamTile{1, 0, false} : StreamTile{0, 0, true};
+  const int j = (n - 2) >> 2, r = (n - 2) & 3;
+  if (n1 == n0 && j == n0 - 1) return {r, j, true};               // nothing follows the last two values
+  if (n1 < n0 && j == n0 - 2 && r == 3) return {0, n0 - 1, true};  // slot 1 has ended: slot 0's last values
+  return {r >> 1, (r & 1) != 0 ? j + 1 : j, (r & 1) == 0};
+}
+
+template <typename T, bool kMasked, bool kHalves>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                   const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, int S,
                   int n_bh, int group, int left, int right, float scale_log2, int* __restrict__ status) {
+  constexpr int kSlots = kHalves ? kMostSlots : kKVSlots;
+  constexpr int kRows = kHalves ? 128 : 256;  // query rows of a CTA
   extern __shared__ uint8_t smem_raw[];
-
-  if (*reinterpret_cast<volatile int*>(status) != 0) return;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   if (pad + kTilesBytes + sizeof(Control) > kSmemBytes) {
     // The dynamic segment starts later than this layout allows for: report, do not run.
+    grid_dependency_wait();
     if (threadIdx.x == 0) atomicCAS(status, 0, FTB_ERR_ALIGN);
     return;
   }
   uint8_t* smem = smem_raw + pad;
-  uint8_t* sQ = smem;                      // 2 tiles
-  uint8_t* sKV = sQ + 2 * kTileBytes;      // ring
+  uint8_t* sQ = smem;                                 // one or two tiles
+  uint8_t* sKV = sQ + (kRows / 128) * kTileBytes;     // ring
   Control& ctl = *reinterpret_cast<Control*>(smem + kTilesBytes);
   volatile int* s_abort = &ctl.abort;
 
-  const int pairs = S / 256;
+  const int pairs = S / kRows;
   int bh = blockIdx.x / pairs;
   int qpair = blockIdx.x - bh * pairs;
   if (kMasked) {
@@ -126,14 +151,18 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     bh = g * group + r % gsize;
   }
   const int row_base = bh * S;            // first row of this (batch, head) in the flattened [B*heads*S, d] view
-  const int q_row0 = row_base + qpair * 256;
+  const int q_row0 = row_base + qpair * kRows;
   // Key/value blocks this CTA walks.  Masked: query i sees keys i-left .. i+right (left < 0: no
   // lower limit; causal attention is left < 0, right = 0).  A query tile walks from the block of the
   // first key its first row sees to the block of the last key its last row sees.  The CTA walks the
   // union, blocks [blk0, blk0 + n_kv); tile 0 takes part in iterations 0..last0 of that walk, tile 1
   // in first1..n_kv-1 (tile 1 starts and ends at most one block after tile 0).
   int blk0 = 0, n_kv = S / 128, first1 = 0, last0 = n_kv - 1;
-  if (kMasked) {
+  if (kMasked && kHalves) {
+    const int r0 = qpair * 128;
+    blk0 = left >= 0 ? max(0, r0 - left) >> 7 : 0;
+    n_kv = min(S / 128 - 1, (r0 + 127 + right) >> 7) - blk0 + 1;
+  } else if (kMasked) {
     const int r0 = qpair * 256;
     const int lo0 = left >= 0 ? max(0, r0 - left) >> 7 : 0;
     const int lo1 = left >= 0 ? max(0, r0 + 128 - left) >> 7 : 0;
@@ -144,14 +173,16 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     first1 = lo1 - lo0;
     last0 = hi0 - lo0;
   }
+  const int n1 = kHalves ? n_kv / 2 : 0, n0 = n_kv - n1;  // halves: blocks of a slot
 
+  grid_launch_dependents();
   if (threadIdx.x == 0) {
     prefetch_tmap(&mapQ);
     prefetch_tmap(&mapK);
     prefetch_tmap(&mapV);
     prefetch_tmap(&mapO);
     mbar_init(&ctl.q_full, 1);
-    for (int i = 0; i < kKVSlots; ++i) {
+    for (int i = 0; i < kSlots; ++i) {
       mbar_init(&ctl.kv_full[i], 1);
       mbar_init(&ctl.kv_empty[i], 1);
     }
@@ -159,32 +190,44 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       mbar_init(&ctl.s_full[i], 1);
       mbar_init(&ctl.p_full[i], 8);
       mbar_init(&ctl.pv_done[i], 1);
-      mbar_init(&ctl.o_staged[i], 8);
+      mbar_init(&ctl.o_staged[i], kHalves ? 16 : 8);
       for (int k = 0; k < 4; ++k) mbar_init(&ctl.pair_bar[i][k], 2);
     }
     ctl.abort = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  // K0, V0, K1, V1, ... stream: tile n into ring slot n % kKVSlots.
+  // K0, V0, K1, V1, ... stream (halves: stream_tile): tile n into ring slot n % kSlots.
   auto load_kv = [&](int n) {
-    const int slot = n % kKVSlots;
+    const int slot = n % kSlots;
     uint8_t* dst = sKV + slot * kTileBytes;
-    const CUtensorMap* m = (n & 1) ? &mapV : &mapK;
-    const int r = row_base + (blk0 + (n >> 1)) * 128;
+    bool is_v = (n & 1) != 0;
+    int block = n >> 1;
+    if (kHalves) {
+      const StreamTile x = stream_tile(n, n0, n1);
+      is_v = x.is_v;
+      block = x.j + (x.t != 0 ? n0 : 0);
+    }
+    const CUtensorMap* m = is_v ? &mapV : &mapK;
+    const int r = row_base + (blk0 + block) * 128;
     mbar_arrive_expect_tx(&ctl.kv_full[slot], kTileBytes);
     tma_load_2d(dst, m, &ctl.kv_full[slot], 0, r);
     tma_load_2d(dst + kHalfBytes, m, &ctl.kv_full[slot], 64, r);
   };
-  const int n_pre = min(kKVSlots, 2 * n_kv);
+  const int n_pre = min(kSlots, 2 * n_kv);
+  // Everything above touches no global memory: it runs while the kernel before this one in the stream drains.
+  grid_dependency_wait();
   if (threadIdx.x == 0) {
-    // Q and the first pass over the (empty) ring are on their way while TMEM is allocated.
-    mbar_arrive_expect_tx(&ctl.q_full, 2 * kTileBytes);
-    for (int t = 0; t < 2; ++t) {
-      tma_load_2d(sQ + t * kTileBytes, &mapQ, &ctl.q_full, 0, q_row0 + t * 128);
-      tma_load_2d(sQ + t * kTileBytes + kHalfBytes, &mapQ, &ctl.q_full, 64, q_row0 + t * 128);
+    ctl.dead = *reinterpret_cast<volatile int*>(status) != 0;  // an earlier wait ran out: do nothing
+    if (!ctl.dead) {
+      // Q and the first pass over the (empty) ring are on their way while TMEM is allocated.
+      mbar_arrive_expect_tx(&ctl.q_full, (kRows / 128) * kTileBytes);
+      for (int t = 0; t < kRows / 128; ++t) {
+        tma_load_2d(sQ + t * kTileBytes, &mapQ, &ctl.q_full, 0, q_row0 + t * 128);
+        tma_load_2d(sQ + t * kTileBytes + kHalfBytes, &mapQ, &ctl.q_full, 64, q_row0 + t * 128);
+      }
+      for (int n = 0; n < n_pre; ++n) load_kv(n);
     }
-    for (int n = 0; n < n_pre; ++n) load_kv(n);
   }
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, 512);
@@ -194,19 +237,20 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl.tmem_base;
+  const bool dead = ctl.dead != 0;
   // TMEM columns: S0 [0,128), S1 [128,256), O0 [256,384), O1 [384,512).  P_t (16-bit pairs)
   // overlays S_t: keys 0..63 in columns [0,32), keys 64..127 in columns [64,96), i.e. each
   // half of the row over the S columns its own thread has read.
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (lane == 0 && !dead) {
       int slot = 0;
       uint32_t phase = 1;  // the first pass was issued above
       for (int n = n_pre; n < 2 * n_kv; ++n) {
         if (!mbar_wait(&ctl.kv_empty[slot], phase ^ 1u, s_abort, status, FTB_ERR_TIMEOUT_SLOT)) break;
         load_kv(n);
-        if (++slot == kKVSlots) {
+        if (++slot == kSlots) {
           slot = 0;
           phase ^= 1u;
         }
@@ -226,20 +270,20 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       const uint64_t dK = make_sdesc_sw128(smem_u32(sKV), 16, 1024);
       const uint64_t dV = make_sdesc_sw128(smem_u32(sKV), kHalfBytes, 1024);
       uint32_t full_bits = 0;  // bit s: parity of the next fill of slot s
-      bool ok = mbar_wait_warp(&ctl.q_full, 0, s_abort, status, FTB_ERR_TIMEOUT_TMA);
+      bool ok = !dead && mbar_wait_warp(&ctl.q_full, 0, s_abort, status, FTB_ERR_TIMEOUT_TMA);
 
       // (No tcgen05 fence after these waits: TMA completes the barriers, and the fence would drain the
       // tensor pipe.)
       auto wait_slot = [&](int n) -> bool {  // n-th tile of the K0, V0, K1, V1, ... stream
-        const int slot = n % kKVSlots;
+        const int slot = n % kSlots;
         if (!mbar_wait_warp(&ctl.kv_full[slot], (full_bits >> slot) & 1u, s_abort, status, FTB_ERR_TIMEOUT_TMA)) return false;
         full_bits ^= 1u << slot;
         return true;
       };
-      // S_t(j) = Q_t . K_j^T
-      auto issue_s = [&](int t, int j) {
-        const uint64_t dq = dQ + static_cast<uint64_t>((t * kTileBytes) >> 4);
-        const uint64_t dk = dK + static_cast<uint64_t>((((2 * j) % kKVSlots) * kTileBytes) >> 4);
+      // S_t = Q_t . K^T, K in ring slot `slot`
+      auto issue_s = [&](int t, int slot) {
+        const uint64_t dq = dQ + static_cast<uint64_t>(kHalves ? 0 : (t * kTileBytes) >> 4);
+        const uint64_t dk = dK + static_cast<uint64_t>((slot * kTileBytes) >> 4);
         if (leader) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
@@ -249,11 +293,11 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           umma_commit(&ctl.s_full[t]);
         }
       };
-      // O_t += P_t(j) . V_j: A = P_t from TMEM (16 keys = 8 packed columns per step; the two
+      // O_t += P_t . V: A = P_t from TMEM (16 keys = 8 packed columns per step; the two
       // key halves start 64 columns apart); B = V, MN-major: 16 keys = two 8-row groups
       // (1024 B apart), the two 64-column halves of d are 16 KB apart.
-      auto issue_pv = [&](int t, int j, bool first) {
-        const uint64_t dv = dV + static_cast<uint64_t>((((2 * j + 1) % kKVSlots) * kTileBytes) >> 4);
+      auto issue_pv = [&](int t, int slot, bool first) {
+        const uint64_t dv = dV + static_cast<uint64_t>((slot * kTileBytes) >> 4);
         if (leader) {
 #pragma unroll
           for (int k = 0; k < 8; ++k)
@@ -263,6 +307,39 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
         }
       };
 
+      if constexpr (kHalves) {
+        int n = 0, slot = 0;  // of the stream; every tile serves one product
+        auto next = [&] {
+          if (leader) umma_commit(&ctl.kv_empty[slot]);
+          ++n;
+          if (++slot == kSlots) slot = 0;
+        };
+        for (int t = 0; t < 2 && ok; ++t)
+          if (t == 0 || n1 > 0) {
+            ok = wait_slot(n);
+            if (ok) {
+              issue_s(t, slot);
+              next();
+            }
+          }
+        for (int j = 0; j < n0 && ok; ++j)
+          for (int t = 0; t < 2 && ok; ++t) {
+            const int mine = t == 0 ? n0 : n1;
+            if (j >= mine) continue;
+            ok = wait_slot(n) && mbar_wait_warp(&ctl.p_full[t], j & 1, s_abort, status, FTB_ERR_TIMEOUT_EPI);
+            if (!ok) break;
+            tc_fence_after();
+            issue_pv(t, slot, j == 0);
+            next();
+            if (j + 1 < mine) {
+              ok = wait_slot(n);
+              if (!ok) break;
+              issue_s(t, slot);
+              next();
+            }
+          }
+        ok = false;
+      }
       if (ok) ok = wait_slot(0);
       if (ok) {
         issue_s(0, 0);
@@ -284,16 +361,16 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             }
             tc_fence_after();
             FA_STAMP_MMA(t, j, 5);
-            issue_pv(t, j, j == first);
+            issue_pv(t, (2 * j + 1) % kSlots, j == first);
           }
           // The tensor pipe runs MMAs in issue order: S_t(j+1) overwrites S_t / P_t only after
           // PV_t(j) has read P_t.
-          if (more && j + 1 >= first && j + 1 <= last) issue_s(t, j + 1);
+          if (more && j + 1 >= first && j + 1 <= last) issue_s(t, (2 * j + 2) % kSlots);
           FA_STAMP_MMA(t, j, 6);
         }
         if (!ok) break;
-        if (leader) umma_commit(&ctl.kv_empty[(2 * j + 1) % kKVSlots]);
-        if (leader && more) umma_commit(&ctl.kv_empty[(2 * j + 2) % kKVSlots]);
+        if (leader) umma_commit(&ctl.kv_empty[(2 * j + 1) % kSlots]);
+        if (leader && more) umma_commit(&ctl.kv_empty[(2 * j + 2) % kSlots]);
       }
     }
   } else {
@@ -310,10 +387,10 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     const float* peer_x = &ctl.xchg[t][h ^ 1][row];
     uint64_t* pair = &ctl.pair_bar[t][q];
     float m_used = 0.f, l = 0.f;
-    bool ok = true;
-    const int j_first = t == 0 ? 0 : first1;
-    const int j_last = t == 0 ? last0 : n_kv - 1;
+    const int j_first = kHalves || t == 0 ? 0 : first1;
+    const int j_last = kHalves ? (t == 0 ? n0 : n1) - 1 : (t == 0 ? last0 : n_kv - 1);
     const int n_mine = j_last - j_first + 1;
+    bool ok = !dead && n_mine > 0;
 
     for (int j = j_first; j <= j_last && ok; ++j) {
       const int it = j - j_first;  // this tile's block count so far: the phase of its barriers
@@ -331,8 +408,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       if (kMasked) {
         // This thread's 64 keys start at key0; its query is `mine`.  Columns below lo_col are before
         // the window, columns above hi_col after it (for causal attention: after the query).
-        const int key0 = (blk0 + j) * 128 + h * 64;
-        const int mine = qpair * 256 + t * 128 + row;
+        const int key0 = (blk0 + j + (kHalves && t != 0 ? n0 : 0)) * 128 + h * 64;
+        const int mine = qpair * kRows + (kHalves ? 0 : t * 128) + row;
         const int lo_col = left >= 0 ? mine - left - key0 : 0;
         const int hi_col = mine + right - key0;
         if (__any_sync(0xffffffffu, lo_col > 0)) {
@@ -370,7 +447,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       mx = fmaxf(mx, *peer_x);
       // A row can have no visible key in a block of its tile's walk: the floor keeps 2^(s - m) at 0
       // there instead of inf - inf, and the first real maximum rescales the (zero) accumulator by 0.
-      const float m_new = kMasked ? fmaxf(mx * scale_log2, -1e30f) : mx * scale_log2;
+      // (Halves: nor need the keys of one half count beside the other's.)
+      const float m_new = kMasked || kHalves ? fmaxf(mx * scale_log2, -1e30f) : mx * scale_log2;
       if (it == 0) {
         m_used = m_new;
       } else {
@@ -438,6 +516,73 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       ok = __all_sync(0xffffffffu, mbar_wait(pair, n_mine & 1, s_abort, status, FTB_ERR_TIMEOUT_EPI));
       if (ok) l += *peer_x;
     }
+    if constexpr (kHalves) {
+      // Both slots' last PV MMAs are done: the accumulators are at rest, and Q and the K/V ring are dead.  (The MMAs
+      // run in the order of their issue, so that the other slot's barrier is one phase behind at most.)
+      const bool empty = n_mine <= 0;  // one block in all: slot 1 has none
+      const int n_other = t == 0 ? n1 : n0;
+      bool fine = empty ? !dead : ok;
+      if (fine && !empty) fine = mbar_wait(&ctl.pv_done[t], (n_mine - 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_MMA);
+      if (fine && n_other > 0)
+        fine = mbar_wait(&ctl.pv_done[t ^ 1], (n_other - 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_MMA);
+      fine = __all_sync(0xffffffffu, fine);
+      tc_fence_after();
+      // A thread finishes 32 of its 64 columns, slot 0 the lower and slot 1 the upper ones, and gives the others to the
+      // thread of the other slot: [slot][key half][column / 4][row], 512 bytes a warp's access; then (m, l) of the rows.
+      float4* give = reinterpret_cast<float4*>(sKV);
+      float2* sums = reinterpret_cast<float2*>(sKV + 2 * kTileBytes);
+      if (empty) m_used = -1e30f;
+      if (fine) {
+        uint32_t o[32];
+        tmem_ld32(o_addr + (t ^ 1) * 32, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          give[((t * 2 + h) * 8 + c) * 128 + row] =
+              empty ? make_float4(0.f, 0.f, 0.f, 0.f)
+                    : make_float4(__uint_as_float(o[4 * c]), __uint_as_float(o[4 * c + 1]), __uint_as_float(o[4 * c + 2]),
+                                  __uint_as_float(o[4 * c + 3]));
+        if (h == 0) sums[t * 128 + row] = make_float2(m_used, l);
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");  // (every softmax warp comes here, whatever its waits said)
+      if (fine && *s_abort == 0) {
+        const float2 other = sums[(t ^ 1) * 128 + row];
+        const float m = fmaxf(m_used, other.x), keep = exp2_fast(m_used - m), take = exp2_fast(other.x - m);
+        const float inv_l = 1.f / (l * keep + other.y * take);
+        uint32_t o[32];
+        tmem_ld32(o_addr + t * 32, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float x[8];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float4 p = give[(((t ^ 1) * 2 + h) * 8 + 2 * c + k) * 128 + row];
+            const float q4[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              x[4 * k + i] = (empty ? q4[i] * take : fmaf(__uint_as_float(o[8 * c + 4 * k + i]), keep, q4[i] * take)) * inv_l;
+          }
+          uint4 u;
+          u.x = Fmt<T>::pack2(x[0], x[1]);
+          u.y = Fmt<T>::pack2(x[2], x[3]);
+          u.z = Fmt<T>::pack2(x[4], x[5]);
+          u.w = Fmt<T>::pack2(x[6], x[7]);
+          *reinterpret_cast<uint4*>(sw128_chunk_ptr(sQ, row, h * 8 + t * 4 + c)) = u;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.o_staged[0]);
+        if (lane == 0 && t == 0 && h == 0 && q == 2 &&
+            mbar_wait(&ctl.o_staged[0], 0, s_abort, status, FTB_ERR_TIMEOUT_EPI)) {
+          tma_store_2d(&mapO, sQ, 0, q_row0);
+          tma_store_2d(&mapO, sQ + kHalfBytes, 64, q_row0);
+          tma_store_commit();
+          tma_store_wait_read<0>();
+        }
+      }
+      ok = false;
+    }
     // Final: O_t / l -> 16-bit -> staging (the Q tile, dead once the last PV is done) -> TMA store.
     if (ok && __all_sync(0xffffffffu,
                          mbar_wait(&ctl.pv_done[t], (n_mine - 1) & 1, s_abort, status, FTB_ERR_TIMEOUT_MMA))) {
@@ -485,16 +630,61 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
   }
 }
 
-template <typename T, bool kMasked>
+template <typename T, bool kMasked, bool kHalves>
 int launch(const CUtensorMap& mQ, const CUtensorMap& mK, const CUtensorMap& mV, const CUtensorMap& mO, int n_bh,
            int S, int left, int right, float scale_log2, int* status, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  auto kfn = flash_attn_kernel<T, kMasked>;
+  auto kfn = flash_attn_kernel<T, kMasked, kHalves>;
   if (!ensure_dynamic_smem(kfn, kSmemBytes, configured)) return FTB_ERR_LAUNCH;
   const int group = kCausalGroup;
-  kfn<<<n_bh * (S / 256), kThreads, kSmemBytes, stream>>>(mQ, mK, mV, mO, S, n_bh, group, left, right, scale_log2, status);
+  const cudaError_t err = launch_dependent(kfn, dim3(n_bh * (S / (kHalves ? 128 : 256))), dim3(kThreads), kSmemBytes, stream,
+                                           mQ, mK, mV, mO, S, n_bh, group, left, right, scale_log2, status);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+  if (err != cudaSuccess) cudaGetLastError();
+  return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+}
+
+template <typename T>
+int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& mK, const CUtensorMap& mV,
+           const CUtensorMap& mO, int n_bh, int S, int left, int right, float scale_log2, int* status, cudaStream_t stream) {
+  if (masked)
+    return halves ? launch<T, true, true>(mQ, mK, mV, mO, n_bh, S, left, right, scale_log2, status, stream)
+                  : launch<T, true, false>(mQ, mK, mV, mO, n_bh, S, left, right, scale_log2, status, stream);
+  return halves ? launch<T, false, true>(mQ, mK, mV, mO, n_bh, S, -1, 0, scale_log2, status, stream)
+                : launch<T, false, false>(mQ, mK, mV, mO, n_bh, S, -1, 0, scale_log2, status, stream);
+}
+
+// Whether a call's CTAs take 128 query rows and half of their blocks a slot, or 256 rows and all of them: by the
+// estimates of both.  A CTA takes kFixed us and kBlock for each block of its longer slot; where there are more CTAs than
+// SMs, equal ones go in whole waves, unequal ones (masks), longest first, about half of one beyond their mean.
+// Measured, us, 256 rows / 128 rows (* taken), 1 x heads x S: causal 16 x 2048 35.3 / 27.1*, 8 x 1024 19.5 / 14.3*, 4 x 4096
+// 63.6 / 37.9*, 32 x 2048 40.2* / 53.6, 64 x 2048 82.2* / 102.6; full 16 x 256 8.3 / 7.5*, 16 x 1024 20.4 / 15.0*, 16 x 2048
+// 36.5* / 43.6 (two waves of 128 rows), 20 x 2048 66.9 / 62.3* (two waves / three), 12 x 4096 130.7 / 112.5*; window of 600
+// 8 x 2048 19.6 / 13.7*, keys i-1000..i+500 8 x 4096 32.9* / 39.7.
+bool halved_walks(bool masked, int n_bh, int S, int left, int right, int sm_count) {
+  constexpr double kFixed = 4.5, kBlock = 1.9;
+  double us[2];
+  for (int halves = 0; halves < 2; ++halves) {
+    const int rows = halves ? 128 : 256, tiles = S / rows;
+    double total = 0, longest = 0;
+    for (int i = 0; i < tiles; ++i) {
+      const int r0 = i * rows;
+      const int lo = masked && left >= 0 && r0 > left ? (r0 - left) >> 7 : 0;
+      const int hi = masked && r0 + rows - 1 < S - right ? (r0 + rows - 1 + right) >> 7 : S / 128 - 1;
+      const int blocks = halves ? (hi - lo + 2) / 2 : hi - lo + 1;
+      const double t = kFixed + kBlock * blocks;
+      total += t;
+      if (t > longest) longest = t;
+    }
+    const double waves = static_cast<double>(n_bh) * tiles / sm_count;
+    if (waves <= 1)
+      us[halves] = longest;
+    else if (masked)
+      us[halves] = std::max(longest, (waves + 0.5) * total / tiles);
+    else
+      us[halves] = std::ceil(waves) * longest;
+  }
+  return us[1] < us[0];
 }
 
 }  // namespace
@@ -536,13 +726,10 @@ int flash_attn_entry(const void* q, const void* k, const void* v, void* o, int B
   if ((rc = make_tmap_2d(&mO, o, dtype, rows, d, d, 128, 64))) return rc;
   const int units = B * heads;
   const float scale_log2 = scale * 1.4426950408889634f;
-  if (masked) {
-    if (dtype == FTB_F16)
-      return launch<__half, true>(mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
-    return launch<__nv_bfloat16, true>(mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
-  }
-  if (dtype == FTB_F16) return launch<__half, false>(mQ, mK, mV, mO, units, S, -1, 0, scale_log2, status, stream);
-  return launch<__nv_bfloat16, false>(mQ, mK, mV, mO, units, S, -1, 0, scale_log2, status, stream);
+  const bool halves = halved_walks(masked, units, S, left, right, current_sm_count());
+  if (dtype == FTB_F16)
+    return launch<__half>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
+  return launch<__nv_bfloat16>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
 }
 }  // namespace
 
