@@ -13,14 +13,13 @@
 //   * h_t goes from the epilogue's registers straight into the next step's B operand in every CTA
 //     of the cluster: a thread holds 8 sequences of one unit, which is one 16-byte row of the
 //     MN-major core matrix, and sends it with st.async, its bytes counted on the receiver's mbarrier
-//     of that source CTA.  No staging tile, no barrier between the epilogue warps; the MMAs over a
-//     source's units start as soon as that source has arrived, the CTA's own units first.
+//     of that source CTA.  No staging tile, no barrier between the epilogue warps.
 // The two state slots need no release: a CTA's step-t output is complete only after it has received
 // every peer's step t-1 output, that is after every peer has multiplied what slot t & 1 held before.
 // The MMA warp keeps all its lanes in the loop: with one lane alone in it the descriptors were
 // divergent values, moved to uniform registers before every MMA (67 cycles an MMA, 2.54 us a step).
-// Measured (H 512, 64 sequences, bf16): 1.88 us a step; 50 steps as launches of the cell kernel 370 us,
-// here 94 us and 9 us for the product of the input halves.
+// Measured (H 512, 64 sequences, bf16): 1.5 us a step; 50 steps as launches of the cell kernel 370 us,
+// here 74 us and 7 us for the product of the input halves.
 //
 // Program: src_enc_outs = map(scan(cell)) of examples/rnn_attention/rnn_attention.py:40-48, 86-110.
 #include "../../include/ftb200.h"
@@ -134,13 +133,19 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
       } else if (lane < a.CL) {
         mbar_arrive_expect_tx(&full[slot][lane], static_cast<uint32_t>(min(128, a.H - 128 * lane)) * kNB * 2);
       }
-      for (int r = 0; r < a.CL; ++r) {
-        if (i > 0) {
-          ok = ok && mbar_wait_cluster(&full[slot][r], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
-          fence_proxy_async_smem();  // the state was stored by threads, the MMA reads it by the async proxy
-        }
-        if (!__all_sync(0xffffffffu, ok)) break;
-        if (r == 0) tc_fence_after();
+      // All sources at once, a lane each: a wait and a fence for each of them, in turn, cost 360 cycles a source where the
+      // MMAs behind them take 90 (H 512: a step 2690 cycles, so 2350).
+      if (i > 0) {
+        if (lane < a.CL)
+          ok = ok && mbar_wait_cluster(&full[slot][lane], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+        __syncwarp();
+        fence_proxy_async_smem();  // the state was stored by threads, the MMA reads it by the async proxy
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int r = 0; r < kMaxCtas; ++r) {
+        if (r >= a.CL) break;
         const uint64_t bd = bdesc0 + static_cast<uint64_t>((slot * slot_bytes + r * 16 * kCoreK) >> 4);
         const uint32_t aw = tmem_w + r * 64;
         if (128 * r + 128 <= a.H) {
@@ -155,7 +160,6 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
             umma_ts(d_tmem, aw + 8 * j, bd + j * ((2 * kCoreK) >> 4), idesc, 1u);
         }
       }
-      if (!__all_sync(0xffffffffu, ok)) break;
       if (leader) umma_commit(&acc_full[i & 1]);
     }
   } else if (warp >= kFirstEpi) {
@@ -202,6 +206,17 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
     const float* pre = a.pre + static_cast<size_t>(n0) * a.H + u;
     T* out = reinterpret_cast<T*>(a.out) + static_cast<size_t>(n0) * a.H + u;
     const uint32_t my_chunk = smem_u32(slots) + (u >> 3) * kCoreK + half * 128 + (u & 7) * 16;
+    // Where the states go: every CTA of the cluster, its own first (slot 0; slot 1 behind it).
+    uint32_t to[kMaxCtas], to_bar[kMaxCtas];
+#pragma unroll
+    for (int k = 0; k < kMaxCtas; ++k) {
+      const int r = rank + k < a.CL ? rank + k : rank + k - a.CL;
+      to[k] = to_bar[k] = 0;
+      if (k < a.CL) {
+        to[k] = map_to_cta(my_chunk, r);
+        to_bar[k] = map_to_cta(smem_u32(&full[0][rank]), r);
+      }
+    }
     float p[8];
     auto load_pre = [&](int i) {
 #pragma unroll
@@ -253,12 +268,10 @@ __global__ void __launch_bounds__(kThreads, 1) rnn_chain_kernel(const ChainArgs 
       for (int n = 0; n < 4; ++n)
         h[n] = Fmt<T>::pack2(tanh_fast(v[2 * n] + bias), tanh_fast(v[2 * n + 1] + bias));
       if (i + 1 < steps) {
-        const uint32_t dst = my_chunk + (i & 1) * slot_bytes, bar = smem_u32(&full[i & 1][rank]);
-        for (int k = 0; k < a.CL; ++k) {
-          int r = rank + k;
-          if (r >= a.CL) r -= a.CL;
-          st_async16(map_to_cta(dst, r), map_to_cta(bar, r), h);
-        }
+#pragma unroll
+        for (int k = 0; k < kMaxCtas; ++k)
+          if (k < a.CL)
+            st_async16(to[k] + (i & 1) * slot_bytes, to_bar[k] + (i & 1) * static_cast<uint32_t>(sizeof(full[0])), h);
       }
       if (i + 2 < steps) {
         begin_acc(i + 2);  // (the accumulator just read)
