@@ -14,7 +14,7 @@
 //     layer, the recurrent K blocks first in tensor memory, the rest of them and the input blocks in
 //     the tensor memory left, then in shared memory;
 //   * the batch is cut into slices of NB columns that never meet (UMMA N = NB), each with its own CTAs.
-//     What grows with NB is the state a CTA reads (36 bytes a cycle) and its tanh's (8 a cycle): slices are
+//     What grows with NB is the state a CTA reads and its gates (20 cycles a column, tanh's 16 a cycle): slices are
 //     as narrow as the device has CTAs for;
 //   * the warps that have stored a step's state read the whole of it back: the chain is one set of warps
 //     with no hand-over but the accumulator's barrier and the operand tile's.  They wait before the

@@ -215,6 +215,12 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         blocks_ts(d_tmem, tmem_w + rec_t * 32, xd, in_t, 0u);
         blocks_ss(d_tmem, w_desc + static_cast<uint64_t>(((kb_h - rec_t) * kWBlockBytes) >> 4), xd + in_t * kBlockDesc,
                   kb_x - in_t, in_t > 0 ? 1u : 0u);
+        // Where there is one input tile it goes back behind the recurrent half, not before it: its next copy would otherwise
+        // be under way while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64
+        // sequences: D8 L100 500 us, behind it 464).  With two, the copy made room for is the one after the next: before
+        // the half it is 1 % faster at H 256.
+        const bool late = a.n_slots == 1;
+        if (!late && leader) umma_commit(&in_empty[slot]);
         if (t > 0) {
           ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           if (!ok) break;
@@ -223,10 +229,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           ++states;
         }
         if (leader) umma_commit(&acc_full[acc]);
-        // The input tile goes back behind the recurrent half, not before it: its next copy would otherwise be under way
-        // while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64 sequences:
-        // D8 L100 505 us, behind it 476).
-        if (leader) umma_commit(&in_empty[slot]);
+        if (late && leader) umma_commit(&in_empty[slot]);
         if (++slot == a.n_slots) {
           slot = 0;
           phase ^= 1u;
