@@ -139,6 +139,18 @@ __device__ __forceinline__ void load_row_shared(const T* row, int gl, float (&ou
     unpack16(w, out + c * (kEPL / Pieces<T>::n), T());
   }
 }
+// The row where `want`, zeros elsewhere, without a branch.
+template <typename T, int LPT>
+__device__ __forceinline__ void load_row_shared_if(bool want, const T* row, int gl, float (&out)[kEPL]) {
+#pragma unroll
+  for (int c = 0; c < Pieces<T>::n; ++c) {
+    uint4 w = make_uint4(0, 0, 0, 0);
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %5, 0;\n@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n}"
+                 : "+r"(w.x), "+r"(w.y), "+r"(w.z), "+r"(w.w)
+                 : "r"(smem_u32(reinterpret_cast<const uint4*>(row) + c * LPT + gl)), "r"(static_cast<int>(want)));
+    unpack16(w, out + c * (kEPL / Pieces<T>::n), T());
+  }
+}
 template <typename T, int LPT>
 __device__ __forceinline__ void store_row_global(T* row, int gl, const float (&in)[kEPL]) {
 #pragma unroll
@@ -485,7 +497,8 @@ __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __r
 
 // The walk of one warp over interior tiles (no global token, no wrapped window position), with the number of random
 // keys known at compile time, and that of window keys (KW > 0) or a bound on it (KW < 0: up to -KW): no per-key
-// bookkeeping, one softmax over the scores.  Window rows and queries come from the stage, random rows from global
+// bookkeeping, one softmax over the scores.  Nothing branches on the window either way: under a bound, rows past the window
+// are loads that do not happen, so the scores' loads, products and shuffles still overlap.  Window rows and queries come from the stage, random rows from global
 // memory.
 //   What bounds it is the latency of the random rows: 6 rows of 256 bytes a token at the example's counts, with 16
 // warps an SM.  So a warp works one pass (32 / LPT tokens) ahead of itself: the random keys of its next pass are
@@ -577,13 +590,13 @@ __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* 
       float sc[NW + KR];
 #pragma unroll
       for (int j = 0; j < NW; ++j) {
-        if (KW < 0 && j >= n_window) {
-          sc[j] = -INFINITY;
-          continue;
-        }
         float kw[kEPL];
-        load_row_shared<T, LPT>(st.k + (row0 + j * a.dilation) * d, gl, kw);
+        if constexpr (KW > 0)
+          load_row_shared<T, LPT>(st.k + (row0 + j * a.dilation) * d, gl, kw);
+        else
+          load_row_shared_if<T, LPT>(j < n_window, st.k + (row0 + j * a.dilation) * d, gl, kw);
         sc[j] = group_dot<LPT>(qv, kw, gmask) * scale2;
+        if (KW < 0 && j >= n_window) sc[j] = -INFINITY;
       }
 #pragma unroll
       for (int r = 0; r < KR; ++r) {
@@ -607,9 +620,11 @@ __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* 
       for (int e = 0; e < kEPL; ++e) acc[e] = 0.f;
 #pragma unroll
       for (int j = 0; j < NW; ++j) {
-        if (KW < 0 && j >= n_window) continue;
-        float vw[kEPL];
-        load_row_shared<T, LPT>(st.v + (row0 + j * a.dilation) * d, gl, vw);
+        float vw[kEPL];  // (zeros where the window is over, as their weights)
+        if constexpr (KW > 0)
+          load_row_shared<T, LPT>(st.v + (row0 + j * a.dilation) * d, gl, vw);
+        else
+          load_row_shared_if<T, LPT>(j < n_window, st.v + (row0 + j * a.dilation) * d, gl, vw);
 #pragma unroll
         for (int e = 0; e < kEPL; ++e) acc[e] = fmaf(sc[j], vw[e], acc[e]);
       }
@@ -701,17 +716,24 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
     }
   }
   if (TT > 0) {
-    static std::atomic<unsigned long long> configured[6];
+    static std::atomic<unsigned long long> configured[13];
     using Kernel = decltype(&sparse_attn_tile_kernel<T, LPT, 0, 0>);
-    // The example's key counts have a routine of their own, 1 to 4 random keys beside a window of up to 7 one
-    // that is told the window's; the rest take the general one, which is issue-bound on its bookkeeping (us, B 2, 16 heads, S 4096, d 64, general /
-    // told the window: window 7 and 4 random keys fp32 67.0 / 53.0, fp16 78.9 / 51.5; 5 and 2 48.4 / 44.4, 54.8 / 39.4;
-    // 3 and 1 34.9 / 30.9, 35.4 / 31.8; the example's 5 and 3, told the window / with its own: fp32 50.7 / 42.9, fp16 39.0 /
-    // 31.6, bf16 36.2 / 30.0).
-    const Kernel kernels[6] = {sparse_attn_tile_kernel<T, LPT, 0, 0>, sparse_attn_tile_kernel<T, LPT, -7, 1>,
-                               sparse_attn_tile_kernel<T, LPT, -7, 2>, sparse_attn_tile_kernel<T, LPT, -7, 3>,
-                               sparse_attn_tile_kernel<T, LPT, -7, 4>, sparse_attn_tile_kernel<T, LPT, 5, 3>};
-    const int fast = a.as_shipped || a.window > 7 || a.R < 1 || a.R > 4 ? 0 : (a.window == 5 && a.R == 3 ? 5 : a.R);
+    // 1 to 4 random keys beside a window of up to 7 have routines with those counts (windows 1 and 3 share one that is
+    // told the window's: 32.4 us for window 1 and 2 random keys, 34.1 under one bound of 7); the rest take the general
+    // one, which is issue-bound on its bookkeeping.  us, B 2, 16 heads, S 4096, d 64, general / one routine told any
+    // window up to 7, each score in a branch of its own / own counts: window 7 and 4 random keys fp32 67.0 / 62.2 /
+    // 53.0, fp16 78.9 / 50.4 / 40.2; 3 and 1 34.9 / 33.6 / 28.9, 35.4 / 29.9 / 24.3; d 128, 5 and 4: 101.6 / 77.3 and
+    // 86.3 / 70.4 told / own.
+    const Kernel kernels[13] = {sparse_attn_tile_kernel<T, LPT, 0, 0>,
+                                sparse_attn_tile_kernel<T, LPT, -3, 1>, sparse_attn_tile_kernel<T, LPT, -3, 2>,
+                                sparse_attn_tile_kernel<T, LPT, -3, 3>, sparse_attn_tile_kernel<T, LPT, -3, 4>,
+                                sparse_attn_tile_kernel<T, LPT, 5, 1>,  sparse_attn_tile_kernel<T, LPT, 5, 2>,
+                                sparse_attn_tile_kernel<T, LPT, 5, 3>,  sparse_attn_tile_kernel<T, LPT, 5, 4>,
+                                sparse_attn_tile_kernel<T, LPT, 7, 1>,  sparse_attn_tile_kernel<T, LPT, 7, 2>,
+                                sparse_attn_tile_kernel<T, LPT, 7, 3>,  sparse_attn_tile_kernel<T, LPT, 7, 4>};
+    const int fast = a.as_shipped || a.window > 7 || a.R < 1 || a.R > 4
+                         ? 0
+                         : (a.window <= 3 ? 0 : (a.window == 5 ? 4 : 8)) + a.R;
     if (ensure_dynamic_smem(kernels[0], kMaxTileSmem, configured[0]) &&
         ensure_dynamic_smem(kernels[fast], kMaxTileSmem, configured[fast])) {
       a.TT = TT;

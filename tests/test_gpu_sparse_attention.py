@@ -213,3 +213,11 @@ def test_interior_walk_reports_positions_outside(ops):
     same = torch.ones(512, dtype=torch.bool)
     same[253] = False
     assert torch.equal(out[0, 0], good[0, 0]) and torch.equal(out[0, 1][same.cuda()], good[0, 1][same.cuda()])
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("R", [1, 2, 3, 4])
+@pytest.mark.parametrize("window", [1, 3, 5, 7])
+def test_every_pair_of_key_counts(ops, dt, window, R):
+    """Each pair of window and random keys that has a routine of its own, with interior and edge tiles."""
+    test_interior_walk_matches_oracle(ops, dt, 1, 3, 261, 64, window, 2, 2, R)
