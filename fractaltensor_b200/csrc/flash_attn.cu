@@ -660,7 +660,9 @@ int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& m
 // Measured, us, 256 rows / 128 rows (* taken), 1 x heads x S: causal 16 x 2048 35.3 / 27.1*, 8 x 1024 19.5 / 14.3*, 4 x 4096
 // 63.6 / 37.9*, 32 x 2048 40.2* / 53.6, 64 x 2048 82.2* / 102.6; full 16 x 256 8.3 / 7.5*, 16 x 1024 20.4 / 15.0*, 16 x 2048
 // 36.5* / 43.6 (two waves of 128 rows), 20 x 2048 66.9 / 62.3* (two waves / three), 12 x 4096 130.7 / 112.5*; window of 600
-// 8 x 2048 19.6 / 13.7*, keys i-1000..i+500 8 x 4096 32.9* / 39.7.
+// 8 x 2048 19.6 / 13.7*, keys i-1000..i+500 8 x 4096 32.9* / 39.7.  Halves that are estimated less than a tenth faster keep the
+// 256 rows: between 0.9 and 1 of the estimate the time is 0.9 to 1.19 of theirs (full 40 x 1024 43.3* / 44.0, 45 x 2048 104.7* /
+// 114.1, 56 x 768 35.1* / 41.7; causal 16 x 2560 54.3* / 48.9), below it 0.53 to 0.97.
 bool halved_walks(bool masked, int n_bh, int S, int left, int right, int sm_count) {
   constexpr double kFixed = 4.5, kBlock = 1.9;
   double us[2];
@@ -684,7 +686,7 @@ bool halved_walks(bool masked, int n_bh, int S, int left, int right, int sm_coun
     else
       us[halves] = std::ceil(waves) * longest;
   }
-  return us[1] < us[0];
+  return us[1] < 0.9 * us[0];
 }
 
 }  // namespace
