@@ -33,6 +33,7 @@
 // S(j+1), ...; the two query tiles are offset so that one is in its softmax while
 // the other one's MMAs run.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "../../include/ftb200.h"
@@ -447,8 +448,9 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       mx = fmaxf(mx, *peer_x);
       // A row can have no visible key in a block of its tile's walk: the floor keeps 2^(s - m) at 0
       // there instead of inf - inf, and the first real maximum rescales the (zero) accumulator by 0.
-      // (Halves: nor need the keys of one half count beside the other's.)
-      const float m_new = kMasked || kHalves ? fmaxf(mx * scale_log2, -1e30f) : mx * scale_log2;
+      // (Halves: nor need the keys of one half count beside the other's.)  It is the lowest finite number:
+      // scores are products of 16-bit numbers, in bf16 of any size, and none that is finite may fall below it.
+      const float m_new = kMasked || kHalves ? fmaxf(mx * scale_log2, -FLT_MAX) : mx * scale_log2;
       if (it == 0) {
         m_used = m_new;
       } else {
@@ -531,7 +533,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
       // thread of the other slot: [slot][key half][column / 4][row], 512 bytes a warp's access; then (m, l) of the rows.
       float4* give = reinterpret_cast<float4*>(sKV);
       float2* sums = reinterpret_cast<float2*>(sKV + 2 * kTileBytes);
-      if (empty) m_used = -1e30f;
+      if (empty) m_used = -FLT_MAX;
       if (fine) {
         uint32_t o[32];
         tmem_ld32(o_addr + (t ^ 1) * 32, o);

@@ -79,3 +79,18 @@ def test_no_key_scores_above_minus_infinity_in_a_half(ops):
     out = ops.flash_attention(q.cuda(), k.cuda(), v.cuda(), scale=0.05)
     ops.check_status()
     assert (out.double().cpu() - ref).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("mask", [{}, dict(causal=True), dict(causal=True, window=300), dict(local=(200, 130))])
+def test_scores_far_below_zero(ops, mask):
+    """Finite scores of -2^106 and one key of -2^105 in bf16: the key whose score is the largest takes all the weight where
+    a query sees it, elsewhere the visible keys share it.  (Powers of two: their product with the scale is exact.)"""
+    S, top = 1024, 600
+    v = dense.make_attention_inputs(1, 1, S, 128, 8, dtype=torch.bfloat16)[2]
+    q, k = torch.zeros_like(v), torch.zeros_like(v)
+    q[..., 0], k[..., 0], k[:, :, top, 0] = 2.0 ** 53, -2.0 ** 53, -2.0 ** 52
+    out = ops.flash_attention(q.cuda(), k.cuda(), v.cuda(), scale=1.0, **mask).double().cpu()
+    ops.check_status()
+    ref = dense.attention_plain(q.double(), k.double(), v.double(), scale=1.0, **mask)
+    # the result is rounded to 8 bits; P, a power of two or equal for all keys, is not in error
+    assert (out - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()
