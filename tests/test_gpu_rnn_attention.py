@@ -203,3 +203,40 @@ def test_vectors_of_all_steps(ops, dt, H, Ls, Lt, lens):
         # fp32 scores of H products (relative 2^-24 * sqrt(H)) in the exponent, then the rounding of the result
         tol = {torch.float32: 1e-5, torch.float16: 1e-3, torch.bfloat16: 8e-3}[dt]
         assert (out[:, n].double().cpu() - ref).abs().max().item() <= tol
+
+
+def _whole(ops, src, trg, q, lens=None):
+    """The C entry itself -> (enc, scores, dec, out), from buffers of sevens."""
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, lib
+    (Ls, N, H), Lt = src.shape, trg.shape[0]
+    buf = lambda *s, dt=src.dtype: torch.full(s, 7.0, dtype=dt, device="cuda")
+    enc, scores, dec, out = buf(Ls, N, H), buf(Ls, N, dt=torch.float32), buf(Lt, N, H), buf(Lt, N, H)
+    bs, bt = (q[k].float().reshape(-1) for k in ("bs", "bt"))
+    Wp_src, Wp_trg = ops.rnn_pack_weights(q["Ws"], q["Us"]), ops.rnn_pack_weights(q["Wt"], q["Ut"])
+    ws = ops.workspace(src.device)
+    check(lib.ftb_rnn_attention_fwd_scratch(_ptr(src), _ptr(trg), _ptr(Wp_src), _ptr(Wp_trg), _ptr(bs), _ptr(bt),
+                                            _ptr(q["enc_proj"]), _ptr(q["dec_proj"]), _ptr(lens), _ptr(enc), _ptr(scores),
+                                            _ptr(dec), _ptr(out), Ls, Lt, N, H, _dtype_code(src), None, 0, _ptr(ws),
+                                            ws.numel(), _stream()), "ftb_rnn_attention_fwd_scratch")
+    ops.check_status()
+    return enc, scores, dec, out
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,Lt", [(1, 33), (2, 700), (1, 5000)])
+def test_steps_shared_by_several_ctas(ops, dt, N, Lt):
+    """A step that is not finite reaches the later ones where other CTAs look at those."""
+    p, g = _params(64, N + Lt, 1.0 / 8)
+    q = {k: v.to(dt).cuda() for k, v in p.items()}
+    src, trg = (torch.randn(n, N, 64, generator=g).to(dt).cuda() for n in (5, Lt))
+    clean = _whole(ops, src, trg, q)
+    assert all(torch.isfinite(t).all() for t in clean)
+    for first in (0, 31, 32, Lt - 1):
+        trg_bad = trg.clone()
+        trg_bad[first, 0, 3] = float("nan")
+        if first + 40 < Lt:
+            trg_bad[first + 40, 0, 0] = float("nan")  # and one behind it
+        _, _, dec, out = _whole(ops, src, trg_bad, q)
+        for got, ref in ((dec, clean[2]), (out, clean[3])):
+            assert torch.isnan(got[first:, 0]).all()
+            assert torch.equal(got[:first], ref[:first]) and torch.equal(got[:, 1:], ref[:, 1:])
