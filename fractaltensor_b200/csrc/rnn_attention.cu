@@ -107,6 +107,7 @@ __device__ __forceinline__ int source_len(const int* src_lens, int n, int Ls) {
 // The attention vector of sequence blockIdx.x, columns 128 * blockIdx.y .., into the rows of all Lt steps; the scores
 // into `scores` [Ls, N].  The CTAs of a sequence compute its len scores each for itself.  Latency: a chain of reads
 // of the encoder's rows for the scores, two reductions over the CTA, and reads of the rows again (from L2) for the sum.
+// The scores of positions past a sequence's length, which its vector does not need, are a CTA's own, behind the columns.
 template <typename T>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_vector_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, const int* __restrict__ src_lens,
@@ -124,6 +125,16 @@ attn_vector_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, co
   grid_dependency_wait();
   const int len = source_len(src_lens, n, Ls);
 
+  if (blockIdx.y * kAttnCols >= H) {
+    for (int j0 = len + wid * kDots; j0 < Ls; j0 += kWarps * kDots) {
+      float s[kDots];
+      row_dots(mine + j0 * step_elems, step_elems, Ls - j0, enc_proj, H, lane, s);
+#pragma unroll
+      for (int r = 0; r < kDots; ++r)
+        if (lane == r && j0 + r < Ls) scores[static_cast<long long>(j0 + r) * N + n] = s[r];
+    }
+    return;
+  }
   float mx = -INFINITY;
   for (int j0 = wid * kDots; j0 < len; j0 += kWarps * kDots) {
     float s[kDots];
@@ -235,7 +246,7 @@ int attn_vectors_t(const void* enc, const void* enc_proj, const int* src_lens, f
   static std::atomic<unsigned long long> configured{0};
   if (!ensure_dynamic_smem(attn_vector_kernel<T>, 48 * 1024, configured)) return FTB_ERR_LAUNCH;
   const cudaError_t err =
-      launch_light(attn_vector_kernel<T>, dim3(N, (H + kAttnCols - 1) / kAttnCols), dim3(kAttnThreads),
+      launch_light(attn_vector_kernel<T>, dim3(N, (H + kAttnCols - 1) / kAttnCols + (src_lens != nullptr)), dim3(kAttnThreads),
                    static_cast<size_t>(Ls) * sizeof(float), stream, static_cast<const T*>(enc),
                    static_cast<const T*>(enc_proj), src_lens, scores, static_cast<T*>(out), Lt, Ls, N, H);
   count_launch();

@@ -282,7 +282,7 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * bf16: tensor cores, fp32 accumulation); Wp_src, Wp_trg from ftb_rnn_pack_weights with I = H;
  * bias_src, bias_trg: fp32 [H] or NULL; enc_proj, dec_proj: [H] of `dtype`; src_lens: int32 [N] on
  * the device, sequence n attends to source positions j < src_lens[n] (NULL: all Ls).
- * Outputs (caller-owned): enc [Ls, N, H] encoder states, enc_scores fp32 [Ls, N] (e_j.enc_proj, j < src_lens[n]),
+ * Outputs (caller-owned): enc [Ls, N, H] encoder states, enc_scores fp32 [Ls, N] (e_j.enc_proj),
  * dec [Lt, N, H] decoder states, out [Lt, N, H] the attention vectors.  Rows of a sequence past its
  * own source / target length hold values nobody should read.  H % 64 == 0, Ls <= 12288.
  * The decoder's term is the same for every score of a step and leaves the softmax as it is, so the

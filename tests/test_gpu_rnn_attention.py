@@ -240,3 +240,17 @@ def test_steps_shared_by_several_ctas(ops, dt, N, Lt):
         for got, ref in ((dec, clean[2]), (out, clean[3])):
             assert torch.isnan(got[first:, 0]).all()
             assert torch.equal(got[:first], ref[:first]) and torch.equal(got[:, 1:], ref[:, 1:])
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H,Ls,lens", [(64, 5, None), (64, 5, [5, 0, 3]), (192, 70, [1, 70, 33, 34, 69])])
+def test_scores_of_all_positions(ops, dt, H, Ls, lens):
+    """enc_scores holds e_j . enc_proj of every row of enc, past a sequence's length too."""
+    N = 2 if lens is None else len(lens)
+    p, g = _params(H, H + Ls, 1.0 / (H ** 0.5))
+    q = {k: v.to(dt).cuda() for k, v in p.items()}
+    src, trg = (torch.randn(n, N, H, generator=g).to(dt).cuda() for n in (Ls, 3))
+    enc, scores, _, _ = _whole(ops, src, trg, q, None if lens is None else torch.tensor(lens, dtype=torch.int32).cuda())
+    ref = (enc.double() @ q["enc_proj"].double())[..., 0]
+    # fp32 sums of H products of at most 1
+    assert (scores.double() - ref).abs().max().item() <= H * 2.0 ** -23
