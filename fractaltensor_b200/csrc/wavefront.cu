@@ -911,6 +911,14 @@ int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias
   if (workspace == nullptr || workspace_bytes < ftb_lstm_stacked_ragged_workspace_bytes(D, L, N)) return FTB_ERR_WORKSPACE;
   int rc = check_device_sm100();
   if (rc) return rc;
+  // The tables are copied from memory that ends with the call: in a graph every replay would read what is there then,
+  // and the rows would go by it.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return FTB_ERR_LAUNCH;
+  }
+  if (capture != cudaStreamCaptureStatusNone) return FTB_ERR_ARG;
   // Sequences by decreasing length (equal ones in their order): active[t] of them are longer than t, and those of
   // length n go to the places from active[n] on.
   std::vector<int> active(static_cast<size_t>(L) + 1, 0), table(static_cast<size_t>(L) + 1 + N);

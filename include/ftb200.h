@@ -149,7 +149,8 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
  * layer's states put back, all on `stream`.  `lens` is a HOST array of N ints >= 1.  With T = sum(lens) and
  * L = max(lens): x: [T,I], the sequences one behind the other; out: [T,H] in the same order, the top layer's hidden
  * states; xt [T,I], hs [D,T,H] and c fp32 [D,N,H] (caller-owned) receive the packed input and the packed results of
- * ftb_lstm_stacked_varlen_fwd.  Not for stream capture. */
+ * ftb_lstm_stacked_varlen_fwd.  Small tables are copied from host memory that ends with the call: on a stream that
+ * is being captured the call is refused (FTB_ERR_ARG). */
 size_t ftb_lstm_stacked_ragged_workspace_bytes(int D, int L, int N);
 int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt, void* hs,
                                 float* c, void* out, int D, int N, int I, int H, int dtype, void* workspace,

@@ -66,3 +66,22 @@ def test_rows_that_begin_anywhere(ops):
         ops.check_status()
     assert outs[0].indices == nest and outs[0].element_shape == (1, H)
     assert torch.equal(outs[0].data, outs[1].data)
+
+
+def test_capture_is_refused(ops):
+    """A graph would keep the address of tables that end with the call.  (Nothing is replayed.)"""
+    from fractaltensor_b200._lib import FtbError
+    g = torch.Generator(device="cuda").manual_seed(3)
+    u = lambda *s: (torch.rand(*s, device="cuda", generator=g) - 0.5).half()
+    Wp, b = ops.lstm_pack_weights(u(1, 4, 64, 64), u(1, 4, 64, 64), u(1, 4, 64))
+    x, lens = u(8, 64), [3, 5]
+    want = ops.lstm_stacked_ragged(x, lens, Wp, b)
+    torch.cuda.synchronize()
+    graph, extra = torch.cuda.CUDAGraph(), torch.zeros(1, device="cuda")
+    with torch.cuda.graph(graph):
+        with pytest.raises(FtbError):
+            ops.lstm_stacked_ragged(x, lens, Wp, b)
+        extra.add_(1)  # the capture goes on
+    del graph
+    assert torch.equal(ops.lstm_stacked_ragged(x, lens, Wp, b), want)
+    ops.check_status()
