@@ -885,17 +885,28 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
   return FTB_OK;
 }
 
-// Tables of a ragged batch behind the workspace of the packed entry point.
-static size_t ragged_table_bytes(int L, int N) { return sizeof(int) * (static_cast<size_t>(L) + 1 + N) + 16; }
+// Row tables of a ragged batch.
+size_t ftb_lstm_stacked_ragged_scratch_bytes(int L, int N) {
+  return L <= 0 || N <= 0 ? 0 : sizeof(int) * (static_cast<size_t>(L) + 1 + N);
+}
 
+// With no scratch they go behind the workspace of the packed entry point.
 size_t ftb_lstm_stacked_ragged_workspace_bytes(int D, int L, int N) {
   if (D <= 0 || L <= 0 || N <= 0) return kWorkspaceBytes;
-  return ftb_lstm_stacked_varlen_workspace_bytes(D, L) + ragged_table_bytes(L, N);
+  return ftb_lstm_stacked_varlen_workspace_bytes(D, L) + ftb_lstm_stacked_ragged_scratch_bytes(L, N) + 16;
 }
 
 int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt, void* hs,
                                 float* c, void* out, int D, int N, int I, int H, int dtype, void* workspace,
-                                size_t workspace_bytes, void* stream_) {
+                                size_t workspace_bytes, void* stream) {
+  return ftb_lstm_stacked_ragged_fwd_scratch(x, Wp, bias_p, lens, xt, hs, c, out, D, N, I, H, dtype, nullptr, 0, workspace,
+                                             workspace_bytes, stream);
+}
+
+int ftb_lstm_stacked_ragged_fwd_scratch(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt,
+                                        void* hs, float* c, void* out, int D, int N, int I, int H, int dtype,
+                                        void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes,
+                                        void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!x || !Wp || !lens || !xt || !hs || !c || !out || D <= 0 || N <= 0 || !valid_dtype(dtype)) return FTB_ERR_ARG;
   if (H <= 0 || I <= 0 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return FTB_ERR_ARG;
@@ -907,8 +918,12 @@ int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias
     T += lens[n];
   }
   if (static_cast<int64_t>(D) * T > 0x7fffffffLL) return FTB_ERR_ARG;
-  if (!aligned16({x, Wp, bias_p, xt, hs, c, out})) return FTB_ERR_ALIGN;
-  if (workspace == nullptr || workspace_bytes < ftb_lstm_stacked_ragged_workspace_bytes(D, L, N)) return FTB_ERR_WORKSPACE;
+  if (!aligned16({x, Wp, bias_p, xt, hs, c, out, scratch})) return FTB_ERR_ALIGN;
+  const size_t packed_bytes = ftb_lstm_stacked_varlen_workspace_bytes(D, L);
+  if (workspace == nullptr ||
+      workspace_bytes < (scratch != nullptr ? packed_bytes : ftb_lstm_stacked_ragged_workspace_bytes(D, L, N)))
+    return FTB_ERR_WORKSPACE;
+  if (scratch != nullptr && scratch_bytes < ftb_lstm_stacked_ragged_scratch_bytes(L, N)) return FTB_ERR_WORKSPACE;
   int rc = check_device_sm100();
   if (rc) return rc;
   // The tables are copied from memory that ends with the call: in a graph every replay would read what is there then,
@@ -936,8 +951,9 @@ int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias
       row += lens[n];
     }
   }
-  const size_t packed_bytes = ftb_lstm_stacked_varlen_workspace_bytes(D, L);
-  int* d_off = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + packed_bytes + 15) & ~static_cast<uintptr_t>(15));
+  int* d_off = scratch != nullptr ? static_cast<int*>(scratch)
+                                  : reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + packed_bytes + 15) &
+                                                           ~static_cast<uintptr_t>(15));
   const int* d_start = d_off + L + 1;
   if (cudaMemcpyAsync(d_off, table.data(), sizeof(int) * table.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess)
     return FTB_ERR_LAUNCH;

@@ -211,15 +211,19 @@ def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
         raise ValueError("Wp %s / lens (sum %d) do not match x %s" % (tuple(Wp.shape), T, tuple(x.shape)))
     if bias_p is not None:
         _req_like(bias_p, "bias_p", torch.float32, (D, 4 * H), x)
-    xt = torch.empty_like(x)
+    # the packed input, and behind it the rows' tables, the call's own: they are read again behind the LSTM
+    rows, tables = x.numel() * x.element_size(), lib.ftb_lstm_stacked_ragged_scratch_bytes(L, N)
+    xt = torch.empty(rows + tables, dtype=torch.uint8, device=x.device)
     hs = torch.empty(D, T, H, dtype=x.dtype, device=x.device)
     c = torch.empty(D, N, H, dtype=torch.float32, device=x.device)
     out = torch.empty(T, H, dtype=x.dtype, device=x.device)
-    ws = workspace(x.device, lib.ftb_lstm_stacked_ragged_workspace_bytes(D, L, N))
+    ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L))
     with torch.cuda.device(x.device):
-        check(lib.ftb_lstm_stacked_ragged_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N)(*lens), _ptr(xt), _ptr(hs),
-                                              _ptr(c), _ptr(out), D, N, I, H, _dtype_code(x), _ptr(ws), ws.numel(),
-                                              _stream()), "ftb_lstm_stacked_ragged_fwd")
+        check(lib.ftb_lstm_stacked_ragged_fwd_scratch(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N)(*lens), _ptr(xt),
+                                                      _ptr(hs), _ptr(c), _ptr(out), D, N, I, H, _dtype_code(x),
+                                                      ctypes.c_void_p(xt.data_ptr() + rows), tables, _ptr(ws),
+                                                      ws.numel(), _stream()),
+              "ftb_lstm_stacked_ragged_fwd_scratch")
     return out
 
 

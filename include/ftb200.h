@@ -150,11 +150,20 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
  * L = max(lens): x: [T,I], the sequences one behind the other; out: [T,H] in the same order, the top layer's hidden
  * states; xt [T,I], hs [D,T,H] and c fp32 [D,N,H] (caller-owned) receive the packed input and the packed results of
  * ftb_lstm_stacked_varlen_fwd.  Small tables are copied from host memory that ends with the call: on a stream that
- * is being captured the call is refused (FTB_ERR_ARG). */
+ * is being captured the call is refused (FTB_ERR_ARG).
+ * The tables of the rows are read before and behind the LSTM.  They lie in the workspace behind those of the packed
+ * entry point; ftb_lstm_stacked_ragged_fwd_scratch takes them in a buffer of their own instead
+ * (ftb_lstm_stacked_ragged_scratch_bytes; the workspace is that of the packed entry point then), so that another host
+ * thread's call with the same stream and workspace in between does not move the rows to that call's places. */
 size_t ftb_lstm_stacked_ragged_workspace_bytes(int D, int L, int N);
+size_t ftb_lstm_stacked_ragged_scratch_bytes(int L, int N);
 int ftb_lstm_stacked_ragged_fwd(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt, void* hs,
                                 float* c, void* out, int D, int N, int I, int H, int dtype, void* workspace,
                                 size_t workspace_bytes, void* stream);
+int ftb_lstm_stacked_ragged_fwd_scratch(const void* x, const void* Wp, const float* bias_p, const int* lens, void* xt,
+                                        void* hs, float* c, void* out, int D, int N, int I, int H, int dtype,
+                                        void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes,
+                                        void* stream);
 
 /* Dilated stacked LSTM forward: layer l reads its own state dilations[l] steps
  * back.  Stands in for dilated_layer()/model() (examples/dilated_rnn/dilated_rnn.py:16-41)

@@ -85,3 +85,37 @@ def test_capture_is_refused(ops):
     del graph
     assert torch.equal(ops.lstm_stacked_ragged(x, lens, Wp, b), want)
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16])
+def test_row_tables_are_the_call_s_own(ops, dt):
+    """Another host thread's call on the stream would put its tables where the stream's workspace has them: nothing of
+    the rows is there.  The C entry without scratch, which has them there, gives the same bits."""
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, ctypes, lib
+    D, H, lens = 2, 64, [3, 9, 4, 9, 1]
+    N, L, T = len(lens), max(lens), sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    u = lambda *s: (torch.rand(*s, device="cuda", generator=g) - 0.5).to(dt)
+    Wp, b = ops.lstm_pack_weights(u(D, 4, H, H), u(D, 4, H, H), u(D, 4, H))
+    x = u(T, H)
+    packed = lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L)
+    room = lib.ftb_lstm_stacked_ragged_workspace_bytes(D, L, N)
+    assert room >= packed + lib.ftb_lstm_stacked_ragged_scratch_bytes(L, N)
+    ws = ops.workspace("cuda", room)
+    rest = ws[packed:]
+    rest.fill_(0xA5)
+    got = ops.lstm_stacked_ragged(x, lens, Wp, b)
+    ops.check_status()
+    same = bool((rest == 0xA5).all())
+    rest.zero_()
+    assert same
+    xt, out = torch.empty_like(x), torch.empty(T, H, dtype=dt, device="cuda")
+    hs, c = torch.empty(D, T, H, dtype=dt, device="cuda"), torch.empty(D, N, H, device="cuda")
+    args = (_ptr(x), _ptr(Wp), _ptr(b), (ctypes.c_int * N)(*lens), _ptr(xt), _ptr(hs), _ptr(c), _ptr(out), D, N, H, H,
+            _dtype_code(x))
+    check(lib.ftb_lstm_stacked_ragged_fwd(*args, _ptr(ws), room, _stream()), "ftb_lstm_stacked_ragged_fwd")
+    ops.check_status()
+    assert torch.equal(out, got)
+    short = ctypes.c_size_t(lib.ftb_lstm_stacked_ragged_scratch_bytes(L, N) - 1)
+    assert lib.ftb_lstm_stacked_ragged_fwd(*args, _ptr(ws), room - 1, _stream()) != 0
+    assert lib.ftb_lstm_stacked_ragged_fwd_scratch(*args, _ptr(c), short, _ptr(ws), packed, _stream()) != 0
