@@ -8,6 +8,7 @@ functions in :mod:`fractaltensor_b200.frontend` convert from and to the nested
 FractalTensor views of the reference's Python programs.
 """
 import ctypes
+import threading
 
 import torch
 
@@ -19,6 +20,7 @@ _DT = {torch.float32: _lib.DTYPE_F32, torch.float16: _lib.DTYPE_F16, torch.bfloa
 _workspaces = {}  # (device index, stream handle): uint8 tensor
 _MAX_WORKSPACES = 64
 _STATUS_BYTES = lib.ftb_workspace_bytes()
+_turns = [threading.Lock() for _ in range(64)]
 
 
 def _dtype_code(t):
@@ -86,6 +88,13 @@ def workspace(device, nbytes=0):
     return ws
 
 
+def _turn(ws):
+    """Held while a call that has tables or counters in `ws` is enqueued: its copies and launches follow one another
+    in the stream, with nothing of another host thread's call on that stream (the default one, say) in between.
+    (Workspaces may share a lock.)"""
+    return _turns[(ws.data_ptr() >> 9) % len(_turns)]
+
+
 def _tuning(layers_per_group=0, bn=0, schedule=0, skew=0, pair=0, fine_deps=0, resident=0):
     return (ctypes.c_int * 7)(int(layers_per_group), int(bn), int(schedule), int(skew), int(pair), int(fine_deps),
                               int(resident))
@@ -149,7 +158,7 @@ def lstm_stacked(x, Wp, bias_p=None, hs=None, c=None, layers_per_group=0, bn=0, 
     _req_like(hs, "hs", x.dtype, (D, L, N, H), x)
     _req_like(c, "c", torch.float32, (D, N, H), x)
     ws = workspace(x.device, lib.ftb_lstm_stacked_workspace_bytes(D, L, N, H))
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _turn(ws):
         check(lib.ftb_lstm_stacked_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), D, L, N, I, H,
                                        _dtype_code(x),
                                        _tuning(layers_per_group, bn, schedule, skew, pair, fine_deps, resident),
@@ -189,7 +198,7 @@ def lstm_stacked_varlen(x, active_rows, Wp, bias_p=None, hs=None, c=None, layers
     _req_like(c, "c", torch.float32, (D, N, H), x)
     rows = (ctypes.c_int * L)(*active_rows)
     ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L))
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _turn(ws):
         check(lib.ftb_lstm_stacked_varlen_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), rows, D, L, I, H,
                                               _dtype_code(x), _tuning(layers_per_group, bn, schedule, 0, pair, 0),
                                               _ptr(ws), ws.numel(), _stream()), "ftb_lstm_stacked_varlen_fwd")
@@ -218,7 +227,7 @@ def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
     c = torch.empty(D, N, H, dtype=torch.float32, device=x.device)
     out = torch.empty(T, H, dtype=x.dtype, device=x.device)
     ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L))
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _turn(ws):
         check(lib.ftb_lstm_stacked_ragged_fwd_scratch(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N)(*lens), _ptr(xt),
                                                       _ptr(hs), _ptr(c), _ptr(out), D, N, I, H, _dtype_code(x),
                                                       ctypes.c_void_p(xt.data_ptr() + rows), tables, _ptr(ws),
@@ -249,7 +258,7 @@ def lstm_dilated(x, Wp, dilations, bias_p=None, hs=None, c=None, bn=0, pair=0, s
     _req_like(c, "c", torch.float32, (D, md * N, H), x)
     dil = (ctypes.c_int * D)(*[int(d) for d in dilations])
     ws = workspace(x.device, lib.ftb_lstm_dilated_workspace_bytes(D, L))
-    with torch.cuda.device(x.device):
+    with torch.cuda.device(x.device), _turn(ws):
         check(lib.ftb_lstm_dilated_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), dil, D, L, N, H,
                                        _dtype_code(x), _tuning(bn=bn, pair=pair, schedule=schedule), _ptr(ws), ws.numel(),
                                        _stream()), "ftb_lstm_dilated_fwd")
@@ -293,7 +302,7 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
     # per level; the tables -> generic persistent kernel; tables and flags -> cluster kernel.
     ws = workspace(X.device, 0 if schedule == 1 else lib.ftb_grid_rnn_workspace_bytes(D, A, B))
     ws_bytes = {1: lib.ftb_workspace_bytes(), 2: lib.ftb_grid_rnn_tables_bytes(D, A, B)}.get(schedule, ws.numel())
-    with torch.cuda.device(X.device):
+    with torch.cuda.device(X.device), _turn(ws):
         check(lib.ftb_grid_rnn_fwd(_ptr(X), _ptr(Y), _ptr(Wpx), _ptr(Wpy), _ptr(bias_x), _ptr(bias_y), _ptr(hx),
                                    _ptr(hy), D, A, B, N, H, _dtype_code(X), _ptr(ws), ws_bytes, _stream()),
               "ftb_grid_rnn_fwd")

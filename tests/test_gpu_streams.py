@@ -130,3 +130,45 @@ def test_a_capture_takes_a_workspace_that_is_there():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, ref) and ops._workspaces == before
+
+
+@pytest.mark.parametrize("program", ["varlen", "ragged", "stacked"])
+def test_host_threads_on_one_stream(program):
+    """Host threads share the default stream and so its workspace: the tables of one thread's call are not those of
+    another's kernels."""
+    import threading
+
+    from fractaltensor_b200 import ops
+
+    def call(seed, N):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        H, D, L = 64, 2, 20
+        u = lambda *s: ((torch.rand(*s, device="cuda", generator=g) * 2 - 1) / H ** 0.5).half()
+        Wp, b = ops.lstm_pack_weights(u(D, 4, H, H), u(D, 4, H, H), u(D, 4, H))
+        if program == "stacked":
+            x = u(L, N, H)
+            return lambda: ops.lstm_stacked(x, Wp, b, schedule=2)[0]
+        lens = [1 + (7 * n + seed) % L for n in range(N)]
+        x = u(sum(lens), H)
+        if program == "ragged":
+            return lambda: ops.lstm_stacked_ragged(x, lens, Wp, b)
+        active = [sum(n > t for n in lens) for t in range(max(lens))]
+        return lambda: ops.lstm_stacked_varlen(x, active, Wp, b)[0]
+
+    calls = [call(s, 5 + 9 * s) for s in range(4)]
+    alone = [c() for c in calls]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        for _ in range(40):
+            if not torch.equal(calls[i](), alone[i]):
+                wrong.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    ops.check_status()
+    assert not wrong
