@@ -50,7 +50,11 @@ __device__ __forceinline__ void push(MD& s, float v) {
   s.m = m;
 }
 
-template <int THREADS>
+// VEC_IN, VEC_OUT: rows of x (of y, too) start on 16-byte boundaries and are moved by 16 bytes, what is left behind the
+// last whole one singly.  A kernel for each, not a branch: with both forms of the loops in one kernel the registers cost a
+// resident CTA in five (20000 x 129 38 us, 31 so), and one loop for the tail and for whole rows is not unrolled
+// (8000 x 9999 205 us, 178 so).
+template <int THREADS, bool VEC_IN, bool VEC_OUT>
 __global__ void __launch_bounds__(THREADS)
 online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int width, int ld, int ld_out,
                       int cache_floats) {
@@ -62,10 +66,7 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
   const int cached_floats = width < cache_floats ? width : cache_floats;  // prefix of the row kept on chip
   grid_launch_dependents();
   grid_dependency_wait();  // the kernel before this one (the projection GEMM, say) wrote x
-  // 16-byte accesses need rows that start on a 16-byte boundary; what is left behind the last whole one goes singly.
-  const bool vec_in = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const bool vec = vec_in && (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-  const int tail = width & ~3;
+  const int tail = (width & ~3) + tid;
 
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const float* xr = x + static_cast<size_t>(r) * ld;
@@ -73,7 +74,7 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
     MD s;
     s.m = -FLT_MAX;
     s.d = 0.f;
-    if (vec_in) {
+    if constexpr (VEC_IN) {
       const float4* x4 = reinterpret_cast<const float4*>(xr);
 #pragma unroll 4
       for (int i = tid; i < width / 4; i += THREADS) {
@@ -86,11 +87,17 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
         push(s, v.z);
         push(s, v.w);
       }
-    }
-    for (int i = (vec_in ? tail : 0) + tid; i < width; i += THREADS) {
-      const float v = xr[i];
-      if (i < cached_floats) row_cache[i] = v;
-      push(s, v);
+      if (tail < width) {
+        const float v = xr[tail];
+        if (tail < cached_floats) row_cache[tail] = v;
+        push(s, v);
+      }
+    } else {
+      for (int i = tid; i < width; i += THREADS) {
+        const float v = xr[i];
+        if (i < cached_floats) row_cache[i] = v;
+        push(s, v);
+      }
     }
     // Threads that saw no element hold (-FLT_MAX, 0): neutral in a merge.
 #pragma unroll
@@ -124,7 +131,7 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
     __syncthreads();
     const float m = final_m;
     const float inv_d = 1.f / final_d;
-    if (vec) {
+    if constexpr (VEC_OUT) {
       const float4* x4 = reinterpret_cast<const float4*>(xr);
       float4* y4 = reinterpret_cast<float4*>(yr);
 #pragma unroll 4
@@ -136,10 +143,15 @@ online_softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int ro
         v.w = exp_fast(fmaxf(v.w - m, kClamp)) * inv_d;
         __stcs(y4 + i, v);
       }
-    }
-    for (int i = (vec ? tail : 0) + tid; i < width; i += THREADS) {
-      const float v = i < cached_floats ? row_cache[i] : xr[i];
-      __stcs(yr + i, exp_fast(fmaxf(v - m, kClamp)) * inv_d);
+      if (tail < width) {
+        const float v = tail < cached_floats ? row_cache[tail] : xr[tail];
+        yr[tail] = exp_fast(fmaxf(v - m, kClamp)) * inv_d;
+      }
+    } else {
+      for (int i = tid; i < width; i += THREADS) {
+        const float v = i < cached_floats ? row_cache[i] : xr[i];
+        yr[i] = exp_fast(fmaxf(v - m, kClamp)) * inv_d;
+      }
     }
     __syncthreads();  // the cache and the reduction slots are reused by the next row
   }
@@ -221,25 +233,25 @@ int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, i
   if (x == y && width > kMaxCacheFloats) return FTB_ERR_ARG;
   const int cache_floats = width <= kMaxCacheFloats ? ((width + 3) & ~3) : kMaxCacheFloats;
   const size_t smem = static_cast<size_t>(cache_floats) * sizeof(float);
-  static std::atomic<unsigned long long> configured_a{0}, configured_b{0};
-  if (!ensure_dynamic_smem(online_softmax_kernel<kSoftmaxThreads>, kMaxCacheFloats * static_cast<int>(sizeof(float)),
-                           configured_a) ||
-      !ensure_dynamic_smem(online_softmax_kernel<1024>, kMaxCacheFloats * static_cast<int>(sizeof(float)),
-                           configured_b))
-    return FTB_ERR_LAUNCH;
   // A whole number of CTAs per SM: as many as the row cache lets be resident (at most 8).  A cache
   // that leaves room for one or two CTAs per SM gets CTAs of 1024 threads to keep loads in flight.
   int per_sm = static_cast<int>((200 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
   const int64_t want = static_cast<int64_t>(current_sm_count()) * per_sm;
   const int grid = static_cast<int>(rows < want ? rows : want);
-  cudaError_t err;
-  if (per_sm <= 2)
-    err = launch_light(online_softmax_kernel<1024>, dim3(grid), dim3(1024), smem, stream, x, y, rows, width, ld,
-                       ld_out, cache_floats);
-  else
-    err = launch_light(online_softmax_kernel<kSoftmaxThreads>, dim3(grid), dim3(kSoftmaxThreads), smem, stream, x, y, rows,
-                       width, ld, ld_out, cache_floats);
+  const bool vec_in = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool vec_out = vec_in && (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  using Kernel = decltype(&online_softmax_kernel<1024, true, true>);
+  const Kernel kernels[2][3] = {
+      {online_softmax_kernel<kSoftmaxThreads, false, false>, online_softmax_kernel<kSoftmaxThreads, true, false>,
+       online_softmax_kernel<kSoftmaxThreads, true, true>},
+      {online_softmax_kernel<1024, false, false>, online_softmax_kernel<1024, true, false>, online_softmax_kernel<1024, true, true>}};
+  static std::atomic<unsigned long long> configured[2][3];
+  const int wide = per_sm <= 2, form = vec_in + vec_out;
+  if (!ensure_dynamic_smem(kernels[wide][form], kMaxCacheFloats * static_cast<int>(sizeof(float)), configured[wide][form]))
+    return FTB_ERR_LAUNCH;
+  const cudaError_t err = launch_light(kernels[wide][form], dim3(grid), dim3(wide ? 1024 : kSoftmaxThreads), smem, stream, x, y,
+                                       rows, width, ld, ld_out, cache_floats);
   count_launch();
   if (err != cudaSuccess) cudaGetLastError();
   return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
