@@ -230,9 +230,10 @@ int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, i
   }
   // Row cache: the row, or its first 48 K floats, in up to 192 KB of shared memory.
   constexpr int kMaxCacheFloats = 48 * 1024;
+  constexpr size_t kMaxSmem = 228 * 1024;  // of an SM
   if (x == y && width > kMaxCacheFloats) return FTB_ERR_ARG;
   const int cache_floats = width <= kMaxCacheFloats ? ((width + 3) & ~3) : kMaxCacheFloats;
-  const size_t smem = static_cast<size_t>(cache_floats) * sizeof(float);
+  size_t smem = static_cast<size_t>(cache_floats) * sizeof(float);
   // A whole number of CTAs per SM: as many as the row cache lets be resident (at most 8).  A cache
   // that leaves room for one or two CTAs per SM gets CTAs of 1024 threads to keep loads in flight.
   int per_sm = static_cast<int>((200 * 1024) / (smem + 1024));
@@ -248,6 +249,9 @@ int online_softmax_rows(const float* x, float* y, int rows, int width, int ld, i
       {online_softmax_kernel<1024, false, false>, online_softmax_kernel<1024, true, false>, online_softmax_kernel<1024, true, true>}};
   static std::atomic<unsigned long long> configured[2][3];
   const int wide = per_sm <= 2, form = vec_in + vec_out;
+  // A row alone on its SM where there are SMs enough: launched while the projection still holds most of them, two CTAs
+  // that fit together would go to the same one (projection and softmax 16 x 20000 x 1024 25.0 us, 22.9 so).
+  if (wide && rows <= current_sm_count() && smem < kMaxSmem / 2) smem = kMaxSmem / 2;
   if (!ensure_dynamic_smem(kernels[wide][form], kMaxCacheFloats * static_cast<int>(sizeof(float)), configured[wide][form]))
     return FTB_ERR_LAUNCH;
   const cudaError_t err = launch_light(kernels[wide][form], dim3(grid), dim3(wide ? 1024 : kSoftmaxThreads), smem, stream, x, y,
