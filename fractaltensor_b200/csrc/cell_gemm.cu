@@ -58,7 +58,7 @@ struct Cfg {
   static constexpr uint32_t kCBoxBytes = BM * 128;
   static constexpr int kCBoxes = kUnits / 32;
   static constexpr uint32_t kCBytes = kStaged ? kCBoxes * kCBoxBytes : 0;
-  static constexpr uint32_t kRowBytes = EPI == EPI_STORE_F32 ? kEpiWarps * 4096 : 0;  // 32 x 32 numbers a warp
+  static constexpr uint32_t kRowBytes = EPI == EPI_STORE_F32 ? kEpiWarps * 2048 : 0;  // 16 x 32 numbers a warp
   static constexpr uint32_t kStagingBytes = kCBytes + kRowBytes;
   static constexpr uint32_t kRingBudget = 229376 - 2048 - kStagingBytes;
   static constexpr int kStages = (kRingBudget / kStageBytes) > 8 ? 8 : (kRingBudget / kStageBytes);
@@ -496,26 +496,34 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
           tmem_ld32(taddr + ch * 32, r);
           tmem_ld_wait();
           const int col0 = col_base + ch * 32;
-          if (EPI == EPI_STORE_F32) {
+          const int row0 = row - lane;
+          if (EPI == EPI_STORE_F32 && row0 + 32 <= rows) {
             // A lane has a row of the chunk, 128 bytes: through shared memory (16-byte pieces exchanged within a row, so
             // that neither side meets a bank twice), so that a store covers four whole rows and not a piece of 32.
-            // (2240 x 10112 x 512, 90 MB of results: 53 us with a row a lane, 33 so.)
-            uint8_t* s_row = smem + S * C::kStageBytes + (warp - 2) * 4096;
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-              *reinterpret_cast<uint4*>(s_row + lane * 128 + ((g ^ (lane & 7)) << 4)) =
-                  make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
-            __syncwarp();
-            const int row0 = row - lane, piece = lane & 7;
+            // (2240 x 10112 x 512, 90 MB of results: 53 us with a row a lane, 33 so.)  In two halves of 16 rows: with
+            // room for all 32 of every warp the ring loses a stage (7 x 40064 x 1024 25.2 us, 23.6 so; 500 rows 88 and 86 with
+            // their softmax; 2240 x 10112 x 512 0.5 us behind).  A warp that has not all of its rows stores a row a lane.
+            uint8_t* s_row = smem + S * C::kStageBytes + (warp - 2) * 2048;
+            const int piece = lane & 7;
             float* to = reinterpret_cast<float*>(it->out) + col0 + 4 * piece;
 #pragma unroll
-            for (int k = 0; k < 32; k += 4) {
-              const int rr = k + (lane >> 3);
-              const float4 v = *reinterpret_cast<const float4*>(s_row + rr * 128 + ((piece ^ (rr & 7)) << 4));
-              if (col0 + 32 <= batch.n_cols && row0 + rr < rows)
-                *reinterpret_cast<float4*>(to + static_cast<size_t>(row0 + rr) * batch.ld_out) = v;
+            for (int part = 0; part < 32; part += 16) {
+              if ((lane & 16) == part) {
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                  *reinterpret_cast<uint4*>(s_row + (lane & 15) * 128 + ((g ^ (lane & 7)) << 4)) =
+                      make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+              }
+              __syncwarp();
+#pragma unroll
+              for (int k = 0; k < 16; k += 4) {
+                const int rr = k + (lane >> 3);
+                const float4 v = *reinterpret_cast<const float4*>(s_row + rr * 128 + ((piece ^ (rr & 7)) << 4));
+                if (col0 + 32 <= batch.n_cols)
+                  *reinterpret_cast<float4*>(to + static_cast<size_t>(row0 + part + rr) * batch.ld_out) = v;
+              }
+              __syncwarp();
             }
-            __syncwarp();
             continue;
           }
           if (col0 + 32 > batch.n_cols || !row_ok) continue;
@@ -531,7 +539,14 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
               }
               v[j] = x;
             }
-            *reinterpret_cast<uint4*>(out_row + col0 + 8 * g) = pack8<T>(v);
+            if (EPI == EPI_STORE_F32) {
+              float4* of = reinterpret_cast<float4*>(reinterpret_cast<float*>(it->out) +
+                                                     static_cast<size_t>(row) * batch.ld_out + col0 + 8 * g);
+              of[0] = make_float4(v[0], v[1], v[2], v[3]);
+              of[1] = make_float4(v[4], v[5], v[6], v[7]);
+            } else {
+              *reinterpret_cast<uint4*>(out_row + col0 + 8 * g) = pack8<T>(v);
+            }
           }
         }
         tc_fence_before();
