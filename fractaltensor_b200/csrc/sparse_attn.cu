@@ -192,7 +192,7 @@ struct SparseArgs {
   int per_head, lead, skip;
   // A launch that walks interior and edge tiles with different routines: the edge enumeration
   // (the one above is then the interior one).
-  int edge_per_head, edge_lead, edge_skip;
+  int edge_TT, edge_per_head, edge_lead, edge_skip;
 };
 
 // Where the rows of one token's head come from: global memory, and for the tiled kernel the stage
@@ -371,13 +371,13 @@ struct Tile {
   long long head;
   int t0, nt, lo, hi;
 };
-__device__ __forceinline__ Tile tile_of(const SparseArgs& a, int per_head, int lead, int skip, long long t) {
+__device__ __forceinline__ Tile tile_of(const SparseArgs& a, int TT, int per_head, int lead, int skip, long long t) {
   const int half = (a.window - 1) * a.dilation / 2;
   Tile x;
   x.head = t / per_head;
   const int idx = static_cast<int>(t - x.head * per_head);
-  x.t0 = (idx < lead ? idx : idx + skip) * a.TT;
-  x.nt = min(a.TT, a.S - x.t0);
+  x.t0 = (idx < lead ? idx : idx + skip) * TT;
+  x.nt = min(TT, a.S - x.t0);
   x.lo = max(0, x.t0 - half);
   x.hi = min(a.S, x.t0 + x.nt + half);
   return x;
@@ -412,7 +412,7 @@ __device__ __forceinline__ void copy_tile(const T* q, const T* k, const T* v, co
 template <typename T, int LPT>
 __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                           const int* __restrict__ rand_pos, T* __restrict__ o, const SparseArgs& a,
-                                          int per_head, int lead, int skip, long long first, long long step,
+                                          int TT, int per_head, int lead, int skip, long long first, long long step,
                                           unsigned char* smem, uint64_t* full, int* s_abort_p,
                                           int* __restrict__ status) {
   constexpr int d = kEPL * LPT;
@@ -421,7 +421,7 @@ __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __r
 
   const int tid = threadIdx.x, lane = tid & 31, gl = lane % LPT;
   const unsigned gmask = group_mask<LPT>(lane);
-  const int S = a.S, ng = a.n_global, G = 2 * a.n_global, TT = a.TT;
+  const int S = a.S, ng = a.n_global, G = 2 * a.n_global;
   const int half = (a.window - 1) * a.dilation / 2;
   const long long n_tiles = a.heads_total * per_head;  // work items of this enumeration
   // Every thread: its share of the tile's random positions (entry e = token * R + r of the tile).
@@ -449,7 +449,7 @@ __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __r
   long long tile = first;
   if (tile >= n_tiles) return;
   {
-    const Tile x = tile_of(a, per_head, lead, skip, tile);
+    const Tile x = tile_of(a, TT, per_head, lead, skip, tile);
     if (tid == 0) copy_tile(q, k, v, a, d, x, Stage<T>(smem, a, d, 0), &full[0]);
     int pre[kPosRegs];
     fetch_pos(x, pre);
@@ -459,14 +459,14 @@ __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __r
 
   for (int it = 0; tile < n_tiles; tile += step, ++it) {
     const int s = it & 1;
-    const Tile x = tile_of(a, per_head, lead, skip, tile);
+    const Tile x = tile_of(a, TT, per_head, lead, skip, tile);
     const Stage<T> st(smem, a, d, s);
     const long long next = tile + step;
     int pre[kPosRegs];
     if (next < n_tiles) {
       // stage s ^ 1 was last read in the previous round; the barrier that closed it orders those
       // reads before these writes
-      const Tile y = tile_of(a, per_head, lead, skip, next);
+      const Tile y = tile_of(a, TT, per_head, lead, skip, next);
       if (tid == 0) copy_tile(q, k, v, a, d, y, Stage<T>(smem, a, d, s ^ 1), &full[s ^ 1]);
       fetch_pos(y, pre);
     }
@@ -532,7 +532,7 @@ __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* 
     if (p.tok - mine < p.x.nt) return;
     p.tok = mine;
     p.tile += gridDim.x;
-    if (p.tile < n_tiles) p.x = tile_of(a, a.per_head, a.lead, a.skip, p.tile);
+    if (p.tile < n_tiles) p.x = tile_of(a, a.TT, a.per_head, a.lead, a.skip, p.tile);
   };
   auto request_positions = [&](const Pass& p, int (&x)[KR]) {
     if (p.tile >= n_tiles) return;
@@ -559,12 +559,12 @@ __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* 
   Pass now;
   now.tile = blockIdx.x;
   if (now.tile >= n_tiles) return;
-  now.x = tile_of(a, a.per_head, a.lead, a.skip, now.tile);
+  now.x = tile_of(a, a.TT, a.per_head, a.lead, a.skip, now.tile);
   now.tok = mine;
   if (threadIdx.x == 0) {
     copy_tile(q, k, v, a, d, now.x, Stage<T>(smem, a, d, 0), &full[0]);
     if (now.tile + gridDim.x < n_tiles)
-      copy_tile(q, k, v, a, d, tile_of(a, a.per_head, a.lead, a.skip, now.tile + gridDim.x), Stage<T>(smem, a, d, 1), &full[1]);
+      copy_tile(q, k, v, a, d, tile_of(a, a.TT, a.per_head, a.lead, a.skip, now.tile + gridDim.x), Stage<T>(smem, a, d, 1), &full[1]);
   }
   Pass next = now;
   int pos[KR];  // of the pass `next`
@@ -649,11 +649,11 @@ __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* 
       const bool last = atomicAdd(&n_read[s], 1) % (kSparseThreads / 32) == kSparseThreads / 32 - 1;
       __threadfence_block();
       const long long after = now.tile + 2 * static_cast<long long>(gridDim.x);
-      if (last && after < n_tiles) copy_tile(q, k, v, a, d, tile_of(a, a.per_head, a.lead, a.skip, after), st, &full[s]);
+      if (last && after < n_tiles) copy_tile(q, k, v, a, d, tile_of(a, a.TT, a.per_head, a.lead, a.skip, after), st, &full[s]);
     }
     __syncwarp();
     now.tile += gridDim.x;
-    if (now.tile < n_tiles) now.x = tile_of(a, a.per_head, a.lead, a.skip, now.tile);
+    if (now.tile < n_tiles) now.x = tile_of(a, a.TT, a.per_head, a.lead, a.skip, now.tile);
   }
 }
 
@@ -685,14 +685,14 @@ sparse_attn_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const 
   if constexpr (KW != 0) {
     // Edge tiles are handed out from the last CTA down, interior tiles from the first up: when the
     // edge tiles are fewer than the CTAs, the CTAs with one interior tile more do not get them.
-    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.edge_per_head, a.edge_lead, a.edge_skip, gridDim.x - 1 - blockIdx.x,
-                       gridDim.x, smem, full, &s_abort, status);
+    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.edge_TT, a.edge_per_head, a.edge_lead, a.edge_skip,
+                       gridDim.x - 1 - blockIdx.x, gridDim.x, smem, full, &s_abort, status);
     // (behind its last barrier: every warp has left the stages, and sees s_abort alike)
     if (s_abort == 0)
       walk_interior<T, LPT, KW, KR>(q, k, v, rand_pos, o, a, smem, interior_full, n_read, &s_abort, status);
   } else {
-    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.per_head, a.lead, a.skip, blockIdx.x, gridDim.x, smem, full, &s_abort,
-                       status);
+    walk_tiles<T, LPT>(q, k, v, rand_pos, o, a, a.TT, a.per_head, a.lead, a.skip, blockIdx.x, gridDim.x, smem, full,
+                       &s_abort, status);
   }
 }
 
@@ -754,17 +754,24 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
         if (err != cudaSuccess) cudaGetLastError();
         return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
       };
-      a.edge_per_head = a.edge_lead = a.edge_skip = 0;
+      a.edge_TT = a.edge_per_head = a.edge_lead = a.edge_skip = 0;
       if (fast != 0 && interior > 0) {
-        // Interior tiles by the routine built for their key counts, the edge tiles of every head by the general one on a share of the CTAs in proportion to their number.
+        // Interior tiles by the routine built for their key counts, the edge tiles of every head by the general one.
         a.per_head = interior;
         a.lead = 0;
         a.skip = lead;
-        a.edge_per_head = lead + trail;
-        a.edge_lead = lead;
-        a.edge_skip = interior;
-        const long long ctas = a.heads_total * a.tiles_per_head;
-        return run(kernels[fast], a, ctas);
+        // An edge tile takes the general routine longer than an interior tile the other, and a call of few tiles ends with
+        // its edges: they are cut into the smallest tiles of which the CTAs with an interior tile less can take one each
+        // (fp32, d 64, window 5, 3 random keys, 4 x 512 6.8 us with tiles of 64, 5.0 so; 8 x 2048 8.6, 6.5; fp16, d 128,
+        // 8 x 1024 14.9, 8.4).
+        const auto edges = [&](int tt) { return (a.S + tt - 1) / tt - interior * (TT / tt); };
+        const long long all = a.heads_total * interior, idle = full - all % full;
+        a.edge_TT = 16;
+        while (a.edge_TT < TT && a.heads_total * edges(a.edge_TT) > idle) a.edge_TT *= 2;
+        a.edge_per_head = edges(a.edge_TT);
+        a.edge_lead = lead * (TT / a.edge_TT);
+        a.edge_skip = interior * (TT / a.edge_TT);
+        return run(kernels[fast], a, all + a.heads_total * a.edge_per_head);
       }
       a.per_head = a.tiles_per_head;
       a.lead = a.skip = 0;
@@ -772,7 +779,7 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
     }
   }
   a.TT = a.tiles_per_head = a.stage_bytes = a.per_head = a.lead = a.skip = 0;
-  a.edge_per_head = a.edge_lead = a.edge_skip = 0;
+  a.edge_TT = a.edge_per_head = a.edge_lead = a.edge_skip = 0;
   const long long warps_needed = (a.heads_total * a.S + 32 / LPT - 1) / (32 / LPT);
   const long long ctas_needed = (warps_needed * 32 + kSparseThreads - 1) / kSparseThreads;
   const long long full = static_cast<long long>(current_sm_count()) * 8;
@@ -833,7 +840,7 @@ extern "C" int ftb_sparse_attn_fwd(const void* q, const void* k, const void* v, 
   a.as_shipped = as_shipped ? 1 : 0;
   a.scale = scale;
   a.TT = a.tiles_per_head = a.stage_bytes = a.per_head = a.lead = a.skip = 0;
-  a.edge_per_head = a.edge_lead = a.edge_skip = 0;
+  a.edge_TT = a.edge_per_head = a.edge_lead = a.edge_skip = 0;
   int* status = static_cast<int*>(workspace);  // sticky, as for the other single-kernel entry points
   switch (dtype) {
     case FTB_F32: return launch_sparse_d<float>(d, q, k, v, rand_pos, o, a, status, stream);

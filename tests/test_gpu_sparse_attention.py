@@ -221,3 +221,23 @@ def test_interior_walk_reports_positions_outside(ops):
 def test_every_pair_of_key_counts(ops, dt, window, R):
     """Each pair of window and random keys that has a routine of its own, with interior and edge tiles."""
     test_interior_walk_matches_oracle(ops, dt, 1, 3, 261, 64, window, 2, 2, R)
+
+
+@pytest.mark.parametrize("dt,d,S", [(torch.float32, 64, 1000), (torch.float16, 64, 1000), (torch.float32, 32, 999),
+                                    (torch.bfloat16, 128, 515)])
+def test_edge_tiles_of_every_size(ops, dt, d, S):
+    """The first and last tokens of a head are cut into tiles of 16, 32 or 64 by how many heads there are (on 148 SMs and
+    S 1000: up to 14 heads, 16, 19): a head's result is the same among any number of heads."""
+    most = 19
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(1, most, S, d, device="cuda", generator=g).to(dt) for _ in range(3))
+    pos = torch.randint(0, S, (1, most, S - 6, 3), device="cuda", generator=g, dtype=torch.int32)
+    call = lambda n: ops.sparse_attention(*(t[:, :n].contiguous() for t in (q, k, v, pos)), window_size=5, dilation=2,
+                                          n_global=3, scale=d ** -0.5)
+    whole = call(most)
+    for n in (1, 2, 14, 16):
+        assert torch.equal(call(n), whole[:, :n])
+    ops.check_status()
+    ref = dense.sparse_attention_dense(q[0, 0].cpu().double() * d ** -0.5, k[0, 0].cpu().double(), v[0, 0].cpu().double(),
+                                       pos[0, 0].cpu(), 5, 2, 3)
+    assert (whole[0, 0].cpu().double() - ref).abs().max().item() <= (1e-5 if dt == torch.float32 else 1e-2)
