@@ -45,6 +45,7 @@ SIGNATURES = {
     "ftb_flash_attn_causal_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_flash_attn_window_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_flash_attn_local_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
+    "ftb_flash_attn_form_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_rnn_pack_weights": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "ftb_rnn_attention_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "ftb_rnn_attention_scratch_bytes": (_sz, [_i, _i, _i, _i]),

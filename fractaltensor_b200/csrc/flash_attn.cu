@@ -705,7 +705,7 @@ extern "C" int ftb_debug_fa_trace(unsigned long long* out) {
 namespace {
 int flash_attn_entry(const void* q, const void* k, const void* v, void* o, int B, int heads, int S, int d,
                      float scale, int dtype, bool masked, int left, int right, void* workspace,
-                     size_t workspace_bytes, void* stream_) {
+                     size_t workspace_bytes, void* stream_, int form = 0) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!q || !k || !v || !o || B <= 0 || heads <= 0 || S <= 0) return FTB_ERR_ARG;
   if (dtype != FTB_F16 && dtype != FTB_BF16) return FTB_ERR_ARG;
@@ -730,7 +730,7 @@ int flash_attn_entry(const void* q, const void* k, const void* v, void* o, int B
   if ((rc = make_tmap_2d(&mO, o, dtype, rows, d, d, 128, 64))) return rc;
   const int units = B * heads;
   const float scale_log2 = scale * 1.4426950408889634f;
-  const bool halves = halved_walks(masked, units, S, left, right, current_sm_count());
+  const bool halves = form == 0 ? halved_walks(masked, units, S, left, right, current_sm_count()) : form == 2;
   if (dtype == FTB_F16)
     return launch<__half>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
   return launch<__nv_bfloat16>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
@@ -763,4 +763,12 @@ extern "C" int ftb_flash_attn_local_fwd(const void* q, const void* k, const void
   if (left < 0 || right < 0) return FTB_ERR_ARG;
   return flash_attn_entry(q, k, v, o, B, heads, S, d, scale, dtype, true, left, right, workspace, workspace_bytes,
                           stream);
+}
+
+extern "C" int ftb_flash_attn_form_fwd(const void* q, const void* k, const void* v, void* o, int B, int heads, int S,
+                                       int d, int masked, int left, int right, int form, float scale, int dtype,
+                                       void* workspace, size_t workspace_bytes, void* stream) {
+  if (form < 0 || form > 2) return FTB_ERR_ARG;
+  return flash_attn_entry(q, k, v, o, B, heads, S, d, scale, dtype, masked != 0, left < 0 ? -1 : left, right, workspace,
+                          workspace_bytes, stream, form);
 }

@@ -257,6 +257,13 @@ int ftb_flash_attn_local_fwd(const void* q, const void* k, const void* v, void* 
                              int d, int left, int right, float scale, int dtype, void* workspace,
                              size_t workspace_bytes, void* stream);
 
+/* Any of the four with the form of the kernel named, for tests and measurements.  form: 0 by the library's rule, 1 CTAs
+ * of 256 query rows, 2 CTAs of 128 rows whose two slots take half of the keys each; results differ by rounding.
+ * masked 0: all keys (left and right are not read); else keys i-left .. i+right, left < 0: no limit. */
+int ftb_flash_attn_form_fwd(const void* q, const void* k, const void* v, void* o, int B, int heads, int S, int d,
+                            int masked, int left, int right, int form, float scale, int dtype, void* workspace,
+                            size_t workspace_bytes, void* stream);
+
 /* Token-level sparse attention: dilated window + random + global keys, per head.  Stands in for
  * per_head_attn / sparse_attn (examples/sparse_attention/sparse_attention.py:24-76).  The first and
  * last n_global tokens of a head attend to each other only.  Every other token i attends to the
