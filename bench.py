@@ -361,7 +361,7 @@ def other_configs(ops, dev, pk, cpu):
     out.append(tensor_entry("attention RNN bf16 H512 N64, 50 source + 50 target steps", ms,
                             2 * Lr * Nr * 2 * (2 * Hr) * Hr, samples_steps_per_s=Nr * 2 * Lr / (ms * 1e-3),
                             note="one scan kernel over the source, all decoder cells as one level: 50 dependent steps of "
-                                 "1.9 us; latency-bound, the tensor roofline is quoted for context",
+                                 "1.5 us; latency-bound, the tensor roofline is quoted for context",
                             cpu_baseline=cpu.get("rnn_attention")))
     del rp, Wps, Wpt, xs_, ys_
 

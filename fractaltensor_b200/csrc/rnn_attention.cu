@@ -20,9 +20,10 @@
 //
 // Layout: time-major padded batches, row (j, n) of `enc` at (j * N + n) * H.  Sequence n attends to
 // encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: len * H encoder
-// elements a sequence in (twice: for the scores and for the sum), Lt * H out; then Lt * H decoder elements in.
-// With the scores in a launch of their own and the weights and sums anew for every step, the whole program (H 512, 64
-// sequences, 50 + 50 positions, bf16) took 155.8 us; as here 114.9.
+// elements a sequence in (for the scores by each of its H / 128 CTAs, and once for the sum), Lt * H out; then Lt * H
+// decoder elements in.  With the scores in a launch of their own and the weights and sums anew for every step, the whole
+// program (H 512, 64 sequences, 50 + 50 positions, bf16) took 155.8 us; as here 114.9 (with the encoder's scan as it was
+// then, in both).
 #include "../../include/ftb200.h"
 #include "ptx.cuh"
 #include "tmap.h"

@@ -22,16 +22,18 @@
 // Tiled kernel (the default): a persistent CTA walks tiles of TT consecutive tokens of one head.
 // The key and value rows the tile's windows can touch, positions [t0 - half, t0 + TT + half), are
 // contiguous in memory, and so are the tile's queries: three bulk asynchronous copies bring them
-// into shared memory under an mbarrier, for the next tile while the current one is computed (two
-// stages).  The tile's random positions are fetched into registers one tile ahead and parked in
-// shared memory.  Window rows, queries and positions then cost shared-memory latency; only the R
-// random rows per token (and window positions that wrap around the ends of the sequence) are
-// gathered from global memory, 16 bytes per lane.
-// With the example's key counts (window 5, 3 random keys) the interior tiles -- no global token,
-// no window position that wraps -- go through a routine with those counts at compile time: all
-// eight scores in registers, one softmax, no per-key bookkeeping (16.7 M warp instructions instead
-// of 29 M at the example's size).  Every CTA first walks its share of the edge tiles of all heads
-// with the general routine, then its share of the interior tiles.
+// into shared memory under an mbarrier, two stages.  Window rows and queries then cost
+// shared-memory latency; only the R random rows per token (and window positions that wrap around
+// the ends of the sequence) are gathered from global memory, 16 bytes per lane.
+//   walk_tiles     any tile, any key counts: the copies of the next tile run while this one is
+//                  computed, its random positions go through registers into shared memory one tile
+//                  ahead, a barrier of the CTA closes a tile.
+//   walk_interior  windows up to 7 beside 1 to 4 random keys, tiles with no global token and no
+//                  window position that wraps: the key counts at compile time, all scores in
+//                  registers, one softmax; a warp reads its positions straight into registers and
+//                  requests random rows a pass ahead, the last warp that has read a stage fills it.
+// Every CTA walks its share of the edge tiles of all heads with the first, then its share of the
+// interior tiles with the second.
 // Direct kernel (fallback when a tile does not fit in shared memory or R > 16): the general token
 // routine with every row gathered from global memory.
 //
@@ -365,7 +367,7 @@ sparse_attn_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   }
 }
 
-// ------------------------------------------------------------------ tiled kernel
+// ------------------------------------------------------------------ tiles
 // A tile: tokens t0 .. t0 + nt - 1 of a head and the key / value rows [lo, hi) that their windows touch.
 struct Tile {
   long long head;
@@ -497,15 +499,17 @@ __device__ __forceinline__ void walk_tiles(const T* __restrict__ q, const T* __r
 
 // The walk of one warp over interior tiles (no global token, no wrapped window position), with the number of random
 // keys known at compile time, and that of window keys (KW > 0) or a bound on it (KW < 0: up to -KW): no per-key
-// bookkeeping, one softmax over the scores.  Nothing branches on the window either way: under a bound, rows past the window
-// are loads that do not happen, so the scores' loads, products and shuffles still overlap.  Window rows and queries come from the stage, random rows from global
-// memory.
-//   What bounds it is the latency of the random rows: 6 rows of 256 bytes a token at the example's counts, with 16
-// warps an SM.  So a warp works one pass (32 / LPT tokens) ahead of itself: the random keys of its next pass are
-// requested into the registers that the scores of this one have just freed, the random values behind the
-// weighted sum, and the positions of the pass after that behind them.  And warps do not wait for one another:
-// the last warp that has read a stage fills it with the tile after the next.  (B 2, 16 heads, S 4096, d 64, the example's
-// counts, fp32: 44.8 us with a pass's rows requested at its beginning and a barrier of the CTA a tile, 41.8 so.)
+// bookkeeping, one softmax over the scores.  Nothing branches on the window either way: under a bound, rows past the
+// window are loads that do not happen, so the scores' loads, products and shuffles still overlap.  Window rows and
+// queries come from the stage, random rows from global memory.
+//   What bounds it is latency at 16 warps an SM: of shuffles and shared memory first, then of the arithmetic, and of the
+// random rows (6 rows of 256 bytes a token at the example's counts) third; these came first while a pass's rows were
+// requested at its beginning.  So a warp works one pass (32 / LPT tokens) ahead of itself: the random keys of its next
+// pass are requested into the registers that the scores of this one have just freed, the random values behind the
+// weighted sum, and the positions of the pass after that behind them.  And warps do not wait for one another: the last
+// warp that has read a stage fills it with the tile after the next.  (B 2, 16 heads, S 4096, d 64, the example's counts,
+// fp32: 44.8 us with a pass's rows requested at its beginning and a barrier of the CTA a tile, 41.8 so.  fp32 with 4
+// random keys spills up to 36 bytes a thread at 128 registers.)
 template <typename T, int LPT, int KW, int KR>
 __device__ __forceinline__ void walk_interior(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                               const int* __restrict__ rand_pos, T* __restrict__ o, const SparseArgs& a,

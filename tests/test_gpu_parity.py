@@ -737,7 +737,7 @@ def test_flash_attention(ops, dt, shape):
 
 def test_flash_attention_large_scores_rescale_path(ops):
     """Scores that grow block after block force the running maximum (and the lazy rescale
-    of the accumulator) to move."""
+    of the accumulator) to move, in the form of the kernel that the library takes for so few tiles."""
     B, h, S = 1, 2, 1024
     q, k, v = dense.make_attention_inputs(B, h, S, 128, 8, dtype=torch.float16)
     ramp = torch.linspace(0.2, 3.0, S)[None, None, :, None]
@@ -800,7 +800,8 @@ def test_flash_attention_causal_ignores_later_keys(ops):
 @pytest.mark.parametrize("window", [1, 5, 64, 127, 128, 129, 200, 256, 300, 511, 1000, 5000])
 def test_flash_attention_window(ops, window):
     """Sliding window ending at the query: windows below, at and above the 128-key block and the
-    256-row CTA sizes, one that covers the whole sequence, and single-key attention (out = v)."""
+    256-row CTA sizes, one that covers the whole sequence, and single-key attention (out = v).  (In the form of the
+    kernel that the library takes for so few tiles; test_gpu_attention_forms.py has both.)"""
     B, h, S = 1, 2, 1280
     q, k, v = dense.make_attention_inputs(B, h, S, 128, 22, dtype=torch.bfloat16)
     sc = 1.0 / math.sqrt(128.0)
@@ -815,7 +816,8 @@ def test_flash_attention_window(ops, window):
                                    (256, 256), (500, 129), (5000, 0), (0, 5000), (5000, 5000)])
 def test_flash_attention_local(ops, local):
     """Two-sided window: edges inside, on and across the 128-key blocks and 256-row CTAs, one-sided
-    in either direction, and windows that cover the whole sequence (= unmasked attention)."""
+    in either direction, and windows that cover the whole sequence (= unmasked attention).  (In the form of the
+    kernel that the library takes for so few tiles; test_gpu_attention_forms.py has both.)"""
     B, h, S = 1, 2, 1280
     q, k, v = dense.make_attention_inputs(B, h, S, 128, 24, dtype=torch.float16)
     sc = 1.0 / math.sqrt(128.0)
