@@ -204,6 +204,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         ok = mbar_wait_warp(&w_smem, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
       if (!ok) break;
       tc_fence_after();
+      const bool late = leader && a.n_slots == 1, early = leader && a.n_slots > 1;
       for (int t = 0; t < steps; ++t, ++k) {
         const int acc = k & 1;
         const uint32_t d_tmem = tmem_base + acc * NB;
@@ -217,10 +218,14 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
                   kb_x - in_t, in_t > 0 ? 1u : 0u);
         // Where there is one input tile it goes back behind the recurrent half, not before it: its next copy would otherwise
         // be under way while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64
-        // sequences: D8 L100 500 us, behind it 464).  With two, the copy made room for is the one after the next: before
-        // the half it is 1 % faster at H 256.
-        const bool late = a.n_slots == 1;
-        if (!late && leader) umma_commit(&in_empty[slot]);
+        // sequences: D8 L100 500 us a call, behind it 460).  With two, the copy made room for is the one after the next: before
+        // the half it is 1 % faster at H 256, and so is this order of slot and commits (D1 L100 N16 H256 156 us, with the
+        // slot's step behind the half 158.5; inside a branch on the number of slots 8 % behind).
+        if (early) umma_commit(&in_empty[slot]);
+        if (++slot == a.n_slots) {
+          slot = 0;
+          phase ^= 1u;
+        }
         if (t > 0) {
           ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           if (!ok) break;
@@ -229,11 +234,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           ++states;
         }
         if (leader) umma_commit(&acc_full[acc]);
-        if (late && leader) umma_commit(&in_empty[slot]);
-        if (++slot == a.n_slots) {
-          slot = 0;
-          phase ^= 1u;
-        }
+        if (late) umma_commit(&in_empty[0]);
       }
       if (ok && leader) umma_commit(&swept);
       ++sweep;
