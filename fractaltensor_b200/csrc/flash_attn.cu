@@ -659,7 +659,7 @@ int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& m
 // Whether a call's CTAs take 128 query rows and half of their blocks a slot, or 256 rows and all of them: by the
 // estimates of both.  A CTA takes kFixed us and kBlock for each block of its longer slot; where there are more CTAs than
 // SMs, equal ones go in whole waves, unequal ones (masks), longest first, about half of one beyond their mean.
-// Measured, us, 256 rows / 128 rows (* taken), 1 x heads x S: causal 16 x 2048 35.3 / 27.1*, 8 x 1024 19.5 / 14.3*, 4 x 4096
+// Measured, us, both forms launched as dependents, 256 rows / 128 rows (* taken), 1 x heads x S: causal 16 x 2048 35.3 / 27.1*, 8 x 1024 19.5 / 14.3*, 4 x 4096
 // 63.6 / 37.9*, 32 x 2048 40.2* / 53.6, 64 x 2048 82.2* / 102.6; full 16 x 256 8.3 / 7.5*, 16 x 1024 20.4 / 15.0*, 16 x 2048
 // 36.5* / 43.6 (two waves of 128 rows), 20 x 2048 66.9 / 62.3* (two waves / three), 12 x 4096 130.7 / 112.5*; window of 600
 // 8 x 2048 19.6 / 13.7*, keys i-1000..i+500 8 x 4096 32.9* / 39.7.  Halves that are estimated less than a tenth faster keep the
