@@ -727,15 +727,18 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
     // one, which is issue-bound on its bookkeeping.  us, B 2, 16 heads, S 4096, d 64, general / one routine told any
     // window up to 7, each score in a branch of its own / own counts: window 7 and 4 random keys fp32 67.0 / 62.2 /
     // 53.0, fp16 78.9 / 50.4 / 40.2; 3 and 1 34.9 / 33.6 / 28.9, 35.4 / 29.9 / 24.3; d 128, 5 and 4: 101.6 / 77.3 and
-    // 86.3 / 70.4 told / own.
+    // 86.3 / 70.4 told / own.  Rows of 1 KB leave the general one bound by memory too: from window 5 on no other there
+    // (fp32, d 256, 1 x 16 x 4096, 5 and 3 107.5 / 107.6, 7 and 4 137.4 / 137.5 general / own; window 1 and 1 65.6 / 47.8).
+    constexpr bool kOwn = LPT * sizeof(T) < 128;
+    constexpr int W5 = kOwn ? 5 : 0, W7 = kOwn ? 7 : 0, R1 = kOwn, R2 = 2 * kOwn, R3 = 3 * kOwn, R4 = 4 * kOwn;
     const Kernel kernels[13] = {sparse_attn_tile_kernel<T, LPT, 0, 0>,
                                 sparse_attn_tile_kernel<T, LPT, -3, 1>, sparse_attn_tile_kernel<T, LPT, -3, 2>,
                                 sparse_attn_tile_kernel<T, LPT, -3, 3>, sparse_attn_tile_kernel<T, LPT, -3, 4>,
-                                sparse_attn_tile_kernel<T, LPT, 5, 1>,  sparse_attn_tile_kernel<T, LPT, 5, 2>,
-                                sparse_attn_tile_kernel<T, LPT, 5, 3>,  sparse_attn_tile_kernel<T, LPT, 5, 4>,
-                                sparse_attn_tile_kernel<T, LPT, 7, 1>,  sparse_attn_tile_kernel<T, LPT, 7, 2>,
-                                sparse_attn_tile_kernel<T, LPT, 7, 3>,  sparse_attn_tile_kernel<T, LPT, 7, 4>};
-    const int fast = a.as_shipped || a.window > 7 || a.R < 1 || a.R > 4
+                                sparse_attn_tile_kernel<T, LPT, W5, R1>, sparse_attn_tile_kernel<T, LPT, W5, R2>,
+                                sparse_attn_tile_kernel<T, LPT, W5, R3>, sparse_attn_tile_kernel<T, LPT, W5, R4>,
+                                sparse_attn_tile_kernel<T, LPT, W7, R1>, sparse_attn_tile_kernel<T, LPT, W7, R2>,
+                                sparse_attn_tile_kernel<T, LPT, W7, R3>, sparse_attn_tile_kernel<T, LPT, W7, R4>};
+    const int fast = a.as_shipped || a.window > (kOwn ? 7 : 3) || a.R < 1 || a.R > 4
                          ? 0
                          : (a.window <= 3 ? 0 : (a.window == 5 ? 4 : 8)) + a.R;
     if (ensure_dynamic_smem(kernels[0], kMaxTileSmem, configured[0]) &&

@@ -224,7 +224,7 @@ def test_every_pair_of_key_counts(ops, dt, window, R):
 
 
 @pytest.mark.parametrize("dt,d,S", [(torch.float32, 64, 1000), (torch.float16, 64, 1000), (torch.float32, 32, 999),
-                                    (torch.bfloat16, 128, 515)])
+                                    (torch.bfloat16, 128, 515), (torch.float32, 256, 515)])
 def test_edge_tiles_of_every_size(ops, dt, d, S):
     """The first and last tokens of a head are cut into tiles of 16, 32 or 64 by how many heads there are (on 148 SMs and
     S 1000: up to 14 heads, 16, 19): a head's result is the same among any number of heads."""
