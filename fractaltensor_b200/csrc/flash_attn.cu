@@ -41,6 +41,11 @@
 #include "tmap.h"
 
 namespace ftb {
+
+// flash_pair.cu
+int flash_pair_launch(const void* q, const void* k, const void* v, void* o, int64_t rows, int n_bh, int S, int dtype,
+                      bool masked, int left, int right, float scale_log2, int* status, cudaStream_t stream);
+
 namespace {
 
 constexpr int kHalfBytes = 128 * 128;  // 128 rows x 64 16-bit columns
@@ -97,7 +102,7 @@ __device__ unsigned long long g_fa_trace[2][32][8];
 // kHalves: both query slots of a CTA hold the same 128 rows, slot 0 walks the first half of their key/value blocks and
 // slot 1 the second, and the two results are put together in shared memory at the end.  A CTA's time is set by its
 // slots' chains, not by the tensor pipe, so that half the blocks are half the time; the price is that a K/V tile
-// serves one slot and not two.  For calls whose query tiles leave SMs idle (halved_walks below).
+// serves one slot and not two.  For calls whose query tiles leave SMs idle (attention_form below).
 // The K/V stream of a walk of n0 and n1 blocks (n1 = n0 or n0 - 1): K(0,0), K(1,0), then for j = 0, 1, ..: V(0,j),
 // K(0,j+1), V(1,j), K(1,j+1), without the tiles that do not exist.
 struct StreamTile {
@@ -656,39 +661,46 @@ int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& m
                 : launch<T, false, false>(mQ, mK, mV, mO, n_bh, S, -1, 0, scale_log2, status, stream);
 }
 
-// Whether a call's CTAs take 128 query rows and half of their blocks a slot, or 256 rows and all of them: by the
-// estimates of both.  A CTA takes kFixed us and kBlock for each block of its longer slot; where there are more CTAs than
-// SMs, equal ones go in whole waves, unequal ones (masks), longest first, about half of one beyond their mean.
-// Measured, us, both forms launched as dependents, 256 rows / 128 rows (* taken), 1 x heads x S: causal 16 x 2048 35.3 / 27.1*, 8 x 1024 19.5 / 14.3*, 4 x 4096
-// 63.6 / 37.9*, 32 x 2048 40.2* / 53.6, 64 x 2048 82.2* / 102.6; full 16 x 256 8.3 / 7.5*, 16 x 1024 20.4 / 15.0*, 16 x 2048
-// 36.5* / 43.6 (two waves of 128 rows), 20 x 2048 66.9 / 62.3* (two waves / three), 12 x 4096 130.7 / 112.5*; window of 600
-// 8 x 2048 19.6 / 13.7*, keys i-1000..i+500 8 x 4096 32.9* / 39.7.  Halves that are estimated less than a tenth faster keep the
-// 256 rows: between 0.9 and 1 of the estimate the time is 0.9 to 1.19 of theirs (full 40 x 1024 43.3* / 44.0, 45 x 2048 104.7* /
-// 114.1, 56 x 768 35.1* / 41.7; causal 16 x 2560 54.3* / 48.9), below it 0.53 to 0.97.
-bool halved_walks(bool masked, int n_bh, int S, int left, int right, int sm_count) {
-  constexpr double kFixed = 4.5, kBlock = 1.9;
-  double us[2];
-  for (int halves = 0; halves < 2; ++halves) {
-    const int rows = halves ? 128 : 256, tiles = S / rows;
-    double total = 0, longest = 0;
+// The form of a call: 1 = CTAs of 256 query rows, 2 = of 128 rows and half of their blocks a slot, 3 = pairs of CTAs (flash_pair.cu),
+// by the estimates of all three in us.  A tile of query rows takes kFixed and kBlock for each block that its longer slot
+// walks, and a pair kEdge for each block that an edge of a mask crosses.  Where there are more tiles than places for
+// them (SMs, pairs of SMs), equal ones go in whole rounds, unequal ones (masks, longest first) about half a round of CTAs beyond
+// their mean, pairs, which take theirs in a balanced order, a tenth.
+// Measured, us, forms 1 / 2 / 3 (* taken): full 16 x 256 8.2 / 7.2* / 7.4, 4 x 512 11.4 / 9.6 / 9.0*, 64 x 512 14.3* / 20.8 / 14.9,
+// 40 x 1024 39.5 / 40.1 / 26.8*, 16 x 2048 35.9 / 43.0 / 33.2*, 20 x 2048 68 / 63 / 45*, 33 x 1280 46.7 / - / 31.5*, 4 x 4096 63 / 37 / 33*,
+// 256 x 2048 490 / 574 / 438*; causal 160 x 256 19.7 / 21.3 / 15.4*, 64 x 512 14.6* / 19.0 / 16.1, 64 x 768 26.7 / 27.8 / 21.8*, 8 x 1024 19.5 /
+// 14.1 / 13.5*, 16 x 2048 37 / 28 / 23.4*, 64 x 2048 82 / 104 / 77*, 16 x 2560 45 / 41 / 32*, 4 x 4096 64 / 39 / 35*; window of 100 32 x 4096 50* /
+// 57 / 54, of 600 8 x 2048 20 / 14.7* / 18.2; keys i-1000..i+500 8 x 4096 34.5* / 40 / 39.5.
+// Between forms 1 and 2 halves that are estimated less than a tenth faster keep the 256 rows: between 0.9 and 1 of the
+// estimate the time is 0.9 to 1.19 of theirs, below it 0.53 to 0.97.
+int attention_form(bool masked, int n_bh, int S, int left, int right, int sm_count) {
+  constexpr double kFixed[3] = {4.5, 5.0, 1.9}, kBlock[3] = {1.85, 2.1, 0.83}, kPairCall = 3.6, kPairMasked = 0.9, kEdge = 0.35;
+  double us[3];
+  for (int form = 0; form < 3; ++form) {
+    const int rows = form == 1 ? 128 : 256, tiles = S / rows;
+    double total = 0, longest = 0, shortest = 1e30;
     for (int i = 0; i < tiles; ++i) {
       const int r0 = i * rows;
       const int lo = masked && left >= 0 && r0 > left ? (r0 - left) >> 7 : 0;
       const int hi = masked && r0 + rows - 1 < S - right ? (r0 + rows - 1 + right) >> 7 : S / 128 - 1;
-      const int blocks = halves ? (hi - lo + 2) / 2 : hi - lo + 1;
-      const double t = kFixed + kBlock * blocks;
+      const int blocks = form == 1 ? (hi - lo + 2) / 2 : hi - lo + 1;
+      double t = kFixed[form] + (form == 2 && masked ? kPairMasked : kBlock[form]) * blocks;
+      if (form == 2 && masked) t += kEdge * std::min(blocks, left >= 0 && r0 > left ? 6 : 2);
       total += t;
-      if (t > longest) longest = t;
+      longest = std::max(longest, t);
+      shortest = std::min(shortest, t);
     }
-    const double waves = static_cast<double>(n_bh) * tiles / sm_count;
+    const double waves = static_cast<double>(n_bh) * tiles / (form == 2 ? sm_count / 2 : sm_count);
     if (waves <= 1)
-      us[halves] = longest;
+      us[form] = longest;
     else if (masked)
-      us[halves] = std::max(longest, (waves + 0.5) * total / tiles);
+      us[form] = std::max(longest + shortest, (waves + (form == 2 ? 0.1 : 0.5)) * total / tiles);
     else
-      us[halves] = std::ceil(waves) * longest;
+      us[form] = std::ceil(waves) * longest;
   }
-  return us[1] < 0.9 * us[0];
+  us[2] += kPairCall;
+  const int single = us[1] < 0.9 * us[0] ? 1 : 0;
+  return us[2] < us[single] ? 3 : single + 1;
 }
 
 }  // namespace
@@ -723,14 +735,16 @@ int flash_attn_entry(const void* q, const void* k, const void* v, void* o, int B
   // every later call on that workspace is a no-op until the caller clears the word.
   int* status = static_cast<int*>(workspace);
 
+  const int units = B * heads;
+  const float scale_log2 = scale * 1.4426950408889634f;
+  if (form == 0) form = attention_form(masked, units, S, left, right, current_sm_count());
+  if (form == 3) return flash_pair_launch(q, k, v, o, rows, units, S, dtype, masked, left, right, scale_log2, status, stream);
+  const bool halves = form == 2;
   CUtensorMap mQ, mK, mV, mO;
   if ((rc = make_tmap_2d(&mQ, q, dtype, rows, d, d, 128, 64))) return rc;
   if ((rc = make_tmap_2d(&mK, k, dtype, rows, d, d, 128, 64))) return rc;
   if ((rc = make_tmap_2d(&mV, v, dtype, rows, d, d, 128, 64))) return rc;
   if ((rc = make_tmap_2d(&mO, o, dtype, rows, d, d, 128, 64))) return rc;
-  const int units = B * heads;
-  const float scale_log2 = scale * 1.4426950408889634f;
-  const bool halves = form == 0 ? halved_walks(masked, units, S, left, right, current_sm_count()) : form == 2;
   if (dtype == FTB_F16)
     return launch<__half>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
   return launch<__nv_bfloat16>(masked, halves, mQ, mK, mV, mO, units, S, left, right, scale_log2, status, stream);
@@ -768,7 +782,7 @@ extern "C" int ftb_flash_attn_local_fwd(const void* q, const void* k, const void
 extern "C" int ftb_flash_attn_form_fwd(const void* q, const void* k, const void* v, void* o, int B, int heads, int S,
                                        int d, int masked, int left, int right, int form, float scale, int dtype,
                                        void* workspace, size_t workspace_bytes, void* stream) {
-  if (form < 0 || form > 2) return FTB_ERR_ARG;
+  if (form < 0 || form > 3) return FTB_ERR_ARG;
   return flash_attn_entry(q, k, v, o, B, heads, S, d, scale, dtype, masked != 0, left < 0 ? -1 : left, right, workspace,
                           workspace_bytes, stream, form);
 }

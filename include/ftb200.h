@@ -258,7 +258,8 @@ int ftb_flash_attn_local_fwd(const void* q, const void* k, const void* v, void* 
                              size_t workspace_bytes, void* stream);
 
 /* Any of the four with the form of the kernel named, for tests and measurements.  form: 0 by the library's rule, 1 CTAs
- * of 256 query rows, 2 CTAs of 128 rows whose two slots take half of the keys each; results differ by rounding.
+ * of 256 query rows, 2 CTAs of 128 rows whose two slots take half of the keys each, 3 pairs of CTAs on 256 rows;
+ * results differ by rounding.
  * masked 0: all keys (left and right are not read); else keys i-left .. i+right, left < 0: no limit. */
 int ftb_flash_attn_form_fwd(const void* q, const void* k, const void* v, void* o, int B, int heads, int S, int d,
                             int masked, int left, int right, int form, float scale, int dtype, void* workspace,
