@@ -771,7 +771,8 @@ int launch_sparse(const void* q, const void* k, const void* v, const int* rand_p
         // its edges: they are cut into the smallest tiles of which the CTAs with an interior tile less can take one each
         // (fp32, d 64, window 5, 3 random keys, 4 x 512 6.8 us with tiles of 64, 5.0 so; 8 x 2048 8.6, 6.5; fp16, d 128,
         // 8 x 1024 14.9, 8.4).
-        const auto edges = [&](int tt) { return (a.S + tt - 1) / tt - interior * (TT / tt); };
+        // (Without global tokens and with a window of one key there are none, and the last interior tile may be a short one.)
+        const auto edges = [&](int tt) { return m == 0 ? 0 : (a.S + tt - 1) / tt - interior * (TT / tt); };
         const long long all = a.heads_total * interior, idle = full - all % full;
         a.edge_TT = 16;
         while (a.edge_TT < TT && a.heads_total * edges(a.edge_TT) > idle) a.edge_TT *= 2;

@@ -241,3 +241,17 @@ def test_edge_tiles_of_every_size(ops, dt, d, S):
     ref = dense.sparse_attention_dense(q[0, 0].cpu().double() * d ** -0.5, k[0, 0].cpu().double(), v[0, 0].cpu().double(),
                                        pos[0, 0].cpu(), 5, 2, 3)
     assert (whole[0, 0].cpu().double() - ref).abs().max().item() <= (1e-5 if dt == torch.float32 else 1e-2)
+
+
+@pytest.mark.parametrize("R", [1, 2, 3, 4])
+@pytest.mark.parametrize("dt,d", [(torch.float32, 64), (torch.float16, 64), (torch.bfloat16, 32)])
+def test_no_edge_tiles(ops, dt, d, R):
+    """A window of one key and no global tokens: every tile is an interior one, a short last one among them."""
+    for S in (1, 17, 32, 48, 70, 96, 130, 144, 500):
+        for heads in (1, 3):
+            q, k, v, pos = _inputs(1, heads, S, d, 0, R, S + heads, dt)
+            out = ops.sparse_attention(q.cuda(), k.cuda(), v.cuda(), pos.cuda(), 1, 1, n_global=0)
+            ops.check_status()
+            ref = dense.sparse_attention_dense(q.double(), k.double(), v.double(), pos, 1, 1, n_global=0)
+            # fp32 sums of a few terms of order 1; 16-bit results are rounded once (2^-11, 2^-8)
+            assert (out.cpu().double() - ref).abs().max().item() <= {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1e-2}[dt]
