@@ -475,7 +475,7 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
           if (PERSIST && plan.trace && warp == 2) plan.trace[tile * 4 + 3] = globaltimer_ns();
 #endif
           if (PAIR)
-            mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+            mbar_arrive_peer(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
           else
             mbar_arrive(&tempty_bar[acc]);
           mbar_arrive(&stg_ready_bar);
@@ -561,7 +561,7 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
           if (PERSIST && plan.trace && warp == 2) plan.trace[tile * 4 + 3] = globaltimer_ns();
 #endif
           if (PAIR)
-            mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+            mbar_arrive_peer(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
           else
             mbar_arrive(&tempty_bar[acc]);
         }

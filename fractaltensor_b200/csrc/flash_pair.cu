@@ -100,9 +100,6 @@ __device__ __forceinline__ uint64_t fma_to_f32x2(uint64_t a, uint64_t b, uint64_
 __device__ __forceinline__ void unpair_f32x2(uint64_t v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
 // Whether the phase is over, without waiting.
 __device__ __forceinline__ bool mbar_test(const uint64_t* bar, uint32_t parity) {
   uint32_t ok;

@@ -345,7 +345,7 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
           if constexpr (decltype(last_)::value) {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+            if (lane == 0) mbar_arrive_peer(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
           }
 #pragma unroll
           for (int cd = 0; cd < n; ++cd) {
