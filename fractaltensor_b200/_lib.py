@@ -49,6 +49,7 @@ SIGNATURES = {
     "ftb_rnn_pack_weights": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "ftb_rnn_attention_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "ftb_rnn_attention_scratch_bytes": (_sz, [_i, _i, _i, _i]),
+    "ftb_rnn_attention_scratch_bytes_all": (_sz, [_i, _i, _i, _i, _i]),
     "ftb_rnn_attention_fwd": (_i, [_vp] * 13 + [_i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "ftb_rnn_attention_fwd_scratch": (_i, [_vp] * 13 + [_i, _i, _i, _i, _i, _vp, _sz, _vp, _sz, _vp]),
     "ftb_sparse_attn_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp]),

@@ -85,8 +85,12 @@ __device__ __forceinline__ void row_dots(const T* rows, long long stride, int co
   for (int r = 0; r < kDots; ++r) s[r] = 0.f;
   for (int h = lane * n; h < H; h += 32 * n) {
     float p[n];
+    if ((reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
+      ld_piece(proj + h, p);
+    } else {
 #pragma unroll
-    for (int i = 0; i < n; ++i) p[i] = ld_f32<T>(proj + h + i);
+      for (int i = 0; i < n; ++i) p[i] = ld_f32<T>(proj + h + i);
+    }
 #pragma unroll
     for (int r = 0; r < kDots; ++r) {
       if (r >= count) continue;
@@ -241,6 +245,261 @@ attn_finish_kernel(T* __restrict__ dec, const T* __restrict__ dec_proj, const fl
     }
 }
 
+// All that follows the encoder's scan in one launch, where the decoder's input halves y_t W (fp32, `pre` [Lt, N, H]) are there
+// already: scores, weights and vector of a sequence, the product of the vector with U, the decoder states of all steps and
+// their terms.  A cluster of H / 128 CTAs takes two sequences, a CTA 128 columns of both: U's 128 rows (128 KB at H 512) are
+// then read once for the two, which with one sequence a cluster would be 32 MB through L2 for 64.  A warp's score rows are
+// shared by the cluster; scores, vectors and partial terms go between its CTAs through shared memory.
+// Latency: what the later stages read (the rows for the sum, U, the input halves) depends on no earlier stage and is requested
+// behind the score rows; what is left is a trip to L2 and three exchanges over the cluster.  H 512, 64 sequences, 50 + 50 positions, bf16, after
+// the scan: 12.5 + 10.7 + 9.2 us as three launches (vector, cells, finish), 15 so, and the product in front of the scan 2 us longer;
+// the whole program 105.5 us before, 94.2 so.  (U by 128 row copies of one warp: 99.4; its rows into registers: 98.9.)
+constexpr int kDecThreads = 512, kDecWarps = kDecThreads / 64;  // of a sequence
+constexpr int kDecMaxH = 512;
+constexpr int kDecMaxSteps = 256;  // of source or target
+constexpr int kDecAhead = 8;       // steps of a warp, and rows of the sum of a thread over 2, requested ahead
+
+__device__ __forceinline__ void st_cluster_f32(float* p, uint32_t rank, float x) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(smem_u32(p), rank)), "f"(x) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void st_cluster_16(T* p, uint32_t rank, T x) {
+  asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(map_to_cta(smem_u32(p), rank)),
+               "h"(*reinterpret_cast<const unsigned short*>(&x)) : "memory");
+}
+// D += A B of 16 x 8 x 16, A rows of 16-bit numbers, fp32 sums.
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, __half) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, __nv_bfloat16) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kDecThreads)
+attn_decode_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, const int* __restrict__ src_lens,
+                   float* __restrict__ scores, const float* __restrict__ pre, const T* __restrict__ U, int ldu,
+                   const float* __restrict__ bias, const T* __restrict__ dec_proj, T* __restrict__ dec, T* __restrict__ out,
+                   int Lt, int Ls, int N, int H, int* __restrict__ status) {
+  constexpr int kN = 8, kColGroups = kAttnCols / kN, kRowGroups = kDecThreads / 2 / kColGroups;
+  constexpr int kMaxCtas = kDecMaxH / kAttnCols;
+  __shared__ float s_score[2][kDecMaxSteps], s_w[2][kDecMaxSteps];
+  __shared__ float s_term[kMaxCtas][2][kDecMaxSteps];  // the CTAs' parts of the decoder's terms
+  __shared__ float s_part[2][kRowGroups][kAttnCols];
+  __shared__ __align__(16) T s_v[2][kDecMaxH];
+  __shared__ __align__(16) float s_z[2][2][kAttnCols];  // [half of K][sequence]: v . U
+  __shared__ uint64_t u_full;
+  __shared__ int s_first[2], s_abort;
+  extern __shared__ __align__(16) unsigned char s_u_raw[];  // this CTA's 128 rows of U, 16 bytes between them
+  T* s_u = reinterpret_cast<T*>(s_u_raw);
+  const int u_stride = H + 8;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, seq = wid / kDecWarps, w = wid % kDecWarps, gt = tid & 255;
+  const uint32_t rank = cluster_ctarank(), ctas = H / kAttnCols;
+  const int n = 2 * (blockIdx.x / ctas) + seq, col0 = rank * kAttnCols;
+  const bool mine = n < N;
+  const long long step_elems = static_cast<long long>(N) * H, row = static_cast<long long>(n) * H;
+  const auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + seq) : "memory"); };
+  if (gt == 0) s_first[seq] = Lt;
+  if (tid == 0) {
+    mbar_init(&u_full, 1);
+    s_abort = 0;
+    fence_barrier_init();
+    mbar_arrive_expect_tx(&u_full, kAttnCols * H * 2);
+  }
+  grid_launch_dependents();
+  cluster_sync_all();  // nobody stores into a CTA that has not started; u_full is set up
+  grid_dependency_wait();
+  const int len = mine ? source_len(src_lens, n, Ls) : 0;
+
+  // scores of all source positions, rows dealt to the warps of the cluster
+  if (mine)
+    for (int j0 = (rank * kDecWarps + w) * kDots; j0 < Ls; j0 += ctas * kDecWarps * kDots) {
+      float s[kDots];
+      row_dots(enc + row + j0 * step_elems, step_elems, Ls - j0, enc_proj, H, lane, s);
+#pragma unroll
+      for (int r = 0; r < kDots; ++r)
+        if (lane == r && j0 + r < Ls) {
+          scores[static_cast<long long>(j0 + r) * N + n] = s[r];
+          for (uint32_t k = 0; k < ctas; ++k) st_cluster_f32(&s_score[seq][j0 + r], k, s[r]);
+        }
+    }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // What later stages read does not depend on the scores: on its way while they come together.  (A copy takes its warp some
+  // 60 cycles: every warp issues its share.)
+  if (lane < kAttnCols / (2 * kDecWarps)) {
+    const int i = wid * (kAttnCols / (2 * kDecWarps)) + lane;
+    bulk_load_1d(s_u + i * u_stride, U + static_cast<long long>(col0 + i) * ldu, H * 2, &u_full);
+  }
+  __syncwarp();
+  const int cg = gt % kColGroups, rg = gt / kColGroups, c = col0 + lane * 4;
+  uint4 ahead_row[kDecAhead / 2];
+  float4 ahead_pre[kDecAhead];
+#pragma unroll
+  for (int i = 0; i < kDecAhead / 2; ++i) {
+    const int j = rg + i * kRowGroups;
+    if (j < len) ahead_row[i] = *reinterpret_cast<const uint4*>(enc + row + j * step_elems + col0 + cg * kN);
+  }
+#pragma unroll
+  for (int i = 0; i < kDecAhead; ++i) {
+    const int t = w + i * kDecWarps;
+    if (mine && t < Lt) ahead_pre[i] = __ldcs(reinterpret_cast<const float4*>(pre + t * step_elems + row + c));
+  }
+  const float4 b = bias != nullptr ? __ldg(reinterpret_cast<const float4*>(bias + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float proj[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) proj[i] = ld_f32<T>(dec_proj + c + i);
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+
+  float mx = -INFINITY;
+  for (int j = lane; j < len; j += 32) mx = fmaxf(mx, s_score[seq][j]);
+  mx = warp_max(mx);
+  float sum = 0.f;
+  for (int j = lane; j < len; j += 32) {
+    const float e = expf(s_score[seq][j] - mx);
+    if (w == 0) s_w[seq][j] = e;
+    sum += e;
+  }
+  sum = warp_sum(sum);
+  const float inv = len > 0 ? 1.f / sum : 0.f;
+  group_sync();
+
+  // weighted sum: a thread takes 16 bytes of every kRowGroups-th row
+  {
+    float acc[kN];
+#pragma unroll
+    for (int i = 0; i < kN; ++i) acc[i] = 0.f;
+    const auto add = [&](int j, const uint4& piece) {
+      float x[kN];
+      ld_piece(reinterpret_cast<const T*>(&piece), x);
+#pragma unroll
+      for (int i = 0; i < kN; ++i) acc[i] = fmaf(s_w[seq][j], x[i], acc[i]);
+    };
+#pragma unroll
+    for (int i = 0; i < kDecAhead / 2; ++i)
+      if (rg + i * kRowGroups < len) add(rg + i * kRowGroups, ahead_row[i]);
+    for (int j = rg + kDecAhead / 2 * kRowGroups; j < len; j += kRowGroups)
+      add(j, *reinterpret_cast<const uint4*>(enc + row + j * step_elems + col0 + cg * kN));
+#pragma unroll
+    for (int i = 0; i < kN; ++i) s_part[seq][rg][cg * kN + i] = acc[i];
+  }
+  group_sync();
+  if (gt < kAttnCols) {
+    float v = 0.f;
+#pragma unroll
+    for (int r = 0; r < kRowGroups; ++r) v += s_part[seq][r][gt];
+    T t;
+    st_f32<T>(&t, v * inv);
+    for (uint32_t r = 0; r < ctas; ++r) st_cluster_16<T>(&s_v[seq][col0 + gt], r, t);
+  }
+  mbar_wait(&u_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+  __syncwarp();
+  cluster_sync_all();
+
+  // The vector into the rows of all steps.
+  const uint2 v = *reinterpret_cast<const uint2*>(&s_v[seq][c]);
+  if (mine)
+    for (int t = w; t < Lt; t += kDecWarps) *reinterpret_cast<uint2*>(out + t * step_elems + row + c) = v;
+  // v . U: 16 units and half of K a warp; the two sequences are columns 0 and 1 of 8.
+  {
+    const int m0 = (wid & 7) * 16, half = wid >> 3, col = lane >> 2;
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    const T* ar = s_u + (m0 + (lane & 15)) * u_stride + (lane >> 4) * 8;
+    for (int k = half * (H / 2); k < (half + 1) * (H / 2); k += 16) {
+      uint32_t a[4];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(smem_u32(ar + k)) : "memory");
+      uint32_t b0 = 0, b1 = 0;
+      if (col < 2) {
+        b0 = *reinterpret_cast<const uint32_t*>(&s_v[col][k + 2 * (lane & 3)]);
+        b1 = *reinterpret_cast<const uint32_t*>(&s_v[col][k + 8 + 2 * (lane & 3)]);
+      }
+      mma16816(d, a, b0, b1, T());
+    }
+    if ((lane & 3) == 0) {
+      s_z[half][0][m0 + col] = d[0];
+      s_z[half][1][m0 + col] = d[1];
+      s_z[half][0][m0 + col + 8] = d[2];
+      s_z[half][1][m0 + col + 8] = d[3];
+    }
+  }
+  __syncthreads();
+
+  // the steps of the sequence: a warp a step, four units a lane
+  if (mine) {
+    const float4 z0 = *reinterpret_cast<const float4*>(&s_z[0][seq][lane * 4]);
+    const float4 z1 = *reinterpret_cast<const float4*>(&s_z[1][seq][lane * 4]);
+    const float zz[4] = {z0.x + z1.x, z0.y + z1.y, z0.z + z1.z, z0.w + z1.w}, bb[4] = {b.x, b.y, b.z, b.w};
+    const auto step = [&](int t, const float4& p) {
+      const float x[4] = {p.x, p.y, p.z, p.w};
+      T d[4];
+      float term = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        st_f32<T>(d + i, tanh_fast((t > 0 ? x[i] + zz[i] : x[i]) + bb[i]));  // step 0 starts from nothing
+        term = fmaf(ld_f32<T>(d + i), proj[i], term);
+      }
+      *reinterpret_cast<uint2*>(dec + t * step_elems + row + c) = *reinterpret_cast<const uint2*>(d);
+      term = warp_sum(term);
+      if (lane < ctas) st_cluster_f32(&s_term[rank][seq][t], lane, term);
+    };
+#pragma unroll
+    for (int i = 0; i < kDecAhead; ++i)
+      if (w + i * kDecWarps < Lt) step(w + i * kDecWarps, ahead_pre[i]);
+    for (int t = w + kDecAhead * kDecWarps; t < Lt; t += kDecWarps)
+      step(t, __ldcs(reinterpret_cast<const float4*>(pre + t * step_elems + row + c)));
+  }
+  __syncwarp();
+  cluster_sync_all();  // (the last access to another CTA's memory lies before it)
+  // Steps whose largest score, the encoder's largest plus the term, is not finite: attn_finish_kernel says what they do.
+  if (mine && len > 0)
+    for (int t = gt; t < Lt; t += 256) {
+      float term = 0.f;
+      for (uint32_t r = 0; r < ctas; ++r) term += s_term[r][seq][t];
+      if (!isfinite(mx + term)) atomicMin(&s_first[seq], t);
+    }
+  group_sync();
+  const float nan = __int_as_float(0x7FFFFFFF);
+  if (mine)
+    for (int t = s_first[seq] + w; t < Lt; t += kDecWarps)
+      for (int h = col0 + lane; h < col0 + kAttnCols; h += 32) {
+        if (t > s_first[seq]) st_f32<T>(dec + t * step_elems + row + h, nan);
+        st_f32<T>(out + t * step_elems + row + h, nan);
+      }
+}
+
+template <typename T>
+int attn_decode_t(const void* enc, const void* enc_proj, const int* src_lens, float* scores, const float* pre, const void* U,
+                  int ldu, const float* bias, const void* dec_proj, void* dec, void* out, int Lt, int Ls, int N, int H,
+                  int* status, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  static std::atomic<unsigned long long> configured{0};
+  if (!ensure_dynamic_smem(attn_decode_kernel<T>, kAttnCols * (kDecMaxH + 8) * 2, configured)) return FTB_ERR_LAUNCH;
+  cfg.gridDim = dim3((N + 1) / 2 * (H / kAttnCols));
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.dynamicSmemBytes = kAttnCols * (H + 8) * 2;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = H / kAttnCols;
+  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, attn_decode_kernel<T>, static_cast<const T*>(enc), static_cast<const T*>(enc_proj),
+                                             src_lens, scores, pre, static_cast<const T*>(U), ldu, bias, static_cast<const T*>(dec_proj),
+                                             static_cast<T*>(dec), static_cast<T*>(out), Lt, Ls, N, H, status);
+  count_launch();
+  if (err != cudaSuccess) cudaGetLastError();
+  return err == cudaSuccess ? FTB_OK : FTB_ERR_LAUNCH;
+}
+
 template <typename T>
 int attn_vectors_t(const void* enc, const void* enc_proj, const int* src_lens, float* scores, void* out, int Lt, int Ls,
                    int N, int H, cudaStream_t stream) {
@@ -282,6 +541,24 @@ int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const 
     case FTB_F16: return attn_vectors_t<__half>(enc, enc_proj, src_lens, scores, out, Lt, Ls, N, H, stream);
     default: return attn_vectors_t<__nv_bfloat16>(enc, enc_proj, src_lens, scores, out, Lt, Ls, N, H, stream);
   }
+}
+
+// Whether launch_attn_decode takes a call (its scratch aside): where all clusters are on the device at once (a CTA an SM; 72
+// sequences at H 512) and a sequence has few steps.  us, the whole program as three launches behind the scan / as one, H 512, bf16:
+// 50 + 50 positions, 55 sequences 109.0 / 98.4, 256 136.1 / 151.6; 26 + 52, 81 sequences 71.8 / 75.9; 27 + 8, 6 sequences 66.5 / 59.4;
+// 20 + 250, 1 sequence 59.1 / 61.7; H 128, 26 + 61, 42 sequences 48.2 / 45.1.
+bool attn_decode_supported(int dtype, int Ls, int Lt, int N, int H, int sm_count) {
+  return dtype != FTB_F32 && H % kAttnCols == 0 && H <= kDecMaxH && Ls <= kDecMaxSteps && Lt <= kDecMaxSteps / 2 &&
+         (N + 1) / 2 * (H / kAttnCols) <= sm_count - 4;
+}
+
+// Everything behind the encoder's scan; pre: the decoder's input halves, U: row u of Wp_trg from its recurrent half on.
+int launch_attn_decode(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, const float* pre,
+                       const void* U, int ldu, const float* bias, const void* dec_proj, void* dec, void* out, int Lt, int Ls,
+                       int N, int H, int* status, cudaStream_t stream) {
+  if (dtype == FTB_F16)
+    return attn_decode_t<__half>(enc, enc_proj, src_lens, scores, pre, U, ldu, bias, dec_proj, dec, out, Lt, Ls, N, H, status, stream);
+  return attn_decode_t<__nv_bfloat16>(enc, enc_proj, src_lens, scores, pre, U, ldu, bias, dec_proj, dec, out, Lt, Ls, N, H, status, stream);
 }
 
 // What decoder terms that are not finite make of the vectors in `out` and the states in `dec`.

@@ -172,12 +172,6 @@ __device__ __forceinline__ float group_dot(const float (&a)[kEPL], const float (
   return s;
 }
 
-__device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 
 struct SparseArgs {
   long long heads_total;  // B * heads

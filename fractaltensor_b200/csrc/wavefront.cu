@@ -57,6 +57,10 @@ int pack_grid(const void* i2h, const void* h2h, void* Wp, int H, int dtype, cuda
 int pack_projection(const void* P, void* Pt, int H, int V, int Vp, int dtype, cudaStream_t s);
 int pack_rnn(const void* W, const void* U, void* Wp, int I, int H, int dtype, cudaStream_t s);
 int rnn_attention_max_src_len();
+bool attn_decode_supported(int dtype, int Ls, int Lt, int N, int H, int sm_count);
+int launch_attn_decode(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, const float* pre,
+                       const void* U, int ldu, const float* bias, const void* dec_proj, void* dec, void* out, int Lt, int Ls,
+                       int N, int H, int* status, cudaStream_t stream);
 int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, void* out,
                         int Lt, int Ls, int N, int H, cudaStream_t stream);
 int launch_attn_finish(int dtype, void* dec, const void* dec_proj, const float* scores, const int* src_lens, void* out,
@@ -1296,6 +1300,13 @@ size_t ftb_rnn_attention_scratch_bytes(int Ls, int N, int H, int dtype) {
   return std::min<size_t>(Ls, kMaxPreBytes / step) * step;
 }
 
+size_t ftb_rnn_attention_scratch_bytes_all(int Ls, int Lt, int N, int H, int dtype) {
+  const size_t encoder = ftb_rnn_attention_scratch_bytes(Ls, N, H, dtype);
+  const size_t step = static_cast<size_t>(N > 0 ? N : 0) * (H > 0 ? H : 0) * sizeof(float);
+  if (Lt <= 0 || encoder == 0 || encoder < Ls * step || !attn_decode_supported(dtype, Ls, Lt, N, H, current_sm_count())) return encoder;
+  return encoder + Lt * step;
+}
+
 size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype) {
   return kWorkspaceBytes + ftb_rnn_attention_scratch_bytes(Ls, N, H, dtype);
 }
@@ -1376,16 +1387,35 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
   const size_t pre_step = static_cast<size_t>(N) * H * sizeof(float);
   const int piece = rnn_chain_supported(dtype, H) && scratch != nullptr
                         ? static_cast<int>(std::min<size_t>(Ls, scratch_bytes / pre_step)) : 0;
+  // With room for the decoder's input halves y_t W behind them, those come with the same product, and the rest is one launch.
+  const bool decode = piece == Ls && scratch_bytes / pre_step >= static_cast<size_t>(Ls) + Lt &&
+                      attn_decode_supported(dtype, Ls, Lt, N, H, cl.sm_count);
+  float* pre_trg = static_cast<float*>(scratch) + static_cast<size_t>(Ls) * N * H;
   for (int j = 0; j < Ls && piece > 0; j += piece) {
     const int steps = std::min(piece, Ls - j);
     float* pre = static_cast<float*>(scratch);
     CellLauncher gemm = cl;
     gemm.epi = EPI_STORE_F32;
+    // Tiles of 256 columns where those of 128 would be more than one round of the SMs.
+    const int rows128 = (steps * N + 127) / 128 + (decode ? (Lt * N + 127) / 128 : 0);
+    if (H % 256 == 0 && rows128 * (H / 128) > cl.sm_count) {
+      gemm.bn = 256;
+      if ((rc = make_tmap_2d(&gemm.mapW, Wp_src, dtype, H, K, K, 256, 64))) return rc;
+      if ((rc = make_tmap_2d(&gemm.mapC, Wp_trg, dtype, H, K, K, 256, 64))) return rc;
+    }
     items[0] = blank_item();
     add_seg(items[0], 0, static_cast<int64_t>(j) * N, H, 0);
     items[0].rows = steps * N;
     items[0].out = pre;
+    if (decode) {
+      items.push_back(blank_item());
+      add_seg(items[1], 1, 0, H, 0);
+      items[1].w_map = 1;
+      items[1].rows = Lt * N;
+      items[1].out = pre_trg;
+    }
     rc = gemm.run(items);
+    items.resize(1);
     if (rc) return rc;
     char* enc_j = static_cast<char*>(enc) + static_cast<size_t>(j) * N * H * es;
     rc = launch_rnn_chain(dtype, pre, Wp_src, K, H, bias_src, j > 0 ? enc_j - static_cast<size_t>(N) * H * es : nullptr,
@@ -1408,6 +1438,9 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
   // of a softmax by one number), so the vectors of all steps are known here: they go to their rows of
   // `out`, where the decoder cells read them as recurrent inputs, all cells run as one level, and a
   // term that is not finite is carried to the steps behind it at the end.
+  if (decode)
+    return launch_attn_decode(dtype, enc, enc_proj, src_lens, enc_scores, pre_trg, static_cast<const char*>(Wp_trg) + H * es, K,
+                              bias_trg, dec_proj, dec, out, Lt, Ls, N, H, status, stream);
   rc = launch_attn_vectors(dtype, enc, enc_proj, src_lens, enc_scores, out, Lt, Ls, N, H, stream);
   if (rc) return rc;
   items.clear();

@@ -477,7 +477,7 @@ def rnn_attention(src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc_proj, dec_pr
     out = torch.empty_like(trg)
     scores = torch.empty(Ls, N, dtype=torch.float32, device=src.device)
     # operands of the call's own, not of the workspace, which calls on other streams use at the same time
-    scratch = torch.empty(lib.ftb_rnn_attention_scratch_bytes(Ls, N, H, _dtype_code(src)), dtype=torch.uint8,
+    scratch = torch.empty(lib.ftb_rnn_attention_scratch_bytes_all(Ls, Lt, N, H, _dtype_code(src)), dtype=torch.uint8,
                           device=src.device)
     ws = workspace(src.device)
     opt = lambda t: _ptr(t) if t is not None else None

@@ -311,9 +311,12 @@ int ftb_rnn_pack_weights(const void* W, const void* U, void* Wp, int I, int H, i
  * The product's result lies in the workspace behind the status word while the call runs.
  * ftb_rnn_attention_fwd_scratch takes it in a buffer of its own instead (ftb_rnn_attention_scratch_bytes, 0:
  * none needed; scratch may be NULL), so that a workspace shared by calls on several streams holds the
- * status word only. */
+ * status word only.  With ftb_rnn_attention_scratch_bytes_all of it (which is the other's number where H is not a multiple
+ * of 128, a source has more than 256 positions, a target more than 128, or the batch more sequences than the device holds at once) the decoder's input halves are in
+ * the first product too, and what follows the scan is one launch. */
 size_t ftb_rnn_attention_workspace_bytes(int Ls, int N, int H, int dtype);
 size_t ftb_rnn_attention_scratch_bytes(int Ls, int N, int H, int dtype);
+size_t ftb_rnn_attention_scratch_bytes_all(int Ls, int Lt, int N, int H, int dtype);
 int ftb_rnn_attention_fwd(const void* src, const void* trg, const void* Wp_src, const void* Wp_trg,
                           const float* bias_src, const float* bias_trg, const void* enc_proj, const void* dec_proj,
                           const int* src_lens, void* enc, float* enc_scores, void* dec, void* out, int Ls, int Lt,
