@@ -59,6 +59,8 @@ SIGNATURES = {
     "ftb_projection_pack": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "ftb_lstm_project_softmax": (_i, [_vp, _vp, _vp, ctypes.c_longlong, _i, _i, _i, _vp, _sz, _vp]),
     "ftb_lstm_project_softmax_rows": (_i, [_vp, _vp, _vp, _vp, ctypes.c_longlong, _i, _i, _i, _vp, _sz, _vp]),
+    "ftb_project_softmax_scratch_bytes": (_sz, [ctypes.c_longlong, _i, _i, _i, _i]),
+    "ftb_project_softmax_fwd": (_i, [_vp, _vp, _i, _vp, ctypes.c_longlong, ctypes.c_longlong, _i, _i, _i, _vp, _sz, _vp, _sz, _vp]),
     "ftb_gemm_nt": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, ctypes.POINTER(_i), _vp, _sz, _vp]),
 }
 

@@ -57,6 +57,11 @@ int pack_grid(const void* i2h, const void* h2h, void* Wp, int H, int dtype, cuda
 int pack_projection(const void* P, void* Pt, int H, int V, int Vp, int dtype, cudaStream_t s);
 int pack_rnn(const void* W, const void* U, void* Wp, int I, int H, int dtype, cudaStream_t s);
 int rnn_attention_max_src_len();
+// project.cu
+bool project_twice_supported(int dtype, long long T, int V, int H, bool unpacked);
+size_t project_twice_scratch(long long T, int V);
+int launch_project_twice(int dtype, const void* h, const void* P, bool unpacked, float* probs, long long ld, int T, int V,
+                         int Vp, int H, void* scratch, int* status, cudaStream_t stream);
 bool attn_decode_supported(int dtype, int Ls, int Lt, int N, int H, int sm_count);
 int launch_attn_decode(int dtype, const void* enc, const void* enc_proj, const int* src_lens, float* scores, const float* pre,
                        const void* U, int ldu, const float* bias, const void* dec_proj, void* dec, void* out, int Lt, int Ls,
@@ -1571,6 +1576,30 @@ int ftb_lstm_project_softmax_rows(const void* h, const void* Pt, float* logits, 
                                   int dtype, void* workspace, size_t workspace_bytes, void* stream) {
   if (probs == logits) return FTB_ERR_ARG;
   return project_softmax(h, Pt, logits, probs, T, V, H, dtype, workspace, workspace_bytes, stream);
+}
+
+size_t ftb_project_softmax_scratch_bytes(long long T, int V, int H, int dtype, int unpacked) {
+  if (T <= 0 || T > 0x7fffffffLL || V <= 0 || V > 48 * 1024 || H <= 0 || !project_twice_supported(dtype, T, V, H, unpacked != 0)) return 0;
+  return project_twice_scratch(T, V);
+}
+
+int ftb_project_softmax_fwd(const void* h, const void* P, int unpacked, float* probs, long long ld, long long T, int V, int H,
+                            int dtype, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes,
+                            void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!h || !P || !probs || !scratch || T <= 0 || T > 0x7fffffffLL || V <= 0 || H <= 0 || H % 64 != 0) return FTB_ERR_ARG;
+  if (dtype != FTB_F16 && dtype != FTB_BF16) return FTB_ERR_ARG;
+  if (V > 48 * 1024) return FTB_ERR_ARG;  // what ftb_lstm_project_softmax takes
+  const int Vp = ftb_projection_padded_cols(V);
+  if (ld != V && ld != Vp) return FTB_ERR_ARG;
+  if (!aligned16({h, P, probs, scratch})) return FTB_ERR_ALIGN;
+  const size_t need = ftb_project_softmax_scratch_bytes(T, V, H, dtype, unpacked);
+  if (need == 0) return FTB_ERR_ARG;
+  if (scratch_bytes < need) return FTB_ERR_WORKSPACE;
+  int* status = nullptr;
+  int rc = begin_call(workspace, workspace_bytes, stream, &status);
+  if (rc) return rc;
+  return launch_project_twice(dtype, h, P, unpacked != 0, probs, ld, static_cast<int>(T), V, Vp, H, scratch, status, stream);
 }
 
 // ------------------------------------------------------------------------------

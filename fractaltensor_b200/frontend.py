@@ -137,7 +137,7 @@ def project_softmax(hs, prev_softmax_proj):
     h = h.reshape(-1, H).contiguous()
     if isinstance(hs, torch.Tensor):
         return ops.lstm_project_softmax(h, ops.projection_pack(P), P.shape[1])
-    probs = ops.lstm_project_softmax_rows(h, ops.projection_pack(P), P.shape[1])
+    probs = ops.project_softmax_rows(h, P)
     return FractalTensor(probs, hs.indices, (1, P.shape[1]))
 
 

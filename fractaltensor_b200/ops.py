@@ -534,6 +534,37 @@ def projection_pack(P):
     return Pt
 
 
+def _project_twice(h, P, unpacked, probs, ld, T, V, H):
+    """The probabilities without logits in memory (the product computed twice), where that form takes the call."""
+    if V % 4 != 0:  # never: not worth the call that says so
+        return False
+    n = lib.ftb_project_softmax_scratch_bytes(T, V, H, _dtype_code(h), int(unpacked))
+    if n == 0:
+        return False
+    scratch = torch.empty(n, dtype=torch.uint8, device=h.device)
+    ws = workspace(h.device)
+    with torch.cuda.device(h.device):
+        check(lib.ftb_project_softmax_fwd(_ptr(h), _ptr(P), int(unpacked), _ptr(probs), ld, T, V, H, _dtype_code(h),
+                                          _ptr(scratch), n, _ptr(ws), ws.numel(), _stream()), "ftb_project_softmax_fwd")
+    return True
+
+
+def project_softmax_rows(h, P):
+    """softmax(h . P) per row into a contiguous fp32 [T,V]: h [..., H], P [H,V] as it is where the kernel reads it
+    (V a multiple of 8, 16-byte rows), else packed first."""
+    _req(h, "h")
+    _req(P, "P", h.dtype)
+    H = h.shape[-1]
+    if P.dim() != 2 or P.shape[0] != H or P.device != h.device:
+        raise ValueError("project_softmax_rows: P %s does not match h %s" % (tuple(P.shape), tuple(h.shape)))
+    T, V = h.numel() // H, P.shape[1]
+    if V % 8 == 0 and P.data_ptr() % 16 == 0 and h.data_ptr() % 16 == 0 and 0 < V <= 48 * 1024 and T > 0 and H % 64 == 0:
+        probs = torch.empty(T, V, dtype=torch.float32, device=h.device)
+        if _project_twice(h, P, True, probs, V, T, V, H):
+            return probs
+    return lstm_project_softmax_rows(h, projection_pack(P), V)
+
+
 def lstm_project_softmax(h, Pt, V, out=None):
     """h: [..., H] hidden states (flattened to [T,H]); Pt from projection_pack; V the vocabulary size
     -> fp32 probabilities [T,V] = softmax(h . P) per row (a view of a [T,Vp] buffer)."""
@@ -547,6 +578,8 @@ def lstm_project_softmax(h, Pt, V, out=None):
     if out is None:
         out = torch.empty(T, Vp, dtype=torch.float32, device=h.device)
     _req_like(out, "out", torch.float32, (T, Vp), h)
+    if _project_twice(h, Pt, False, out, Vp, T, int(V), H):
+        return out[:, :V]
     ws = workspace(h.device)
     with torch.cuda.device(h.device):
         check(lib.ftb_lstm_project_softmax(_ptr(h), _ptr(Pt), _ptr(out), T, int(V), H, _dtype_code(h), _ptr(ws),
@@ -566,8 +599,10 @@ def lstm_project_softmax_rows(h, Pt, V):
     T = h.numel() // H
     if tuple(Pt.shape) != (Vp, H) or Pt.device != h.device:
         raise ValueError("lstm_project_softmax: Pt %s does not match h %s and V=%d" % (tuple(Pt.shape), tuple(h.shape), V))
-    logits = torch.empty(T, Vp, dtype=torch.float32, device=h.device)
     probs = torch.empty(T, V, dtype=torch.float32, device=h.device)
+    if _project_twice(h, Pt, False, probs, V, T, V, H):
+        return probs
+    logits = torch.empty(T, Vp, dtype=torch.float32, device=h.device)
     ws = workspace(h.device)
     with torch.cuda.device(h.device):
         check(lib.ftb_lstm_project_softmax_rows(_ptr(h), _ptr(Pt), _ptr(logits), _ptr(probs), T, V, H, _dtype_code(h),

@@ -365,6 +365,15 @@ int ftb_lstm_project_softmax(const void* h, const void* Pt, float* probs, long l
 int ftb_lstm_project_softmax_rows(const void* h, const void* Pt, float* logits, float* probs, long long T, int V, int H,
                                   int dtype, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same probabilities without logits in memory: the product is computed twice, the first time for the maxima and sums of the
+ * rows.  P: the projection [H, V] itself (unpacked 1; V % 8 == 0) or Pt of ftb_projection_pack (unpacked 0); rows of probs `ld`
+ * apart, V, or V rounded up to 128 with zeros behind the V probabilities.  scratch: ftb_project_softmax_scratch_bytes, which is
+ * 0 for what this form does not take (H > 640) and where the other is the faster. */
+size_t ftb_project_softmax_scratch_bytes(long long T, int V, int H, int dtype, int unpacked);
+int ftb_project_softmax_fwd(const void* h, const void* P, int unpacked, float* probs, long long ld, long long T, int V, int H,
+                            int dtype, void* scratch, size_t scratch_bytes, void* workspace, size_t workspace_bytes,
+                            void* stream);
+
 /* Plain GEMM out[M,N] = A[M,K] . Bt[N,K]^T through the cell kernel's main loop
  * (support op; the reference's KeCuteGemm, kaleido/core/device/kernels/cutlass_wmma.h:115-181).
  * 16-bit dtypes: K % 64 == 0, N % 128 == 0.  fp32: K % 64 == 0, N % 64 == 0. */

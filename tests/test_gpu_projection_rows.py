@@ -41,3 +41,80 @@ def test_softmax_of_rows_that_begin_anywhere(ops, rows, width):
         # fp32 sums of up to 60004 terms and an exponential of relative error 2^-22 or so
         assert ((ys.double() - ref).abs() / ref).max().item() <= 1e-4
         assert by[:at_y].eq(7).all() and by[at_y + rows * width:].eq(7).all()
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,V,H", [(1, 8, 64), (127, 248, 128), (129, 256, 192), (257, 264, 512), (300, 2000, 640), (2500, 1000, 256), (700, 10104, 64)])
+def test_product_computed_twice(ops, dt, T, V, H):
+    """Probabilities without logits in memory: from the projection as it is and from its transpose, into rows without gaps and
+    into padded ones, whose padding is zero.  Edges of 256 rows and columns, several row blocks a pair of CTAs."""
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, lib
+    g = torch.Generator(device="cuda").manual_seed(T + V)
+    P = torch.randn(H, V, device="cuda", generator=g).to(dt) * 0.5
+    h = torch.randn(T, H, device="cuda", generator=g).to(dt) * 0.5
+    ref = torch.softmax(h.double() @ P.double(), -1)
+    Pt, Vp, ws = ops.projection_pack(P), lib.ftb_projection_padded_cols(V), ops.workspace(h.device)
+    scratch = torch.full((T * ((V + 255) // 256) * 16,), 255, dtype=torch.uint8, device="cuda")
+    got = []
+    for unpacked, ld in ((1, V), (1, Vp), (0, V), (0, Vp)):
+        if lib.ftb_project_softmax_scratch_bytes(T, V, H, _dtype_code(h), unpacked) == 0:
+            continue
+        probs = torch.full((T, ld), 7.0, device="cuda")
+        check(lib.ftb_project_softmax_fwd(_ptr(h), _ptr(P if unpacked else Pt), unpacked, _ptr(probs), ld, T, V, H, _dtype_code(h),
+                                          _ptr(scratch), scratch.numel(), _ptr(ws), ws.numel(), _stream()), "ftb_project_softmax_fwd")
+        ops.check_status()
+        assert probs[:, V:].eq(0).all()
+        got.append(probs[:, :V])
+    assert len(got) >= 2 and torch.equal(ops.project_softmax_rows(h, P), got[0])
+    for x in got:
+        assert torch.equal(x, got[0])
+        # a logit is H / 16 sums on the tensor cores, each cut off after 2^-23 of a number of up to 32 or so; a probability's
+        # relative error is its logit's error, and two more of the exponential and of the row's sum
+        assert ((x.double() - ref).abs() / ref.clamp_min(1e-20)).max().item() <= (H / 16 + 2) * 2.0 ** -18
+        assert (x.double().sum(-1) - 1).abs().max().item() <= 2e-6
+
+
+def test_packed_operand_of_many_logits(ops):
+    """The transposed operand where the entry points take it: the same numbers as from the projection itself."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    P = torch.randn(64, 10000, device="cuda", generator=g).bfloat16()
+    h = torch.randn(1700, 64, device="cuda", generator=g).bfloat16()
+    a, b, c = ops.project_softmax_rows(h, P), ops.lstm_project_softmax_rows(h, ops.projection_pack(P), 10000), ops.lstm_project_softmax(h, ops.projection_pack(P), 10000)
+    ops.check_status()
+    assert a.is_contiguous() and torch.equal(a, b) and torch.equal(a, c)
+    P4 = P[:, :9996].contiguous()  # rows of probabilities on 16 bytes, rows of the projection not
+    assert (ops.project_softmax_rows(h, P4).double() - torch.softmax(h.double() @ P4.double(), -1)).abs().max().item() <= 1e-5
+
+
+def test_rows_that_are_not_finite(ops):
+    """A row of logits with a NaN or +inf is NaN, the others are untouched; columns of -inf have probability 0 beside finite ones."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    P, h = torch.randn(64, 512, device="cuda", generator=g).half(), torch.randn(300, 64, device="cuda", generator=g).half()
+    clean = ops.project_softmax_rows(h, P)
+    bad = h.clone()
+    bad[7, 3], bad[290, 0] = float("nan"), float("inf")
+    out = ops.project_softmax_rows(bad, P)
+    ops.check_status()
+    rows = torch.isnan(out).any(-1)
+    assert rows[7] and rows[290] and rows.sum().item() == 2
+    assert torch.equal(out[~rows], clean[~rows])
+
+
+def test_projections_behind_one_another(ops):
+    """Both passes are dependent launches: a call reads what the call before wrote, and the scratch of one is the next one's."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    P, h = torch.randn(512, 512, device="cuda", generator=g).half(), torch.randn(1500, 512, device="cuda", generator=g).half()
+
+    def links(between=lambda: None):
+        x = h
+        for _ in range(6):
+            x = ops.project_softmax_rows(x, P)
+            between()
+            x = (x * 400).half()
+            between()
+        return x
+
+    want = links(torch.cuda.synchronize)
+    for _ in range(3):
+        assert torch.equal(links(), want)
+    ops.check_status()
