@@ -9,6 +9,7 @@ FractalTensor views of the reference's Python programs.
 """
 import ctypes
 import threading
+from array import array
 
 import torch
 
@@ -53,12 +54,31 @@ def _req_like(t, name, dtype, shape, ref):
     return t
 
 
+# Plain integers: the declared argument types take them, and an object of ctypes for each is a third of a call's host time.
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else 0
 
 
 def _stream():
-    return ctypes.c_void_p(host.current_stream(-1))
+    return host.current_stream(-1)
+
+
+class _on:
+    """torch.cuda.device(device) for the case that it is the current one already, which costs a look."""
+    __slots__ = ("device", "before")
+
+    def __init__(self, device):
+        self.device = device.index
+
+    def __enter__(self):
+        now = torch.cuda.current_device()
+        self.before = None if self.device is None or self.device == now else now
+        if self.before is not None:
+            torch.cuda.set_device(self.device)
+
+    def __exit__(self, *_):
+        if self.before is not None:
+            torch.cuda.set_device(self.before)
 
 
 def workspace(device, nbytes=0):
@@ -127,7 +147,7 @@ def lstm_pack_weights(W, U, bias=None):
     if bias is not None:
         bias = _req(bias.reshape(D, 4, H).contiguous(), "bias", W.dtype)
         bias_p = torch.empty(D, 4 * H, dtype=torch.float32, device=W.device)
-    with torch.cuda.device(W.device):
+    with _on(W.device):
         check(lib.ftb_lstm_pack_weights(_ptr(W), _ptr(U), _ptr(bias), _ptr(Wp), _ptr(bias_p), D, I, H,
                                         _dtype_code(W), _stream()), "ftb_lstm_pack_weights")
     return Wp, bias_p
@@ -158,7 +178,7 @@ def lstm_stacked(x, Wp, bias_p=None, hs=None, c=None, layers_per_group=0, bn=0, 
     _req_like(hs, "hs", x.dtype, (D, L, N, H), x)
     _req_like(c, "c", torch.float32, (D, N, H), x)
     ws = workspace(x.device, lib.ftb_lstm_stacked_workspace_bytes(D, L, N, H))
-    with torch.cuda.device(x.device), _turn(ws):
+    with _on(x.device), _turn(ws):
         check(lib.ftb_lstm_stacked_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), D, L, N, I, H,
                                        _dtype_code(x),
                                        _tuning(layers_per_group, bn, schedule, skew, pair, fine_deps, resident),
@@ -198,7 +218,7 @@ def lstm_stacked_varlen(x, active_rows, Wp, bias_p=None, hs=None, c=None, layers
     _req_like(c, "c", torch.float32, (D, N, H), x)
     rows = (ctypes.c_int * L)(*active_rows)
     ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L))
-    with torch.cuda.device(x.device), _turn(ws):
+    with _on(x.device), _turn(ws):
         check(lib.ftb_lstm_stacked_varlen_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), rows, D, L, I, H,
                                               _dtype_code(x), _tuning(layers_per_group, bn, schedule, 0, pair, 0),
                                               _ptr(ws), ws.numel(), _stream()), "ftb_lstm_stacked_varlen_fwd")
@@ -227,10 +247,10 @@ def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
     c = torch.empty(D, N, H, dtype=torch.float32, device=x.device)
     out = torch.empty(T, H, dtype=x.dtype, device=x.device)
     ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L))
-    with torch.cuda.device(x.device), _turn(ws):
-        check(lib.ftb_lstm_stacked_ragged_fwd_scratch(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N)(*lens), _ptr(xt),
+    with _on(x.device), _turn(ws):
+        check(lib.ftb_lstm_stacked_ragged_fwd_scratch(_ptr(x), _ptr(Wp), _ptr(bias_p), (ctypes.c_int * N).from_buffer(array("i", lens)), _ptr(xt),
                                                       _ptr(hs), _ptr(c), _ptr(out), D, N, I, H, _dtype_code(x),
-                                                      ctypes.c_void_p(xt.data_ptr() + rows), tables, _ptr(ws),
+                                                      xt.data_ptr() + rows, tables, _ptr(ws),
                                                       ws.numel(), _stream()),
               "ftb_lstm_stacked_ragged_fwd_scratch")
     return out
@@ -258,7 +278,7 @@ def lstm_dilated(x, Wp, dilations, bias_p=None, hs=None, c=None, bn=0, pair=0, s
     _req_like(c, "c", torch.float32, (D, md * N, H), x)
     dil = (ctypes.c_int * D)(*[int(d) for d in dilations])
     ws = workspace(x.device, lib.ftb_lstm_dilated_workspace_bytes(D, L))
-    with torch.cuda.device(x.device), _turn(ws):
+    with _on(x.device), _turn(ws):
         check(lib.ftb_lstm_dilated_fwd(_ptr(x), _ptr(Wp), _ptr(bias_p), _ptr(hs), _ptr(c), dil, D, L, N, H,
                                        _dtype_code(x), _tuning(bn=bn, pair=pair, schedule=schedule), _ptr(ws), ws.numel(),
                                        _stream()), "ftb_lstm_dilated_fwd")
@@ -274,7 +294,7 @@ def grid_pack_weights(i2h, h2h):
     if H2 != 2 * H or tuple(h2h.shape) != (D, H, H):
         raise ValueError("expected i2h [D,2H,H] and h2h [D,H,H]")
     Wp = torch.empty(D, H, 3 * H, dtype=i2h.dtype, device=i2h.device)
-    with torch.cuda.device(i2h.device):
+    with _on(i2h.device):
         for d in range(D):
             check(lib.ftb_grid_pack_weights(_ptr(i2h[d]), _ptr(h2h[d]), _ptr(Wp[d]), H, _dtype_code(i2h), _stream()),
                   "ftb_grid_pack_weights")
@@ -302,7 +322,7 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
     # per level; the tables -> generic persistent kernel; tables and flags -> cluster kernel.
     ws = workspace(X.device, 0 if schedule == 1 else lib.ftb_grid_rnn_workspace_bytes(D, A, B))
     ws_bytes = {1: lib.ftb_workspace_bytes(), 2: lib.ftb_grid_rnn_tables_bytes(D, A, B)}.get(schedule, ws.numel())
-    with torch.cuda.device(X.device), _turn(ws):
+    with _on(X.device), _turn(ws):
         check(lib.ftb_grid_rnn_fwd(_ptr(X), _ptr(Y), _ptr(Wpx), _ptr(Wpy), _ptr(bias_x), _ptr(bias_y), _ptr(hx),
                                    _ptr(hy), D, A, B, N, H, _dtype_code(X), _ptr(ws), ws_bytes, _stream()),
               "ftb_grid_rnn_fwd")
@@ -334,7 +354,7 @@ def b2b_gemm(A, B, C, out=None):
         out = torch.empty(batch, M, P, dtype=A.dtype, device=A.device)
     _req_like(out, "out", A.dtype, (batch, M, P), A)
     ws = workspace(A.device)
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         check(lib.ftb_b2b_gemm(_ptr(A), _ptr(B), _ptr(C), _ptr(out), batch, M, N, K, P, _dtype_code(A), _ptr(ws),
                                ws.numel(), _stream()), "ftb_b2b_gemm")
     return out
@@ -369,7 +389,7 @@ def flash_attention(q, k, v, scale=None, out=None, causal=False, window=None, lo
         out = torch.empty_like(q)
     _req_like(out, "out", q.dtype, q.shape, q)
     ws = workspace(q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if local is not None:
             if causal or window is not None:
                 raise ValueError("flash_attention: local=(left, right) stands alone")
@@ -428,7 +448,7 @@ def sparse_attention(q, k, v, rand_pos, window_size=5, dilation=2, n_global=3, s
         out = torch.empty_like(q)
     _req_like(out, "out", q.dtype, q.shape, q)
     ws = workspace(q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         check(lib.ftb_sparse_attn_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(rand_pos) if R else None, _ptr(out), B, heads,
                                       S, d, int(window_size), int(dilation), int(n_global), R, float(scale),
                                       1 if as_shipped else 0, _dtype_code(q), _ptr(ws), ws.numel(), _stream()),
@@ -444,7 +464,7 @@ def rnn_pack_weights(W, U):
     if tuple(U.shape) != (H, H):
         raise ValueError("expected W [I,H] and U [H,H]")
     Wp = torch.empty(H, I + H, dtype=W.dtype, device=W.device)
-    with torch.cuda.device(W.device):
+    with _on(W.device):
         check(lib.ftb_rnn_pack_weights(_ptr(W), _ptr(U), _ptr(Wp), I, H, _dtype_code(W), _stream()),
               "ftb_rnn_pack_weights")
     return Wp
@@ -481,7 +501,7 @@ def rnn_attention(src, trg, Wp_src, Wp_trg, bias_src, bias_trg, enc_proj, dec_pr
                           device=src.device)
     ws = workspace(src.device)
     opt = lambda t: _ptr(t) if t is not None else None
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         check(lib.ftb_rnn_attention_fwd_scratch(_ptr(src), _ptr(trg), _ptr(Wp_src), _ptr(Wp_trg), opt(bias_src),
                                                 opt(bias_trg), _ptr(enc_proj), _ptr(dec_proj), opt(src_lens), _ptr(enc),
                                                 _ptr(scores), _ptr(dec), _ptr(out), Ls, Lt, N, H, _dtype_code(src),
@@ -502,7 +522,7 @@ def gemm_nt(A, Bt, out=None, bn=0, pair=0):
         out = torch.empty(M, N, dtype=A.dtype, device=A.device)
     _req_like(out, "out", A.dtype, (M, N), A)
     ws = workspace(A.device)
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         check(lib.ftb_gemm_nt(_ptr(A), _ptr(Bt), _ptr(out), M, N, K, _dtype_code(A), _tuning(bn=bn, pair=pair), _ptr(ws), ws.numel(),
                               _stream()), "ftb_gemm_nt")
     return out
@@ -517,7 +537,7 @@ def online_softmax(x, out=None):
         out = torch.empty_like(x)
     _req_like(out, "out", torch.float32, x.shape, x)
     rows, width = x.shape
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.ftb_online_softmax(_ptr(x), _ptr(out), rows, width, _stream()), "ftb_online_softmax")
     return out
 
@@ -529,7 +549,7 @@ def projection_pack(P):
         raise ValueError("projection_pack: expected a 16-bit [H,V] matrix")
     H, V = P.shape
     Pt = torch.empty(lib.ftb_projection_padded_cols(V), H, dtype=P.dtype, device=P.device)
-    with torch.cuda.device(P.device):
+    with _on(P.device):
         check(lib.ftb_projection_pack(_ptr(P), _ptr(Pt), H, V, _dtype_code(P), _stream()), "ftb_projection_pack")
     return Pt
 
@@ -543,7 +563,7 @@ def _project_twice(h, P, unpacked, probs, ld, T, V, H):
         return False
     scratch = torch.empty(n, dtype=torch.uint8, device=h.device)
     ws = workspace(h.device)
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(lib.ftb_project_softmax_fwd(_ptr(h), _ptr(P), int(unpacked), _ptr(probs), ld, T, V, H, _dtype_code(h),
                                           _ptr(scratch), n, _ptr(ws), ws.numel(), _stream()), "ftb_project_softmax_fwd")
     return True
@@ -581,7 +601,7 @@ def lstm_project_softmax(h, Pt, V, out=None):
     if _project_twice(h, Pt, False, out, Vp, T, int(V), H):
         return out[:, :V]
     ws = workspace(h.device)
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(lib.ftb_lstm_project_softmax(_ptr(h), _ptr(Pt), _ptr(out), T, int(V), H, _dtype_code(h), _ptr(ws),
                                            ws.numel(), _stream()), "ftb_lstm_project_softmax")
     return out[:, :V]
@@ -604,7 +624,7 @@ def lstm_project_softmax_rows(h, Pt, V):
         return probs
     logits = torch.empty(T, Vp, dtype=torch.float32, device=h.device)
     ws = workspace(h.device)
-    with torch.cuda.device(h.device):
+    with _on(h.device):
         check(lib.ftb_lstm_project_softmax_rows(_ptr(h), _ptr(Pt), _ptr(logits), _ptr(probs), T, V, H, _dtype_code(h),
                                                 _ptr(ws), ws.numel(), _stream()), "ftb_lstm_project_softmax_rows")
     return probs
@@ -622,7 +642,7 @@ def embedding_gather(table, ids, out=None):
         out = torch.empty(T, H, dtype=table.dtype, device=table.device)
     _req_like(out, "out", table.dtype, (T, H), table)
     ws = workspace(table.device)
-    with torch.cuda.device(table.device):
+    with _on(table.device):
         check(lib.ftb_embedding_gather(_ptr(table), _ptr(ids), _ptr(out), T, V, H, _dtype_code(table), _ptr(ws),
                                        ws.numel(), _stream()), "ftb_embedding_gather")
     return out
