@@ -662,30 +662,37 @@ int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& m
 }
 
 // The form of a call: 1 = CTAs of 256 query rows, 2 = of 128 rows and half of their blocks a slot, 3 = pairs of CTAs (flash_pair.cu),
-// by the estimates of all three in us.  A tile of query rows takes kFixed and kBlock for each block that its longer slot
-// walks, and a pair kEdge for each block that an edge of a mask crosses.  Where there are more tiles than places for
-// them (SMs, pairs of SMs), equal ones go in whole rounds, unequal ones (masks, longest first) about half a round of CTAs beyond
-// their mean, pairs, which take theirs in a balanced order, a tenth.
-// Measured, us, forms 1 / 2 / 3 (* taken): full 16 x 256 8.2 / 7.2* / 7.4, 4 x 512 11.4 / 9.6 / 9.0*, 64 x 512 14.3* / 20.8 / 14.9,
-// 40 x 1024 39.5 / 40.1 / 26.8*, 16 x 2048 35.9 / 43.0 / 33.2*, 20 x 2048 68 / 63 / 45*, 33 x 1280 46.7 / - / 31.5*, 4 x 4096 63 / 37 / 33*,
-// 256 x 2048 490 / 574 / 438*; causal 160 x 256 19.7 / 21.3 / 15.4*, 64 x 512 14.6* / 19.0 / 16.1, 64 x 768 26.7 / 27.8 / 21.8*, 8 x 1024 19.5 /
-// 14.1 / 13.5*, 16 x 2048 37 / 28 / 23.4*, 64 x 2048 82 / 104 / 77*, 16 x 2560 45 / 41 / 32*, 4 x 4096 64 / 39 / 35*; window of 100 32 x 4096 50* /
-// 57 / 54, of 600 8 x 2048 20 / 14.7* / 18.2; keys i-1000..i+500 8 x 4096 34.5* / 40 / 39.5.
-// Between forms 1 and 2 halves that are estimated less than a tenth faster keep the 256 rows: between 0.9 and 1 of the
-// estimate the time is 0.9 to 1.19 of theirs, below it 0.53 to 0.97.
+// by estimates in us.  A tile of query rows takes a fixed time and one for each block that its longer slot walks, and a pair one for
+// each block that an edge of a mask crosses.  Where there are more tiles than places for them (SMs, pairs of SMs), equal ones go
+// in whole rounds, unequal ones (masks, longest first) half a round of CTAs beyond their mean, pairs, which take theirs in a
+// balanced order, a quarter, and no less than the longest and the shortest together.
+// Forms 1 and 2: halves that are estimated less than a tenth faster keep the 256 rows: between 0.9 and 1 of the estimate the
+// time is 0.9 to 1.19 of theirs, below it 0.53 to 0.97.  Form 3 against the one of them: its constants are fitted to 150 calls
+// over the sizes and masks of 1 to 16 x 4 to 16 heads and 256 to 4096 keys; the estimates of the other two, made for full and
+// causal walks, lie a fifth below what short masked walks take, which the factor makes up for.  Of those calls 55 take pairs, which
+// run at 0.95 to 1.6 times the other form's rate; all 150 gain 6.0 % (the best form of each would gain 7.5, a factor of 1.25 6.7; but
+// of 40 other calls one lost 13 % by that: keys i-49..i+184, 54 x 1024, 33.8 / 38.7).
+// Measured, us, forms 1 / 2 / 3 (* taken): full 16 x 256 8.2 / 7.2* / 7.4, 7 x 512 13.0 / 10.4 / 9.5*, 99 x 512 30.4 / 34.3 / 19.3*,
+// 40 x 1024 39.5 / 40.1 / 26.8*, 16 x 2048 35.9 / 43.0 / 33.2*, 20 x 2048 68 / 63 / 45*, 4 x 4096 63 / 37 / 33*, 256 x 2048 490 / 574 /
+// 438*; causal 15 x 256 8.3 / 6.9* / 8.0, 66 x 512 12.8* / 19.7 / 13.9, 36 x 1024 20.4 / 26.7 / 17.4*, 16 x 2048 37 / 28 / 23.4*, 84 x 3328 266 /
+// 294 / 225*; window of 65 77 x 768 24.1* / 29.0 / 28.7, of 1307 42 x 3584 110* / 139 / 111; keys i-751..i+392 42 x 1024 40 / 39 / 29.5*.
 int attention_form(bool masked, int n_bh, int S, int left, int right, int sm_count) {
-  constexpr double kFixed[3] = {4.5, 5.0, 1.9}, kBlock[3] = {1.85, 2.1, 0.83}, kPairCall = 3.6, kPairMasked = 0.9, kEdge = 0.35;
+  constexpr double kFixed = 4.5, kBlock = 1.9;
+  constexpr double kPairCall = 4.6, kPair = 2.25, kPairBlock = 0.83, kPairMasked = 2.7, kPairMaskedBlock = 0.8, kPairEdge = 0.55, kBelow = 1.2;
   double us[3];
   for (int form = 0; form < 3; ++form) {
     const int rows = form == 1 ? 128 : 256, tiles = S / rows;
     double total = 0, longest = 0, shortest = 1e30;
     for (int i = 0; i < tiles; ++i) {
       const int r0 = i * rows;
-      const int lo = masked && left >= 0 && r0 > left ? (r0 - left) >> 7 : 0;
+      const bool begins_late = masked && left >= 0 && r0 > left;
+      const int lo = begins_late ? (r0 - left) >> 7 : 0;
       const int hi = masked && r0 + rows - 1 < S - right ? (r0 + rows - 1 + right) >> 7 : S / 128 - 1;
-      const int blocks = form == 1 ? (hi - lo + 2) / 2 : hi - lo + 1;
-      double t = kFixed[form] + (form == 2 && masked ? kPairMasked : kBlock[form]) * blocks;
-      if (form == 2 && masked) t += kEdge * std::min(blocks, left >= 0 && r0 > left ? 6 : 2);
+      const int blocks = hi - lo + 1;
+      const double t = form == 0   ? kFixed + kBlock * blocks
+                       : form == 1 ? kFixed + kBlock * ((blocks + 1) / 2)
+                       : masked    ? kPairMasked + kPairMaskedBlock * blocks + kPairEdge * std::min(blocks, begins_late ? 6 : 2)
+                                   : kPair + kPairBlock * blocks;
       total += t;
       longest = std::max(longest, t);
       shortest = std::min(shortest, t);
@@ -694,13 +701,12 @@ int attention_form(bool masked, int n_bh, int S, int left, int right, int sm_cou
     if (waves <= 1)
       us[form] = longest;
     else if (masked)
-      us[form] = std::max(longest + shortest, (waves + (form == 2 ? 0.1 : 0.5)) * total / tiles);
+      us[form] = std::max(form == 2 ? longest + shortest : longest, (waves + (form == 2 ? 0.25 : 0.5)) * total / tiles);
     else
       us[form] = std::ceil(waves) * longest;
   }
-  us[2] += kPairCall;
   const int single = us[1] < 0.9 * us[0] ? 1 : 0;
-  return us[2] < us[single] ? 3 : single + 1;
+  return kPairCall + us[2] < kBelow * us[single] ? 3 : single + 1;
 }
 
 }  // namespace
