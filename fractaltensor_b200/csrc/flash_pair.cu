@@ -69,18 +69,7 @@ constexpr uint32_t kTilesBytes = 2 * kTileBytes + (kSlotsK + kSlotsV) * kSlotByt
 constexpr uint32_t kSmemBytes = 232448;
 static_assert(kTilesBytes + sizeof(Control) + 512 <= kSmemBytes, "shared memory budget");
 
-__device__ __forceinline__ void umma_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same without the rows of one CTA of the pair: off0 / off1 = all ones leave the leader's / the peer's rows as they are.
+// umma_ts_pair without the rows of one CTA of the pair: off0 / off1 = all ones leave the leader's / the peer's rows as they are.
 __device__ __forceinline__ void umma_ts_pair_rows(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                                   uint32_t off0, uint32_t off1, uint32_t accumulate) {
   asm volatile(

@@ -8,9 +8,10 @@
 
 namespace ftb {
 
-// csrc/lstm_flow.cu (16-bit): batch slices of nb columns, S of them, G layers beside each other.
+// csrc/lstm_flow.cu (16-bit): batch slices of nb columns, S of them, G layers beside each other, CTAs in pairs or not.
 struct FlowPlan {
   int nb, S, G;
+  bool pair;
   double est_us;
 };
 bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, FlowPlan* plan);

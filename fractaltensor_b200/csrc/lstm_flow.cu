@@ -13,13 +13,18 @@
 //   * weights never move during a sweep over time: a CTA owns 128 packed gate rows (32 units) of one
 //     layer, the recurrent K blocks first in tensor memory, the rest of them and the input blocks in
 //     the tensor memory left, then in shared memory;
+//   * CTAs of neighbouring gate rows run as pairs where that is faster (take_pairs): one MMA over both (.cta_group::2),
+//     each with its own weights and accumulator and half the state's rows, so that a state passes L2 half as often.  The
+//     state's hand-over is ordered by a fence over this CTA's shared memory alone: mbarrier.arrive.release.cluster would
+//     wait for the warp's own stores to the output array too (D8 L100 N64 H512 490 us a call, with the fence 411; single
+//     CTAs 510);
 //   * the batch is cut into slices of NB columns that never meet (UMMA N = NB), each with its own CTAs.
 //     What grows with NB is the state a CTA reads and its gates (20 cycles a column, tanh's 16 a cycle): slices are
 //     as narrow as the device has CTAs for;
 //   * the warps that have stored a step's state read the whole of it back: the chain is one set of warps
 //     with no hand-over but the accumulator's barrier and the operand tile's.  They wait before the
 //     first read for as long as it last took the state to arrive: reads that come too early load the L2
-//     that the state has to pass through (8.5 us a step without the pause, 4.4 with it: D8 H512 N64);
+//     that the state has to pass through (8.5 us a step without the pause, 4.4 with it: D8 H512 N64, single CTAs);
 //   * the layer below is read through TMA behind a flag per cell (a counter of the tiles stored), which
 //     a warp of its own raises: its fences are off the chain, the layers above just run further behind;
 //   * the input half of step t + 1 is issued right after the recurrent half of step t.
@@ -33,7 +38,7 @@
 // Same arithmetic in the same order as the other 16-bit schedules: bit-identical results.
 //
 // Roles: warp 0 MMA issuer, warp 1 TMA producer (input tiles, shared-memory weights), warp 2 publisher,
-// warps 4.. epilogue and state.  Cooperative launch.
+// warps 4.. epilogue and state.  Cooperative launch.  Of a pair the even CTA issues the MMAs.
 //
 // Program: stacked_lstm() (examples/stacked_rnn/stacked_lstm1.py:66-76, stacked_rnn.py:69-79) in place
 // of kaleido/core/device/kernels/lstm/stacked_lstm/region{1,2,3}.h.
@@ -49,28 +54,35 @@ namespace {
 
 using namespace flow;
 
-template <typename T, int NB>
-__global__ void __launch_bounds__(FlowCfg<NB>::kThreads, 1)
+template <typename T, int NB, bool kPair>
+__global__ void __launch_bounds__(FlowCfg<NB, kPair>::kThreads, 1)
 lstm_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapH,
                  const __grid_constant__ CUtensorMap mapW, const FlowArgs a) {
   const int tile = blockIdx.x % a.n_tiles;
   const int slice = (blockIdx.x / a.n_tiles) % a.S;
-  body<T, NB>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S));
+  body<T, NB, kPair>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S));
 }
 
-template <typename T, int NB>
+template <typename T, int NB, bool kPair>
 int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, const FlowArgs& a, uint32_t smem,
            cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  auto kfn = lstm_flow_kernel<T, NB>;
+  auto kfn = lstm_flow_kernel<T, NB, kPair>;
   if (!ensure_dynamic_smem(kfn, kMaxSmem, configured)) return FTB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(std::min(a.G, a.D) * a.S * a.n_tiles);
-  cfg.blockDim = dim3(FlowCfg<NB>::kThreads);
+  cfg.blockDim = dim3(FlowCfg<NB, kPair>::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attrs[1];
+  cudaLaunchAttribute attrs[2];
   int na = 0;
+  if (kPair) {
+    attrs[na].id = cudaLaunchAttributeClusterDimension;
+    attrs[na].val.clusterDim.x = 2;
+    attrs[na].val.clusterDim.y = 1;
+    attrs[na].val.clusterDim.z = 1;
+    ++na;
+  }
   // FTB_NO_COOPERATIVE=1 drops the cooperative attribute (profilers that cannot replay cooperative
   // launches); FTB_REFUSE_COOPERATIVE=1 answers as if the driver had refused the launch (tests of the
   // fallback).
@@ -97,14 +109,28 @@ int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, 
   return FTB_OK;
 }
 
+// Whether the CTAs of a slice run as pairs: half the state for each of them to read, against hand-overs that wait for both.
+// What they read weighs when all of them read much of it together.  Single CTAs / pairs, medians over 24 to 29 of 680 calls
+// (D 1..16, N 1..256, L 16..128), by the bytes of states that the whole grid reads a step, H <= 512:
+//   slices of 16: below 0.7 MB 0.97, 0.7..1.1 MB 0.98, 1.1..1.3 MB 1.00, 1.6..2.2 MB 1.02
+//   slices of 32: below 0.6 MB 0.99, 0.9..1.3 MB 1.00, 1.3..1.6 MB 1.02, 2.1..2.6 MB 1.07, 3.3..4.6 MB 1.10
+//   slices of 64: below 0.4 MB 0.99, 0.6..1 MB 1.01, 1..1.4 MB 1.03, 2.5..3.4 MB 1.06, 4.9..6.4 MB 1.22
+// Above H 512, where a warp of a single CTA takes its rows in two rounds: slices of 16 1.19 to 1.24, of 32 1.31 to 1.34.
+// Slices of 128 are always pairs: H 128 1.20, 256 1.18.  What pairs save in shared memory lets wider slices of wider layers
+// fit: H 832 on 16 sequences (D7 L28 N15 436 -> 205 us), H 704 on 32, H 640 on 64.
+bool take_pairs(int nb, int G, int N, int H) {
+  return nb == 128 || H > 512 || 2e-6 * (H / kUnits) * G * N * H > (nb == 64 ? 1.1 : 1.4);
+}
+
 // Shared memory of a CTA with nb columns: the input tiles it leaves room for (0: does not fit).
-int input_slots(int nb, int I, int H, uint32_t* smem) {
+int input_slots(int nb, bool pair, int I, int H, uint32_t* smem) {
   const int kb_h = H / BK, kb_x = std::max(I, H) / BK, copy_kb = 128 / nb;
   const int in_smem = std::max(0, kb_h + kb_x - (512 - 2 * nb) / 32);
-  const uint32_t block = nb * BK * 2, slot = (kb_x + copy_kb - 1) / copy_kb * copy_kb * block;
+  const uint32_t block = (pair ? nb / 2 : nb) * BK * 2, slot = (kb_x + copy_kb - 1) / copy_kb * copy_kb * block;
   const uint32_t fixed = 1024 + kb_h * block + in_smem * kWBlockBytes;
   if (fixed >= kMaxSmem) return 0;
-  const int slots = std::min<int>(kMaxSlots, (kMaxSmem - fixed) / slot);
+  // (one for pairs: D8 L100 N64 H512 411 us a call, with two 420; D4 L100 N64 H256 on slices of 64 303 / 306)
+  const int slots = std::min<int>(pair ? 1 : kMaxSlots, (kMaxSmem - fixed) / slot);
   *smem = fixed + slots * slot;
   return slots;
 }
@@ -118,19 +144,25 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, 
   const int tiles = H / kUnits;
   bool found = false;
   for (int nb = 16; nb <= 128; nb *= 2) {
-    uint32_t smem = 0;
-    if (input_slots(nb, I, H, &smem) < 1) continue;
     const int S = (N + nb - 1) / nb;
     if (S * tiles > sm_count) continue;
     int G = std::min(D, sm_count / (S * tiles));
     const int sweeps = (D + G - 1) / G;
     G = (D + sweeps - 1) / sweeps;
-    // Measured steps: 1.8 / 2.0 us at 16 columns and H 256 / 512, 2.2 / 2.6 at 32, 3.0 / 4.3 at 64, more with more CTAs
-    // at work; a state of more than eight K blocks is read in two rounds.
-    const double busy = static_cast<double>(S * tiles * G) / sm_count;
-    const double step = 1.2 + nb / 64.0 + nb * H / 16800.0 + (H > 512 ? 0.5 : 0.0) + 0.3 * busy * nb / 64.0;
-    const double us = sweeps * ((L + G - 1) * step + 10.0);
-    if (!found || us < plan->est_us) *plan = {nb, S, G, us};
+    const bool pair = take_pairs(nb, G, N, H);
+    uint32_t smem = 0;
+    if (input_slots(nb, pair, I, H, &smem) < 1) continue;
+    // A step, what a layer above adds to the sweep's fill, the states' share of L2 and the call itself, fitted to 420 calls
+    // on every slice that fits (within 20 %, 5 % in the root mean square).  Behind it a twentieth, for which the kernels
+    // that stream weights keep what is nearly even: they are estimated within 20 % too.
+    const double h = H / 512.0, over = std::max(0.0, h - 1.0);
+    const double step = pair ? (nb == 16   ? 1.28 + 0.45 * h + 0.12 * over
+                                : nb == 32 ? 1.30 + 0.67 * h + 0.10 * over
+                                : nb == 64 ? 1.66 + 0.94 * h + 1.42 * over
+                                           : 2.41 + 1.55 * h)
+                             : (nb == 16 ? 1.21 + 0.51 * h : nb == 32 ? 1.41 + 0.60 * h : 1.78 + 0.87 * h);
+    const double us = 1.05 * (sweeps * ((L + G - 1) * step + 2.8 * (G - 1)) + 2.9e-6 * D * L * N * H + 17.0);
+    if (!found || us < plan->est_us) *plan = {nb, S, G, pair, us};
     found = true;
   }
   return found;
@@ -143,7 +175,8 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
                      cudaStream_t stream) {
   FlowArgs a;
   uint32_t smem = 0;
-  a.n_slots = input_slots(plan.nb, I, H, &smem);
+  const bool pair = plan.pair;
+  a.n_slots = input_slots(plan.nb, pair, I, H, &smem);
   if (a.n_slots < 1) return FTB_ERR_ARG;
   a.D = D; a.L = L; a.N = N; a.I = I; a.H = H; a.G = plan.G; a.S = plan.S;
   a.n_tiles = H / kUnits;
@@ -157,23 +190,29 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   a.nb_below = plan.nb;
   a.flags = flags;
   a.status = status;
-  const uint32_t nb = plan.nb, planes = 128 / plan.nb;
+  const uint32_t nb = plan.nb, held = pair ? nb / 2 : nb, planes = 128 / nb;
   CUtensorMap mX, mH, mW;
   int rc;
-  if ((rc = make_tmap_3d(&mX, x, dtype, 64, T, I / BK, static_cast<uint64_t>(I) * 2, 128, 64, nb, planes))) return rc;
+  if ((rc = make_tmap_3d(&mX, x, dtype, 64, T, I / BK, static_cast<uint64_t>(I) * 2, 128, 64, held, planes))) return rc;
   if ((rc = make_tmap_3d(&mH, hs, dtype, 64, static_cast<uint64_t>(D) * T, H / BK, static_cast<uint64_t>(H) * 2, 128, 64,
-                         nb, planes)))
+                         held, planes)))
     return rc;
   if ((rc = make_tmap_2d(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H, I + H, kGateRows, BK))) return rc;
   if (cudaMemsetAsync(hs, 0xFF, static_cast<size_t>(D) * T * H * 2, stream) != cudaSuccess ||
       cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(D) * L * a.S, stream) != cudaSuccess)
     return FTB_ERR_LAUNCH;
-#define FTB_FLOW_LAUNCH(TT)                                         \
-  switch (plan.nb) {                                                \
-    case 16: return launch<TT, 16>(mX, mH, mW, a, smem, stream);        \
-    case 32: return launch<TT, 32>(mX, mH, mW, a, smem, stream);        \
-    case 64: return launch<TT, 64>(mX, mH, mW, a, smem, stream);        \
-    default: return launch<TT, 128>(mX, mH, mW, a, smem, stream);       \
+#define FTB_FLOW_LAUNCH(TT)                                                                      \
+  switch (plan.nb) {                                                                             \
+    case 16:                                                                                     \
+      return pair ? launch<TT, 16, true>(mX, mH, mW, a, smem, stream)                            \
+                  : launch<TT, 16, false>(mX, mH, mW, a, smem, stream);                          \
+    case 32:                                                                                     \
+      return pair ? launch<TT, 32, true>(mX, mH, mW, a, smem, stream)                            \
+                  : launch<TT, 32, false>(mX, mH, mW, a, smem, stream);                          \
+    case 64:                                                                                     \
+      return pair ? launch<TT, 64, true>(mX, mH, mW, a, smem, stream)                            \
+                  : launch<TT, 64, false>(mX, mH, mW, a, smem, stream);                          \
+    default: return launch<TT, 128, true>(mX, mH, mW, a, smem, stream);                          \
   }
   if (dtype == FTB_F16) {
     FTB_FLOW_LAUNCH(__half)

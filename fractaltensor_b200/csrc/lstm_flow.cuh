@@ -18,14 +18,18 @@ constexpr int kMaxSlots = 2;     // input tiles [NB x I] in shared memory
 constexpr int kMaxPause = 4000;  // cycles
 constexpr uint32_t kMaxSmem = 226 * 1024;
 
-template <int NB>
+template <int NB, bool kPair = false>
 struct FlowCfg {
+  static constexpr int kCtas = kPair ? 2 : 1;              // that share one MMA
+  static constexpr int kHeld = NB / kCtas;                 // rows of a state that a CTA holds
   static constexpr int kWarps = NB == 16 ? 4 : (NB == 32 ? 8 : (NB == 48 ? 12 : 16));  // epilogue warps
   static constexpr int kChunks = NB * 4 / kWarps / 16;         // of 16 columns, of a warp
-  static constexpr int kRows = NB / kWarps;                // state rows a warp reads
+  static constexpr int kRows = kHeld / kWarps;             // state rows a warp reads
+  static constexpr int kSpan = kRows < 4 ? kRows : 4;      // of them at a time,
+  static constexpr int kParts = 4 / kSpan;                 // each by so many groups of eight lanes
   static constexpr int kThreads = 32 * (kFirstEpi + kWarps);
-  static constexpr uint32_t kBlockBytes = NB * BK * 2;     // one K block of a state
-  static constexpr int kCopyKb = 128 / NB;                 // K blocks of one TMA copy (16 KB)
+  static constexpr uint32_t kBlockBytes = kHeld * BK * 2;  // one K block of a state
+  static constexpr int kCopyKb = 128 / NB;                 // K blocks of one TMA copy (16 KB, a pair's CTAs 8 KB each)
   static constexpr int kTmemBlocks = (512 - 2 * NB) / 32;  // weight blocks beside the two accumulators
 };
 
@@ -79,11 +83,12 @@ __device__ __forceinline__ void ld_relaxed_gpu_2x64(const void* p, uint64_t& a, 
 // A word of four hidden states has arrived when its last one is not the fill pattern.
 __device__ __forceinline__ bool arrived(uint64_t w) { return (w >> 48) != 0xFFFFu; }
 
-// One CTA: packed gate rows `tile` of batch slice `slice`, layers j, j + G, ..
-template <typename T, int NB>
+// One CTA: packed gate rows `tile` of batch slice `slice`, layers j, j + G, ..  kPair: two CTAs of a cluster, tiles 2 i
+// and 2 i + 1, share each MMA; each holds the state rows of its half of the slice.
+template <typename T, int NB, bool kPair = false>
 __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapW,
                                      const FlowArgs& a, const int tile, const int slice, const int j) {
-  using C = FlowCfg<NB>;
+  using C = FlowCfg<NB, kPair>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t in_full[kMaxSlots], in_empty[kMaxSlots];
   __shared__ uint64_t st_full;          // the previous step's state is in its operand tile
@@ -113,29 +118,44 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       mbar_init(&in_full[i], 1);
       mbar_init(&in_empty[i], 1);
     }
-    mbar_init(&st_full, C::kWarps);
+    mbar_init(&st_full, C::kCtas * C::kWarps);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], C::kWarps);
+      mbar_init(&acc_empty[i], C::kCtas * C::kWarps);
     }
     n_stored = 0;
-    mbar_init(&w_tmem, C::kWarps);
+    mbar_init(&w_tmem, C::kCtas * C::kWarps);
     mbar_init(&w_smem, 1);
     mbar_init(&swept, 1);
     s_abort = 0;
     fence_barrier_init();
   }
   if (warp == 0) {
-    tmem_alloc(&tmem_base_s, 512);
-    tmem_relinquish();
+    if constexpr (kPair) {
+      tmem_alloc_pair(&tmem_base_s, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&tmem_base_s, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (kPair) cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
   const uint32_t tmem_w = tmem_base + 2 * NB;
 
   const int n_base = slice * NB;
+  // Which CTA of the pair this is.  The even one issues the MMAs, and what they wait for is counted on its barriers.
+  const int rank = kPair ? static_cast<int>(cluster_ctarank()) : 0;
+  const int held_base = n_base + rank * C::kHeld;
+  auto commit = [](uint64_t* bar) {
+    if constexpr (kPair) umma_commit_pair(bar); else umma_commit(bar);
+  };
+  auto arrive_at_issuer = [](uint64_t* bar) {
+    if constexpr (kPair) mbar_arrive_peer(map_to_cta(smem_u32(bar), 0)); else mbar_arrive(bar);
+  };
   const int n_groups = (a.D + a.G - 1) / a.G;
   // Steps this slice takes part in (ragged: until its longest sequence, its first one, ends).
   int steps = a.L;
@@ -147,10 +167,16 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
     }
   }
 
-  if (warp == 0) {
+  if (warp == 0 && rank == 0) {
     // -------------------------------------------------------------- MMA issuer
     const bool leader = elect_one();
-    constexpr uint32_t idesc = make_idesc_f16(kGateRows, NB, Fmt<T>::kind, 0, 0);
+    constexpr uint32_t idesc = make_idesc_f16(C::kCtas * kGateRows, NB, Fmt<T>::kind, 0, 0);
+    auto mma_ts = [](uint32_t d, uint32_t aw, uint64_t bd, uint32_t id, uint32_t accumulate) {
+      if constexpr (kPair) umma_ts_pair(d, aw, bd, id, accumulate); else umma_ts(d, aw, bd, id, accumulate);
+    };
+    auto mma_ss = [](uint32_t d, uint64_t ad, uint64_t bd, uint32_t id, uint32_t accumulate) {
+      if constexpr (kPair) umma_ss_pair(d, ad, bd, id, accumulate); else umma_ss(d, ad, bd, id, accumulate);
+    };
     const uint64_t in_desc = make_sdesc_sw128(smem_u32(s_in), 16, 1024);
     const uint64_t state_desc = make_sdesc_sw128(smem_u32(s_state), 16, 1024);
     const uint64_t w_desc = make_sdesc_sw128(smem_u32(s_w), 16, 1024);
@@ -163,14 +189,14 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         if (leader) {
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            umma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
+            mma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
         }
       }
       if (n & 2) {
         if (leader) {
 #pragma unroll
           for (int i = 0; i < 8; ++i)
-            umma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
+            mma_ts(d_tmem, aw + 8 * i, bd + (i >> 2) * kBlockDesc + 2 * (i & 3), idesc, i > 0 ? 1u : accumulate);
         }
         aw += 2 * 32;
         bd += 2 * kBlockDesc;
@@ -179,7 +205,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (n & 1) {
         if (leader) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) umma_ts(d_tmem, aw + 8 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
+          for (int i = 0; i < 4; ++i) mma_ts(d_tmem, aw + 8 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
         }
       }
     };
@@ -187,7 +213,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       for (; n > 0; --n, ad += kWBlockBytes >> 4, bd += kBlockDesc, accumulate = 1) {
         if (leader) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) umma_ss(d_tmem, ad + 2 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
+          for (int i = 0; i < 4; ++i) mma_ss(d_tmem, ad + 2 * i, bd + 2 * i, idesc, i > 0 ? 1u : accumulate);
         }
       }
     };
@@ -218,10 +244,10 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
                   kb_x - in_t, in_t > 0 ? 1u : 0u);
         // Where there is one input tile it goes back behind the recurrent half, not before it: its next copy would otherwise
         // be under way while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64
-        // sequences: D8 L100 500 us a call, behind it 460).  With two, the copy made room for is the one after the next: before
+        // sequences and single CTAs: D8 L100 500 us a call, behind it 460).  With two, the copy made room for is the one after the next: before
         // the half it is 1 % faster at H 256, and so is this order of slot and commits (D1 L100 N16 H256 156 us, with the
         // slot's step behind the half 158.5; inside a branch on the number of slots 8 % behind).
-        if (early) umma_commit(&in_empty[slot]);
+        if (early) commit(&in_empty[slot]);
         if (++slot == a.n_slots) {
           slot = 0;
           phase ^= 1u;
@@ -233,10 +259,10 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           blocks_ss(d_tmem, w_desc, state_desc + rec_t * kBlockDesc, kb_h - rec_t, 1u);
           ++states;
         }
-        if (leader) umma_commit(&acc_full[acc]);
-        if (late) umma_commit(&in_empty[0]);
+        if (leader) commit(&acc_full[acc]);
+        if (late) commit(&in_empty[0]);
       }
-      if (ok && leader) umma_commit(&swept);
+      if (ok && leader) commit(&swept);
       ++sweep;
     }
   } else if (warp == 1) {
@@ -253,16 +279,20 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (n_rec + n_in > 0) {
         if (sweep > 0) ok = mbar_wait_warp(&swept, (sweep - 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
         if (ok && lane == 0) {
-          mbar_arrive_expect_tx(&w_smem, (n_rec + n_in) * kWBlockBytes);
-          for (int b = 0; b < n_rec + n_in; ++b)
-            tma_load_2d(s_w + b * kWBlockBytes, &mapW, &w_smem, b < n_rec ? a.I + (rec_t + b) * BK : (in_t + b - n_rec) * BK,
-                        l * 4 * a.H + tile * kGateRows);
+          if (rank == 0) mbar_arrive_expect_tx(&w_smem, C::kCtas * (n_rec + n_in) * kWBlockBytes);
+          for (int b = 0; b < n_rec + n_in; ++b) {
+            const int x = b < n_rec ? a.I + (rec_t + b) * BK : (in_t + b - n_rec) * BK, y = l * 4 * a.H + tile * kGateRows;
+            if constexpr (kPair)
+              tma_load_2d_pair(s_w + b * kWBlockBytes, &mapW, map_to_cta(smem_u32(&w_smem), 0), x, y);
+            else
+              tma_load_2d(s_w + b * kWBlockBytes, &mapW, &w_smem, x, y);
+          }
         }
       }
       ++sweep;
       const int copies = (kb_x + C::kCopyKb - 1) / C::kCopyKb;
       for (int t = 0; t < steps && ok; ++t) {
-        const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + n_base;
+        const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + held_base;
         if (l > 0) {
           if (lane == 0) {
             // the layer below may be cut differently: its slices that hold this one's rows
@@ -279,10 +309,15 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         if (!ok) break;
         if (lane == 0) {
           // (K blocks past the last one arrive as zeros and are not multiplied)
-          mbar_arrive_expect_tx(&in_full[slot], copies * C::kCopyKb * C::kBlockBytes);
-          for (int c = 0; c < copies; ++c)
-            tma_load_3d(s_in + slot * slot_bytes + c * C::kCopyKb * C::kBlockBytes, l == 0 ? &mapX : &mapH,
-                        &in_full[slot], 0, static_cast<int>(row), c * C::kCopyKb);
+          if (rank == 0) mbar_arrive_expect_tx(&in_full[slot], C::kCtas * copies * C::kCopyKb * C::kBlockBytes);
+          for (int c = 0; c < copies; ++c) {
+            uint8_t* dst = s_in + slot * slot_bytes + c * C::kCopyKb * C::kBlockBytes;
+            const CUtensorMap* map = l == 0 ? &mapX : &mapH;
+            if constexpr (kPair)
+              tma_load_3d_pair(dst, map, map_to_cta(smem_u32(&in_full[slot]), 0), 0, static_cast<int>(row), c * C::kCopyKb);
+            else
+              tma_load_3d(dst, map, &in_full[slot], 0, static_cast<int>(row), c * C::kCopyKb);
+          }
         }
         if (++slot == a.n_slots) {
           slot = 0;
@@ -337,8 +372,10 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
     // cell state of four sequences from n_own on.
     const int n_own = sub * C::kChunks * 16 + 4 * gate;
     const int n_store = n_own + (ub0 ? 2 : 0) + (ub1 ? 1 : 0);
-    // What this lane reads of a state: chunk `lane & 7` of every K block of rows n_load, n_load + 4, ..
-    const int n_load = w * C::kRows + (lane >> 3);
+    // What this lane reads of a state: chunk `lane & 7` of K blocks `part`, part + kParts, .. of rows n_load, n_load + 4, ..
+    // (counted in the rows that this CTA holds)
+    const int n_load = w * C::kRows + (C::kParts == 1 ? lane >> 3 : (lane >> 3) % C::kSpan);
+    const int part = C::kParts == 1 ? 0 : (lane >> 3) / C::kSpan;
     volatile int* abort_flag = &s_abort;
     int k = 0, sweep = 0, pause = 300;
     bool ok = true;
@@ -368,7 +405,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&w_tmem);
+        if (lane == 0) arrive_at_issuer(&w_tmem);
       }
       float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias_p != nullptr)
@@ -393,7 +430,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        if (lane == 0) arrive_at_issuer(&acc_empty[acc]);
 #pragma unroll
         for (int ch = 0; ch < C::kChunks; ++ch) {
           float v[16];
@@ -430,25 +467,25 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         // The state of this step, for the next: eight K blocks of four rows in flight at a time.
         const bool more = t + 1 < steps;
 #pragma unroll
-        for (int rh = 0; rh < C::kRows; rh += 4) {
+        for (int rh = 0; rh < C::kRows; rh += C::kSpan) {
           const int n = n_load + rh;
-          const bool mine = n_base + n < next.active;
-          const T* src = hs_l + (now.first + n_base + n) * a.H + (lane & 7) * 8;
+          const bool mine = held_base + n < next.active;
+          const T* src = hs_l + (now.first + held_base + n) * a.H + (lane & 7) * 8;
           uint8_t* dst = s_state + n * 128 + (((lane & 7) ^ (n & 7)) << 4);
-          for (int kb0 = 0; kb0 < kb_h && more && ok; kb0 += 8) {
+          for (int kb0 = part; kb0 - part < kb_h && more && ok; kb0 += 8 * C::kParts) {
             uint64_t x[8], y[8];
             uint32_t missing = 0;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               x[i] = y[i] = 0;
-              if (mine && kb0 + i < kb_h) missing |= 1u << i;
+              if (mine && kb0 + i * C::kParts < kb_h) missing |= 1u << i;
             }
             uint64_t t0 = 0;
             for (uint32_t it = 1;; ++it) {
 #pragma unroll
               for (int i = 0; i < 8; ++i)
-                if (missing & (1u << i)) ld_relaxed_gpu_2x64(src + (kb0 + i) * BK, x[i], y[i]);
-              if (it == 1 && rh == 0 && kb0 == 0) {
+                if (missing & (1u << i)) ld_relaxed_gpu_2x64(src + (kb0 + i * C::kParts) * BK, x[i], y[i]);
+              if (it == 1 && rh == 0 && kb0 == part) {
                 // this warp's part of the step is on its way: count it in for the publisher
                 __syncwarp();
                 if (lane == 0) {
@@ -471,12 +508,13 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-              if (kb0 + i < kb_h) *reinterpret_cast<ulonglong2*>(dst + (kb0 + i) * C::kBlockBytes) = make_ulonglong2(x[i], y[i]);
+              if (kb0 + i * C::kParts < kb_h)
+                *reinterpret_cast<ulonglong2*>(dst + (kb0 + i * C::kParts) * C::kBlockBytes) = make_ulonglong2(x[i], y[i]);
           }
         }
         if (more) {
           // Everything in the first round: try a little earlier next time; else later.
-          const bool early = rounds > (C::kRows / 4) * ((kb_h + 7) / 8);
+          const bool early = rounds > (C::kRows / C::kSpan) * ((kb_h + 8 * C::kParts - 1) / (8 * C::kParts));
           pause = early ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
           if (!ok) {
             if (lane == 0 && *abort_flag == 0) {
@@ -487,7 +525,9 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&st_full);
+          if (lane == 0) {
+            if constexpr (kPair) mbar_arrive_peer_smem(map_to_cta(smem_u32(&st_full), 0)); else mbar_arrive(&st_full);
+          }
         } else {
           __syncwarp();
           if (lane == 0) {
@@ -514,6 +554,8 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  // Neither CTA of a pair may leave while the other can still signal its barriers.
+  if constexpr (kPair) cluster_sync_all();
   if (warp == 0) {
     if (s_abort) {
       // Give copies and MMAs still in flight time to land before TMEM and shared memory go back.
@@ -521,7 +563,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    if constexpr (kPair) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
   }
 }
 

@@ -471,10 +471,10 @@ static int fit_groups(int D, int G, int ctas, int sm_count) {
 
 // About what the 16-bit kernels that stream weights take (us), by groups of G layers: sweeps * (L + G - 1) steps of
 // a length fitted to 504 problems (H 128..1024, D 1..16, N 16..256, L 64; within 20 %, 6 % in the root mean
-// square).  Measured, us (generic / static / weights on the M side / everything on chip; * taken): D 8, N 200, H 640 1013*
-// / 1436 / - / 1747; D 12, N 200, H 512 1092* / 1369 / - / 1792; D 16, N 256, H 512 1423 / 1118* / - / 2507; D 4, N 256, H 512
-// 716 / 550* / - / 596; D 12, N 160, H 320 974 / 781 / - / 678*; D 12, N 128, H 512 983 / 1073 / 819* / 943; D 12, N 128, H 128
-// 541 / 506 / 291 / 236*.
+// square).  Measured, us (generic / static / weights on the M side / everything on chip; * taken): D 8, N 200, H 640 928*
+// / 1251 / - / 1339; D 12, N 200, H 512 997* / 1191 / - / 1289; D 16, N 256, H 512 1277 / 1030* / - / 1861; D 4, N 256, H 512
+// 681 / 512 / - / 452*; D 12, N 160, H 320 870 / 665 / - / 628*; D 12, N 128, H 512 925 / 962 / 821 / 681*; D 12, N 128, H 128
+// 509 / 424 / 292 / 232*; D 7, N 15, H 832 1730 / 1327 / 895 / 345*.
 struct StackedEstimate {
   int D, L, N, sm_count, m, n_tiles;
   double h;

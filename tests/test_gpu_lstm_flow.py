@@ -25,7 +25,7 @@ def _params(ops, D, I, H, dt, g):
     (5, 9, 70, 320, 320),    # odd number of K blocks, slices of 32
     (8, 5, 64, 512, 512),    # slices of 64, input weights partly in shared memory
     (12, 6, 30, 640, 640),   # layers in groups: weights replaced between sweeps
-    (2, 5, 8, 768, 768),     # the widest state that fits: two rounds of loads
+    (2, 5, 8, 768, 768),     # a state of more than eight K blocks
     (1, 4, 40, 192, 64),     # input wider than the state
     (16, 4, 256, 64, 64),    # slices of 32 and more at the narrowest state
     (4, 5, 256, 256, 256),
@@ -41,11 +41,27 @@ def test_same_bits_as_levels(ops, dt, D, L, N, I, H):
         assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
 
 
+@pytest.mark.parametrize("D,L,N,H", [
+    (2, 5, 9, 832),      # slices of 16, 8 sequences a CTA: the second CTA's half with one sequence; the widest state
+    (1, 1, 1, 768),      # nothing for the second CTA
+    (3, 6, 17, 576),     # one sequence in the second slice
+    (5, 7, 33, 448),     # slices of 32, odd number of K blocks (zeros in an input copy)
+    (2, 6, 100, 704),    # sixteen K blocks and fewer in one round of loads, weights of half the blocks in shared memory
+    (8, 12, 120, 640),   # slices of 64, three sweeps
+    (12, 5, 232, 384),   # slices of 64, four sweeps
+    (12, 40, 232, 384),  # slices of 128
+    (16, 20, 250, 320),
+])
+def test_pairs_same_bits_as_levels(ops, D, L, N, H):
+    test_same_bits_as_levels(ops, torch.float16, D, L, N, H, H)
+
+
 @pytest.mark.parametrize("D,H,lens", [
     (3, 128, [9, 9, 7, 3, 1] * 5),                  # ends inside a slice
     (2, 256, list(range(1, 41))),                   # every length, slices that end early
     (2, 512, [5] * 16 + [2] * 17),                  # a slice that runs two steps only
     (10, 640, [6, 6, 4, 1]),                        # groups of layers on a ragged batch
+    (2, 640, [9] * 3 + [4] * 30 + [1] * 14),        # pairs: slices whose second CTA's sequences end first
 ])
 def test_ragged_same_bits_as_levels(ops, D, H, lens):
     g = torch.Generator(device="cuda").manual_seed(H + len(lens))
