@@ -1,5 +1,5 @@
-// Stacked LSTM forward with every weight on chip and hidden states that carry their own arrival:
-// the 16-bit path of models whose layer tiles fit on the device (lstm_flow_plan below).
+// Stacked LSTM forward with recurrent weights (and as many others as fit) on chip and hidden states that carry their own
+// arrival: the 16-bit path of models whose layer tiles fit on the device (lstm_flow_plan below).
 //
 // A step of a layer is a chain: recurrent MMAs, gates, hidden state to the layer's other CTAs, next
 // step.  With a flag per tile that chain was 5.5 us at H 512 and 64 sequences: store the tile through
@@ -25,6 +25,11 @@
 //     with no hand-over but the accumulator's barrier and the operand tile's.  They wait before the
 //     first read for as long as it last took the state to arrive: reads that come too early load the L2
 //     that the state has to pass through (8.5 us a step without the pause, 4.4 with it: D8 H512 N64, single CTAs);
+//   * what does not fit of the input weights passes through a ring of shared memory every step (kStream): the input half
+//     is off the chain, and its weights come from L2 while the state is under way.  Against the kernels that keep
+//     no weights (csrc/lstm_wmajor.cu and others), us: D4 L73 N14 H896 561 -> 256, D1 L63 N118 H896 573 -> 249, D9 L72 N19 H1024
+//     1800 -> 1055, D16 L100 N64 H1024 3820 -> 3420.  Rings of 2 / 3 / 4 blocks: the first 267 / 261 / 256, the third
+//     1170 / 1076 / 1055;
 //   * the layer below is read through TMA behind a flag per cell (a counter of the tiles stored), which
 //     a warp of its own raises: its fences are off the chain, the layers above just run further behind;
 //   * the input half of step t + 1 is issued right after the recurrent half of step t.
@@ -37,7 +42,7 @@
 //
 // Same arithmetic in the same order as the other 16-bit schedules: bit-identical results.
 //
-// Roles: warp 0 MMA issuer, warp 1 TMA producer (input tiles, shared-memory weights), warp 2 publisher,
+// Roles: warp 0 MMA issuer, warp 1 TMA producer (input tiles, shared-memory weights), warp 2 publisher, warp 3 the ring,
 // warps 4.. epilogue and state.  Cooperative launch.  Of a pair the even CTA issues the MMAs.
 //
 // Program: stacked_lstm() (examples/stacked_rnn/stacked_lstm1.py:66-76, stacked_rnn.py:69-79) in place
@@ -54,20 +59,20 @@ namespace {
 
 using namespace flow;
 
-template <typename T, int NB, bool kPair>
+template <typename T, int NB, bool kPair, bool kStream>
 __global__ void __launch_bounds__(FlowCfg<NB, kPair>::kThreads, 1)
 lstm_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapH,
                  const __grid_constant__ CUtensorMap mapW, const FlowArgs a) {
   const int tile = blockIdx.x % a.n_tiles;
   const int slice = (blockIdx.x / a.n_tiles) % a.S;
-  body<T, NB, kPair>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S));
+  body<T, NB, kPair, kStream>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S));
 }
 
-template <typename T, int NB, bool kPair>
+template <typename T, int NB, bool kPair, bool kStream = false>
 int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, const FlowArgs& a, uint32_t smem,
            cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  auto kfn = lstm_flow_kernel<T, NB, kPair>;
+  auto kfn = lstm_flow_kernel<T, NB, kPair, kStream>;
   if (!ensure_dynamic_smem(kfn, kMaxSmem, configured)) return FTB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(std::min(a.G, a.D) * a.S * a.n_tiles);
@@ -122,23 +127,35 @@ bool take_pairs(int nb, int G, int N, int H) {
   return nb == 128 || H > 512 || 2e-6 * (H / kUnits) * G * N * H > (nb == 64 ? 1.1 : 1.4);
 }
 
-// Shared memory of a CTA with nb columns: the input tiles it leaves room for (0: does not fit).
-int input_slots(int nb, bool pair, int I, int H, uint32_t* smem) {
-  const int kb_h = H / BK, kb_x = std::max(I, H) / BK, copy_kb = 128 / nb;
-  const int in_smem = std::max(0, kb_h + kb_x - (512 - 2 * nb) / 32);
+// Shared memory of a CTA with nb columns.
+struct Fit {
+  int slots;       // input tiles it leaves room for (0: does not fit)
+  int held, ring;  // weight blocks kept there; blocks of the ring that the others pass through (0: all are kept)
+  int streamed;
+  uint32_t smem;
+};
+Fit fit(int nb, bool pair, int I, int H) {
+  const int kb_h = H / BK, kb_x = std::max(I, H) / BK, copy_kb = 128 / nb, tmem_blocks = (512 - 2 * nb) / 32;
+  const int in_smem = std::max(0, kb_h + kb_x - tmem_blocks);
   const uint32_t block = (pair ? nb / 2 : nb) * BK * 2, slot = (kb_x + copy_kb - 1) / copy_kb * copy_kb * block;
   const uint32_t fixed = 1024 + kb_h * block + in_smem * kWBlockBytes;
-  if (fixed >= kMaxSmem) return 0;
-  // (one for pairs: D8 L100 N64 H512 411 us a call, with two 420; D4 L100 N64 H256 on slices of 64 303 / 306)
-  const int slots = std::min<int>(pair ? 1 : kMaxSlots, (kMaxSmem - fixed) / slot);
-  *smem = fixed + slots * slot;
-  return slots;
+  if (fixed + slot <= kMaxSmem) {
+    // (one for pairs: D8 L100 N64 H512 411 us a call, with two 420; D4 L100 N64 H256 on slices of 64 303 / 306)
+    const int slots = std::min<int>(pair ? 1 : kMaxSlots, (kMaxSmem - fixed) / slot);
+    return {slots, in_smem, 0, 0, fixed + slots * slot};
+  }
+  const uint32_t tiles = 1024 + kb_h * block + slot;
+  if (!pair || tiles >= kMaxSmem) return {};
+  const int room = (kMaxSmem - tiles) / kWBlockBytes, n_rec = std::max(0, kb_h - tmem_blocks);
+  const int ring = std::min(kMaxRing, room - n_rec);
+  if (ring < 2) return {};
+  return {1, room - ring, ring, in_smem - (room - ring), tiles + room * kWBlockBytes};
 }
 
 }  // namespace
 
-// How the kernel would run a problem; est_us: about what that takes.
-bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, FlowPlan* plan) {
+// How the kernel would run a problem; est_us: about what that takes.  stream: input weights may pass through a ring.
+bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, bool stream, FlowPlan* plan) {
   if (dtype != FTB_F16 && dtype != FTB_BF16) return false;
   if (N < 1 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return false;
   const int tiles = H / kUnits;
@@ -150,17 +167,21 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, 
     const int sweeps = (D + G - 1) / G;
     G = (D + sweeps - 1) / sweeps;
     const bool pair = take_pairs(nb, G, N, H);
-    uint32_t smem = 0;
-    if (input_slots(nb, pair, I, H, &smem) < 1) continue;
+    const Fit f = fit(nb, pair, I, H);
+    if (f.slots < 1 || (f.ring > 0 && !stream)) continue;
     // A step, what a layer above adds to the sweep's fill, the states' share of L2 and the call itself, fitted to 420 calls
     // on every slice that fits (within 20 %, 5 % in the root mean square).  Behind it a twentieth, for which the kernels
     // that stream weights keep what is nearly even: they are estimated within 20 % too.
     const double h = H / 512.0, over = std::max(0.0, h - 1.0);
-    const double step = pair ? (nb == 16   ? 1.28 + 0.45 * h + 0.12 * over
-                                : nb == 32 ? 1.30 + 0.67 * h + 0.10 * over
-                                : nb == 64 ? 1.66 + 0.94 * h + 1.42 * over
-                                           : 2.41 + 1.55 * h)
-                             : (nb == 16 ? 1.21 + 0.51 * h : nb == 32 ? 1.41 + 0.60 * h : 1.78 + 0.87 * h);
+    double step = pair ? (nb == 16   ? 1.28 + 0.45 * h + 0.12 * over
+                          : nb == 32 ? 1.30 + 0.67 * h + 0.10 * over
+                          : nb == 64 ? 1.66 + 0.94 * h + 1.42 * over
+                                     : 2.41 + 1.55 * h)
+                       : (nb == 16 ? 1.21 + 0.51 * h : nb == 32 ? 1.41 + 0.60 * h : 1.78 + 0.87 * h);
+    // A block that passes through the ring costs its turn of the MMA warp, and all of them together their bytes from L2
+    // (another 260 calls of H 448..1024, as close).
+    const double mb = 1e-6 * S * tiles * G * f.streamed * kWBlockBytes;
+    if (f.ring > 0) step += nb <= 32 ? 0.10 * f.streamed + 0.019 * mb : nb == 64 ? 0.06 * f.streamed + 0.029 * mb : 0.02 * f.streamed;
     const double us = 1.05 * (sweeps * ((L + G - 1) * step + 2.8 * (G - 1)) + 2.9e-6 * D * L * N * H + 17.0);
     if (!found || us < plan->est_us) *plan = {nb, S, G, pair, us};
     found = true;
@@ -174,10 +195,13 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
                      int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
                      cudaStream_t stream) {
   FlowArgs a;
-  uint32_t smem = 0;
   const bool pair = plan.pair;
-  a.n_slots = input_slots(plan.nb, pair, I, H, &smem);
-  if (a.n_slots < 1) return FTB_ERR_ARG;
+  const Fit f = fit(plan.nb, pair, I, H);
+  if (f.slots < 1) return FTB_ERR_ARG;
+  const uint32_t smem = f.smem;
+  a.n_slots = f.slots;
+  a.held = f.held;
+  a.ring = f.ring;
   a.D = D; a.L = L; a.N = N; a.I = I; a.H = H; a.G = plan.G; a.S = plan.S;
   a.n_tiles = H / kUnits;
   a.T = T;
@@ -201,24 +225,27 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   if (cudaMemsetAsync(hs, 0xFF, static_cast<size_t>(D) * T * H * 2, stream) != cudaSuccess ||
       cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(D) * L * a.S, stream) != cudaSuccess)
     return FTB_ERR_LAUNCH;
-#define FTB_FLOW_LAUNCH(TT)                                                                      \
-  switch (plan.nb) {                                                                             \
-    case 16:                                                                                     \
-      return pair ? launch<TT, 16, true>(mX, mH, mW, a, smem, stream)                            \
-                  : launch<TT, 16, false>(mX, mH, mW, a, smem, stream);                          \
-    case 32:                                                                                     \
-      return pair ? launch<TT, 32, true>(mX, mH, mW, a, smem, stream)                            \
-                  : launch<TT, 32, false>(mX, mH, mW, a, smem, stream);                          \
-    case 64:                                                                                     \
-      return pair ? launch<TT, 64, true>(mX, mH, mW, a, smem, stream)                            \
-                  : launch<TT, 64, false>(mX, mH, mW, a, smem, stream);                          \
-    default: return launch<TT, 128, true>(mX, mH, mW, a, smem, stream);                          \
+#define FTB_FLOW_ARGS mX, mH, mW, a, smem, stream
+#define FTB_FLOW_LAUNCH(TT)                                                                                     \
+  switch (plan.nb) {                                                                                            \
+    case 16:                                                                                                    \
+      if (f.ring > 0) return launch<TT, 16, true, true>(FTB_FLOW_ARGS);                                         \
+      return pair ? launch<TT, 16, true>(FTB_FLOW_ARGS) : launch<TT, 16, false>(FTB_FLOW_ARGS);                 \
+    case 32:                                                                                                    \
+      if (f.ring > 0) return launch<TT, 32, true, true>(FTB_FLOW_ARGS);                                         \
+      return pair ? launch<TT, 32, true>(FTB_FLOW_ARGS) : launch<TT, 32, false>(FTB_FLOW_ARGS);                 \
+    case 64:                                                                                                    \
+      if (f.ring > 0) return launch<TT, 64, true, true>(FTB_FLOW_ARGS);                                         \
+      return pair ? launch<TT, 64, true>(FTB_FLOW_ARGS) : launch<TT, 64, false>(FTB_FLOW_ARGS);                 \
+    default:                                                                                                    \
+      return f.ring > 0 ? launch<TT, 128, true, true>(FTB_FLOW_ARGS) : launch<TT, 128, true>(FTB_FLOW_ARGS);    \
   }
   if (dtype == FTB_F16) {
     FTB_FLOW_LAUNCH(__half)
   }
   FTB_FLOW_LAUNCH(__nv_bfloat16)
 #undef FTB_FLOW_LAUNCH
+#undef FTB_FLOW_ARGS
 }
 
 }  // namespace ftb

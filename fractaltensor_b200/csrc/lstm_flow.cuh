@@ -15,6 +15,7 @@ constexpr int BK = 64;
 constexpr uint32_t kWBlockBytes = kGateRows * BK * 2;
 constexpr int kFirstEpi = 4;
 constexpr int kMaxSlots = 2;     // input tiles [NB x I] in shared memory
+constexpr int kMaxRing = 4;      // input weight blocks on their way through shared memory
 constexpr int kMaxPause = 4000;  // cycles
 constexpr uint32_t kMaxSmem = 226 * 1024;
 
@@ -37,6 +38,7 @@ struct FlowArgs {
   int D, L, N, I, H, G, S;
   int n_tiles;          // 4H / 128
   int n_slots;          // input tiles
+  int held, ring;       // kStream: weight blocks kept in shared memory, blocks of the ring for the others
   int64_t T;            // rows of a layer's output: off[L], or L * N
   const int* off;       // [L + 1] first row of every step (ragged batch), or nullptr: t * N
   const float* bias_p;  // [D, 4H] packed order, or nullptr
@@ -84,8 +86,9 @@ __device__ __forceinline__ void ld_relaxed_gpu_2x64(const void* p, uint64_t& a, 
 __device__ __forceinline__ bool arrived(uint64_t w) { return (w >> 48) != 0xFFFFu; }
 
 // One CTA: packed gate rows `tile` of batch slice `slice`, layers j, j + G, ..  kPair: two CTAs of a cluster, tiles 2 i
-// and 2 i + 1, share each MMA; each holds the state rows of its half of the slice.
-template <typename T, int NB, bool kPair = false>
+// and 2 i + 1, share each MMA; each holds the state rows of its half of the slice.  kStream: the last input weight blocks,
+// which do not fit, pass through a ring every step.
+template <typename T, int NB, bool kPair = false, bool kStream = false>
 __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapW,
                                      const FlowArgs& a, const int tile, const int slice, const int j) {
   using C = FlowCfg<NB, kPair>;
@@ -94,6 +97,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
   __shared__ uint64_t st_full;          // the previous step's state is in its operand tile
   __shared__ uint64_t acc_full[2], acc_empty[2];
   __shared__ uint64_t w_tmem, w_smem;   // the sweep's weights are in place
+  __shared__ uint64_t ring_full[kStream ? kMaxRing : 1], ring_empty[kStream ? kMaxRing : 1];
   __shared__ uint64_t swept;            // every MMA of the sweep is done
   __shared__ uint32_t tmem_base_s;
   __shared__ int n_stored;              // epilogue warps that have stored a step, summed over steps
@@ -109,6 +113,8 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
   uint8_t* s_state = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* s_in = s_state + kb_h * C::kBlockBytes;
   uint8_t* s_w = s_in + a.n_slots * slot_bytes;
+  // Input weight blocks in shared memory, of the kb_x - in_t that tensor memory does not hold.
+  auto kept_in = [&](int n) { return kStream ? min(n, a.held - (kb_h - rec_t)) : n; };
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&mapX);
@@ -123,6 +129,11 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], C::kCtas * C::kWarps);
     }
+    if constexpr (kStream)
+      for (int i = 0; i < kMaxRing; ++i) {
+        mbar_init(&ring_full[i], 1);
+        mbar_init(&ring_empty[i], 1);
+      }
     n_stored = 0;
     mbar_init(&w_tmem, C::kCtas * C::kWarps);
     mbar_init(&w_smem, 1);
@@ -218,15 +229,16 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       }
     };
     int slot = 0, sweep = 0, k = 0, states = 0;  // k: steps started, states: states received
-    uint32_t phase = 0;
+    int rs = 0;
+    uint32_t phase = 0, ring_phase = 0;
     bool ok = true;
     for (int g = 0; g < n_groups && ok; ++g) {
       const int l = g * a.G + j;
       if (l >= a.D) continue;
       const int kb_x = l == 0 ? a.I / BK : kb_h;
-      const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
+      const int in_t = min(C::kTmemBlocks - rec_t, kb_x), in_s = kept_in(kb_x - in_t);
       ok = mbar_wait_warp(&w_tmem, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
-      if (ok && (in_t < kb_x || rec_t < kb_h))
+      if (ok && (in_s > 0 || rec_t < kb_h))
         ok = mbar_wait_warp(&w_smem, sweep & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
       if (!ok) break;
       tc_fence_after();
@@ -241,7 +253,22 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         const uint64_t xd = in_desc + static_cast<uint64_t>((slot * slot_bytes) >> 4);
         blocks_ts(d_tmem, tmem_w + rec_t * 32, xd, in_t, 0u);
         blocks_ss(d_tmem, w_desc + static_cast<uint64_t>(((kb_h - rec_t) * kWBlockBytes) >> 4), xd + in_t * kBlockDesc,
-                  kb_x - in_t, in_t > 0 ? 1u : 0u);
+                  in_s, in_t > 0 ? 1u : 0u);
+        if constexpr (kStream) {
+          const uint64_t ring_desc = w_desc + static_cast<uint64_t>((a.held * kWBlockBytes) >> 4);
+          for (int b = in_t + in_s; b < kb_x; ++b) {
+            ok = mbar_wait_warp(&ring_full[rs], ring_phase, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+            if (!ok) break;
+            tc_fence_after();
+            blocks_ss(d_tmem, ring_desc + static_cast<uint64_t>((rs * kWBlockBytes) >> 4), xd + b * kBlockDesc, 1, b > 0 ? 1u : 0u);
+            if (leader) commit(&ring_empty[rs]);
+            if (++rs == a.ring) {
+              rs = 0;
+              ring_phase ^= 1u;
+            }
+          }
+          if (!ok) break;
+        }
         // Where there is one input tile it goes back behind the recurrent half, not before it: its next copy would otherwise
         // be under way while the warps read the state, through the same L2 and into the same SM (64 KB each at H 512, 64
         // sequences and single CTAs: D8 L100 500 us a call, behind it 460).  With two, the copy made room for is the one after the next: before
@@ -275,7 +302,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (l >= a.D) continue;
       const int kb_x = l == 0 ? a.I / BK : kb_h;
       const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
-      const int n_rec = kb_h - rec_t, n_in = kb_x - in_t;
+      const int n_rec = kb_h - rec_t, n_in = kept_in(kb_x - in_t);
       if (n_rec + n_in > 0) {
         if (sweep > 0) ok = mbar_wait_warp(&swept, (sweep - 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
         if (ok && lane == 0) {
@@ -361,6 +388,35 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         __threadfence();
         red_release_gpu_add(a.flags + (static_cast<int64_t>(l) * a.L + t) * a.S + slice, 1);
       }
+    }
+  } else if (kStream && warp == 3) {
+    // ----------------------------------- TMA: the input weights that are not kept, every step again
+    int rs = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int g = 0; g < n_groups && ok; ++g) {
+      const int l = g * a.G + j;
+      if (l >= a.D) continue;
+      const int kb_x = l == 0 ? a.I / BK : kb_h;
+      const int in_t = min(C::kTmemBlocks - rec_t, kb_x), first = in_t + kept_in(kb_x - in_t);
+      for (int t = 0; t < steps && ok; ++t)
+        for (int b = first; b < kb_x; ++b) {
+          ok = mbar_wait_warp(&ring_empty[rs], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
+          if (!ok) break;
+          if (lane == 0) {
+            if (rank == 0) mbar_arrive_expect_tx(&ring_full[rs], C::kCtas * kWBlockBytes);
+            uint8_t* dst = s_w + (a.held + rs) * kWBlockBytes;
+            const int y = l * 4 * a.H + tile * kGateRows;
+            if constexpr (kPair)
+              tma_load_2d_pair(dst, &mapW, map_to_cta(smem_u32(&ring_full[rs]), 0), b * BK, y);
+            else
+              tma_load_2d(dst, &mapW, &ring_full[rs], b * BK, y);
+          }
+          if (++rs == a.ring) {
+            rs = 0;
+            phase ^= 1u;
+          }
+        }
     }
   } else if (warp >= kFirstEpi && warp < kFirstEpi + C::kWarps) {
     // ------------------------------------------------------- epilogue and state

@@ -598,9 +598,10 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
     const int Gs = layers_per_group > 0 ? G : fit_groups(D, G, 2 * ((N + 255) / 256) * ((4 * H + 255) / 256), cl.sm_count);
     const bool can_static = tune.pair != 1 && (bn == 0 || bn == 256) && !tune.fine_deps &&
                             lstm_static_supported(dtype, D, N, I, H, Gs, cl.sm_count);
-    // Everything on chip: schedule 5, and the automatic choice where that is expected to be faster.
+    // Everything on chip: schedule 5, and the automatic choice where that is expected to be faster (with a part of the
+    // input weights read from L2 every step if need be).
     FlowPlan flow;
-    const bool can_flow = layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, &flow) &&
+    const bool can_flow = layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, schedule != 5, &flow) &&
                           workspace_bytes >= lay.total + flow_flag_bytes(D, L, flow.S);
     if (schedule == 5 && !can_flow) return FTB_ERR_ARG;
     const StackedEstimate est(D, L, N, H, cl.sm_count);
@@ -807,7 +808,7 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
   FlowPlan flow;
   const size_t off_bytes = (sizeof(int) * (L + 1) + 255) & ~static_cast<size_t>(255);
   const bool can_flow = tune.layers_per_group == 0 && tune.pair == 0 && tune.bn == 0 &&
-                        lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, &flow) &&
+                        lstm_flow_plan(dtype, D, L, N, I, H, cl.sm_count, tune.schedule != 5, &flow) &&
                         workspace_bytes >= lay.total + off_bytes + flow_flag_bytes(D, L, flow.S);
   if (tune.schedule == 5 && !can_flow) return FTB_ERR_ARG;
   // the generic schedule takes about 14 us a step and group of layers at any size

@@ -56,6 +56,29 @@ def test_pairs_same_bits_as_levels(ops, D, L, N, H):
     test_same_bits_as_levels(ops, torch.float16, D, L, N, H, H)
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,L,N,H", [
+    (1, 20, 1, 1024),    # slices of 16: nine blocks of sixteen through a ring of four
+    (3, 11, 5, 896),     # five through a ring of four: the ring's turn differs from step to step
+    (9, 16, 19, 1024),   # slices of 32, several sweeps: the ring goes on into the next layer's weights
+    (1, 9, 118, 896),
+    (10, 20, 60, 832),   # slices of 64, two input blocks of thirteen kept
+    (4, 30, 60, 960),    # ring of three
+    (4, 40, 64, 1024),   # ring of two, none kept
+    (4, 20, 256, 512),   # slices of 128
+])
+def test_streamed_input_weights_same_bits_as_levels(ops, dt, D, L, N, H):
+    """The automatic choice at sizes where the estimate is far on this kernel's side: its others read all weights each step."""
+    g = torch.Generator(device="cuda").manual_seed(D * 100 + N)
+    Wp, b = _params(ops, D, H, H, dt, g)
+    x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1, pair=1)
+    for _ in range(3):
+        h, c = ops.lstm_stacked(x, Wp, b)
+        ops.check_status()
+        assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
 @pytest.mark.parametrize("D,H,lens", [
     (3, 128, [9, 9, 7, 3, 1] * 5),                  # ends inside a slice
     (2, 256, list(range(1, 41))),                   # every length, slices that end early
