@@ -14,7 +14,7 @@ struct FlowPlan {
   bool pair;
   double est_us;
 };
-bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, bool stream, FlowPlan* plan);
+bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int sm_count, bool stream, FlowPlan* plan);
 int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* off,
                      int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
                      cudaStream_t stream);

@@ -59,6 +59,17 @@ namespace {
 
 using namespace flow;
 
+// The output array before the sweep, all 0xFFFF, and the counters, all 0.  The sweep's kernel starts beside this one and
+// loads its weights meanwhile: one CTA an SM of 256 threads leaves it room.  Against two memsets before the sweep, us a call:
+// D1 L30 N8 H128 49.5 -> 47.5, D4 L16 N45 H256 53 -> 51.5, D15 L92 N50 H128 247 -> 240, D8 L100 N64 H512 (52 MB) 390 -> 388.
+__global__ void __launch_bounds__(256) flow_fill_kernel(uint4* hs, int64_t n, int* flags, int n_flags) {
+  grid_launch_dependents();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x, first = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const uint32_t ones = 0xFFFFFFFFu;
+  for (int64_t i = first; i < n; i += stride) hs[i] = make_uint4(ones, ones, ones, ones);
+  for (int64_t i = first; i < n_flags; i += stride) flags[i] = 0;
+}
+
 template <typename T, int NB, bool kPair, bool kStream>
 __global__ void __launch_bounds__(FlowCfg<NB, kPair>::kThreads, 1)
 lstm_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapH,
@@ -79,8 +90,12 @@ int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, 
   cfg.blockDim = dim3(FlowCfg<NB, kPair>::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attrs[2];
+  cudaLaunchAttribute attrs[3];
   int na = 0;
+  // beside the fill of the output array
+  attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[na].val.programmaticStreamSerializationAllowed = 1;
+  ++na;
   if (kPair) {
     attrs[na].id = cudaLaunchAttributeClusterDimension;
     attrs[na].val.clusterDim.x = 2;
@@ -115,7 +130,7 @@ int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, 
 }
 
 // Whether the CTAs of a slice run as pairs: half the state for each of them to read, against hand-overs that wait for both.
-// What they read weighs when all of them read much of it together.  Single CTAs / pairs, medians over 24 to 29 of 680 calls
+// What they read weighs when all of them read much of it together (rows: of a step, on average).  Single CTAs / pairs, medians over 24 to 29 of 680 calls
 // (D 1..16, N 1..256, L 16..128), by the bytes of states that the whole grid reads a step, H <= 512:
 //   slices of 16: below 0.7 MB 0.97, 0.7..1.1 MB 0.98, 1.1..1.3 MB 1.00, 1.6..2.2 MB 1.02
 //   slices of 32: below 0.6 MB 0.99, 0.9..1.3 MB 1.00, 1.3..1.6 MB 1.02, 2.1..2.6 MB 1.07, 3.3..4.6 MB 1.10
@@ -123,8 +138,8 @@ int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, 
 // Above H 512, where a warp of a single CTA takes its rows in two rounds: slices of 16 1.19 to 1.24, of 32 1.31 to 1.34.
 // Slices of 128 are always pairs: H 128 1.20, 256 1.18.  What pairs save in shared memory lets wider slices of wider layers
 // fit: H 832 on 16 sequences (D7 L28 N15 436 -> 205 us), H 704 on 32, H 640 on 64.
-bool take_pairs(int nb, int G, int N, int H) {
-  return nb == 128 || H > 512 || 2e-6 * (H / kUnits) * G * N * H > (nb == 64 ? 1.1 : 1.4);
+bool take_pairs(int nb, int G, double rows, int H) {
+  return nb == 128 || H > 512 || 2e-6 * (H / kUnits) * G * rows * H > (nb == 64 ? 1.1 : 1.4);
 }
 
 // Shared memory of a CTA with nb columns.
@@ -144,8 +159,10 @@ Fit fit(int nb, bool pair, int I, int H) {
     const int slots = std::min<int>(pair ? 1 : kMaxSlots, (kMaxSmem - fixed) / slot);
     return {slots, in_smem, 0, 0, fixed + slots * slot};
   }
+  // (not on slices of 128: too little room is left, D14 L86 N113 H576 1293 us, the generic kernel 1202; D4 L64 N256 H512 430, slices of 64
+  // 445)
   const uint32_t tiles = 1024 + kb_h * block + slot;
-  if (!pair || tiles >= kMaxSmem) return {};
+  if (!pair || nb == 128 || tiles >= kMaxSmem) return {};
   const int room = (kMaxSmem - tiles) / kWBlockBytes, n_rec = std::max(0, kb_h - tmem_blocks);
   const int ring = std::min(kMaxRing, room - n_rec);
   if (ring < 2) return {};
@@ -154,8 +171,8 @@ Fit fit(int nb, bool pair, int I, int H) {
 
 }  // namespace
 
-// How the kernel would run a problem; est_us: about what that takes.  stream: input weights may pass through a ring.
-bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, bool stream, FlowPlan* plan) {
+// How the kernel would run a problem of T rows; est_us: about what that takes.  stream: input weights may pass through a ring.
+bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int sm_count, bool stream, FlowPlan* plan) {
   if (dtype != FTB_F16 && dtype != FTB_BF16) return false;
   if (N < 1 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return false;
   const int tiles = H / kUnits;
@@ -166,23 +183,23 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int I, int H, int sm_count, 
     int G = std::min(D, sm_count / (S * tiles));
     const int sweeps = (D + G - 1) / G;
     G = (D + sweeps - 1) / sweeps;
-    const bool pair = take_pairs(nb, G, N, H);
+    const bool pair = take_pairs(nb, G, static_cast<double>(T) / L, H);
     const Fit f = fit(nb, pair, I, H);
     if (f.slots < 1 || (f.ring > 0 && !stream)) continue;
-    // A step, what a layer above adds to the sweep's fill, the states' share of L2 and the call itself, fitted to 420 calls
-    // on every slice that fits (within 20 %, 5 % in the root mean square).  Behind it a twentieth, for which the kernels
-    // that stream weights keep what is nearly even: they are estimated within 20 % too.
+    // A step, what every layer adds to the first's start, a sweep's weights, the states' share of L2 and the call itself, fitted
+    // to 680 calls on every slice that fits (within 20 %, 5 % in the root mean square).  A sweep begins when its CTAs are done
+    // with the one before and the layer below has begun.
     const double h = H / 512.0, over = std::max(0.0, h - 1.0);
-    double step = pair ? (nb == 16   ? 1.28 + 0.45 * h + 0.12 * over
-                          : nb == 32 ? 1.30 + 0.67 * h + 0.10 * over
-                          : nb == 64 ? 1.66 + 0.94 * h + 1.42 * over
-                                     : 2.41 + 1.55 * h)
-                       : (nb == 16 ? 1.21 + 0.51 * h : nb == 32 ? 1.41 + 0.60 * h : 1.78 + 0.87 * h);
-    // A block that passes through the ring costs its turn of the MMA warp, and all of them together their bytes from L2
-    // (another 260 calls of H 448..1024, as close).
+    double step = pair ? (nb == 16   ? 1.56 + 0.08 * h + 0.75 * over
+                          : nb == 32 ? 1.35 + 0.57 * h + 0.30 * over
+                          : nb == 64 ? 1.78 + 0.70 * h + 2.36 * over
+                                     : 2.31 + 1.65 * h)
+                       : (nb == 16 ? 1.17 + 0.53 * h : nb == 32 ? 1.35 + 0.65 * h : 1.67 + 1.04 * h);
+    // A block that passes through the ring costs its turn of the MMA warp, and all of them together their bytes from L2.
     const double mb = 1e-6 * S * tiles * G * f.streamed * kWBlockBytes;
-    if (f.ring > 0) step += nb <= 32 ? 0.10 * f.streamed + 0.019 * mb : nb == 64 ? 0.06 * f.streamed + 0.029 * mb : 0.02 * f.streamed;
-    const double us = 1.05 * (sweeps * ((L + G - 1) * step + 2.8 * (G - 1)) + 2.9e-6 * D * L * N * H + 17.0);
+    if (f.ring > 0) step += nb <= 32 ? 0.083 * f.streamed + 0.026 * mb : 0.015 * f.streamed + 0.036 * mb;
+    const double steps = L * step, start = (G - 1) * (step + 3.1);
+    const double us = 14.0 + (sweeps - 1) * std::max(steps, start) + steps + start + 4.7 * sweeps + 3.3e-6 * D * T * H;
     if (!found || us < plan->est_us) *plan = {nb, S, G, pair, us};
     found = true;
   }
@@ -222,9 +239,12 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
                          held, planes)))
     return rc;
   if ((rc = make_tmap_2d(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H, I + H, kGateRows, BK))) return rc;
-  if (cudaMemsetAsync(hs, 0xFF, static_cast<size_t>(D) * T * H * 2, stream) != cudaSuccess ||
-      cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(D) * L * a.S, stream) != cudaSuccess)
-    return FTB_ERR_LAUNCH;
+  const int64_t chunks = static_cast<int64_t>(D) * T * H / 8;
+  const int n_flags = D * L * a.S;
+  flow_fill_kernel<<<static_cast<int>(std::min<int64_t>(148, (std::max<int64_t>(chunks, n_flags) + 255) / 256)), 256, 0, stream>>>(
+      static_cast<uint4*>(hs), chunks, flags, n_flags);
+  if (cudaGetLastError() != cudaSuccess) return FTB_ERR_LAUNCH;
+  count_launch();
 #define FTB_FLOW_ARGS mX, mH, mW, a, smem, stream
 #define FTB_FLOW_LAUNCH(TT)                                                                                     \
   switch (plan.nb) {                                                                                            \
@@ -237,8 +257,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
     case 64:                                                                                                    \
       if (f.ring > 0) return launch<TT, 64, true, true>(FTB_FLOW_ARGS);                                         \
       return pair ? launch<TT, 64, true>(FTB_FLOW_ARGS) : launch<TT, 64, false>(FTB_FLOW_ARGS);                 \
-    default:                                                                                                    \
-      return f.ring > 0 ? launch<TT, 128, true, true>(FTB_FLOW_ARGS) : launch<TT, 128, true>(FTB_FLOW_ARGS);    \
+    default: return launch<TT, 128, true>(FTB_FLOW_ARGS);                                                       \
   }
   if (dtype == FTB_F16) {
     FTB_FLOW_LAUNCH(__half)

@@ -316,6 +316,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           }
         }
       }
+      if (sweep == 0) grid_dependency_wait();  // weights need not wait for the fill of the output array and the counters
       ++sweep;
       const int copies = (kb_x + C::kCopyKb - 1) / C::kCopyKb;
       for (int t = 0; t < steps && ok; ++t) {
@@ -357,6 +358,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
     volatile int* abort_flag = &s_abort;
     volatile int* stored = &n_stored;
     int want = 0;
+    grid_dependency_wait();
     for (int g = 0; g < n_groups && lane == 0; ++g) {
       const int l = g * a.G + j;
       if (l >= a.D) continue;
@@ -463,6 +465,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         __syncwarp();
         if (lane == 0) arrive_at_issuer(&w_tmem);
       }
+      if (sweep == 1) grid_dependency_wait();
       float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias_p != nullptr)
         bias = __ldg(reinterpret_cast<const float4*>(a.bias_p + static_cast<size_t>(l) * 4 * a.H + tile * kGateRows) + (r_loc >> 2));
