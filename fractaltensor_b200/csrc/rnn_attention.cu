@@ -18,6 +18,8 @@
 // not finite does not cancel: it makes every weight of its step NaN, and in the chain every later step
 // of the sequence.
 //
+// For 16-bit states of up to 512 units attn_decode_kernel does all of this, the product with U and the cells in one launch.
+//
 // Layout: time-major padded batches, row (j, n) of `enc` at (j * N + n) * H.  Sequence n attends to
 // encoder positions j < src_lens[n] (all Ls when src_lens is NULL).  L2-bound row work: len * H encoder
 // elements a sequence in (for the scores by each of its H / 128 CTAs, and once for the sum), Lt * H out; then Lt * H
