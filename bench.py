@@ -360,7 +360,7 @@ def other_configs(ops, dev, pk, cpu):
     ms = timed(lambda: ops.rnn_attention(xs_, ys_, Wps, Wpt, None, None, ep, dp), 10)
     out.append(tensor_entry("attention RNN bf16 H512 N64, 50 source + 50 target steps", ms,
                             2 * Lr * Nr * 2 * (2 * Hr) * Hr, samples_steps_per_s=Nr * 2 * Lr / (ms * 1e-3),
-                            note="one scan kernel over the source, all decoder cells as one level: 50 dependent steps of "
+                            note="one scan kernel over the source, everything behind it one launch: 50 dependent steps of "
                                  "1.5 us; latency-bound, the tensor roofline is quoted for context",
                             cpu_baseline=cpu.get("rnn_attention")))
     del rp, Wps, Wpt, xs_, ys_
