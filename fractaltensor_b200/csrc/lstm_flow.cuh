@@ -572,9 +572,11 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           }
         }
         if (more) {
-          // Everything in the first round: try a little earlier next time; else later.
+          // Everything in the first round: try a little earlier next time; else later.  (Down more slowly on wide slices of pairs,
+          // whose repeats load L2 most: D8 L100 N64 H512 384 -> 378 us, D15 L87 N66 H448 861 -> 847; D1 L100 N16 H256, narrow,
+          // 164 -> 165.)
           const bool early = rounds > (C::kRows / C::kSpan) * ((kb_h + 8 * C::kParts - 1) / (8 * C::kParts));
-          pause = early ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
+          pause = early ? min(pause + 100, kMaxPause) : pause - (pause >> (kPair && NB >= 64 ? 6 : 5));
           if (!ok) {
             if (lane == 0 && *abort_flag == 0) {
               *abort_flag = 1;
