@@ -45,9 +45,26 @@ struct ProjectArgs {
 // Numbers e^x are sums and shares of 2^(x log2 e - r), r a whole number at or above the largest exponent: what is rescaled when r
 // moves, or when sums with different r meet, is multiplied by a power of two.  (A factor e^(m - m') would be a second
 // approximate exponential in the sums beside the one in the numbers they divide, whose mean error then no longer cancels: 5 % more error of the result.)
+// From 2^23 on a whole number can lie further from the largest exponent than 2^x has range, and beyond 2.36e38 the exponent
+// itself is no fp32 number: there the numbers are shares of 2^(x log2 e - r - rest), with what r lacks.  A row with nothing but
+// -inf so far has the lowest finite number as its maximum, and sums of 0.
+constexpr float kWhole = 8388608.f, kPlain = kWhole - 256.f;
+struct Ref {
+  float r, rest;
+};
 __device__ __forceinline__ float exponent_of(float m) { return ceilf(m * kLog2e); }
+__device__ __forceinline__ Ref ref_of(float m) {
+  const float r = fminf(fmaxf(exponent_of(m), -FLT_MAX), FLT_MAX);
+  return {r, fabsf(r) < kWhole ? 0.f : fmaf(m, kLog2e, -r)};
+}
 __device__ __forceinline__ float pow2_whole(float n) {  // 2^n, n <= 0 and whole; 0 below 2^-126
   return __int_as_float((max(__float2int_rz(n), -127) + 127) << 23);
+}
+// Whether sums with references of smaller maxima meet this one's by whole powers of two: their rest is 0, or nothing is left of them.
+__device__ __forceinline__ bool plain(const Ref& to) { return fabsf(to.r) < kPlain; }
+// What a sum with reference `from` is multiplied by where `to`, of a maximum no smaller, takes its place.
+__device__ __forceinline__ float rescale(const Ref& from, const Ref& to) {
+  return plain(to) ? pow2_whole(from.r - to.r) : exp2_fast((from.r - to.r) + (from.rest - to.rest));
 }
 
 template <typename T, bool kStats, bool kUnpacked>
@@ -184,7 +201,7 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
     uint8_t* s_row = s_out + (warp - 4) * 2048;
     const uint32_t empty_bar[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
-    float m = 0.f, inv_d = 0.f, shift = 0.f, least = 0.f;  // second pass: of this thread's row
+    float m = 0.f, inv_d = 0.f, shift = 0.f, rest = 0.f, least = 0.f;  // second pass: of this thread's row
     int before = -1;
     if (!kStats) grid_dependency_wait();
     for (int i = first; i < last; ++i) {
@@ -217,14 +234,25 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             d = fmaf(d, pow2_whole(exponent_of(m) - r), s[0]);
             m = top;
           }
+          if (!plain(ref_of(m))) {  // (rare: once more, one pair after the other)
+            d = 0.f;
+#pragma unroll 1
+            for (int e = 0; e < 2 * a.n_tiles; ++e) {
+              const float2 one = __ldcg(p + static_cast<long long>(e) * a.T);
+              d = fmaf(one.y, rescale(ref_of(one.x), ref_of(m)), d);
+            }
+          }
         }
         inv_d = 1.f / d;
-        shift = -exponent_of(m);
-        least = fmaf(m, kLog2e, shift) + kClamp * kLog2e;
+        const Ref ref = ref_of(m);
+        shift = -ref.r;
+        rest = ref.rest;
+        least = fmaf(m, kLog2e, shift) - rest + kClamp * kLog2e;
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (k >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA))) break;
       tc_fence_after();
       float top = -FLT_MAX, d = 0.f;
+      Ref from = ref_of(top);
 #pragma unroll 1
       for (int ch = 0; ch < 4; ++ch) {
         uint32_t r[32];
@@ -251,19 +279,20 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
 #pragma unroll
             for (int e = 0; e < 4; ++e) mx[e] = fmax3(mx[e], __uint_as_float(r[j + e]), __uint_as_float(r[j + 4 + e]));
           const float now = fmaxf(fmax3(top, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-          const float up = exponent_of(now);
+          const Ref to = ref_of(now);
           float s[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) s[j] = exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -up));
+          for (int j = 0; j < 8; ++j) s[j] = exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -to.r) - to.rest);
 #pragma unroll
-          for (int j = 8; j < 32; ++j) s[j & 7] += exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -up));
-          d = fmaf(d, pow2_whole(exponent_of(top) - up), ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+          for (int j = 8; j < 32; ++j) s[j & 7] += exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -to.r) - to.rest);
+          d = fmaf(d, rescale(from, to), ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+          from = to;
           top = now;
         } else {
           if (c0 >= a.n_store) continue;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            r[j] = c0 + j < a.V ? __float_as_uint(exp2_fast(fmaxf(fmaf(__uint_as_float(r[j]), kLog2e, shift), least)) * inv_d) : 0u;
+            r[j] = c0 + j < a.V ? __float_as_uint(exp2_fast(fmaxf(fmaf(__uint_as_float(r[j]), kLog2e, shift) - rest, least)) * inv_d) : 0u;
           // A lane has a row of 32 numbers; a store covers whole rows: through shared memory, 16 rows at a time, 16-byte pieces
           // exchanged within a row so that neither side meets a bank twice.
 #pragma unroll

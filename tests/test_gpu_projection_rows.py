@@ -87,7 +87,7 @@ def test_packed_operand_of_many_logits(ops):
 
 
 def test_rows_that_are_not_finite(ops):
-    """A row of logits with a NaN or +inf is NaN, the others are untouched; columns of -inf have probability 0 beside finite ones."""
+    """A row of logits with a NaN or +inf is NaN, the others are untouched."""
     g = torch.Generator(device="cuda").manual_seed(5)
     P, h = torch.randn(64, 512, device="cuda", generator=g).half(), torch.randn(300, 64, device="cuda", generator=g).half()
     clean = ops.project_softmax_rows(h, P)
@@ -98,6 +98,90 @@ def test_rows_that_are_not_finite(ops):
     rows = torch.isnan(out).any(-1)
     assert rows[7] and rows[290] and rows.sum().item() == 2
     assert torch.equal(out[~rows], clean[~rows])
+
+
+def _logits_by_value(dt, columns, T):
+    """h [T,64] and P [64,V] whose product is scale(row) * (columns[0] + columns[1] + ..): in fp32 without rounding for these."""
+    P = torch.zeros(64, columns[0].numel(), device="cuda", dtype=dt)
+    for i, c in enumerate(columns):
+        P[i] = c.to(dt)
+    h = torch.zeros(T, 64, device="cuda", dtype=dt)
+    h[:, :len(columns)] = 1
+    h[1::3] *= 0.5
+    return h, P
+
+
+def _softmax_64(h, P, n):
+    x = (h[:, :n, None].double() * P[None, :n].double()).sum(1)
+    x = (x - x.amax(-1, keepdim=True).clamp_min(-3.4028234663852886e38))
+    # (-inf and all that is far below the maximum count nothing in the sum and e^-64 as a number: the row kernel's clamp)
+    return x.clamp_min(-64).exp() / x.exp().sum(-1, keepdim=True)
+
+
+def _three_routes(ops, h, P):
+    """The product twice, from the projection itself and from its transpose, and logits with the row kernel behind them."""
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, lib
+    T, (H, V) = h.shape[0], P.shape
+    Pt, ws, twice, rows = ops.projection_pack(P), ops.workspace(h.device), [], torch.empty(T, lib.ftb_projection_padded_cols(V), device="cuda")
+    for unpacked, ld in ((1, V), (1, rows.shape[1]), (0, V), (0, rows.shape[1])):
+        n = lib.ftb_project_softmax_scratch_bytes(T, V, H, _dtype_code(h), unpacked)
+        if n == 0:
+            continue
+        scratch, out = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.empty(T, ld, device="cuda")
+        check(lib.ftb_project_softmax_fwd(_ptr(h), _ptr(P if unpacked else Pt), unpacked, _ptr(out), ld, T, V, H, _dtype_code(h),
+                                          _ptr(scratch), n, _ptr(ws), ws.numel(), _stream()), "ftb_project_softmax_fwd")
+        twice.append(out[:, :V])
+    check(lib.ftb_lstm_project_softmax(_ptr(h), _ptr(Pt), _ptr(rows), T, V, H, _dtype_code(h), _ptr(ws), ws.numel(), _stream()),
+          "ftb_lstm_project_softmax")
+    ops.check_status()
+    return twice, rows[:, :V]
+
+
+def _check_against_both(got, rows, ref):
+    # exponents of up to 92 in 2^-24 of themselves, 2^-22 of an exponential and of its sum: 1e-5, as for the other sizes here
+    for x in got:
+        assert torch.equal(torch.isinf(x), torch.isinf(rows)) and not torch.isnan(x).any()
+        fin = ~torch.isinf(rows)
+        assert ((x.double() - rows.double()).abs() <= 2e-5 * rows.double())[fin].all()
+        assert ((x.double() - ref).abs() <= 1e-5 * ref)[fin].all() and torch.isinf(ref[~fin]).all()
+
+
+@pytest.mark.parametrize("dt,value", [(torch.float16, float("-inf")), (torch.bfloat16, float("-inf")), (torch.bfloat16, -3.3895313892515355e38),
+                                      (torch.bfloat16, -1e30), (torch.bfloat16, -2e9), (torch.bfloat16, 3.3895313892515355e38), (torch.bfloat16, 1e30),
+                                      (torch.float16, 65504.0)])
+@pytest.mark.parametrize("first,last", [(0, 1), (0, 32), (0, 128), (0, 256), (32, 64), (100, 420), (256, 512), (480, 512), (511, 512), (520, 632), (0, 632)])
+def test_columns_far_from_the_others(ops, dt, value, first, last):
+    """Columns of -inf (a vocabulary's padding words, masked) or of numbers at the end of the range beside ordinary ones: where a
+    chunk of 32 columns, a half of 128, a tile, the short last chunk or all of the row has no other number, too."""
+    g = torch.Generator(device="cuda").manual_seed(last)
+    c = torch.randn(632, device="cuda", generator=g) * 4
+    c[first:last] = value
+    h, P = _logits_by_value(dt, [c], 300)
+    twice, rows = _three_routes(ops, h, P)
+    assert len(twice) == 2
+    _check_against_both(twice, rows, _softmax_64(h, P, 1))
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+def test_exponents_around_two_to_the_23(ops, sign):
+    """Logits a few units apart around 2^23 / log2 e = 5814540, where a maximum's exponent stops being taken as a whole number."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    near = torch.randint(-40, 41, (640,), device="cuda", generator=g).float()
+    near[:256] -= 80  # (a tile on one side)
+    h, P = _logits_by_value(torch.bfloat16, [sign * torch.full((640,), 5799936.0, device="cuda"), sign * torch.full((640,), 14592.0, device="cuda"), near], 300)
+    twice, rows = _three_routes(ops, h, P)
+    # (what log2 e lacks as an fp32 number, 1.3e-8 of it, is common to a row but for the distance of its numbers)
+    _check_against_both(twice, rows, _softmax_64(h, P, 3))
+
+
+def test_masked_words_of_many_logits(ops):
+    """The transposed operand (16 million probabilities and more) and both row strides, with the first words masked."""
+    c = torch.randn(49152, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)) * 4
+    c[:300] = c[40000:] = float("-inf")
+    h, P = _logits_by_value(torch.bfloat16, [c], 330)
+    twice, rows = _three_routes(ops, h, P)
+    assert len(twice) == 4
+    _check_against_both(twice, rows, _softmax_64(h, P, 1))
 
 
 def test_projections_behind_one_another(ops):
