@@ -309,6 +309,7 @@ cell_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
           }
         }
       }
+      if (PAIR && ok) ring_drain(empty_bar, S, stage, phase, &s_abort, status);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer

@@ -236,9 +236,9 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     if (warp == 0) {
       // ------------------------------------------------------------ queries and K tiles
       if (leader) {
-        int slot = 0;
+        int slot = 0, w = 0;
         uint32_t phase = 0;
-        for (int w = 0; ok && unit_of<kMasked>(sh, w, G, cid, u); ++w) {
+        for (; ok && unit_of<kMasked>(sh, w, G, cid, u); ++w) {
           const int b = w & 1;
           ok = mbar_wait(&ctl.q_empty[b], ((w >> 1) & 1) ^ 1u, s_abort, status, FTB_ERR_TIMEOUT_SLOT);
           if (!ok) break;
@@ -262,10 +262,12 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             }
           }
         }
+        if (ok && ring_drain(ctl.k_empty, kSlotsK, slot, phase, s_abort, status))
+          ring_drain(ctl.q_empty, 2, w & 1, (w >> 1) & 1, s_abort, status);
       }
     } else if (warp == 3) {
       // ------------------------------------------------------------ V tiles
-      if (leader)
+      if (leader) {
         for (int w = 0; ok && unit_of<kMasked>(sh, w, G, cid, u); ++w)
           for (int j = 0; j < u.n; ++j, ++n) {
             const int slot = n & 3;
@@ -276,6 +278,8 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             tma_load_2d_pair(sV + slot * kSlotBytes, &mapV, map_to_cta(smem_u32(&ctl.v_full[slot]), 0),
                              static_cast<int>(rank) * 64, u.row_base + (u.blk0 + j) * 128);
           }
+        if (ok) ring_drain(ctl.pv_done, kSlotsV, n & 3, (n >> 2) & 1, s_abort, status);
+      }
     } else if (warp == 1 && rank == 0) {
       // ------------------------------------------------------------ S = Q K^T
       constexpr uint32_t idesc = make_idesc_f16(256, 128, Fmt<T>::kind, 0, 0);

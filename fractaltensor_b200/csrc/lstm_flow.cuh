@@ -353,6 +353,10 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         }
       }
     }
+    // (the input tiles first: with the last sweep's back, `swept` is at most that sweep behind)
+    if constexpr (kPair)
+      if (ok && ring_drain(in_empty, a.n_slots, slot, phase, &s_abort, status))
+        mbar_wait(&swept, (sweep - 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
   } else if (warp == 2) {
     // ----------------------------------- publisher: cell (l, t) can be read through TMA
     volatile int* abort_flag = &s_abort;
@@ -420,6 +424,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           }
         }
     }
+    if (kPair && ok) ring_drain(ring_empty, a.ring, rs, phase, &s_abort, status);
   } else if (warp >= kFirstEpi && warp < kFirstEpi + C::kWarps) {
     // ------------------------------------------------------- epilogue and state
     const int q = warp & 3, w = warp - kFirstEpi, sub = w >> 2;

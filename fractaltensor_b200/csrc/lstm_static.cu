@@ -235,6 +235,7 @@ lstm_static_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
           return true;
         });
       }
+      if (ok) ring_drain(empty_bar, kStages, stage, phase, &s_abort, status);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer

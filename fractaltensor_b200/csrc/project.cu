@@ -154,6 +154,7 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
           ++blocks;
         }
       }
+      if (ok) ring_drain(b_empty, a.stages, stage, phase, &s_abort, status);
     }
   } else if (warp == 1 && rank == 0) {
     const bool leader = elect_one();

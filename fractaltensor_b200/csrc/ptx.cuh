@@ -126,6 +126,22 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, g_status, code));
 }
 
+// Waits until every slot of a ring has been given back; `at`, `phase`: where its next fill would go, and the parity of the fills
+// of this pass.  The producers of a CTA pair do so before they leave: the leader's MMA warp gives slots back to both CTAs by
+// commits, which arrive on their own and which a barrier of the cluster does not wait for, and a CTA's shared memory must not go to
+// the next kernel while one is on its way there.
+__device__ __forceinline__ bool ring_drain(uint64_t* empty, int n, int at, uint32_t phase, volatile int* s_abort, int* g_status) {
+  bool ok = true;
+  for (int i = 0; i < n && ok; ++i) {
+    ok = mbar_wait(&empty[at], phase ^ 1u, s_abort, g_status, FTB_ERR_TIMEOUT_SLOT);
+    if (++at == n) {
+      at = 0;
+      phase ^= 1u;
+    }
+  }
+  return ok;
+}
+
 // ------------------------------------------------- two fp32 numbers to an instruction
 // (each half rounds as the scalar instruction does)
 __device__ __forceinline__ uint64_t dup_f32x2(float x) {

@@ -843,6 +843,10 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       }
     }
     if (warp == kFirstEpiWarp && lane == 0) { ACCT_WRITE(0, 12); }  // accumulator complete
+    // The peers' commits for the last two slots, which no step waits for, have to be in before this CTA leaves (ring_drain, ptx.cuh).
+    if (self_producer && ok && warp == kFirstEpiWarp && lane == 0)
+      for (int i = max(0, n_steps - 3); i <= n_steps - 2 && ok; ++i)
+        ok = mbar_wait(&self_free[i & 1], (i >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
   }
 
   // ------------------------------------------------------------------ teardown
