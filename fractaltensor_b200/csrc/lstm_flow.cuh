@@ -280,7 +280,11 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           phase ^= 1u;
         }
         if (t > 0) {
-          ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
+          // (the other CTA's rows are ordered by an acquire of the cluster's scope, as their release is)
+          if constexpr (kPair)
+            ok = __all_sync(0xffffffffu, mbar_wait_cluster(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP));
+          else
+            ok = mbar_wait_warp(&st_full, states & 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           if (!ok) break;
           blocks_ts(d_tmem, tmem_w, state_desc, rec_t, 1u);
           blocks_ss(d_tmem, w_desc, state_desc + rec_t * kBlockDesc, kb_h - rec_t, 1u);

@@ -474,7 +474,8 @@ __device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // An arrival that hands over shared memory of this CTA: ordered against that alone, not against what the thread has
-// written elsewhere.
+// written elsewhere.  The other side waits with mbar_wait_cluster: releases and acquires order each other only where each one's
+// scope includes the other's thread.
 __device__ __forceinline__ void mbar_arrive_peer_smem(uint32_t cluster_addr) {
   asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");

@@ -1,4 +1,4 @@
-"""Commits that signal the other CTA of a pair (tcgen05.commit with a multicast arrive): a CTA may leave only when every one
+"""What the CTAs of a pair tell each other.  Commits that signal the other CTA of a pair (tcgen05.commit with a multicast arrive): a CTA may leave only when every one
 that is addressed to it has arrived.  A model of who waits for which, with commits that arrive late and in any order: why the
 barriers that hand on data are not enough, and waiting for the last slots of each ring (ring_drain, csrc/ptx.cuh) is."""
 import os
@@ -50,3 +50,13 @@ def test_kernels_wait_for_each_ring(name):
     src = open(os.path.join(b.CSRC, name)).read()
     rings = src.count("ring_drain(") + src.count("mbar_wait(&swept, ")
     assert "umma_commit_pair" in src and rings == KERNELS[name][1]
+
+
+def test_scopes_of_a_state_s_hand_over_include_each_other():
+    """The state of a pair's other CTA is released at the cluster's scope; the wait in front of the MMAs that read it has that
+    scope too (on a device the bits come out right either way: the scopes are a matter of the text)."""
+    flow, ptx = (open(os.path.join(b.CSRC, f)).read() for f in ("lstm_flow.cuh", "ptx.cuh"))
+    assert "mbar_arrive_peer_smem(map_to_cta(smem_u32(&st_full), 0))" in flow and "mbar_wait_cluster(&st_full, " in flow
+    release = ptx[ptx.index("void mbar_arrive_peer_smem"):].split("\n}")[0]
+    acquire = ptx[ptx.index("bool mbar_wait_cluster"):].split("\n}")[0]
+    assert "fence.release" in release and "cta.cluster;" in release and "try_wait.parity.acquire.cluster" in acquire
