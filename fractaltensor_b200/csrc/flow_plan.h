@@ -8,13 +8,16 @@
 
 namespace ftb {
 
-// csrc/lstm_flow.cu (16-bit): batch slices of nb columns, S of them, G layers beside each other, CTAs in pairs or not.
+// csrc/lstm_flow.cu (16-bit): batch slices of nb columns, S of them, G layers beside each other, CTAs in pairs or not, weight
+// blocks of the ring that input weights pass through (0: all are kept).
 struct FlowPlan {
   int nb, S, G;
   bool pair;
+  int ring;
   double est_us;
 };
 bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int sm_count, bool stream, FlowPlan* plan);
+bool lstm_flow_form(int dtype, int D, int N, int I, int H, int sm_count, int nb, bool pair, bool ring, FlowPlan* plan);
 int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* off,
                      int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
                      cudaStream_t stream);

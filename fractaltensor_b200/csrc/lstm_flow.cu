@@ -171,18 +171,40 @@ Fit fit(int nb, bool pair, int I, int H) {
 
 }  // namespace
 
+static bool flow_takes(int dtype, int D, int N, int I, int H) {
+  return (dtype == FTB_F16 || dtype == FTB_BF16) && N >= 1 && H % 64 == 0 && I % 64 == 0 && (D == 1 || I == H);
+}
+
+// Slices of a layer and layers beside each other with slices of nb sequences; false: a layer does not fit on the device.
+static bool flow_grid(int D, int N, int H, int sm_count, int nb, FlowPlan* plan) {
+  const int tiles = H / kUnits;
+  plan->nb = nb;
+  plan->S = (N + nb - 1) / nb;
+  if (plan->S * tiles > sm_count) return false;
+  const int most = std::min(D, sm_count / (plan->S * tiles)), sweeps = (D + most - 1) / most;
+  plan->G = (D + sweeps - 1) / sweeps;
+  return true;
+}
+
+// The kernel with slices, pairs and ring named; false: there is no such form of it.
+bool lstm_flow_form(int dtype, int D, int N, int I, int H, int sm_count, int nb, bool pair, bool ring, FlowPlan* plan) {
+  if (!flow_takes(dtype, D, N, I, H) || !(nb == 16 || nb == 32 || nb == 64 || (nb == 128 && pair))) return false;
+  const Fit f = fit(nb, pair, I, H);
+  plan->pair = pair;
+  plan->ring = f.ring;
+  plan->est_us = 0.0;
+  return f.slots >= 1 && (f.ring > 0) == ring && flow_grid(D, N, H, sm_count, nb, plan);
+}
+
 // How the kernel would run a problem of T rows; est_us: about what that takes.  stream: input weights may pass through a ring.
 bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int sm_count, bool stream, FlowPlan* plan) {
-  if (dtype != FTB_F16 && dtype != FTB_BF16) return false;
-  if (N < 1 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return false;
+  if (!flow_takes(dtype, D, N, I, H)) return false;
   const int tiles = H / kUnits;
   bool found = false;
   for (int nb = 16; nb <= 128; nb *= 2) {
-    const int S = (N + nb - 1) / nb;
-    if (S * tiles > sm_count) continue;
-    int G = std::min(D, sm_count / (S * tiles));
-    const int sweeps = (D + G - 1) / G;
-    G = (D + sweeps - 1) / sweeps;
+    FlowPlan p;
+    if (!flow_grid(D, N, H, sm_count, nb, &p)) continue;
+    const int S = p.S, G = p.G, sweeps = (D + G - 1) / G;
     const bool pair = take_pairs(nb, G, static_cast<double>(T) / L, H);
     const Fit f = fit(nb, pair, I, H);
     if (f.slots < 1 || (f.ring > 0 && !stream)) continue;
@@ -200,7 +222,7 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int
     if (f.ring > 0) step += nb <= 32 ? 0.083 * f.streamed + 0.026 * mb : 0.015 * f.streamed + 0.036 * mb;
     const double steps = L * step, start = (G - 1) * (step + 3.1);
     const double us = 14.0 + (sweeps - 1) * std::max(steps, start) + steps + start + 4.7 * sweeps + 3.3e-6 * D * T * H;
-    if (!found || us < plan->est_us) *plan = {nb, S, G, pair, us};
+    if (!found || us < plan->est_us) *plan = {nb, S, G, pair, f.ring, us};
     found = true;
   }
   return found;

@@ -494,6 +494,63 @@ struct StackedEstimate {
   double generic(int G) const { return steps(G) * (11.9 + 1.2 * h + 0.23 * m * G); }
 };
 
+// Layers whose packed weights stay within about half of L2.
+static int l2_group(int D, int H, int K, size_t es) {
+  int dev = 0, l2 = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+  const double per_layer = 4.0 * H * K * es;
+  if (per_layer * D <= 0.55 * l2) return D;
+  return std::max(1, std::min(static_cast<int>((0.55 * l2) / per_layer), D));
+}
+
+// What a 16-bit stacked call may run, and what it takes of that when no schedule is named.
+struct StackedChoice {
+  int Gw, Gs;  // layers per group
+  bool can_wmajor, can_static, take_static, can_flow, on_chip;
+  FlowPlan flow;
+};
+static StackedChoice stacked_choice(int dtype, int D, int L, int N, int I, int H, int G, const Tuning& tune, int sm_count) {
+  StackedChoice ch;
+  // Static tile ownership (schedule 3, and the automatic choice when it applies): CTA pairs
+  // keep their slice of a layer, cell state in registers, for a whole sweep over time.
+  // Weights-major static ownership (schedule 4, and the automatic choice for batches of at most
+  // 128 sequences): the batch is the N side of the MMA, so a small batch wastes no tensor work.
+  const int pair_ctas = 2 * ((N + 255) / 256) * ((4 * H + 255) / 256);
+  ch.Gw = tune.layers_per_group > 0 ? G : fit_groups(D, G, 4 * H / 128, sm_count);
+  ch.can_wmajor = lstm_wmajor_supported(dtype, D, N, I, H, ch.Gw, sm_count);
+  ch.Gs = tune.layers_per_group > 0 ? G : fit_groups(D, G, pair_ctas, sm_count);
+  ch.can_static = tune.pair != 1 && (tune.bn == 0 || tune.bn == 256) && !tune.fine_deps &&
+                  lstm_static_supported(dtype, D, N, I, H, ch.Gs, sm_count);
+  // Everything on chip: schedule 5, and the automatic choice where that is expected to be faster (with a part of the
+  // input weights read from L2 every step if need be).
+  ch.can_flow = tune.layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, static_cast<int64_t>(L) * N, I, H, sm_count,
+                                                             tune.schedule != 5, &ch.flow);
+  const StackedEstimate est(D, L, N, H, sm_count);
+  const double wmajor_us = est.wmajor(ch.Gw), static_us = est.static_pairs(ch.Gs), generic_us = est.generic(G);
+  // Groups that had to be cut to what fits on the device, for static ownership, are more sweeps than those of the
+  // generic kernel, which takes groups of any size.
+  ch.take_static = ch.can_static && (pair_ctas * G <= sm_count || static_us < 1.03 * generic_us);
+  const double old_us = ch.can_wmajor ? wmajor_us : (ch.take_static ? static_us : generic_us);
+  // The kernel with weights on chip has to come out a twentieth faster but for 8 us: the others are estimated less closely,
+  // small calls of theirs a little low (D13 L45 N154 H704 estimated 1518 / generic 1568 us, measured 1627 / 1411; D14 L27 N2
+  // H128 estimated 111 / weights on the M side 112, measured 104 / 118).
+  ch.on_chip = ch.can_flow && ch.flow.est_us < 0.95 * old_us + 8.0;
+  return ch;
+}
+
+int ftb_lstm_stacked_form(int D, int L, int N, int I, int H, int dtype, int* form) {
+  if (!form || D <= 0 || L <= 0 || N <= 0 || H <= 0 || I <= 0 || H % 64 != 0 || I % 64 != 0 || (D > 1 && I != H)) return FTB_ERR_ARG;
+  if (dtype != FTB_F16 && dtype != FTB_BF16) return FTB_ERR_ARG;
+  const StackedChoice ch = stacked_choice(dtype, D, L, N, I, H, l2_group(D, H, I + H, dtype_size(dtype)), Tuning(nullptr),
+                                          current_sm_count());
+  form[0] = ch.on_chip ? 5 : (ch.can_wmajor ? 4 : (ch.take_static ? 3 : 2));
+  form[1] = ch.on_chip ? ch.flow.nb : 0;
+  form[2] = ch.on_chip ? (ch.flow.pair ? 2 : 1) : 0;
+  form[3] = ch.on_chip ? ch.flow.ring : 0;
+  return FTB_OK;
+}
+
 int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, int D, int L,
                          int N, int I, int H, int dtype, const int* tuning, void* workspace, size_t workspace_bytes,
                          void* stream_) {
@@ -543,18 +600,7 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
     if (rc) return rc;
   }
 
-  int G = layers_per_group;
-  if (G <= 0) {
-    // Keep a group's packed weights within about half of L2.
-    int dev = 0, l2 = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-    const double per_layer = 4.0 * H * K * es;
-    G = static_cast<int>((0.55 * l2) / per_layer);
-    G = std::max(1, std::min(G, D));
-    if (per_layer * D <= 0.55 * l2) G = D;
-  }
-  G = std::min(G, D);
+  const int G = layers_per_group > 0 ? std::min(layers_per_group, D) : l2_group(D, H, K, es);
 
   const int n_cells = D * L;
   const PlanLayout lay = plan_layout(n_cells, stacked_max_tiles_per_cell(N, H));
@@ -588,41 +634,17 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
   if (persistent) {
     if (workspace_bytes < lay.total) return FTB_ERR_WORKSPACE;
     char* ws = static_cast<char*>(workspace);
-    // Static tile ownership (schedule 3, and the automatic choice when it applies): CTA pairs
-    // keep their slice of a layer, cell state in registers, for a whole sweep over time.
-    // Weights-major static ownership (schedule 4, and the automatic choice for batches of at most
-    // 128 sequences): the batch is the N side of the MMA, so a small batch wastes no tensor work.
-    const int tiles = 4 * H / 128;
-    const int Gw = layers_per_group > 0 ? G : fit_groups(D, G, tiles, cl.sm_count);
-    const bool can_wmajor = lstm_wmajor_supported(dtype, D, N, I, H, Gw, cl.sm_count);
-    const int Gs = layers_per_group > 0 ? G : fit_groups(D, G, 2 * ((N + 255) / 256) * ((4 * H + 255) / 256), cl.sm_count);
-    const bool can_static = tune.pair != 1 && (bn == 0 || bn == 256) && !tune.fine_deps &&
-                            lstm_static_supported(dtype, D, N, I, H, Gs, cl.sm_count);
-    // Everything on chip: schedule 5, and the automatic choice where that is expected to be faster (with a part of the
-    // input weights read from L2 every step if need be).
-    FlowPlan flow;
-    const bool can_flow = layers_per_group == 0 && lstm_flow_plan(dtype, D, L, N, static_cast<int64_t>(L) * N, I, H, cl.sm_count, schedule != 5, &flow) &&
-                          workspace_bytes >= lay.total + flow_flag_bytes(D, L, flow.S);
+    const StackedChoice ch = stacked_choice(dtype, D, L, N, I, H, G, tune, cl.sm_count);
+    const bool can_flow = ch.can_flow && workspace_bytes >= lay.total + flow_flag_bytes(D, L, ch.flow.S);
     if (schedule == 5 && !can_flow) return FTB_ERR_ARG;
-    const StackedEstimate est(D, L, N, H, cl.sm_count);
-    const double wmajor_us = est.wmajor(Gw), static_us = est.static_pairs(Gs), generic_us = est.generic(G);
-    // Groups that had to be cut to what fits on the device, for static ownership, are more sweeps than those of the
-    // generic kernel, which takes groups of any size.
-    const bool cut = 2 * ((N + 255) / 256) * ((4 * H + 255) / 256) * G > cl.sm_count;
-    const bool take_static = can_static && (!cut || static_us < 1.03 * generic_us);
-    const double old_us = can_wmajor ? wmajor_us : (take_static ? static_us : generic_us);
-    // The kernel with weights on chip has to come out a twentieth faster but for 8 us: the others are estimated less closely,
-    // small calls of theirs a little low (D13 L45 N154 H704 estimated 1518 / generic 1568 us, measured 1627 / 1411; D14 L27 N2
-    // H128 estimated 111 / weights on the M side 112, measured 104 / 118).
-    const bool on_chip = can_flow && flow.est_us < 0.95 * old_us + 8.0;
-    if (schedule == 5 || (schedule == 0 && on_chip && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
-      rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, nullptr, static_cast<int64_t>(L) * N, D, L, N, I, H, flow,
+    if (schedule == 5 || (schedule == 0 && can_flow && ch.on_chip && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
+      rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, nullptr, static_cast<int64_t>(L) * N, D, L, N, I, H, ch.flow,
                             reinterpret_cast<int*>(ws + lay.total), status, stream);
       if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
       goto level_schedule;
     }
-    if (schedule == 4 && !can_wmajor) return FTB_ERR_ARG;
-    if (schedule == 4 || (schedule == 0 && can_wmajor && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
+    if (schedule == 4 && !ch.can_wmajor) return FTB_ERR_ARG;
+    if (schedule == 4 || (schedule == 0 && ch.can_wmajor && tune.pair == 0 && bn == 0 && !tune.fine_deps)) {
       // tuning[6]: 0 = as many recurrent weight blocks on chip as fit, -1 = none, n = n blocks
       const int resident = tune.resident == 0 ? -1 : (tune.resident < 0 ? 0 : tune.resident);
       unsigned long long* trace = nullptr;
@@ -630,18 +652,18 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
       trace = reinterpret_cast<unsigned long long*>(ws + lay.trace);
 #endif
       // one flag per (cell, tile), in the per-tile counter area (at least 4H/128 ints per cell)
-      rc = launch_lstm_wmajor(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, Gw, resident,
+      rc = launch_lstm_wmajor(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, ch.Gw, resident,
                               reinterpret_cast<int*>(ws + lay.tile_done), status, trace, stream);
       if (rc != FTB_ERR_LAUNCH || schedule != 0) return rc;
       goto level_schedule;
     }
-    if (schedule == 3 && !can_static) return FTB_ERR_ARG;
-    if (schedule == 3 || (schedule == 0 && take_static)) {
+    if (schedule == 3 && !ch.can_static) return FTB_ERR_ARG;
+    if (schedule == 3 || (schedule == 0 && ch.take_static)) {
       unsigned long long* trace = nullptr;
 #ifdef FTB_TRACE
       trace = reinterpret_cast<unsigned long long*>(ws + lay.trace);
 #endif
-      rc = launch_lstm_static(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, Gs,
+      rc = launch_lstm_static(dtype, x, Wp, bias_p, hs, c, D, L, N, I, H, ch.Gs,
                               reinterpret_cast<int*>(ws + lay.done), status, trace, stream);
       // A cooperative launch can be refused (device shared through MPS, SMs reserved, ...).
       // With an explicit schedule that is the caller's error to see; the automatic choice
@@ -897,6 +919,34 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
     }
   }
   return FTB_OK;
+}
+
+int ftb_lstm_flow_form_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* active_rows,
+                           int D, int L, int N, int I, int H, int dtype, int nb, int pair, int ring, void* workspace,
+                           size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!x || !Wp || !hs || !c || D <= 0 || L <= 0 || N <= 0 || H <= 0 || I <= 0) return FTB_ERR_ARG;
+  if (!aligned16({x, Wp, bias_p, hs, c})) return FTB_ERR_ALIGN;
+  std::vector<int> first(L + 1, 0);
+  for (int t = 0; t < L; ++t) {
+    const int rows = active_rows != nullptr ? active_rows[t] : N;
+    if (rows <= 0 || rows > (t > 0 && active_rows != nullptr ? active_rows[t - 1] : N) || (t == 0 && rows != N)) return FTB_ERR_ARG;
+    if (static_cast<int64_t>(D) * (first[t] + static_cast<int64_t>(rows)) > 0x7fffffffLL) return FTB_ERR_ARG;
+    first[t + 1] = first[t] + rows;
+  }
+  FlowPlan flow;
+  if (!lstm_flow_form(dtype, D, N, I, H, current_sm_count(), nb, pair == 2, ring != 0, &flow)) return FTB_ERR_ARG;
+  int* status = nullptr;
+  int rc = begin_call(workspace, workspace_bytes, stream, &status);
+  if (rc) return rc;
+  const size_t table = (sizeof(int) * (L + 1) + 255) & ~static_cast<size_t>(255);
+  if (workspace_bytes < kWorkspaceBytes + table + flow_flag_bytes(D, L, flow.S)) return FTB_ERR_WORKSPACE;
+  int* off = reinterpret_cast<int*>(static_cast<char*>(workspace) + kWorkspaceBytes);
+  if (active_rows != nullptr &&
+      cudaMemcpyAsync(off, first.data(), sizeof(int) * (L + 1), cudaMemcpyHostToDevice, stream) != cudaSuccess)
+    return FTB_ERR_LAUNCH;
+  return launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, active_rows != nullptr ? off : nullptr, first[L], D, L, N, I, H, flow,
+                          off + table / sizeof(int), status, stream);
 }
 
 // Row tables of a ragged batch.

@@ -107,6 +107,18 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
                          int N, int I, int H, int dtype, const int* tuning, void* workspace, size_t workspace_bytes,
                          void* stream);
 
+/* What ftb_lstm_stacked_fwd takes for a 16-bit problem with everything automatic and enough workspace: form[0] the schedule (2 to
+ * 5), and for 5 form[1] the sequences of a slice, form[2] 1 single CTAs or 2 pairs, form[3] blocks of the ring that input
+ * weights pass through (0: all are kept). */
+int ftb_lstm_stacked_form(int D, int L, int N, int I, int H, int dtype, int* form);
+
+/* Schedule 5 with that form named, for tests and measurements; active_rows as in ftb_lstm_stacked_varlen_fwd (N = active_rows[0]),
+ * or NULL.  nb 16, 32, 64 or, in pairs, 128; pair 1 or 2; ring 0 or 1: FTB_ERR_ARG where the weights leave no such choice or a
+ * layer does not fit on the device.  The workspace of either entry point is enough.  Every form gives the same bits. */
+int ftb_lstm_flow_form_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* active_rows,
+                           int D, int L, int N, int I, int H, int dtype, int nb, int pair, int ring, void* workspace,
+                           size_t workspace_bytes, void* stream);
+
 /* Stacked LSTM forward without a caller workspace.  No counterpart in the reference: it exists
  * for hosts that cannot allocate device memory where they call the forward pass (in a
  * real-time loop, in a plugin that is only handed input and output buffers, under a

@@ -22,12 +22,12 @@ def _params(ops, D, I, H, dt, g):
     (1, 1, 1, 64, 64),       # one step: nothing handed on
     (3, 7, 16, 128, 128),    # a full slice of 16
     (2, 6, 17, 256, 256),    # one sequence in the second slice
-    (5, 9, 70, 320, 320),    # odd number of K blocks, slices of 32
-    (8, 5, 64, 512, 512),    # slices of 64, input weights partly in shared memory
+    (5, 9, 70, 320, 320),    # odd number of K blocks
+    (8, 5, 64, 512, 512),    # input weights partly in shared memory
     (12, 6, 30, 640, 640),   # layers in groups: weights replaced between sweeps
     (2, 5, 8, 768, 768),     # a state of more than eight K blocks
     (1, 4, 40, 192, 64),     # input wider than the state
-    (16, 4, 256, 64, 64),    # slices of 32 and more at the narrowest state
+    (16, 4, 256, 64, 64),    # the narrowest state
     (4, 5, 256, 256, 256),
 ])
 def test_same_bits_as_levels(ops, dt, D, L, N, I, H):
@@ -39,6 +39,77 @@ def test_same_bits_as_levels(ops, dt, D, L, N, I, H):
         h, c = ops.lstm_stacked(x, Wp, b, schedule=5)
         ops.check_status()
         assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+def _form(D, L, N, H, dt):
+    """What the automatic choice takes: schedule, sequences of a slice, 1 single CTAs or 2 pairs, blocks of the ring."""
+    import ctypes
+    from fractaltensor_b200._lib import DTYPE_BF16, DTYPE_F16, check, lib
+    form = (ctypes.c_int * 4)()
+    check(lib.ftb_lstm_stacked_form(D, L, N, H, H, DTYPE_F16 if dt == torch.float16 else DTYPE_BF16, form), "ftb_lstm_stacked_form")
+    return list(form)
+
+
+def _named_form(ops, x, Wp, b, N, active, nb, pair, ring):
+    import ctypes
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, lib
+    D, H, L = Wp.shape[0], x.shape[-1], (len(active) if active else x.shape[0])
+    hs = torch.full((D,) + tuple(x.shape[:-1]) + (H,), 3.0, dtype=x.dtype, device="cuda")
+    c = torch.full((D, N, H), 3.0, device="cuda")
+    ws = ops.workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(D, L) if active else lib.ftb_lstm_stacked_workspace_bytes(D, L, N, H))
+    check(lib.ftb_lstm_flow_form_fwd(_ptr(x), _ptr(Wp), _ptr(b), _ptr(hs), _ptr(c), (ctypes.c_int * L)(*active) if active else None,
+                                     D, L, N, H, H, _dtype_code(x), nb, pair, ring, _ptr(ws), ws.numel(), _stream()), "ftb_lstm_flow_form_fwd")
+    ops.check_status()
+    return hs, c
+
+
+FORMS = [  # every one that can be launched: (nb, pair, ring), with last slices and second CTAs that are partly empty
+    (3, 7, 17, 128, 16, 1, 0), (12, 6, 30, 640, 16, 1, 0),   # four sweeps
+    (5, 9, 70, 320, 32, 1, 0), (9, 5, 33, 512, 32, 1, 0),    # three sweeps
+    (8, 5, 64, 512, 64, 1, 0), (15, 7, 196, 64, 64, 1, 0), (12, 5, 200, 256, 64, 1, 0), (2, 6, 65, 192, 64, 1, 0),
+    (2, 5, 9, 832, 16, 2, 0), (3, 6, 17, 576, 16, 2, 0), (9, 6, 24, 256, 16, 2, 0),
+    (5, 7, 33, 448, 32, 2, 0), (7, 6, 47, 512, 32, 2, 0),
+    (8, 12, 120, 640, 64, 2, 0), (12, 5, 232, 384, 64, 2, 0), (2, 5, 65, 128, 64, 2, 0),
+    (12, 6, 232, 384, 128, 2, 0), (3, 5, 129, 128, 128, 2, 0), (2, 4, 97, 448, 128, 2, 0),
+    (1, 20, 1, 1024, 16, 2, 1), (3, 11, 5, 896, 16, 2, 1), (10, 6, 24, 1024, 16, 2, 1),  # five sweeps
+    (9, 16, 19, 1024, 32, 2, 1), (3, 7, 33, 896, 32, 2, 1),
+    (10, 9, 60, 832, 64, 2, 1), (4, 9, 60, 960, 64, 2, 1), (4, 9, 64, 1024, 64, 2, 1), (3, 5, 65, 832, 64, 2, 1),
+]
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,L,N,H,nb,pair,ring", FORMS)
+def test_named_forms_same_bits_as_levels(ops, dt, D, L, N, H, nb, pair, ring):
+    """Slices, pairs and ring by name, on a rectangular batch and on a ragged one of as many sequences."""
+    g = torch.Generator(device="cuda").manual_seed(D * 100 + N)
+    Wp, b = _params(ops, D, H, H, dt, g)
+    x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1, pair=1)
+    for _ in range(2):
+        h, c = _named_form(ops, x, Wp, b, N, None, nb, pair, ring)
+        assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+    lens = sorted((1 + (7 * n) % L for n in range(N - 1)), reverse=True)
+    active = [sum(n > t for n in [L] + lens) for t in range(L)]
+    x = torch.randn(sum(active), H, device="cuda", generator=g).to(dt)
+    ref_h, ref_c = ops.lstm_stacked_varlen(x, active, Wp, b, schedule=1, pair=1)
+    h, c = _named_form(ops, x, Wp, b, N, active, nb, pair, ring)
+    assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+def test_forms_there_are(ops):
+    from fractaltensor_b200._lib import FtbError
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for N, H, nb, pair, ring in ((4, 128, 48, 1, 0), (4, 128, 128, 1, 0), (4, 128, 16, 2, 1), (4, 896, 16, 1, 1), (4, 896, 16, 2, 0),
+                                 (97, 512, 128, 2, 0), (1200, 128, 16, 1, 0)):
+        Wp, b = _params(ops, 1, H, H, torch.float16, g)
+        with pytest.raises(FtbError) as e:
+            _named_form(ops, torch.zeros(2, N, H, dtype=torch.float16, device="cuda"), Wp, b, N, None, nb, pair, ring)
+        assert e.value.code == 1
+    # the automatic choice reaches single CTAs, pairs and the ring on slices of several widths
+    for shape, form in (((2, 100, 8, 128), [5, 16, 1, 0]), ((15, 47, 196, 64), [5, 64, 1, 0]), ((4, 5, 256, 256), [5, 32, 2, 0]), ((8, 100, 64, 512), [5, 64, 2, 0]),
+                        ((12, 40, 232, 384), [5, 128, 2, 0]), ((1, 20, 1, 1024), [5, 16, 2, 4])):
+        assert _form(*shape, torch.float16) == form
+    assert _form(16, 100, 256, 1024, torch.bfloat16)[0] == 3
 
 
 @pytest.mark.parametrize("D,L,N,H", [
@@ -68,6 +139,7 @@ def test_pairs_same_bits_as_levels(ops, D, L, N, H):
 ])
 def test_streamed_input_weights_same_bits_as_levels(ops, dt, D, L, N, H):
     """The automatic choice at sizes where the estimate is far on this kernel's side: its others read all weights each step."""
+    assert _form(D, L, N, H, dt)[0] == 5 and _form(D, L, N, H, dt)[3] > 0
     g = torch.Generator(device="cuda").manual_seed(D * 100 + N)
     Wp, b = _params(ops, D, H, H, dt, g)
     x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
@@ -149,9 +221,11 @@ def test_automatic_choice_is_the_fastest_kernel(ops, D, N, H):
     assert ms(0) <= 1.15 * min(ms(s) for s in (2, 3, 4, 5))
 
 
-@pytest.mark.parametrize("D,L,N,H", [(2, 10, 8, 128), (8, 20, 64, 512), (1, 20, 1, 1024)])
+@pytest.mark.parametrize("D,L,N,H", [(2, 100, 8, 128), (8, 20, 64, 512), (1, 20, 1, 1024)])
 def test_captured_calls_fill_the_output_anew(ops, D, L, N, H):
     """Single CTAs, pairs and the ring in a CUDA graph, two calls one behind the other: each replay fills what the one before left."""
+    form = _form(D, L, N, H, torch.float16)
+    assert form[0] == 5 and (form[2], form[3] > 0) == {128: (1, False), 512: (2, False), 1024: (2, True)}[H]
     g = torch.Generator(device="cuda").manual_seed(H)
     dt = torch.float16
     Wp, b = _params(ops, D, H, H, dt, g)
