@@ -258,7 +258,7 @@ attn_finish_kernel(T* __restrict__ dec, const T* __restrict__ dec_proj, const fl
 // the whole program 105.5 us before, 94.2 so.  (U by 128 row copies of one warp: 99.4; its rows into registers: 98.9.)
 constexpr int kDecThreads = 512, kDecWarps = kDecThreads / 64;  // of a sequence
 constexpr int kDecMaxH = 512;
-constexpr int kDecMaxSteps = 256;  // of source or target
+constexpr int kDecMaxSource = 256, kDecMaxSteps = 128;  // source positions, target steps
 constexpr int kDecAhead = 8;       // steps of a warp, and rows of the sum of a thread over 2, requested ahead
 
 __device__ __forceinline__ void st_cluster_f32(float* p, uint32_t rank, float x) {
@@ -289,7 +289,7 @@ attn_decode_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, co
                    int Lt, int Ls, int N, int H, int* __restrict__ status) {
   constexpr int kN = 8, kColGroups = kAttnCols / kN, kRowGroups = kDecThreads / 2 / kColGroups;
   constexpr int kMaxCtas = kDecMaxH / kAttnCols;
-  __shared__ float s_score[2][kDecMaxSteps], s_w[2][kDecMaxSteps];
+  __shared__ float s_score[2][kDecMaxSource], s_w[2][kDecMaxSource];
   __shared__ float s_term[kMaxCtas][2][kDecMaxSteps];  // the CTAs' parts of the decoder's terms
   __shared__ float s_part[2][kRowGroups][kAttnCols];
   __shared__ __align__(16) T s_v[2][kDecMaxH];
@@ -550,7 +550,7 @@ int launch_attn_vectors(int dtype, const void* enc, const void* enc_proj, const 
 // 50 + 50 positions, 55 sequences 109.0 / 98.4, 256 136.1 / 151.6; 26 + 52, 81 sequences 71.8 / 75.9; 27 + 8, 6 sequences 66.5 / 59.4;
 // 20 + 250, 1 sequence 59.1 / 61.7; H 128, 26 + 61, 42 sequences 48.2 / 45.1.
 bool attn_decode_supported(int dtype, int Ls, int Lt, int N, int H, int sm_count) {
-  return dtype != FTB_F32 && H % kAttnCols == 0 && H <= kDecMaxH && Ls <= kDecMaxSteps && Lt <= kDecMaxSteps / 2 &&
+  return dtype != FTB_F32 && H % kAttnCols == 0 && H <= kDecMaxH && Ls <= kDecMaxSource && Lt <= kDecMaxSteps &&
          (N + 1) / 2 * (H / kAttnCols) <= sm_count - 4;
 }
 
