@@ -399,7 +399,7 @@ attn_decode_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, co
     st_f32<T>(&t, v * inv);
     for (uint32_t r = 0; r < ctas; ++r) st_cluster_16<T>(&s_v[seq][col0 + gt], r, t);
   }
-  mbar_wait(&u_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
+  const bool u_there = mbar_wait(&u_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
   __syncwarp();
   cluster_sync_all();
 
@@ -473,6 +473,11 @@ attn_decode_kernel(const T* __restrict__ enc, const T* __restrict__ enc_proj, co
         if (t > s_first[seq]) st_f32<T>(dec + t * step_elems + row + h, nan);
         st_f32<T>(out + t * step_elems + row + h, nan);
       }
+  if (!u_there) {
+    // The wait ran out: give the copies of U time to land before the shared memory goes back.
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
 }
 
 template <typename T>
