@@ -45,6 +45,7 @@ SIGNATURES = {
     "ftb_flash_attn_causal_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_flash_attn_window_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_flash_attn_local_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
+    "ftb_flash_attn_form": (_i, [_i] * 6),
     "ftb_flash_attn_form_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "ftb_lstm_stacked_form": (_i, [_i] * 6 + [ctypes.POINTER(_i)]),
     "ftb_lstm_flow_form_fwd": (_i, [_vp] * 5 + [ctypes.POINTER(_i)] + [_i] * 9 + [_vp, _sz, _vp]),

@@ -43,6 +43,7 @@
 namespace ftb {
 
 // flash_pair.cu
+int flash_pair_group(int S);
 int flash_pair_launch(const void* q, const void* k, const void* v, void* o, int64_t rows, int n_bh, int S, int dtype,
                       bool masked, int left, int right, float scale_log2, int* status, cudaStream_t stream);
 
@@ -664,46 +665,61 @@ int launch(bool masked, bool halves, const CUtensorMap& mQ, const CUtensorMap& m
 // The form of a call: 1 = CTAs of 256 query rows, 2 = of 128 rows and half of their blocks a slot, 3 = pairs of CTAs (flash_pair.cu),
 // by estimates in us.  A tile of query rows takes a fixed time and one for each block that its longer slot walks, and a pair one for
 // each block that an edge of a mask crosses.  Where there are more tiles than places for them (SMs, pairs of SMs), equal ones go
-// in whole rounds, unequal ones (masks, longest first) half a round of CTAs beyond their mean, pairs, which take theirs in a
-// balanced order, a quarter, and no less than the longest and the shortest together.
+// in whole rounds, unequal ones (masks) half a round of CTAs beyond their mean, pairs, which take theirs in a balanced order, a
+// quarter.  Of at most two rounds of pairs the largest sum is taken: behind a window all tiles but the first few are equally long (keys
+// i-161..i+745, 12 x 2304, 107 tiles: 25.9 us as form 1, 31.3 as pairs; 6 x 4096, i-723..i+1049: 37.4 as form 2, 41.5 as pairs).
 // Forms 1 and 2: halves that are estimated less than a tenth faster keep the 256 rows: between 0.9 and 1 of the estimate the
 // time is 0.9 to 1.19 of theirs, below it 0.53 to 0.97.  Form 3 against the one of them: its constants are fitted to 150 calls
 // over the sizes and masks of 1 to 16 x 4 to 16 heads and 256 to 4096 keys; the estimates of the other two, made for full and
-// causal walks, lie a fifth below what short masked walks take, which the factor makes up for.  Of those calls 55 take pairs, which
-// run at 0.95 to 1.6 times the other form's rate; all 150 gain 6.0 % (the best form of each would gain 7.5, a factor of 1.25 6.7; but
-// of 40 other calls one lost 13 % by that: keys i-49..i+184, 54 x 1024, 33.8 / 38.7).
-// Measured, us, forms 1 / 2 / 3 (* taken): full 16 x 256 8.2 / 7.2* / 7.4, 7 x 512 13.0 / 10.4 / 9.5*, 99 x 512 30.4 / 34.3 / 19.3*,
+// causal walks, lie a fifth below what short masked walks take, so that pairs are taken up to 1.2 times their estimate.  Of 820 other
+// calls none is more than 5 % slower by that than without pairs, and four more than 2 %; all gain 7.5 % (the best form of each would
+// gain 8.2; a factor of 1.1 gives 6.6, one call 5 % slower; of 1.3 7.7, 39 slower by up to 17 %).
+// Measured, us, forms 1 / 2 / 3 (* taken): full 16 x 256 8.2 / 7.2* / 7.4, 7 x 512 13.0 / 10.4* / 9.5, 99 x 512 30.4 / 34.3 / 19.3*,
 // 40 x 1024 39.5 / 40.1 / 26.8*, 16 x 2048 35.9 / 43.0 / 33.2*, 20 x 2048 68 / 63 / 45*, 4 x 4096 63 / 37 / 33*, 256 x 2048 490 / 574 /
 // 438*; causal 15 x 256 8.3 / 6.9* / 8.0, 66 x 512 12.8* / 19.7 / 13.9, 36 x 1024 20.4 / 26.7 / 17.4*, 16 x 2048 37 / 28 / 23.4*, 84 x 3328 266 /
-// 294 / 225*; window of 65 77 x 768 24.1* / 29.0 / 28.7, of 1307 42 x 3584 110* / 139 / 111; keys i-751..i+392 42 x 1024 40 / 39 / 29.5*.
+// 294 / 225*; window of 65 77 x 768 24.1* / 29.0 / 28.7, of 1307 42 x 3584 110 / 139 / 111*; keys i-751..i+392 42 x 1024 40 / 39 / 29.5*,
+// i-49..i+184 54 x 1024 33.8* / - / 38.7.
 int attention_form(bool masked, int n_bh, int S, int left, int right, int sm_count) {
   constexpr double kFixed = 4.5, kBlock = 1.9;
   constexpr double kPairCall = 4.6, kPair = 2.25, kPairBlock = 0.83, kPairMasked = 2.7, kPairMaskedBlock = 0.8, kPairEdge = 0.55, kBelow = 1.2;
   double us[3];
   for (int form = 0; form < 3; ++form) {
     const int rows = form == 1 ? 128 : 256, tiles = S / rows;
-    double total = 0, longest = 0, shortest = 1e30;
-    for (int i = 0; i < tiles; ++i) {
+    const auto time_of = [&](int i) {
       const int r0 = i * rows;
       const bool begins_late = masked && left >= 0 && r0 > left;
       const int lo = begins_late ? (r0 - left) >> 7 : 0;
       const int hi = masked && r0 + rows - 1 < S - right ? (r0 + rows - 1 + right) >> 7 : S / 128 - 1;
       const int blocks = hi - lo + 1;
-      const double t = form == 0   ? kFixed + kBlock * blocks
-                       : form == 1 ? kFixed + kBlock * ((blocks + 1) / 2)
-                       : masked    ? kPairMasked + kPairMaskedBlock * blocks + kPairEdge * std::min(blocks, begins_late ? 6 : 2)
-                                   : kPair + kPairBlock * blocks;
+      return form == 0   ? kFixed + kBlock * blocks
+             : form == 1 ? kFixed + kBlock * ((blocks + 1) / 2)
+             : masked    ? kPairMasked + kPairMaskedBlock * blocks + kPairEdge * std::min(blocks, begins_late ? 6 : 2)
+                         : kPair + kPairBlock * blocks;
+    };
+    double total = 0, longest = 0, shortest = 1e30;
+    for (int i = 0; i < tiles; ++i) {
+      const double t = time_of(i);
       total += t;
       longest = std::max(longest, t);
       shortest = std::min(shortest, t);
     }
-    const double waves = static_cast<double>(n_bh) * tiles / (form == 2 ? sm_count / 2 : sm_count);
-    if (waves <= 1)
+    const int places = form == 2 ? sm_count / 2 : sm_count;
+    const double waves = static_cast<double>(n_bh) * tiles / places;
+    if (waves <= 1) {
       us[form] = longest;
-    else if (masked)
+    } else if (masked && form == 2 && waves <= 2) {
+      const int group = flash_pair_group(S), units = n_bh * tiles;
+      const auto unit_time = [&](int u) {  // as the kernel deals them out
+        const int g = u / (group * tiles);
+        return time_of(tiles - 1 - (u - g * group * tiles) / std::min(group, n_bh - g * group));
+      };
+      us[form] = longest;
+      for (int u = places; u < units; ++u) us[form] = std::max(us[form], unit_time(u) + unit_time(2 * places - 1 - u));
+    } else if (masked) {
       us[form] = std::max(form == 2 ? longest + shortest : longest, (waves + (form == 2 ? 0.25 : 0.5)) * total / tiles);
-    else
+    } else {
       us[form] = std::ceil(waves) * longest;
+    }
   }
   const int single = us[1] < 0.9 * us[0] ? 1 : 0;
   return kPairCall + us[2] < kBelow * us[single] ? 3 : single + 1;
@@ -783,6 +799,11 @@ extern "C" int ftb_flash_attn_local_fwd(const void* q, const void* k, const void
   if (left < 0 || right < 0) return FTB_ERR_ARG;
   return flash_attn_entry(q, k, v, o, B, heads, S, d, scale, dtype, true, left, right, workspace, workspace_bytes,
                           stream);
+}
+
+extern "C" int ftb_flash_attn_form(int n_bh, int S, int masked, int left, int right, int sm_count) {
+  if (n_bh <= 0 || S <= 0 || S % 256 != 0 || sm_count < 2 || (masked && right < 0)) return 0;
+  return attention_form(masked != 0, n_bh, S, left < 0 || left >= S ? -1 : left, std::min(right, S), sm_count);
 }
 
 extern "C" int ftb_flash_attn_form_fwd(const void* q, const void* k, const void* v, void* o, int B, int heads, int S,

@@ -560,14 +560,19 @@ flash_pair_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
   }
 }
 
+}  // namespace
+
+// (batch, head) entries whose units are dealt out together: 64 MB of K and V.
+int flash_pair_group(int S) { return static_cast<int>(std::max<long long>(16, (64ll << 20) / (512ll * S))); }
+
+namespace {
 template <typename T, bool kMasked>
 int launch(const CUtensorMap& mQ, const CUtensorMap& mK, const CUtensorMap& mV, const CUtensorMap& mO, int n_bh,
            int S, int left, int right, float scale_log2, int* status, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
   auto kfn = flash_pair_kernel<T, kMasked>;
   if (!ensure_dynamic_smem(kfn, kSmemBytes, configured)) return FTB_ERR_LAUNCH;
-  const int group = static_cast<int>(std::max<long long>(16, (64ll << 20) / (512ll * S)));  // 64 MB of K and V
-  Shape sh = {S, n_bh, group, left, right};
+  Shape sh = {S, n_bh, flash_pair_group(S), left, right};
   const long long units = static_cast<long long>(n_bh) * (S / 256);
   const int clusters = static_cast<int>(std::min<long long>(units, current_sm_count() / 2));
   const cudaError_t err = launch_dependent(kfn, dim3(2 * clusters), dim3(kThreads), kSmemBytes, stream, mQ, mK, mV, mO, sh,

@@ -263,7 +263,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   if ((rc = make_tmap_2d(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H, I + H, kGateRows, BK))) return rc;
   const int64_t chunks = static_cast<int64_t>(D) * T * H / 8;
   const int n_flags = D * L * a.S;
-  flow_fill_kernel<<<static_cast<int>(std::min<int64_t>(148, (std::max<int64_t>(chunks, n_flags) + 255) / 256)), 256, 0, stream>>>(
+  flow_fill_kernel<<<static_cast<int>(std::min<int64_t>(current_sm_count(), (std::max<int64_t>(chunks, n_flags) + 255) / 256)), 256, 0, stream>>>(
       static_cast<uint4*>(hs), chunks, flags, n_flags);
   if (cudaGetLastError() != cudaSuccess) return FTB_ERR_LAUNCH;
   count_launch();

@@ -269,6 +269,9 @@ int ftb_flash_attn_local_fwd(const void* q, const void* k, const void* v, void* 
                              int d, int left, int right, float scale, int dtype, void* workspace,
                              size_t workspace_bytes, void* stream);
 
+/* The form that the library's rule takes on a device of sm_count SMs, n_bh = B * heads; 0: no such call. */
+int ftb_flash_attn_form(int n_bh, int S, int masked, int left, int right, int sm_count);
+
 /* Any of the four with the form of the kernel named, for tests and measurements.  form: 0 by the library's rule, 1 CTAs
  * of 256 query rows, 2 CTAs of 128 rows whose two slots take half of the keys each, 3 pairs of CTAs on 256 rows;
  * results differ by rounding.
