@@ -172,7 +172,6 @@ __device__ __forceinline__ float group_dot(const float (&a)[kEPL], const float (
   return s;
 }
 
-
 struct SparseArgs {
   long long heads_total;  // B * heads
   int S, window, dilation, n_global, R, as_shipped;

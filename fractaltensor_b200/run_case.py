@@ -8,6 +8,8 @@
     python -m fractaltensor_b200.run_case b2b --batch 16 --M 16384
     python -m fractaltensor_b200.run_case attn --B 4 --heads 16 --S 2048
     python -m fractaltensor_b200.run_case sparse_attn --B 2 --heads 16 --S 4096 --dtype fp32
+    python -m fractaltensor_b200.run_case project --M 2240 --H 512 --V 10000
+    python -m fractaltensor_b200.run_case rnn_attn --L 50 --N 64 --H 512
 
 A small, fixed workload to put under a profiler or to time by hand; prints the
 average time per call measured with CUDA events.
@@ -24,7 +26,7 @@ DT = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["lstm", "varlen", "dilated", "grid", "b2b", "attn", "softmax", "sparse_attn"])
+    ap.add_argument("case", choices=["lstm", "varlen", "dilated", "grid", "b2b", "attn", "softmax", "sparse_attn", "project", "rnn_attn"])
     ap.add_argument("--D", type=int, default=16)
     ap.add_argument("--L", type=int, default=20)
     ap.add_argument("--N", type=int, default=256)
@@ -47,6 +49,8 @@ def main():
     ap.add_argument("--causal", action="store_true", help="attn: keys 0..i for query i")
     ap.add_argument("--window", type=int, default=None, help="attn with --causal: keys i-window+1..i")
     ap.add_argument("--local", type=int, nargs=2, default=None, help="attn: keys i-LEFT..i+RIGHT")
+    ap.add_argument("--form", type=int, default=0, help="attn: the form of the kernel (1 to 3; 0 by the library's rule)")
+    ap.add_argument("--V", type=int, default=10000, help="project: vocabulary, over M rows of H")
     ap.add_argument("--head-dim", type=int, default=64, help="sparse_attn: elements per head")
     ap.add_argument("--as-shipped", action="store_true", help="sparse_attn: the softmax dimension of the shipped example")
     ap.add_argument("--graph", action="store_true",
@@ -117,6 +121,25 @@ def main():
             q, k, v = sets[turn[0]]
             return ops.sparse_attention(q, k, v, pos, 5, 2, 3, scale=1 / math.sqrt(a.head_dim),
                                         as_shipped=a.as_shipped, out=outs[turn[0]])
+    elif a.case == "project":
+        h, P = rnd(a.M, a.H).to(dt), (rnd(a.H, a.V) / 4).to(dt)
+        fn = lambda: ops.project_softmax_rows(h, P)
+    elif a.case == "rnn_attn":
+        # L positions of source and target; sentences of all lengths up to L
+        src, trg = rnd(a.L, a.N, a.H).to(dt), rnd(a.L, a.N, a.H).to(dt)
+        bound = 1 / math.sqrt(a.H)
+        weights = [ops.rnn_pack_weights(uni(bound, a.H, a.H).to(dt), uni(bound, a.H, a.H).to(dt)) for _ in range(2)]
+        biases, projections = [uni(bound, a.H) for _ in range(2)], [uni(1.0, a.H).to(dt) for _ in range(2)]
+        lens = (torch.arange(a.N, device=dev, dtype=torch.int32) % a.L) + 1
+        fn = lambda: ops.rnn_attention(src, trg, *weights, *biases, *projections, lens)
+    elif a.form:
+        left, right = a.local if a.local is not None else (a.window - 1 if a.window is not None else -1, 0)
+        q, k, v = (rnd(a.B, a.heads, a.S, 128).to(dt) for _ in range(3))
+        out, ws = torch.empty_like(q), ops.workspace(dev)
+        fn = lambda: ops.check(ops.lib.ftb_flash_attn_form_fwd(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), a.B, a.heads, a.S, 128, int(a.causal or a.local is not None),
+            left, right, a.form, 1 / math.sqrt(128), ops._dtype_code(q), ws.data_ptr(), ws.numel(),
+            torch.cuda.current_stream().cuda_stream), "ftb_flash_attn_form_fwd")
     else:
         q, k, v = (rnd(a.B, a.heads, a.S, 128).to(dt) for _ in range(3))
         out = torch.empty_like(q)

@@ -198,7 +198,7 @@ def test_fractal_tensor_element_type():
     assert ft.astype(torch.float16).element_type is T.float16
 
 
-REFERENCE_ROOT = os.environ.get("FTB_REFERENCE_ROOT", "/root/reference")
+REFERENCE_ROOT = os.environ.get("FTB_REFERENCE_ROOT", "")
 
 
 @pytest.mark.skipif(not os.path.isdir(os.path.join(REFERENCE_ROOT, "kaleido")),
