@@ -87,7 +87,8 @@ __device__ __forceinline__ void row_dots(const T* rows, long long stride, int co
   for (int r = 0; r < kDots; ++r) s[r] = 0.f;
   for (int h = lane * n; h < H; h += 32 * n) {
     float p[n];
-    if ((reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
+    // (16-bit only: for fp32 the branch costs more than three loads from L1, H 64, 1 sequence, 8 + 4096 positions 78.0 us without it, 80.0)
+    if (sizeof(T) == 2 && (reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
       ld_piece(proj + h, p);
     } else {
 #pragma unroll
