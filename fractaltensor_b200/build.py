@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libftb200.so")
 HOST_SRC = os.path.join(CSRC, "host_calls.cpp")
 HOST = os.path.join(HERE, "_host.so")
-SOURCES = ["tmap.cu", "pack.cu", "cell_gemm.cu", "cell_simt.cu", "lstm_simt_static.cu", "lstm_simt_flow.cu", "lstm_static.cu", "lstm_wmajor.cu", "lstm_flow.cu", "rnn_cluster.cu", "wavefront.cu", "b2b_gemm.cu", "flash_attn.cu", "flash_pair.cu",
+SOURCES = ["tmap.cu", "pack.cu", "cell_gemm.cu", "cell_simt.cu", "lstm_simt_static.cu", "lstm_simt_flow.cu", "lstm_static.cu", "lstm_wmajor.cu", "lstm_flow.cu", "rnn_cluster.cu", "grid_flow.cu", "wavefront.cu", "b2b_gemm.cu", "flash_attn.cu", "flash_pair.cu",
            "online_softmax.cu", "project.cu", "embedding.cu", "sparse_attn.cu", "rnn_attention.cu", "rnn_chain.cu"]
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",

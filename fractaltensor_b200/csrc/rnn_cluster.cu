@@ -1,27 +1,19 @@
-// Latency-bound recurrences with small hidden size (H <= 256): the dilated stacked LSTM
-// and the 2-D grid RNN, one thread-block cluster per chain of dependent steps.
+// A latency-bound recurrence with small hidden size (H <= 256): the dilated stacked LSTM, one thread-block
+// cluster per chain of dependent steps.  (The grid RNN: csrc/grid_flow.cu.)
 //
-// These programs are chains of small cells: 512 dependent steps of [256 x 512].[512 x 1024]
-// in the first layer of the dilated LSTM, 63 anti-diagonals of [64 x 768].[768 x 256] cells
-// in the grid.  Run as a generic wavefront, every dependent level costs a trip through
+// The program is chains of small cells: 512 dependent steps of [256 x 512].[512 x 1024] in the first layer.  Run as a generic wavefront, every dependent level costs a trip through
 // global memory (store, fence, flag, poll, TMA load: 6-9 us) plus a re-read of the layer's
 // weights from L2.  Here
-//   * the weights never move: a cluster of CL CTAs owns one chain (one layer and batch slice of
-//     the dilated LSTM; one grid row and batch slice of the grid RNN), CTA r of the cluster owns
-//     128 packed weight rows (32 LSTM units x 4 gates, or 128 tanh units) for the whole launch,
-//     and that slice of the weights sits in tensor memory as the A operand of every MMA
-//     ("recurrent weights resident on chip");
+//   * the weights never move: a cluster of CL CTAs owns one chain (one layer and batch slice), CTA r of the
+//     cluster owns 128 packed weight rows (32 LSTM units x 4 gates) for the whole launch, and that slice of the
+//     weights sits in tensor memory as the A operand of every MMA ("recurrent weights resident on chip");
 //   * the batch is the N side of the MMA (NB = 128 or 64 columns per slice);
-//   * the state a chain hands to its own next step -- h(t) of a layer with dilation 1, h_y of
-//     the grid cell to the left -- never leaves the cluster: it goes into the next step's B operand in
-//     every CTA of the cluster (distributed shared memory), bytes counted on the receiver's mbarrier.
-//     In the grid an epilogue thread packs eight sequences of its unit, one 16-byte row of the
-//     un-swizzled MN-major core-matrix layout, and stores it with st.async straight from its registers: no
-//     staging, no barrier between the warps (32 x 32, H 256, 64 sequences: 280 -> 257 us).  In the
-//     dilated LSTM each CTA writes its units into a staging tile, a contiguous block of the K-major
-//     layout, and copies it with one bulk copy per piece and peer: eight peers' 32 KB a step are bound by
-//     the bytes, and 16 at a time take longer (3.1 us a step instead of 3.0);
-//   * everything that crosses chains (the layer below, the grid row above, a layer's own state
+//   * the state a chain hands to its own next step, h(t) of a layer with dilation 1, never leaves the
+//     cluster: it goes into the next step's B operand in every CTA of the cluster (distributed shared memory),
+//     bytes counted on the receiver's mbarrier.  Each CTA writes its units into a staging tile, a contiguous
+//     block of the un-swizzled K-major layout, and copies it with one bulk copy per piece and peer: eight peers'
+//     32 KB a step are bound by the bytes, and st.async of 16 at a time takes longer (3.1 us a step instead of 3.0);
+//   * everything that crosses chains (the layer below, a layer's own state
 //     `dilation` >= 2 steps back) goes through global memory with one release flag per
 //     (cell, tile), polled by a whole warp, and TMA loads; those consumers run a few steps behind
 //     their producers, so this latency adds to the pipeline's depth, not to every step.  The
@@ -30,14 +22,11 @@
 // then the recurrent state(s)): the results are bit-identical.
 //
 // Roles: warp 0 producer of the TMA-fed operand blocks, warp 1 MMA issuer (owns TMEM), warp 2
-// output store and flag publisher, warp 3 idle, warps 4.. epilogue (16 for the LSTM cell, 8 for the
-// tanh cell).  tcgen05 cta_group::1; no multicast loads;
+// output store and flag publisher, warp 3 the second producer, warps 4.. epilogue.  tcgen05 cta_group::1; no multicast loads;
 // cooperative cluster launch (a chain waits for flags of other clusters).
 //
 // Programs: dilated_layer()/model() (examples/dilated_rnn/dilated_rnn.py:16-41) in place of
-// DilatedLstmRegion1/2 (kaleido/core/device/kernels/lstm/dilated_lstm/region{1,2}.h), and
-// stacked_grid_rnns() (examples/grid_rnn/grid_rnn.py:42-122) in place of the grid regions
-// (benchmarks/rnn/fractaltensor/grid_lstm/regions/region{1..8}.h).
+// DilatedLstmRegion1/2 (kaleido/core/device/kernels/lstm/dilated_lstm/region{1,2}.h).
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -52,15 +41,14 @@ namespace {
 
 constexpr int BK = 64;
 constexpr int kFirstEpiWarp = 4;
-// Epilogue warps: four per TMEM lane quadrant for the LSTM cell (five MUFU operations and a quad
-// transpose per element: latency-bound with fewer), two for the tanh cell.
-__host__ __device__ constexpr int epi_warps(int mode) { return mode == 0 ? 16 : 8; }
-__host__ __device__ constexpr int cta_threads(int mode) { return 32 * (kFirstEpiWarp + epi_warps(mode)); }
+// Epilogue warps: four per TMEM lane quadrant (five MUFU operations and a quad transpose per element:
+// latency-bound with fewer).
+constexpr int kEpiWarps = 16;
+constexpr int kCtaThreads = 32 * (kFirstEpiWarp + kEpiWarps);
+constexpr int kOutUnits = 32;  // hidden units of a CTA
 constexpr uint32_t kStageBytes = 16384;
 
 constexpr int kMaxLayers = 16;
-
-enum ClusterMode : int { kDilated = 0, kGrid = 1 };
 
 #ifdef FTB_TRACE
 // Debug builds: globaltimer stamps of CTA rank 0 of every cluster, [cluster][step][16].
@@ -86,23 +74,19 @@ __device__ unsigned long long* g_cluster_acct = nullptr;
 #endif
 
 struct ClusterArgs {
-  int D, L, N, H;  // layers, steps of a chain (dilated: time steps; grid: B), batch, hidden size
-  int A;           // grid: rows of the grid (chains per layer and slice); dilated: 1
-  int S;           // grid: batch slices of NB columns; dilated: counters per cell (the most slices of a layer)
+  int D, L, N, H;  // layers, time steps, batch, hidden size
+  int S;           // counters per cell (the most slices of a layer)
   int CL;          // CTAs per cluster
   int max_dil;
   int dil[kMaxLayers];
-  int nb[kMaxLayers];              // dilated: batch columns per chain of the layer
-  bool flow;                       // dilated: layers with dilation 1 run flow::body
-  int first_cluster[kMaxLayers + 1];  // dilated: index of the layer's first cluster
-  const void* W0;       // dilated: Wp [D,4H,2H]; grid: Wpx [D,H,3H]
-  const void* W1;       // grid: Wpy
-  const float* bias0;   // dilated: bias_p [D,4H]; grid: bias_x [D,H]   (or nullptr)
-  const float* bias1;   // grid: bias_y
-  void* out0;           // dilated: hs [D,L,N,H]; grid: hx [D,A,B,N,H]
-  void* out1;           // grid: hy
-  float* c;             // dilated: fp32 [D, max_dil*N, H]
-  int* flags;           // grid: [cells][CL] flags; dilated: [cells][S] counters of CTAs; zero before the launch
+  int nb[kMaxLayers];                 // batch columns per chain of the layer
+  bool flow;                          // layers with dilation 1 run flow::body
+  int first_cluster[kMaxLayers + 1];  // index of the layer's first cluster
+  const void* W;      // Wp [D,4H,2H]
+  const float* bias;  // bias_p [D,4H] or nullptr
+  void* out;          // hs [D,L,N,H]
+  float* c;           // fp32 [D, max_dil*N, H]
+  int* flags;         // [cells][S] counters of CTAs; zero before the launch
   int* status;
 };
 
@@ -119,10 +103,6 @@ struct StepPlan {
   bool self;       // the cluster's own previous output is an operand (through shared memory)
   int self_wkb0, self_nkb;
 };
-
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // Whole-warp bounded wait until the n flags at `flags` have all reached `target` (lane i polls flags i, i+32, ...).
 __device__ __forceinline__ bool warp_wait_flags(const int* flags, int n, int target, int lane, volatile int* s_abort, int* g_status) {
@@ -192,115 +172,69 @@ __device__ __forceinline__ __half to_elem<__half>(float v) { return __float2half
 template <>
 __device__ __forceinline__ __nv_bfloat16 to_elem<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// What this CTA multiplies at step `i` of its chain.  Every role calls it with the same arguments.
-//   dilated: chain = (layer l, slice s), step = time step t.
-//   grid:    chain = (layer d, row a, slice s), step = column b.
-template <int MODE, int NB>
-__device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, int row_a, int slice, int rank, int i) {
+// What this CTA multiplies at time step `i` of its chain (layer, slice).  Every role calls it with the same arguments.
+template <int NB>
+__device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, int slice, int i) {
   StepPlan p;
   p.nseg = 0;
   p.self = false;
   p.self_wkb0 = p.self_nkb = 0;
   const int kbh = a.H / BK;
-  if (MODE == kDilated) {
-    const int d = a.dil[layer];
-    Segment& x = p.seg[p.nseg++];
-    x.nkb = kbh;
-    x.wkb0 = 0;
-    if (layer == 0) {
-      x.map = 0;
-      x.row = i * a.N + slice * NB;
-      x.flags = nullptr;
-      x.nflags = 0;
-    } else {
-      x.map = 1;
-      x.row = ((layer - 1) * a.L + i) * a.N + slice * NB;
-      // One counter per slice of a cell.  The layer below may be cut differently: its slices that hold this
-      // one's rows own consecutive counters.
-      const int nbp = a.nb[layer - 1];
-      const int first = slice * NB / nbp;
-      x.flags = a.flags + ((layer - 1) * a.L + i) * a.S + first;
-      x.nflags = (min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
-      x.target = a.CL;
-    }
-    if (i >= d) {
-      if (d == 1) {
-        p.self = true;
-        p.self_wkb0 = kbh;
-        p.self_nkb = kbh;
-      } else {
-        Segment& h = p.seg[p.nseg++];
-        h.map = 1;
-        h.row = (layer * a.L + i - d) * a.N + slice * NB;
-        h.nkb = kbh;
-        h.wkb0 = kbh;
-        h.flags = a.flags + (layer * a.L + i - d) * a.S + slice;
-        h.nflags = 1;
-        h.target = a.CL;
-      }
-    }
+  const int d = a.dil[layer];
+  Segment& x = p.seg[p.nseg++];
+  x.nkb = kbh;
+  x.wkb0 = 0;
+  if (layer == 0) {
+    x.map = 0;
+    x.row = i * a.N + slice * NB;
+    x.flags = nullptr;
+    x.nflags = 0;
   } else {
-    // packed K order of a grid cell: [state_x | state_y | input]; issue order: input, state_x, state_y
-    const bool ydir = rank >= a.CL / 2;
-    const int cell = (layer * a.A + row_a) * a.L + i;  // a.L = B
-    Segment& in = p.seg[p.nseg++];
-    in.nkb = kbh;
-    in.wkb0 = 2 * kbh;
-    if (layer == 0) {
-      in.map = ydir ? 1 : 0;
-      in.row = ((row_a * a.L + i) * a.N) + slice * NB;
-      in.flags = nullptr;
-      in.nflags = 0;
-    } else {
-      const int below = ((layer - 1) * a.A + row_a) * a.L + i;
-      in.map = ydir ? 3 : 2;
-      in.row = below * a.N + slice * NB;
-      in.flags = a.flags + (below * a.S + slice) * a.CL + (ydir ? a.CL / 2 : 0);
-      in.nflags = a.CL / 2;
-      in.target = 1;
-    }
-    if (row_a > 0) {
-      const int up = (layer * a.A + row_a - 1) * a.L + i;
-      Segment& sx = p.seg[p.nseg++];
-      sx.map = 2;
-      sx.row = up * a.N + slice * NB;
-      sx.nkb = kbh;
-      sx.wkb0 = 0;
-      sx.flags = a.flags + (up * a.S + slice) * a.CL;  // the x-direction tiles come first
-      sx.nflags = a.CL / 2;
-      sx.target = 1;
-    }
-    if (i > 0) {
+    x.map = 1;
+    x.row = ((layer - 1) * a.L + i) * a.N + slice * NB;
+    // One counter per slice of a cell.  The layer below may be cut differently: its slices that hold this
+    // one's rows own consecutive counters.
+    const int nbp = a.nb[layer - 1];
+    const int first = slice * NB / nbp;
+    x.flags = a.flags + ((layer - 1) * a.L + i) * a.S + first;
+    x.nflags = (min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
+    x.target = a.CL;
+  }
+  if (i >= d) {
+    if (d == 1) {
       p.self = true;
       p.self_wkb0 = kbh;
       p.self_nkb = kbh;
+    } else {
+      Segment& h = p.seg[p.nseg++];
+      h.map = 1;
+      h.row = (layer * a.L + i - d) * a.N + slice * NB;
+      h.nkb = kbh;
+      h.wkb0 = kbh;
+      h.flags = a.flags + (layer * a.L + i - d) * a.S + slice;
+      h.nflags = 1;
+      h.target = a.CL;
     }
-    (void)cell;
   }
   return p;
 }
 
-// map0..map3: activation inputs (boxes of NB rows x 64 columns, 128-byte swizzle).  mapO0/mapO1:
-// outputs (dilated: hs; grid: hx, hy) as un-swizzled boxes of NB rows x this CTA's units; mapT0/mapT1:
-// the same with the row count of the last, partial batch slice.
-template <typename T, int MODE, int NB>
-__device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUtensorMap& map1, const CUtensorMap& map2,
-                                             const CUtensorMap& map3, const CUtensorMap& mapO0,
-                                             const CUtensorMap& mapO1, const CUtensorMap& mapT0,
-                                             const CUtensorMap& mapT1, const ClusterArgs& a, const int rank,
-                                             const int cid, const int layer, const int row_a, const int slice) {
-  constexpr int kEpiWarps = epi_warps(MODE);
+// mapX, mapH: the inputs and the hidden states (boxes of NB rows x 64 columns, 128-byte swizzle).  mapO: the hidden states
+// as un-swizzled boxes of NB rows x this CTA's units; mapT: the same with the row count of the last, partial batch slice.
+template <typename T, int NB>
+__device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapO,
+                                             const CUtensorMap& mapT, const ClusterArgs& a, const int rank, const int cid,
+                                             const int layer, const int slice) {
   constexpr int kSub = kEpiWarps / 4;              // epilogue warps per TMEM lane quadrant
   constexpr int kBlocksPerStage = 128 / NB;        // [NB x 64] 16-bit blocks per 16 KB stage
   constexpr uint32_t kBlockBytes = NB * BK * 2;
-  constexpr int kRing = MODE == kDilated ? 4 : 6;  // stages of the TMA-fed ring when the chain also uses the self slots
-  constexpr int kOutUnits = MODE == kDilated ? 32 : 128;                   // units this CTA produces
+  constexpr int kRing = 4;  // stages of the TMA-fed ring when the chain also uses the self slots
   constexpr uint32_t kOutTileBytes = static_cast<uint32_t>(NB) * kOutUnits * 2;  // row-major [NB][units] staging
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t ring_full[12], ring_empty[12];  // up to 12 ring stages
   __shared__ uint64_t self_full[2];   // the slot holds the whole previous output (bytes counted)
   __shared__ uint64_t self_free[2];   // producers only: every CTA of the cluster has multiplied the slot's contents
-  __shared__ uint64_t stg_ready;      // the eight epilogue warps have written the step's staging tile
+  __shared__ uint64_t stg_ready;      // the epilogue warps have written the step's staging tile
   __shared__ int seg_seq;             // operand segments issued into the ring so far (two producer warps)
   __shared__ int out_issued[2];       // epilogue warps that have staged an even / odd step's outputs, summed over steps
   __shared__ int out_stored;          // steps whose output staging tile the publisher has finished reading
@@ -315,19 +249,15 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   int* status = a.status;
 
   const int kbh = a.H / BK;
-  const int n_wkb = MODE == kDilated ? 2 * kbh : 3 * kbh;  // K blocks of this CTA's weight tile, all in TMEM
+  const int n_wkb = 2 * kbh;  // K blocks of this CTA's weight tile, all in TMEM
   const int K = n_wkb * BK;
   // Does the chain hand its own output to its next step through the cluster's shared memory?
-  const bool self_chain = MODE == kGrid ? true : (a.dil[layer] == 1);
-  // Units of the self operand this CTA produces: dilated: 32 of H; grid: 128 of H, y-direction tiles only.
-  const bool self_producer = self_chain && (MODE == kDilated || rank >= a.CL / 2);
-  const int self_units = MODE == kDilated ? 32 : 128;
-  const int self_first_chunk = (MODE == kDilated ? rank : rank - a.CL / 2) * (self_units / 8);
-  const uint16_t producer_mask = static_cast<uint16_t>(MODE == kDilated ? ((1u << a.CL) - 1u)
-                                                                        : (((1u << a.CL) - 1u) & ~((1u << (a.CL / 2)) - 1u)));
+  const bool self_chain = a.dil[layer] == 1;
+  const int self_first_chunk = rank * (kOutUnits / 8);  // of the self operand, 8 units each: this CTA's
+  const uint16_t producer_mask = static_cast<uint16_t>((1u << a.CL) - 1u);
   const uint32_t self_slot_bytes = static_cast<uint32_t>(a.H / 8) * NB * 16;  // H units x NB rows, 16-bit
-  const uint32_t stage_tile_bytes = MODE == kDilated ? static_cast<uint32_t>(self_units / 8) * NB * 16 : 0u;
-  // Shared memory: [self slot 0][self slot 1][staging 0][staging 1 (dilated)][output tile 0][output tile 1][ring ...];
+  constexpr uint32_t stage_tile_bytes = static_cast<uint32_t>(kOutUnits / 8) * NB * 16;
+  // Shared memory: [self slot 0][self slot 1][staging 0][staging 1][output tile 0][output tile 1][ring ...];
   // chains without a self operand have the output tiles and a longer ring only.
   uint8_t* s_self = smem;
   uint8_t* s_stg = s_self + (self_chain ? 2 * self_slot_bytes : 0);
@@ -338,14 +268,10 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   const int seg_stages = (a.H / BK + kBlocksPerStage - 1) / kBlocksPerStage;
 
   if (threadIdx.x == 0) {
-    prefetch_tmap(&map0);
-    prefetch_tmap(&map1);
-    prefetch_tmap(&map2);
-    prefetch_tmap(&map3);
-    prefetch_tmap(&mapO0);
-    prefetch_tmap(&mapO1);
-    prefetch_tmap(&mapT0);
-    prefetch_tmap(&mapT1);
+    prefetch_tmap(&mapX);
+    prefetch_tmap(&mapH);
+    prefetch_tmap(&mapO);
+    prefetch_tmap(&mapT);
     for (int i = 0; i < 12; ++i) {
       mbar_init(&ring_full[i], 1);
       mbar_init(&ring_empty[i], 1);
@@ -378,9 +304,9 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   const uint32_t tmem_base = tmem_base_s;
   const uint32_t tmem_w = tmem_base + 2 * NB;  // the weight tile sits behind the two accumulators
 
-  const CUtensorMap* maps[4] = {&map0, &map1, &map2, &map3};
+  const CUtensorMap* maps[2] = {&mapX, &mapH};
   const int n_steps = a.L;
-  const int my_flag_cell0 = MODE == kDilated ? (layer * a.L) : ((layer * a.A + row_a) * a.L);
+  const int my_flag_cell0 = layer * a.L;
 
   if (warp == 0 || warp == 3) {
     // ------------------------------------------ producers of the TMA-fed operand blocks
@@ -402,7 +328,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     volatile int* seq = &seg_seq;
     ACCT_DECL(4);
     for (int i = 0; i < n_steps && ok; ++i) {
-      const StepPlan p = plan_step<MODE, NB>(a, layer, row_a, slice, rank, i);
+      const StepPlan p = plan_step<NB>(a, layer, slice, i);
       for (int s = 0; s < p.nseg && ok; ++s) {
         const Segment& sg = p.seg[s];
         if ((s & 1) == mine) {
@@ -417,7 +343,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
             // (Producers write their outputs with TMA stores and consumers read them with TMA loads: both
             // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.
             // Threads store the output of flow::body.)
-            if (MODE == kDilated && a.flow && s == 0 && layer > 0 && a.dil[layer - 1] == 1) fence_proxy_async_all();
+            if (a.flow && s == 0 && layer > 0 && a.dil[layer - 1] == 1) fence_proxy_async_all();
             FTB_CL_STAMP(i, 7 + 2 * s);
             ACCT_BEGIN();
             if (*seq != q) {
@@ -470,9 +396,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_f16(128, NB, Fmt<T>::kind, 0, 0);
       const uint64_t ring_desc0 = make_sdesc_sw128(smem_u32(s_ring), 16, 1024);
-      // (K chunks of 16 bytes, or groups of 8 units, NB * 16 bytes apart; groups of 8 sequences 128)
+      // (K chunks of 16 bytes NB * 16 bytes apart; groups of 8 sequences 128)
       const uint64_t self_desc0 = make_sdesc_plain(smem_u32(s_self), NB * 16, 128);
-      constexpr uint32_t idesc_self = make_idesc_f16(128, NB, Fmt<T>::kind, 0, MODE == kGrid ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = mbar_wait_warp(&res_full, 0, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
@@ -484,21 +409,10 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       // What this thread needs of a step's plan, without the addresses the other roles compute (it is
       // the one thread every MMA of the CTA goes through: its own instructions are the step's floor).
       const int kbh = a.H / BK;
-      const int d_layer = MODE == kDilated ? a.dil[layer] : 1;
+      const int d_layer = a.dil[layer];
       for (int i = 0; i < n_steps && ok; ++i) {
-        int nseg, wkb0[2];
-        bool self;
-        if (MODE == kDilated) {
-          nseg = (d_layer > 1 && i >= d_layer) ? 2 : 1;
-          wkb0[0] = 0;
-          wkb0[1] = kbh;
-          self = d_layer == 1 && i >= 1;
-        } else {
-          nseg = row_a > 0 ? 2 : 1;
-          wkb0[0] = 2 * kbh;  // packed K order of a grid cell: [state_x | state_y | input]
-          wkb0[1] = 0;
-          self = i > 0;
-        }
+        const int nseg = (d_layer > 1 && i >= d_layer) ? 2 : 1;
+        const bool self = d_layer == 1 && i >= 1;
         const int acc = i & 1;
         ACCT_BEGIN();
         ok = mbar_wait_warp(&tempty_bar[acc], ((i >> 1) & 1) ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
@@ -516,7 +430,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           if (!ok) break;
           FTB_CL_STAMP(i, 12 + s);
           const uint64_t bd0 = ring_desc0 + static_cast<uint64_t>((stage * kStageBytes) >> 4);
-          const uint32_t aw = tmem_w + wkb0[s] * 32;
+          const uint32_t aw = tmem_w + s * kbh * 32;
           ACCT_BEGIN();
           for (int kb = 0; kb < kbh; ++kb) {
             if (leader) {
@@ -543,17 +457,11 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
           const int slot = (i - 1) & 1;
           if (leader) mbar_arrive_expect_tx(&self_full[slot], self_slot_bytes);
           ACCT_BEGIN();
-          if (MODE == kGrid) {
-            ok = __all_sync(0xffffffffu, mbar_wait_cluster(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status,
-                                                           FTB_ERR_TIMEOUT_TMA));
-            fence_proxy_async_smem();  // stored by threads, read by the async proxy
-          } else {
-            ok = mbar_wait_warp(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
-          }
+          ok = mbar_wait_warp(&self_full[slot], ((i - 1) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_TMA);
           ACCT_END(2);
           if (!ok) break;
           FTB_CL_STAMP(i, 2);
-          // K = 16 is two 16-byte chunks (two groups of 8 units), NB * 16 bytes apart; the descriptor
+          // K = 16 is two 16-byte chunks, NB * 16 bytes apart; the descriptor
           // of MMA j is the slot's plus j * 2 * NB (bytes / 16): nothing is rebuilt per MMA.
           const uint64_t bd = self_desc0 + static_cast<uint64_t>((slot * self_slot_bytes) >> 4);
           const uint32_t aw = tmem_w + kbh * 32;
@@ -561,7 +469,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
             if (leader) {
 #pragma unroll
               for (int kk = 0; kk < BK / 16; ++kk)
-                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd + static_cast<uint64_t>(kb * 4 + kk) * (2 * NB), idesc_self, 1u);
+                umma_ts(d_tmem, aw + kb * 32 + kk * 8, bd + static_cast<uint64_t>(kb * 4 + kk) * (2 * NB), idesc, 1u);
             }
           }
           if (leader) umma_commit_to(&self_free[slot], producer_mask);
@@ -577,7 +485,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       ACCT_WRITE(2, 10);  // self operand
       ACCT_WRITE(3, 11);  // whole loop
       ACCT_WRITE(4, 15);  // MMA issue (ring operands)
-      if (MODE == kDilated && a.dil[layer] > 1) { ACCT_WRITE(5, 10); }  // commits (the slot of the self operand, unused here)
+      if (a.dil[layer] > 1) { ACCT_WRITE(5, 10); }  // commits (the slot of the self operand, unused here)
     }
   } else if (warp == 2) {
     // ------------------------------------------------ output store and flag publisher
@@ -590,9 +498,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     if (lane == 0) {
       volatile int* stored = &out_stored;
       const int n_valid = min(NB, a.N - slice * NB);
-      const bool ydir = MODE == kGrid && rank >= a.CL / 2;
-      const CUtensorMap* om = n_valid == NB ? (ydir ? &mapO1 : &mapO0) : (ydir ? &mapT1 : &mapT0);
-      const int unit0 = MODE == kDilated ? rank * 32 : (ydir ? rank - a.CL / 2 : rank) * 128;
+      const CUtensorMap* om = n_valid == NB ? &mapO : &mapT;
+      const int unit0 = rank * kOutUnits;
       ACCT_DECL(2);
       for (int i = 0; i < n_steps; ++i) {
         volatile int* issued = &out_issued[i & 1];
@@ -615,16 +522,13 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
         ACCT_END(0);
         ACCT_BEGIN();
         __threadfence_block();
-        const int cell_row = (MODE == kDilated ? (layer * a.L + i) : ((layer * a.A + row_a) * a.L + i)) * a.N + slice * NB;
+        const int cell_row = (layer * a.L + i) * a.N + slice * NB;
         tma_store_2d(om, s_out + (i & 1) * kOutTileBytes, unit0, cell_row);
         tma_store_commit();
         tma_store_wait_read<0>();
         *stored = i + 1;  // the tile may be overwritten (two steps from now)
         tma_store_wait<0>();
-        if (MODE == kDilated)
-          red_release_gpu_add(a.flags + (my_flag_cell0 + i) * a.S + slice, 1);
-        else
-          st_release_gpu(a.flags + ((my_flag_cell0 + i) * a.S + slice) * a.CL + rank, 1);
+        red_release_gpu_add(a.flags + (my_flag_cell0 + i) * a.S + slice, 1);
         ACCT_END(1);
         FTB_CL_STAMP(i, 11);
       }
@@ -633,7 +537,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     }
   } else if (warp >= kFirstEpiWarp) {
     // ---------------------------------------------------------------- epilogue
-    constexpr int kCols = NB / kSub;  // batch columns per warp (32 in both modes)
+    constexpr int kCols = NB / kSub;  // batch columns per warp
     static_assert(kCols == 32 || kCols == 16, "an epilogue warp takes 16 or 32 accumulator columns");
     const int q = warp & 3;
     const int sub = (warp - kFirstEpiWarp) >> 2;
@@ -641,15 +545,8 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     // Resident weights -> TMEM: thread r copies its packed weight row, two 16-bit values per 32-bit
     // column (the layout of an A operand in tensor memory); the warps of a quadrant alternate K blocks.
     {
-      const T* wbase;
-      if (MODE == kDilated) {
-        wbase = reinterpret_cast<const T*>(a.W0) + (static_cast<size_t>(layer) * 4 * a.H + rank * 128 + r_loc) * K;
-      } else {
-        const bool ydir = rank >= a.CL / 2;
-        const int tile = ydir ? rank - a.CL / 2 : rank;
-        wbase = reinterpret_cast<const T*>(ydir ? a.W1 : a.W0) + (static_cast<size_t>(layer) * a.H + tile * 128 + r_loc) * K;
-      }
-      const uint4* wrow = reinterpret_cast<const uint4*>(wbase);
+      const uint4* wrow =
+          reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.W) + (static_cast<size_t>(layer) * 4 * a.H + rank * 128 + r_loc) * K);
       for (int kb = sub; kb < n_wkb; kb += kSub) {
         uint32_t v[32];
 #pragma unroll
@@ -665,35 +562,21 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       if (lane == 0) mbar_arrive(&res_full);
     }
 
-    // Per-thread constants of the two epilogues.
+    // After the quad transpose this thread has all gates of one hidden unit.
     const int gate = lane & 3;
-    int unit;        // hidden unit this thread produces (dilated: after the quad transpose)
-    int u_local;     // the same, counted inside this CTA's tile
+    const int u_local = r_loc >> 2, unit = rank * kOutUnits + u_local;
     float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float bias1 = 0.f;
-    if (MODE == kDilated) {
-      u_local = r_loc >> 2;
-      unit = rank * 32 + u_local;
-      if (a.bias0 != nullptr)
-        bias4 = __ldg(reinterpret_cast<const float4*>(a.bias0 + static_cast<size_t>(layer) * 4 * a.H + rank * 128) + u_local);
-    } else {
-      const bool ydir = rank >= a.CL / 2;
-      u_local = r_loc;
-      unit = (ydir ? rank - a.CL / 2 : rank) * 128 + r_loc;
-      const float* bp = ydir ? a.bias1 : a.bias0;
-      if (bp != nullptr) bias1 = __ldg(bp + static_cast<size_t>(layer) * a.H + unit);
-    }
-    const int dil = MODE == kDilated ? a.dil[layer] : 1;
-    constexpr int kOwn = kCols / 4;  // LSTM: (unit, batch column) elements per thread
+    if (a.bias != nullptr)
+      bias4 = __ldg(reinterpret_cast<const float4*>(a.bias + static_cast<size_t>(layer) * 4 * a.H + rank * 128) + u_local);
+    const int dil = a.dil[layer];
+    constexpr int kOwn = kCols / 4;  // (unit, batch column) elements per thread
     float creg[kOwn];
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) creg[i] = 0.f;
     const int n_valid = min(NB, a.N - slice * NB);  // batch columns of this slice that exist
-    // Where this thread's unit sits (a) in the staging tile (dilated): 16-byte chunk (u_local / 8) of NB rows,
-    // then row n, then the unit's 2 bytes; (b) in the self operand (grid): NB * 16 bytes for 8 units, 128 for
-    // 8 sequences of them, 16 for a unit's; (c) in the row-major output tile.
+    // Where this thread's unit sits (a) in the staging tile: 16-byte chunk (u_local / 8) of NB rows, then row n, then the
+    // unit's 2 bytes; (b) in the row-major output tile.
     const uint32_t stg_unit_off = static_cast<uint32_t>(u_local >> 3) * NB * 16 + (u_local & 7) * 2;
-    const uint32_t self_unit_off = smem_u32(s_self) + static_cast<uint32_t>(unit >> 3) * NB * 16 + (unit & 7) * 16;
     const uint32_t out_unit_off = static_cast<uint32_t>(u_local) * 2;
     volatile int* stored = &out_stored;
     ACCT_DECL(2);
@@ -703,15 +586,15 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       const int acc = i & 1;
       // cell state of a layer with dilation > 1 lives in global memory between the steps that share it
       float* c_rows = nullptr;
-      if (MODE == kDilated && dil > 1)
+      if (dil > 1)
         c_rows = a.c + (static_cast<size_t>(layer) * a.max_dil + (i % dil)) * a.N * a.H + static_cast<size_t>(slice) * NB * a.H;
-      if (MODE == kDilated && dil > 1 && i >= dil) {
+      if (dil > 1 && i >= dil) {
 #pragma unroll
         for (int ci = 0; ci < kOwn; ++ci) {
           const int n = sub * kCols + 4 * ci + gate;
           creg[ci] = n < n_valid ? __ldcg(c_rows + static_cast<size_t>(n) * a.H + unit) : 0.f;
         }
-      } else if (MODE == kDilated && dil > 1) {
+      } else if (dil > 1) {
 #pragma unroll
         for (int ci = 0; ci < kOwn; ++ci) creg[ci] = 0.f;
       }
@@ -751,50 +634,21 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-      if (MODE == kDilated) {
 #pragma unroll
-        for (int kq = 0; kq < kCols / 4; ++kq) {
-          quad_transpose(v[4 * kq], v[4 * kq + 1], v[4 * kq + 2], v[4 * kq + 3], lane);
-          const float gi = v[4 * kq + 0] + bias4.x;
-          const float gf = v[4 * kq + 1] + bias4.y;
-          const float go = v[4 * kq + 2] + bias4.z;
-          const float gc = v[4 * kq + 3] + bias4.w;
-          const float c_new = sigmoid_fast(gf) * creg[kq] + sigmoid_fast(gi) * tanh_fast(gc);
-          creg[kq] = c_new;
-          const T h_new = to_elem<T>(sigmoid_fast(go) * tanh_fast(c_new));
-          const int n = sub * kCols + 4 * kq + gate;
-          *reinterpret_cast<T*>(outp + n * (kOutUnits * 2)) = h_new;
-          if (self_producer) *reinterpret_cast<T*>(stg + n * 16) = h_new;
-        }
-      } else {
-        const bool send = self_producer && i + 1 < n_steps;
-        if (send && i >= 2)  // the slot's last contents have been multiplied everywhere
-          ok = mbar_wait(&self_free[i & 1], ((i - 2) >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
-        if (!__all_sync(0xffffffffu, ok)) {
-          ok = false;
-          break;
-        }
-#pragma unroll
-        for (int g = 0; g < kCols / 8; ++g) {
-          uint32_t row[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            row[k] = Fmt<T>::pack2(tanh_fast(v[8 * g + 2 * k] + bias1), tanh_fast(v[8 * g + 2 * k + 1] + bias1));
-          const int n = sub * kCols + 8 * g;
-          if (send) {
-            const uint32_t dst = self_unit_off + (i & 1) * self_slot_bytes + (n / 8) * 128;
-            const uint32_t bar = smem_u32(&self_full[i & 1]);
-            for (int k = 0; k < a.CL; ++k) {
-              const uint32_t peer = (rank + k) & (a.CL - 1);  // (2 or 4 CTAs)
-              st_async16(map_to_cta(dst, peer), map_to_cta(bar, peer), row);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            *reinterpret_cast<uint16_t*>(outp + (n + k) * (kOutUnits * 2)) = static_cast<uint16_t>(row[k >> 1] >> (16 * (k & 1)));
-        }
+      for (int kq = 0; kq < kCols / 4; ++kq) {
+        quad_transpose(v[4 * kq], v[4 * kq + 1], v[4 * kq + 2], v[4 * kq + 3], lane);
+        const float gi = v[4 * kq + 0] + bias4.x;
+        const float gf = v[4 * kq + 1] + bias4.y;
+        const float go = v[4 * kq + 2] + bias4.z;
+        const float gc = v[4 * kq + 3] + bias4.w;
+        const float c_new = sigmoid_fast(gf) * creg[kq] + sigmoid_fast(gi) * tanh_fast(gc);
+        creg[kq] = c_new;
+        const T h_new = to_elem<T>(sigmoid_fast(go) * tanh_fast(c_new));
+        const int n = sub * kCols + 4 * kq + gate;
+        *reinterpret_cast<T*>(outp + n * (kOutUnits * 2)) = h_new;
+        if (self_chain) *reinterpret_cast<T*>(stg + n * 16) = h_new;
       }
-      if (MODE == kDilated && (dil > 1 || i == n_steps - 1)) {
+      if (dil > 1 || i == n_steps - 1) {
         float* c_out = dil > 1 ? c_rows : a.c + static_cast<size_t>(layer) * a.max_dil * a.N * a.H + static_cast<size_t>(slice) * NB * a.H;
 #pragma unroll
         for (int ci = 0; ci < kOwn; ++ci) {
@@ -806,8 +660,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
       fence_proxy_async_smem();  // plain shared-memory stores -> the bulk copies' and the TMA store's reads
       __syncwarp();
       if (warp == kFirstEpiWarp && lane == 0) { FTB_CL_STAMP(i, 14); }
-      if constexpr (MODE == kDilated)
-      if (self_producer && i + 1 < n_steps) {
+      if (self_chain && i + 1 < n_steps) {
         // Hand the step's output to every CTA of the cluster, once all of them have multiplied what the
         // destination slot held before (two steps ago).
         // Once all epilogue warps have staged their parts, the tile goes to every CTA of the cluster by
@@ -844,7 +697,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
     }
     if (warp == kFirstEpiWarp && lane == 0) { ACCT_WRITE(0, 12); }  // accumulator complete
     // The peers' commits for the last two slots, which no step waits for, have to be in before this CTA leaves (ring_drain, ptx.cuh).
-    if (self_producer && ok && warp == kFirstEpiWarp && lane == 0)
+    if (self_chain && ok && warp == kFirstEpiWarp && lane == 0)
       for (int i = max(0, n_steps - 3); i <= n_steps - 2 && ok; ++i)
         ok = mbar_wait(&self_free[i & 1], (i >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_EPI);
   }
@@ -864,22 +717,6 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& map0, const CUte
   }
 }
 
-// Grid RNN: every cluster has the same shape; cluster -> (layer, grid row, batch slice).
-template <typename T, int MODE, int NB>
-__global__ void __launch_bounds__(cta_threads(MODE), 1)
-rnn_cluster_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
-                   const __grid_constant__ CUtensorMap map2, const __grid_constant__ CUtensorMap map3,
-                   const __grid_constant__ CUtensorMap mapO0, const __grid_constant__ CUtensorMap mapO1,
-                   const __grid_constant__ CUtensorMap mapT0, const __grid_constant__ CUtensorMap mapT1,
-                   const ClusterArgs a) {
-  const int cid = blockIdx.x / a.CL;
-  const int slice = cid % a.S;
-  const int ra = cid / a.S;
-  const int layer = ra / a.A;
-  const int row_a = ra - layer * a.A;
-  cluster_body<T, MODE, NB>(map0, map1, map2, map3, mapO0, mapO1, mapT0, mapT1, a, cluster_ctarank(), cid, layer, row_a, slice);
-}
-
 // Dilated LSTM: a layer's clusters take 64 or 128 sequences each (a.nb[layer]).  A layer whose step
 // depends on its own previous step (dilation 1) is a chain of hand-offs inside the cluster, whose
 // latency grows with the slice (state bytes every CTA receives, accumulator columns per epilogue
@@ -887,7 +724,7 @@ rnn_cluster_kernel(const __grid_constant__ CUtensorMap map0, const __grid_consta
 // x128/h128/o128/t128: the input, the hidden states, the output tile and the output tile of the
 // batch's last (short) slice as boxes of 128 rows; x64... the same with 64 rows.
 template <typename T>
-__global__ void __launch_bounds__(cta_threads(kDilated), 1)
+__global__ void __launch_bounds__(kCtaThreads, 1)
 rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __grid_constant__ CUtensorMap h128,
                            const __grid_constant__ CUtensorMap x64, const __grid_constant__ CUtensorMap h64,
                            const __grid_constant__ CUtensorMap o128, const __grid_constant__ CUtensorMap o64,
@@ -898,9 +735,9 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
   while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
   const int slice = cid - a.first_cluster[layer];
   if (a.nb[layer] == 64)
-    cluster_body<T, kDilated, 64>(x64, h64, h64, h64, o64, o64, t64, t64, a, cluster_ctarank(), cid, layer, 0, slice);
+    cluster_body<T, 64>(x64, h64, o64, t64, a, cluster_ctarank(), cid, layer, slice);
   else
-    cluster_body<T, kDilated, 128>(x128, h128, h128, h128, o128, o128, t128, t128, a, cluster_ctarank(), cid, layer, 0, slice);
+    cluster_body<T, 128>(x128, h128, o128, t128, a, cluster_ctarank(), cid, layer, slice);
 }
 
 // The same program without clusters, where it fits: what the layers with dilation >= 2 exchange goes through
@@ -913,7 +750,7 @@ struct DilatedMaps {
   CUtensorMap nx, nh, nw;                                   // of flow::body
 };
 template <typename T, int kNarrow>
-__global__ void __launch_bounds__(cta_threads(kDilated), 1)
+__global__ void __launch_bounds__(kCtaThreads, 1)
 rnn_dilated_flow_kernel(const __grid_constant__ DilatedMaps m, const __grid_constant__ ClusterArgs a,
                         const __grid_constant__ flow::FlowArgs f) {
   const int cid = blockIdx.x / a.CL, rank = blockIdx.x - cid * a.CL;
@@ -925,10 +762,9 @@ rnn_dilated_flow_kernel(const __grid_constant__ DilatedMaps m, const __grid_cons
     fl.nb_below = layer > 0 ? a.nb[layer - 1] : kNarrow;
     flow::body<T, kNarrow>(m.nx, m.nh, m.nw, fl, rank, slice, layer);
   } else if (a.nb[layer] == 64) {
-    cluster_body<T, kDilated, 64>(m.x64, m.h64, m.h64, m.h64, m.o64, m.o64, m.t64, m.t64, a, rank, cid, layer, 0, slice);
+    cluster_body<T, 64>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
   } else {
-    cluster_body<T, kDilated, 128>(m.x128, m.h128, m.h128, m.h128, m.o128, m.o128, m.t128, m.t128, a, rank, cid, layer, 0,
-                                   slice);
+    cluster_body<T, 128>(m.x128, m.h128, m.o128, m.t128, a, rank, cid, layer, slice);
   }
 }
 
@@ -991,23 +827,17 @@ int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned lon
   return FTB_OK;
 }
 
-template <typename T, int MODE, int NB>
-int launch(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
-  static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_cluster_kernel<T, MODE, NB>, a.CL, cta_threads(MODE), configured, grid, smem_bytes, stream, m[0],
-                       m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
-}
 template <typename T>
 int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, cta_threads(kDilated), configured, grid, smem_bytes, stream, m[0],
+  return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, kCtaThreads, configured, grid, smem_bytes, stream, m[0],
                        m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
 }
 template <typename T, int kNarrow>
 int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs& f, int grid, uint32_t smem_bytes,
                         cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, cta_threads(kDilated), configured, grid, smem_bytes, stream, m,
+  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, kCtaThreads, configured, grid, smem_bytes, stream, m,
                        a, f);
 }
 template <typename T>
@@ -1018,10 +848,11 @@ int launch_dilated_flow(int narrow, const DilatedMaps& m, const ClusterArgs& a, 
   return launch_dilated_flow<T, 48>(m, a, f, grid, smem_bytes, stream);
 }
 
-uint32_t smem_for(bool any_self, int H, int NB, int self_units, int out_units, int ring_self) {
-  // worst case over the chains of the launch; must agree with the kernel's carve-up
-  const uint32_t out_tiles = 2u * NB * out_units * 2;
-  const uint32_t with_self = 2u * (H / 8) * NB * 16 + 2u * (self_units / 8) * NB * 16 + out_tiles + ring_self * kStageBytes;
+uint32_t smem_for(bool any_self, int H) {
+  // worst case over the chains of the launch (slices of 128); must agree with the kernel's carve-up
+  constexpr int NB = 128;
+  const uint32_t out_tiles = 2u * NB * kOutUnits * 2;
+  const uint32_t with_self = 2u * (H / 8) * NB * 16 + 2u * (kOutUnits / 8) * NB * 16 + out_tiles + 4u * kStageBytes;
   const uint32_t without = out_tiles + 12u * kStageBytes;
   return (any_self ? std::max(with_self, without) : without) + 1024;
 }
@@ -1077,7 +908,7 @@ bool dilated_prefers_clusters(int N, int CL) { return (CL == 2 && N <= 64) || (C
 int dilated_max_clusters(int dtype, int cl, uint32_t smem) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl * 32);
-  cfg.blockDim = dim3(cta_threads(kDilated));
+  cfg.blockDim = dim3(kCtaThreads);
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1123,7 +954,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
                                 const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
                                 int sm_count, cudaStream_t stream) {
   ClusterArgs a = {};
-  a.D = D; a.L = L; a.N = N; a.H = H; a.A = 1;
+  a.D = D; a.L = L; a.N = N; a.H = H;
   a.CL = 4 * H / 128;
   a.max_dil = 1;
   bool any_self = false;
@@ -1132,11 +963,11 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     a.max_dil = std::max(a.max_dil, dilations[l]);
     any_self = any_self || dilations[l] == 1;
   }
-  a.W0 = Wp; a.bias0 = bias_p; a.out0 = hs; a.c = c; a.flags = flags; a.status = status;
+  a.W = Wp; a.bias = bias_p; a.out = hs; a.c = c; a.flags = flags; a.status = status;
   const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
   CUtensorMap m[8];
   int rc;
-  const uint32_t cluster_smem = smem_for(any_self, H, 128, 32, 32, 4);
+  const uint32_t cluster_smem = smem_for(any_self, H);
   auto cut_for_clusters = [&] { return dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, cluster_smem), a.nb); };
   int clusters = schedule == 4 || (schedule == 0 && dilated_prefers_clusters(N, a.CL)) ? cut_for_clusters() : 0;
   if (clusters <= 0 && dilated_flow_widths(dilations, D, N, a.CL, sm_count, a.nb)) {
@@ -1172,7 +1003,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     for (int l = 0; l < D; ++l)
       if (dilations[l] == 1 && cudaMemsetAsync(static_cast<char*>(hs) + l * layer_bytes, 0xFF, layer_bytes, stream) != cudaSuccess)
         return FTB_ERR_LAUNCH;
-    const uint32_t smem = smem_for(false, H, 128, 32, 32, 0);
+    const uint32_t smem = smem_for(false, H);
     const int grid = a.first_cluster[D] * a.CL;
     if (dtype == FTB_F16) return launch_dilated_flow<__half>(narrow, dm, a, f, grid, smem, stream);
     return launch_dilated_flow<__nv_bfloat16>(narrow, dm, a, f, grid, smem, stream);
@@ -1197,48 +1028,6 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   const int grid = clusters * a.CL;
   if (dtype == FTB_F16) return launch_dilated<__half>(m, a, grid, cluster_smem, stream);
   return launch_dilated<__nv_bfloat16>(m, a, grid, cluster_smem, stream);
-}
-
-// --------------------------------------------------------------------- grid RNN
-constexpr int kGridNB = 64;
-
-bool grid_rnn_cluster_supported(int dtype, int D, int A, int B, int N, int H, int sm_count) {
-  if (dtype != FTB_F16 && dtype != FTB_BF16) return false;
-  if (H != 128 && H != 256) return false;  // 2 * H / 128 = 2 or 4 CTAs per cluster; 3H/64 K blocks fit TMEM
-  if (D < 1 || A < 1 || B < 1 || N < 1) return false;
-  const int S = (N + kGridNB - 1) / kGridNB;
-  return D * A * S * (2 * H / 128) <= sm_count;
-}
-
-// X,Y: [A,B,N,H]; Wpx,Wpy: [D,H,3H]; hx,hy: [D,A,B,N,H]; flags: D*A*B*S*CL ints (zeroed here).
-int launch_grid_rnn_cluster(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy,
-                            const float* bias_x, const float* bias_y, void* hx, void* hy, int D, int A, int B, int N,
-                            int H, int* flags, int* status, cudaStream_t stream) {
-  ClusterArgs a = {};
-  a.D = D; a.L = B; a.N = N; a.H = H; a.A = A;
-  a.S = (N + kGridNB - 1) / kGridNB;
-  a.CL = 2 * H / 128;
-  a.max_dil = 1;
-  a.W0 = Wpx; a.W1 = Wpy; a.bias0 = bias_x; a.bias1 = bias_y; a.out0 = hx; a.out1 = hy; a.flags = flags; a.status = status;
-  CUtensorMap m[8];
-  int rc;
-  const uint64_t grid_rows = static_cast<uint64_t>(A) * B * N;
-  if ((rc = make_operand_map(&m[0], X, dtype, grid_rows, H, kGridNB))) return rc;
-  if ((rc = make_operand_map(&m[1], Y, dtype, grid_rows, H, kGridNB))) return rc;
-  if ((rc = make_operand_map(&m[2], hx, dtype, grid_rows * D, H, kGridNB))) return rc;
-  if ((rc = make_operand_map(&m[3], hy, dtype, grid_rows * D, H, kGridNB))) return rc;
-  // output boxes: NB (or the last slice's) rows x the 128 units of a CTA, un-swizzled
-  const int tail = N - (a.S - 1) * kGridNB;
-  if ((rc = make_tmap_2d(&m[4], hx, dtype, grid_rows * D, H, H, kGridNB, 128, false))) return rc;
-  if ((rc = make_tmap_2d(&m[5], hy, dtype, grid_rows * D, H, H, kGridNB, 128, false))) return rc;
-  if ((rc = make_tmap_2d(&m[6], hx, dtype, grid_rows * D, H, H, tail, 128, false))) return rc;
-  if ((rc = make_tmap_2d(&m[7], hy, dtype, grid_rows * D, H, H, tail, 128, false))) return rc;
-  const size_t n_flags = static_cast<size_t>(D) * A * B * a.S * a.CL;
-  if (cudaMemsetAsync(flags, 0, sizeof(int) * n_flags, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
-  const int grid = D * A * a.S * a.CL;
-  const uint32_t smem = smem_for(true, H, kGridNB, 0, 128, 6);
-  if (dtype == FTB_F16) return launch<__half, kGrid, kGridNB>(m, a, grid, smem, stream);
-  return launch<__nv_bfloat16, kGrid, kGridNB>(m, a, grid, smem, stream);
 }
 
 }  // namespace ftb

@@ -45,10 +45,6 @@ size_t lstm_dilated_cluster_flag_ints(int D, int L);
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
                                 const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
                                 int sm_count, cudaStream_t stream);
-bool grid_rnn_cluster_supported(int dtype, int D, int A, int B, int N, int H, int sm_count);
-int launch_grid_rnn_cluster(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy,
-                            const float* bias_x, const float* bias_y, void* hx, void* hy, int D, int A, int B, int N,
-                            int H, int* flags, int* status, cudaStream_t stream);
 int launch_cell_simt(int epi, const float* const* act, const int* ld_act, const float* const* w, int ldw,
                      const CellBatch& batch, cudaStream_t stream);
 int pack_lstm(const void* W, const void* U, const void* bias, void* Wp, float* bias_p, int D, int I, int H, int dtype,
@@ -1287,14 +1283,13 @@ int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* 
   const int n_items = 2 * D * A * B;
   const int levels = (D - 1) + (A - 1) + (B - 1) + 1;
   const PlanLayout lay = plan_layout(n_items, 0);
-  // Cluster schedule (the choice when it applies and the workspace has room for its flags behind the
-  // tables): one thread-block cluster per grid row and batch slice, weights resident in tensor
-  // memory, h_y handed to the next column through the cluster's shared memory.
-  if (grid_rnn_cluster_supported(dtype, D, A, B, N, H, cl.sm_count) &&
-      workspace_bytes >= ftb_grid_rnn_workspace_bytes(D, A, B)) {
-    rc = launch_grid_rnn_cluster(dtype, X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy, D, A, B, N, H,
-                                 reinterpret_cast<int*>(static_cast<char*>(workspace) + lay.total), status, stream);
-    if (rc != FTB_ERR_LAUNCH) return rc;  // a refused cooperative cluster launch falls back to the generic wavefront
+  // Weights on chip, states that carry their own arrival (csrc/grid_flow.cu): the choice where it applies and the workspace has
+  // room for its counters behind the tables.
+  GridFlowPlan flow;
+  if (workspace_bytes >= ftb_grid_rnn_workspace_bytes(D, A, B) && grid_flow_plan(dtype, D, A, B, N, H, cl.sm_count, &flow)) {
+    rc = launch_grid_flow(dtype, X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy, D, A, B, N, H, flow,
+                          reinterpret_cast<int*>(static_cast<char*>(workspace) + lay.total), status, stream);
+    if (rc != FTB_ERR_LAUNCH) return rc;  // a refused cooperative launch falls back to the generic wavefront
   }
   const bool persistent = dtype != FTB_F32 && workspace_bytes >= lay.total;
   if (persistent) {
@@ -1519,6 +1514,23 @@ int ftb_rnn_attention_fwd_scratch(const void* src, const void* trg, const void* 
   return launch_attn_finish(dtype, dec, dec_proj, enc_scores, src_lens, out, Lt, Ls, N, H, stream);
 }
 
+int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
+                           const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype, int nb,
+                           void* workspace, size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!X || !Y || !Wpx || !Wpy || !hx || !hy || D <= 0 || A <= 0 || B <= 0 || N <= 0) return FTB_ERR_ARG;
+  if (static_cast<int64_t>(D) * A * B * N > 0x7fffffffLL) return FTB_ERR_ARG;
+  if (!aligned16({X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy})) return FTB_ERR_ALIGN;
+  GridFlowPlan flow;
+  if (!grid_flow_form(dtype, D, A, N, H, current_sm_count(), nb, &flow)) return FTB_ERR_ARG;
+  int* status = nullptr;
+  const int rc = begin_call(workspace, workspace_bytes, stream, &status);
+  if (rc) return rc;
+  if (workspace_bytes < kWorkspaceBytes + sizeof(int) * grid_flow_ints(D, A, B)) return FTB_ERR_WORKSPACE;
+  return launch_grid_flow(dtype, X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy, D, A, B, N, H, flow,
+                          reinterpret_cast<int*>(static_cast<char*>(workspace) + kWorkspaceBytes), status, stream);
+}
+
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {
   if (D <= 0 || A <= 0 || B <= 0) return kWorkspaceBytes;
   return plan_layout(2 * D * A * B, 0).total;
@@ -1526,10 +1538,8 @@ size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {
 
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B) {
   if (D <= 0 || A <= 0 || B <= 0) return kWorkspaceBytes;
-  // tables of the generic persistent schedule, then the flags of the cluster schedule: one per cell,
-  // batch slice and CTA of a cluster; clusters x CTAs never exceed the SM count (taken as <= 256)
-  const size_t per_column = std::max<size_t>(static_cast<size_t>(D) * A * 4, 256);
-  return plan_layout(2 * D * A * B, 0).total + sizeof(int) * per_column * B;
+  // tables of the generic persistent schedule, then the counters of the one with weights on chip
+  return plan_layout(2 * D * A * B, 0).total + sizeof(int) * grid_flow_ints(D, A, B);
 }
 
 int ftb_gemm_nt(const void* A, const void* Bt, void* out, int M, int N, int K, int dtype, const int* tuning,

@@ -303,7 +303,7 @@ def grid_pack_weights(i2h, h2h):
 
 def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
     """X,Y: [A,B,N,H]; Wpx,Wpy: [D,H,3H]; bias fp32 [D,H] -> (hx, hy) each [D,A,B,N,H].
-    schedule: 0 auto (16-bit inputs: the cluster kernel where it applies, else the generic persistent
+    schedule: 0 auto (16-bit inputs: weights on chip where they fit, H up to 256, else the generic persistent
     kernel), 1 one launch per anti-diagonal, 2 the generic persistent kernel."""
     _req(X, "X")
     _req(Y, "Y", X.dtype)
@@ -319,7 +319,7 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
     hx = torch.empty(D, A, B, N, H, dtype=X.dtype, device=X.device)
     hy = torch.empty_like(hx)
     # The library picks the schedule by the room the workspace offers: status word only -> one launch
-    # per level; the tables -> generic persistent kernel; tables and flags -> cluster kernel.
+    # per level; the tables -> generic persistent kernel; tables and counters -> weights on chip.
     ws = workspace(X.device, 0 if schedule == 1 else lib.ftb_grid_rnn_workspace_bytes(D, A, B))
     ws_bytes = {1: lib.ftb_workspace_bytes(), 2: lib.ftb_grid_rnn_tables_bytes(D, A, B)}.get(schedule, ws.numel())
     with _on(X.device), _turn(ws):

@@ -210,19 +210,23 @@ int ftb_grid_pack_weights(const void* i2h, const void* h2h, void* Wp, int H, int
  * Wpx,Wpy: [D,H,3H] from ftb_grid_pack_weights; bias_x,bias_y: fp32 [D,H] or NULL;
  * hx,hy (out): [D,A,B,N,H].  state_x = hx[a-1][b], state_y = hy[a][b-1].
  * Both directions of a level run in one launch.  With ftb_grid_rnn_workspace_bytes(D, A, B)
- * bytes of workspace (16-bit dtypes) the whole grid runs as one launch: for H of 128 or 256 and
- * D*A*ceil(N/64)*(H/64) <= the SM count, the cluster schedule (one thread-block cluster per grid
- * row and slice of 64 sequences walks the columns; weights resident in tensor memory; h_y handed to
- * the next column through the cluster's shared memory; h_x of the row above through global flags);
- * otherwise, or with a workspace of at least ftb_grid_rnn_tables_bytes(D, A, B) but less than
- * ftb_grid_rnn_workspace_bytes(D, A, B) bytes, the generic persistent wavefront, whose schedule
- * tables are copied from host memory on `stream`; with less than that, one launch per level.
+ * bytes of workspace (16-bit dtypes) the whole grid runs as one launch: for H up to 256 with the
+ * weights on chip and states that carry their own arrival (csrc/grid_flow.cu); for wider H, more
+ * than 32 slices of the batch, or with a workspace of at least ftb_grid_rnn_tables_bytes(D, A, B) but
+ * less than ftb_grid_rnn_workspace_bytes(D, A, B) bytes, as the generic persistent wavefront, whose
+ * schedule tables are copied from host memory on `stream`; with less than that, one launch per level.
  * All schedules give the same bits. */
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B);
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B);
 int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
                      const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype,
                      void* workspace, size_t workspace_bytes, void* stream);
+
+/* The same with the weights on chip and slices of nb (16, 32 or 64) sequences; FTB_ERR_ARG where there is
+ * no such form.  Any of the 16-bit schedules gives its bits. */
+int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
+                           const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype, int nb,
+                           void* workspace, size_t workspace_bytes, void* stream);
 
 /* Back-to-back GEMM D = (A.B).C per batch entry, fp32 accumulation, the
  * intermediate rounded to the 16-bit input type.  Stands in for B2BGemm /
