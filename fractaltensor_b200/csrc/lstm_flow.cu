@@ -33,9 +33,8 @@
 //   * the layer below is read through TMA behind a flag per cell (a counter of the tiles stored), which
 //     a warp of its own raises: its fences are off the chain, the layers above just run further behind;
 //   * the input half of step t + 1 is issued right after the recurrent half of step t.
-// The epilogue splits the batch columns so that a thread ends up with four consecutive sequences of
-// its unit (4 x 4 transposes over the quad that holds the unit's gates), keeps their cell state in
-// fp32 registers for the sweep, and two more shuffles make words of four units.
+// A thread reads all gates of its unit for four sequences of every 16 (accumulator fragments, body in lstm_flow.cuh), keeps their
+// cell state in fp32 registers for the sweep, and two shuffles make words of four units.
 //
 // A ragged batch (sorted by decreasing length, rows of a step packed) is the same kernel: the rows of
 // step t start at off[t], and columns whose sequence has ended are neither stored nor waited for.
@@ -260,7 +259,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   if ((rc = make_tmap_3d(&mH, hs, dtype, 64, static_cast<uint64_t>(D) * T, H / BK, static_cast<uint64_t>(H) * 2, 128, 64,
                          held, planes)))
     return rc;
-  if ((rc = make_tmap_2d(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H, I + H, kGateRows, BK))) return rc;
+  if ((rc = make_tmap_gates(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H))) return rc;
   const int64_t chunks = static_cast<int64_t>(D) * T * H / 8;
   const int n_flags = D * L * a.S;
   flow_fill_kernel<<<static_cast<int>(std::min<int64_t>(current_sm_count(), (std::max<int64_t>(chunks, n_flags) + 255) / 256)), 256, 0, stream>>>(

@@ -312,11 +312,11 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         if (ok && lane == 0) {
           if (rank == 0) mbar_arrive_expect_tx(&w_smem, C::kCtas * (n_rec + n_in) * kWBlockBytes);
           for (int b = 0; b < n_rec + n_in; ++b) {
-            const int x = b < n_rec ? a.I + (rec_t + b) * BK : (in_t + b - n_rec) * BK, y = l * 4 * a.H + tile * kGateRows;
+            const int x = b < n_rec ? a.I + (rec_t + b) * BK : (in_t + b - n_rec) * BK, w = (l * 4 * a.H + tile * kGateRows) / 32;
             if constexpr (kPair)
-              tma_load_2d_pair(s_w + b * kWBlockBytes, &mapW, map_to_cta(smem_u32(&w_smem), 0), x, y);
+              tma_load_4d_pair(s_w + b * kWBlockBytes, &mapW, map_to_cta(smem_u32(&w_smem), 0), x, 0, 0, w);
             else
-              tma_load_2d(s_w + b * kWBlockBytes, &mapW, &w_smem, x, y);
+              tma_load_4d(s_w + b * kWBlockBytes, &mapW, &w_smem, x, 0, 0, w);
           }
         }
       }
@@ -416,11 +416,11 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           if (lane == 0) {
             if (rank == 0) mbar_arrive_expect_tx(&ring_full[rs], C::kCtas * kWBlockBytes);
             uint8_t* dst = s_w + (a.held + rs) * kWBlockBytes;
-            const int y = l * 4 * a.H + tile * kGateRows;
+            const int w = (l * 4 * a.H + tile * kGateRows) / 32;
             if constexpr (kPair)
-              tma_load_2d_pair(dst, &mapW, map_to_cta(smem_u32(&ring_full[rs]), 0), b * BK, y);
+              tma_load_4d_pair(dst, &mapW, map_to_cta(smem_u32(&ring_full[rs]), 0), b * BK, 0, 0, w);
             else
-              tma_load_2d(dst, &mapW, &ring_full[rs], b * BK, y);
+              tma_load_4d(dst, &mapW, &ring_full[rs], b * BK, 0, 0, w);
           }
           if (++rs == a.ring) {
             rs = 0;
@@ -432,13 +432,15 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
   } else if (warp >= kFirstEpi && warp < kFirstEpi + C::kWarps) {
     // ------------------------------------------------------- epilogue and state
     const int q = warp & 3, w = warp - kFirstEpi, sub = w >> 2;
-    const int r_loc = q * 32 + lane, gate = lane & 3;
-    const int unit = tile * kUnits + (r_loc >> 2);
+    // The gates of a unit sit in tensor memory 8 lanes apart (8 units of gate i, 8 of f, of o, of c in each quadrant), so that
+    // fragments of 16 lanes leave a thread with all gates of unit lane / 4 and no exchange between threads is needed (against a
+    // 4 x 4 transpose over four lanes for every four columns).
+    const int u_quad = q * 8 + (lane >> 2), unit = tile * kUnits + u_quad;
     const bool ub0 = (lane & 4) != 0, ub1 = (lane & 8) != 0;
-    // After the exchange below this lane stores four units of sequence n_store of each chunk; it keeps the
-    // cell state of four sequences from n_own on.
-    const int n_own = sub * C::kChunks * 16 + 4 * gate;
-    const int n_store = n_own + (ub0 ? 2 : 0) + (ub1 ? 1 : 0);
+    // This lane has sequences n_own, n_own + 1, n_own + 8, n_own + 9 of each chunk of 16; after the exchange below it stores four
+    // units of n_store.
+    const int n_own = sub * C::kChunks * 16 + 2 * (lane & 3);
+    const int n_store = n_own + (ub0 ? 8 : 0) + (ub1 ? 1 : 0);
     // What this lane reads of a state: chunk `lane & 7` of K blocks `part`, part + kParts, .. of rows n_load, n_load + 4, ..
     // (counted in the rows that this CTA holds)
     const int n_load = w * C::kRows + (C::kParts == 1 ? lane >> 3 : (lane >> 3) % C::kSpan);
@@ -453,12 +455,12 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (!ok) break;
       ++sweep;
       {
-        // Weights -> tensor memory: thread r copies packed row r, two 16-bit values per 32-bit column
+        // Weights -> tensor memory: a thread copies one packed row to its lane, two 16-bit values per 32-bit column
         // (the layout of an A operand there); the warps of a quadrant take K blocks in turn.
         const int kb_x = l == 0 ? a.I / BK : kb_h;
         const int in_t = min(C::kTmemBlocks - rec_t, kb_x);
         const T* wrow = reinterpret_cast<const T*>(a.Wp) +
-                        (static_cast<size_t>(l) * 4 * a.H + tile * kGateRows + r_loc) * (a.I + a.H);
+                        (static_cast<size_t>(l) * 4 * a.H + tile * kGateRows + q * 32 + 4 * (lane & 7) + (lane >> 3)) * (a.I + a.H);
         for (int b = sub; b < rec_t + in_t; b += C::kWarps / 4) {
           const uint4* src = reinterpret_cast<const uint4*>(wrow + (b < rec_t ? a.I + b * BK : (b - rec_t) * BK));
           uint32_t v[32];
@@ -477,7 +479,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (sweep == 1) grid_dependency_wait();
       float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias_p != nullptr)
-        bias = __ldg(reinterpret_cast<const float4*>(a.bias_p + static_cast<size_t>(l) * 4 * a.H + tile * kGateRows) + (r_loc >> 2));
+        bias = __ldg(reinterpret_cast<const float4*>(a.bias_p + static_cast<size_t>(l) * 4 * a.H + tile * kGateRows) + u_quad);
       T* hs_l = reinterpret_cast<T*>(a.hs) + static_cast<size_t>(l) * a.T * a.H;
       float creg[C::kChunks][4];
 #pragma unroll
@@ -491,28 +493,27 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         ok = mbar_wait_warp(&acc_full[acc], (k >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after();
-        uint32_t r[C::kChunks][16];
+        uint32_t r_if[C::kChunks][8], r_oc[C::kChunks][8];
 #pragma unroll
-        for (int ch = 0; ch < C::kChunks; ++ch)
-          tmem_ld16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NB + (sub * C::kChunks + ch) * 16, r[ch]);
+        for (int ch = 0; ch < C::kChunks; ++ch) {
+          const uint32_t at = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NB + (sub * C::kChunks + ch) * 16;
+          tmem_ld_frag16(at, r_if[ch]);
+          tmem_ld_frag16(at + (16u << 16), r_oc[ch]);
+        }
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive_at_issuer(&acc_empty[acc]);
 #pragma unroll
         for (int ch = 0; ch < C::kChunks; ++ch) {
-          float v[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[ch][i]);
           float h[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            // lane q of a quad: gate q of sequences i, 4 + i, 8 + i, 12 + i -> all gates of sequence 4 q + i
-            quad_transpose(v[i], v[4 + i], v[8 + i], v[12 + i], lane);
-            const float gi = v[i] + bias.x;
-            const float gf = v[4 + i] + bias.y;
-            const float go = v[8 + i] + bias.z;
-            const float gc = v[12 + i] + bias.w;
+            const int at = 4 * (i >> 1) + (i & 1);
+            const float gi = __uint_as_float(r_if[ch][at]) + bias.x;
+            const float gf = __uint_as_float(r_if[ch][at + 2]) + bias.y;
+            const float go = __uint_as_float(r_oc[ch][at]) + bias.z;
+            const float gc = __uint_as_float(r_oc[ch][at + 2]) + bias.w;
             const float c_new = sigmoid_fast(gf) * creg[ch][i] + sigmoid_fast(gi) * tanh_fast(gc);
             creg[ch][i] = c_new;
             h[i] = sigmoid_fast(go) * tanh_fast(c_new);
@@ -611,7 +612,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           for (int ch = 0; ch < C::kChunks; ++ch)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const int n = n_base + n_own + ch * 16 + i;
+              const int n = n_base + n_own + ch * 16 + 8 * (i >> 1) + (i & 1);
               if (n < now.active && n >= next.active)
                 a.c_out[(static_cast<size_t>(l) * a.c_rows + n) * a.H + unit] = creg[ch][i];
             }

@@ -991,7 +991,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     const uint32_t planes = 128 / narrow;  // of a copy of flow::body
     if ((rc = make_tmap_3d(&dm.nx, x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
     if ((rc = make_tmap_3d(&dm.nh, hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
-    if ((rc = make_tmap_2d(&dm.nw, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H, 2 * H, flow::kGateRows, 64))) return rc;
+    if ((rc = make_tmap_gates(&dm.nw, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H))) return rc;
     flow::FlowArgs f = {};
     f.D = D; f.L = L; f.N = N; f.I = H; f.H = H; f.G = D; f.S = a.S;
     f.n_tiles = a.CL;

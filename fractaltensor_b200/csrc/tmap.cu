@@ -72,6 +72,21 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, u
   return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
 }
 
+int make_tmap_gates(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t K) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return FTB_ERR_DRIVER;
+  const size_t row = K * dtype_size(dtype);
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row & 15)) return FTB_ERR_ALIGN;
+  if (rows % 32 != 0) return FTB_ERR_ARG;
+  cuuint64_t dims[4] = {K, 8, 4, rows / 32};
+  cuuint64_t strides[3] = {4 * row, row, 32 * row};
+  cuuint32_t box[4] = {64, 8, 4, 4};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(out, tmap_dtype(dtype), 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
+}
+
 namespace {
 // What a device is does not change: its attributes are asked for once (0 = not asked yet).  Devices
 // past the table are asked on every call.
