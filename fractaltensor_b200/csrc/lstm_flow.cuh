@@ -62,19 +62,6 @@ __device__ __forceinline__ Rows rows_of(const FlowArgs& a, int t) {
   return {r0, __ldg(a.off + t + 1) - r0};
 }
 
-__device__ __forceinline__ void quad_transpose(float& a0, float& a1, float& a2, float& a3, int lane) {
-  const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
-  float r;
-  r = __shfl_xor_sync(0xffffffffu, b0 ? a0 : a1, 1);
-  if (b0) a0 = r; else a1 = r;
-  r = __shfl_xor_sync(0xffffffffu, b0 ? a2 : a3, 1);
-  if (b0) a2 = r; else a3 = r;
-  r = __shfl_xor_sync(0xffffffffu, b1 ? a0 : a2, 2);
-  if (b1) a0 = r; else a2 = r;
-  r = __shfl_xor_sync(0xffffffffu, b1 ? a1 : a3, 2);
-  if (b1) a1 = r; else a3 = r;
-}
-
 __device__ __forceinline__ void st_relaxed_gpu64(void* p, uint32_t lo, uint32_t hi) {
   const uint64_t v = static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32);
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");

@@ -41,10 +41,9 @@ namespace {
 
 constexpr int BK = 64;
 constexpr int kFirstEpiWarp = 4;
-// Epilogue warps: four per TMEM lane quadrant (five MUFU operations and a quad transpose per element:
-// latency-bound with fewer).
-constexpr int kEpiWarps = 16;
-constexpr int kCtaThreads = 32 * (kFirstEpiWarp + kEpiWarps);
+// Epilogue warps: four per TMEM lane quadrant (five MUFU operations per element: latency-bound with fewer).
+constexpr int kAllEpiWarps = 16;
+constexpr int kCtaThreads = 32 * (kFirstEpiWarp + kAllEpiWarps);
 constexpr int kOutUnits = 32;  // hidden units of a CTA
 constexpr uint32_t kStageBytes = 16384;
 
@@ -126,12 +125,6 @@ __device__ __forceinline__ bool warp_wait_flags(const int* flags, int n, int tar
   }
 }
 
-template <int N>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
-  if constexpr (N == 32) tmem_ld32(taddr, r);
-  else tmem_ld16(taddr, r);
-}
-
 // Shared-memory operand descriptor for an un-swizzled K-major tile: core matrices of 8 rows x 16 B
 // stored contiguously (128 B); `lbo` = bytes between the two 16-byte K chunks of an MMA's K = 16,
 // `sbo` = bytes between consecutive 8-row groups.
@@ -162,15 +155,6 @@ __device__ __forceinline__ void umma_commit_to(uint64_t* bar, uint16_t mask) {
       "h"(mask)
       : "memory");
 }
-
-using flow::quad_transpose;
-
-template <typename T>
-__device__ __forceinline__ T to_elem(float v);
-template <>
-__device__ __forceinline__ __half to_elem<__half>(float v) { return __float2half_rn(v); }
-template <>
-__device__ __forceinline__ __nv_bfloat16 to_elem<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
 // What this CTA multiplies at time step `i` of its chain (layer, slice).  Every role calls it with the same arguments.
 template <int NB>
@@ -220,12 +204,15 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
 }
 
 // mapX, mapH: the inputs and the hidden states (boxes of NB rows x 64 columns, 128-byte swizzle).  mapO: the hidden states
-// as un-swizzled boxes of NB rows x this CTA's units; mapT: the same with the row count of the last, partial batch slice.
-template <typename T, int NB>
+// as 64-byte-swizzled boxes of NB rows x this CTA's units; mapT: the same with the row count of the last, partial batch slice.
+// kSplit: the even steps are the first eight epilogue warps', the odd ones the others', so that what a step waits for (accumulator,
+// cell state, output tile) is covered by the other half's work.  For even dilations: a cell state then stays one half's.
+template <typename T, int NB, bool kSplit>
 __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapO,
                                              const CUtensorMap& mapT, const ClusterArgs& a, const int rank, const int cid,
                                              const int layer, const int slice) {
-  constexpr int kSub = kEpiWarps / 4;              // epilogue warps per TMEM lane quadrant
+  constexpr int kEpiWarps = kSplit ? kAllEpiWarps / 2 : kAllEpiWarps;  // of a step
+  constexpr int kSub = kEpiWarps / 4;              // of them per TMEM lane quadrant
   constexpr int kBlocksPerStage = 128 / NB;        // [NB x 64] 16-bit blocks per 16 KB stage
   constexpr uint32_t kBlockBytes = NB * BK * 2;
   constexpr int kRing = 4;  // stages of the TMA-fed ring when the chain also uses the self slots
@@ -288,7 +275,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
     mbar_init(&tfull_bar[1], 1);
     mbar_init(&tempty_bar[0], kEpiWarps);
     mbar_init(&tempty_bar[1], kEpiWarps);
-    mbar_init(&res_full, kEpiWarps);
+    mbar_init(&res_full, kAllEpiWarps);
     s_abort = 0;
     fence_barrier_init();
   }
@@ -537,17 +524,18 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
     }
   } else if (warp >= kFirstEpiWarp) {
     // ---------------------------------------------------------------- epilogue
-    constexpr int kCols = NB / kSub;  // batch columns per warp
-    static_assert(kCols == 32 || kCols == 16, "an epilogue warp takes 16 or 32 accumulator columns");
-    const int q = warp & 3;
-    const int sub = (warp - kFirstEpiWarp) >> 2;
-    const int r_loc = q * 32 + lane;  // row of the 128-row tile = TMEM lane
-    // Resident weights -> TMEM: thread r copies its packed weight row, two 16-bit values per 32-bit
-    // column (the layout of an A operand in tensor memory); the warps of a quadrant alternate K blocks.
+    constexpr int kCols = NB / kSub;          // batch columns of a warp
+    constexpr int kRound = kCols < 32 ? kCols : 32;  // of them in registers at a time
+    static_assert(kCols % 16 == 0 && kCols % kRound == 0, "columns come in fragments of 16");
+    const int q = warp & 3, e = warp - kFirstEpiWarp;
+    const int half = kSplit ? e >> 3 : 0, sub = kSplit ? (e & 7) >> 2 : e >> 2;
+    // Resident weights -> TMEM: a thread copies one packed weight row to its lane, two 16-bit values per 32-bit
+    // column (the layout of an A operand in tensor memory); the warps of a quadrant alternate K blocks.  The gates of
+    // a unit are put 8 lanes apart, so that fragments of 16 lanes leave a thread with all of them (csrc/lstm_flow.cuh).
     {
       const uint4* wrow =
-          reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.W) + (static_cast<size_t>(layer) * 4 * a.H + rank * 128 + r_loc) * K);
-      for (int kb = sub; kb < n_wkb; kb += kSub) {
+          reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.W) + (static_cast<size_t>(layer) * 4 * a.H + rank * 128 + q * 32 + 4 * (lane & 7) + (lane >> 3)) * K);
+      for (int kb = e >> 2; kb < n_wkb; kb += kAllEpiWarps / 4) {
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -562,9 +550,13 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
       if (lane == 0) mbar_arrive(&res_full);
     }
 
-    // After the quad transpose this thread has all gates of one hidden unit.
-    const int gate = lane & 3;
-    const int u_local = r_loc >> 2, unit = rank * kOutUnits + u_local;
+    const int u_local = q * 8 + (lane >> 2), unit = rank * kOutUnits + u_local;
+    const bool ub0 = (lane & 4) != 0, ub1 = (lane & 8) != 0;
+    // This thread has batch columns n_own, n_own + 1, n_own + 8, n_own + 9 of every 16; after the exchange below it stores four
+    // units of column n_store.
+    const int n_own = sub * kCols + 2 * (lane & 3);
+    const int n_store = n_own + (ub0 ? 8 : 0) + (ub1 ? 1 : 0);
+    auto own = [&](int ci) { return n_own + (ci >> 2) * 16 + ((ci >> 1) & 1) * 8 + (ci & 1); };
     float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.bias != nullptr)
       bias4 = __ldg(reinterpret_cast<const float4*>(a.bias + static_cast<size_t>(layer) * 4 * a.H + rank * 128) + u_local);
@@ -574,26 +566,23 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
 #pragma unroll
     for (int i = 0; i < kOwn; ++i) creg[i] = 0.f;
     const int n_valid = min(NB, a.N - slice * NB);  // batch columns of this slice that exist
-    // Where this thread's unit sits (a) in the staging tile: 16-byte chunk (u_local / 8) of NB rows, then row n, then the
-    // unit's 2 bytes; (b) in the row-major output tile.
-    const uint32_t stg_unit_off = static_cast<uint32_t>(u_local >> 3) * NB * 16 + (u_local & 7) * 2;
-    const uint32_t out_unit_off = static_cast<uint32_t>(u_local) * 2;
+    // Where this thread's four units of column n sit (a) in the staging tile: 16-byte chunk q of NB rows, then row n, then
+    // 8 bytes; (b) in the row-major output tile of 64-byte rows, 16-byte chunks swizzled by the row.
+    const uint32_t stg_off = static_cast<uint32_t>(q) * NB * 16 + (lane >> 4) * 8;
+    const uint32_t out_off = ((q ^ ((n_store >> 1) & 3)) << 4) + (lane >> 4) * 8;  // (rows 16 apart are swizzled alike)
     volatile int* stored = &out_stored;
     ACCT_DECL(2);
 
     bool ok = true;
-    for (int i = 0; i < n_steps && ok; ++i) {
+    for (int i = half; i < n_steps && ok; i += kSplit ? 2 : 1) {
       const int acc = i & 1;
       // cell state of a layer with dilation > 1 lives in global memory between the steps that share it
       float* c_rows = nullptr;
       if (dil > 1)
-        c_rows = a.c + (static_cast<size_t>(layer) * a.max_dil + (i % dil)) * a.N * a.H + static_cast<size_t>(slice) * NB * a.H;
+        c_rows = a.c + (static_cast<size_t>(layer) * a.max_dil + (i % dil)) * a.N * a.H + static_cast<size_t>(slice) * NB * a.H + unit;
       if (dil > 1 && i >= dil) {
 #pragma unroll
-        for (int ci = 0; ci < kOwn; ++ci) {
-          const int n = sub * kCols + 4 * ci + gate;
-          creg[ci] = n < n_valid ? __ldcg(c_rows + static_cast<size_t>(n) * a.H + unit) : 0.f;
-        }
+        for (int ci = 0; ci < kOwn; ++ci) creg[ci] = own(ci) < n_valid ? __ldcg(c_rows + static_cast<size_t>(own(ci)) * a.H) : 0.f;
       } else if (dil > 1) {
 #pragma unroll
         for (int ci = 0; ci < kOwn; ++ci) creg[ci] = 0.f;
@@ -620,41 +609,56 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
       tc_fence_after();
       if (warp == kFirstEpiWarp && lane == 0) { FTB_CL_STAMP(i, 4); }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NB + sub * kCols;
-      uint8_t* stg = s_stg + (i & 1) * stage_tile_bytes + stg_unit_off;
-      uint8_t* outp = s_out + (i & 1) * kOutTileBytes + out_unit_off;
-      float v[kCols];
-      {
-        uint32_t r[kCols];
-        tmem_ld_cols<kCols>(taddr, r);
+      uint8_t* stg = s_stg + (i & 1) * stage_tile_bytes + stg_off;
+      uint8_t* outp = s_out + (i & 1) * kOutTileBytes + out_off;
+#pragma unroll
+      for (int r0 = 0; r0 < kCols; r0 += kRound) {
+        uint32_t r_if[kRound / 16][8], r_oc[kRound / 16][8];
+#pragma unroll
+        for (int ch = 0; ch < kRound / 16; ++ch) {
+          tmem_ld_frag16(taddr + r0 + ch * 16, r_if[ch]);
+          tmem_ld_frag16(taddr + r0 + ch * 16 + (16u << 16), r_oc[ch]);
+        }
         tmem_ld_wait();
+        if (r0 + kRound == kCols) {
+          // the accumulator is in registers: the MMA issuer may reuse it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+        }
 #pragma unroll
-        for (int k = 0; k < kCols; ++k) v[k] = __uint_as_float(r[k]);
-      }
-      // the accumulator is in registers: the MMA issuer may reuse it
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+        for (int ch = 0; ch < kRound / 16; ++ch) {
+          float h[4];
 #pragma unroll
-      for (int kq = 0; kq < kCols / 4; ++kq) {
-        quad_transpose(v[4 * kq], v[4 * kq + 1], v[4 * kq + 2], v[4 * kq + 3], lane);
-        const float gi = v[4 * kq + 0] + bias4.x;
-        const float gf = v[4 * kq + 1] + bias4.y;
-        const float go = v[4 * kq + 2] + bias4.z;
-        const float gc = v[4 * kq + 3] + bias4.w;
-        const float c_new = sigmoid_fast(gf) * creg[kq] + sigmoid_fast(gi) * tanh_fast(gc);
-        creg[kq] = c_new;
-        const T h_new = to_elem<T>(sigmoid_fast(go) * tanh_fast(c_new));
-        const int n = sub * kCols + 4 * kq + gate;
-        *reinterpret_cast<T*>(outp + n * (kOutUnits * 2)) = h_new;
-        if (self_chain) *reinterpret_cast<T*>(stg + n * 16) = h_new;
+          for (int k = 0; k < 4; ++k) {
+            const int at = 4 * (k >> 1) + (k & 1);
+            float& c = creg[r0 / 4 + ch * 4 + k];
+            const float gi = __uint_as_float(r_if[ch][at]) + bias4.x;
+            const float gf = __uint_as_float(r_if[ch][at + 2]) + bias4.y;
+            const float go = __uint_as_float(r_oc[ch][at]) + bias4.z;
+            const float gc = __uint_as_float(r_oc[ch][at + 2]) + bias4.w;
+            const float c_new = sigmoid_fast(gf) * c + sigmoid_fast(gi) * tanh_fast(gc);
+            c = c_new;
+            h[k] = sigmoid_fast(go) * tanh_fast(c_new);
+          }
+          // (unit, 4 sequences) -> (4 units, 1 sequence): trade halves with the units next to this one, twice
+          const uint32_t p01 = Fmt<T>::pack2(h[0], h[1]), p23 = Fmt<T>::pack2(h[2], h[3]);
+          uint32_t other = __shfl_xor_sync(0xffffffffu, ub0 ? p01 : p23, 4);
+          const uint32_t lo = ub0 ? other : p01, hi = ub0 ? p23 : other;  // units u & ~1 and u | 1
+          const uint32_t w0 = __byte_perm(lo, hi, 0x5410), w1 = __byte_perm(lo, hi, 0x7632);
+          other = __shfl_xor_sync(0xffffffffu, ub1 ? w0 : w1, 8);
+          const uint2 word = ub1 ? make_uint2(other, w1) : make_uint2(w0, other);
+          const int n = n_store + r0 + ch * 16;
+          *reinterpret_cast<uint2*>(outp + n * (kOutUnits * 2)) = word;
+          if (self_chain) *reinterpret_cast<uint2*>(stg + n * 16) = word;
+        }
       }
       if (dil > 1 || i == n_steps - 1) {
-        float* c_out = dil > 1 ? c_rows : a.c + static_cast<size_t>(layer) * a.max_dil * a.N * a.H + static_cast<size_t>(slice) * NB * a.H;
+        float* c_out = dil > 1 ? c_rows
+                               : a.c + static_cast<size_t>(layer) * a.max_dil * a.N * a.H + static_cast<size_t>(slice) * NB * a.H + unit;
 #pragma unroll
-        for (int ci = 0; ci < kOwn; ++ci) {
-          const int n = sub * kCols + 4 * ci + gate;
-          if (n < n_valid) c_out[static_cast<size_t>(n) * a.H + unit] = creg[ci];
-        }
+        for (int ci = 0; ci < kOwn; ++ci)
+          if (own(ci) < n_valid) c_out[static_cast<size_t>(own(ci)) * a.H] = creg[ci];
       }
       if (warp == kFirstEpiWarp && lane == 0) { FTB_CL_STAMP(i, 5); }
       fence_proxy_async_smem();  // plain shared-memory stores -> the bulk copies' and the TMA store's reads
@@ -734,10 +738,15 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
   int layer = 0;
   while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
   const int slice = cid - a.first_cluster[layer];
-  if (a.nb[layer] == 64)
-    cluster_body<T, 64>(x64, h64, o64, t64, a, cluster_ctarank(), cid, layer, slice);
-  else
-    cluster_body<T, 128>(x128, h128, o128, t128, a, cluster_ctarank(), cid, layer, slice);
+  const int rank = cluster_ctarank();
+  const bool split = a.dil[layer] % 2 == 0;
+  if (a.nb[layer] == 64) {
+    if (split) cluster_body<T, 64, true>(x64, h64, o64, t64, a, rank, cid, layer, slice);
+    else cluster_body<T, 64, false>(x64, h64, o64, t64, a, rank, cid, layer, slice);
+  } else {
+    if (split) cluster_body<T, 128, true>(x128, h128, o128, t128, a, rank, cid, layer, slice);
+    else cluster_body<T, 128, false>(x128, h128, o128, t128, a, rank, cid, layer, slice);
+  }
 }
 
 // The same program without clusters, where it fits: what the layers with dilation >= 2 exchange goes through
@@ -761,10 +770,15 @@ rnn_dilated_flow_kernel(const __grid_constant__ DilatedMaps m, const __grid_cons
     flow::FlowArgs fl = f;
     fl.nb_below = layer > 0 ? a.nb[layer - 1] : kNarrow;
     flow::body<T, kNarrow>(m.nx, m.nh, m.nw, fl, rank, slice, layer);
-  } else if (a.nb[layer] == 64) {
-    cluster_body<T, 64>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
+    return;
+  }
+  const bool split = a.dil[layer] % 2 == 0;
+  if (a.nb[layer] == 64) {
+    if (split) cluster_body<T, 64, true>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
+    else cluster_body<T, 64, false>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
   } else {
-    cluster_body<T, 128>(m.x128, m.h128, m.o128, m.t128, a, rank, cid, layer, slice);
+    if (split) cluster_body<T, 128, true>(m.x128, m.h128, m.o128, m.t128, a, rank, cid, layer, slice);
+    else cluster_body<T, 128, false>(m.x128, m.h128, m.o128, m.t128, a, rank, cid, layer, slice);
   }
 }
 
@@ -780,7 +794,7 @@ template <typename Kernel, typename... Args>
 int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned long long>& configured, int grid,
                   uint32_t smem_bytes, cudaStream_t stream, const Args&... args) {
   // the largest request of this instantiation (static shared memory comes on top of it)
-  constexpr int kMaxDynamic = 226 * 1024;
+  constexpr int kMaxDynamic = 225 * 1024;
   if (smem_bytes > static_cast<uint32_t>(kMaxDynamic) || !ensure_dynamic_smem(kfn, kMaxDynamic, configured))
     return FTB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
@@ -921,11 +935,11 @@ int dilated_max_clusters(int dtype, int cl, uint32_t smem) {
   cudaError_t e;
   if (dtype == FTB_F16) {
     static std::atomic<unsigned long long> configured{0};
-    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__half>, 226 * 1024, configured)) return 0;
+    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__half>, 225 * 1024, configured)) return 0;
     e = cudaOccupancyMaxActiveClusters(&n, rnn_cluster_dilated_kernel<__half>, &cfg);
   } else {
     static std::atomic<unsigned long long> configured{0};
-    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__nv_bfloat16>, 226 * 1024, configured)) return 0;
+    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__nv_bfloat16>, 225 * 1024, configured)) return 0;
     e = cudaOccupancyMaxActiveClusters(&n, rnn_cluster_dilated_kernel<__nv_bfloat16>, &cfg);
   }
   if (e != cudaSuccess) {
@@ -984,8 +998,8 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
       const int tail = N - ((N + wide - 1) / wide - 1) * wide;
       if ((rc = make_operand_map(wide == 64 ? &dm.x64 : &dm.x128, x, dtype, x_rows, H, wide))) return rc;
       if ((rc = make_operand_map(wide == 64 ? &dm.h64 : &dm.h128, hs, dtype, h_rows, H, wide))) return rc;
-      if ((rc = make_tmap_2d(wide == 64 ? &dm.o64 : &dm.o128, hs, dtype, h_rows, H, H, wide, 32, false))) return rc;
-      if ((rc = make_tmap_2d(wide == 64 ? &dm.t64 : &dm.t128, hs, dtype, h_rows, H, H, tail, 32, false))) return rc;
+      if ((rc = make_tmap_2d_sw64(wide == 64 ? &dm.o64 : &dm.o128, hs, dtype, h_rows, H, H, wide))) return rc;
+      if ((rc = make_tmap_2d_sw64(wide == 64 ? &dm.t64 : &dm.t128, hs, dtype, h_rows, H, H, tail))) return rc;
     }
     const uint64_t row_bytes = static_cast<uint64_t>(H) * 2;
     const uint32_t planes = 128 / narrow;  // of a copy of flow::body
@@ -1017,12 +1031,12 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   if ((rc = make_operand_map(&m[1], hs, dtype, h_rows, H, 128))) return rc;
   if ((rc = make_operand_map(&m[2], x, dtype, x_rows, H, 64))) return rc;
   if ((rc = make_operand_map(&m[3], hs, dtype, h_rows, H, 64))) return rc;
-  // output boxes: the slice's (or the last, short slice's) rows x the 32 units of a CTA, un-swizzled
+  // output boxes: the slice's (or the last, short slice's) rows x the 32 units of a CTA
   const int tail128 = N - ((N + 127) / 128 - 1) * 128, tail64 = N - ((N + 63) / 64 - 1) * 64;
-  if ((rc = make_tmap_2d(&m[4], hs, dtype, h_rows, H, H, 128, 32, false))) return rc;
-  if ((rc = make_tmap_2d(&m[5], hs, dtype, h_rows, H, H, 64, 32, false))) return rc;
-  if ((rc = make_tmap_2d(&m[6], hs, dtype, h_rows, H, H, tail128, 32, false))) return rc;
-  if ((rc = make_tmap_2d(&m[7], hs, dtype, h_rows, H, H, tail64, 32, false))) return rc;
+  if ((rc = make_tmap_2d_sw64(&m[4], hs, dtype, h_rows, H, H, 128))) return rc;
+  if ((rc = make_tmap_2d_sw64(&m[5], hs, dtype, h_rows, H, H, 64))) return rc;
+  if ((rc = make_tmap_2d_sw64(&m[6], hs, dtype, h_rows, H, H, tail128))) return rc;
+  if ((rc = make_tmap_2d_sw64(&m[7], hs, dtype, h_rows, H, H, tail64))) return rc;
   const size_t n_flags = static_cast<size_t>(D) * L * a.S;
   if (cudaMemsetAsync(flags, 0, sizeof(int) * n_flags, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
   const int grid = clusters * a.CL;

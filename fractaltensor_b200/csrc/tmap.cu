@@ -35,21 +35,33 @@ CUtensorMapDataType tmap_dtype(int dt) {
 }
 }  // namespace
 
-int make_tmap_2d(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld,
-                 uint32_t box_rows, uint32_t box_cols, bool swizzle128) {
+namespace {
+int encode_2d(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
+              uint32_t box_cols, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return FTB_ERR_DRIVER;
   const size_t es = dtype_size(dtype);
   if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld * es) & 15)) return FTB_ERR_ALIGN;
-  if (box_rows > 256 || box_cols > 256 || (swizzle128 && box_cols * es > 128)) return FTB_ERR_ARG;
+  if (box_rows > 256 || box_cols > 256 || (swizzle == CU_TENSOR_MAP_SWIZZLE_128B && box_cols * es > 128)) return FTB_ERR_ARG;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * es};
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(out, tmap_dtype(dtype), 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
+}
+}  // namespace
+
+int make_tmap_2d(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld,
+                 uint32_t box_rows, uint32_t box_cols, bool swizzle128) {
+  return encode_2d(out, base, dtype, rows, cols, ld, box_rows, box_cols,
+                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+int make_tmap_2d_sw64(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld,
+                      uint32_t box_rows) {
+  return encode_2d(out, base, dtype, rows, cols, ld, box_rows, static_cast<uint32_t>(64 / dtype_size(dtype)), CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, uint64_t rows, uint64_t planes,

@@ -21,6 +21,9 @@ inline size_t dtype_size(int dt) { return dt == FTB_F32 ? 4 : 2; }
 // times the element size must be 128 bytes or less.  Returns 0 on success.
 int make_tmap_2d(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld,
                  uint32_t box_rows, uint32_t box_cols, bool swizzle128 = true);
+// The same with 64-byte rows in the 64-byte swizzle (16-byte piece p of row r at p ^ (r / 2 % 4)).
+int make_tmap_2d_sw64(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t cols, uint64_t ld,
+                      uint32_t box_rows);
 
 // 3-D variant: dims (cols, rows, planes) with byte strides for rows and planes.
 int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, uint64_t rows, uint64_t planes,
