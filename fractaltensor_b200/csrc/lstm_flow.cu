@@ -75,7 +75,7 @@ lstm_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
                  const __grid_constant__ CUtensorMap mapW, const FlowArgs a) {
   const int tile = blockIdx.x % a.n_tiles;
   const int slice = (blockIdx.x / a.n_tiles) % a.S;
-  body<T, NB, kPair, kStream>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S));
+  body<T, NB, kPair, kStream>(mapX, mapH, mapW, a, tile, slice, blockIdx.x / (a.n_tiles * a.S), NB);
 }
 
 template <typename T, int NB, bool kPair, bool kStream = false>
@@ -232,7 +232,7 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int
 int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* off,
                      int64_t T, int D, int L, int N, int I, int H, const FlowPlan& plan, int* flags, int* status,
                      cudaStream_t stream) {
-  FlowArgs a;
+  FlowArgs a = {};
   const bool pair = plan.pair;
   const Fit f = fit(plan.nb, pair, I, H);
   if (f.slots < 1) return FTB_ERR_ARG;
@@ -249,7 +249,7 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   a.hs = hs;
   a.c_out = c;
   a.c_rows = N;
-  a.nb_below = plan.nb;
+  a.flag_steps = L;
   a.flags = flags;
   a.status = status;
   const uint32_t nb = plan.nb, held = pair ? nb / 2 : nb, planes = 128 / nb;

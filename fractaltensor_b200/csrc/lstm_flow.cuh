@@ -47,7 +47,10 @@ struct FlowArgs {
   float* c_out;         // [D, c_rows, H], the first N of c_rows
   int c_rows;
   int* flags;           // [D * L * S] tiles of the slice's cell (l, t) that can be read through TMA
-  int nb_below;         // sequences of a slice of the layer below
+  // A layer of the dilated LSTM whose step is `fold` time steps of N1 sequences (N = fold * N1, the last step may be short).
+  // fold 0: a step is a time step in every layer.
+  int fold, N1;
+  int flag_steps;       // cells of a layer in `flags`
   int* status;
 };
 
@@ -56,7 +59,10 @@ struct Rows {  // rows of a step: the first one and how many sequences still run
   int active;
 };
 __device__ __forceinline__ Rows rows_of(const FlowArgs& a, int t) {
-  if (a.off == nullptr) return {static_cast<int64_t>(t) * a.N, t < a.L ? a.N : 0};
+  if (a.off == nullptr) {
+    const int64_t first = static_cast<int64_t>(t) * a.N;
+    return {first, t < a.L ? static_cast<int>(min(static_cast<int64_t>(a.N), a.T - first)) : 0};
+  }
   if (t >= a.L) return {0, 0};
   const int r0 = __ldg(a.off + t);
   return {r0, __ldg(a.off + t + 1) - r0};
@@ -72,12 +78,45 @@ __device__ __forceinline__ void ld_relaxed_gpu_2x64(const void* p, uint64_t& a, 
 // A word of four hidden states has arrived when its last one is not the fill pattern.
 __device__ __forceinline__ bool arrived(uint64_t w) { return (w >> 48) != 0xFFFFu; }
 
+// Whole-warp bounded wait for the counters of a step: how many of the next `n` steps (at most 4) can be read, 0 when the wait
+// ran out.  counter(s, f): the f-th counter of step s from now, or nullptr.  Looking at four steps costs no more than at one, and
+// a producer that is behind does without the look, and the proxy fence, of the steps that were ready with it: 900 and 1000 cycles.
+template <typename F>
+__device__ __forceinline__ int wait_steps(int n, int target, F counter, int lane, volatile int* s_abort, int* g_status) {
+  const int step = lane >> 3;
+  uint64_t t0 = 0;
+  for (uint32_t it = 1;; ++it) {
+    bool ready = step < n;
+    if (ready) {
+      const int* p;
+      for (int f = lane & 7; (p = counter(step, f)) != nullptr; f += 8) ready = ready && ld_acquire_gpu(p) >= target;
+    }
+    const uint32_t all = __ballot_sync(0xffffffffu, ready);
+    if ((all & 0xffu) == 0xffu) {
+      __syncwarp();
+      return all == ~0u ? 4 : (all & 0xffffffu) == 0xffffffu ? 3 : (all & 0xffffu) == 0xffffu ? 2 : 1;
+    }
+    if ((it & 0x3F) == 0) {
+      if (t0 == 0) t0 = globaltimer_ns();
+      if (__any_sync(0xffffffffu, *s_abort != 0 || globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS)) {
+        if (lane == 0 && *s_abort == 0) {
+          *s_abort = 1;
+          atomicCAS(g_status, 0, FTB_ERR_TIMEOUT_DEP);
+        }
+        return 0;
+      }
+    }
+  }
+}
+
 // One CTA: packed gate rows `tile` of batch slice `slice`, layers j, j + G, ..  kPair: two CTAs of a cluster, tiles 2 i
 // and 2 i + 1, share each MMA; each holds the state rows of its half of the slice.  kStream: the last input weight blocks,
-// which do not fit, pass through a ring every step.
+// which do not fit, pass through a ring every step.  The layer below is cut into slices of nb_below sequences, of fold_below time
+// steps.
 template <typename T, int NB, bool kPair = false, bool kStream = false>
 __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap& mapH, const CUtensorMap& mapW,
-                                     const FlowArgs& a, const int tile, const int slice, const int j) {
+                                     const FlowArgs& a, const int tile, const int slice, const int j, const int nb_below,
+                                     const int fold_below = 1) {
   using C = FlowCfg<NB, kPair>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t in_full[kMaxSlots], in_empty[kMaxSlots];
@@ -157,6 +196,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
   const int n_groups = (a.D + a.G - 1) / a.G;
   // Steps this slice takes part in (ragged: until its longest sequence, its first one, ends).
   int steps = a.L;
+  if (a.fold > 0 && rows_of(a, a.L - 1).active <= n_base) --steps;
   if (a.off != nullptr) {
     steps = 0;
     for (int hi = a.L; steps < hi;) {
@@ -310,18 +350,31 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       if (sweep == 0) grid_dependency_wait();  // weights need not wait for the fill of the output array and the counters
       ++sweep;
       const int copies = (kb_x + C::kCopyKb - 1) / C::kCopyKb;
+      int ready = 0;  // steps of the layer below that can be read
       for (int t = 0; t < steps && ok; ++t) {
         const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + held_base;
-        if (l > 0) {
-          if (lane == 0) {
-            // the layer below may be cut differently: its slices that hold this one's rows
-            const int* flags = a.flags + (static_cast<int64_t>(l - 1) * a.L + t) * a.S;
-            const int last = (min(n_base + NB, a.N) - 1) / a.nb_below;
-            for (int i = n_base / a.nb_below; i <= last && ok; ++i)
-              ok = flag_wait_ge(flags + i, a.n_tiles, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
-          }
-          ok = __all_sync(0xffffffffu, ok);
+        if (l > 0 && t >= ready) {
+          // the layer below may be cut differently: its slices that hold this one's rows
+          const int* flags = a.flags + static_cast<int64_t>(l - 1) * a.flag_steps * a.S;
+          auto counter = [&](int ahead, int f) -> const int* {
+            if (a.fold == 0) {
+              const int i = n_base / nb_below + f;
+              return i > (min(n_base + NB, a.N) - 1) / nb_below ? nullptr : flags + static_cast<int64_t>(t + ahead) * a.S + i;
+            }
+            const Rows rows = rows_of(a, t + ahead);
+            const int64_t per = static_cast<int64_t>(fold_below) * a.N1, end = rows.first + min(n_base + NB, rows.active);
+            for (int64_t r = rows.first + n_base; r < end; --f) {
+              const int64_t step = r / per;
+              const int i = static_cast<int>(r - step * per) / nb_below;
+              if (f == 0) return flags + step * a.S + i;
+              r = step * per + min((i + 1) * static_cast<int64_t>(nb_below), per);
+            }
+            return nullptr;
+          };
+          const int n = wait_steps(min(4, steps - t), a.n_tiles, counter, lane, &s_abort, status);
+          ok = n > 0;
           if (!ok) break;
+          ready = t + n;
           fence_proxy_async_all();  // threads of other CTAs stored what TMA reads
         }
         ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
@@ -383,7 +436,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
         __threadfence_block();
         fence_proxy_async_all();
         __threadfence();
-        red_release_gpu_add(a.flags + (static_cast<int64_t>(l) * a.L + t) * a.S + slice, 1);
+        red_release_gpu_add(a.flags + (static_cast<int64_t>(l) * a.flag_steps + t) * a.S + slice, 1);
       }
     }
   } else if (kStream && warp == 3) {

@@ -79,7 +79,7 @@ struct ClusterArgs {
   int max_dil;
   int dil[kMaxLayers];
   int nb[kMaxLayers];                 // batch columns per chain of the layer
-  bool flow;                          // layers with dilation 1 run flow::body
+  int fold[kMaxLayers];               // time steps of a step of a layer that runs flow::body, 0: it does not
   int first_cluster[kMaxLayers + 1];  // index of the layer's first cluster
   const void* W;      // Wp [D,4H,2H]
   const float* bias;  // bias_p [D,4H] or nullptr
@@ -102,28 +102,6 @@ struct StepPlan {
   bool self;       // the cluster's own previous output is an operand (through shared memory)
   int self_wkb0, self_nkb;
 };
-
-// Whole-warp bounded wait until the n flags at `flags` have all reached `target` (lane i polls flags i, i+32, ...).
-__device__ __forceinline__ bool warp_wait_flags(const int* flags, int n, int target, int lane, volatile int* s_abort, int* g_status) {
-  uint64_t t0 = 0;
-  uint32_t it = 0;
-  for (;;) {
-    bool ready = true;
-    for (int i = lane; i < n; i += 32) ready = ready && (ld_acquire_gpu(flags + i) >= target);
-    if (__all_sync(0xffffffffu, ready)) return true;
-    if (((++it) & 0x3F) == 0) {
-      if (t0 == 0) t0 = globaltimer_ns();
-      const bool give_up = *s_abort != 0 || globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS;
-      if (__any_sync(0xffffffffu, give_up)) {
-        if (lane == 0 && *s_abort == 0) {
-          *s_abort = 1;
-          atomicCAS(g_status, 0, FTB_ERR_TIMEOUT_DEP);
-        }
-        return false;
-      }
-    }
-  }
-}
 
 // Shared-memory operand descriptor for an un-swizzled K-major tile: core matrices of 8 rows x 16 B
 // stored contiguously (128 B); `lbo` = bytes between the two 16-byte K chunks of an MMA's K = 16,
@@ -178,10 +156,11 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
     x.row = ((layer - 1) * a.L + i) * a.N + slice * NB;
     // One counter per slice of a cell.  The layer below may be cut differently: its slices that hold this
     // one's rows own consecutive counters.
-    const int nbp = a.nb[layer - 1];
-    const int first = slice * NB / nbp;
-    x.flags = a.flags + ((layer - 1) * a.L + i) * a.S + first;
-    x.nflags = (min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
+    const int nbp = a.nb[layer - 1], fold = max(a.fold[layer - 1], 1), step = i / fold;
+    const int row0 = (i - step * fold) * a.N;
+    const int first = (row0 + slice * NB) / nbp;
+    x.flags = a.flags + ((layer - 1) * a.L + step) * a.S + first;
+    x.nflags = (row0 + min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
     x.target = a.CL;
   }
   if (i >= d) {
@@ -313,6 +292,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
     uint32_t phase = 0;
     bool ok = true;
     volatile int* seq = &seg_seq;
+    int ready = 0;  // steps whose segment of this warp can be read
     ACCT_DECL(4);
     for (int i = 0; i < n_steps && ok; ++i) {
       const StepPlan p = plan_step<NB>(a, layer, slice, i);
@@ -320,17 +300,32 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
         const Segment& sg = p.seg[s];
         if ((s & 1) == mine) {
           ACCT_BEGIN();
-          if (sg.flags != nullptr && !warp_wait_flags(sg.flags, sg.nflags, sg.target, lane, &s_abort, status)) {
-            ok = false;
-            break;
+          if (sg.flags != nullptr && i >= ready) {
+            // (the layer below may count steps of two time steps: then the next ones' counters lie elsewhere)
+            const int* at = sg.flags;
+            int count = sg.nflags;
+            if (s == 1 || a.fold[layer - 1] < 2) {
+              at += (lane >> 3) * a.S;
+            } else if (i + (lane >> 3) < n_steps) {
+              const StepPlan next = plan_step<NB>(a, layer, slice, i + (lane >> 3));
+              at = next.seg[0].flags;
+              count = next.seg[0].nflags;
+            }
+            auto counter = [&](int, int f) -> const int* { return f < count ? at + f : nullptr; };
+            const int n = flow::wait_steps(min(4, n_steps - i), sg.target, counter, lane, &s_abort, status);
+            if (n == 0) {
+              ok = false;
+              break;
+            }
+            ready = i + n;
+            // (Producers write their outputs with TMA stores and consumers read them with TMA loads: both
+            // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.
+            // Threads store the output of flow::body.)
+            if (lane == 0 && s == 0 && layer > 0 && a.fold[layer - 1] > 0) fence_proxy_async_all();
           }
           ACCT_END(0);
           bool fine = true;
           if (lane == 0) {
-            // (Producers write their outputs with TMA stores and consumers read them with TMA loads: both
-            // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.
-            // Threads store the output of flow::body.)
-            if (a.flow && s == 0 && layer > 0 && a.dil[layer - 1] == 1) fence_proxy_async_all();
             FTB_CL_STAMP(i, 7 + 2 * s);
             ACCT_BEGIN();
             if (*seq != q) {
@@ -751,29 +746,38 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
 
 // The same program without clusters, where it fits: what the layers with dilation >= 2 exchange goes through
 // global memory anyway (2.2 us a step on slices of 64; on 128 a layer with dilation 2, which waits for the trip
-// there and back, takes 3.0).  A layer with dilation 1 runs as csrc/lstm_flow.cu does, on slices of kNarrow
-// sequences whose state is its own flag: 1.6 us a step at H 256 and 32 sequences where a cluster's hand-off of
-// 64 takes 2.6, and no GPC has to hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).
+// there and back, takes 3.0).  A layer with dilation 1 runs as csrc/lstm_flow.cu does, on narrow slices whose state is
+// its own flag: 1.6 us a step at H 256 and 32 sequences where a cluster's hand-off of 64 takes 2.6, and no GPC has to
+// hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).  A layer with dilation 2 does so too where its slices fit: as a layer
+// of 2 N sequences and half the steps, whose trip there and back it no longer waits for (dilated_flow_widths).
 struct DilatedMaps {
   CUtensorMap x64, h64, o64, t64, x128, h128, o128, t128;  // as above
-  CUtensorMap nx, nh, nw;                                   // of flow::body
+  CUtensorMap nx[2], nh[2], nw;                             // of flow::body, by time steps of a step - 1
 };
-template <typename T, int kNarrow>
+template <typename T>
 __global__ void __launch_bounds__(kCtaThreads, 1)
 rnn_dilated_flow_kernel(const __grid_constant__ DilatedMaps m, const __grid_constant__ ClusterArgs a,
-                        const __grid_constant__ flow::FlowArgs f) {
+                        const __grid_constant__ flow::FlowArgs f1, const __grid_constant__ flow::FlowArgs f2) {
   const int cid = blockIdx.x / a.CL, rank = blockIdx.x - cid * a.CL;
   int layer = 0;
   while (layer + 1 < a.D && cid >= a.first_cluster[layer + 1]) ++layer;
   const int slice = cid - a.first_cluster[layer];
-  if (a.dil[layer] == 1) {
-    flow::FlowArgs fl = f;
-    fl.nb_below = layer > 0 ? a.nb[layer - 1] : kNarrow;
-    flow::body<T, kNarrow>(m.nx, m.nh, m.nw, fl, rank, slice, layer);
+  const int fold = a.fold[layer], nb = a.nb[layer];
+  const int nb_below = layer > 0 ? a.nb[layer - 1] : nb, fold_below = layer > 0 ? max(a.fold[layer - 1], 1) : 1;
+  if (fold == 1) {
+    if (nb == 16) flow::body<T, 16>(m.nx[0], m.nh[0], m.nw, f1, rank, slice, layer, nb_below, fold_below);
+    else if (nb == 32) flow::body<T, 32>(m.nx[0], m.nh[0], m.nw, f1, rank, slice, layer, nb_below, fold_below);
+    else flow::body<T, 48>(m.nx[0], m.nh[0], m.nw, f1, rank, slice, layer, nb_below, fold_below);
+    return;
+  }
+  if (fold == 2) {
+    if (nb == 16) flow::body<T, 16>(m.nx[1], m.nh[1], m.nw, f2, rank, slice, layer, nb_below, fold_below);
+    else if (nb == 32) flow::body<T, 32>(m.nx[1], m.nh[1], m.nw, f2, rank, slice, layer, nb_below, fold_below);
+    else flow::body<T, 64>(m.nx[1], m.nh[1], m.nw, f2, rank, slice, layer, nb_below, fold_below);
     return;
   }
   const bool split = a.dil[layer] % 2 == 0;
-  if (a.nb[layer] == 64) {
+  if (nb == 64) {
     if (split) cluster_body<T, 64, true>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
     else cluster_body<T, 64, false>(m.x64, m.h64, m.o64, m.t64, a, rank, cid, layer, slice);
   } else {
@@ -847,19 +851,12 @@ int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_
   return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, kCtaThreads, configured, grid, smem_bytes, stream, m[0],
                        m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
 }
-template <typename T, int kNarrow>
-int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs& f, int grid, uint32_t smem_bytes,
+template <typename T>
+int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs (&f)[2], int grid, uint32_t smem_bytes,
                         cudaStream_t stream) {
   static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_dilated_flow_kernel<T, kNarrow>, 1, kCtaThreads, configured, grid, smem_bytes, stream, m,
-                       a, f);
-}
-template <typename T>
-int launch_dilated_flow(int narrow, const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs& f, int grid,
-                        uint32_t smem_bytes, cudaStream_t stream) {
-  if (narrow == 16) return launch_dilated_flow<T, 16>(m, a, f, grid, smem_bytes, stream);
-  if (narrow == 32) return launch_dilated_flow<T, 32>(m, a, f, grid, smem_bytes, stream);
-  return launch_dilated_flow<T, 48>(m, a, f, grid, smem_bytes, stream);
+  return launch_kernel(rnn_dilated_flow_kernel<T>, 1, kCtaThreads, configured, grid, smem_bytes, stream, m, a, f[0],
+                       f[1]);
 }
 
 uint32_t smem_for(bool any_self, int H) {
@@ -892,30 +889,49 @@ int dilated_slices(const int* dilations, int D, int N, int max_clusters, int* nb
   return s128 <= 8 && total <= max_clusters ? total : 0;
 }
 
-// Slice widths of the layers for a launch without clusters, false: it does not fit or no layer has dilation 1.
-// Dilation 1: 16, 32 or 48; the others 64, or 128 from dilation 3 on (a step's trip through global memory is hidden
-// behind the steps between); the narrowest that fit beside each other.
-bool dilated_flow_widths(const int* dilations, int D, int N, int CL, int sm_count, int* nb) {
-  int ones = 0;
-  for (int l = 0; l < D; ++l) ones += dilations[l] == 1;
-  if (ones == 0) return false;
+// How a launch without clusters cuts the layers, false: it does not fit or no layer has dilation 1.  Layers of dilation 1 run
+// flow::body on slices of 16, 32 or 48 sequences; those of dilation 2 too, on slices of 16, 32 or 64 of 2 N, or like the others as
+// cells of slices of 64 or 128 whose states make a trip through global memory.  The slowest layer sets the pace; its time per time
+// step is estimated from layers alone and beside others (us, H 128 / 256; 16, 32, 48 and 64 columns 1.5, 1.55, 1.87, 2.1 / 1.6, 1.85,
+// 2.15, 2.55 a step of flow::body; cells of 64 and 128 1.15, 1.5 / 1.5, 2.5, a trip 3.6, 4.2 / 4.7, 5.0), the narrowest cut wins a
+// tie.  Dilations 1 2 4 and 1 .. 32, us a time step with dilation 2 as cells / as it is taken: H 128, 17 sequences 1.85 / 1.50, 1.80 /
+// 1.57; H 256, 33 2.09 / 1.75, 2.16 / 1.81; 128 2.25 / 2.00, 2.32 / 2.18; 256 as cells (2.40; 2.68 as 2 N sequences).
+bool dilated_flow_widths(const int* dilations, int D, int N, int H, int CL, int sm_count, int* nb, int* fold) {
+  bool one = false, two = false;
+  for (int l = 0; l < D; ++l) {
+    one = one || dilations[l] == 1;
+    two = two || dilations[l] == 2;
+  }
+  if (!one) return false;
+  const double h = H / 128.0 - 1.0;  // -0.5, 0, 1
+  auto flow_step = [&](int w) { return w == 16 ? 1.5 + 0.1 * h : w == 32 ? 1.55 + 0.3 * h : w == 48 ? 1.87 + 0.28 * h : 2.1 + 0.45 * h; };
+  auto cell = [&](int w, int d) {
+    return w == 64 ? std::max(1.15 + 0.35 * h, (3.6 + 1.1 * h) / d) : std::max(1.5 + h, (4.2 + 0.8 * h) / d);
+  };
+  double best = 0.0;
   for (int wide = 64; wide <= 128; wide *= 2)
-    for (int narrow = 16; narrow <= 48; narrow += 16) {
-      int ctas = 0;
-      for (int l = 0; l < D; ++l) {
-        nb[l] = dilations[l] == 1 ? narrow : (dilations[l] == 2 ? 64 : wide);
-        ctas += CL * ((N + nb[l] - 1) / nb[l]);
+    for (int second : {16, 32, 64, 0}) {  // 0: dilation 2 as cells
+      if (second > 0 && !two) continue;
+      for (int narrow = 16; narrow <= 48; narrow += 16) {
+        int ctas = 0;
+        double pace = 0.0;
+        auto cut = [&](int l, int* f) {
+          *f = dilations[l] == 1 ? 1 : dilations[l] == 2 && second > 0 ? 2 : 0;
+          return *f == 1 ? narrow : *f == 2 ? second : dilations[l] == 2 ? 64 : wide;
+        };
+        for (int l = 0; l < D; ++l) {
+          int f;
+          const int w = cut(l, &f), slices = (std::max(f, 1) * N + w - 1) / w;
+          ctas += slices > 64 ? sm_count + 1 : CL * slices;  // (64: counters a cell)
+          pace = std::max(pace, f > 0 ? flow_step(w) / f : cell(w, dilations[l]));
+        }
+        if (ctas > sm_count || (best > 0.0 && pace >= best)) continue;
+        best = pace;
+        for (int l = 0; l < D; ++l) nb[l] = cut(l, &fold[l]);
       }
-      if (ctas <= sm_count) return true;
     }
-  return false;
+  return best > 0.0;
 }
-// Clusters of 2 and 4 CTAs hand a state on fast enough for batches of up to 64 (us, 3 layers of 512 steps, with
-// clusters / without: H 64, N 24 895 / 911, N 64 985 / 1105; H 128, N 24 1082 / 932, N 32 1082 / 1022, N 48 1083 / 1108; above
-// 64 sequences and at H 256 they lose: H 64, N 128 1236 / 1114; H 256, N 64 1469 / 1164, N 256 and six layers 1613 / 1330,
-// 1654 with every layer but the first on slices of 128).
-bool dilated_prefers_clusters(int N, int CL) { return (CL == 2 && N <= 64) || (CL == 4 && N > 32 && N <= 64); }
-
 // Clusters of `cl` CTAs of the dilated kernel that can be resident at once on the current device (a
 // cluster needs its CTAs' SMs inside one GPC, so this is less than SMs / cl: 15 clusters of 8 on a
 // 148-SM B200).  0 when the query fails.
@@ -962,8 +978,8 @@ bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count
 size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 64; }
 
 // x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).  schedule 4: with
-// clusters where they fit, 5: without (FTB_ERR_ARG where that does not
-// fit), 0: the faster of the two.
+// clusters where they fit, 5: without (FTB_ERR_ARG where that does not fit), 0: without where it fits, which is the faster of the
+// two at every size timed (H 64 to 256, 8 to 256 sequences, 3 and 6 layers: 1.01 to 1.6 times).
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
                                 const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
                                 int sm_count, cudaStream_t stream) {
@@ -983,15 +999,14 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   int rc;
   const uint32_t cluster_smem = smem_for(any_self, H);
   auto cut_for_clusters = [&] { return dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, cluster_smem), a.nb); };
-  int clusters = schedule == 4 || (schedule == 0 && dilated_prefers_clusters(N, a.CL)) ? cut_for_clusters() : 0;
-  if (clusters <= 0 && dilated_flow_widths(dilations, D, N, a.CL, sm_count, a.nb)) {
-    a.flow = true;
-    int narrow = 0;
+  int clusters = schedule == 4 ? cut_for_clusters() : 0;
+  if (clusters <= 0 && dilated_flow_widths(dilations, D, N, H, a.CL, sm_count, a.nb, a.fold)) {
+    int width[2] = {0, 0};  // of the slices of layers that run flow::body, by time steps of a step - 1
     for (int l = 0; l < D; ++l) {
-      const int slices = (N + a.nb[l] - 1) / a.nb[l];
+      const int slices = (std::max(a.fold[l], 1) * N + a.nb[l] - 1) / a.nb[l];
       a.S = std::max(a.S, slices);
       a.first_cluster[l + 1] = a.first_cluster[l] + slices;
-      if (dilations[l] == 1) narrow = a.nb[l];
+      if (a.fold[l] > 0) width[a.fold[l] - 1] = a.nb[l];
     }
     DilatedMaps dm;
     for (int wide = 64; wide <= 128; wide *= 2) {
@@ -1002,25 +1017,33 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
       if ((rc = make_tmap_2d_sw64(wide == 64 ? &dm.t64 : &dm.t128, hs, dtype, h_rows, H, H, tail))) return rc;
     }
     const uint64_t row_bytes = static_cast<uint64_t>(H) * 2;
-    const uint32_t planes = 128 / narrow;  // of a copy of flow::body
-    if ((rc = make_tmap_3d(&dm.nx, x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
-    if ((rc = make_tmap_3d(&dm.nh, hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, narrow, planes))) return rc;
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t w = width[i] > 0 ? width[i] : width[0], planes = 128 / w;  // of a copy of flow::body
+      if ((rc = make_tmap_3d(&dm.nx[i], x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, w, planes))) return rc;
+      if ((rc = make_tmap_3d(&dm.nh[i], hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, w, planes))) return rc;
+    }
     if ((rc = make_tmap_gates(&dm.nw, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H))) return rc;
-    flow::FlowArgs f = {};
-    f.D = D; f.L = L; f.N = N; f.I = H; f.H = H; f.G = D; f.S = a.S;
-    f.n_tiles = a.CL;
-    f.n_slots = flow::kMaxSlots;
-    f.T = static_cast<int64_t>(L) * N;
-    f.bias_p = bias_p; f.Wp = Wp; f.hs = hs; f.c_out = c; f.c_rows = a.max_dil * N; f.flags = flags; f.status = status;
+    flow::FlowArgs f[2] = {};
+    for (int i = 0; i < 2; ++i) {
+      f[i].fold = i + 1; f[i].N1 = N; f[i].flag_steps = L;
+      f[i].D = D; f[i].L = (L + i) / (i + 1); f[i].N = N * (i + 1); f[i].I = H; f[i].H = H; f[i].G = D; f[i].S = a.S;
+      f[i].n_tiles = a.CL;
+      f[i].n_slots = flow::kMaxSlots;
+      f[i].T = static_cast<int64_t>(L) * N;
+      f[i].bias_p = bias_p; f[i].Wp = Wp; f[i].hs = hs; f[i].c_out = c; f[i].c_rows = a.max_dil * N; f[i].flags = flags;
+      f[i].status = status;
+    }
     if (cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(D) * L * a.S, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
     const size_t layer_bytes = static_cast<size_t>(L) * N * H * 2;
-    for (int l = 0; l < D; ++l)
-      if (dilations[l] == 1 && cudaMemsetAsync(static_cast<char*>(hs) + l * layer_bytes, 0xFF, layer_bytes, stream) != cudaSuccess)
+    for (int l = 0, n; l < D; l += std::max(n, 1)) {  // neighbouring layers in one go
+      for (n = 0; l + n < D && a.fold[l + n] > 0;) ++n;
+      if (n > 0 && cudaMemsetAsync(static_cast<char*>(hs) + l * layer_bytes, 0xFF, n * layer_bytes, stream) != cudaSuccess)
         return FTB_ERR_LAUNCH;
+    }
     const uint32_t smem = smem_for(false, H);
     const int grid = a.first_cluster[D] * a.CL;
-    if (dtype == FTB_F16) return launch_dilated_flow<__half>(narrow, dm, a, f, grid, smem, stream);
-    return launch_dilated_flow<__nv_bfloat16>(narrow, dm, a, f, grid, smem, stream);
+    if (dtype == FTB_F16) return launch_dilated_flow<__half>(dm, a, f, grid, smem, stream);
+    return launch_dilated_flow<__nv_bfloat16>(dm, a, f, grid, smem, stream);
   }
   if (schedule == 5) return FTB_ERR_ARG;
   if (clusters <= 0) clusters = cut_for_clusters();

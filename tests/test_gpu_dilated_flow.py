@@ -61,6 +61,20 @@ def test_nan_states_are_states(ops, dt):
     assert torch.equal(torch.nan_to_num(h), torch.nan_to_num(ref))
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("L,N,H,dils", [
+    (1, 5, 128, [1, 2]),             # one step: half of the second layer's columns have none
+    (2, 17, 64, [2, 1]),             # the folded layer reads the input
+    (7, 9, 256, [1, 2, 2]),          # an odd number of steps; folded on folded, slices that straddle two time steps
+    (23, 33, 256, [1, 2, 4, 2, 1]),  # beside cells of dilation 4, above and below
+    (30, 100, 128, [1, 2, 4, 8]),
+    (12, 256, 128, [1, 2]),
+])
+def test_layers_of_dilation_two(ops, dt, L, N, H, dils):
+    """As layers of 2 N sequences and half the steps, where their slices fit."""
+    _against_levels(ops, dt, L, N, H, dils, 5)
+
+
 def test_schedule_5_where_it_does_not_apply(ops):
     """No layer of dilation 1: the generic persistent kernel, as for schedule 2."""
     _against_levels(ops, torch.float16, 9, 40, 128, [2, 3], 5)
