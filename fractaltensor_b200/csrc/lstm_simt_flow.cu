@@ -49,7 +49,7 @@ constexpr int kLoadWarps = 4;
 constexpr int kMul = 4;  // multiplying warps of a half
 
 // Named barriers (0 is __syncthreads).
-enum Bar : int { kInFull = 1, kInEmpty = 1 + kMaxSlots, kPartsTaken = 1 + 2 * kMaxSlots, kEarlyDone, kLateWarpsMeet };
+enum Bar : int { kInFull = 1, kInEmpty = 1 + kMaxSlots, kPartsTaken = 1 + 2 * kMaxSlots, kEarlyDone, kLateWarpsMeet, kEarlyWarpsMeet };
 __device__ __forceinline__ void bar_wait(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -61,7 +61,8 @@ template <int TM>
 struct SimtFlowCfg {
   // A lane's part of a chunk's TM x 32 products; 16 lanes make up the chunk.
   static constexpr int kRows = TM == 32 ? 8 : 4, kCols = TM == 8 ? 4 : 8;
-  static constexpr int kLateWarps = TM == 32 ? 8 : 4;  // the first kMul multiply; a cell per thread
+  static constexpr int kLateWarps = 4;
+  static constexpr int kCells = TM == 32 ? 2 : 1;  // of a thread of theirs, 16 rows apart
   // first warp of each role: the input half's multiplication, the recurrent half's and the cells, input tiles
   static constexpr int kLate = kMul, kLoad = kMul + kLateWarps;
   static constexpr int kThreads = 32 * (kLoad + kLoadWarps);
@@ -101,21 +102,22 @@ __device__ __forceinline__ bool arrived(const uint4& v) {
   return v.x != 0xFFFFFFFFu && v.y != 0xFFFFFFFFu && v.z != 0xFFFFFFFFu && v.w != 0xFFFFFFFFu;
 }
 
-// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: eight 16-byte chunks a lane
-// (four rows, two chunks of each) in flight.  With `poll` a chunk is repeated until its four words are
+// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: kInFlight rows, two 16-byte chunks a lane
+// of each, in flight.  With `poll` a chunk is repeated until its four words are
 // states; the others (inputs of the call) are taken as they are.  Returns the number of rounds of loads
 // beyond the first of each eight.  (Not inlined, like multiply: with both in the kernel's body the registers
 // do not suffice and their loops spill.)
+template <int kInFlight>
 __device__ __noinline__ int load_rows(float* dst, const float* src, int rows, int H, int w, int warps, bool poll,
                                       uint32_t sleep_ns, volatile int* s_abort, int* status) {
   const int lane = threadIdx.x & 31, ld = row_words(H);
   int extra = 0;
-  for (int r0 = w; r0 < rows; r0 += 4 * warps)
+  for (int r0 = w; r0 < rows; r0 += kInFlight * warps)
     for (int k0 = 4 * lane; __any_sync(0xffffffffu, k0 < H); k0 += 256) {
-      uint4 v[8];
+      uint4 v[2 * kInFlight];
       uint32_t mine = 0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 2 * kInFlight; ++i) {
         v[i] = make_uint4(0, 0, 0, 0);
         if (r0 + (i >> 1) * warps < rows && k0 + (i & 1) * 128 < H) mine |= 1u << i;
       }
@@ -123,10 +125,10 @@ __device__ __noinline__ int load_rows(float* dst, const float* src, int rows, in
       uint64_t t0 = 0;
       for (uint32_t it = 0;;) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 2 * kInFlight; ++i)
           if (missing & (1u << i)) v[i] = ld_relaxed_gpu_v4(src + (r0 + (i >> 1) * warps) * H + k0 + (i & 1) * 128);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 2 * kInFlight; ++i)
           if ((missing & (1u << i)) && (!poll || arrived(v[i]))) missing &= ~(1u << i);
         if (__all_sync(0xffffffffu, missing == 0) || __any_sync(0xffffffffu, *s_abort != 0)) break;
         ++extra;
@@ -143,7 +145,7 @@ __device__ __noinline__ int load_rows(float* dst, const float* src, int rows, in
         }
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 2 * kInFlight; ++i)
         if (mine & (1u << i)) {
           const int k = k0 + (i & 1) * 128;
           *reinterpret_cast<uint4*>(dst + (r0 + (i >> 1) * warps) * ld + k + 4 * (k / TK)) = v[i];
@@ -165,7 +167,7 @@ __device__ __noinline__ void multiply(const float* A, const float* W, int lda, i
     uint64_t acc[R][C / 2] = {};
     const float* a = A + ry * lda + c * kLdChunk;
     const float* b = W + c * TK * kLdW + C * cx;
-#pragma unroll 4
+#pragma unroll
     for (int k = 0; k < TK; k += 2, a += 2, b += 2 * kLdW) {
       float2 av[R];
 #pragma unroll
@@ -195,6 +197,23 @@ __device__ __noinline__ void multiply(const float* A, const float* W, int lda, i
       for (int h = 0; h < C / 2; h += 2)
         *reinterpret_cast<ulonglong2*>(out + (ry + i * G) * TN + 2 * h) = make_ulonglong2(acc[i][h], acc[i][h + 1]);
   }
+}
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+// Chunks from .. to-1 of four columns, in order.
+__device__ __forceinline__ float4 chunk_sum(const float* q, int stride, int from, int to) {
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int ch = from; ch < to; ++ch) sum = add4(sum, *reinterpret_cast<const float4*>(q + ch * stride));
+  return sum;
+}
+// n chunks in kGroups groups, the groups in order.
+template <int kGroups>
+__device__ __forceinline__ float4 group_sums(const float* q, int stride, int n) {
+  float4 v = chunk_sum(q, stride, 0, n / kGroups);
+#pragma unroll
+  for (int g = 1; g < kGroups; ++g) v = add4(v, chunk_sum(q, stride, n * g / kGroups, n * (g + 1) / kGroups));
+  return v;
 }
 
 template <int TM>
@@ -255,47 +274,58 @@ lstm_simt_flow_kernel(const __grid_constant__ SimtFlowArgs a) {
         if (k > 0) bar_wait(kPartsTaken, kWithLate);
         multiply<TM>(sI + slot * TM * lda, sW, lda, chunks, sP, warp);
         if (k + a.n_slots < total) bar_post(kInEmpty + slot, kWithLoad);
+        // The sums of the input half, which leaves those of the recurrent half alone on the chain: the first two of the four
+        // groups are the input's.  (The first step of a sweep is an input half alone: its chunks make up all four.)
+        bar_wait(kEarlyWarpsMeet, 32 * kMul);
+#pragma unroll
+        for (int i = 0; i < C::kCells; ++i)
+          if ((tid >> 3) + 16 * i < TM) {
+            float* q = sP + ((tid >> 3) + 16 * i) * TN + 4 * (tid & 7);
+            *reinterpret_cast<float4*>(q) = t == 0 ? group_sums<4>(q, TM * TN, chunks) : group_sums<2>(q, TM * TN, chunks);
+          }
         bar_post(kEarlyDone, kWithLate);
       }
     } else if (warp < C::kLoad) {
       // -------------------------------- recurrent half, cells, then the layer's whole state for the next step
       const int cell = tid - 32 * C::kLate;
-      const int row = cell >> 3, u = cell & 7, unit = n_tile * 8 + u;
+      const int row = cell >> 3, u = cell & 7, unit = n_tile * 8 + u;  // and the row 16 further, TM 32
       float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias != nullptr) b = *reinterpret_cast<const float4*>(a.bias + static_cast<size_t>(l) * 4 * H + 4 * unit);
-      float c = 0.f;
+      float c[C::kCells] = {};
       for (int t = 0; t < a.L; ++t, ++k) {
-        if (t > 0 && warp < C::kLate + kMul)
-          multiply<TM>(sS, sW + H * kLdW, lda, chunks, sP + chunks * TM * TN, warp - C::kLate);
+        if (t > 0) multiply<TM>(sS, sW + H * kLdW, lda, chunks, sP + chunks * TM * TN, warp - C::kLate);
         bar_wait(kEarlyDone, kWithLate);  // (the late warps meet here too)
         float* out = hs_l + t * step_elems;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < TM) {
-          // The first step of a sweep is an input half alone: its chunks are dealt out to all four groups.
-          const float* q = sP + row * TN + 4 * u;
-          const int n = t == 0 ? chunks : 2 * chunks;
+        float4 v[C::kCells];
 #pragma unroll
-          for (int g = 0, ch = 0; g < 4; ++g) {
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (const int end = n * (g + 1) / 4; ch < end; ++ch) {
-              const float4 pc = *reinterpret_cast<const float4*>(q + ch * TM * TN);
-              sum.x += pc.x; sum.y += pc.y; sum.z += pc.z; sum.w += pc.w;
+        for (int i = 0; i < C::kCells; ++i) {
+          v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (row + 16 * i < TM) {
+            const float* q = sP + (row + 16 * i) * TN + 4 * u;
+            v[i] = *reinterpret_cast<const float4*>(q);
+            if (t > 0) {
+              const float* r = q + chunks * TM * TN;
+              v[i] = add4(v[i], chunk_sum(r, TM * TN, 0, chunks / 2));
+              v[i] = add4(v[i], chunk_sum(r, TM * TN, chunks / 2, chunks));
             }
-            if (g == 0) v = sum;
-            else { v.x += sum.x; v.y += sum.y; v.z += sum.z; v.w += sum.w; }
           }
         }
         if (row < rows) {
-          const float gi = sigmoid_acc(v.x + b.x);
-          const float gf = sigmoid_acc(v.y + b.y);
-          const float go = sigmoid_acc(v.z + b.z);
-          const float gc = tanhf(v.w + b.w);
-          const float cn = gf * c + gi * gc;
-          c = cn;
-          uint32_t bits = __float_as_uint(go * tanhf(cn));
-          if (bits == 0xFFFFFFFFu) bits = 0x7FFFFFFFu;
-          st_relaxed_gpu32(out + static_cast<size_t>(row) * H + unit, bits);
+          uint32_t bits[C::kCells];
+#pragma unroll
+          for (int i = 0; i < C::kCells; ++i) {
+            const float gi = sigmoid_acc(v[i].x + b.x);
+            const float gf = sigmoid_acc(v[i].y + b.y);
+            const float go = sigmoid_acc(v[i].z + b.z);
+            const float gc = tanhf(v[i].w + b.w);
+            const float cn = gf * c[i] + gi * gc;
+            c[i] = cn;
+            bits[i] = __float_as_uint(go * tanhf(cn));
+            if (bits[i] == 0xFFFFFFFFu) bits[i] = 0x7FFFFFFFu;
+          }
+#pragma unroll
+          for (int i = 0; i < C::kCells; ++i)
+            if (row + 16 * i < rows) st_relaxed_gpu32(out + static_cast<size_t>(row + 16 * i) * H + unit, bits[i]);
         }
         __syncwarp();
         // (After the cells, not before: the early warps' multiplication would slow them to a third.)
@@ -305,21 +335,23 @@ lstm_simt_flow_kernel(const __grid_constant__ SimtFlowArgs a) {
             const long long c0 = clock64();
             while (clock64() - c0 < pause) __nanosleep(20);
           }
-          const int extra = load_rows(sS, out, rows, H, warp - C::kLate, C::kLateWarps, true, 0, &s_abort, status);
+          const int extra = load_rows<TM == 32 ? 8 : 4>(sS, out, rows, H, warp - C::kLate, C::kLateWarps, true, 0, &s_abort, status);
           // Everything at the first look: a little earlier next time; else later.  (Looks that come too early
           // load the L2 that the states have to pass through.)
           pause = extra > 0 ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
           bar_wait(kLateWarpsMeet, kLateThreads);
         }
       }
-      if (row < rows) a.c[(static_cast<size_t>(l) * a.N + row0 + row) * H + unit] = c;
+#pragma unroll
+      for (int i = 0; i < C::kCells; ++i)
+        if (row + 16 * i < rows) a.c[(static_cast<size_t>(l) * a.N + row0 + row + 16 * i) * H + unit] = c[i];
     } else {
       // ------------------------------------------------------------ input tiles
       const float* src = l == 0 ? a.x + static_cast<size_t>(row0) * H : hs_l - static_cast<size_t>(a.L) * step_elems;
       for (int t = 0; t < a.L; ++t, ++k) {
         const int slot = a.n_slots == 2 ? (k & 1) : 0;
         if (k >= a.n_slots) bar_wait(kInEmpty + slot, kWithLoad);
-        load_rows(sI + slot * TM * lda, src + t * step_elems, rows, H, warp - C::kLoad, kLoadWarps, l > 0, 200, &s_abort,
+        load_rows<4>(sI + slot * TM * lda, src + t * step_elems, rows, H, warp - C::kLoad, kLoadWarps, l > 0, 200, &s_abort,
                   status);
         bar_post(kInFull + slot, kWithLoad);
       }
