@@ -102,8 +102,8 @@ __device__ __forceinline__ bool arrived(const uint4& v) {
   return v.x != 0xFFFFFFFFu && v.y != 0xFFFFFFFFu && v.z != 0xFFFFFFFFu && v.w != 0xFFFFFFFFu;
 }
 
-// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: kInFlight rows, two 16-byte chunks a lane
-// of each, in flight.  With `poll` a chunk is repeated until its four words are
+// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: eight 16-byte chunks a lane
+// (four rows, two chunks of each) in flight.  With `poll` a chunk is repeated until its four words are
 // states; the others (inputs of the call) are taken as they are.  Returns the number of rounds of loads
 // beyond the first of each eight.  (Not inlined, like multiply: with both in the kernel's body the registers
 // do not suffice and their loops spill.)
@@ -154,13 +154,81 @@ __device__ __noinline__ int load_rows(float* dst, const float* src, int rows, in
   return extra;
 }
 
+// The late warps' part of a state, rows w, w + warps, .. (kRows of them) of the next step's operand: what load_rows does, with
+// the addresses and masks made once a sweep.  On the chain, beside the early warps' multiplication, every instruction counts:
+// as load_rows 450 cycles until the first load, 400 to 650 until the last, 350 to 600 for the stores.
+template <int kRows>
+struct StateLoad {
+  int first, src_row, dst_row, wide;  // (numbers)
+  int dst_first;
+  uint32_t mine;
+
+  __device__ __forceinline__ StateLoad(int rows, int H, int w, int warps) {
+    const int lane = threadIdx.x & 31, ld = row_words(H);
+    first = w * H + 4 * lane;
+    src_row = warps * H;
+    dst_first = w * ld + 4 * lane + 4 * (4 * lane / TK);
+    dst_row = warps * ld;
+    wide = H;
+    mine = 0;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (w + i * warps < rows) mine |= 1u << i;
+  }
+  __device__ __forceinline__ int load(const float* src, float* dst, volatile int* s_abort, int* status) const {
+    const int lane = threadIdx.x & 31;
+    int extra = 0;
+    src += first;
+    dst += dst_first;
+    for (int k0 = 4 * lane; k0 - 4 * lane < wide; k0 += 256, src += 256, dst += 256 + 32) {
+      uint4 v[2][kRows];
+      uint32_t missing[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) missing[j] = k0 + j * 128 < wide ? mine : 0u;
+      const uint32_t taken[2] = {missing[0], missing[1]};
+      uint64_t t0 = 0;
+      for (uint32_t it = 1;; ++it) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < kRows; ++i)
+            if (missing[j] & (1u << i)) v[j][i] = ld_relaxed_gpu_v4(src + i * src_row + j * 128);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < kRows; ++i)
+            if ((missing[j] & (1u << i)) && arrived(v[j][i])) missing[j] &= ~(1u << i);
+        if (__all_sync(0xffffffffu, (missing[0] | missing[1]) == 0)) break;
+        ++extra;
+        if (__any_sync(0xffffffffu, *s_abort != 0)) break;
+        if ((it & 0x3F) == 0) {
+          if (t0 == 0) t0 = globaltimer_ns();
+          if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > FTB_WAIT_TIMEOUT_NS || ld_relaxed_gpu(status) != 0)) {
+            if (lane == 0) {
+              *s_abort = 1;
+              atomicCAS(status, 0, FTB_ERR_TIMEOUT_DEP);
+            }
+            break;
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+          if (taken[j] & (1u << i)) *reinterpret_cast<uint4*>(dst + i * dst_row + j * (128 + 16)) = v[j][i];
+    }
+    return extra;
+  }
+};
+
 // Products of the TM rows A[row][lda] with W[k][kLdW], n_chunks (even) chunks of 32 wide; chunk c's sums, in
 // ascending order of k, to p[c][TM][32].  Warp w of kMul, a half-warp to a chunk: a lane has rows ry, ry + G, ..
 // (neighbouring rows fall on different banks) and kCols columns, two of them to an FMA (fma.rn.f32x2: each
 // half rounds as fmaf does).  H 256, 148 CTAs, cycles of four warps at TM 8 / 16 / 32: 1306 / 2071 / 4260; scalar
 // with the next k's operands prefetched 1311 / 2114 / 4849.
 template <int TM>
-__device__ __noinline__ void multiply(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
+__device__ __forceinline__ void multiply_here(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
   constexpr int R = SimtFlowCfg<TM>::kRows, C = SimtFlowCfg<TM>::kCols, G = TM / R;
   const int lane = threadIdx.x & 31, cx = lane & (TN / C - 1), ry = (lane & 15) / (TN / C);
   for (int c = 2 * w + (lane >> 4); c < n_chunks; c += 2 * kMul) {
@@ -197,6 +265,18 @@ __device__ __noinline__ void multiply(const float* A, const float* W, int lda, i
       for (int h = 0; h < C / 2; h += 2)
         *reinterpret_cast<ulonglong2*>(out + (ry + i * G) * TN + 2 * h) = make_ulonglong2(acc[i][h], acc[i][h + 1]);
   }
+}
+
+// (A call, where inlining it leaves the rest of the kernel too few registers: at 32 rows 384 us for 4 x 64 x 32 x 256 against 403;
+// at 8 rows 155 against 151 for 2 x 64 x 8 x 256.)
+template <int TM>
+__device__ __noinline__ void multiply_call(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
+  multiply_here<TM>(A, W, lda, n_chunks, p, w);
+}
+template <int TM>
+__device__ __forceinline__ void multiply(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
+  if constexpr (TM == 8) multiply_here<TM>(A, W, lda, n_chunks, p, w);
+  else multiply_call<TM>(A, W, lda, n_chunks, p, w);
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -292,6 +372,7 @@ lstm_simt_flow_kernel(const __grid_constant__ SimtFlowArgs a) {
       float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias != nullptr) b = *reinterpret_cast<const float4*>(a.bias + static_cast<size_t>(l) * 4 * H + 4 * unit);
       float c[C::kCells] = {};
+      const StateLoad<TM / C::kLateWarps> state(rows, H, warp - C::kLate, C::kLateWarps);
       for (int t = 0; t < a.L; ++t, ++k) {
         if (t > 0) multiply<TM>(sS, sW + H * kLdW, lda, chunks, sP + chunks * TM * TN, warp - C::kLate);
         bar_wait(kEarlyDone, kWithLate);  // (the late warps meet here too)
@@ -335,7 +416,11 @@ lstm_simt_flow_kernel(const __grid_constant__ SimtFlowArgs a) {
             const long long c0 = clock64();
             while (clock64() - c0 < pause) __nanosleep(20);
           }
-          const int extra = load_rows<TM == 32 ? 8 : 4>(sS, out, rows, H, warp - C::kLate, C::kLateWarps, true, 0, &s_abort, status);
+          int extra;
+          if constexpr (TM == 32)
+            extra = load_rows<8>(sS, out, rows, H, warp - C::kLate, C::kLateWarps, true, 0, &s_abort, status);
+          else
+            extra = state.load(out, sS, &s_abort, status);
           // Everything at the first look: a little earlier next time; else later.  (Looks that come too early
           // load the L2 that the states have to pass through.)
           pause = extra > 0 ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
