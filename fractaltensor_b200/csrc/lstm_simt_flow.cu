@@ -14,10 +14,9 @@
 //     multiplies per word it reads is the rate: 8 rows x 8 columns of one 32-wide K chunk, four products a word;
 //   * TM is 8, 16 or 32: small batches multiply no rows that are not there, and small models spread theirs
 //     over the device.
-// What bounds a step at 32 rows is the multiplication (4260 cycles alone, 6000 beside the early warps); at 8 rows
-// the trip of the state through L2 (2300 of 5500 cycles).  Against one serial pass (us, D x L x N x H): 4 x 64 x
-// 32 x 256 550 -> 482, 4 x 64 x 16 x 256 526 -> 264, 2 x 64 x 8 x 256 499 -> 202, 1 x 100 x 64 x 256 816 -> 361,
-// 3 x 64 x 20 x 192 441 -> 250.
+// A step of 32 rows in cycles: the recurrent half's multiplication 4200 of 10 000, its sums 800, two cells a thread 1160, the
+// state's trip and loads 3600; of 8 rows 1300, 400, 620 and 1500 of 4000.  Against one serial pass (us, D x L x N x H): 4 x 64 x 32 x
+// 256 550 -> 385, 4 x 64 x 16 x 256 526 -> 218, 2 x 64 x 8 x 256 499 -> 151.
 // The sums are the level kernel's (csrc/cell_simt.cu): every chunk of 32 in ascending order, a group's chunks in
 // order, the four groups in order; all fp32 schedules give the same bits.
 //
@@ -226,7 +225,8 @@ struct StateLoad {
 // ascending order of k, to p[c][TM][32].  Warp w of kMul, a half-warp to a chunk: a lane has rows ry, ry + G, ..
 // (neighbouring rows fall on different banks) and kCols columns, two of them to an FMA (fma.rn.f32x2: each
 // half rounds as fmaf does).  H 256, 148 CTAs, cycles of four warps at TM 8 / 16 / 32: 1306 / 2071 / 4260; scalar
-// with the next k's operands prefetched 1311 / 2114 / 4849.
+// with the next k's operands prefetched 1311 / 2114 / 4849.  (Before the loop over k was
+// unrolled whole: 4 x 64 x 32 x 256 431 -> 406 us; with the next operands prefetched by hand as well 410.)
 template <int TM>
 __device__ __forceinline__ void multiply_here(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
   constexpr int R = SimtFlowCfg<TM>::kRows, C = SimtFlowCfg<TM>::kCols, G = TM / R;
@@ -490,10 +490,10 @@ int launch(const SimtFlowArgs& a, size_t smem, cudaStream_t stream) {
 
 }  // namespace
 
-// How the kernel would run a problem; est_us: about what that takes.  False: not for this kernel.  Layers that do not fit on the device beside each other cost a sweep each.  Measured
-// steps, us, at H 64 / 128 / 192 / 256 / 320 / 384: 8 rows 2.7 / 2.9 / 3.1 / 3.2 / 4.3 / 4.5, 16 rows 3.4 / 3.4 / 3.7 /
-// 3.8 / 5.6 / 5.7, 32 rows 5.3 / 5.4 / 5.8 / 7.0.  A row of more than 256 is read in two rounds; 32 rows at H 256 leave
-// room for one input tile only.
+// How the kernel would run a problem; est_us: about what that takes.  False: not for this kernel.  Layers that do not fit on the
+// device beside each other cost a sweep each.  Measured steps, us, at H 64 / 128 / 192 / 256 / 320 / 384: 8 rows 1.75 / 1.8 / 1.9 /
+// 2.0 / 2.9 / 3.0, 16 rows - / 2.6 / - / 2.9 / 4.3 / 4.6, 32 rows - / - / 4.9 / 5.5.  A row of more than 256 is read in two rounds; 32
+// rows at H 256 leave room for one input tile only.
 bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFlowPlan* plan) {
   if (I != H || H % 64 != 0) return false;
   bool found = false;
@@ -504,9 +504,9 @@ bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFl
     const int per_sweep = std::min<int>(D, static_cast<int>(sm_count / tiles));
     const int sweeps = (D + per_sweep - 1) / per_sweep;
     const double h = H / 256.0;
-    const double step = tm == 8    ? 2.6 + 0.55 * h + (H > 256 ? 1.0 : 0.0)
-                        : tm == 16 ? 3.2 + 0.6 * h + (H > 256 ? 1.65 : 0.0)
-                                   : 5.0 + 0.8 * h + (H >= 256 ? 1.2 : 0.0);
+    const double step = tm == 8    ? 1.65 + 0.35 * h + (H > 256 ? 0.75 : 0.0)
+                        : tm == 16 ? 2.2 + 0.68 * h + (H > 256 ? 1.3 : 0.0)
+                                   : 4.1 + 1.1 * h + (H >= 256 ? 0.28 : 0.0);
     const double us = static_cast<double>(sweeps) * (L + per_sweep - 1) * step;
     if (!found || us < plan->est_us) *plan = {tm, us};
     found = true;
