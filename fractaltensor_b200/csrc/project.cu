@@ -1,6 +1,6 @@
 // Vocabulary projection with its softmax, probs = softmax(h . P) per row, without the logits in memory: the product is
-// computed twice.  The first pass keeps of every row and 128 columns the pair (maximum, sum of e^(x - maximum)) of the
-// online softmax (online_softmax.cu), the second multiplies again, puts the pairs of its rows together and writes
+// computed twice.  The first pass keeps of every row, pair of CTAs and half of its tiles the pair (maximum, sum of e^(x - maximum))
+// of the online softmax (online_softmax.cu), the second multiplies again, puts the pairs of its rows together and writes
 // e^(max(x - m, -64)) / d, the same number as the row kernel there.
 //
 // As a product into fp32 logits and a softmax over them, 2240 words x 10000 x 512 cost 33 + 35 us: 90 MB written, read and
@@ -13,7 +13,10 @@
 // (ftb_projection_pack), K-major.
 //
 //   warp 0        TMA producer (both CTAs)      warp 1        MMA issuer (leader)
-//   warps 4..11   epilogue: a row a thread, 128 columns of a tile a warp
+//   warps 4..11   epilogue, 128 columns of a tile a warp: a row a thread in the first pass; in the second accumulator fragments, of
+//                 which a quad has 8 neighbouring numbers of a row, one sector: they go to memory as they are.  (Through shared memory,
+//                 by stores of whole rows or by bulk copies, a tile took the MMAs 6100 cycles and not 4400: they read 64
+//                 bytes a cycle there.  2240 x 10000 x 512 58.4 -> 52.3 us, 7000 x 12000 x 256 141 -> 117.)
 #include <algorithm>
 #include <cfloat>
 
@@ -29,14 +32,13 @@ constexpr int kThreads = 384, kEpiWarps = 8;
 constexpr uint32_t kABlock = 128 * BK * 2, kBBlock = 128 * BK * 2;  // one K block of this CTA's rows, of its half of the columns
 constexpr int kMaxKBlocks = 10;   // H <= 640: 160 KB of rows, three K blocks of columns beside them
 constexpr int kMaxStages = 8;
-constexpr uint32_t kStaging = kEpiWarps * 2048;  // 16 rows x 32 numbers a warp
 constexpr uint32_t kSmemBudget = 229376;
 constexpr float kClamp = -64.f, kLog2e = 1.4426950408889634f;
 
 struct ProjectArgs {
   int T, V, H, kb, stages;
   int n_tiles, tiles;   // column tiles; all tiles
-  float2* stats;        // [2 n_tiles][T]
+  float2* stats;        // [2 n_tiles][T]: of a row block, two for each pair of CTAs that has tiles of it
   float* probs;
   long long ld;         // of probs
   int n_store;          // columns of probs that are written: V, or all of a padded row; a multiple of 4, as ld
@@ -82,7 +84,6 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const uint32_t rank = cluster_ctarank();
   uint8_t* sA = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sB = sA + a.kb * kABlock;
-  uint8_t* s_out = sB + a.stages * kBBlock;
   if (threadIdx.x == 0) {
     prefetch_tmap(&mapA);
     prefetch_tmap(&mapB);
@@ -117,6 +118,8 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const int G = gridDim.x >> 1, c = blockIdx.x >> 1;
   const int first = static_cast<int>(static_cast<long long>(a.tiles) * c / G);
   const int last = static_cast<int>(static_cast<long long>(a.tiles) * (c + 1) / G);
+  // The pair that has a tile.
+  auto pair_of = [&](int tile) { return static_cast<int>(((static_cast<long long>(tile) + 1) * G - 1) / a.tiles); };
 
   if (warp == 0) {
     if (elect_one()) {
@@ -200,72 +203,88 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
-    uint8_t* s_row = s_out + (warp - 4) * 2048;
     const uint32_t empty_bar[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
-    float m = 0.f, inv_d = 0.f, shift = 0.f, rest = 0.f, least = 0.f;  // second pass: of this thread's row
+    // First pass: the running pair of this thread's row.  Second: of four rows, lane / 4 and 8, 16, 24 further.
+    float top = -FLT_MAX, d = 0.f;
+    float inv_d[4], shift[4], rest[4], least[4];
     int before = -1;
     if (!kStats) grid_dependency_wait();
     for (int i = first; i < last; ++i) {
       const int mb = i / a.n_tiles, nb = i - mb * a.n_tiles, k = i - first, acc = k & 1;
       const int row0 = mb * 256 + static_cast<int>(rank) * 128 + q * 32, row = row0 + lane;
       const int col0 = nb * kTileN + half * 128;
-      if (!kStats && mb != before) {
+      if (mb != before) {
         before = mb;
-        m = -FLT_MAX;
-        float d = 0.f;
-        if (row < a.T) {
-          const float2* p = a.stats + row;
-          for (int e0 = 0; e0 < 2 * a.n_tiles; e0 += 16) {
-            float2 x[16];
+        if (kStats) {
+          top = -FLT_MAX;
+          d = 0.f;
+        } else {
+          // the pairs of this thread's row
+          const int entries = 2 * (pair_of((mb + 1) * a.n_tiles - 1) - pair_of(mb * a.n_tiles) + 1);
+          float m = -FLT_MAX, sum = 0.f;
+          if (row < a.T) {
+            const float2* p = a.stats + row;
+            for (int e0 = 0; e0 < entries; e0 += 16) {
+              float2 x[16];
 #pragma unroll
-            for (int e = 0; e < 16; ++e)
-              x[e] = e0 + e < 2 * a.n_tiles ? __ldcg(p + static_cast<long long>(e0 + e) * a.T) : make_float2(-FLT_MAX, 0.f);
-            float top = m;
+              for (int e = 0; e < 16; ++e)
+                x[e] = e0 + e < entries ? __ldcg(p + static_cast<long long>(e0 + e) * a.T) : make_float2(-FLT_MAX, 0.f);
+              float now = m;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) top = fmaxf(top, x[e].x);
-            const float r = exponent_of(top);
-            // (sums by halves: 80 additions one behind the other would cost what the exponentials' own error is)
-            float s[16];
+              for (int e = 0; e < 16; ++e) now = fmaxf(now, x[e].x);
+              const float r = exponent_of(now);
+              // (sums by halves: additions one behind the other would cost what the exponentials' own error is)
+              float s[16];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) s[e] = x[e].y * pow2_whole(exponent_of(x[e].x) - r);
+              for (int e = 0; e < 16; ++e) s[e] = x[e].y * pow2_whole(exponent_of(x[e].x) - r);
 #pragma unroll
-            for (int w = 8; w > 0; w >>= 1)
+              for (int w = 8; w > 0; w >>= 1)
 #pragma unroll
-              for (int e = 0; e < w; ++e) s[e] += s[e + w];
-            d = fmaf(d, pow2_whole(exponent_of(m) - r), s[0]);
-            m = top;
-          }
-          if (!plain(ref_of(m))) {  // (rare: once more, one pair after the other)
-            d = 0.f;
+                for (int e = 0; e < w; ++e) s[e] += s[e + w];
+              sum = fmaf(sum, pow2_whole(exponent_of(m) - r), s[0]);
+              m = now;
+            }
+            if (!plain(ref_of(m))) {  // (rare: once more, one pair after the other)
+              sum = 0.f;
 #pragma unroll 1
-            for (int e = 0; e < 2 * a.n_tiles; ++e) {
-              const float2 one = __ldcg(p + static_cast<long long>(e) * a.T);
-              d = fmaf(one.y, rescale(ref_of(one.x), ref_of(m)), d);
+              for (int e = 0; e < entries; ++e) {
+                const float2 one = __ldcg(p + static_cast<long long>(e) * a.T);
+                sum = fmaf(one.y, rescale(ref_of(one.x), ref_of(m)), sum);
+              }
             }
           }
+          const Ref ref = ref_of(m);
+          const float inv = 1.f / sum, low = fmaf(m, kLog2e, -ref.r) - ref.rest + kClamp * kLog2e;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int of = 8 * e + (lane >> 2);
+            inv_d[e] = __shfl_sync(0xffffffffu, inv, of);
+            shift[e] = __shfl_sync(0xffffffffu, -ref.r, of);
+            rest[e] = __shfl_sync(0xffffffffu, ref.rest, of);
+            least[e] = __shfl_sync(0xffffffffu, low, of);
+          }
         }
-        inv_d = 1.f / d;
-        const Ref ref = ref_of(m);
-        shift = -ref.r;
-        rest = ref.rest;
-        least = fmaf(m, kLog2e, shift) - rest + kClamp * kLog2e;
       }
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (k >> 1) & 1, &s_abort, status, FTB_ERR_TIMEOUT_MMA))) break;
       tc_fence_after();
-      float top = -FLT_MAX, d = 0.f;
-      Ref from = ref_of(top);
+      float tile_top = -FLT_MAX, tile_d = 0.f;
+      Ref from = ref_of(tile_top);
 #pragma unroll 1
       for (int ch = 0; ch < 4; ++ch) {
-        uint32_t r[32];
-        tmem_ld32(lane_addr + acc * kTileN + ch * 32, r);
-        tmem_ld_wait();
-        if (ch == 3) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_peer(empty_bar[acc]);
-        }
+        const uint32_t at = lane_addr + acc * kTileN + ch * 32;
         const int c0 = col0 + ch * 32;
+        auto release = [&] {  // the accumulator is in registers
+          tmem_ld_wait();
+          if (ch == 3) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_peer(empty_bar[acc]);
+          }
+        };
         if (kStats) {
+          uint32_t r[32];
+          tmem_ld32(at, r);
+          release();
           if (c0 >= a.V) continue;
           if (c0 + 32 > a.V) {
 #pragma unroll
@@ -279,45 +298,66 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
           for (int j = 8; j < 32; j += 8)
 #pragma unroll
             for (int e = 0; e < 4; ++e) mx[e] = fmax3(mx[e], __uint_as_float(r[j + e]), __uint_as_float(r[j + 4 + e]));
-          const float now = fmaxf(fmax3(top, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+          const float now = fmaxf(fmax3(tile_top, mx[0], mx[1]), fmaxf(mx[2], mx[3]));
           const Ref to = ref_of(now);
           float s[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) s[j] = exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -to.r) - to.rest);
 #pragma unroll
           for (int j = 8; j < 32; ++j) s[j & 7] += exp2_fast(fmaf(__uint_as_float(r[j]), kLog2e, -to.r) - to.rest);
-          d = fmaf(d, rescale(from, to), ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+          tile_d = fmaf(tile_d, rescale(from, to), ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
           from = to;
-          top = now;
+          tile_top = now;
         } else {
+          uint32_t r[2][2][8];  // 16 rows, 16 columns
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int w = 0; w < 2; ++w) tmem_ld_frag16(at + (static_cast<uint32_t>(16 * h) << 16) + 16 * w, r[h][w]);
+          release();
           if (c0 >= a.n_store) continue;
+          const int c = c0 + 2 * (lane & 3);
+          const int c_out = c0 + 2 * (lane & 2) + 8 * (lane & 1);  // first of the four that this lane stores of every 16
+          float* out = a.probs + static_cast<long long>(row0 + (lane >> 2)) * a.ld + c_out;
+          const bool whole = c0 + 32 <= a.V;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            r[j] = c0 + j < a.V ? __float_as_uint(exp2_fast(fmaxf(fmaf(__uint_as_float(r[j]), kLog2e, shift) - rest, least)) * inv_d) : 0u;
-          // A lane has a row of 32 numbers; a store covers whole rows: through shared memory, 16 rows at a time, 16-byte pieces
-          // exchanged within a row so that neither side meets a bank twice.
+          for (int e = 0; e < 4; ++e) {
+            auto prob = [&](uint32_t x) {
+              return exp2_fast(fmaxf(fmaf(__uint_as_float(x), kLog2e, shift[e]) - rest[e], least[e])) * inv_d[e];
+            };
+            float2 v[4];
 #pragma unroll
-          for (int part = 0; part < 32; part += 16) {
-            if ((lane & 16) == part) {
-#pragma unroll
-              for (int g = 0; g < 8; ++g)
-                *reinterpret_cast<uint4*>(s_row + (lane & 15) * 128 + ((g ^ (lane & 7)) << 4)) =
-                    make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+            for (int g = 0; g < 4; ++g) {  // eight columns each
+              const uint32_t* x = &r[e >> 1][g >> 1][4 * (g & 1) + 2 * (e & 1)];
+              v[g] = make_float2(prob(x[0]), prob(x[1]));
+              if (!whole) {
+                if (c + 8 * g >= a.V) v[g].x = 0.f;
+                if (c + 8 * g + 1 >= a.V) v[g].y = 0.f;
+              }
             }
-            __syncwarp();
-            const int piece = lane & 7;
+            // Neighbours trade two groups of columns, so that a thread has four numbers of one and a quad 16 of a row: even lanes
+            // keep groups 0 and 2, odd ones 1 and 3.
+            const bool odd = (lane & 1) != 0;
+            float* to = out + static_cast<long long>(8 * e) * a.ld;
 #pragma unroll
-            for (int g = 0; g < 16; g += 4) {
-              const int rr = g + (lane >> 3);
-              const float4 v = *reinterpret_cast<const float4*>(s_row + rr * 128 + ((piece ^ (rr & 7)) << 4));
-              if (row0 + part + rr < a.T && c0 + 4 * piece < a.n_store)
-                __stcs(reinterpret_cast<float4*>(a.probs + (row0 + part + rr) * a.ld + c0 + 4 * piece), v);
+            for (int g = 0; g < 4; g += 2) {
+              const float2 give = odd ? v[g] : v[g + 1], keep = odd ? v[g + 1] : v[g];
+              const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1));
+              if (row0 + 8 * e + (lane >> 2) < a.T && c_out + 8 * g < a.n_store)
+                __stcs(reinterpret_cast<float4*>(to + 8 * g),
+                       odd ? make_float4(got.x, got.y, keep.x, keep.y) : make_float4(keep.x, keep.y, got.x, got.y));
             }
-            __syncwarp();
           }
         }
       }
-      if (kStats && row < a.T) __stcg(a.stats + static_cast<long long>(2 * nb + half) * a.T + row, make_float2(top, d));
+      if (kStats) {  // (tile by tile: chunk by chunk through all of them adds up more roundings)
+        const float now = fmaxf(top, tile_top);
+        const Ref to = ref_of(now);
+        d = fmaf(d, rescale(ref_of(top), to), tile_d * rescale(from, to));
+        top = now;
+      }
+      if (kStats && row < a.T && (i + 1 == last || (i + 1) / a.n_tiles != mb))
+        __stcg(a.stats + static_cast<long long>(2 * (c - pair_of(mb * a.n_tiles)) + half) * a.T + row, make_float2(top, d));
     }
   }
 
@@ -356,8 +396,8 @@ int launch_passes(const CUtensorMap& mA, const CUtensorMap& mB, const ProjectArg
 
 // What the kernel takes, and where it is the faster form: rows that begin on 16 bytes (for others the stores go singly, and
 // cost what the logits did), and behind a packed operand only where the logits are many.  us, product and softmax / twice:
-// unpacked, H 512, V 10000: 40 words 22.5 / 21.0, 300 30.6 / 28.8, 2240 79.9 / 55.1, 5000 170 / 103; V 2000: 300 20.5 / 18.6, 5000 43.1 / 39.0;
-// packed: V 2004, 300 words 23.6 / 26.0, 5000 45.1 / 46.2; V 10004, 2240 words 83.3 / 67.7; V 10001, 2240 words 90.3 / 91.5.
+// unpacked, H 512, V 10000: 40 words 22.5 / 21.0, 300 30.6 / 28.8, 2240 79.9 / 52.3, 5000 170 / 94.6; V 2000: 300 20.5 / 18.6, 5000 43.1 / 39.0;
+// packed: V 2004, 300 words 23.6 / 26.0, 5000 45.1 / 46.2; V 10004, 2240 words 83.3 / 69.0; V 10001, 2240 words 90.3 / 91.5.
 bool project_twice_supported(int dtype, long long T, int V, int H, bool unpacked) {
   return (dtype == FTB_F16 || dtype == FTB_BF16) && H % BK == 0 && H <= kMaxKBlocks * BK &&
          (unpacked ? V % 8 == 0 : V % 4 == 0 && T * V >= 16000000);
@@ -374,12 +414,12 @@ int launch_project_twice(int dtype, const void* h, const void* P, bool unpacked,
   const long long tiles = static_cast<long long>((T + 255) / 256) * a.n_tiles;
   if (tiles > 0x7fffffffLL) return FTB_ERR_ARG;
   a.tiles = static_cast<int>(tiles);
-  a.stages = std::min<int>(kMaxStages, (kSmemBudget - kStaging - a.kb * kABlock) / kBBlock);
+  a.stages = std::min<int>(kMaxStages, (kSmemBudget - a.kb * kABlock) / kBBlock);
   a.stats = static_cast<float2*>(scratch);
   a.probs = probs;
   a.ld = ld;
   a.n_store = static_cast<int>(ld);
-  const uint32_t smem = a.kb * kABlock + a.stages * kBBlock + kStaging + 1024;
+  const uint32_t smem = a.kb * kABlock + a.stages * kBBlock + 1024;
   CUtensorMap mA, mB;
   int rc;
   if ((rc = make_tmap_2d(&mA, h, dtype, T, H, H, 128, BK))) return rc;
