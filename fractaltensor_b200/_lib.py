@@ -94,6 +94,7 @@ class _NoHost:
         return None
 
     b2b_gemm = flash_attention = sparse_attention = _decline
+    embedding_gather = lstm_pack_weights = lstm_stacked_ragged = project_softmax = _decline
 
     @staticmethod
     def current_stream(dev):

@@ -5,7 +5,8 @@
 // host time per call: such a call was bound by the host, whatever the kernel did.  The functions here
 // take the call's objects as they are, read shapes, types and pointers from the tensors in C++,
 // allocate the result through the same caching allocator and enter the C ABI with the current
-// stream of the inputs' device (4..6 us per call, most of it the allocation and the launch).
+// stream of the inputs' device (4..6 us per call, most of it the allocation and the launch).  The calls of the word
+// program (lookup, packing, ragged LSTM, projection) are here too: a pass of a small model was bound by their host time.
 //
 // They are the accepting half only: whatever is not the plain, valid call (a wrong type or shape, a
 // tensor on the CPU, no workspace on that device yet, no memory for the result) is answered with
@@ -18,6 +19,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/version.h>
+
+#include <algorithm>
+#include <vector>
 
 #include "../../include/ftb200.h"
 
@@ -235,6 +239,151 @@ PyObject* sparse_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   });
 }
 
+// (table, ids, out, workspaces)
+PyObject* embedding_gather(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 4);
+    const at::Tensor *table = cuda_tensor(args[0]), *ids = cuda_tensor(args[1]);
+    DECLINE_UNLESS(table && ids && table->dim() == 2 && ids->scalar_type() == at::kLong && ids->device() == table->device());
+    const int64_t V = table->size(0), H = table->size(1), T = ids->numel();
+    const int dt = dtype_code(*table);
+    DECLINE_UNLESS(dt >= 0 && H <= 0x7fffffff);
+    const c10::DeviceIndex dev = table->device().index();
+    const at::Tensor ws = workspace_of(args[3], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws.defined());
+    at::Tensor out;
+    DECLINE_UNLESS(given_result(args[2], *table, {T, H}, &out));
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::cuda::CUDAGuard guard(dev);
+      if (!out.defined()) out = new_result(*table, {T, H});
+      rc = ftb_embedding_gather(table->data_ptr(), static_cast<const long long*>(ids->data_ptr()), out.data_ptr(), T, V,
+                                static_cast<int>(H), dt, ws.data_ptr(), ws.numel(), stream_of(dev));
+    }
+    return rc == 0 ? THPVariable_Wrap(out) : PyLong_FromLong(rc);
+  });
+}
+
+// (W, U, bias | None) -> (Wp, bias_p | None)
+PyObject* lstm_pack_weights(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 3);
+    const at::Tensor *W = cuda_tensor(args[0]), *U = cuda_tensor(args[1]);
+    DECLINE_UNLESS(W && U && same_kind(*W, *U) && W->dim() == 4 && U->dim() == 4);
+    const int64_t D = W->size(0), I = W->size(2), H = W->size(3);
+    DECLINE_UNLESS(W->size(1) == 4 && U->size(0) == D && U->size(1) == 4 && U->size(2) == H && U->size(3) == H);
+    DECLINE_UNLESS(D <= 0x7fffffff && I <= 0x7fffffff && H <= 0x7fffffff);
+    const at::Tensor* b = nullptr;
+    if (args[2] != Py_None) {
+      b = cuda_tensor(args[2]);
+      DECLINE_UNLESS(b && same_kind(*b, *W) && b->numel() == D * 4 * H);
+    }
+    const int dt = dtype_code(*W);
+    DECLINE_UNLESS(dt >= 0);
+    at::Tensor Wp, bias_p;
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::DeviceIndex dev = W->device().index();
+      const c10::cuda::CUDAGuard guard(dev);
+      Wp = new_result(*W, {D, 4 * H, I + H});
+      if (b) bias_p = at::empty({D, 4 * H}, at::TensorOptions().dtype(at::kFloat).device(W->device()));
+      rc = ftb_lstm_pack_weights(W->data_ptr(), U->data_ptr(), b ? b->data_ptr() : nullptr, Wp.data_ptr(),
+                                 b ? static_cast<float*>(bias_p.data_ptr()) : nullptr, static_cast<int>(D), static_cast<int>(I),
+                                 static_cast<int>(H), dt, stream_of(dev));
+    }
+    if (rc != 0) return PyLong_FromLong(rc);
+    PyObject* bias = Py_None;
+    if (b) bias = THPVariable_Wrap(bias_p); else Py_INCREF(bias);
+    return Py_BuildValue("(NN)", THPVariable_Wrap(Wp), bias);
+  });
+}
+
+// (x, lens, Wp, bias_p | None, workspace): the caller holds the workspace's turn
+PyObject* lstm_stacked_ragged(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 5);
+    const at::Tensor *x = cuda_tensor(args[0]), *Wp = cuda_tensor(args[2]), *ws = cuda_tensor(args[4]);
+    DECLINE_UNLESS(x && Wp && ws && same_kind(*x, *Wp) && ws->device() == x->device() && ws->scalar_type() == at::kByte);
+    DECLINE_UNLESS(x->dim() == 2 && Wp->dim() == 3 && PyList_CheckExact(args[1]));
+    const Py_ssize_t N = PyList_GET_SIZE(args[1]);
+    DECLINE_UNLESS(N > 0 && N <= 0x7fffffff);
+    std::vector<int> lens(static_cast<size_t>(N));
+    int64_t T = 0;
+    int L = 0;
+    for (Py_ssize_t i = 0; i < N; ++i) {
+      int64_t v;
+      DECLINE_UNLESS(get_int(PyList_GET_ITEM(args[1], i), &v) && v > 0);
+      lens[i] = static_cast<int>(v);
+      L = std::max(L, lens[i]);
+      T += v;
+    }
+    const int64_t D = Wp->size(0), H = Wp->size(1) / 4, I = x->size(1);
+    DECLINE_UNLESS(x->size(0) == T && Wp->size(1) == 4 * H && Wp->size(2) == I + H && D <= 0x7fffffff && I + H <= 0x7fffffff);
+    const at::Tensor* b = nullptr;
+    if (args[3] != Py_None) {
+      b = cuda_tensor(args[3]);
+      DECLINE_UNLESS(b && b->scalar_type() == at::kFloat && b->device() == x->device() && b->dim() == 2 && b->size(0) == D &&
+                     b->size(1) == 4 * H);
+    }
+    const int dt = dtype_code(*x);
+    DECLINE_UNLESS(dt >= 0);
+    at::Tensor out;
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::DeviceIndex dev = x->device().index();
+      const c10::cuda::CUDAGuard guard(dev);
+      const auto bytes = at::TensorOptions().dtype(at::kByte).device(x->device());
+      // the packed input, and behind it the rows' tables, the call's own: they are read again behind the LSTM
+      const int64_t rows = x->numel() * x->element_size();
+      const size_t tables = ftb_lstm_stacked_ragged_scratch_bytes(L, static_cast<int>(N));
+      const at::Tensor xt = at::empty({rows + static_cast<int64_t>(tables)}, bytes);
+      const at::Tensor hs = new_result(*x, {D, T, H});
+      const at::Tensor c = at::empty({D, N, H}, bytes.dtype(at::kFloat));
+      out = new_result(*x, {T, H});
+      rc = ftb_lstm_stacked_ragged_fwd_scratch(x->data_ptr(), Wp->data_ptr(), b ? static_cast<const float*>(b->data_ptr()) : nullptr,
+                                               lens.data(), xt.data_ptr(), hs.data_ptr(), static_cast<float*>(c.data_ptr()),
+                                               out.data_ptr(), static_cast<int>(D), static_cast<int>(N), static_cast<int>(I),
+                                               static_cast<int>(H), dt, static_cast<char*>(xt.data_ptr()) + rows, tables,
+                                               ws->data_ptr(), ws->numel(), stream_of(dev));
+    }
+    return rc == 0 ? THPVariable_Wrap(out) : PyLong_FromLong(rc);
+  });
+}
+
+// (h, P, workspaces): probabilities from P [H, V] as it is
+PyObject* project_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    DECLINE_UNLESS(n == 3);
+    const at::Tensor *h = cuda_tensor(args[0]), *P = cuda_tensor(args[1]);
+    DECLINE_UNLESS(h && P && same_kind(*h, *P) && P->dim() == 2 && h->dim() > 0);
+    const int64_t H = P->size(0), V = P->size(1);
+    DECLINE_UNLESS(h->size(-1) == H && H > 0 && H % 64 == 0 && V > 0 && V % 8 == 0 && V <= 48 * 1024);
+    const int64_t T = h->numel() / H;
+    const int dt = dtype_code(*h);
+    DECLINE_UNLESS(dt >= 0 && T > 0 && (reinterpret_cast<uintptr_t>(h->data_ptr()) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(P->data_ptr()) & 15) == 0);
+    const size_t bytes = ftb_project_softmax_scratch_bytes(T, static_cast<int>(V), static_cast<int>(H), dt, 1);
+    DECLINE_UNLESS(bytes > 0);
+    const c10::DeviceIndex dev = h->device().index();
+    const at::Tensor ws = workspace_of(args[2], dev, ftb_workspace_bytes());
+    DECLINE_UNLESS(ws.defined());
+    at::Tensor probs;
+    int rc;
+    {
+      const WithoutGil released;
+      const c10::cuda::CUDAGuard guard(dev);
+      probs = at::empty({T, V}, at::TensorOptions().dtype(at::kFloat).device(h->device()));
+      const at::Tensor scratch = at::empty({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).device(h->device()));
+      rc = ftb_project_softmax_fwd(h->data_ptr(), P->data_ptr(), 1, static_cast<float*>(probs.data_ptr()), V, T, static_cast<int>(V),
+                                   static_cast<int>(H), dt, scratch.data_ptr(), bytes, ws.data_ptr(), ws.numel(), stream_of(dev));
+    }
+    return rc == 0 ? THPVariable_Wrap(probs) : PyLong_FromLong(rc);
+  });
+}
+
 // (device index, -1: the current one) -> handle of its current stream.  (torch.cuda.current_stream makes a
 // stream object for it: 2 us, three times in a call of the word program.)
 PyObject* current_stream(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -258,6 +407,10 @@ PyMethodDef kMethods[] = {
     {"b2b_gemm", as_method(b2b_gemm), METH_FASTCALL, nullptr},
     {"flash_attention", as_method(flash_attention), METH_FASTCALL, nullptr},
     {"sparse_attention", as_method(sparse_attention), METH_FASTCALL, nullptr},
+    {"embedding_gather", as_method(embedding_gather), METH_FASTCALL, nullptr},
+    {"lstm_pack_weights", as_method(lstm_pack_weights), METH_FASTCALL, nullptr},
+    {"lstm_stacked_ragged", as_method(lstm_stacked_ragged), METH_FASTCALL, nullptr},
+    {"project_softmax", as_method(project_softmax), METH_FASTCALL, nullptr},
     {"current_stream", as_method(current_stream), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

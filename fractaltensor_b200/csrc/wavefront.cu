@@ -734,9 +734,10 @@ level_schedule:
   return FTB_OK;
 }
 
-int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
-                                const int* active_rows, int D, int L, int I, int H, int dtype, const int* tuning,
-                                void* workspace, size_t workspace_bytes, void* stream_) {
+// first_rows: the first row of every step and their number, [L + 1], on the device already, or nullptr.
+static int stacked_varlen(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* active_rows,
+                          const int* first_rows, int D, int L, int I, int H, int dtype, const int* tuning, void* workspace,
+                          size_t workspace_bytes, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const Tuning tune(tuning);
   if (!x || !Wp || !hs || !c || !active_rows || D <= 0 || L <= 0 || !valid_dtype(dtype)) return FTB_ERR_ARG;
@@ -836,10 +837,13 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
   // the generic schedule takes about 14 us a step and group of layers at any size
   if (tune.schedule == 5 || (tune.schedule == 0 && can_flow && flow.est_us < ((D + G - 1) / G) * (L + G - 1) * 10.0)) {
     char* ws = static_cast<char*>(workspace);
-    std::vector<int> first(off.begin(), off.end());
-    if (cudaMemcpyAsync(ws + lay.total, first.data(), sizeof(int) * (L + 1), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-      return FTB_ERR_LAUNCH;
-    rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, reinterpret_cast<int*>(ws + lay.total), T, D, L, N, I, H, flow,
+    if (first_rows == nullptr) {
+      std::vector<int> first(off.begin(), off.end());
+      if (cudaMemcpyAsync(ws + lay.total, first.data(), sizeof(int) * (L + 1), cudaMemcpyHostToDevice, stream) != cudaSuccess)
+        return FTB_ERR_LAUNCH;
+      first_rows = reinterpret_cast<int*>(ws + lay.total);
+    }
+    rc = launch_lstm_flow(dtype, x, Wp, bias_p, hs, c, first_rows, T, D, L, N, I, H, flow,
                           reinterpret_cast<int*>(ws + lay.total + off_bytes), status, stream);
     if (rc != FTB_ERR_LAUNCH || tune.schedule != 0) return rc;
   }
@@ -915,6 +919,12 @@ int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias
     }
   }
   return FTB_OK;
+}
+
+int ftb_lstm_stacked_varlen_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
+                                const int* active_rows, int D, int L, int I, int H, int dtype, const int* tuning,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+  return stacked_varlen(x, Wp, bias_p, hs, c, active_rows, nullptr, D, L, I, H, dtype, tuning, workspace, workspace_bytes, stream);
 }
 
 int ftb_lstm_flow_form_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c, const int* active_rows,
@@ -1020,8 +1030,7 @@ int ftb_lstm_stacked_ragged_fwd_scratch(const void* x, const void* Wp, const flo
   const long long es = static_cast<long long>(dtype_size(dtype));
   rc = launch_ragged_rows(x, xt, d_start, d_off, N, L, I * es, true, stream);
   if (rc) return rc;
-  rc = ftb_lstm_stacked_varlen_fwd(xt, Wp, bias_p, hs, c, active.data(), D, L, I, H, dtype, nullptr, workspace, packed_bytes,
-                                   stream_);
+  rc = stacked_varlen(xt, Wp, bias_p, hs, c, active.data(), d_off, D, L, I, H, dtype, nullptr, workspace, packed_bytes, stream_);
   if (rc) return rc;
   return launch_ragged_rows(static_cast<const char*>(hs) + static_cast<size_t>(D - 1) * T * H * es, out, d_start, d_off, N, L,
                             H * es, false, stream);

@@ -137,6 +137,9 @@ def check_status(device=None):
 # ----------------------------------------------------------------------- LSTM
 def lstm_pack_weights(W, U, bias=None):
     """W: [D,4,I,H], U: [D,4,H,H], bias: [D,4,H] or [D,4,1,H] -> (Wp [D,4H,I+H], bias_p fp32 [D,4H] | None)."""
+    done = host.lstm_pack_weights(W, U, bias)
+    if done is not None:
+        return _done(done, "ftb_lstm_pack_weights")
     _req(W, "W")
     _req(U, "U", W.dtype)
     D, four, I, H = W.shape
@@ -229,6 +232,12 @@ def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
     """Stacked LSTM over a batch of sequences of different lengths, one behind the other and in any order.
 
     x: [T,I] with T = sum(lens), lens: N positive ints; Wp: [D,4H,I+H] -> the top layer's states [T,H] in x's order."""
+    if type(lens) is list and lens and isinstance(x, torch.Tensor) and x.is_cuda and isinstance(Wp, torch.Tensor) and Wp.dim() == 3:
+        ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(Wp.shape[0], max(lens)))
+        with _turn(ws):
+            done = host.lstm_stacked_ragged(x, lens, Wp, bias_p, ws)
+        if done is not None:
+            return _done(done, "ftb_lstm_stacked_ragged_fwd_scratch")
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)
     N, L, T = len(lens), max(lens), sum(lens)
@@ -572,6 +581,9 @@ def _project_twice(h, P, unpacked, probs, ld, T, V, H):
 def project_softmax_rows(h, P):
     """softmax(h . P) per row into a contiguous fp32 [T,V]: h [..., H], P [H,V] as it is where the kernel reads it
     (V a multiple of 8, 16-byte rows), else packed first."""
+    done = host.project_softmax(h, P, _workspaces)
+    if done is not None:
+        return _done(done, "ftb_project_softmax_fwd")
     _req(h, "h")
     _req(P, "P", h.dtype)
     H = h.shape[-1]
@@ -632,6 +644,9 @@ def lstm_project_softmax_rows(h, Pt, V):
 
 def embedding_gather(table, ids, out=None):
     """table: [V,H]; ids: int64 [T] (any nesting flattened) -> out [T,H] = table[ids]."""
+    done = host.embedding_gather(table, ids, out, _workspaces)
+    if done is not None:
+        return _done(done, "ftb_embedding_gather")
     _req(table, "table")
     _req(ids, "ids", torch.int64)
     if table.dim() != 2:

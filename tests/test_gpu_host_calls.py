@@ -76,3 +76,44 @@ def test_an_error_of_the_library_is_raised_without_a_second_call(monkeypatch):
             call()
         assert e.value.code == 1
     assert again == []
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.float32])
+def test_calls_of_the_word_program_through_python_and_native(monkeypatch, dt):
+    """The same results through the native front and through the Python checks, and the same errors."""
+    from fractaltensor_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: (torch.randn(*s, device="cuda", generator=g) * 0.1).to(dt)
+    D, H, V, lens = 2, 64, 2008, [3, 7, 1, 7]
+    T = sum(lens)
+    table, ids = r(50, H), torch.randint(0, 50, (T,), device="cuda", generator=g)
+    W, U, b, P = r(D, 4, H, H), r(D, 4, H, H), r(D, 4, 1, H), r(H, V)
+
+    def program():
+        x = ops.embedding_gather(table, ids)
+        Wp, bias = ops.lstm_pack_weights(W, U, b)
+        Wp0, none = ops.lstm_pack_weights(W, U)
+        h = ops.lstm_stacked_ragged(x, lens, Wp, bias)
+        return [x, Wp, bias, Wp0, h, ops.lstm_stacked_ragged(x, lens, Wp)] + ([ops.project_softmax_rows(h, P)] if dt != torch.float32 else []), none
+
+    def errors():
+        x, (Wp, bias) = ops.embedding_gather(table, ids), ops.lstm_pack_weights(W, U, b)
+        out = []
+        for call in (lambda: ops.embedding_gather(table, ids.int()), lambda: ops.embedding_gather(table, ids, x[1:]),
+                     lambda: ops.lstm_pack_weights(W, U[:1], b), lambda: ops.lstm_pack_weights(W, U, b[:1]),
+                     lambda: ops.lstm_stacked_ragged(x, [3, 7, 1], Wp, bias), lambda: ops.lstm_stacked_ragged(x, [3, 8, 0, 7], Wp, bias),
+                     lambda: ops.lstm_stacked_ragged(x, lens, Wp, bias[:, 1:]), lambda: ops.lstm_stacked_ragged(x[:, ::2], lens, Wp, bias),
+                     lambda: ops.project_softmax_rows(x, P[:32])):
+            with pytest.raises(Exception) as e:
+                call()
+            out.append(type(e.value))
+        return out
+
+    native, none = program()
+    assert none is None
+    wrong = errors()
+    ops.check_status()
+    monkeypatch.setattr(ops, "host", type("Host", (_lib._NoHost,), {"current_stream": staticmethod(_lib.host.current_stream)}))
+    plain, _ = program()
+    assert all(torch.equal(a, b) for a, b in zip(native, plain)) and wrong == errors()
+    ops.check_status()

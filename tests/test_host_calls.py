@@ -14,6 +14,15 @@ def test_declines_what_is_not_a_cuda_tensor():
     assert host.sparse_attention(q, q, q, None, None, 5, 2, 3, 1.0, False, {}) is None
 
 
+def test_calls_of_the_word_program_decline_too():
+    from fractaltensor_b200._lib import host
+    t = torch.zeros(8, 64, dtype=torch.float16)
+    assert host.embedding_gather(t, torch.zeros(3, dtype=torch.int64), None, {}) is None
+    assert host.lstm_pack_weights(torch.zeros(1, 4, 64, 64), torch.zeros(1, 4, 64, 64), None) is None
+    assert host.lstm_stacked_ragged(t, [8], torch.zeros(1, 256, 128), None, t) is None
+    assert host.project_softmax(t, t, {}) is None
+
+
 def _import_with(prelude):
     """Runs `prelude` and imports the package in a process of its own -> what it printed."""
     import os
