@@ -256,7 +256,7 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
           if (lane == 0) ok = flag_wait_ge(g.flags + (cell * g.S + ch.s) * 2 + ydir, g.tiles, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          fence_proxy_async_all();  // threads of other CTAs stored what TMA reads
+          fence_proxy_async_global();  // threads of other CTAs stored what TMA reads
         }
         ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
         if (!ok) break;
@@ -302,8 +302,7 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
             break;
           }
           __threadfence_block();
-          fence_proxy_async_all();
-          __threadfence();
+          // (The release takes the other warps' stores along; the proxy fence is the reader's, between its acquire and its copy.)
           const int64_t cell = (static_cast<int64_t>(ch.d) * g.A + ch.a) * g.B + b;
           red_release_gpu_add(g.flags + (cell * g.S + ch.s) * 2 + ydir, 1);
         }

@@ -375,7 +375,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           ok = n > 0;
           if (!ok) break;
           ready = t + n;
-          fence_proxy_async_all();  // threads of other CTAs stored what TMA reads
+          fence_proxy_async_global();  // threads of other CTAs stored what TMA reads
         }
         ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
         if (!ok) break;
@@ -434,8 +434,7 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
           break;
         }
         __threadfence_block();
-        fence_proxy_async_all();
-        __threadfence();
+        // (The release takes the other warps' stores along; the proxy fence is the reader's, between its acquire and its copy.)
         red_release_gpu_add(a.flags + (static_cast<int64_t>(l) * a.flag_steps + t) * a.S + slice, 1);
       }
     }

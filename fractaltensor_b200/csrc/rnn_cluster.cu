@@ -321,7 +321,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
             // (Producers write their outputs with TMA stores and consumers read them with TMA loads: both
             // sides are in the async proxy, so the flag's release/acquire is all the ordering there is.
             // Threads store the output of flow::body.)
-            if (lane == 0 && s == 0 && layer > 0 && a.fold[layer - 1] > 0) fence_proxy_async_all();
+            if (lane == 0 && s == 0 && layer > 0 && a.fold[layer - 1] > 0) fence_proxy_async_global();
           }
           ACCT_END(0);
           bool fine = true;
