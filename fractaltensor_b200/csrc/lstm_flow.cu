@@ -208,19 +208,19 @@ bool lstm_flow_plan(int dtype, int D, int L, int N, int64_t T, int I, int H, int
     const Fit f = fit(nb, pair, I, H);
     if (f.slots < 1 || (f.ring > 0 && !stream)) continue;
     // A step, what every layer adds to the first's start, a sweep's weights, the states' share of L2 and the call itself, fitted
-    // to 680 calls on every slice that fits (within 20 %, 5 % in the root mean square).  A sweep begins when its CTAs are done
-    // with the one before and the layer below has begun.
+    // to 5277 calls on every form that fits (3 to 7 % in the root mean square; of the forms of a call the one taken is 0.3 % behind
+    // the fastest on average, 15 % at most).  A sweep begins when its CTAs are done with the one before and the layer below has begun.
     const double h = H / 512.0, over = std::max(0.0, h - 1.0);
-    double step = pair ? (nb == 16   ? 1.56 + 0.08 * h + 0.75 * over
-                          : nb == 32 ? 1.35 + 0.57 * h + 0.30 * over
-                          : nb == 64 ? 1.78 + 0.70 * h + 2.36 * over
-                                     : 2.31 + 1.65 * h)
-                       : (nb == 16 ? 1.17 + 0.53 * h : nb == 32 ? 1.35 + 0.65 * h : 1.67 + 1.04 * h);
+    double step = pair ? (nb == 16   ? 1.24 + 0.42 * h + 0.32 * over
+                          : nb == 32 ? 1.37 + 0.43 * h + 0.44 * over
+                          : nb == 64 ? 1.84 + 0.76 * h + 0.77 * over
+                                     : 2.20 + 1.41 * h + 0.30 * over)
+                       : (nb == 16 ? 1.11 + 0.57 * h : nb == 32 ? 1.13 + 0.78 * h : 1.55 + 1.26 * h);
     // A block that passes through the ring costs its turn of the MMA warp, and all of them together their bytes from L2.
     const double mb = 1e-6 * S * tiles * G * f.streamed * kWBlockBytes;
-    if (f.ring > 0) step += nb <= 32 ? 0.083 * f.streamed + 0.026 * mb : 0.015 * f.streamed + 0.036 * mb;
-    const double steps = L * step, start = (G - 1) * (step + 3.1);
-    const double us = 14.0 + (sweeps - 1) * std::max(steps, start) + steps + start + 4.7 * sweeps + 3.3e-6 * D * T * H;
+    if (f.ring > 0) step += nb == 16 ? 0.094 * f.streamed + 0.020 * mb : nb == 32 ? 0.082 * f.streamed + 0.020 * mb : 0.078 * f.streamed + 0.018 * mb;
+    const double steps = L * step, start = (G - 1) * (step + 2.3);
+    const double us = 12.5 + (sweeps - 1) * std::max(steps, start) + steps + start + 4.7 * sweeps + 3.3e-6 * D * T * H;
     if (!found || us < plan->est_us) *plan = {nb, S, G, pair, f.ring, us};
     found = true;
   }
