@@ -224,9 +224,11 @@ struct StateLoad {
 // Products of the TM rows A[row][lda] with W[k][kLdW], n_chunks (even) chunks of 32 wide; chunk c's sums, in
 // ascending order of k, to p[c][TM][32].  Warp w of kMul, a half-warp to a chunk: a lane has rows ry, ry + G, ..
 // (neighbouring rows fall on different banks) and kCols columns, two of them to an FMA (fma.rn.f32x2: each
-// half rounds as fmaf does).  H 256, 148 CTAs, cycles of four warps at TM 8 / 16 / 32: 1306 / 2071 / 4260; scalar
-// with the next k's operands prefetched 1311 / 2114 / 4849.  (Before the loop over k was
-// unrolled whole: 4 x 64 x 32 x 256 431 -> 406 us; with the next operands prefetched by hand as well 410.)
+// half rounds as fmaf does).  H 256, 148 CTAs, cycles of four warps alone at TM 8 / 16 / 32, unrolled whole: 1100 / 1750 / 3250 (packed
+// FMAs on registers alone would take 650 / 1300 / 2600).  The loop over k is unrolled whole at 8 and 16 rows (4 x 64 x 16 x 256 219 us,
+// by eight k 233).  At 32 rows that is 27 KB of code: two SMs share what fetches it, and where their CTAs are not in step, with
+// tiles of different heights or layers beside each other, everything on both of them took up to 1.8 times as long.
+// Four k at a time, us whole / four: 3 layers of 64 steps, H 192, 36 sequences 455 / 365, 32 350 / 362; 4 of H 128, 43 449 / 352.
 template <int TM>
 __device__ __forceinline__ void multiply_here(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
   constexpr int R = SimtFlowCfg<TM>::kRows, C = SimtFlowCfg<TM>::kCols, G = TM / R;
@@ -235,7 +237,8 @@ __device__ __forceinline__ void multiply_here(const float* A, const float* W, in
     uint64_t acc[R][C / 2] = {};
     const float* a = A + ry * lda + c * kLdChunk;
     const float* b = W + c * TK * kLdW + C * cx;
-#pragma unroll
+    constexpr int kUnroll = TM == 32 ? 2 : TK / 2;
+#pragma unroll kUnroll
     for (int k = 0; k < TK; k += 2, a += 2, b += 2 * kLdW) {
       float2 av[R];
 #pragma unroll
@@ -267,16 +270,16 @@ __device__ __forceinline__ void multiply_here(const float* A, const float* W, in
   }
 }
 
-// (A call, where inlining it leaves the rest of the kernel too few registers: at 32 rows 384 us for 4 x 64 x 32 x 256 against 403;
-// at 8 rows 155 against 151 for 2 x 64 x 8 x 256.)
+// (A call at 16 rows, where inlining it leaves the rest of the kernel too few registers.  At 8 rows 151 us inlined against 155 for
+// 2 x 64 x 8 x 256; at 32 rows, with four k at a time, 383 against 426 for 4 x 64 x 32 x 256.)
 template <int TM>
 __device__ __noinline__ void multiply_call(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
   multiply_here<TM>(A, W, lda, n_chunks, p, w);
 }
 template <int TM>
 __device__ __forceinline__ void multiply(const float* A, const float* W, int lda, int n_chunks, float* p, int w) {
-  if constexpr (TM == 8) multiply_here<TM>(A, W, lda, n_chunks, p, w);
-  else multiply_call<TM>(A, W, lda, n_chunks, p, w);
+  if constexpr (TM == 16) multiply_call<TM>(A, W, lda, n_chunks, p, w);
+  else multiply_here<TM>(A, W, lda, n_chunks, p, w);
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -492,8 +495,7 @@ int launch(const SimtFlowArgs& a, size_t smem, cudaStream_t stream) {
 
 // How the kernel would run a problem; est_us: about what that takes.  False: not for this kernel.  Layers that do not fit on the
 // device beside each other cost a sweep each.  Measured steps, us, at H 64 / 128 / 192 / 256 / 320 / 384: 8 rows 1.75 / 1.8 / 1.9 /
-// 2.0 / 2.9 / 3.0, 16 rows - / 2.6 / - / 2.9 / 4.3 / 4.6, 32 rows - / - / 4.9 / 5.5.  A row of more than 256 is read in two rounds; 32
-// rows at H 256 leave room for one input tile only.
+// 2.0 / 2.9 / 3.0, 16 rows - / 2.6 / 2.7 / 2.85 / 4.3 / 4.6, 32 rows 4.7 / 4.85 / 5.05 / 5.3.  A row of more than 256 is read in two rounds.
 bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFlowPlan* plan) {
   if (I != H || H % 64 != 0) return false;
   bool found = false;
@@ -506,7 +508,7 @@ bool lstm_simt_flow_plan(int D, int L, int N, int I, int H, int sm_count, SimtFl
     const double h = H / 256.0;
     const double step = tm == 8    ? 1.65 + 0.35 * h + (H > 256 ? 0.75 : 0.0)
                         : tm == 16 ? 2.2 + 0.68 * h + (H > 256 ? 1.3 : 0.0)
-                                   : 4.1 + 1.1 * h + (H >= 256 ? 0.28 : 0.0);
+                                   : 4.44 + 0.83 * h;
     const double us = static_cast<double>(sweeps) * (L + per_sweep - 1) * step;
     if (!found || us < plan->est_us) *plan = {tm, us};
     found = true;
