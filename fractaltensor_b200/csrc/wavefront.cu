@@ -611,7 +611,7 @@ int ftb_lstm_stacked_fwd(const void* x, const void* Wp, const float* bias_p, voi
       // 5 names it, 2 to 4 the other one).  A step of its is shorter, but its tiles need more CTAs where 32 rows do
       // not fit beside the weights (H of 320 and more) or the batch is large, and layers that do not fit beside each
       // other cost a sweep each: the automatic choice takes the one with the smaller estimate (us, this one / the other,
-      // L 64: D 3, N 32 at H 256 480 / 523, at H 320 1075 / 638; D 3, N 16, H 320 390 / 582; D 3, N 200, H 64 650 / 512).
+      // L 64: D 3, N 32 at H 256 367 / 517, at H 320 859 / 626; D 3, N 16, H 320 315 / 580; D 3, N 200, H 64 487 / 507).
       SimtFlowPlan flow;
       const bool can_flow = lstm_simt_flow_plan(D, L, N, I, H, cl.sm_count, &flow);
       if (can_flow && (schedule == 5 || (schedule == 0 && flow.est_us < lstm_simt_static_us(D, L, N, I, H, cl.sm_count))))
