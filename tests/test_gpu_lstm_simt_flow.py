@@ -40,6 +40,21 @@ def test_same_bits_as_levels(ops, D, L, N, H, schedule):
         assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
 
 
+@pytest.mark.parametrize("D,L,N,H", [
+    (3, 24, 36, 192),  # 4 rows: no second cell of a thread
+    (4, 40, 48, 128),  # 16: every first cell and no second one
+    (2, 20, 49, 256),  # 17: one second cell
+])
+def test_short_tile_beside_full_ones_of_32_rows(ops, D, L, N, H):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    Wp, b = _params(ops, D, H, g)
+    x = torch.randn(L, N, H, device="cuda", generator=g)
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1)
+    h, c = ops.lstm_stacked(x, Wp, b, schedule=5)
+    ops.check_status()
+    assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
 def test_nan_states_are_states(ops):
     """A NaN hidden state is a value like any other (0x7FFFFFFF, not the fill pattern): nothing waits for it."""
     g = torch.Generator(device="cuda").manual_seed(7)
