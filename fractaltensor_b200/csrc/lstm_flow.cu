@@ -255,10 +255,10 @@ int launch_lstm_flow(int dtype, const void* x, const void* Wp, const float* bias
   const uint32_t nb = plan.nb, held = pair ? nb / 2 : nb, planes = 128 / nb;
   CUtensorMap mX, mH, mW;
   int rc;
-  if ((rc = make_tmap_3d(&mX, x, dtype, 64, T, I / BK, static_cast<uint64_t>(I) * 2, 128, 64, held, planes))) return rc;
-  if ((rc = make_tmap_3d(&mH, hs, dtype, 64, static_cast<uint64_t>(D) * T, H / BK, static_cast<uint64_t>(H) * 2, 128, 64,
-                         held, planes)))
-    return rc;
+  a.by_step = off == nullptr;
+  const uint64_t rows = a.by_step ? N : T, steps = a.by_step ? L : 1;
+  if ((rc = make_tmap_steps(&mX, x, dtype, steps, rows, I, held, planes))) return rc;
+  if ((rc = make_tmap_steps(&mH, hs, dtype, a.by_step ? D * steps : 1, a.by_step ? rows : D * rows, H, held, planes))) return rc;
   if ((rc = make_tmap_gates(&mW, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, I + H))) return rc;
   const int64_t chunks = static_cast<int64_t>(D) * T * H / 8;
   const int n_flags = D * L * a.S;

@@ -51,6 +51,11 @@ struct FlowArgs {
   // fold 0: a step is a time step in every layer.
   int fold, N1;
   int flag_steps;       // cells of a layer in `flags`
+  // mapX and mapH are of steps of N rows, so that a slice that is not full reads no rows past the step's; else (a ragged batch, the
+  // dilated LSTM) of all rows as one step.  Rows past the step's belong to the next step, which the layer below is storing and
+  // polling meanwhile, and what follows closely behind it held it up: D8 L100 H512, 40 sequences on slices of 64, pairs 403 -> 336
+  // us, 56 401 -> 358, 64 369 / 370; D18 L151 N33 1269 -> 959.  (A ragged batch by boxes of 8 and 16 rows: 380 -> 477.)
+  bool by_step;
   int* status;
 };
 
@@ -352,7 +357,10 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
       const int copies = (kb_x + C::kCopyKb - 1) / C::kCopyKb;
       int ready = 0;  // steps of the layer below that can be read
       for (int t = 0; t < steps && ok; ++t) {
-        const int64_t row = (l == 0 ? 0 : (l - 1) * a.T) + rows_of(a, t).first + held_base;
+        // (the maps' steps: the call's, or all rows as one)
+        const int below = l == 0 ? 0 : l - 1;
+        const int step = a.by_step ? below * a.L + t : 0;
+        const int row = a.by_step ? held_base : static_cast<int>(below * a.T + rows_of(a, t).first + held_base);
         if (l > 0 && t >= ready) {
           // the layer below may be cut differently: its slices that hold this one's rows
           const int* flags = a.flags + static_cast<int64_t>(l - 1) * a.flag_steps * a.S;
@@ -386,9 +394,9 @@ __device__ __forceinline__ void body(const CUtensorMap& mapX, const CUtensorMap&
             uint8_t* dst = s_in + slot * slot_bytes + c * C::kCopyKb * C::kBlockBytes;
             const CUtensorMap* map = l == 0 ? &mapX : &mapH;
             if constexpr (kPair)
-              tma_load_3d_pair(dst, map, map_to_cta(smem_u32(&in_full[slot]), 0), 0, static_cast<int>(row), c * C::kCopyKb);
+              tma_load_4d_pair(dst, map, map_to_cta(smem_u32(&in_full[slot]), 0), 0, row, c * C::kCopyKb, step);
             else
-              tma_load_3d(dst, map, &in_full[slot], 0, static_cast<int>(row), c * C::kCopyKb);
+              tma_load_4d(dst, map, &in_full[slot], 0, row, c * C::kCopyKb, step);
           }
         }
         if (++slot == a.n_slots) {

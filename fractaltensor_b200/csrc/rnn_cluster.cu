@@ -1016,11 +1016,10 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
       if ((rc = make_tmap_2d_sw64(wide == 64 ? &dm.o64 : &dm.o128, hs, dtype, h_rows, H, H, wide))) return rc;
       if ((rc = make_tmap_2d_sw64(wide == 64 ? &dm.t64 : &dm.t128, hs, dtype, h_rows, H, H, tail))) return rc;
     }
-    const uint64_t row_bytes = static_cast<uint64_t>(H) * 2;
     for (int i = 0; i < 2; ++i) {
       const uint32_t w = width[i] > 0 ? width[i] : width[0], planes = 128 / w;  // of a copy of flow::body
-      if ((rc = make_tmap_3d(&dm.nx[i], x, dtype, 64, x_rows, H / 64, row_bytes, 128, 64, w, planes))) return rc;
-      if ((rc = make_tmap_3d(&dm.nh[i], hs, dtype, 64, h_rows, H / 64, row_bytes, 128, 64, w, planes))) return rc;
+      if ((rc = make_tmap_steps(&dm.nx[i], x, dtype, 1, x_rows, H, w, planes))) return rc;
+      if ((rc = make_tmap_steps(&dm.nh[i], hs, dtype, 1, h_rows, H, w, planes))) return rc;
     }
     if ((rc = make_tmap_gates(&dm.nw, Wp, dtype, static_cast<uint64_t>(D) * 4 * H, 2 * H))) return rc;
     flow::FlowArgs f[2] = {};

@@ -84,6 +84,22 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, u
   return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
 }
 
+int make_tmap_steps(CUtensorMap* out, const void* base, int dtype, uint64_t steps, uint64_t rows, uint64_t K, uint32_t box_rows,
+                    uint32_t box_planes) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return FTB_ERR_DRIVER;
+  const size_t row = K * dtype_size(dtype);
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row & 15)) return FTB_ERR_ALIGN;
+  if (K % 64 != 0 || box_rows > 256 || box_planes > 256) return FTB_ERR_ARG;
+  cuuint64_t dims[4] = {64, rows, K / 64, steps};
+  cuuint64_t strides[3] = {row, 128, rows * row};
+  cuuint32_t box[4] = {64, box_rows, box_planes, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(out, tmap_dtype(dtype), 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? FTB_OK : FTB_ERR_DRIVER;
+}
+
 int make_tmap_gates(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t K) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return FTB_ERR_DRIVER;

@@ -30,6 +30,11 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int dtype, uint64_t cols, u
                  uint64_t row_stride_bytes, uint64_t plane_stride_bytes, uint32_t box_cols, uint32_t box_rows,
                  uint32_t box_planes, bool swizzle128 = true);
 
+// 16-bit states [step][row][K] as boxes of box_rows rows x box_planes 64-wide K blocks of one step: rows past the step's arrive
+// as zeros and are not read.
+int make_tmap_steps(CUtensorMap* out, const void* base, int dtype, uint64_t steps, uint64_t rows, uint64_t K, uint32_t box_rows,
+                    uint32_t box_planes);
+
 // Packed LSTM weights [rows, K] (four gates of a unit in consecutive rows) as [row / 32][gate][unit][K]: a box of 64 columns x
 // 128 rows puts the gates of a unit 8 rows apart, those of 32 rows together.
 int make_tmap_gates(CUtensorMap* out, const void* base, int dtype, uint64_t rows, uint64_t K);

@@ -96,6 +96,52 @@ def test_named_forms_same_bits_as_levels(ops, dt, D, L, N, H, nb, pair, ring):
     assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
 
 
+@pytest.mark.parametrize("D,L,N,H,nb,pair", [
+    (3, 9, 70, 256, 64, 2),   # 6 sequences in the last slice: none for the second CTA of its pair
+    (4, 7, 15, 512, 64, 2),
+    (2, 5, 1, 128, 128, 2),
+    (5, 6, 49, 320, 64, 1),
+])
+def test_slices_with_empty_halves(ops, D, L, N, H, nb, pair):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    Wp, b = _params(ops, D, H, H, torch.float16, g)
+    x = torch.randn(L, N, H, device="cuda", generator=g).half()
+    ref_h, ref_c = ops.lstm_stacked(x, Wp, b, schedule=1, pair=1)
+    h, c = _named_form(ops, x, Wp, b, N, None, nb, pair, 0)
+    assert torch.equal(h, ref_h) and torch.equal(c, ref_c)
+
+
+def test_a_slice_that_is_not_full_costs_no_more_than_a_full_one(ops):
+    """Layers beside each other: what a layer reads of the one below must not be rows that are being stored and polled.
+    40 of 64 sequences take 0.91 of the full slice's time; with rows of the next step in the same copies 1.09."""
+    from fractaltensor_b200.ops import _dtype_code, _ptr, _stream, check, lib
+    D, L, H, dt = 8, 100, 512, torch.float16
+    g = torch.Generator(device="cuda").manual_seed(2)
+    Wp, b = _params(ops, D, H, H, dt, g)
+    took = {}
+    calls = {}
+    for N in (40, 64):
+        x = torch.randn(L, N, H, device="cuda", generator=g).to(dt)
+        hs, c = torch.empty(D, L, N, H, dtype=dt, device="cuda"), torch.empty(D, N, H, device="cuda")
+        ws = ops.workspace(x.device, lib.ftb_lstm_stacked_workspace_bytes(D, L, N, H))
+        calls[N] = lambda x=x, hs=hs, c=c, ws=ws, N=N: check(lib.ftb_lstm_flow_form_fwd(
+            _ptr(x), _ptr(Wp), _ptr(b), _ptr(hs), _ptr(c), None, D, L, N, H, H, _dtype_code(x), 64, 2, 0, _ptr(ws), ws.numel(),
+            _stream()), "ftb_lstm_flow_form_fwd")
+        took[N] = []
+    for _ in range(8):  # in turn, so that both meet the same clocks
+        for N in (40, 64):
+            calls[N]()
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(8):
+                calls[N]()
+            end.record()
+            end.synchronize()
+            took[N].append(start.elapsed_time(end))
+    ops.check_status()
+    assert min(took[40]) < min(took[64]), took
+
+
 def test_forms_there_are(ops):
     from fractaltensor_b200._lib import FtbError
     g = torch.Generator(device="cuda").manual_seed(1)
