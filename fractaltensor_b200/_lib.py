@@ -38,6 +38,7 @@ SIGNATURES = {
     "ftb_lstm_dilated_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, ctypes.POINTER(_i), _i, _i, _i, _i, _i, ctypes.POINTER(_i), _vp, _sz, _vp]),
     "ftb_grid_pack_weights": (_i, [_vp, _vp, _vp, _i, _i, _vp]),
     "ftb_grid_rnn_workspace_bytes": (_sz, [_i, _i, _i]),
+    "ftb_grid_rnn_call_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _i]),
     "ftb_grid_rnn_tables_bytes": (_sz, [_i, _i, _i]),
     "ftb_grid_rnn_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "ftb_grid_flow_form_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp]),

@@ -34,11 +34,12 @@ int launch_lstm_simt_flow(const float* x, const float* Wp, const float* bias_p, 
 // csrc/grid_flow.cu (16-bit grid RNN): batch slices of nb columns, S of them, `groups` (layer, row, slice) chains beside each other.
 struct GridFlowPlan {
   int nb, S, groups;
+  size_t ints;  // counters
   double est_us;
 };
-size_t grid_flow_ints(int D, int A, int B);
-bool grid_flow_form(int dtype, int D, int A, int N, int H, int sm_count, int nb, GridFlowPlan* plan);
-bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, GridFlowPlan* plan);
+size_t grid_flow_ints(int D, int A, int B, int N);
+bool grid_flow_form(int dtype, int D, int A, int B, int N, int H, int sm_count, int nb, GridFlowPlan* plan);
+bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, size_t max_ints, GridFlowPlan* plan);
 int launch_grid_flow(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
                      const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, const GridFlowPlan& plan,
                      int* counters, int* status, cudaStream_t stream);

@@ -43,7 +43,8 @@ constexpr int kFirstEpi = 4;
 constexpr int kSlots = 4;    // input tiles
 constexpr int kAhead = 16;   // columns that are filled ahead of the sweep,
 constexpr int kFill = 8;     // so many to a count (two counts ahead: who waits for a count can still do the columns of the one before)
-constexpr int kMaxPause = 4000;  // cycles
+constexpr int kColumnCounts = 4;  // of a chain, one for each CTA of its group
+constexpr int kMaxPause = 4000;   // cycles
 constexpr uint32_t kOneCta = 120 * 1024;  // shared memory of which only one CTA fits on an SM: both would want all of tensor memory
 
 template <int NB, bool kPair>
@@ -70,7 +71,7 @@ struct GridArgs {
   void *hx, *hy;         // [D, A, B, N, H]
   int* ready;            // [D * A * S][counts] CTAs of the chain that have filled these kFill columns
   int counts;            // of a chain
-  int* flags;            // [D * A * B * S * 2] tiles of the cell and direction that can be read through TMA (D > 1)
+  int* columns;          // [D * A * S][2 directions][2 tiles] columns of the chain that the layer above can read through TMA
   int* status;
 };
 
@@ -94,6 +95,9 @@ __device__ __forceinline__ Chain chain_of(const GridArgs& g, int c) {
 }
 __device__ __forceinline__ int* ready_of(const GridArgs& g, int d, int a, int s, int count) {
   return g.ready + (static_cast<int64_t>(d * g.A + a) * g.S + s) * g.counts + count;
+}
+__device__ __forceinline__ int* columns_of(const GridArgs& g, int d, int a, int s, bool ydir) {
+  return g.columns + (static_cast<int64_t>(d * g.A + a) * g.S + s) * kColumnCounts + 2 * ydir;
 }
 
 template <typename T, int NB, bool kPair>
@@ -253,9 +257,11 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
       for (int b = 0; b < g.B && ok; ++b) {
         const int64_t cell = (static_cast<int64_t>(max(ch.d - 1, 0)) * g.A + ch.a) * g.B + b;
         if (ch.d > 0) {
-          if (lane == 0) ok = flag_wait_ge(g.flags + (cell * g.S + ch.s) * 2 + ydir, g.tiles, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
+          if (lane < g.tiles)
+            ok = flag_wait_ge(columns_of(g, ch.d - 1, ch.a, ch.s, ydir) + lane, b + 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
+          __syncwarp();
           fence_proxy_async_global();  // threads of other CTAs stored what TMA reads
         }
         ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
@@ -303,8 +309,7 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
           }
           __threadfence_block();
           // (The release takes the other warps' stores along; the proxy fence is the reader's, between its acquire and its copy.)
-          const int64_t cell = (static_cast<int64_t>(ch.d) * g.A + ch.a) * g.B + b;
-          red_release_gpu_add(g.flags + (cell * g.S + ch.s) * 2 + ydir, 1);
+          red_release_gpu_add(columns_of(g, ch.d, ch.a, ch.s, ydir) + tile, 1);
         }
       }
     }
@@ -603,27 +608,33 @@ int launch(const CUtensorMap* m, const GridArgs& g, uint32_t smem, cudaStream_t 
 
 }  // namespace
 
-// At most 32 slices: what the workspace has counters for.
 constexpr int kGridMaxSlices = 32;
-size_t grid_flow_ints(int D, int A, int B) { return static_cast<size_t>(D) * A * kGridMaxSlices * (1 + 3 * static_cast<size_t>(B)); }
+static size_t grid_flow_counters(int D, int A, int B, int64_t S) {
+  return static_cast<size_t>(D) * A * S * ((static_cast<size_t>(B) + kFill - 1) / kFill + kColumnCounts);
+}
+// Counters of a call of N sequences on the narrowest slices; N 0: of any batch.
+size_t grid_flow_ints(int D, int A, int B, int N) {
+  return grid_flow_counters(D, A, B, N == 0 ? kGridMaxSlices : std::min<int64_t>(kGridMaxSlices, (N + INT64_C(15)) / 16));
+}
 
 // The kernel with slices of nb sequences; false: there is no such form of it.
-bool grid_flow_form(int dtype, int D, int A, int N, int H, int sm_count, int nb, GridFlowPlan* plan) {
+bool grid_flow_form(int dtype, int D, int A, int B, int N, int H, int sm_count, int nb, GridFlowPlan* plan) {
   if ((dtype != FTB_F16 && dtype != FTB_BF16) || H < 64 || H > 256 || H % 64 != 0 || N < 1) return false;
   if (!(nb == 16 || nb == 32 || nb == 64)) return false;
   plan->nb = nb;
   plan->S = (N + nb - 1) / nb;
   plan->groups = std::min(static_cast<int64_t>(sm_count / (2 * ((H + 127) / 128))), static_cast<int64_t>(D) * A * plan->S);
+  plan->ints = grid_flow_counters(D, A, B, plan->S);
   plan->est_us = 0.0;
   return plan->S <= kGridMaxSlices && plan->groups >= 1;
 }
 
-// How the kernel would run a problem; est_us: about what that takes.
-bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, GridFlowPlan* plan) {
+// How the kernel would run a problem with room for max_ints counters; est_us: about what that takes.
+bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, size_t max_ints, GridFlowPlan* plan) {
   bool found = false;
   for (int nb = 16; nb <= 64; nb *= 2) {
     GridFlowPlan p;
-    if (!grid_flow_form(dtype, D, A, N, H, sm_count, nb, &p)) continue;
+    if (!grid_flow_form(dtype, D, A, B, N, H, sm_count, nb, &p) || p.ints > max_ints) continue;
     // Steps until the last chain is done: a chain starts behind the one before it in its group (two steps later with other
     // weights), a step after the row above and three after the layer below, and takes B.
     std::vector<double> free_at(p.groups, 0.0), start(static_cast<size_t>(D) * A * p.S, 0.0);
@@ -654,7 +665,7 @@ bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, 
   return found;
 }
 
-// X, Y: [A, B, N, H]; Wpx, Wpy: [D, H, 3H]; hx, hy: [D, A, B, N, H]; counters: grid_flow_ints (zeroed here).
+// X, Y: [A, B, N, H]; Wpx, Wpy: [D, H, 3H]; hx, hy: [D, A, B, N, H]; counters: plan.ints of them (zeroed here).
 int launch_grid_flow(int dtype, const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
                      const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, const GridFlowPlan& plan,
                      int* counters, int* status, cudaStream_t stream) {
@@ -665,7 +676,7 @@ int launch_grid_flow(int dtype, const void* X, const void* Y, const void* Wpx, c
   g.Wx = Wpx; g.Wy = Wpy; g.bx = bias_x; g.by = bias_y; g.hx = hx; g.hy = hy;
   g.ready = counters;
   g.counts = (B + kFill - 1) / kFill;
-  g.flags = counters + static_cast<size_t>(D) * A * plan.S * g.counts;
+  g.columns = counters + static_cast<size_t>(D) * A * plan.S * g.counts;
   g.status = status;
   const bool pair = g.tiles == 2;
   const uint32_t held = pair ? plan.nb / 2 : plan.nb, planes = H / BK;
@@ -678,8 +689,7 @@ int launch_grid_flow(int dtype, const void* X, const void* Y, const void* Wpx, c
     if (rc) return rc;
   }
   const uint32_t smem = std::max(kOneCta, 1024 + (2 + kSlots) * planes * held * BK * 2);
-  const size_t n_counters = static_cast<size_t>(D) * A * plan.S * (g.counts + (D > 1 ? 2 * static_cast<size_t>(B) : 0));
-  if (cudaMemsetAsync(counters, 0, sizeof(int) * n_counters, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
+  if (cudaMemsetAsync(counters, 0, sizeof(int) * plan.ints, stream) != cudaSuccess) return FTB_ERR_LAUNCH;
 #define FTB_GRID_LAUNCH(TT)                                                                              \
   switch (plan.nb) {                                                                                     \
     case 16: return pair ? launch<TT, 16, true>(m, g, smem, stream) : launch<TT, 16, false>(m, g, smem, stream); \

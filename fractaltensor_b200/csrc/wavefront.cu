@@ -1295,7 +1295,8 @@ int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* 
   // Weights on chip, states that carry their own arrival (csrc/grid_flow.cu): the choice where it applies and the workspace has
   // room for its counters behind the tables.
   GridFlowPlan flow;
-  if (workspace_bytes >= ftb_grid_rnn_workspace_bytes(D, A, B) && grid_flow_plan(dtype, D, A, B, N, H, cl.sm_count, &flow)) {
+  if (workspace_bytes > lay.total &&
+      grid_flow_plan(dtype, D, A, B, N, H, cl.sm_count, (workspace_bytes - lay.total) / sizeof(int), &flow)) {
     rc = launch_grid_flow(dtype, X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy, D, A, B, N, H, flow,
                           reinterpret_cast<int*>(static_cast<char*>(workspace) + lay.total), status, stream);
     if (rc != FTB_ERR_LAUNCH) return rc;  // a refused cooperative launch falls back to the generic wavefront
@@ -1531,11 +1532,11 @@ int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const 
   if (static_cast<int64_t>(D) * A * B * N > 0x7fffffffLL) return FTB_ERR_ARG;
   if (!aligned16({X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy})) return FTB_ERR_ALIGN;
   GridFlowPlan flow;
-  if (!grid_flow_form(dtype, D, A, N, H, current_sm_count(), nb, &flow)) return FTB_ERR_ARG;
+  if (!grid_flow_form(dtype, D, A, B, N, H, current_sm_count(), nb, &flow)) return FTB_ERR_ARG;
   int* status = nullptr;
   const int rc = begin_call(workspace, workspace_bytes, stream, &status);
   if (rc) return rc;
-  if (workspace_bytes < kWorkspaceBytes + sizeof(int) * grid_flow_ints(D, A, B)) return FTB_ERR_WORKSPACE;
+  if (workspace_bytes < kWorkspaceBytes + sizeof(int) * flow.ints) return FTB_ERR_WORKSPACE;
   return launch_grid_flow(dtype, X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy, D, A, B, N, H, flow,
                           reinterpret_cast<int*>(static_cast<char*>(workspace) + kWorkspaceBytes), status, stream);
 }
@@ -1547,8 +1548,13 @@ size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {
 
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B) {
   if (D <= 0 || A <= 0 || B <= 0) return kWorkspaceBytes;
-  // tables of the generic persistent schedule, then the counters of the one with weights on chip
-  return plan_layout(2 * D * A * B, 0).total + sizeof(int) * grid_flow_ints(D, A, B);
+  // tables of the generic persistent schedule, then the counters of the one with weights on chip, of any batch
+  return plan_layout(2 * D * A * B, 0).total + sizeof(int) * grid_flow_ints(D, A, B, 0);
+}
+
+size_t ftb_grid_rnn_call_workspace_bytes(int D, int A, int B, int N, int H, int dtype) {
+  if (D <= 0 || A <= 0 || B <= 0 || N <= 0 || H <= 0 || dtype == FTB_F32) return kWorkspaceBytes;
+  return plan_layout(2 * D * A * B, 0).total + (H <= 256 ? sizeof(int) * grid_flow_ints(D, A, B, N) : 0);
 }
 
 int ftb_gemm_nt(const void* A, const void* Bt, void* out, int M, int N, int K, int dtype, const int* tuning,

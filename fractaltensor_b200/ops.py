@@ -329,8 +329,14 @@ def grid_rnn(X, Y, Wpx, Wpy, bias_x=None, bias_y=None, schedule=0):
     hy = torch.empty_like(hx)
     # The library picks the schedule by the room the workspace offers: status word only -> one launch
     # per level; the tables -> generic persistent kernel; tables and counters -> weights on chip.
-    ws = workspace(X.device, 0 if schedule == 1 else lib.ftb_grid_rnn_workspace_bytes(D, A, B))
-    ws_bytes = {1: lib.ftb_workspace_bytes(), 2: lib.ftb_grid_rnn_tables_bytes(D, A, B)}.get(schedule, ws.numel())
+    if schedule == 1:
+        room = lib.ftb_workspace_bytes()
+    elif schedule == 2:
+        room = lib.ftb_grid_rnn_tables_bytes(D, A, B)
+    else:
+        room = lib.ftb_grid_rnn_call_workspace_bytes(D, A, B, N, H, _dtype_code(X))
+    ws = workspace(X.device, room)
+    ws_bytes = room if schedule in (1, 2) else ws.numel()
     with _on(X.device), _turn(ws):
         check(lib.ftb_grid_rnn_fwd(_ptr(X), _ptr(Y), _ptr(Wpx), _ptr(Wpy), _ptr(bias_x), _ptr(bias_y), _ptr(hx),
                                    _ptr(hy), D, A, B, N, H, _dtype_code(X), _ptr(ws), ws_bytes, _stream()),

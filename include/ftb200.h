@@ -209,14 +209,15 @@ int ftb_grid_pack_weights(const void* i2h, const void* h2h, void* Wp, int H, int
  * X,Y: [A,B,N,H] inputs of the x and y directions at grid point (a,b);
  * Wpx,Wpy: [D,H,3H] from ftb_grid_pack_weights; bias_x,bias_y: fp32 [D,H] or NULL;
  * hx,hy (out): [D,A,B,N,H].  state_x = hx[a-1][b], state_y = hy[a][b-1].
- * Both directions of a level run in one launch.  With ftb_grid_rnn_workspace_bytes(D, A, B)
- * bytes of workspace (16-bit dtypes) the whole grid runs as one launch: for H up to 256 with the
+ * Both directions of a level run in one launch.  With ftb_grid_rnn_call_workspace_bytes(D, A, B, N, H,
+ * dtype) bytes of workspace, or ftb_grid_rnn_workspace_bytes(D, A, B), which is enough for any N, H and
+ * dtype, the whole grid of a 16-bit dtype runs as one launch: for H up to 256 with the
  * weights on chip and states that carry their own arrival (csrc/grid_flow.cu); for wider H, more
- * than 32 slices of the batch, or with a workspace of at least ftb_grid_rnn_tables_bytes(D, A, B) but
- * less than ftb_grid_rnn_workspace_bytes(D, A, B) bytes, as the generic persistent wavefront, whose
- * schedule tables are copied from host memory on `stream`; with less than that, one launch per level.
- * All schedules give the same bits. */
+ * than 32 slices of the batch, or with a workspace of just ftb_grid_rnn_tables_bytes(D, A, B) bytes,
+ * as the generic persistent wavefront, whose schedule tables are copied from host memory on `stream`;
+ * with less than that, one launch per level.  All schedules give the same bits. */
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B);
+size_t ftb_grid_rnn_call_workspace_bytes(int D, int A, int B, int N, int H, int dtype);
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B);
 int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
                      const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype,

@@ -93,6 +93,21 @@ def test_bad_arguments_are_rejected_without_a_device(lib):
     assert lib.ftb_lstm_dilated_fwd(one, one, z, one, one, dil, 2, 4, 1, 64, 1, None, one, 256, z) == 1  # dilation 0
 
 
+def test_workspace_of_a_grid_goes_by_its_batch(lib):
+    """Counters of the kernel with weights on chip: 16 bytes a cell at most, for the slices that the batch has."""
+    tables = lambda *g: lib.ftb_grid_rnn_tables_bytes(*g)
+    for grid in ((1, 256, 256), (1, 1000, 1000), (3, 40, 300), (2, 7, 1)):
+        cells, rows = grid[0] * grid[1] * grid[2], grid[0] * grid[1]
+        assert lib.ftb_grid_rnn_workspace_bytes(*grid) - tables(*grid) <= 16 * cells + 32 * rows * 20
+        one = lib.ftb_grid_rnn_call_workspace_bytes(*grid, 1, 64, 1) - tables(*grid)
+        assert 0 < one <= cells // 2 + 20 * rows
+        most = max(lib.ftb_grid_rnn_call_workspace_bytes(*grid, n, 256, 2) for n in (1, 16, 17, 400, 2048, 100000))
+        assert most == lib.ftb_grid_rnn_workspace_bytes(*grid)
+        assert lib.ftb_grid_rnn_call_workspace_bytes(*grid, 64, 320, 1) == tables(*grid)  # too wide for that kernel
+        assert lib.ftb_grid_rnn_call_workspace_bytes(*grid, 64, 256, 0) == lib.ftb_workspace_bytes()  # fp32: a launch a level
+    assert lib.ftb_grid_rnn_call_workspace_bytes(1, 4, 4, 0, 64, 1) == lib.ftb_workspace_bytes()
+
+
 def test_misaligned_pointers_are_rejected_without_a_device(lib):
     """Every kernel moves 16 bytes at a time (float4 on the fp32 path, TMA on the 16-bit path): a
     pointer off a 16-byte boundary is answered with FTB_ERR_ALIGN (2) before any launch."""

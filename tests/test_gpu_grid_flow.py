@@ -56,6 +56,24 @@ def test_same_bits_as_levels(ops, dt, D, A, B, N, H):
             assert torch.equal(hx, rx) and torch.equal(hy, ry)
 
 
+@pytest.mark.parametrize("D,A,B,N,H", [(1, 6, 9, 40, 256), (3, 7, 20, 70, 128), (2, 5, 8, 33, 192)])
+def test_workspaces_of_every_size(ops, D, A, B, N, H):
+    """What a call asks for, room for the counters of wider slices alone, for the tables alone, and for neither."""
+    from fractaltensor_b200._lib import check, lib
+    args = _inputs(ops, D, A, B, N, H, torch.float16, N)
+    rx, ry = ops.grid_rnn(*args, schedule=1)
+    tables, full = lib.ftb_grid_rnn_tables_bytes(D, A, B), lib.ftb_grid_rnn_call_workspace_bytes(D, A, B, N, H, 1)
+    for size in (full, tables + (full - tables) // 2, tables + 4, tables, lib.ftb_workspace_bytes()):
+        hx, hy = torch.randn_like(rx), torch.randn_like(ry)
+        room = torch.zeros(size + 256, dtype=torch.uint8, device="cuda")
+        room[size:] = 77  # behind the workspace: not the call's
+        check(lib.ftb_grid_rnn_fwd(*(ops._ptr(t) for t in args), ops._ptr(hx), ops._ptr(hy), D, A, B, N, H, 1, ops._ptr(room), size,
+                                   ops._stream()), "ftb_grid_rnn_fwd")
+        torch.cuda.synchronize()
+        assert int(room[:4].view(torch.int32)) == 0 and bool((room[size:] == 77).all())
+        assert torch.equal(hx, rx) and torch.equal(hy, ry), size
+
+
 def test_nan_states_are_states(ops):
     """A NaN state (0x7FFF) is a value like any other, also where an input has the fill pattern's bits."""
     X, Y, Wx, Wy, bx, by = _inputs(ops, 1, 5, 6, 20, 128, torch.float16)
