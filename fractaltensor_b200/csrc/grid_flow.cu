@@ -10,8 +10,8 @@
 //   * the weights of a direction (3H x 128 units a CTA) sit in tensor memory.  Above 128 units the two CTAs of a direction are a
 //     pair (.cta_group::2) and each holds half of the sequences' states;
 //   * the batch is cut into slices of NB columns, and (layer, row, slice) chains are dealt to the groups of CTAs that the device
-//     holds in the order in which they can start (row + layer), so any grid runs: a group that is done with its chain takes the
-//     next one, with other weights where the layer changes;
+//     holds in the order in which they can start (row + layer), so that grids of any size run, of up to 4096 sequences: a group
+//     that is done with its chain takes the next one, with other weights where the layer changes;
 //   * nobody fills the arrays before the launch.  A warp of every CTA writes 0xFFFF into its own part kAhead columns ahead of the
 //     sweep, counts every kFill columns of a chain in (`ready`), and waits there for those that this CTA reads: its chain's others
 //     and the chain above.  The epilogue looks at a column when that warp says so (`n_clear`), steps after it did.
@@ -608,7 +608,7 @@ int launch(const CUtensorMap* m, const GridArgs& g, uint32_t smem, cudaStream_t 
 
 }  // namespace
 
-constexpr int kGridMaxSlices = 32;
+constexpr int kGridMaxSlices = 64;
 static size_t grid_flow_counters(int D, int A, int B, int64_t S) {
   return static_cast<size_t>(D) * A * S * ((static_cast<size_t>(B) + kFill - 1) / kFill + kColumnCounts);
 }
@@ -635,8 +635,8 @@ bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, 
   for (int nb = 16; nb <= 64; nb *= 2) {
     GridFlowPlan p;
     if (!grid_flow_form(dtype, D, A, B, N, H, sm_count, nb, &p) || p.ints > max_ints) continue;
-    // Steps until the last chain is done: a chain starts behind the one before it in its group (two steps later with other
-    // weights), a step after the row above and three after the layer below, and takes B.
+    // Steps until the last chain is done: a chain starts a step behind the one before it in its group (two with other weights), a
+    // step after the row above and three after the layer below, and takes B.
     std::vector<double> free_at(p.groups, 0.0), start(static_cast<size_t>(D) * A * p.S, 0.0);
     std::vector<int> layer(p.groups, -1);
     double last = 0.0;
@@ -645,7 +645,7 @@ bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, 
       for (int d = std::max(0, m - A + 1); d <= std::min(m, D - 1); ++d)
         for (int s = 0; s < p.S; ++s, ++c) {
           const int a = m - d, g = c % p.groups;
-          double t = free_at[g] + (layer[g] >= 0 && layer[g] != d ? 2.0 : 0.0);
+          double t = free_at[g] + (layer[g] < 0 ? 0.0 : layer[g] != d ? 2.0 : 1.0);
           if (a > 0) t = std::max(t, start[static_cast<size_t>(d * A + a - 1) * p.S + s] + 1.0);
           if (d > 0) t = std::max(t, start[static_cast<size_t>((d - 1) * A + a) * p.S + s] + 3.0);
           start[static_cast<size_t>(d * A + a) * p.S + s] = t;
@@ -654,13 +654,22 @@ bool grid_flow_plan(int dtype, int D, int A, int B, int N, int H, int sm_count, 
           last = std::max(last, t + B);
         }
     // A step, fitted to 170 grids (D 1..3, A and B 2..48, N 1..400, H 64..256; 9, 6 and 5 % in the root mean square for the three
-    // widths).  Rows and chains beside each other weigh with the bytes that they read.  The width taken is within 0.3 % of the
-    // fastest on average (worst 11 %), and 0.15 to 0.7 times the generic wavefront's time.
+    // widths).  Rows and chains beside each other weigh with the bytes that they read.  The width taken is within 0.1 % of the
+    // fastest on average (worst 7 %) of 123 grids of 6 to 40 rows and columns and 4 to 64 sequences, and 0.15 to 0.7 times the
+    // generic wavefront's time; of 700 grids of 1 to 64 rows and columns and 1 to 4096 sequences within 0.8 % (worst 36 %).
     const double h = H / 256.0, load = h * p.groups / (sm_count / (2 * ((H + 127) / 128))) * std::min(N, nb) / nb;
     const double step = nb == 16 ? 1.05 + 0.37 * h + 0.13 * load : nb == 32 ? 1.13 + 0.38 * h + 0.42 * load : 1.40 + 0.69 * h + 0.73 * load;
     p.est_us = (nb == 16 ? 12.8 : nb == 32 ? 14.4 : 16.7) + last * step;
     if (!found || p.est_us < plan->est_us) *plan = p;
     found = true;
+  }
+  // Chains of a few columns, many of them one behind the other, spend their time between chains: there the generic wavefront is
+  // the faster one, whose tiles large batches fill (us, this / generic: D2 A40 B1 N3613 H256 1024 / 421, D3 A14 B1 N1715 H192 268 /
+  // 146, D3 A20 B2 N2798 H192 732 / 538; D3 A32 B15 N1999 H256 4494 / 5245).  Its time by levels and by rounds of tiles, fitted to 184
+  // grids of up to 4 columns and 100 sequences or more (11 % in the root mean square); of the 700 it is taken for 20.
+  if (found && B <= 4 && static_cast<int64_t>(D) * A * plan->S > 4 * plan->groups) {
+    const double h = H / 256.0, rounds = 2.0 * D * A * B * ((N + 127) / 128) / sm_count;
+    if (10.8 + (A + B + D - 2) * (5.5 + 1.87 * h) + rounds * (1.45 + 6.37 * h) < plan->est_us) return false;
   }
   return found;
 }

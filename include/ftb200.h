@@ -212,8 +212,8 @@ int ftb_grid_pack_weights(const void* i2h, const void* h2h, void* Wp, int H, int
  * Both directions of a level run in one launch.  With ftb_grid_rnn_call_workspace_bytes(D, A, B, N, H,
  * dtype) bytes of workspace, or ftb_grid_rnn_workspace_bytes(D, A, B), which is enough for any N, H and
  * dtype, the whole grid of a 16-bit dtype runs as one launch: for H up to 256 with the
- * weights on chip and states that carry their own arrival (csrc/grid_flow.cu); for wider H, more
- * than 32 slices of the batch, or with a workspace of just ftb_grid_rnn_tables_bytes(D, A, B) bytes,
+ * weights on chip and states that carry their own arrival (csrc/grid_flow.cu); for wider H, more than
+ * 4096 sequences, large batches on rows of a few columns, or with a workspace of just ftb_grid_rnn_tables_bytes(D, A, B) bytes,
  * as the generic persistent wavefront, whose schedule tables are copied from host memory on `stream`;
  * with less than that, one launch per level.  All schedules give the same bits. */
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B);

@@ -91,6 +91,41 @@ def test_nan_states_are_states(ops):
 def test_forms_that_do_not_exist(ops):
     args = _inputs(ops, 1, 2, 2, 600, 64, torch.float16)
     hx = torch.empty(1, 2, 2, 600, 64, dtype=torch.float16, device="cuda")
-    for nb in (8, 48, 128, 16):  # 16: more slices than there are counters for
+    for nb in (8, 48, 128):
         with pytest.raises(RuntimeError):
             _form(ops, args, nb, hx, torch.empty_like(hx))
+    args = _inputs(ops, 1, 2, 2, 1030, 64, torch.float16)
+    hx = torch.empty(1, 2, 2, 1030, 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(RuntimeError):
+        _form(ops, args, 16, hx, torch.empty_like(hx))  # more slices than there are counters for
+
+
+@pytest.mark.parametrize("D,A,B,N,H", [
+    (1, 2, 3, 2049, 64), (2, 2, 2, 2300, 256),     # more than 32 slices of 64
+    (1, 2, 5, 4096, 64), (1, 2, 5, 4097, 64),      # the last batch that has counters, the first that has none
+    (2, 30, 1, 1100, 256), (3, 12, 2, 1200, 192),  # a few columns, many chains: the generic wavefront by the rule
+    (2, 30, 5, 300, 256),                          # one column more
+])
+def test_large_batches(ops, D, A, B, N, H):
+    args = _inputs(ops, D, A, B, N, H, torch.bfloat16, N)
+    rx, ry = ops.grid_rnn(*args, schedule=1)
+    hx, hy = ops.grid_rnn(*args)
+    ops.check_status()
+    assert torch.equal(hx, rx) and torch.equal(hy, ry)
+
+
+def test_many_short_chains_do_not_take_long(ops):
+    """Rows of one column and a large batch: the generic wavefront's 0.13 ms, not the 0.27 of one chain behind another."""
+    args = _inputs(ops, 3, 14, 1, 1715, 192, torch.float16)
+    took = {0: [], 2: []}
+    for _ in range(8):  # in turn, so that both meet the same clocks
+        for schedule in (0, 2):
+            ops.grid_rnn(*args, schedule=schedule)
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                ops.grid_rnn(*args, schedule=schedule)
+            end.record()
+            end.synchronize()
+            took[schedule].append(start.elapsed_time(end))
+    assert min(took[0]) < 1.2 * min(took[2]), took
