@@ -30,8 +30,12 @@ namespace {
 constexpr int BK = 64, kTileN = 256;
 constexpr int kThreads = 384, kEpiWarps = 8;
 constexpr uint32_t kABlock = 128 * BK * 2, kBBlock = 128 * BK * 2;  // one K block of this CTA's rows, of its half of the columns
-constexpr int kMaxKBlocks = 10;   // H <= 640: 160 KB of rows, three K blocks of columns beside them
+constexpr int kMaxKBlocks = 10;   // H <= 640: 160 KB of rows, four K blocks of columns beside them
 constexpr int kMaxStages = 8;
+// Tiles whose sums are added one behind the other before they are added to those before them: with many rows a pair of CTAs has
+// all tiles of a row block, and in one running sum the rounding errors of a row's sum were 1.6 (40 tiles) to 1.9 times (192) those
+// of tiles that many pairs share.
+constexpr int kSumTiles = 8;
 constexpr uint32_t kSmemBudget = 229376;
 constexpr float kClamp = -64.f, kLog2e = 1.4426950408889634f;
 
@@ -204,8 +208,10 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const int q = warp & 3, half = (warp - 4) >> 2;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
     const uint32_t empty_bar[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
-    // First pass: the running pair of this thread's row.  Second: of four rows, lane / 4 and 8, 16, 24 further.
-    float top = -FLT_MAX, d = 0.f;
+    // First pass: the pairs of this thread's row, of up to kSumTiles tiles and of all before them.  Second: of four rows, lane / 4 and
+    // 8, 16, 24 further.
+    float top = -FLT_MAX, d = 0.f, all_top = -FLT_MAX, all_d = 0.f;
+    int summed = 0;
     float inv_d[4], shift[4], rest[4], least[4];
     int before = -1;
     if (!kStats) grid_dependency_wait();
@@ -216,8 +222,9 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       if (mb != before) {
         before = mb;
         if (kStats) {
-          top = -FLT_MAX;
-          d = 0.f;
+          top = all_top = -FLT_MAX;
+          d = all_d = 0.f;
+          summed = 0;
         } else {
           // the pairs of this thread's row
           const int entries = 2 * (pair_of((mb + 1) * a.n_tiles - 1) - pair_of(mb * a.n_tiles) + 1);
@@ -351,13 +358,23 @@ project_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         }
       }
       if (kStats) {  // (tile by tile: chunk by chunk through all of them adds up more roundings)
+        const bool stored = i + 1 == last || (i + 1) / a.n_tiles != mb;
         const float now = fmaxf(top, tile_top);
         const Ref to = ref_of(now);
         d = fmaf(d, rescale(ref_of(top), to), tile_d * rescale(from, to));
         top = now;
+        if (++summed == kSumTiles || stored) {
+          const float both = fmaxf(all_top, top);
+          const Ref to_both = ref_of(both);
+          all_d = fmaf(all_d, rescale(ref_of(all_top), to_both), d * rescale(to, to_both));
+          all_top = both;
+          top = -FLT_MAX;
+          d = 0.f;
+          summed = 0;
+        }
+        if (stored && row < a.T)
+          __stcg(a.stats + static_cast<long long>(2 * (c - pair_of(mb * a.n_tiles)) + half) * a.T + row, make_float2(all_top, all_d));
       }
-      if (kStats && row < a.T && (i + 1 == last || (i + 1) / a.n_tiles != mb))
-        __stcg(a.stats + static_cast<long long>(2 * (c - pair_of(mb * a.n_tiles)) + half) * a.T + row, make_float2(top, d));
     }
   }
 
