@@ -218,7 +218,7 @@ constexpr int kMaxCtas = 1024;  // entries of the per-CTA first-item table
 struct PlanLayout {
   size_t items, dep, target, cta_first, done, tile_done, c_done, counters_end, trace, total;
 };
-PlanLayout plan_layout(int n_items, int max_tiles_per_item = 64) {
+PlanLayout plan_layout(size_t n_items, int max_tiles_per_item = 64) {
   PlanLayout p;
   auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
   p.items = kWorkspaceBytes;
@@ -226,7 +226,7 @@ PlanLayout plan_layout(int n_items, int max_tiles_per_item = 64) {
   p.target = up(p.dep + sizeof(int32_t) * 2 * kMaxSeg * n_items);
   p.cta_first = up(p.target + sizeof(int32_t) * n_items);
   p.done = up(p.cta_first + sizeof(int32_t) * kMaxCtas);
-  const size_t max_tiles = static_cast<size_t>(n_items) * max_tiles_per_item;
+  const size_t max_tiles = n_items * max_tiles_per_item;
   p.tile_done = up(p.done + sizeof(int32_t) * 2 * n_items);
   p.c_done = up(p.tile_done + sizeof(int32_t) * max_tiles);
   p.counters_end = up(p.c_done + sizeof(int32_t) * max_tiles);
@@ -453,7 +453,7 @@ constexpr int kMostFlowSlices = 128;  // of a layer: two CTAs or more each
 
 size_t ftb_lstm_stacked_workspace_bytes(int D, int L, int N, int H) {
   if (D <= 0 || L <= 0 || N <= 0 || H <= 0) return kWorkspaceBytes;
-  return plan_layout(D * L, stacked_max_tiles_per_cell(N, H)).total + flow_flag_bytes(D, L, (N + 15) / 16);
+  return plan_layout(static_cast<size_t>(D) * L, stacked_max_tiles_per_cell(N, H)).total + flow_flag_bytes(D, L, (N + 15) / 16);
 }
 
 // Layers per group of the static-ownership kernels: at most `G` (what L2 holds) and what fits on the
@@ -1039,7 +1039,7 @@ int ftb_lstm_stacked_ragged_fwd_scratch(const void* x, const void* Wp, const flo
 size_t ftb_lstm_stacked_varlen_workspace_bytes(int D, int L) {
   if (D <= 0 || L <= 0) return kWorkspaceBytes;
   // tables of the generic schedule; first rows of the steps and arrival counters of the on-chip one
-  return plan_layout(D * L, 0).total + sizeof(int) * (L + 1) + 256 + flow_flag_bytes(D, L, kMostFlowSlices);
+  return plan_layout(static_cast<size_t>(D) * L, 0).total + sizeof(int) * (static_cast<size_t>(L) + 1) + 256 + flow_flag_bytes(D, L, kMostFlowSlices);
 }
 
 int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
@@ -1200,7 +1200,7 @@ int ftb_lstm_dilated_fwd(const void* x, const void* Wp, const float* bias_p, voi
 size_t ftb_lstm_dilated_workspace_bytes(int D, int L) {
   if (D <= 0 || L <= 0) return kWorkspaceBytes;
   // tables of the generic persistent schedule, then the flags of the cluster schedule
-  return plan_layout(D * L, 0).total + sizeof(int) * lstm_dilated_cluster_flag_ints(D, L);
+  return plan_layout(static_cast<size_t>(D) * L, 0).total + sizeof(int) * lstm_dilated_cluster_flag_ints(D, L);
 }
 
 int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
@@ -1543,18 +1543,18 @@ int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const 
 
 size_t ftb_grid_rnn_tables_bytes(int D, int A, int B) {
   if (D <= 0 || A <= 0 || B <= 0) return kWorkspaceBytes;
-  return plan_layout(2 * D * A * B, 0).total;
+  return plan_layout(static_cast<size_t>(2) * D * A * B, 0).total;
 }
 
 size_t ftb_grid_rnn_workspace_bytes(int D, int A, int B) {
   if (D <= 0 || A <= 0 || B <= 0) return kWorkspaceBytes;
   // tables of the generic persistent schedule, then the counters of the one with weights on chip, of any batch
-  return plan_layout(2 * D * A * B, 0).total + sizeof(int) * grid_flow_ints(D, A, B, 0);
+  return plan_layout(static_cast<size_t>(2) * D * A * B, 0).total + sizeof(int) * grid_flow_ints(D, A, B, 0);
 }
 
 size_t ftb_grid_rnn_call_workspace_bytes(int D, int A, int B, int N, int H, int dtype) {
   if (D <= 0 || A <= 0 || B <= 0 || N <= 0 || H <= 0 || dtype == FTB_F32) return kWorkspaceBytes;
-  return plan_layout(2 * D * A * B, 0).total + (H <= 256 ? sizeof(int) * grid_flow_ints(D, A, B, N) : 0);
+  return plan_layout(static_cast<size_t>(2) * D * A * B, 0).total + (H <= 256 ? sizeof(int) * grid_flow_ints(D, A, B, N) : 0);
 }
 
 int ftb_gemm_nt(const void* A, const void* Bt, void* out, int M, int N, int K, int dtype, const int* tuning,

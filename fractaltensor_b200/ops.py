@@ -232,7 +232,9 @@ def lstm_stacked_ragged(x, lens, Wp, bias_p=None):
     """Stacked LSTM over a batch of sequences of different lengths, one behind the other and in any order.
 
     x: [T,I] with T = sum(lens), lens: N positive ints; Wp: [D,4H,I+H] -> the top layer's states [T,H] in x's order."""
-    if type(lens) is list and lens and isinstance(x, torch.Tensor) and x.is_cuda and isinstance(Wp, torch.Tensor) and Wp.dim() == 3:
+    # (the lengths have to be x's before a workspace is made for the longest)
+    if (type(lens) is list and lens and isinstance(x, torch.Tensor) and x.is_cuda and x.dim() == 2 and isinstance(Wp, torch.Tensor) and
+            Wp.dim() == 3 and sum(lens) == x.shape[0] and min(lens) > 0):
         ws = workspace(x.device, lib.ftb_lstm_stacked_varlen_workspace_bytes(Wp.shape[0], max(lens)))
         with _turn(ws):
             done = host.lstm_stacked_ragged(x, lens, Wp, bias_p, ws)

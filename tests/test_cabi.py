@@ -93,6 +93,14 @@ def test_bad_arguments_are_rejected_without_a_device(lib):
     assert lib.ftb_lstm_dilated_fwd(one, one, z, one, one, dil, 2, 4, 1, 64, 1, None, one, 256, z) == 1  # dilation 0
 
 
+def test_workspace_sizes_past_two_to_the_31(lib):
+    """Cells are counted in 64 bits: no smaller answer for a larger problem."""
+    for size in (lambda n: lib.ftb_lstm_stacked_varlen_workspace_bytes(n, n), lambda n: lib.ftb_lstm_dilated_workspace_bytes(n, n),
+                 lambda n: lib.ftb_lstm_stacked_workspace_bytes(n, n, 1, 64), lambda n: lib.ftb_grid_rnn_workspace_bytes(1, n, n),
+                 lambda n: lib.ftb_grid_rnn_tables_bytes(1, n, n), lambda n: lib.ftb_grid_rnn_call_workspace_bytes(1, n, n, 1, 64, 1)):
+        assert size(100000) / size(10000) > 95
+
+
 def test_workspace_of_a_grid_goes_by_its_batch(lib):
     """Counters of the kernel with weights on chip: 32 bytes a cell at most, half a byte for one slice."""
     tables = lambda *g: lib.ftb_grid_rnn_tables_bytes(*g)

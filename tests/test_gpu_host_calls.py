@@ -117,3 +117,20 @@ def test_calls_of_the_word_program_through_python_and_native(monkeypatch, dt):
     plain, _ = program()
     assert all(torch.equal(a, b) for a, b in zip(native, plain)) and wrong == errors()
     ops.check_status()
+
+
+def test_lengths_that_are_not_the_rows_cost_no_workspace():
+    """Refused as they were by the Python checks, before the tables of the longest are made."""
+    from fractaltensor_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: (torch.randn(*s, device="cuda", generator=g) * 0.1).half()
+    x, (Wp, b) = r(18, 64), ops.lstm_pack_weights(r(3, 4, 64, 64), r(3, 4, 64, 64), r(3, 4, 64))
+    ops.lstm_stacked_ragged(x, [3, 7, 1, 7], Wp, b)
+    torch.cuda.synchronize()
+    room, held = [w.numel() for w in ops._workspaces.values()], torch.cuda.memory_allocated()
+    for lens in ([1000000], [17, 200000], [3, 7, 1], [2 ** 40], [18 + 2 ** 33, -2 ** 33], [-2, 20], [18, 0], [10 ** 9, 10 ** 9]):
+        with pytest.raises(ValueError):
+            ops.lstm_stacked_ragged(x, lens, Wp, b)
+    with pytest.raises(ValueError):
+        ops.lstm_stacked_ragged(x.reshape(2, 9, 64), [18], Wp, b)
+    assert [w.numel() for w in ops._workspaces.values()] == room and torch.cuda.memory_allocated() <= held
