@@ -109,8 +109,26 @@ def test_calls_of_the_word_program_through_python_and_native(monkeypatch, dt):
             out.append(type(e.value))
         return out
 
+    ops.embedding_gather(table, ids)  # (that call and the projection leave it to the Python checks to make a stream's first workspace)
+    taken = {}
+
+    def recorded(name):
+        native_call = getattr(_lib.host, name)
+
+        def call(*args):
+            done = native_call(*args)
+            taken.setdefault(name, []).append(done is not None and type(done) is not int)
+            return done
+        return call
+
+    names = ["embedding_gather", "lstm_pack_weights", "lstm_stacked_ragged"] + (["project_softmax"] if dt != torch.float32 else [])
+    front = {name: staticmethod(recorded(name)) for name in names}
+    monkeypatch.setattr(ops, "host", type("Host", (_lib._NoHost,), {"current_stream": staticmethod(_lib.host.current_stream), **front}))
     native, none = program()
     assert none is None
+    # every one of them by the native front, not by the Python checks behind it
+    assert taken == {"embedding_gather": [True], "lstm_pack_weights": [True, True], "lstm_stacked_ragged": [True, True],
+                     **({"project_softmax": [True]} if dt != torch.float32 else {})}
     wrong = errors()
     ops.check_status()
     monkeypatch.setattr(ops, "host", type("Host", (_lib._NoHost,), {"current_stream": staticmethod(_lib.host.current_stream)}))
