@@ -83,24 +83,21 @@ struct ClusterArgs {
   int first_cluster[kMaxLayers + 1];  // index of the layer's first cluster
   const void* W;      // Wp [D,4H,2H]
   const float* bias;  // bias_p [D,4H] or nullptr
-  void* out;          // hs [D,L,N,H]
   float* c;           // fp32 [D, max_dil*N, H]
   int* flags;         // [cells][S] counters of CTAs; zero before the launch
   int* status;
 };
 
-// One TMA-fed operand segment of a step: activation rows `row`.. of tensor map `map`, nkb 64-wide K
-// blocks, multiplied with the weight K blocks wkb0.. of this CTA's tile; flags to wait for first.
+// One TMA-fed operand segment of a step: all K blocks of activation rows `row`.. of tensor map `map`; flags to wait for first.
+// The first is the input half's, the second, where there is one, the recurrent half's.
 struct Segment {
-  int map, row, nkb, wkb0;
+  int map, row;
   const int* flags;  // nullptr: an input of the call
   int nflags, target;
 };
 struct StepPlan {
   int nseg;
   Segment seg[2];
-  bool self;       // the cluster's own previous output is an operand (through shared memory)
-  int self_wkb0, self_nkb;
 };
 
 // Shared-memory operand descriptor for an un-swizzled K-major tile: core matrices of 8 rows x 16 B
@@ -134,18 +131,13 @@ __device__ __forceinline__ void umma_commit_to(uint64_t* bar, uint16_t mask) {
       : "memory");
 }
 
-// What this CTA multiplies at time step `i` of its chain (layer, slice).  Every role calls it with the same arguments.
+// What this CTA loads at time step `i` of its chain (layer, slice).  (The state of a layer with dilation 1 comes through shared memory.)
 template <int NB>
 __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, int slice, int i) {
   StepPlan p;
   p.nseg = 0;
-  p.self = false;
-  p.self_wkb0 = p.self_nkb = 0;
-  const int kbh = a.H / BK;
   const int d = a.dil[layer];
   Segment& x = p.seg[p.nseg++];
-  x.nkb = kbh;
-  x.wkb0 = 0;
   if (layer == 0) {
     x.map = 0;
     x.row = i * a.N + slice * NB;
@@ -163,21 +155,13 @@ __device__ __forceinline__ StepPlan plan_step(const ClusterArgs& a, int layer, i
     x.nflags = (row0 + min(slice * NB + NB, a.N) - 1) / nbp - first + 1;
     x.target = a.CL;
   }
-  if (i >= d) {
-    if (d == 1) {
-      p.self = true;
-      p.self_wkb0 = kbh;
-      p.self_nkb = kbh;
-    } else {
-      Segment& h = p.seg[p.nseg++];
-      h.map = 1;
-      h.row = (layer * a.L + i - d) * a.N + slice * NB;
-      h.nkb = kbh;
-      h.wkb0 = kbh;
-      h.flags = a.flags + (layer * a.L + i - d) * a.S + slice;
-      h.nflags = 1;
-      h.target = a.CL;
-    }
+  if (d > 1 && i >= d) {
+    Segment& h = p.seg[p.nseg++];
+    h.map = 1;
+    h.row = (layer * a.L + i - d) * a.N + slice * NB;
+    h.flags = a.flags + (layer * a.L + i - d) * a.S + slice;
+    h.nflags = 1;
+    h.target = a.CL;
   }
   return p;
 }
@@ -348,7 +332,7 @@ __device__ __forceinline__ void cluster_body(const CUtensorMap& mapX, const CUte
             ACCT_END(2);
             ACCT_BEGIN();
             if (fine) {
-              mbar_arrive_expect_tx(&ring_full[stage], sg.nkb * kBlockBytes);
+              mbar_arrive_expect_tx(&ring_full[stage], kbh * kBlockBytes);
               tma_load_3d(s_ring + stage * kStageBytes, maps[sg.map], &ring_full[stage], 0, sg.row, 0);
               *seq = q + 1;
             }
@@ -795,12 +779,9 @@ int make_operand_map(CUtensorMap* out, const void* base, int dtype, uint64_t row
 }
 
 template <typename Kernel, typename... Args>
-int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned long long>& configured, int grid,
-                  uint32_t smem_bytes, cudaStream_t stream, const Args&... args) {
-  // the largest request of this instantiation (static shared memory comes on top of it)
-  constexpr int kMaxDynamic = 225 * 1024;
-  if (smem_bytes > static_cast<uint32_t>(kMaxDynamic) || !ensure_dynamic_smem(kfn, kMaxDynamic, configured))
-    return FTB_ERR_LAUNCH;
+int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned long long>& configured, uint32_t max_dynamic,
+                  int grid, uint32_t smem_bytes, cudaStream_t stream, const Args&... args) {
+  if (smem_bytes > max_dynamic || !ensure_dynamic_smem(kfn, max_dynamic, configured)) return FTB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -845,27 +826,30 @@ int launch_kernel(Kernel kfn, int cluster, int threads, std::atomic<unsigned lon
   return FTB_OK;
 }
 
-template <typename T>
-int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
-  static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, kCtaThreads, configured, grid, smem_bytes, stream, m[0],
-                       m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
-}
-template <typename T>
-int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs (&f)[2], int grid, uint32_t smem_bytes,
-                        cudaStream_t stream) {
-  static std::atomic<unsigned long long> configured{0};
-  return launch_kernel(rnn_dilated_flow_kernel<T>, 1, kCtaThreads, configured, grid, smem_bytes, stream, m, a, f[0],
-                       f[1]);
-}
-
-uint32_t smem_for(bool any_self, int H) {
+constexpr uint32_t smem_for(bool any_self, int H) {
   // worst case over the chains of the launch (slices of 128); must agree with the kernel's carve-up
   constexpr int NB = 128;
   const uint32_t out_tiles = 2u * NB * kOutUnits * 2;
   const uint32_t with_self = 2u * (H / 8) * NB * 16 + 2u * (kOutUnits / 8) * NB * 16 + out_tiles + 4u * kStageBytes;
   const uint32_t without = out_tiles + 12u * kStageBytes;
   return (any_self ? std::max(with_self, without) : without) + 1024;
+}
+// The largest requests of the two kernels: their static shared memory, the barriers of all their bodies, comes on top (227 KB in
+// all; without clusters no state is kept in shared memory, whatever H is).
+constexpr uint32_t kClusterSmem = smem_for(true, 256);
+
+template <typename T>
+int launch_dilated(const CUtensorMap* m, const ClusterArgs& a, int grid, uint32_t smem_bytes, cudaStream_t stream) {
+  static std::atomic<unsigned long long> configured{0};
+  return launch_kernel(rnn_cluster_dilated_kernel<T>, a.CL, kCtaThreads, configured, kClusterSmem, grid, smem_bytes, stream, m[0],
+                       m[1], m[2], m[3], m[4], m[5], m[6], m[7], a);
+}
+template <typename T>
+int launch_dilated_flow(const DilatedMaps& m, const ClusterArgs& a, const flow::FlowArgs (&f)[2], int grid, uint32_t smem_bytes,
+                        cudaStream_t stream) {
+  static std::atomic<unsigned long long> configured{0};
+  return launch_kernel(rnn_dilated_flow_kernel<T>, 1, kCtaThreads, configured, smem_for(false, 256), grid, smem_bytes, stream, m, a, f[0],
+                       f[1]);
 }
 
 }  // namespace
@@ -951,11 +935,11 @@ int dilated_max_clusters(int dtype, int cl, uint32_t smem) {
   cudaError_t e;
   if (dtype == FTB_F16) {
     static std::atomic<unsigned long long> configured{0};
-    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__half>, 225 * 1024, configured)) return 0;
+    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__half>, kClusterSmem, configured)) return 0;
     e = cudaOccupancyMaxActiveClusters(&n, rnn_cluster_dilated_kernel<__half>, &cfg);
   } else {
     static std::atomic<unsigned long long> configured{0};
-    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__nv_bfloat16>, 225 * 1024, configured)) return 0;
+    if (!ensure_dynamic_smem(rnn_cluster_dilated_kernel<__nv_bfloat16>, kClusterSmem, configured)) return 0;
     e = cudaOccupancyMaxActiveClusters(&n, rnn_cluster_dilated_kernel<__nv_bfloat16>, &cfg);
   }
   if (e != cudaSuccess) {
@@ -993,7 +977,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
     a.max_dil = std::max(a.max_dil, dilations[l]);
     any_self = any_self || dilations[l] == 1;
   }
-  a.W = Wp; a.bias = bias_p; a.out = hs; a.c = c; a.flags = flags; a.status = status;
+  a.W = Wp; a.bias = bias_p; a.c = c; a.flags = flags; a.status = status;
   const uint64_t x_rows = static_cast<uint64_t>(L) * N, h_rows = static_cast<uint64_t>(D) * L * N;
   CUtensorMap m[8];
   int rc;

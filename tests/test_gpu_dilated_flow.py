@@ -75,6 +75,23 @@ def test_layers_of_dilation_two(ops, dt, L, N, H, dils):
     _against_levels(ops, dt, L, N, H, dils, 5)
 
 
+@pytest.mark.parametrize("N,H,dils", [(17, 256, [1]), (40, 64, [1, 2]), (256, 256, [1, 2, 4, 8, 16, 32]), (90, 128, [4, 1, 2])])
+def test_schedule_5_is_the_kernel_without_clusters(ops, monkeypatch, N, H, dils):
+    """A refused launch is its error there, and not the generic kernel's result, so that the comparisons above are of this kernel."""
+    from fractaltensor_b200._lib import FtbError
+    D = len(dils)
+    Wp = torch.zeros(D, 4 * H, 2 * H, dtype=torch.float16, device="cuda")
+    x = torch.zeros(5, N, H, dtype=torch.float16, device="cuda")
+    ops.lstm_dilated(x, Wp, dils, schedule=5)
+    monkeypatch.setenv("FTB_REFUSE_COOPERATIVE", "1")
+    with pytest.raises(FtbError) as e:
+        ops.lstm_dilated(x, Wp, dils, schedule=5)
+    assert e.value.code == 5
+    ops.lstm_dilated(x, Wp, dils)  # the automatic choice falls back
+    monkeypatch.undo()
+    ops.check_status()
+
+
 def test_schedule_5_where_it_does_not_apply(ops):
     """No layer of dilation 1: the generic persistent kernel, as for schedule 2."""
     _against_levels(ops, torch.float16, 9, 40, 128, [2, 3], 5)
