@@ -888,7 +888,9 @@ bool dilated_flow_widths(const int* dilations, int D, int N, int H, int CL, int 
   }
   if (!one) return false;
   const double h = H / 128.0 - 1.0;  // -0.5, 0, 1
-  auto flow_step = [&](int w) { return w == 16 ? 1.5 + 0.1 * h : w == 32 ? 1.55 + 0.3 * h : w == 48 ? 1.87 + 0.28 * h : 2.1 + 0.45 * h; };
+  // (not below H 128: at H 64 a step of 16 takes 1.3 and one of 32 1.5, and all is latency)
+  const double hf = std::max(h, 0.0);
+  auto flow_step = [&](int w) { return w == 16 ? 1.5 + 0.1 * hf : w == 32 ? 1.55 + 0.3 * hf : w == 48 ? 1.87 + 0.28 * hf : 2.1 + 0.45 * hf; };
   auto cell = [&](int w, int d) {
     return w == 64 ? std::max(1.15 + 0.35 * h, (3.6 + 1.1 * h) / d) : std::max(1.5 + h, (4.2 + 0.8 * h) / d);
   };
@@ -916,6 +918,11 @@ bool dilated_flow_widths(const int* dilations, int D, int N, int H, int CL, int 
     }
   return best > 0.0;
 }
+// Short sequences of a few narrow states: the arrays that the form without clusters has filled before it starts cost more than its
+// shorter steps give back.  us, with clusters / without, H 64: 4 layers, L 8, N 26 34.8 / 41.2; 6 layers, L 12, N 28 46.2 / 51.3, L 22, N 3
+// 60.2 / 64.7, L 43, N 29 99.5 / 102.6; L 64 and more 0.92 to 1.0 times without, above 64 sequences 0.73 to 0.94; H 128 0.73 to 0.99, H 256
+// 0.62 to 0.98 (400 calls of 8 to 512 steps).
+bool dilated_prefers_clusters(int L, int N, int CL) { return CL == 2 && L < 48 && N <= 64; }
 // Clusters of `cl` CTAs of the dilated kernel that can be resident at once on the current device (a
 // cluster needs its CTAs' SMs inside one GPC, so this is less than SMs / cl: 15 clusters of 8 on a
 // 148-SM B200).  0 when the query fails.
@@ -962,8 +969,7 @@ bool lstm_dilated_cluster_supported(int dtype, int D, int N, int H, int sm_count
 size_t lstm_dilated_cluster_flag_ints(int D, int L) { return static_cast<size_t>(D) * L * 64; }
 
 // x: [L,N,H]; Wp: [D,4H,2H]; hs: [D,L,N,H]; c: [D, max_dil*N, H]; flags: D*L*S ints (zeroed here).  schedule 4: with
-// clusters where they fit, 5: without (FTB_ERR_ARG where that does not fit), 0: without where it fits, which is the faster of the
-// two at every size timed (H 64 to 256, 8 to 256 sequences, 3 and 6 layers: 1.01 to 1.6 times).
+// clusters where they fit, 5: without (FTB_ERR_ARG where that does not fit), 0: the faster of the two.
 int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const float* bias_p, void* hs, float* c,
                                 const int* dilations, int D, int L, int N, int H, int schedule, int* flags, int* status,
                                 int sm_count, cudaStream_t stream) {
@@ -983,7 +989,7 @@ int launch_lstm_dilated_cluster(int dtype, const void* x, const void* Wp, const 
   int rc;
   const uint32_t cluster_smem = smem_for(any_self, H);
   auto cut_for_clusters = [&] { return dilated_slices(dilations, D, N, dilated_max_clusters(dtype, a.CL, cluster_smem), a.nb); };
-  int clusters = schedule == 4 ? cut_for_clusters() : 0;
+  int clusters = schedule == 4 || (schedule == 0 && dilated_prefers_clusters(L, N, a.CL)) ? cut_for_clusters() : 0;
   if (clusters <= 0 && dilated_flow_widths(dilations, D, N, H, a.CL, sm_count, a.nb, a.fold)) {
     int width[2] = {0, 0};  // of the slices of layers that run flow::body, by time steps of a step - 1
     for (int l = 0; l < D; ++l) {
