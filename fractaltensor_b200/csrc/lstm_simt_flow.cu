@@ -101,11 +101,10 @@ __device__ __forceinline__ bool arrived(const uint4& v) {
   return v.x != 0xFFFFFFFFu && v.y != 0xFFFFFFFFu && v.z != 0xFFFFFFFFu && v.w != 0xFFFFFFFFu;
 }
 
-// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: eight 16-byte chunks a lane
-// (four rows, two chunks of each) in flight.  With `poll` a chunk is repeated until its four words are
-// states; the others (inputs of the call) are taken as they are.  Returns the number of rounds of loads
-// beyond the first of each eight.  (Not inlined, like multiply: with both in the kernel's body the registers
-// do not suffice and their loops spill.)
+// Rows 0 .. rows-1 of [.., H] at src -> dst[row][row_words(H)], by warp `w` of `warps`: two 16-byte chunks of each of kInFlight
+// rows a lane in flight.  With `poll` a chunk is repeated until its four words are states; the others (inputs of the call) are
+// taken as they are.  Returns the number of rounds of loads beyond the first.  (Not inlined: beside the multiplications in the
+// kernel's body the registers do not suffice and its loops spill.)
 template <int kInFlight>
 __device__ __noinline__ int load_rows(float* dst, const float* src, int rows, int H, int w, int warps, bool poll,
                                       uint32_t sleep_ns, volatile int* s_abort, int* status) {
@@ -218,6 +217,17 @@ struct StateLoad {
           if (taken[j] & (1u << i)) *reinterpret_cast<uint4*>(dst + i * dst_row + j * (128 + 16)) = v[j][i];
     }
     return extra;
+  }
+};
+
+// 32 rows: 16 loads a lane in flight leave no registers for addresses kept beside the rest (inlined 383 -> 490 us a call).
+template <>
+struct StateLoad<8> {
+  int rows, H, w, warps;
+
+  __device__ __forceinline__ StateLoad(int rows, int H, int w, int warps) : rows(rows), H(H), w(w), warps(warps) {}
+  __device__ __forceinline__ int load(const float* src, float* dst, volatile int* s_abort, int* status) const {
+    return load_rows<8>(dst, src, rows, H, w, warps, true, 0, s_abort, status);
   }
 };
 
@@ -419,11 +429,7 @@ lstm_simt_flow_kernel(const __grid_constant__ SimtFlowArgs a) {
             const long long c0 = clock64();
             while (clock64() - c0 < pause) __nanosleep(20);
           }
-          int extra;
-          if constexpr (TM == 32)
-            extra = load_rows<8>(sS, out, rows, H, warp - C::kLate, C::kLateWarps, true, 0, &s_abort, status);
-          else
-            extra = state.load(out, sS, &s_abort, status);
+          const int extra = state.load(out, sS, &s_abort, status);
           // Everything at the first look: a little earlier next time; else later.  (Looks that come too early
           // load the L2 that the states have to pass through.)
           pause = extra > 0 ? min(pause + 100, kMaxPause) : pause - (pause >> 5);
