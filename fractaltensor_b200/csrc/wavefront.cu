@@ -1532,7 +1532,8 @@ int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const 
   if (static_cast<int64_t>(D) * A * B * N > 0x7fffffffLL) return FTB_ERR_ARG;
   if (!aligned16({X, Y, Wpx, Wpy, bias_x, bias_y, hx, hy})) return FTB_ERR_ALIGN;
   GridFlowPlan flow;
-  if (!grid_flow_form(dtype, D, A, B, N, H, current_sm_count(), nb, &flow)) return FTB_ERR_ARG;
+  // (a named form has at most 32 slices; the automatic choice counts up to 64)
+  if (!grid_flow_form(dtype, D, A, B, N, H, current_sm_count(), nb, &flow) || flow.S > 32) return FTB_ERR_ARG;
   int* status = nullptr;
   const int rc = begin_call(workspace, workspace_bytes, stream, &status);
   if (rc) return rc;

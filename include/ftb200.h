@@ -223,7 +223,7 @@ int ftb_grid_rnn_fwd(const void* X, const void* Y, const void* Wpx, const void* 
                      const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype,
                      void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same with the weights on chip and slices of nb (16, 32 or 64) sequences; FTB_ERR_ARG where there is
+/* The same with the weights on chip and up to 32 slices of nb (16, 32 or 64) sequences; FTB_ERR_ARG where there is
  * no such form.  Any of the 16-bit schedules gives its bits. */
 int ftb_grid_flow_form_fwd(const void* X, const void* Y, const void* Wpx, const void* Wpy, const float* bias_x,
                            const float* bias_y, void* hx, void* hy, int D, int A, int B, int N, int H, int dtype, int nb,

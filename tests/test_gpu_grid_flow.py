@@ -91,13 +91,9 @@ def test_nan_states_are_states(ops):
 def test_forms_that_do_not_exist(ops):
     args = _inputs(ops, 1, 2, 2, 600, 64, torch.float16)
     hx = torch.empty(1, 2, 2, 600, 64, dtype=torch.float16, device="cuda")
-    for nb in (8, 48, 128):
+    for nb in (8, 48, 128, 16):  # 16: more slices than there are counters for
         with pytest.raises(RuntimeError):
             _form(ops, args, nb, hx, torch.empty_like(hx))
-    args = _inputs(ops, 1, 2, 2, 1030, 64, torch.float16)
-    hx = torch.empty(1, 2, 2, 1030, 64, dtype=torch.float16, device="cuda")
-    with pytest.raises(RuntimeError):
-        _form(ops, args, 16, hx, torch.empty_like(hx))  # more slices than there are counters for
 
 
 @pytest.mark.parametrize("D,A,B,N,H", [
