@@ -43,8 +43,7 @@ constexpr int kFirstEpi = 4;
 constexpr int kSlots = 4;    // input tiles
 constexpr int kAhead = 16;   // columns that are filled ahead of the sweep,
 constexpr int kFill = 8;     // so many to a count (two counts ahead: who waits for a count can still do the columns of the one before)
-constexpr int kColumnCounts = 4;  // of a chain, one for each CTA of its group
-constexpr int kMaxPause = 4000;   // cycles
+constexpr int kMaxPause = 4000;  // cycles
 constexpr uint32_t kOneCta = 120 * 1024;  // shared memory of which only one CTA fits on an SM: both would want all of tensor memory
 
 template <int NB, bool kPair>
@@ -71,7 +70,7 @@ struct GridArgs {
   void *hx, *hy;         // [D, A, B, N, H]
   int* ready;            // [D * A * S][counts] CTAs of the chain that have filled these kFill columns
   int counts;            // of a chain
-  int* columns;          // [D * A * S][2 directions][2 tiles] columns of the chain that the layer above can read through TMA
+  int* flags;            // [D * A * B * S * 2] tiles of the cell and direction that can be read through TMA (D > 1)
   int* status;
 };
 
@@ -95,9 +94,6 @@ __device__ __forceinline__ Chain chain_of(const GridArgs& g, int c) {
 }
 __device__ __forceinline__ int* ready_of(const GridArgs& g, int d, int a, int s, int count) {
   return g.ready + (static_cast<int64_t>(d * g.A + a) * g.S + s) * g.counts + count;
-}
-__device__ __forceinline__ int* columns_of(const GridArgs& g, int d, int a, int s, bool ydir) {
-  return g.columns + (static_cast<int64_t>(d * g.A + a) * g.S + s) * kColumnCounts + 2 * ydir;
 }
 
 template <typename T, int NB, bool kPair>
@@ -257,11 +253,9 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
       for (int b = 0; b < g.B && ok; ++b) {
         const int64_t cell = (static_cast<int64_t>(max(ch.d - 1, 0)) * g.A + ch.a) * g.B + b;
         if (ch.d > 0) {
-          if (lane < g.tiles)
-            ok = flag_wait_ge(columns_of(g, ch.d - 1, ch.a, ch.s, ydir) + lane, b + 1, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
+          if (lane == 0) ok = flag_wait_ge(g.flags + (cell * g.S + ch.s) * 2 + ydir, g.tiles, &s_abort, status, FTB_ERR_TIMEOUT_DEP);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          __syncwarp();
           fence_proxy_async_global();  // threads of other CTAs stored what TMA reads
         }
         ok = mbar_wait_warp(&in_empty[slot], phase ^ 1u, &s_abort, status, FTB_ERR_TIMEOUT_SLOT);
@@ -309,7 +303,8 @@ grid_flow_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
           }
           __threadfence_block();
           // (The release takes the other warps' stores along; the proxy fence is the reader's, between its acquire and its copy.)
-          red_release_gpu_add(columns_of(g, ch.d, ch.a, ch.s, ydir) + tile, 1);
+          const int64_t cell = (static_cast<int64_t>(ch.d) * g.A + ch.a) * g.B + b;
+          red_release_gpu_add(g.flags + (cell * g.S + ch.s) * 2 + ydir, 1);
         }
       }
     }
@@ -610,7 +605,7 @@ int launch(const CUtensorMap* m, const GridArgs& g, uint32_t smem, cudaStream_t 
 
 constexpr int kGridMaxSlices = 64;
 static size_t grid_flow_counters(int D, int A, int B, int64_t S) {
-  return static_cast<size_t>(D) * A * S * ((static_cast<size_t>(B) + kFill - 1) / kFill + kColumnCounts);
+  return static_cast<size_t>(D) * A * S * ((static_cast<size_t>(B) + kFill - 1) / kFill + (D > 1 ? 2 * static_cast<size_t>(B) : 0));
 }
 // Counters of a call of N sequences on the narrowest slices; N 0: of any batch.
 size_t grid_flow_ints(int D, int A, int B, int N) {
@@ -685,7 +680,7 @@ int launch_grid_flow(int dtype, const void* X, const void* Y, const void* Wpx, c
   g.Wx = Wpx; g.Wy = Wpy; g.bx = bias_x; g.by = bias_y; g.hx = hx; g.hy = hy;
   g.ready = counters;
   g.counts = (B + kFill - 1) / kFill;
-  g.columns = counters + static_cast<size_t>(D) * A * plan.S * g.counts;
+  g.flags = counters + static_cast<size_t>(D) * A * plan.S * g.counts;
   g.status = status;
   const bool pair = g.tiles == 2;
   const uint32_t held = pair ? plan.nb / 2 : plan.nb, planes = H / BK;
