@@ -129,12 +129,13 @@ int launch(const CUtensorMap& mX, const CUtensorMap& mH, const CUtensorMap& mW, 
 }
 
 // Whether the CTAs of a slice run as pairs: half the state for each of them to read, against hand-overs that wait for both.
-// What they read weighs when all of them read much of it together (rows: of a step, on average).  Single CTAs / pairs, medians over 24 to 29 of 680 calls
-// (D 1..16, N 1..256, L 16..128), by the bytes of states that the whole grid reads a step, H <= 512:
-//   slices of 16: below 0.7 MB 0.97, 0.7..1.1 MB 0.98, 1.1..1.3 MB 1.00, 1.6..2.2 MB 1.02
-//   slices of 32: below 0.6 MB 0.99, 0.9..1.3 MB 1.00, 1.3..1.6 MB 1.02, 2.1..2.6 MB 1.07, 3.3..4.6 MB 1.10
-//   slices of 64: below 0.4 MB 0.99, 0.6..1 MB 1.01, 1..1.4 MB 1.03, 2.5..3.4 MB 1.06, 4.9..6.4 MB 1.22
-// Above H 512, where a warp of a single CTA takes its rows in two rounds: slices of 16 1.19 to 1.24, of 32 1.31 to 1.34.
+// What they read weighs when all of them read much of it together (rows: of a step, on average).  Single CTAs / pairs, medians over 11 to 32 of 721
+// forms of 400 calls (D 1..16, N 1..256, L 16..128), by the bytes of states that the whole grid reads a step, H <= 512:
+//   slices of 16: below 0.8 MB 0.96 to 0.98, 0.9..1.2 MB 1.00, 1.2..1.8 MB 1.01, 1.8..2.3 MB 1.02
+//   slices of 32: below 0.6 MB 0.94 to 0.96, 0.8..1 MB 0.96, 1..1.1 MB 0.98, 1.2..1.6 MB 1.00, 1.6..2 MB 1.04, 2..2.6 MB 1.07, 2.7..4.7 MB 1.10
+//   slices of 64: below 0.4 MB 0.95, 0.5..0.7 MB 0.97, 0.9..1.5 MB 1.00, 1.5..1.9 MB 0.98, 2..2.6 MB 1.03, 2.7..4.1 MB 1.05, 4.3..7.5 MB 1.14 to 1.24
+// (geometric mean of what is taken over the faster of the two: 1.002, 1.003, 1.004; by the best line for these calls 1.002, 1.003, 1.004).
+// Above H 512, where a warp of a single CTA takes its rows in two rounds: slices of 16 1.16 to 1.24, of 32 1.31 to 1.33.
 // Slices of 128 are always pairs: H 128 1.20, 256 1.18.  What pairs save in shared memory lets wider slices of wider layers
 // fit: H 832 on 16 sequences (D7 L28 N15 436 -> 205 us), H 704 on 32, H 640 on 64.
 bool take_pairs(int nb, int G, double rows, int H) {

@@ -1,5 +1,5 @@
 // Device side of the stacked LSTM whose hidden states carry their own arrival: csrc/lstm_flow.cu says how it
-// works.  Also a layer of dilation 1 of the dilated LSTM (csrc/rnn_cluster.cu).
+// works.  Also a layer of dilation 1 or 2 of the dilated LSTM (csrc/rnn_cluster.cu).
 #pragma once
 
 #include "ptx.cuh"
@@ -46,7 +46,7 @@ struct FlowArgs {
   void* hs;             // [D, T, H], all 0xFFFF before the launch
   float* c_out;         // [D, c_rows, H], the first N of c_rows
   int c_rows;
-  int* flags;           // [D * L * S] tiles of the slice's cell (l, t) that can be read through TMA
+  int* flags;           // [D][flag_steps][S] tiles of the slice's cell (l, t) that can be read through TMA
   // A layer of the dilated LSTM whose step is `fold` time steps of N1 sequences (N = fold * N1, the last step may be short).
   // fold 0: a step is a time step in every layer.
   int fold, N1;

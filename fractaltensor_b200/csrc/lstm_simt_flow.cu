@@ -14,8 +14,9 @@
 //     multiplies per word it reads is the rate: 8 rows x 8 columns of one 32-wide K chunk, four products a word;
 //   * TM is 8, 16 or 32: small batches multiply no rows that are not there, and small models spread theirs
 //     over the device.
-// A step of 32 rows in cycles: the recurrent half's multiplication 4200 of 10 000, its sums 800, two cells a thread 1160, the
-// state's trip and loads 3600; of 8 rows 1300, 400, 620 and 1500 of 4000.  Against one serial pass (us, D x L x N x H): 4 x 64 x 32 x
+// A step of 32 rows in cycles (stamps of one CTA): the recurrent half's multiplication 4840 of 10 450, its sums 850, two cells a thread
+// 1080, the pause before the first look 450, the states 2920; of 16 rows 2240 of 5490, 480, 600, 550 and 1430; of 8 rows 1110 of 3930,
+// 430, 610, 410 and 1130.  Against one serial pass (us, D x L x N x H): 4 x 64 x 32 x
 // 256 550 -> 385, 4 x 64 x 16 x 256 526 -> 218, 2 x 64 x 8 x 256 499 -> 151.
 // The sums are the level kernel's (csrc/cell_simt.cu): every chunk of 32 in ascending order, a group's chunks in
 // order, the four groups in order; all fp32 schedules give the same bits.

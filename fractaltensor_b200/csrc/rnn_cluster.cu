@@ -1,9 +1,12 @@
-// A latency-bound recurrence with small hidden size (H <= 256): the dilated stacked LSTM, one thread-block
-// cluster per chain of dependent steps.  (The grid RNN: csrc/grid_flow.cu.)
+// A latency-bound recurrence with small hidden size (H <= 256): the dilated stacked LSTM.  (The grid RNN: csrc/grid_flow.cu.)
 //
-// The program is chains of small cells: 512 dependent steps of [256 x 512].[512 x 1024] in the first layer.  Run as a generic wavefront, every dependent level costs a trip through
-// global memory (store, fence, flag, poll, TMA load: 6-9 us) plus a re-read of the layer's
-// weights from L2.  Here
+// The program is chains of small cells: 512 dependent steps of [256 x 512].[512 x 1024] in the first layer.  Run as a generic
+// wavefront, every dependent level costs a trip through global memory (store, fence, flag, poll, TMA load: 6-9 us) plus a
+// re-read of the layer's weights from L2.  Two kernels keep the weights on chip.  rnn_dilated_flow_kernel, the choice nearly
+// wherever it fits, has no clusters: layers of dilation 1 and 2 run flow::body (lstm_flow.cuh), whose states are their own flags,
+// the others cluster_body with one CTA in place of each of a cluster's.  rnn_cluster_dilated_kernel, for short sequences of a few
+// narrow states and for what the other one has too few SMs for, runs cluster_body for all layers, a thread-block cluster per chain of
+// dependent steps.  There
 //   * the weights never move: a cluster of CL CTAs owns one chain (one layer and batch slice), CTA r of the
 //     cluster owns 128 packed weight rows (32 LSTM units x 4 gates) for the whole launch, and that slice of the
 //     weights sits in tensor memory as the A operand of every MMA ("recurrent weights resident on chip");
@@ -729,8 +732,8 @@ rnn_cluster_dilated_kernel(const __grid_constant__ CUtensorMap x128, const __gri
 }
 
 // The same program without clusters, where it fits: what the layers with dilation >= 2 exchange goes through
-// global memory anyway (2.2 us a step on slices of 64; on 128 a layer with dilation 2, which waits for the trip
-// there and back, takes 3.0).  A layer with dilation 1 runs as csrc/lstm_flow.cu does, on narrow slices whose state is
+// global memory anyway (at H 256 a step takes 1.5 us on slices of 64, 2.5 on 128, or its part of the trip there and back,
+// 4.7 and 5.0 over the dilation: 2.35 on slices of 64 with dilation 2).  A layer with dilation 1 runs as csrc/lstm_flow.cu does, on narrow slices whose state is
 // its own flag: 1.6 us a step at H 256 and 32 sequences where a cluster's hand-off of 64 takes 2.6, and no GPC has to
 // hold a chain's CTAs (15 clusters of 8 leave 28 SMs idle).  A layer with dilation 2 does so too where its slices fit: as a layer
 // of 2 N sequences and half the steps, whose trip there and back it no longer waits for (dilated_flow_widths).

@@ -271,7 +271,7 @@ def lstm_dilated(x, Wp, dilations, bias_p=None, hs=None, c=None, bn=0, pair=0, s
     """x: [L,N,H]; Wp: [D,4H,2H]; dilations: D ints -> (hs [D,L,N,H], c fp32 [D,max_dil*N,H]).
     schedule: 0 auto, 1 one launch per level, 2 generic persistent kernel; H of 64, 128 or 256, weights resident in
     tensor memory: 4 one thread-block cluster per layer and batch slice, 5 no clusters, states of layers with
-    dilation 1 through the output array."""
+    dilation 1, and 2 where their slices fit, through the output array."""
     _req(x, "x")
     _req(Wp, "Wp", x.dtype)
     L, N, H = x.shape

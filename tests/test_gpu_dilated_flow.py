@@ -1,5 +1,5 @@
-"""Dilated LSTM without clusters (csrc/rnn_cluster.cu): layers of dilation 1 on slices of 16, 32 or 48 sequences
-that hand their state on through the output array, the others on slices of 64 or 128; bit for bit the
+"""Dilated LSTM without clusters (csrc/rnn_cluster.cu): layers of dilation 1 on slices of 16, 32 or 48 sequences, and of
+dilation 2 where they fit, hand their state on through the output array, the others are on slices of 64 or 128; bit for bit the
 result of one launch per level."""
 import pytest
 import torch
@@ -29,7 +29,7 @@ def test_same_bits_as_levels(ops, dt, L, N, H, dils):
 
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("L,N,H,dils", [
-    (9, 33, 128, [1]),              # the automatic choice at 2 and 4 CTAs and up to 64 sequences
+    (9, 33, 128, [1]),              # clusters of 4 CTAs, here and below; then of 2
     (20, 64, 128, [1, 2, 4]),
     (20, 64, 64, [1, 1, 2]),
     (7, 5, 64, [1, 3]),
@@ -40,7 +40,7 @@ def test_same_bits_as_levels(ops, dt, L, N, H, dils):
 ])
 @pytest.mark.parametrize("schedule", [4, 0])
 def test_clusters_same_bits_as_levels(ops, dt, L, N, H, dils, schedule):
-    """One thread-block cluster per layer and slice (schedule 4), which the automatic choice takes for some of these."""
+    """One thread-block cluster per layer and slice (schedule 4); the automatic choice takes it for short sequences of 64 units."""
     _against_levels(ops, dt, L, N, H, dils, schedule)
 
 

@@ -1164,7 +1164,7 @@ def test_embed_lstm_projection_chain(ops):
         pos += n
 
 
-# ------------------------------------- cluster kernels of the dilated LSTM and the grid RNN
+# ------------------- dilated LSTM by clusters, grid RNN: weights on chip
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("case", [
     (1, 3, 32, 256, [1]), (1, 9, 128, 256, [1]), (2, 8, 128, 256, [1, 2]), (3, 19, 200, 256, [1, 2, 4]),
@@ -1173,7 +1173,7 @@ def test_embed_lstm_projection_chain(ops):
 def test_dilated_cluster_schedule(ops, dt, case):
     """The cluster kernel (weights in tensor memory, the state of dilation-1 layers through the cluster's
     shared memory, everything else through global flags): the same bits as one launch per level, for
-    batches that fill, underfill and overflow the 128-sequence slices, and it is the automatic choice."""
+    batches that fill, underfill and overflow the 128-sequence slices; the automatic choice and the generic kernel too."""
     D, L, N, H, dils = case
     x, W, U, b = dense.make_lstm_inputs(D, L, N, H, H, 4, 1.0 / 8, dtype=dt, bias=True)
     xd, Wd, Ud, bd = _dev(x, W, U, b)
@@ -1204,8 +1204,7 @@ def test_dilated_cluster_schedule_needs_its_shapes(ops):
 @pytest.mark.parametrize("shape", [(1, 1, 4, 64, 256), (1, 3, 4, 16, 256), (2, 3, 4, 64, 128), (1, 9, 7, 64, 256),
                                    (1, 5, 6, 100, 256), (1, 32, 2, 3, 256), (3, 2, 5, 64, 128)])
 def test_grid_cluster_schedule(ops, dt, shape):
-    """The cluster kernel of the grid RNN (one cluster per grid row and batch slice; h_y to the next column
-    through the cluster's shared memory, h_x of the row above through global flags): the same bits as
+    """The automatic choice, weights on chip and states that carry their own arrival (csrc/grid_flow.cu): the same bits as
     one launch per anti-diagonal and as the generic persistent kernel."""
     D, A, B, N, H = shape
     X, Y, p = dense.make_grid_inputs(D, A, B, N, H, 6, 1.0 / 8, dtype=dt, bias=True)
