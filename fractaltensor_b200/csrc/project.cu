@@ -413,8 +413,13 @@ int launch_passes(const CUtensorMap& mA, const CUtensorMap& mB, const ProjectArg
 
 // What the kernel takes, and where it is the faster form: rows that begin on 16 bytes (for others the stores go singly, and
 // cost what the logits did), and behind a packed operand only where the logits are many.  us, product and softmax / twice:
-// unpacked, H 512, V 10000: 40 words 22.5 / 21.0, 300 30.6 / 28.8, 2240 79.9 / 52.3, 5000 170 / 94.6; V 2000: 300 20.5 / 18.6, 5000 43.1 / 39.0;
-// packed: V 2004, 300 words 23.6 / 26.0, 5000 45.1 / 46.2; V 10004, 2240 words 83.3 / 69.0; V 10001, 2240 words 90.3 / 91.5.
+// unpacked (packing counted), H 512, V 10000: 40 words 21.3 / 22.8, 300 29.0 / 29.1, 2240 79.2 / 49.5, 5000 169 / 97.2; V 2000: 300 22.6 /
+// 20.6, 5000 48.6 / 39.3.  Packed, by millions of probabilities (90 calls of 64 to 20000 words, V 200 to 40000, H 64 to 640; twice as a
+// share of product and softmax): up to 4 1.15, 4 to 8 1.07, 8 to 12 0.98, 12 to 16 0.84, 16 to 30 0.80, 30 to 60 0.65, more 0.63.
+// V 10004: 1000 words 37.0 / 35.8, 1600 50.5 / 43.4, 2240 71.4 / 52.9, 5000 160 / 110.  The line stays at 16 million, not at 12: this
+// kernel's probabilities are 1.04 to 1.15 times as far from 64 bits.  (Rows on 16 bytes and not on 32, V % 8 == 4: runs of 64 bytes
+// touch three sectors.  Through whole rows in shared memory the largest were up to 7 % faster, 17732 x 5884 x 512 214 / 229, and all
+// others slower, 0.957 of it on average; runs of 128 bytes by another exchange 4 to 15 % slower, but for the largest.)
 bool project_twice_supported(int dtype, long long T, int V, int H, bool unpacked) {
   return (dtype == FTB_F16 || dtype == FTB_BF16) && H % BK == 0 && H <= kMaxKBlocks * BK &&
          (unpacked ? V % 8 == 0 : V % 4 == 0 && T * V >= 16000000);

@@ -86,6 +86,19 @@ def test_packed_operand_of_many_logits(ops):
     assert (ops.project_softmax_rows(h, P4).double() - torch.softmax(h.double() @ P4.double(), -1)).abs().max().item() <= 1e-5
 
 
+@pytest.mark.parametrize("T,V,twice", [(1599, 10004, False), (1600, 10004, True), (1600, 10000, True), (16002, 1002, False), (800, 20004, True)])
+def test_packed_operand_around_the_rule(ops, T, V, twice):
+    """16 million probabilities, rows on 16 and on 32 bytes, and rows on neither: the same within rounding on both sides."""
+    from fractaltensor_b200._lib import DTYPE_F16, lib
+    assert (lib.ftb_project_softmax_scratch_bytes(T, V, 128, DTYPE_F16, 0) > 0) == twice
+    g = torch.Generator(device="cuda").manual_seed(T)
+    P, h = torch.randn(128, V, device="cuda", generator=g).half(), torch.randn(T, 128, device="cuda", generator=g).half()
+    got, padded = ops.lstm_project_softmax_rows(h, ops.projection_pack(P), V), ops.lstm_project_softmax(h, ops.projection_pack(P), V)
+    ops.check_status()
+    # (logits of magnitude up to about 60: 60 * 2^-24 of them, and as much of a probability)
+    assert torch.equal(got, padded) and (got.double() - torch.softmax(h.double() @ P.double(), -1)).abs().max().item() <= 1e-5
+
+
 def test_rows_that_are_not_finite(ops):
     """A row of logits with a NaN or +inf is NaN, the others are untouched."""
     g = torch.Generator(device="cuda").manual_seed(5)
